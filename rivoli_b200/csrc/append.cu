@@ -22,6 +22,8 @@ __global__ void append_kv_slab_kernel(const float* __restrict__ latent, const fl
                                       int n_blocks) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int blk = warp;  // kvl/128 warps
+    rv_grid_dep_trigger();
+    rv_grid_dep_wait();
     const float* src = latent + blk * 128 + lane * 4;  // scalar loads: no alignment demand on the caller
     const float4 v = make_float4(src[0], src[1], src[2], src[3]);
     float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
@@ -40,13 +42,16 @@ RIVOLI_API int rivoli_append_kv(const float* latent, const float* rope, unsigned
     if (pos < 0 || kvl <= 0 || ropn <= 0 || n_blocks <= 0) return 1001;
     if (kvl > 1024 || kvl < 128 || (kvl % 128) != 0 || ropn > kvl) return 1002;
     rv_drain_error();
-    append_kv_slab_kernel<<<1, (kvl / 128) * 32>>>(latent, rope, lc8, lscale, rc, pos, kvl, ropn, n_blocks);
+    rv_launch_dependent(append_kv_slab_kernel, dim3(1), dim3((unsigned)(kvl / 128) * 32), 0, (cudaStream_t)0, latent, rope, lc8, lscale, rc, pos,
+                        kvl, ropn, n_blocks);
     return rv_launch_status();
 }
 
 __global__ void gather_rope_kernel(const float* __restrict__ q, float* __restrict__ qrope, int h, int qh,
                                    int nope, int ropn) {
     int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    rv_grid_dep_trigger();
+    rv_grid_dep_wait();
     if (idx >= h * ropn) return;
     qrope[idx] = q[(size_t)(idx / ropn) * qh + nope + idx % ropn];
 }
@@ -54,20 +59,22 @@ __global__ void gather_rope_kernel(const float* __restrict__ q, float* __restric
 RIVOLI_API int rivoli_gather_rope(const float* q, float* qrope, int h, int qh, int nope, int ropn) {
     if (h <= 0 || qh <= 0 || nope < 0 || ropn <= 0) return 1001;
     rv_drain_error();
-    gather_rope_kernel<<<(h * ropn + 255) / 256, 256>>>(q, qrope, h, qh, nope, ropn);
+    rv_launch_dependent(gather_rope_kernel, dim3((unsigned)(h * ropn + 255) / 256), dim3(256), 0, (cudaStream_t)0, q, qrope, h, qh, nope, ropn);
     return rv_launch_status();
 }
 
 __global__ void index_append_slab_kernel(const float* __restrict__ k, unsigned short* __restrict__ kcache,
                                          int pos, int hd) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
+    rv_grid_dep_trigger();
+    rv_grid_dep_wait();
     if (i < hd) kcache[(size_t)pos * hd + i] = rv_f32_to_bf16(k[i]);
 }
 
 RIVOLI_API int rivoli_index_append(const float* k, unsigned short* kcache, int pos, int hd) {
     if (hd <= 0 || pos < 0) return 1001;
     rv_drain_error();
-    index_append_slab_kernel<<<(hd + 255) / 256, 256>>>(k, kcache, pos, hd);
+    rv_launch_dependent(index_append_slab_kernel, dim3((unsigned)(hd + 255) / 256), dim3(256), 0, (cudaStream_t)0, k, kcache, pos, hd);
     return rv_launch_status();
 }
 

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/rivoli_kernels.h"
 
 #define RIVOLI_API extern "C" __attribute__((visibility("default")))
@@ -34,6 +36,20 @@ static inline void rv_launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3
     cfg.attrs = at; cfg.numAttrs = 1;
     (void)cudaLaunchKernelEx(&cfg, kernel, args...);   // the caller reads the launch status afterwards
 }
+
+// Opts a kernel in to `bytes` of dynamic shared memory, once per kernel and device (the attribute lives as long as the
+// context; setting it costs the host about half a microsecond). `bytes` is the most that any launch of this kernel asks
+// for, so threads that race to the first call set the same value.
+template <auto Kernel>
+static inline void rv_allow_smem(int bytes) {
+    static std::atomic<uint64_t> done{0};
+    int dev = 0;
+    (void)cudaGetDevice(&dev);
+    const uint64_t bit = 1ull << (dev & 63);
+    if (dev < 64 && (done.load(std::memory_order_acquire) & bit)) return;
+    if (cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess)
+        done.fetch_or(dev < 64 ? bit : 0, std::memory_order_release);
+}
 #endif
 
 // Measurement hook (rivoli_dsa_step_set_timing_events): when set, the decode-step entry points record event k
@@ -47,6 +63,13 @@ static inline void rv_stage_event(int k, cudaStream_t st) {
 }
 
 static inline bool rv_is_pow2(int x) { return x > 0 && (x & (x - 1)) == 0; }
+__host__ __device__ __forceinline__ int rv_log2(int x) {   // of a power of two
+#ifdef __CUDA_ARCH__
+    return 31 - __clz(x);
+#else
+    return 31 - __builtin_clz((unsigned)x);
+#endif
+}
 
 // Geometry guard shared by every paged entry point. Decided on the host; nothing is
 // dereferenced on the device when it fails.

@@ -15,32 +15,10 @@
 //       rivoli_index_select_paged take.
 #include "codec.cuh"
 #include "common.cuh"
+#include "fold_gemv.cuh"
 #include "tc_common.cuh"
 
 namespace {
-
-__device__ __forceinline__ int if_shift(int block) { return 31 - __clz(block); }
-
-template <int R>
-__global__ void __launch_bounds__(256)
-gemv_fp8_kernel(const float* __restrict__ x, const uint8_t* __restrict__ packed, const float* __restrict__ scale,
-                int o_dim, int i_dim, int block, float* __restrict__ y) {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= o_dim) return;
-    const int bsh = if_shift(block), sc_cols = (i_dim + block - 1) / block;
-    const uint8_t* row = packed + (size_t)o * i_dim;
-    const float* srow = scale + (size_t)(o >> bsh) * sc_cols;
-    float acc[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) acc[r] = 0.0f;
-    for (int i = 0; i < i_dim; ++i) {
-        const float ws = __fmul_rn(rv_e4m3_to_f32(row[i]), srow[i >> bsh]);
-#pragma unroll
-        for (int r = 0; r < R; ++r) acc[r] = __fadd_rn(acc[r], __fmul_rn(ws, x[(size_t)r * i_dim + i]));
-    }
-#pragma unroll
-    for (int r = 0; r < R; ++r) y[(size_t)r * o_dim + o] = acc[r];
-}
 
 // One block; sums in f64 (the reference's host test removes the summation-order error the same way),
 // then the reference's f32 formula with var = E[x^2] - mean^2.
@@ -49,6 +27,8 @@ layernorm_kernel(const float* __restrict__ x, const float* __restrict__ w, const
                  float eps, float* __restrict__ y) {
     __shared__ double ss[256], sq[256];
     const int t = threadIdx.x;
+    rv_grid_dep_trigger();
+    rv_grid_dep_wait();
     double s = 0.0, q = 0.0;
     for (int i = t; i < n; i += 256) { const double v = (double)x[i]; s += v; q += v * v; }
     ss[t] = s; sq[t] = q;
@@ -63,19 +43,18 @@ layernorm_kernel(const float* __restrict__ x, const float* __restrict__ w, const
     for (int i = t; i < n; i += 256) y[i] = __fadd_rn(__fmul_rn(__fmul_rn(__fsub_rn(x[i], mean), inv), w[i]), b[i]);
 }
 
-__device__ __forceinline__ void rope_pair(float a, float b, int j, int seg, int pos, double theta, float* lo, float* hi) {
-    const double ang = (double)pos * pow(theta, -2.0 * (double)j / (double)seg);
-    const float cs = (float)cos(ang), sn = (float)sin(ang);
-    *lo = __fsub_rn(__fmul_rn(a, cs), __fmul_rn(b, sn));
-    *hi = __fadd_rn(__fmul_rn(b, cs), __fmul_rn(a, sn));
-}
-
 __global__ void rope_interleave_kernel(float* __restrict__ base, int stride, int seg, int pos, double theta) {
     const int s = blockIdx.x, j = threadIdx.x, half = seg / 2;
     float* v = base + (size_t)s * stride;
+    rv_grid_dep_trigger();
+    // the angle (f64) needs nothing from the kernel before
+    const double ang = (double)pos * pow(theta, -2.0 * (double)j / (double)seg);
+    const float cs = (float)cos(ang), sn = (float)sin(ang);
+    rv_grid_dep_wait();
     const float a = v[2 * j], b = v[2 * j + 1];
     __syncthreads();   // every pair is read before any element is written: in place, race free
-    rope_pair(a, b, j, seg, pos, theta, &v[j], &v[half + j]);
+    v[j] = __fsub_rn(__fmul_rn(a, cs), __fmul_rn(b, sn));
+    v[half + j] = __fadd_rn(__fmul_rn(b, cs), __fmul_rn(a, sn));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -105,7 +84,7 @@ front_gemm_simt_kernel(FrontArgs A) {
     const int kper = ((J.K + J.k_splits - 1) / J.k_splits + FT_KC - 1) / FT_KC * FT_KC;
     const int k0 = split * kper, k1 = min(J.K, k0 + kper);
     const int o = tile * FT_N + (threadIdx.x & 63), bq = threadIdx.x >> 6;   // this kernel always plans tile_n == FT_N
-    const int bsh = if_shift(A.block), sc_cols = (J.K + A.block - 1) / A.block;
+    const int bsh = rv_log2(A.block), sc_cols = (J.K + A.block - 1) / A.block;
     // sequences bq, bq + 4, ... ; at most 32 accumulators per thread per pass
     for (int b0 = 0; b0 < A.B; b0 += 128) {
         float acc[32];
@@ -428,9 +407,8 @@ RIVOLI_API int rivoli_gemv_fp8(const float* x, const unsigned char* packed, cons
     if (block & (block - 1)) return 1003;
     if (nrow != 1 && nrow != 2) return 1004;
     rv_drain_error();
-    if (nrow == 2) gemv_fp8_kernel<2><<<ceil_div(o_dim, 256), 256>>>(x, packed, scale, o_dim, i_dim, block, y);
-    else gemv_fp8_kernel<1><<<ceil_div(o_dim, 256), 256>>>(x, packed, scale, o_dim, i_dim, block, y);
-    return rv_launch_status();
+    return launch_fold_gemv(FoldGemv{x, (size_t)i_dim, 0, packed, 0, 0, scale, rv_log2(block), ceil_div(i_dim, block), i_dim, o_dim,
+                                     y, (size_t)o_dim, 0, 0, 0}, 1, nrow, 0);
 }
 
 // The reference switches to a split-K kernel for long rows (linalg.hip:296-321); here both names run the
@@ -443,7 +421,7 @@ RIVOLI_API int rivoli_gemv_fp8_splitk(const float* x, const unsigned char* packe
 RIVOLI_API int rivoli_layernorm(const float* x, const float* w, const float* b, int n, float eps, float* y) {
     if (n <= 0) return 1001;
     rv_drain_error();
-    layernorm_kernel<<<1, 256>>>(x, w, b, n, eps, y);
+    rv_launch_dependent(layernorm_kernel, dim3(1), dim3(256), 0, (cudaStream_t)0, x, w, b, n, eps, y);
     return rv_launch_status();
 }
 
@@ -451,7 +429,7 @@ RIVOLI_API int rivoli_rope_interleave(float* base, int count, int stride, int se
     if (count <= 0 || seg <= 0 || (seg & 1) || (seg / 2) > 1024) return 1001;
     if (count > 1 && stride < seg) return 1001;
     rv_drain_error();
-    rope_interleave_kernel<<<count, seg / 2>>>(base, stride, seg, pos, theta);
+    rv_launch_dependent(rope_interleave_kernel, dim3((unsigned)count), dim3((unsigned)(seg / 2)), 0, (cudaStream_t)0, base, stride, seg, pos, theta);
     return rv_launch_status();
 }
 

@@ -1,8 +1,8 @@
 // The two contractions through kv_b either side of MLA attention.
 //
 //   rivoli_mla_absorb_fp8 / rivoli_mla_value_fp8 : the reference's single-token f32 operators
-//       (crates/backend/kernels/mla.hip:12-231): same symbols, arguments, guard codes. One thread
-//       per output, the reference's fold order (d, resp. i, ascending; q * (e4m3 * scale)), no
+//       (crates/backend/kernels/mla.hip:12-231): same symbols, arguments, guard codes. The
+//       reference's fold order (d, resp. i, ascending; q * (e4m3 * scale)), no
 //       contraction - bit-identical to the host references of its tests
 //       (crates/engine/tests/kernel_attend.rs:361-390).
 //   rivoli_mla_absorb_batched_bf16 / rivoli_mla_value_batched_bf16 : the batched decode form
@@ -12,54 +12,79 @@
 // kv_b: e4m3 codes [H*(nope+vh) rows][kvl cols], scale[(row / block) * ceil(kvl/block) + col / block].
 #include "codec.cuh"
 #include "common.cuh"
+#include "fold_gemv.cuh"
+#include "tc_common.cuh"
 
 namespace {
 
-__device__ __forceinline__ int kp_shift(int block) { return 31 - __clz(block); }
+// One output column per pair of lanes' 16-bit word: thread t owns the columns 2t, 2t + 1 of the CTA's 128, for R query
+// rows, and folds over d. What bounds it: 6.3 MB of codes (1 us) and a chain of nope additions; the codes of up to
+// AB_DCH rows are requested at once (16-byte copies into shared memory, 24 KB of the CTA's 128 columns) so that the
+// chain never waits for memory. 64 threads per 128 columns keep every scheduler of 148 SMs busy with 64 heads x 4
+// blocks. One thread per column with byte loads from global memory took 81 us at 64 x 512 x 192; this takes 5.1.
+constexpr int AB_COLS = 128, AB_THREADS = 64, AB_DCH = 192;
 
-template <int R>
-__global__ void __launch_bounds__(256)
+template <int R, bool VEC>
+__global__ void __launch_bounds__(AB_THREADS)
 absorb_f32_kernel(const float* __restrict__ q, const uint8_t* __restrict__ kvb, const float* __restrict__ scale, int H,
                   int qh, int nope, int vh, int kvl, int block, float* __restrict__ qabs) {
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (size_t)H * kvl) return;
-    const int head = (int)(idx / kvl), i = (int)(idx % kvl);
-    const int bsh = kp_shift(block), sc_cols = (kvl + block - 1) / block;
+    __shared__ __align__(16) uint8_t codes[AB_DCH][AB_COLS];
+    __shared__ float qs[R][AB_DCH];
+    const int tid = threadIdx.x, head = blockIdx.y, c0 = blockIdx.x * AB_COLS, i = c0 + 2 * tid;
+    const int bsh = rv_log2(block), sc_cols = (kvl + block - 1) / block;
     const size_t rbase = (size_t)head * (nope + vh);
-    float acc[R];
+    const int cols = min(AB_COLS, kvl - c0);
+    rv_grid_dep_trigger();
+    for (int d = tid; d < nope; d += AB_THREADS)              // (a prefetch returns no data: safe before the wait)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(kvb + (rbase + d) * kvl + c0));
+    rv_grid_dep_wait();
+    float acc[R][2];
 #pragma unroll
-    for (int r = 0; r < R; ++r) acc[r] = 0.0f;
-    for (int d = 0; d < nope; ++d) {
-        const size_t row = rbase + d;
-        const float ws = __fmul_rn(rv_e4m3_to_f32(kvb[row * kvl + i]), scale[(row >> bsh) * sc_cols + (i >> bsh)]);
+    for (int r = 0; r < R; ++r) acc[r][0] = acc[r][1] = 0.0f;
+    for (int d0 = 0; d0 < nope; d0 += AB_DCH) {
+        const int dn = min(AB_DCH, nope - d0);
+        __syncthreads();
+        if (VEC) {
+            for (int e = tid; e < dn * (AB_COLS / 16); e += AB_THREADS) {
+                const int d = e >> 3, c = (e & 7) * 16;
+                if (c < cols) tc::cp_async16(tc::smem_u32(&codes[d][c]), kvb + (rbase + d0 + d) * kvl + c0 + c);
+            }
+            tc::cp_async_commit();
+        } else {
+            for (int e = tid; e < dn * AB_COLS; e += AB_THREADS) {
+                const int d = e >> 7, c = e & 127;
+                if (c < cols) codes[d][c] = kvb[(rbase + d0 + d) * kvl + c0 + c];
+            }
+        }
 #pragma unroll
-        for (int r = 0; r < R; ++r) acc[r] = __fadd_rn(acc[r], __fmul_rn(q[(size_t)r * H * qh + (size_t)head * qh + d], ws));
+        for (int r = 0; r < R; ++r)
+            for (int d = tid; d < dn; d += AB_THREADS) qs[r][d] = q[(size_t)r * H * qh + (size_t)head * qh + d0 + d];
+        if (VEC) tc::cp_async_wait<0>();
+        __syncthreads();
+        if (2 * tid >= cols) continue;
+        for (int d = 0; d < dn;) {
+            // rows up to the next scale block share their scales
+            const size_t row = rbase + d0 + d;
+            const int stop = min(dn, d + (int)(block - (row & (size_t)(block - 1))));
+            const float* srow = scale + (row >> bsh) * sc_cols;
+            const float s0 = srow[i >> bsh], s1 = i + 1 < kvl ? srow[(i + 1) >> bsh] : 0.0f;
+#pragma unroll 8
+            for (; d < stop; ++d) {
+                const float2 f = rv_e4m3x2_to_f32x2(*reinterpret_cast<const uint16_t*>(&codes[d][2 * tid]));
+                const float w0 = __fmul_rn(f.x, s0), w1 = __fmul_rn(f.y, s1);
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    acc[r][0] = __fadd_rn(acc[r][0], __fmul_rn(qs[r][d], w0));
+                    acc[r][1] = __fadd_rn(acc[r][1], __fmul_rn(qs[r][d], w1));
+                }
+            }
+        }
     }
 #pragma unroll
-    for (int r = 0; r < R; ++r) qabs[(size_t)r * H * kvl + idx] = acc[r];
-}
-
-template <int R>
-__global__ void __launch_bounds__(256)
-value_f32_kernel(const float* __restrict__ clat, const uint8_t* __restrict__ kvb, const float* __restrict__ scale, int H,
-                 int nope, int vh, int kvl, int block, float* __restrict__ ctx) {
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (size_t)H * vh) return;
-    const int head = (int)(idx / vh), j = (int)(idx % vh);
-    const int bsh = kp_shift(block), sc_cols = (kvl + block - 1) / block;
-    const size_t row = (size_t)head * (nope + vh) + nope + j;
-    const uint8_t* w = kvb + row * kvl;
-    const float* srow = scale + (row >> bsh) * sc_cols;
-    float acc[R];
+    for (int r = 0; r < R; ++r)
 #pragma unroll
-    for (int r = 0; r < R; ++r) acc[r] = 0.0f;
-    for (int i = 0; i < kvl; ++i) {
-        const float ws = __fmul_rn(rv_e4m3_to_f32(w[i]), srow[i >> bsh]);
-#pragma unroll
-        for (int r = 0; r < R; ++r) acc[r] = __fadd_rn(acc[r], __fmul_rn(clat[(size_t)r * H * kvl + (size_t)head * kvl + i], ws));
-    }
-#pragma unroll
-    for (int r = 0; r < R; ++r) ctx[(size_t)r * H * vh + idx] = acc[r];
+        for (int e = 0; e < 2; ++e)
+            if (i + e < kvl) qabs[((size_t)r * H + head) * kvl + i + e] = acc[r][e];
 }
 
 // Batched bf16, any geometry: one thread per (sequence, head, output), the same folds.
@@ -75,7 +100,7 @@ absorb_batched_simt_kernel(const uint16_t* __restrict__ q, const uint8_t* __rest
     const int head = (int)(bh % H);
     const uint16_t* qr = q + bh * qh;
     if (i >= kvl) { q_abs[idx] = qr[nope + (i - kvl)]; return; }   // the rope segment rides along, bit for bit
-    const int bsh = kp_shift(block), sc_cols = (kvl + block - 1) / block;
+    const int bsh = rv_log2(block), sc_cols = (kvl + block - 1) / block;
     const size_t rbase = (size_t)head * (nope + vh);
     float acc = 0.0f;
     for (int d = 0; d < nope; ++d) {
@@ -95,7 +120,7 @@ value_batched_simt_kernel(const uint16_t* __restrict__ clat, const uint8_t* __re
     const int j = (int)(idx % vh);
     const size_t bh = idx / vh;
     const int head = (int)(bh % H);
-    const int bsh = kp_shift(block), sc_cols = (kvl + block - 1) / block;
+    const int bsh = rv_log2(block), sc_cols = (kvl + block - 1) / block;
     const size_t row = (size_t)head * (nope + vh) + nope + j;
     const uint8_t* w = kvb + row * kvl;
     const float* srow = scale + (row >> bsh) * sc_cols;
@@ -118,10 +143,15 @@ RIVOLI_API int rivoli_mla_absorb_fp8(const float* q, const unsigned char* kvb, c
                                      int nope, int vh, int kvl, int block, int nrow, float* qabs) {
     if (int e = guard_dims(H, qh, nope, vh, kvl, block)) return e;
     if (nrow != 1 && nrow != 2) return 1004;
-    const unsigned grid = (unsigned)(((size_t)H * kvl + 255) / 256);
+    const dim3 grid((unsigned)((kvl + AB_COLS - 1) / AB_COLS), (unsigned)H);
+    const bool vec = kvl % 16 == 0 && ((uintptr_t)kvb & 15) == 0;
     rv_drain_error();
-    if (nrow == 2) absorb_f32_kernel<2><<<grid, 256>>>(q, kvb, kvb_scale, H, qh, nope, vh, kvl, block, qabs);
-    else absorb_f32_kernel<1><<<grid, 256>>>(q, kvb, kvb_scale, H, qh, nope, vh, kvl, block, qabs);
+#define RV_AB(RR, VV)                                                                                                     \
+    rv_launch_dependent(absorb_f32_kernel<RR, VV>, grid, dim3(AB_THREADS), 0, (cudaStream_t)0, q, kvb, kvb_scale, H, qh,  \
+                        nope, vh, kvl, block, qabs)
+    if (nrow == 2) { if (vec) RV_AB(2, true); else RV_AB(2, false); }
+    else { if (vec) RV_AB(1, true); else RV_AB(1, false); }
+#undef RV_AB
     return rv_launch_status();
 }
 
@@ -130,11 +160,9 @@ RIVOLI_API int rivoli_mla_value_fp8(const float* clat, const unsigned char* kvb,
     if (int e = guard_dims(H, 1, nope, vh, kvl, block)) return e;
     if (nrow != 1 && nrow != 2) return 1004;
     if (kvl & 3) return 1002;   // the reference's value kernel loads weights as words (mla.hip:216-225)
-    const unsigned grid = (unsigned)(((size_t)H * vh + 255) / 256);
     rv_drain_error();
-    if (nrow == 2) value_f32_kernel<2><<<grid, 256>>>(clat, kvb, kvb_scale, H, nope, vh, kvl, block, ctx);
-    else value_f32_kernel<1><<<grid, 256>>>(clat, kvb, kvb_scale, H, nope, vh, kvl, block, ctx);
-    return rv_launch_status();
+    return launch_fold_gemv(FoldGemv{clat, (size_t)H * kvl, (size_t)kvl, kvb, (size_t)(nope + vh), (size_t)nope, kvb_scale, rv_log2(block),
+                                     (kvl + block - 1) / block, kvl, vh, ctx, (size_t)H * vh, (size_t)vh, 0, 0}, H, nrow, 0);
 }
 
 // Defined in kvb_proj_mma.cu: 0 if the geometry is outside the tensor-core kernels.
