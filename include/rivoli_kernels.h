@@ -65,10 +65,9 @@ int rivoli_index_topk(const float* scores, int nt, int k, unsigned int* rows);
 /* Replaces crates/backend/kernels/attn.hip:279-308 (launch_attend, hip_attn.rs:101-128):
  * clat[h] = sum_t softmax_t((qabs_h.L_t + qrope_h.R_t)*scale) * L_t over the fp8 latent cache
  * (per-128 block scales) and bf16 roped keys; rows NULL = dense over 0..nr, else the nr
- * listed tokens. partial = scratch of rivoli_mla_attend_scratch_floats() floats, or NULL
- * (single split). Guards: 1001 sizes; 1002 16*(kvl+rope)*4 > 65536 or rope > 128; 1004 kvl>512 or kvl%128.
- * Any H is accepted: one CTA takes as many heads as fit its shared memory (all 64 at the model's width) and
- * larger head counts are tiled over the grid (the reference tiles them in blocks of 16). */
+ * listed tokens. partial = scratch of rivoli_mla_attend_scratch_floats() floats, or NULL (this library splits the rows
+ * over a thread-block cluster and merges on the chip either way; the scratch is left alone). Guards: 1001 sizes; 1002 16*(kvl+rope)*4 > 65536 or rope > 128; 1004 kvl>512 or kvl%128.
+ * Any H is accepted: heads are tiled over the grid in pairs (the reference tiles them in blocks of 16). */
 int rivoli_mla_attend(const float* qabs, const float* qrope, const unsigned char* Lc8,
                       const float* Lscale, const unsigned short* Rc, const unsigned int* rows, int H,
                       int nr, int kvl, int rope, int n_blocks, float scale, float* clat,
@@ -76,11 +75,8 @@ int rivoli_mla_attend(const float* qabs, const float* qrope, const unsigned char
 
 /* rivoli_mla_attend without the caller's `partial` scratch. No counterpart in the reference.
  * For callers that cannot allocate device memory (everything already handed to their own
- * arenas, a thread that must not block on the allocator, a host contract that forbids it):
- * the split partials live in a fixed 2,105,344-byte array inside the library, sized for
- * H <= 64 and kvl <= 512; larger shapes are refused with 1002. Calls nothing that allocates.
- * The first call on a device looks the array's address up (do it before any stream
- * capture). All calls on a device share the array: do not let two of them overlap on the GPU. */
+ * arenas, a thread that must not block on the allocator, a host contract that forbids it).
+ * H <= 64 and kvl <= 512; larger shapes are refused with 1002. Calls nothing that allocates. */
 int rivoli_mla_attend_static(const float* qabs, const float* qrope, const unsigned char* Lc8,
                              const float* Lscale, const unsigned short* Rc, const unsigned int* rows, int H,
                              int nr, int kvl, int rope, int n_blocks, float scale, float* clat);

@@ -9,19 +9,71 @@
 //                                   f32 cross-check of the tensor-core kernel and the path
 //                                   used for geometries that kernel does not cover.
 //
-// One CTA attends a GROUP of heads of one (sequence, split) - all of them whenever their q rows fit
-// shared memory, otherwise groups tiled over gridDim.z - so each cached row is read from HBM once per
-// (split, head group) (the reference re-reads it ceil(H/16) times). q sits in shared memory as f32
-// for the whole CTA; rows are dequantised 16 at a time into a shared tile; warp w owns heads
-// w, w + n_warps, ... of the group and its lanes own the columns i = lane (mod 32), so the online
-// accumulator is lane-private registers.
+// What bounds it: instruction issue. There are 2 * H * rows * (2 kvl + rope) f32 operations and only a megabyte or two
+// of rows, so the work is spread over every SM and the loop holds little but the arithmetic:
+//   * a WARP takes AT_HG = 2 heads and a run of rows, two rows per step. Its lanes own the columns (lane l the kvl / 32
+//     consecutive latent columns from l * kvl / 32; kvl 384 differs), q and the output sums of the heads stay in registers, and a cached
+//     row is decoded once and used for both heads, once as key and once as value. AT_RING rows per warp are in flight as
+//     asynchronous copies into the warp's own slots of shared memory (16 bytes per lane and row at kvl 512): loads into
+//     registers a step ahead were waited for on the spot, at the register limit (1,700 of 2,900 cycles per step);
+//   * products are the packed form (fma.rn.f32x2: two f32 multiply-adds per issued instruction, each rounded as usual);
+//   * the four scores of a step (2 rows x 2 heads) are summed over the warp with six shuffles, after which each group
+//     of eight lanes holds one of them: one exponential per lane and step;
+//   * the sums are rescaled when a score leaves its head's reference maximum AT_LAG behind, and only then;
+//   * the rows of a head pair are split over the warps of a CTA and the up to eight CTAs of a thread-block cluster,
+//     which merge their (maximum, sum, output) through shared and distributed shared memory (plain loads of mapped
+//     addresses): no partials in global memory and no second launch. Two CTAs share an SM, so that a cluster needs four
+//     SMs and all clusters of a launch are resident at once.
+// A warp resolves the addresses of 32 rows at a time (token -> page -> pool row -> scale), lane by lane.
+// Measured at 64 heads x 2,048 of 8,193 rows, one sequence: 23 us; one CTA for all heads per 256 rows (eight
+// CTAs), rows dequantised into shared memory and a combine launch took 1,098 us.
+#include <cooperative_groups.h>
+
 #include "codec.cuh"
 #include "common.cuh"
+#include "tc_common.cuh"
 
-constexpr int AT_THREADS = 1024;
-constexpr int AT_WARPS = 32;
-constexpr int AT_TT = 16;          // rows per staged tile
-constexpr int AT_MAX_SPLITS = 16;  // bounds the caller's scratch (attn.hip:67)
+namespace cg = cooperative_groups;
+
+constexpr int AT_HG = 2;             // heads per warp (the reduction below is written for two)
+constexpr int AT_WARPS = 6;          // two CTAs of six warps per SM: 170 registers per thread
+constexpr int AT_THREADS = AT_WARPS * 32;
+constexpr float AT_LAG = 8.0f;
+constexpr int AT_MAX_CLUSTER = 8;
+constexpr int AT_MAX_SPLITS = 16;    // sizes the caller's scratch (attn.hip:67); this kernel needs none
+
+constexpr int AT_RING = 8;           // rows in flight per warp (64 rope columns: the model's shape)
+// Shared memory per warp: a row in flight is its latent codes, its rope columns and (slab) one scale per lane; the same
+// bytes hold the warp's outputs afterwards.
+__host__ __device__ constexpr int at_row_bytes(bool paged, int kvl) { return kvl + (paged ? 64 : 256); }
+__host__ __device__ constexpr int at_warp_bytes(bool paged, int kvl) {
+    return AT_RING * at_row_bytes(paged, kvl) > AT_HG * kvl * 4 ? AT_RING * at_row_bytes(paged, kvl) : AT_HG * kvl * 4;
+}
+__device__ __forceinline__ void at_cp_async4(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// Column of word k (four columns) of lane `lane`, NL columns per lane.
+template <int NL>
+__device__ __forceinline__ int at_col(int lane, int k) { return NL == 12 ? 128 * k + 4 * lane : lane * NL + 4 * k; }
+
+// Two f32 in a register pair, and the packed multiply-add.
+typedef unsigned long long at_f2;
+__device__ __forceinline__ at_f2 at_pack(float lo, float hi) {
+    at_f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 at_unpack(at_f2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ at_f2 at_fma2(at_f2 a, at_f2 b, at_f2 c) {
+    at_f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
 
 struct AttSlab {
     const float* qabs; const float* qrope; const unsigned char* lc8; const float* lscale;
@@ -34,259 +86,386 @@ struct AttPaged {
     int rows_lo, rows_hi;   // the launch serves sequences with rows_lo <= n_rows < rows_hi only (others are left untouched)
 };
 
-template <bool PAGED, int HPW>
-__global__ void __launch_bounds__(AT_THREADS, 1)
-attend_simt_kernel(AttSlab sp, AttPaged pp, int H, int hg, int kvl, int rope, float scale, int nr_single,
-                   int n_splits, float* __restrict__ partial) {
-    extern __shared__ __align__(16) float smem[];
-    const int W = kvl + rope;
-    const int nthreads = blockDim.x, nwarps = nthreads >> 5;
-    const int head0 = blockIdx.z * hg;             // this CTA's head group: [head0, head0 + Hc)
-    const int Hc = min(hg, H - head0);
-    float* qs = smem;                      // [hg][W]
-    float* tile = smem + (size_t)hg * W;   // [AT_TT][W]
-    __shared__ float tscale[AT_TT];
-    __shared__ const uint8_t* trow[AT_TT];
-
+// WIDE: the slab's rows and q allow wide loads. At kvl 384 a run of 12 columns would straddle the slab's scale blocks:
+// there a lane owns four columns of each block instead (at_col) and the slab's values are scaled as they are decoded. NL = kvl / 32 latent columns per lane (4, 8, 12, 16). ROPE64: 64 rope columns, a neighbouring pair per lane; otherwise
+// up to 128, lane + 32 k. Grid (cluster size, head pairs, sequences), clusters along x.
+template <bool PAGED, bool WIDE, int NL, bool ROPE64>
+__global__ void __launch_bounds__(AT_THREADS, 2)
+attend_simt_kernel(AttSlab sp, AttPaged pp, int H, int rope, float scale, int nr_single) {
+    constexpr int KVL = NL * 32, HG = AT_HG, N2 = NL / 2, NR = ROPE64 ? 1 : 4;   // NR: rope words per lane
+    constexpr bool RING = WIDE && ROPE64;
+    constexpr int ROW_BYTES = at_row_bytes(PAGED, KVL), WARP_FLOATS = at_warp_bytes(PAGED, KVL) / 4;
+    extern __shared__ __align__(16) float at_smem[];           // per warp: rows in flight, then its outputs [HG][KVL]
+    __shared__ float s_m[AT_WARPS][HG], s_l[AT_WARPS][HG];      // their maxima and sums
+    __shared__ float s_w[AT_MAX_CLUSTER][HG];                    // weights in the merge, of warps and then of CTAs
+    __shared__ float c_m[HG], c_l[HG];                          // the CTA's, read by its cluster
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int split = blockIdx.x, b = blockIdx.y;
+    unsigned char* at_warp_smem = reinterpret_cast<unsigned char*>(at_smem + (size_t)warp * WARP_FLOATS);
+    const int n_cta = gridDim.x, rank = blockIdx.x, head0 = blockIdx.y * HG, b = blockIdx.z;
+    const int W = KVL + rope;
+    rv_grid_dep_trigger();             // a dependent kernel may set itself up; it waits for this grid before reading
+    rv_grid_dep_wait();                // the counts, rows and q may come from the kernel before
     int nr = nr_single;
     if (PAGED) {  // clamp device-side counts so a bad entry can never index past a table
-        rv_grid_dep_trigger();             // a dependent kernel may set itself up; it waits for this grid before reading
-        rv_grid_dep_wait();                // the counts (and rows) may come from the kernel before
         nr = pp.n_rows[b];
         // a row list whose first entry is the dense marker stands for "row j = token j" over the first n_rows tokens
         if (pp.rows && pp.rows[(size_t)b * pp.row_stride] == 0xffffffffu) pp.rows = nullptr;
         const long long cap = pp.rows ? pp.row_stride : (long long)pp.max_pages * pp.page_tokens;
         nr = (int)max(0LL, min((long long)nr, cap));
-        if (nr < pp.rows_lo || nr >= pp.rows_hi) return;   // another kernel of the same call serves this sequence
-    }
-    const int nacc = kvl / 32;             // lane-owned latent columns (<= 16)
-    const int nrp = (rope + 31) / 32;      // lane-owned rope columns (<= 4)
-
-    // q -> shared f32
-    if (PAGED) {
-        const uint16_t* q = pp.q + ((size_t)b * H + head0) * W;
-        for (int i = tid; i < Hc * W; i += nthreads) qs[i] = rv_bf16_to_f32(q[i]);
-    } else {
-        for (int i = tid; i < Hc * W; i += nthreads) {
-            const int h = i / W, c = i - h * W;
-            qs[i] = c < kvl ? sp.qabs[(size_t)(head0 + h) * kvl + c] : sp.qrope[(size_t)(head0 + h) * rope + (c - kvl)];
-        }
+        if (nr < pp.rows_lo || nr >= pp.rows_hi) return;   // another kernel of the same call serves this sequence (uniform over the cluster)
     }
 
-    // this split's row range, tile aligned
-    const int ntiles = (nr + AT_TT - 1) / AT_TT;
-    const int tps = (ntiles + n_splits - 1) / n_splits;
-    const int r_begin = split * tps * AT_TT;
-    const int r_end = min(nr, r_begin + tps * AT_TT);
-
-    float acc[HPW][16];
-    float m[HPW], l[HPW];
+    // q of the warp's heads (a head past H repeats the last one; it is not stored)
+    at_f2 ql[HG][N2];
+    float qr[HG][ROPE64 ? 2 : 4];
 #pragma unroll
-    for (int j = 0; j < HPW; ++j) {
-        m[j] = -INFINITY; l[j] = 0.0f;
-#pragma unroll
-        for (int k = 0; k < 16; ++k) acc[j][k] = 0.0f;
-    }
-
-    for (int t0 = r_begin; t0 < r_end; t0 += AT_TT) {
-        const int tcount = min(AT_TT, r_end - t0);
-        __syncthreads();  // previous tile consumed (and q staged, first time round)
+    for (int j = 0; j < HG; ++j) {
+        const int h = min(head0 + j, H - 1);
         if (PAGED) {
-            if (tid < tcount) {
-                const uint32_t t = pp.rows ? pp.rows[(size_t)b * pp.row_stride + t0 + tid] : (uint32_t)(t0 + tid);
-                const int lp = (int)(t / (uint32_t)pp.page_tokens);
-                int page = lp < pp.max_pages ? pp.block_table[(size_t)b * pp.max_pages + lp] : -1;
-                if (page < 0 || page >= pp.n_pool_pages) page = 0;  // guarded: never read outside the pool
-                const size_t r = (size_t)page * pp.page_tokens + (t & (uint32_t)(pp.page_tokens - 1));
-                trow[tid] = pp.pool + r * W;
-                tscale[tid] = pp.pscale[r];
-            }
-            __syncthreads();
-            const int cpr = W / 16;  // 16-byte chunks per row
-            for (int c = tid; c < tcount * cpr; c += nthreads) {
-                const int row = c / cpr, ch = c - row * cpr;
-                const uint4 p = *reinterpret_cast<const uint4*>(trow[row] + ch * 16);
-                const float sc = tscale[row];
-                const uint32_t wv[4] = {p.x, p.y, p.z, p.w};
-                float* dst = tile + (size_t)row * W + ch * 16;
+            const uint16_t* q = pp.q + ((size_t)b * H + h) * W;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const float2 a = rv_e4m3x2_to_f32x2((uint16_t)(wv[k] & 0xffff));
-                    const float2 c2 = rv_e4m3x2_to_f32x2((uint16_t)(wv[k] >> 16));
-                    dst[4 * k + 0] = __fmul_rn(a.x, sc); dst[4 * k + 1] = __fmul_rn(a.y, sc);
-                    dst[4 * k + 2] = __fmul_rn(c2.x, sc); dst[4 * k + 3] = __fmul_rn(c2.y, sc);
-                }
+            for (int k = 0; k < N2; k += 2) {
+                const uint16_t* c = q + at_col<NL>(lane, k / 2);
+                const uint2 v = WIDE ? *reinterpret_cast<const uint2*>(c)
+                                           : make_uint2((uint32_t)c[0] | (uint32_t)c[1] << 16, (uint32_t)c[2] | (uint32_t)c[3] << 16);
+                ql[j][k] = at_pack(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u));
+                ql[j][k + 1] = at_pack(__uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+            }
+            if (ROPE64) {
+                qr[j][0] = rv_bf16_to_f32(q[KVL + 2 * lane]); qr[j][1] = rv_bf16_to_f32(q[KVL + 2 * lane + 1]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < NR; ++k) qr[j][k] = lane + 32 * k < rope ? rv_bf16_to_f32(q[KVL + lane + 32 * k]) : 0.0f;
             }
         } else {
-            for (int idx = tid; idx < tcount * W; idx += nthreads) {
-                const int row = idx / W, c = idx - row * W;
-                const size_t t = sp.rows ? (size_t)sp.rows[t0 + row] : (size_t)(t0 + row);
-                tile[idx] = c < kvl
-                    ? __fmul_rn(rv_e4m3_to_f32(sp.lc8[t * kvl + c]), sp.lscale[t * sp.n_blocks + c / 128])
-                    : rv_bf16_to_f32(sp.rc[t * rope + (c - kvl)]);
-            }
-        }
-        __syncthreads();
-
-        for (int tt = 0; tt < tcount; ++tt) {
-            const float* row = tile + (size_t)tt * W;
-            float lv[16], rv[4];
+            const float* q = sp.qabs + (size_t)h * KVL;
+            if (WIDE) {
 #pragma unroll
-            for (int k = 0; k < 16; ++k) lv[k] = k < nacc ? row[lane + 32 * k] : 0.0f;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) rv[k] = (k < nrp && lane + 32 * k < rope) ? row[kvl + lane + 32 * k] : 0.0f;
-#pragma unroll
-            for (int j = 0; j < HPW; ++j) {
-                const int hl = warp + nwarps * j;        // head within the group
-                if (hl >= Hc) continue;                  // warp-uniform
-                const float* qh = qs + (size_t)hl * W;
-                float part = 0.0f;
-#pragma unroll
-                for (int k = 0; k < 16; ++k) if (k < nacc) part = fmaf(qh[lane + 32 * k], lv[k], part);
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (k < nrp && lane + 32 * k < rope) part = fmaf(qh[kvl + lane + 32 * k], rv[k], part);
-                const float s = rv_warp_sum(part) * scale;
-                const float m_new = fmaxf(m[j], s);
-                const float corr = expf(m[j] - m_new);
-                const float p = expf(s - m_new);
-#pragma unroll
-                for (int k = 0; k < 16; ++k) acc[j][k] = fmaf(p, lv[k], acc[j][k] * corr);
-                l[j] = fmaf(l[j], corr, p);
-                m[j] = m_new;
-            }
-        }
-    }
-
-#pragma unroll
-    for (int j = 0; j < HPW; ++j) {
-        if (warp + nwarps * j >= Hc) continue;
-        const int head = head0 + warp + nwarps * j;
-        if (n_splits > 1) {
-            // unnormalised partial + (m, l); an empty split stores (-inf, 0, 0)
-            float* base = partial + (size_t)b * n_splits * H * (kvl + 2);
-            float* pa = base + ((size_t)split * H + head) * kvl;
-            float* pml = base + (size_t)n_splits * H * kvl + ((size_t)split * H + head) * 2;
-#pragma unroll
-            for (int k = 0; k < 16; ++k) if (k < nacc) pa[lane + 32 * k] = acc[j][k];
-            if (lane == 0) { pml[0] = m[j]; pml[1] = l[j]; }
-        } else {
-            const float inv = l[j] > 0.0f ? 1.0f / l[j] : 0.0f;
-            if (PAGED) {
-                uint16_t* o = pp.out + ((size_t)b * H + head) * kvl;
-#pragma unroll
-                for (int k = 0; k < 16; ++k) if (k < nacc) o[lane + 32 * k] = rv_f32_to_bf16(acc[j][k] * inv);
-                if (lane == 0) {
-                    if (pp.out_m) pp.out_m[(size_t)b * H + head] = m[j];
-                    if (pp.out_lse) pp.out_lse[(size_t)b * H + head] = l[j] > 0.0f ? m[j] + logf(l[j]) : -INFINITY;
+                for (int k = 0; k < N2; k += 2) {
+                    const float4 v = *reinterpret_cast<const float4*>(q + at_col<NL>(lane, k / 2));
+                    ql[j][k] = at_pack(v.x, v.y); ql[j][k + 1] = at_pack(v.z, v.w);
                 }
             } else {
 #pragma unroll
-                for (int k = 0; k < 16; ++k) if (k < nacc) sp.clat[(size_t)head * kvl + lane + 32 * k] = acc[j][k] * inv;
+                for (int k = 0; k < N2; ++k) { const float* c = q + at_col<NL>(lane, k / 2) + 2 * (k & 1); ql[j][k] = at_pack(c[0], c[1]); }
+            }
+            const float* r = sp.qrope + (size_t)h * rope;
+            if (ROPE64) { qr[j][0] = r[2 * lane]; qr[j][1] = r[2 * lane + 1]; }
+            else {
+#pragma unroll
+                for (int k = 0; k < NR; ++k) qr[j][k] = lane + 32 * k < rope ? r[lane + 32 * k] : 0.0f;
             }
         }
     }
-}
 
-// Merge the split partials of one (sequence, head): w_s = exp(m_s - m_g), ascending split
-// order (crates/backend/kernels/attn.hip:241-273).
-template <bool PAGED>
-__global__ void __launch_bounds__(128)
-attend_combine_kernel(const float* __restrict__ partial, int H, int kvl, int n_splits, float* __restrict__ clat,
-                      uint16_t* __restrict__ out, float* __restrict__ out_m, float* __restrict__ out_lse,
-                      const int32_t* __restrict__ n_rows, long long cap, int rows_lo, int rows_hi, int serve_empty,
-                      const uint32_t* __restrict__ rows, long long row_stride, long long dense_cap) {
-    __shared__ float w[AT_MAX_SPLITS];
-    __shared__ float inv_l;
-    const int head = blockIdx.x, b = blockIdx.y;
-    if (PAGED && n_rows) {   // same clamp and range rule as the kernels that wrote the partials
-        if (rows && rows[(size_t)b * row_stride] == 0xffffffffu) cap = dense_cap;   // dense marker: see the attention kernels
-        const int nr = (int)max(0LL, min((long long)n_rows[b], cap));
-        if ((nr < rows_lo || nr >= rows_hi) && !(nr == 0 && serve_empty)) return;
+    // this warp's rows: an even share of nr over the cluster's warps
+    const int n_shares = n_cta * AT_WARPS, share = rank * AT_WARPS + warp;
+    const int r_begin = (int)((long long)nr * share / n_shares), r_end = (int)((long long)nr * (share + 1) / n_shares);
+
+    at_f2 acc[HG][N2];
+    const int my_row = lane >> 4, my_head = (lane >> 3) & 1;      // the score this lane's group of eight ends up with
+    float m = -INFINITY, l = 0.0f;                                // reference maximum of my_head, sum of its rows of parity my_row
+#pragma unroll
+    for (int j = 0; j < HG; ++j)
+#pragma unroll
+        for (int k = 0; k < N2; ++k) acc[j][k] = 0ull;
+
+    constexpr int NS = !PAGED && NL == 12 ? 3 : 1;               // scales per lane and row
+    struct Raw { uint32_t c[NL / 4]; uint32_t r[NR]; float s[NS]; };
+    const int my_blk = NS == 3 ? lane % 3 : lane * NL / 128;     // slab: scale block of this lane's columns (three blocks: the one it fetches)
+    unsigned char* ring = at_warp_smem;                          // RING: [AT_RING rows][latent codes | rope | scales (slab)]
+    for (int t0 = r_begin; t0 < r_end; t0 += 32) {
+        const int tn = min(32, r_end - t0);
+        // lane i locates row t0 + i
+        uint32_t where = 0u;
+        float tok_s = 0.0f;
+        if (lane < tn) {
+            const uint32_t* list = PAGED ? pp.rows ? pp.rows + (size_t)b * pp.row_stride : nullptr : sp.rows;
+            const uint32_t t = list ? list[t0 + lane] : (uint32_t)(t0 + lane);
+            if (PAGED) {
+                const int lp = (int)(t / (uint32_t)pp.page_tokens);
+                int page = lp < pp.max_pages ? pp.block_table[(size_t)b * pp.max_pages + lp] : -1;
+                if (page < 0 || page >= pp.n_pool_pages) page = 0;  // guarded: never read outside the pool
+                where = (uint32_t)page * (uint32_t)pp.page_tokens + (t & (uint32_t)(pp.page_tokens - 1));
+                tok_s = pp.pscale[where];
+            } else {
+                where = t;
+            }
+        }
+        auto fetch = [&](int i, Raw& v) {                         // row t0 + i, waited for where it is used
+            const size_t r = __shfl_sync(0xffffffffu, where, i);
+            const unsigned char* row = PAGED ? pp.pool + r * W : sp.lc8 + r * KVL;
+#pragma unroll
+            for (int k = 0; k < NL / 4; ++k) {
+                const unsigned char* c = row + at_col<NL>(lane, k);
+                v.c[k] = PAGED || WIDE ? *reinterpret_cast<const uint32_t*>(c)
+                                       : (uint32_t)c[0] | (uint32_t)c[1] << 8 | (uint32_t)c[2] << 16 | (uint32_t)c[3] << 24;
+            }
+#pragma unroll
+            for (int k = 0; k < NR; ++k)
+                v.r[k] = lane + 32 * k >= rope ? 0u : PAGED ? pp.pool[r * W + KVL + lane + 32 * k] : sp.rc[r * rope + lane + 32 * k];
+#pragma unroll
+            for (int k = 0; k < NS; ++k) v.s[k] = PAGED ? __shfl_sync(0xffffffffu, tok_s, i) : sp.lscale[r * sp.n_blocks + (NS == 3 ? k : my_blk)];
+        };
+        // RING: a row's pieces go to this warp's slots in shared memory (every lane copies what it will read itself, but
+        // for the paged rope codes, two lanes' in one word, and the scales of three blocks)
+        auto request = [&](int i) {
+            const uint32_t r = __shfl_sync(0xffffffffu, where, i);
+            const uint32_t dst = tc::smem_u32(ring + (i % AT_RING) * ROW_BYTES);
+            const unsigned char* row = PAGED ? pp.pool + (size_t)r * W : sp.lc8 + (size_t)r * KVL;
+            if constexpr (NL == 16) tc::cp_async16(dst + lane * 16, row + lane * 16);
+            else {
+#pragma unroll
+                for (int k = 0; k < NL / 4; ++k) at_cp_async4(dst + at_col<NL>(lane, k), row + at_col<NL>(lane, k));
+            }
+            if (PAGED) {
+                if (lane < 16) at_cp_async4(dst + KVL + lane * 4, row + KVL + lane * 4);
+            } else {
+                at_cp_async4(dst + KVL + lane * 4, sp.rc + (size_t)r * 64 + 2 * lane);
+                at_cp_async4(dst + KVL + 128 + lane * 4, sp.lscale + (size_t)r * sp.n_blocks + my_blk);
+            }
+        };
+        auto take = [&](int i, Raw& v) {
+            const unsigned char* row = ring + (i % AT_RING) * ROW_BYTES;
+            if constexpr (NL == 16) {
+                const uint4 p = *reinterpret_cast<const uint4*>(row + lane * 16);
+                v.c[0] = p.x; v.c[1] = p.y; v.c[2] = p.z; v.c[3] = p.w;
+            } else {
+#pragma unroll
+                for (int k = 0; k < NL / 4; ++k) v.c[k] = *reinterpret_cast<const uint32_t*>(row + at_col<NL>(lane, k));
+            }
+            v.r[0] = PAGED ? *reinterpret_cast<const uint16_t*>(row + KVL + lane * 2) : *reinterpret_cast<const uint32_t*>(row + KVL + lane * 4);
+#pragma unroll
+            for (int k = 0; k < NS; ++k) v.s[k] = PAGED ? __shfl_sync(0xffffffffu, tok_s, i) : *reinterpret_cast<const float*>(row + KVL + 128 + (NS == 3 ? k : lane) * 4);
+        };
+        if (RING) {
+#pragma unroll
+            for (int g = 0; g < AT_RING; g += 2) {
+                if (g < tn) { request(g); request(min(g + 1, tn - 1)); }
+                tc::cp_async_commit();
+            }
+        }
+        for (int i = 0; i < tn; i += 2) {
+            const bool live = i + my_row < tn;                   // the second row of the last step may not exist
+            Raw now[2];
+            if (RING) {
+                tc::cp_async_wait<AT_RING / 2 - 1>();
+                if (PAGED || NS == 3) __syncwarp();
+                take(i, now[0]);
+                if (i + 1 < tn) take(i + 1, now[1]); else now[1] = now[0];
+                if (PAGED || NS == 3) __syncwarp();
+            } else {
+                fetch(i, now[0]);
+                fetch(min(i + 1, tn - 1), now[1]);
+            }
+            at_f2 lv[2][N2];                                     // the codes' values; the lane's columns share one scale
+            float rv[2][ROPE64 ? 2 : 4], rs[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+#pragma unroll
+                for (int k = 0; k < NL / 4; ++k) {
+                    float2 x = rv_e4m3x2_to_f32x2((uint16_t)now[u].c[k]), y = rv_e4m3x2_to_f32x2((uint16_t)(now[u].c[k] >> 16));
+                    if (NS == 3) { const float sk = now[u].s[k % NS]; x.x *= sk; x.y *= sk; y.x *= sk; y.y *= sk; }
+                    lv[u][2 * k] = at_pack(x.x, x.y);
+                    lv[u][2 * k + 1] = at_pack(y.x, y.y);
+                }
+                if (ROPE64) {
+                    if (PAGED) { const float2 x = rv_e4m3x2_to_f32x2((uint16_t)now[u].r[0]); rv[u][0] = x.x; rv[u][1] = x.y; }
+                    else { rv[u][0] = __uint_as_float(now[u].r[0] << 16); rv[u][1] = __uint_as_float(now[u].r[0] & 0xffff0000u); }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < NR; ++k) rv[u][k] = PAGED ? rv_e4m3_to_f32((uint8_t)now[u].r[k]) : rv_bf16_to_f32((uint16_t)now[u].r[k]);
+                }
+                rs[u] = NS == 3 ? 1.0f : now[u].s[0];
+            }
+            if (RING) {                                          // the slots just read take the rows AT_RING further on
+                if (i + AT_RING < tn) { request(i + AT_RING); request(min(i + AT_RING + 1, tn - 1)); }
+                tc::cp_async_commit();
+            }
+            float part[2][HG];
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+#pragma unroll
+                for (int j = 0; j < HG; ++j) {
+                    at_f2 p2 = 0ull;
+                    float pr = 0.0f;
+#pragma unroll
+                    for (int k = 0; k < N2; ++k) p2 = at_fma2(ql[j][k], lv[u][k], p2);
+#pragma unroll
+                    for (int k = 0; k < (ROPE64 ? 2 : 4); ++k) pr = fmaf(qr[j][k], rv[u][k], pr);
+                    const float2 p = at_unpack(p2);
+                    // the rope columns have the token's scale in the paged cache, none in the slab
+                    part[u][j] = PAGED ? (p.x + p.y + pr) * rs[u] : fmaf(p.x + p.y, rs[u], pr);
+                }
+            // four sums over the warp
+            float a0 = my_row ? part[1][0] : part[0][0], a1 = my_row ? part[1][1] : part[0][1];
+            a0 += __shfl_xor_sync(0xffffffffu, my_row ? part[0][0] : part[1][0], 16);
+            a1 += __shfl_xor_sync(0xffffffffu, my_row ? part[0][1] : part[1][1], 16);
+            float s = my_head ? a1 : a0;
+            s += __shfl_xor_sync(0xffffffffu, my_head ? a0 : a1, 8);
+            s += __shfl_xor_sync(0xffffffffu, s, 4);
+            s += __shfl_xor_sync(0xffffffffu, s, 2);
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            s = live ? s * scale : -INFINITY;
+            // the reference m follows the maximum at a distance: a weight may reach e^AT_LAG, which f32 holds as well as
+            // 1, and the sums are rescaled at a warp's first rows and then hardly ever
+            if (__any_sync(0xffffffffu, s > m + AT_LAG)) {
+                const float m_new = fmaxf(m, fmaxf(s, __shfl_xor_sync(0xffffffffu, s, 16)));
+                const float corr = m_new == m ? 1.0f : expf(m - m_new);
+                m = m_new;
+                l *= corr;
+#pragma unroll
+                for (int j = 0; j < HG; ++j) {
+                    const float cj = __shfl_sync(0xffffffffu, corr, 8 * j);
+#pragma unroll
+                    for (int k = 0; k < N2; ++k) { const float2 o = at_unpack(acc[j][k]); acc[j][k] = at_pack(o.x * cj, o.y * cj); }
+                }
+            }
+            const float p = expf(s - m);
+            l += p;
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+#pragma unroll
+                for (int j = 0; j < HG; ++j) {
+                    const float w = __shfl_sync(0xffffffffu, p, 16 * u + 8 * j) * rs[u];
+                    const at_f2 w2 = at_pack(w, w);
+#pragma unroll
+                    for (int k = 0; k < N2; ++k) acc[j][k] = at_fma2(w2, lv[u][k], acc[j][k]);
+                }
+        }
     }
-    const float* base = partial + (size_t)b * n_splits * H * (kvl + 2);
-    const float* ml = base + (size_t)n_splits * H * kvl;
-    if (threadIdx.x == 0) {
-        float m_g = -INFINITY;
-        for (int s = 0; s < n_splits; ++s) m_g = fmaxf(m_g, ml[((size_t)s * H + head) * 2]);
-        float l_g = 0.0f;
-        for (int s = 0; s < n_splits; ++s) {
-            const float* p = ml + ((size_t)s * H + head) * 2;
-            w[s] = isfinite(m_g) ? expf(p[0] - m_g) : 0.0f;
-            l_g += p[1] * w[s];
-        }
-        inv_l = l_g > 0.0f ? 1.0f / l_g : 0.0f;
-        if (PAGED) {
-            if (out_m) out_m[(size_t)b * H + head] = m_g;
-            if (out_lse) out_lse[(size_t)b * H + head] = l_g > 0.0f ? m_g + logf(l_g) : -INFINITY;
-        }
+    l += __shfl_xor_sync(0xffffffffu, l, 16);                    // both row parities
+    if (RING) tc::cp_async_wait<0>();                            // (nothing is in flight; the slots become the output buffer)
+
+    // ---- the CTA's warps meet in shared memory (a warp without rows has m = -inf, l = 0) ----
+    if ((lane & 23) == 0) { s_m[warp][my_head] = m; s_l[warp][my_head] = l; }
+    if (r_begin < r_end) {
+#pragma unroll
+        for (int j = 0; j < HG; ++j)
+#pragma unroll
+            for (int k = 0; k < N2; k += 2) {
+                const float2 x = at_unpack(acc[j][k]), y = at_unpack(acc[j][k + 1]);
+                *reinterpret_cast<float4*>(at_smem + (size_t)warp * WARP_FLOATS + j * KVL + at_col<NL>(lane, k / 2)) = make_float4(x.x, x.y, y.x, y.y);
+            }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < kvl; i += blockDim.x) {
-        float sum = 0.0f;
-        for (int s = 0; s < n_splits; ++s) sum += base[((size_t)s * H + head) * kvl + i] * w[s];
-        if (PAGED) out[((size_t)b * H + head) * kvl + i] = rv_f32_to_bf16(sum * inv_l);
-        else clat[(size_t)head * kvl + i] = sum * inv_l;
+    auto store = [&](int h, int c, float v) {
+        if (PAGED) pp.out[((size_t)b * H + h) * KVL + c] = rv_f32_to_bf16(v);
+        else sp.clat[(size_t)h * KVL + c] = v;
+    };
+    auto stats = [&](int h, float mg, float lg) {
+        if (PAGED) {
+            if (pp.out_m) pp.out_m[(size_t)b * H + h] = mg;
+            if (pp.out_lse) pp.out_lse[(size_t)b * H + h] = lg > 0.0f ? mg + logf(lg) : -INFINITY;
+        }
+    };
+    // the CTA's maximum and sum per head, and the weight of each warp's outputs at that maximum
+    if (tid < AT_WARPS * HG) {
+        const int j = tid % HG, w = tid / HG;
+        float mx = -INFINITY, sum = 0.0f;
+#pragma unroll
+        for (int v = 0; v < AT_WARPS; ++v) mx = fmaxf(mx, s_m[v][j]);
+#pragma unroll
+        for (int v = 0; v < AT_WARPS; ++v)
+            if (s_l[v][j] > 0.0f) sum += s_l[v][j] * expf(s_m[v][j] - mx);
+        s_w[w][j] = s_l[w][j] > 0.0f ? expf(s_m[w][j] - mx) : 0.0f;
+        if (w == 0) { c_m[j] = mx; c_l[j] = sum; }
     }
+    __syncthreads();
+    auto cta_sum = [&](int j, int c) {                            // column c of head j over the CTA's warps
+        float v = 0.0f;
+#pragma unroll
+        for (int w = 0; w < AT_WARPS; ++w)
+            if (s_w[w][j] > 0.0f) v = fmaf(at_smem[(size_t)w * WARP_FLOATS + j * KVL + c], s_w[w][j], v);
+        return v;
+    };
+    if (n_cta == 1) {
+        for (int e = tid; e < HG * KVL; e += AT_THREADS) {
+            const int j = e / KVL, c = e - j * KVL;
+            if (head0 + j < H) store(head0 + j, c, c_l[j] > 0.0f ? cta_sum(j, c) * (1.0f / c_l[j]) : 0.0f);
+        }
+        if (tid < HG && head0 + tid < H) stats(head0 + tid, c_m[tid], c_l[tid]);
+        return;
+    }
+    // ---- and the cluster's CTAs through distributed shared memory ----
+    cg::cluster_group cluster = cg::this_cluster();
+    constexpr int PER = (HG * KVL + AT_THREADS - 1) / AT_THREADS;
+    float mine[PER];
+#pragma unroll
+    for (int e = 0; e < PER; ++e) { const int c = tid + e * AT_THREADS; mine[e] = c < HG * KVL ? cta_sum(c / KVL, c % KVL) : 0.0f; }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < PER; ++e) if (tid + e * AT_THREADS < HG * KVL) at_smem[tid + e * AT_THREADS] = mine[e];
+    cluster.sync();                                               // every CTA's (m, l, output)
+    if (tid < 32) {                                               // weight of each CTA's outputs, normalised: lane = (CTA, head)
+        const int j = lane % HG, q = lane / HG;
+        static_assert(HG * AT_MAX_CLUSTER <= 32, "one lane per (CTA, head)");
+        const float mq = q < n_cta ? cluster.map_shared_rank(c_m, q)[j] : -INFINITY, lq = q < n_cta ? cluster.map_shared_rank(c_l, q)[j] : 0.0f;
+        float mg = mq;
+#pragma unroll
+        for (int o = HG; o < HG * AT_MAX_CLUSTER; o <<= 1) mg = fmaxf(mg, __shfl_xor_sync(0xffffffffu, mg, o));
+        const float wq = lq > 0.0f ? expf(mq - mg) : 0.0f;
+        float lg = lq * wq;
+#pragma unroll
+        for (int o = HG; o < HG * AT_MAX_CLUSTER; o <<= 1) lg += __shfl_xor_sync(0xffffffffu, lg, o);
+        if (q < AT_MAX_CLUSTER) s_w[q][j] = wq > 0.0f ? wq / lg : 0.0f;
+        if (q == 0 && rank == 0 && head0 + j < H) stats(head0 + j, mg, lg);
+    }
+    __syncthreads();
+    const int c_lo = HG * KVL * rank / n_cta, c_hi = HG * KVL * (rank + 1) / n_cta;   // this CTA merges and stores these columns
+    for (int e = c_lo + tid; e < c_hi; e += AT_THREADS) {
+        const int j = e / KVL;
+        float v = 0.0f, o[AT_MAX_CLUSTER];
+#pragma unroll
+        for (int q = 0; q < AT_MAX_CLUSTER; ++q) o[q] = q < n_cta ? cluster.map_shared_rank(at_smem, q)[e] : 0.0f;   // all in flight
+#pragma unroll
+        for (int q = 0; q < AT_MAX_CLUSTER; ++q)
+            if (q < n_cta && s_w[q][j] > 0.0f) v = fmaf(o[q], s_w[q][j], v);   // (a CTA without rows left its array unwritten)
+        if (head0 + j < H) store(head0 + j, e - j * KVL, v);
+    }
+    cluster.sync();                                               // nobody reads this CTA's memory any more
 }
 
-// Launch plan: a CTA takes `hg` heads - all H when their q rows fit shared memory beside the row tile,
-// otherwise (or when `hg_req` asks for smaller groups) H is tiled over gridDim.z - with one warp per head up
-// to 32 warps, then 2 or 4 heads per warp. `dependent` launches the kernel as a programmatic dependent of the
-// kernel before it in the stream (paged form only: it waits for that kernel before reading the counts).
+// CTAs per (sequence, head group): enough that the grid covers the SMs about twice over, at most one cluster of eight,
+// and no more than leave every warp about two rows (rows_most: what the host knows of the longest sequence).
+static int simt_cluster(int B, int groups, long long rows_most) {
+    int n = 1;
+    while (n < AT_MAX_CLUSTER && (long long)B * groups * n * 2 <= 2 * 148 && (long long)n * AT_WARPS * 2 < rows_most) n *= 2;
+    return n;
+}
+
 template <bool PAGED>
-static int launch_attend_simt(const AttSlab& sp, const AttPaged& pp, int H, int kvl, int rope, float scale,
-                              int nr_single, int B, int n_splits, float* partial, cudaStream_t st, int hg_req = 0,
-                              bool dependent = false) {
-    const int W = kvl + rope;
-    auto smem_of = [&](int h) { return ((size_t)h * W + (size_t)AT_TT * W) * sizeof(float); };
-    const size_t smem_max = 227 * 1024 - 512;
-    int hg = (hg_req > 0 && hg_req < H) ? hg_req : H;
-    while (hg > 1 && (hg > 4 * AT_WARPS || smem_of(hg) > smem_max)) hg = (hg + 1) / 2;
-    if (smem_of(hg) > smem_max) return 1006;
-    const size_t smem = smem_of(hg);
-    const int groups = (H + hg - 1) / hg;
-    const int warps = hg < AT_WARPS ? hg : AT_WARPS;
-    const int hpw = (hg + warps - 1) / warps;
-    dim3 grid(n_splits, B, groups);
+static int launch_attend_simt(const AttSlab& sp, const AttPaged& pp, bool wide, int H, int kvl, int rope, float scale,
+                              int nr_single, int B, long long rows_most, cudaStream_t st) {
+    const int groups = (H + AT_HG - 1) / AT_HG, n = simt_cluster(B, groups, rows_most);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)n, (unsigned)groups, (unsigned)B); cfg.blockDim = dim3(AT_THREADS);
+    cfg.dynamicSmemBytes = (size_t)AT_WARPS * at_warp_bytes(PAGED, kvl); cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = (unsigned)n; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = n > 1 ? 2 : 1;
     rv_drain_error();
-#define RV_ATT(HPW)                                                                                       \
+#define RV_ATT(WIDE, NL, R64)                                                                             \
     do {                                                                                                  \
-        cudaFuncSetAttribute(attend_simt_kernel<PAGED, HPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                             (int)smem);                                                                  \
-        if (dependent)                                                                                    \
-            rv_launch_dependent(attend_simt_kernel<PAGED, HPW>, grid, dim3(warps * 32), smem, st, sp, pp, H, hg, kvl,  \
-                                rope, scale, nr_single, n_splits, partial);                               \
-        else                                                                                              \
-            attend_simt_kernel<PAGED, HPW><<<grid, warps * 32, smem, st>>>(sp, pp, H, hg, kvl, rope, scale, \
-                                                                          nr_single, n_splits, partial);  \
+        rv_allow_smem<attend_simt_kernel<PAGED, WIDE, NL, R64>>(AT_WARPS * at_warp_bytes(PAGED, NL * 32)); \
+        (void)cudaLaunchKernelEx(&cfg, attend_simt_kernel<PAGED, WIDE, NL, R64>, sp, pp, H, rope, scale, nr_single); \
     } while (0)
-    if (hpw <= 1) RV_ATT(1);
-    else if (hpw <= 2) RV_ATT(2);
-    else RV_ATT(4);
+#define RV_ATT2(NL)                                                                                       \
+    do {                                                                                                  \
+        if (!wide) RV_ATT(false, NL, false);                                                              \
+        else if (rope == 64) RV_ATT(true, NL, true);                                                      \
+        else RV_ATT(true, NL, false);                                                                     \
+    } while (0)
+    if (kvl == 512) RV_ATT2(16);
+    else if (kvl == 384) RV_ATT2(12);
+    else if (kvl == 256) RV_ATT2(8);
+    else RV_ATT2(4);
+#undef RV_ATT2
 #undef RV_ATT
-    int e = rv_launch_status();
-    if (e || n_splits <= 1) return e;
-    const long long cap = PAGED ? (pp.rows ? pp.row_stride : (long long)pp.max_pages * pp.page_tokens) : 0;
-    attend_combine_kernel<PAGED><<<dim3(H, B), 128, 0, st>>>(partial, H, kvl, n_splits, sp.clat, pp.out,
-                                                              pp.out_m, pp.out_lse, PAGED ? pp.n_rows : nullptr, cap,
-                                                              pp.rows_lo, pp.rows_hi, 0, pp.rows, pp.row_stride,
-                                                              (long long)pp.max_pages * pp.page_tokens);
     return rv_launch_status();
-}
-
-// Combine launcher shared with the tensor-core kernel (same partial layout). Sequences whose row count
-// lies outside [rows_lo, rows_hi) are left untouched (another kernel of the same call wrote them), except
-// that an empty sequence is served when serve_empty is set.
-extern "C" void rivoli_attend_combine_paged(const float* partial, int H, int kvl, int n_splits, int B, uint16_t* out,
-                                            float* out_m, float* out_lse, const int32_t* n_rows, long long cap,
-                                            int rows_lo, int rows_hi, int serve_empty, const uint32_t* rows,
-                                            long long row_stride, long long dense_cap, cudaStream_t st) {
-    attend_combine_kernel<true><<<dim3(H, B), 128, 0, st>>>(partial, H, kvl, n_splits, nullptr, out, out_m, out_lse,
-                                                            n_rows, cap, rows_lo, rows_hi, serve_empty, rows, row_stride,
-                                                            dense_cap);
 }
 
 RIVOLI_API size_t rivoli_mla_attend_scratch_floats(int H, int kvl) {
@@ -304,75 +483,31 @@ RIVOLI_API int rivoli_mla_attend(const float* qabs, const float* qrope, const un
     if (((size_t)16 * kvl + (size_t)16 * rope) * sizeof(float) > 65536) return 1002;
     if (kvl > 512 || (kvl % 128) != 0) return 1004;
     if (rope > 128) return 1002;
-    // Any H: heads beyond what one CTA's shared memory holds are tiled over gridDim.z (the reference tiles
-    // them in blocks of 16, attn.hip:119-130). Split plan: a pure function of (H, nr, scratch present) ->
-    // same shape, same summation order.
-    int n_splits = 1;
-    if (partial) {
-        n_splits = (nr + 255) / 256;
-        if (n_splits > AT_MAX_SPLITS) n_splits = AT_MAX_SPLITS;
-        if (n_splits < 1) n_splits = 1;
-    }
+    // `partial` is the reference's scratch for a split: this library merges the splits on the chip and leaves it alone,
+    // so the result does not depend on whether it was lent.
+    (void)partial;
     AttSlab sp{qabs, qrope, Lc8, Lscale, Rc, rows, n_blocks, clat};
-    AttPaged pp{};
-    return launch_attend_simt<false>(sp, pp, H, kvl, rope, scale, nr, 1, n_splits, partial, 0);
+    const bool wide = ((((uintptr_t)Lc8 | (uintptr_t)qabs) & 15) | ((uintptr_t)Rc & 3)) == 0;
+    return launch_attend_simt<false>(sp, AttPaged{}, wide, H, kvl, rope, scale, nr, 1, nr, 0);
 }
 
-// ------------------------------------------------------------------------------------------
-// rivoli_mla_attend_static: rivoli_mla_attend for callers that have no device memory to lend.
-//
-// Some users of this library are not in a position to call cudaMalloc at all: an engine that
-// carved up the whole device into its own arenas at start-up and treats any later driver
-// allocation as a bug, a decode thread that must never block on the allocator (cudaMalloc
-// and cudaFree serialise against the whole device), or a plugin host whose contract says
-// the plugin owns no device memory. For them the split-KV partials that rivoli_mla_attend
-// takes as the caller's `partial` scratch live here instead, in a fixed array inside the
-// library image. It is sized for the model geometry only (H <= 64 heads, kvl <= 512):
-// 16 splits x 64 x 514 floats = 2,105,344 bytes, which every GPU that loads this library
-// carries until the process exits.
-//
-// The array's name is only a host-side handle for the symbol, never a device address, so the
-// address is looked up once per device (with that device current) by cudaGetSymbolAddress
-// and that pointer is what the kernels receive. The FIRST call on a device performs that
-// look-up; make it before any stream capture begins on that device.
-//
-// All calls share the one array and it keeps whatever the last call left there. Nothing
-// in it has to start at zero (every split, an empty one included, stores its partial before
-// the combine reads it), but two calls that are in flight on the GPU at the same time (two
-// streams, or two host threads on one device) would overwrite each other's partials: keep
-// calls on one device ordered. Runs on the legacy default stream like rivoli_mla_attend.
-// ------------------------------------------------------------------------------------------
-constexpr int NA_MAX_H = 64, NA_MAX_KVL = 512, NA_MAX_DEVICES = 64;
-static __device__ __align__(256) float g_attend_static_partial[AT_MAX_SPLITS * NA_MAX_H * (NA_MAX_KVL + 2)];
-static float* g_attend_static_ptr[NA_MAX_DEVICES];   // per-device address of the array above (host side)
+// rivoli_mla_attend for callers that have no device memory to lend (everything carved into their own arenas, a decode
+// thread that must not wait for the allocator, a plugin contract that forbids it). The kernel needs no scratch, so this
+// is the same launch, limited to H <= 64 and kvl <= 512 as documented.
+constexpr int NA_MAX_H = 64, NA_MAX_KVL = 512;
 
 RIVOLI_API int rivoli_mla_attend_static(const float* qabs, const float* qrope, const unsigned char* Lc8,
                                         const float* Lscale, const unsigned short* Rc, const unsigned int* rows,
                                         int H, int nr, int kvl, int rope, int n_blocks, float scale, float* clat) {
-    if (H <= 0 || nr <= 0 || kvl <= 0 || rope <= 0 || n_blocks <= 0) return 1001;
-    if (((size_t)16 * kvl + (size_t)16 * rope) * sizeof(float) > 65536) return 1002;
-    if (kvl > 512 || (kvl % 128) != 0) return 1004;
-    if (rope > 128) return 1002;
-    if (H > NA_MAX_H || kvl > NA_MAX_KVL) return 1002;   // beyond the built-in scratch: use rivoli_mla_attend
-    int dev = -1;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return -(int)e;
-    if (dev < 0 || dev >= NA_MAX_DEVICES) return 1008;
-    if (!g_attend_static_ptr[dev]) {
-        float* p = nullptr;
-        e = cudaGetSymbolAddress((void**)&p, g_attend_static_partial);
-        if (e != cudaSuccess) return -(int)e;
-        g_attend_static_ptr[dev] = p;
+    if (H > NA_MAX_H || kvl > NA_MAX_KVL) {
+        if (nr <= 0 || rope <= 0 || n_blocks <= 0) return 1001;
+        if (((size_t)16 * kvl + (size_t)16 * rope) * sizeof(float) > 65536) return 1002;
+        return (kvl > 512 || (kvl % 128) != 0) ? 1004 : 1002;
     }
-    int n_splits = (nr + 255) / 256;                    // same plan as rivoli_mla_attend with scratch
-    if (n_splits > AT_MAX_SPLITS) n_splits = AT_MAX_SPLITS;
-    if (n_splits < 1) n_splits = 1;
-    AttSlab sp{qabs, qrope, Lc8, Lscale, Rc, rows, n_blocks, clat};
-    AttPaged pp{};
-    return launch_attend_simt<false>(sp, pp, H, kvl, rope, scale, nr, 1, n_splits, g_attend_static_ptr[dev], 0);
+    return rivoli_mla_attend(qabs, qrope, Lc8, Lscale, Rc, rows, H, nr, kvl, rope, n_blocks, scale, clat, nullptr);
 }
 
-// Split count of the SIMT paged path: a pure function of the batch size.
+// Sizes the scratch that callers of the paged form lend: a pure function of the batch size.
 static int simt_paged_splits(int B) {
     int n = (2 * 148 + B - 1) / B;
     if (n > AT_MAX_SPLITS) n = AT_MAX_SPLITS;
@@ -395,25 +530,23 @@ RIVOLI_API int rivoli_attend_simt_paged_bf16(const DsaGeom* g, const uint16_t* q
     if (B <= 0 || !q || !latent_pool || !latent_scale || !block_table || !n_rows || !out) return 1001;
     if (rows && row_stride <= 0) return 1001;
     if (((uintptr_t)latent_pool & 15) || ((g->kv_lora + g->rope_dim) % 16) != 0) return 1005;
-    int n_splits = scratch ? simt_paged_splits(B) : 1;
-    AttSlab sp{};
+    (void)scratch;   // the splits merge on the chip
     AttPaged pp{q, latent_pool, latent_scale, block_table, rows, row_stride, n_rows, g->page_tokens,
                 g->max_pages_per_seq, g->n_pool_pages, out, out_m, out_lse, 0, 0x7fffffff};
-    return launch_attend_simt<true>(sp, pp, g->n_heads, g->kv_lora, g->rope_dim, g->softmax_scale, 0, B,
-                                    n_splits, (float*)scratch, (cudaStream_t)stream);
+    const long long most = rows ? row_stride : (long long)g->max_pages_per_seq * g->page_tokens;
+    return launch_attend_simt<true>(AttSlab{}, pp, ((uintptr_t)q & 7) == 0, g->n_heads, g->kv_lora, g->rope_dim, g->softmax_scale, 0, B, most,
+                                    (cudaStream_t)stream);
 }
 
-// The sequences of a batch with 0 < n_rows < rows_hi, on the CUDA-core kernel, eight heads per CTA and no
-// split (no scratch): the short-context arm of rivoli_mla_attend_paged_bf16, launched in front of the
-// tensor-core kernel as a programmatic dependent of whatever precedes it in the stream.
+// The sequences of a batch with 0 < n_rows < rows_hi on the CUDA-core kernel: the short-context arm of
+// rivoli_mla_attend_paged_bf16, launched in front of the tensor-core kernel as a programmatic dependent of whatever
+// precedes it in the stream.
 extern "C" int rivoli_attend_simt_short_rows(const DsaGeom* g, const uint16_t* q, const uint8_t* latent_pool,
                                              const float* latent_scale, const int32_t* block_table,
                                              const uint32_t* rows, int row_stride, const int32_t* n_rows, int B,
                                              uint16_t* out, float* out_m, float* out_lse, int rows_hi,
                                              cudaStream_t st) {
-    AttSlab sp{};
     AttPaged pp{q, latent_pool, latent_scale, block_table, rows, row_stride, n_rows, g->page_tokens,
                 g->max_pages_per_seq, g->n_pool_pages, out, out_m, out_lse, 1, rows_hi};
-    return launch_attend_simt<true>(sp, pp, g->n_heads, g->kv_lora, g->rope_dim, g->softmax_scale, 0, B, 1, nullptr,
-                                    st, 8, true);
+    return launch_attend_simt<true>(AttSlab{}, pp, ((uintptr_t)q & 7) == 0, g->n_heads, g->kv_lora, g->rope_dim, g->softmax_scale, 0, B, rows_hi, st);
 }
