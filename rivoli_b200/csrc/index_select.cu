@@ -27,6 +27,9 @@
 // A batch that fills the chip by itself runs this kernel as ONE CTA of 1024 threads per sequence (a cluster of one):
 // for that shape the exchanges, the cluster barriers and the list copies are compiled out (SOLO below).
 //
+// VALUES: the same selection over given scores (rivoli_index_topk and its batched form): no error band (eps = 0), no key
+// scales and no re-score - the band is the k-th value's bin itself and its tokens are ranked by the scores as they are.
+//
 // If the band does not fit the list (tie-dominated scores: thousands of tokens at the cut) the cluster takes
 // the slow path instead: every band token is re-scored chunk by chunk, the exact keys replace the approximate
 // ones in the registers, and an exact 4 x 8-bit radix selection runs over the whole cluster.
@@ -122,7 +125,7 @@ __device__ __forceinline__ uint32_t sel_block_excl(uint32_t v, SelXc& xc) {
     return pre + incl - v;
 }
 
-template <int EPT, int NT>
+template <int EPT, int NT, bool VALUES>
 __global__ void __launch_bounds__(NT, (NT == 512 && EPT <= 16) ? 2 : 1)
 index_select_cluster_kernel(SelArgs A) {
     constexpr int NW = NT / 32;
@@ -136,7 +139,7 @@ index_select_cluster_kernel(SelArgs A) {
     __shared__ SelXc xc;
     uint32_t* qf = sel_smem;                                              // [SEL_HD / 4][32] packed q codes, [word][head]
     float* kfw = reinterpret_cast<float*>(qf + (SEL_HD / 4) * 32);        // [NW][SEL_TOK][SEL_HD] key rows as f32
-    uint32_t* hist = reinterpret_cast<uint32_t*>(kfw + NW * SEL_TOK * SEL_HD);   // [SEL_BINS]; later `dec`
+    uint32_t* hist = VALUES ? sel_smem : reinterpret_cast<uint32_t*>(kfw + NW * SEL_TOK * SEL_HD);   // [SEL_BINS]; later `dec`
     uint32_t* l_tok = hist + SEL_BINS;                                    // [SEL_LIST] this CTA's band tokens
     uint32_t* l_key = l_tok + SEL_LIST;                                   // [SEL_LIST] their exact keys
     uint32_t* a_tok = l_key + SEL_LIST;                                   // [SEL_LIST] the cluster's band, gathered
@@ -150,10 +153,10 @@ index_select_cluster_kernel(SelArgs A) {
     const int b = (int)blockIdx.x / C, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     rv_grid_dep_trigger();   // the next kernel may set itself up; it waits for this grid before reading rows
     rv_grid_dep_wait();      // scores, query codes and the error constant come from the kernels before
-    const int nt = min(A.seq_len[b], A.score_stride);
+    const int nt = min(VALUES && !A.seq_len ? A.nt_single : A.seq_len[b], A.score_stride);
     const int kk = min(A.k, nt);
     uint32_t* out = A.rows + (size_t)b * A.k;
-    if (r == 0 && tid == 0) A.n_sel[b] = kk > 0 ? kk : 0;
+    if (r == 0 && tid == 0 && (!VALUES || A.n_sel)) A.n_sel[b] = kk > 0 ? kk : 0;
     if (kk <= 0) return;                                                  // uniform over the cluster
     constexpr int CH = EPT * NT;
     const int i0 = r * CH + tid * EPT;
@@ -167,11 +170,22 @@ index_select_cluster_kernel(SelArgs A) {
     }
 
     // ---- 1. approximate keys: (unscaled tensor-core score) * key scale of the token --------------------------
-    const float* s = A.scores + (size_t)b * A.score_stride;
+    const float* s = A.scores + (size_t)b * (VALUES ? (size_t)A.value_stride : (size_t)A.score_stride);
     const int32_t* bt = A.block_table + (size_t)b * g.max_pages_per_seq;
     uint32_t key[EPT];
     float skm = 0.0f;
-    {
+    if constexpr (VALUES) {
+        if (A.vec_ok && nvalid == EPT) {
+#pragma unroll
+            for (int j = 0; j < EPT; j += 4) {
+                const float4 a = *reinterpret_cast<const float4*>(s + i0 + j);
+                key[j] = topk_key(a.x); key[j + 1] = topk_key(a.y); key[j + 2] = topk_key(a.z); key[j + 3] = topk_key(a.w);
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < EPT; ++j) key[j] = j < nvalid ? topk_key(s[i0 + j]) : 0u;
+        }
+    } else {
         float sc[EPT], sk[EPT];
         if (A.vec_ok && nvalid == EPT) {
             size_t rr[EPT / 4];
@@ -208,7 +222,7 @@ index_select_cluster_kernel(SelArgs A) {
             skm = fmaxf(skm, sk[j]);
         }
     }
-    rv_rescore_stage_q(A.qcodes + (size_t)b * nh * hd, nh, qf);
+    if constexpr (!VALUES) rv_rescore_stage_q(A.qcodes + (size_t)b * nh * hd, nh, qf);
     for (int i = tid; i < SEL_BINS; i += NT) hist[i] = 0u;
     if (tid == 0) xc.list_n = 0;
     int buf = 0;
@@ -235,7 +249,7 @@ index_select_cluster_kernel(SelArgs A) {
             }
         }
     }
-    const float eps = sk_max * A.cb[b];
+    const float eps = VALUES ? 0.0f : sk_max * A.cb[b];
 
     // ---- 2. one histogram pass: 4096 bins spread linearly IN VALUE between the smallest and the largest score ----
     // bin(v) = min(4095, int((v - vmin) * inv_w)) is monotone in v, which is all the selection needs: tokens in
@@ -246,6 +260,7 @@ index_select_cluster_kernel(SelArgs A) {
     float inv_w = (float)SEL_BINS / (vmax - vmin);
     if (!(inv_w > 0.0f) || !(inv_w < 3.0e38f)) inv_w = 0.0f;
     auto bin_of = [&](uint32_t k) -> uint32_t {
+        if (VALUES && inv_w == 0.0f) return 0u;   // given scores may hold infinities and NaNs: one bin, ordered by key bits alone
         const float t = (topk_unkey(k) - vmin) * inv_w;
         return (uint32_t)fminf(t, (float)(SEL_BINS - 1));
     };
@@ -336,9 +351,13 @@ index_select_cluster_kernel(SelArgs A) {
             mn = 0xffffffffu; mx = 0u;
             for (int q = 0; q < C; ++q) { mn = min(mn, xc.bmin[q]); mx = max(mx, xc.bmax[q]); }
         }
-        const float lo_f = topk_unkey(mn) - 2.0f * eps, hi_f = topk_unkey(mx) + 2.0f * eps;
-        k_lo = lo_f == lo_f ? topk_key(lo_f) : 0u;
-        k_hi = hi_f == hi_f ? topk_key(hi_f) : 0xffffffffu;
+        if constexpr (VALUES) {
+            k_lo = mn; k_hi = mx;
+        } else {
+            const float lo_f = topk_unkey(mn) - 2.0f * eps, hi_f = topk_unkey(mx) + 2.0f * eps;
+            k_lo = lo_f == lo_f ? topk_key(lo_f) : 0u;
+            k_hi = hi_f == hi_f ? topk_key(hi_f) : 0xffffffffu;
+        }
     }
     uint32_t m_in = 0u, m_band = 0u;
 #pragma unroll
@@ -368,7 +387,10 @@ index_select_cluster_kernel(SelArgs A) {
         uint32_t pos = my_pos;
 #pragma unroll
         for (int j = 0; j < EPT; ++j)
-            if (m_band & (1u << j)) { if (pos < SEL_LIST) l_tok[pos] = (uint32_t)(i0 + j); ++pos; }
+            if (m_band & (1u << j)) {
+                if (pos < SEL_LIST) { l_tok[pos] = (uint32_t)(i0 + j); if (VALUES) l_key[pos] = key[j]; }
+                ++pos;
+            }
     }
     __syncthreads();
     const uint32_t n_in_mine = __reduce_add_sync(0xffffffffu, lane < NW ? xc.red[buf][lane] : 0u);
@@ -386,8 +408,8 @@ index_select_cluster_kernel(SelArgs A) {
     }
 
     // this lane's head constants for the exact re-score (nh <= 32)
-    const float my_sq = lane < nh ? A.qscales[(size_t)b * nh + lane] : 0.0f;
-    const float my_wh = lane < nh ? __fmul_rn(A.w[(size_t)b * nh + lane], g.index_wscale) : 0.0f;
+    const float my_sq = !VALUES && lane < nh ? A.qscales[(size_t)b * nh + lane] : 0.0f;
+    const float my_wh = !VALUES && lane < nh ? __fmul_rn(A.w[(size_t)b * nh + lane], g.index_wscale) : 0.0f;
     // Exact key of the first `ln` listed tokens -> l_key[position] (0 and ~0 are reserved for "surely out" / "surely in").
     auto rescore = [&](uint32_t ln) {
         rv_rescore_listed<NW, SEL_TOK>(l_tok, ln, qf, kfw + warp * (SEL_TOK * hd), bt, g, A.index_pool, A.index_scale,
@@ -406,8 +428,10 @@ index_select_cluster_kernel(SelArgs A) {
 
     if (n_band <= (uint32_t)SEL_LIST) {
         // ---- 4. common case: the whole band fits the list --------------------------------------------------
-        rescore(n_band_mine);
-        __syncthreads();
+        if constexpr (!VALUES) {
+            rescore(n_band_mine);
+            __syncthreads();
+        }
         const uint32_t* all_tok = l_tok;                                      // the cluster's band: a lone CTA's own lists
         const uint32_t* all_key = l_key;
         if constexpr (!SOLO) {
@@ -459,7 +483,7 @@ index_select_cluster_kernel(SelArgs A) {
     // ---- slow path (tie-dominated scores): the band does not fit the list --------------------------------------
     // Exact keys replace the approximate ones in the registers: surely-in -> all ones, surely-out -> 0, band ->
     // exact key (re-scored in chunks of SEL_LIST consecutive tokens, so a chunk's band always fits the list).
-    for (int c0 = r * CH; c0 < min(nt, (r + 1) * CH); c0 += SEL_LIST) {
+    for (int c0 = r * CH; !VALUES && c0 < min(nt, (r + 1) * CH); c0 += SEL_LIST) {
         __syncthreads();
         if (tid == 0) xc.list_n = 0;
         __syncthreads();
@@ -484,7 +508,7 @@ index_select_cluster_kernel(SelArgs A) {
     }
 #pragma unroll
     for (int j = 0; j < EPT; ++j)
-        if (j < nvalid && !(m_band & (1u << j))) key[j] = ((m_in >> j) & 1u) ? 0xffffffffu : 0u;
+        if (!VALUES && j < nvalid && !(m_band & (1u << j))) key[j] = ((m_in >> j) & 1u) ? 0xffffffffu : 0u;
     // exact cluster-wide radix selection, four 8-bit digits, MSB first; per-warp histograms so that ties never
     // serialise a CTA on one bin; whist aliases `hist`, the CTA's digit histogram goes to a_tok[0..256)
     uint32_t pivot = 0u, mask = 0u, need = (uint32_t)kk;
@@ -607,29 +631,29 @@ extern "C" __attribute__((visibility("default"))) void rivoli_index_select_test_
 
 namespace rivoli {
 
-int launch_index_select_cluster(const SelArgs& a, int B, cudaStream_t st) {
-    int C = 1, ept = 4, nt = 512;
-    if (!select_cluster_plan(B, a.score_stride, &C, &ept, &nt)) return 1002;
-    const size_t smem = ((size_t)(SEL_HD / 4) * 32 + (size_t)(nt / 32) * SEL_TOK * SEL_HD + SEL_BINS + 4 * SEL_LIST) * 4;
+template <bool VALUES>
+static int launch_select(const SelArgs& a, int B, int C, int ept, int nt, cudaStream_t st) {
+    const size_t lists = SEL_BINS + 4 * SEL_LIST;
+    const size_t smem = (lists + (VALUES ? 0 : (size_t)(SEL_HD / 4) * 32 + (size_t)(nt / 32) * SEL_TOK * SEL_HD)) * 4;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(B * C)); cfg.blockDim = dim3((unsigned)nt); cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)C; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = (unsigned)C; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
     cfg.attrs = at; cfg.numAttrs = 2;
     rv_drain_error();
-#define RV_SEL(EPT, NT)                                                                                                   \
-    do {                                                                                                                  \
-        cudaFuncSetAttribute(index_select_cluster_kernel<EPT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        (void)cudaLaunchKernelEx(&cfg, index_select_cluster_kernel<EPT, NT>, a);                                          \
+#define RV_SEL(EPT, NT)                                                                             \
+    do {                                                                                            \
+        rv_allow_smem<index_select_cluster_kernel<EPT, NT, VALUES>>((int)smem);                     \
+        (void)cudaLaunchKernelEx(&cfg, index_select_cluster_kernel<EPT, NT, VALUES>, a);            \
     } while (0)
     if (nt == 1024) {
         if (ept == 4) RV_SEL(4, 1024);
         else if (ept == 8) RV_SEL(8, 1024);
         else if (ept == 16) RV_SEL(16, 1024);
-        else return 1002;   // the plan takes 1024-thread CTAs only up to 16 keys per thread
+        else return 1002;   // the plans take 1024-thread CTAs only up to 16 keys per thread
     } else {
         if (ept == 4) RV_SEL(4, 512);
         else if (ept == 8) RV_SEL(8, 512);
@@ -638,6 +662,30 @@ int launch_index_select_cluster(const SelArgs& a, int B, cudaStream_t st) {
     }
 #undef RV_SEL
     return rv_launch_status();
+}
+
+int launch_index_select_cluster(const SelArgs& a, int B, cudaStream_t st) {
+    int C = 1, ept = 4, nt = 512;
+    if (!select_cluster_plan(B, a.score_stride, &C, &ept, &nt)) return 1002;
+    return launch_select<false>(a, B, C, ept, nt, st);
+}
+
+int launch_topk_values(const float* scores, long long stride, const int32_t* seq_len, int nt_single, int B, int k,
+                       uint32_t* rows, int32_t* n_sel, int max_nt, cudaStream_t st) {
+    if (max_nt > SEL_MAX_CLUSTER * 512 * 32 || stride > 0x7fffffff) return 1002;
+    SelArgs a{};
+    a.scores = scores; a.score_stride = max_nt; a.value_stride = stride; a.seq_len = seq_len; a.nt_single = nt_single;
+    a.rows = rows; a.n_sel = n_sel; a.k = k;
+    a.vec_ok = ((uintptr_t)scores & 15) == 0 && stride % 4 == 0;
+    // no re-score to spread: one CTA of 1024 threads up to 16,384 scores (no exchanges between CTAs; 8,193 scores: 9.7 us,
+    // four radix passes over shared memory took 14.2), beyond that clusters of eight
+    int C = 1, nt = 1024, ept = 4;
+    while (ept < 16 && nt * ept < max_nt) ept *= 2;
+    if (nt * ept < max_nt) {
+        C = SEL_MAX_CLUSTER; nt = 512; ept = 4;
+        while (ept < 32 && (long long)C * nt * ept < max_nt) ept *= 2;
+    }
+    return launch_select<true>(a, B, C, ept, nt, st);
 }
 
 }  // namespace rivoli
