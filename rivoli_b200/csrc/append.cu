@@ -7,7 +7,7 @@
 //
 // All of it is HBM-bound byte work: one warp per 128-wide (or per-vector) quantisation
 // group, absmax by warp shuffle (max is order independent, so the result is bit exact),
-// IEEE division by the scale, packed code stores (16 bytes per lane on the latent row).
+// quotients as if by IEEE division (quant.cuh), packed code stores.
 #include "codec.cuh"
 #include "common.cuh"
 #include "quant.cuh"
@@ -78,17 +78,21 @@ RIVOLI_API int rivoli_index_append(const float* k, unsigned short* kcache, int p
     return rv_launch_status();
 }
 
-__global__ void __launch_bounds__(128)
+template <int PASSES>
+__global__ void __launch_bounds__(256)
 kv_append_paged_kernel(DsaGeom g, const uint16_t* __restrict__ latent, const uint16_t* __restrict__ index_key,
                        const int32_t* __restrict__ row_seq, const int32_t* __restrict__ row_pos, int n_rows,
                        const int32_t* __restrict__ block_table, uint8_t* __restrict__ latent_pool,
                        float* __restrict__ latent_scale, uint8_t* __restrict__ index_pool,
                        float* __restrict__ index_scale, int32_t* __restrict__ status) {
     const int lane = threadIdx.x & 31;
-    const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
+    const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
+    rv_grid_dep_trigger();
+    rv_grid_dep_wait();
     if (row >= n_rows) return;
-    append_row_paged(g, latent, index_key, row, row_seq ? row_seq[row] : row, row_pos[row], block_table, latent_pool,
-                     latent_scale, index_pool, index_scale, status, lane);
+    AppendRow<PASSES> a;
+    append_row_load<PASSES>(a, g, latent, index_key, row, row_seq ? row_seq[row] : row, row_pos[row], block_table, lane);
+    append_row_store<PASSES>(a, g, latent_pool, latent_scale, index_pool, index_scale, status, lane);
 }
 
 RIVOLI_API int rivoli_kv_append_paged(const DsaGeom* g, const uint16_t* latent, const uint16_t* index_key,
@@ -106,9 +110,13 @@ RIVOLI_API int rivoli_kv_append_paged(const DsaGeom* g, const uint16_t* latent, 
         ((uintptr_t)latent_scale & 3))
         return 1005;
     rv_drain_error();
-    kv_append_paged_kernel<<<(n_rows + 3) / 4, 128, 0, (cudaStream_t)stream>>>(
-        *g, latent, index_key, row_seq, row_pos, n_rows, block_table, latent_pool, latent_scale,
-        index_pool, index_scale, status);
+    const dim3 grid((unsigned)((n_rows + 7) / 8));
+    if (rv_append_chunks(*g) <= 3 * 32)
+        rv_launch_dependent(kv_append_paged_kernel<3>, grid, dim3(256), 0, (cudaStream_t)stream, *g, latent, index_key, row_seq, row_pos,
+                            n_rows, block_table, latent_pool, latent_scale, index_pool, index_scale, status);
+    else
+        rv_launch_dependent(kv_append_paged_kernel<5>, grid, dim3(256), 0, (cudaStream_t)stream, *g, latent, index_key, row_seq, row_pos,
+                            n_rows, block_table, latent_pool, latent_scale, index_pool, index_scale, status);
     return rv_launch_status();
 }
 
@@ -118,8 +126,10 @@ index_q_quant_kernel(const uint16_t* __restrict__ q, int n_vec, int hd, uint8_t*
                      float* __restrict__ scales) {
     const int lane = threadIdx.x & 31;
     const int v = blockIdx.x * 4 + (threadIdx.x >> 5);
+    rv_grid_dep_trigger();
+    rv_grid_dep_wait();
     if (v >= n_vec) return;
-    const float s = quant_vec16(q + (size_t)v * hd, hd, codes + (size_t)v * hd, lane);
+    const float s = quant_vec(q + (size_t)v * hd, hd, codes + (size_t)v * hd, lane);
     if (lane == 0) scales[v] = s;
 }
 
@@ -129,6 +139,6 @@ RIVOLI_API int rivoli_index_q_quant(const uint16_t* q, int n_vec, int hd, uint8_
     if ((hd % 16) != 0 || hd > 512) return 1004;
     if (((uintptr_t)q | (uintptr_t)codes) & 15) return 1005;
     rv_drain_error();
-    index_q_quant_kernel<<<(n_vec + 3) / 4, 128, 0, (cudaStream_t)stream>>>(q, n_vec, hd, codes, scales);
+    rv_launch_dependent(index_q_quant_kernel, dim3((unsigned)((n_vec + 3) / 4)), dim3(128), 0, (cudaStream_t)stream, q, n_vec, hd, codes, scales);
     return rv_launch_status();
 }

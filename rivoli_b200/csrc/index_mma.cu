@@ -146,8 +146,9 @@ step_prologue_kernel(DsaGeom g, AppendArgs ap, int B, const uint16_t* __restrict
     }
     const int row = ((int)blockIdx.x - B) * 32 + (threadIdx.x >> 5);
     if (row >= B) return;
-    append_row_paged(g, ap.latent, ap.index_key, row, row, ap.row_pos[row], ap.block_table, ap.latent_pool,
-                     ap.latent_scale, ap.index_pool, ap.index_scale, ap.status, threadIdx.x & 31);
+    AppendRow<3> a;
+    append_row_load<3>(a, g, ap.latent, ap.index_key, row, row, ap.row_pos[row], ap.block_table, threadIdx.x & 31);
+    append_row_store<3>(a, g, ap.latent_pool, ap.latent_scale, ap.index_pool, ap.index_scale, ap.status, threadIdx.x & 31);
 }
 
 // ---------------------------------------------------------------------------------------------
