@@ -59,6 +59,48 @@ assert C.sizeof(DsaGeom) == 48 and C.alignment(DsaGeom) == 4
 
 _lib = None
 
+# Argument types of the entry points, by their order in include/rivoli_kernels.h: p pointer, i int, f float, d double,
+# z size_t, q 64-bit integer. With them ctypes converts plain integers itself: a call of 25 arguments costs the host
+# half of what wrapping each in a ctypes object does.
+_SIGNATURES = {
+    "append_kv": "pppppiiii", "gather_rope": "ppiiii", "index_append": "ppii", "index_score": "ppppiiiiffp",
+    "index_topk": "piip", "mla_attend": "ppppppiiiiifpp", "mla_attend_static": "ppppppiiiiifp",
+    "mla_attend_scratch_floats": "ii", "device_sync": "",
+    "kv_append_paged": "pppppi" + "p" * 7, "index_q_quant": "piippp", "index_score_paged": "p" * 8 + "ipip",
+    "index_topk_batched": "pipiippp", "index_select_scratch_bytes": "pii", "index_select_uses_mma": "pi",
+    "index_select_paged": "p" * 7 + "iipppp", "dsa_append_select_paged": "p" * 13 + "iipppp",
+    "dsa_decode_step_paged": "p" * 13 + "ii" + "p" * 8 + "ip",
+    "step_pipe_create": "pii", "step_pipe_destroy": "p", "step_pipe_input_bytes": "pi", "step_pipe_output_bytes": "pi",
+    "step_pipe_input_offsets": "pip", "dsa_step_host": "pppppp", "step_pipe_wait": "pq", "step_pipe_drain": "p",
+    "step_pipe_leg_ms": "pp", "step_pipe_stream": "pi",
+    "index_select_status": "piipp", "index_select_band_stats": "piippp", "stale_compose_rows": "ppppppiippp",
+    "mla_attend_paged_scratch_bytes": "pi", "mla_attend_paged_uses_mma": "p", "mla_attend_paged_status": "ppp",
+    "mla_attend_paged_bf16": "ppppppipippppp", "attend_simt_paged_bf16": "ppppppipippppp",
+    "attend_simt_scratch_bytes": "pi", "attend_merge_partials": "ppiiipp",
+    "shard_candidate_bytes": "pi", "shard_partial_bytes": "pi", "shard_scratch_bytes": "pii",
+    "shard_candidates": "p" * 7 + "iipppp", "shard_cut_attend": "ppii" + "p" * 5 + "i" + "p" * 6, "shard_merge": "ppiipp",
+    "shard_step_paged": "ppii" + "p" * 9 + "ii" + "p" * 8, "shard_nccl_unique_id": "p", "shard_nccl_comm_create": "piip",
+    "shard_nccl_comm_destroy": "p",
+    "pagepool_create": "iiii", "pagepool_destroy": "p", "pagepool_shuffle": "pz", "pagepool_reserve": "pii",
+    "pagepool_release": "pi", "pagepool_n_free": "p", "pagepool_seq_pages": "pi", "pagepool_block_table": "p",
+    "pagepool_free_list": "p",
+    "mla_absorb_fp8": "pppiiiiiiip", "mla_value_fp8": "pppiiiiiip", "mla_absorb_batched_bf16": "ppp" + "i" * 8 + "pip",
+    "mla_value_batched_bf16": "ppp" + "i" * 6 + "pip", "kvb_proj_status": "p",
+    "gemv_fp8": "pppiiiip", "layernorm": "pppifp", "rope_interleave": "piiiid",
+    "index_frontend_scratch_bytes": "pi", "index_frontend_bf16": "ppppi" + "p" * 12 + "ip", "index_frontend_status": "p",
+    "act_quant_f4_rotated": "piip", "index_score_blocks": "ppppiiiip", "gather_attn_shared_kv": "ppppiiiifpp",
+    "v4_select_scratch_bytes": "pi", "v4_select_blocks_bf16": "pi" + "p" * 8 + "ip", "v4_index_pack_bf16": "pippipppp",
+    "v4_sparse_attend_bf16": "pippppipip", "act_quant_f8_prefix": "ppiiiip", "kv_compress_deposit": "ppppppiip",
+    "kv_compress_prefill": "pppppip", "kv_compress_decode": "ppppip",
+    "v4_compress_step_bf16": "pi" + "p" * 8 + "ipiipppp",
+    "dsa_step_set_timing_events": "p", "attend_mma_test_hook": "iii", "index_select_test_cluster": "i", "kernels_arch": "",
+}
+_CTYPE = {"p": C.c_void_p, "i": C.c_int, "f": C.c_float, "d": C.c_double, "z": C.c_size_t, "q": C.c_longlong}
+_RESTYPE = {"mla_attend_scratch_floats": C.c_size_t, "kernels_arch": C.c_char_p, "pagepool_create": C.c_void_p,
+            "step_pipe_create": C.c_void_p, "step_pipe_stream": C.c_void_p, "dsa_step_host": C.c_longlong,
+            "step_pipe_input_bytes": C.c_size_t, "step_pipe_output_bytes": C.c_size_t,
+            "pagepool_block_table": C.POINTER(C.c_int32), "pagepool_free_list": C.POINTER(C.c_int32)}
+
 
 def library_path() -> str:
     return _SO
@@ -73,91 +115,75 @@ def lib() -> C.CDLL:
                 f"{_SO} is missing: build it with `python -m rivoli_b200.build` "
                 "(nvcc, sm_100a). rivoli_b200 has no CPU fallback.")
         L = C.CDLL(_SO)
-        L.rivoli_mla_attend_scratch_floats.restype = C.c_size_t
-        L.rivoli_mla_attend_paged_scratch_bytes.restype = C.c_size_t
-        L.rivoli_attend_simt_scratch_bytes.restype = C.c_size_t
-        L.rivoli_index_select_scratch_bytes.restype = C.c_size_t
-        L.rivoli_index_frontend_scratch_bytes.restype = C.c_size_t
-        L.rivoli_v4_select_scratch_bytes.restype = C.c_size_t
-        L.rivoli_kernels_arch.restype = C.c_char_p
-        L.rivoli_pagepool_create.restype = C.c_void_p
-        L.rivoli_pagepool_block_table.restype = C.POINTER(C.c_int32)
-        L.rivoli_pagepool_free_list.restype = C.POINTER(C.c_int32)
-        for n in ("destroy", "shuffle", "reserve", "release", "n_free", "seq_pages", "block_table", "free_list"):
-            getattr(L, f"rivoli_pagepool_{n}").argtypes = None
+        for name, sig in _SIGNATURES.items():
+            f = getattr(L, "rivoli_" + name)
+            f.argtypes = [_CTYPE[c] for c in sig]
+            f.restype = _RESTYPE.get(name, C.c_size_t if name.endswith("_bytes") else C.c_int)
         _lib = L
     return _lib
 
 
 def _ptr(x):
-    if x is None:
-        return C.c_void_p(0)
-    if isinstance(x, int):
-        return C.c_void_p(x)
-    return C.c_void_p(x.data_ptr())
+    """Device address of a tensor, an address as it is, None for NULL."""
+    return x if x is None or type(x) is int else x.data_ptr()
 
 
 def _stream(s):
-    if s is None:
-        return C.c_void_p(0)
-    if isinstance(s, int):
-        return C.c_void_p(s)
-    return C.c_void_p(s.cuda_stream)
+    return s if s is None or type(s) is int else s.cuda_stream
 
 
 def ensure_status(r: int, name: str) -> None:
     """0 = ok, positive = argument guard, negative = -(cudaError_t) (hip.rs:328-336)."""
-    if r != 0:
+    if r:
         raise BackendError(name, int(r))
 
 
 # --- Part 1: the reference's launchers ------------------------------------------------------------
 def launch_append_kv(latent, rope, lc8, lscale, rc, pos: int, kvl: int, ropn: int, n_blocks: int) -> None:
     ensure_status(lib().rivoli_append_kv(_ptr(latent), _ptr(rope), _ptr(lc8), _ptr(lscale), _ptr(rc),
-                                         C.c_int(pos), C.c_int(kvl), C.c_int(ropn), C.c_int(n_blocks)),
+                                         pos, kvl, ropn, n_blocks),
                   "append_kv")
 
 
 def launch_gather_rope(q, qrope, h: int, qh: int, nope: int, ropn: int) -> None:
-    ensure_status(lib().rivoli_gather_rope(_ptr(q), _ptr(qrope), C.c_int(h), C.c_int(qh), C.c_int(nope),
-                                           C.c_int(ropn)), "gather_rope")
+    ensure_status(lib().rivoli_gather_rope(_ptr(q), _ptr(qrope), h, qh, nope,
+                                           ropn), "gather_rope")
 
 
 def launch_index_append(k, kcache, pos: int, hd: int) -> None:
-    ensure_status(lib().rivoli_index_append(_ptr(k), _ptr(kcache), C.c_int(pos), C.c_int(hd)), "index_append")
+    ensure_status(lib().rivoli_index_append(_ptr(k), _ptr(kcache), pos, hd), "index_append")
 
 
 def launch_index_score(q, w, kcache, heads, nt: int, nh: int, nact: int, hd: int, wscale: float,
                        dscale: float, scores) -> None:
-    ensure_status(lib().rivoli_index_score(_ptr(q), _ptr(w), _ptr(kcache), _ptr(heads), C.c_int(nt),
-                                           C.c_int(nh), C.c_int(nact), C.c_int(hd), C.c_float(wscale),
-                                           C.c_float(dscale), _ptr(scores)), "index_score")
+    ensure_status(lib().rivoli_index_score(_ptr(q), _ptr(w), _ptr(kcache), _ptr(heads), nt,
+                                           nh, nact, hd, wscale,
+                                           dscale, _ptr(scores)), "index_score")
 
 
 def launch_index_topk(scores, nt: int, k: int, rows) -> None:
-    ensure_status(lib().rivoli_index_topk(_ptr(scores), C.c_int(nt), C.c_int(k), _ptr(rows)), "index_topk")
+    ensure_status(lib().rivoli_index_topk(_ptr(scores), nt, k, _ptr(rows)), "index_topk")
 
 
 def launch_attend(qabs, qrope, lc8, lscale, rc, rows, h: int, nr: int, kvl: int, rope: int, n_blocks: int,
                   scale: float, clat, partial) -> None:
     ensure_status(lib().rivoli_mla_attend(_ptr(qabs), _ptr(qrope), _ptr(lc8), _ptr(lscale), _ptr(rc),
-                                          _ptr(rows), C.c_int(h), C.c_int(nr), C.c_int(kvl), C.c_int(rope),
-                                          C.c_int(n_blocks), C.c_float(scale), _ptr(clat), _ptr(partial)),
+                                          _ptr(rows), h, nr, kvl, rope,
+                                          n_blocks, scale, _ptr(clat), _ptr(partial)),
                   "mla_attend")
 
 
 def launch_attend_static(qabs, qrope, lc8, lscale, rc, rows, h: int, nr: int, kvl: int, rope: int, n_blocks: int,
                          scale: float, clat) -> None:
-    """``launch_attend`` for callers that cannot lend device scratch: the split partials live in
-    an array built into the library (h <= 64, kvl <= 512). One call at a time per device."""
+    """``launch_attend`` for callers that cannot lend device scratch (h <= 64, kvl <= 512)."""
     ensure_status(lib().rivoli_mla_attend_static(_ptr(qabs), _ptr(qrope), _ptr(lc8), _ptr(lscale), _ptr(rc),
-                                                 _ptr(rows), C.c_int(h), C.c_int(nr), C.c_int(kvl), C.c_int(rope),
-                                                 C.c_int(n_blocks), C.c_float(scale), _ptr(clat)),
+                                                 _ptr(rows), h, nr, kvl, rope,
+                                                 n_blocks, scale, _ptr(clat)),
                   "mla_attend_static")
 
 
 def attend_scratch_floats(h: int, kvl: int) -> int:
-    return int(lib().rivoli_mla_attend_scratch_floats(C.c_int(h), C.c_int(kvl)))
+    return int(lib().rivoli_mla_attend_scratch_floats(h, kvl))
 
 
 def device_sync() -> None:
@@ -168,14 +194,14 @@ def device_sync() -> None:
 def launch_kv_append_paged(g: DsaGeom, latent, index_key, row_seq, row_pos, n_rows: int, block_table,
                            latent_pool, latent_scale, index_pool, index_scale, status=None, stream=None) -> None:
     ensure_status(lib().rivoli_kv_append_paged(C.byref(g), _ptr(latent), _ptr(index_key), _ptr(row_seq),
-                                               _ptr(row_pos), C.c_int(n_rows), _ptr(block_table),
+                                               _ptr(row_pos), n_rows, _ptr(block_table),
                                                _ptr(latent_pool), _ptr(latent_scale), _ptr(index_pool),
                                                _ptr(index_scale), _ptr(status), _stream(stream)),
                   "kv_append_paged")
 
 
 def launch_index_q_quant(q, n_vec: int, hd: int, codes, scales, stream=None) -> None:
-    ensure_status(lib().rivoli_index_q_quant(_ptr(q), C.c_int(n_vec), C.c_int(hd), _ptr(codes), _ptr(scales),
+    ensure_status(lib().rivoli_index_q_quant(_ptr(q), n_vec, hd, _ptr(codes), _ptr(scales),
                                              _stream(stream)), "index_q_quant")
 
 
@@ -183,23 +209,23 @@ def launch_index_score_paged(g: DsaGeom, qcodes, qscales, w, index_pool, index_s
                              B: int, scores, score_stride: int, stream=None) -> None:
     ensure_status(lib().rivoli_index_score_paged(C.byref(g), _ptr(qcodes), _ptr(qscales), _ptr(w),
                                                  _ptr(index_pool), _ptr(index_scale), _ptr(block_table),
-                                                 _ptr(seq_len), C.c_int(B), _ptr(scores),
-                                                 C.c_int(score_stride), _stream(stream)), "index_score_paged")
+                                                 _ptr(seq_len), B, _ptr(scores),
+                                                 score_stride, _stream(stream)), "index_score_paged")
 
 
 def launch_index_topk_batched(scores, score_stride: int, seq_len, B: int, k: int, rows, n_sel,
                               stream=None) -> None:
-    ensure_status(lib().rivoli_index_topk_batched(_ptr(scores), C.c_int(score_stride), _ptr(seq_len),
-                                                  C.c_int(B), C.c_int(k), _ptr(rows), _ptr(n_sel),
+    ensure_status(lib().rivoli_index_topk_batched(_ptr(scores), score_stride, _ptr(seq_len),
+                                                  B, k, _ptr(rows), _ptr(n_sel),
                                                   _stream(stream)), "index_topk_batched")
 
 
 def index_select_scratch_bytes(g: DsaGeom, B: int, score_stride: int) -> int:
-    return int(lib().rivoli_index_select_scratch_bytes(C.byref(g), C.c_int(B), C.c_int(score_stride)))
+    return int(lib().rivoli_index_select_scratch_bytes(C.byref(g), B, score_stride))
 
 
 def index_select_uses_mma(g: DsaGeom, score_stride: int) -> bool:
-    return bool(lib().rivoli_index_select_uses_mma(C.byref(g), C.c_int(score_stride)))
+    return bool(lib().rivoli_index_select_uses_mma(C.byref(g), score_stride))
 
 
 def launch_index_select_paged(g: DsaGeom, index_q, w, index_pool, index_scale, block_table, seq_len, B: int,
@@ -207,7 +233,7 @@ def launch_index_select_paged(g: DsaGeom, index_q, w, index_pool, index_scale, b
     """Fused indexer (q quant + scores + exact top-k); rows identical to the unfused chain."""
     ensure_status(lib().rivoli_index_select_paged(C.byref(g), _ptr(index_q), _ptr(w), _ptr(index_pool),
                                                   _ptr(index_scale), _ptr(block_table), _ptr(seq_len),
-                                                  C.c_int(B), C.c_int(score_stride), _ptr(rows), _ptr(n_sel),
+                                                  B, score_stride, _ptr(rows), _ptr(n_sel),
                                                   _ptr(scratch), _stream(stream)), "index_select_paged")
 
 
@@ -217,7 +243,7 @@ def launch_dsa_append_select_paged(g: DsaGeom, latent, index_key, row_pos, block
     ensure_status(lib().rivoli_dsa_append_select_paged(
         C.byref(g), _ptr(latent), _ptr(index_key), _ptr(row_pos), _ptr(block_table), _ptr(latent_pool),
         _ptr(latent_scale), _ptr(index_pool), _ptr(index_scale), _ptr(status), _ptr(index_q), _ptr(w), _ptr(seq_len),
-        C.c_int(B), C.c_int(score_stride), _ptr(rows), _ptr(n_sel), _ptr(scratch), _stream(stream)),
+        B, score_stride, _ptr(rows), _ptr(n_sel), _ptr(scratch), _stream(stream)),
         "dsa_append_select_paged")
 
 
@@ -229,8 +255,8 @@ def launch_dsa_decode_step_paged(g: DsaGeom, latent, index_key, row_pos, block_t
     ensure_status(lib().rivoli_dsa_decode_step_paged(
         C.byref(g), _ptr(latent), _ptr(index_key), _ptr(row_pos), _ptr(block_table), _ptr(latent_pool),
         _ptr(latent_scale), _ptr(index_pool), _ptr(index_scale), _ptr(status), _ptr(index_q), _ptr(w), _ptr(seq_len),
-        C.c_int(B), C.c_int(score_stride), _ptr(rows), _ptr(n_sel), _ptr(select_scratch), _ptr(q), _ptr(out),
-        _ptr(out_m), _ptr(out_lse), _ptr(attend_scratch), C.c_int(min_rows_hint), _stream(stream)),
+        B, score_stride, _ptr(rows), _ptr(n_sel), _ptr(select_scratch), _ptr(q), _ptr(out),
+        _ptr(out_m), _ptr(out_lse), _ptr(attend_scratch), min_rows_hint, _stream(stream)),
         "dsa_decode_step_paged")
 
 
@@ -247,19 +273,14 @@ class StepPipe:
 
     def __init__(self, g: DsaGeom, B: int, depth: int = 2):
         L = lib()
-        L.rivoli_step_pipe_create.restype = C.c_void_p
-        L.rivoli_step_pipe_stream.restype = C.c_void_p
-        L.rivoli_step_pipe_input_bytes.restype = C.c_size_t
-        L.rivoli_step_pipe_output_bytes.restype = C.c_size_t
-        L.rivoli_dsa_step_host.restype = C.c_longlong
-        self._h = C.c_void_p(L.rivoli_step_pipe_create(C.byref(g), C.c_int(B), C.c_int(depth)))
+        self._h = C.c_void_p(L.rivoli_step_pipe_create(C.byref(g), B, depth))
         if not self._h:
             raise BackendError("step_pipe_create", 1008)
         self.g, self.B, self.depth = g, B, depth
-        self.input_bytes = int(L.rivoli_step_pipe_input_bytes(C.byref(g), C.c_int(B)))
-        self.output_bytes = int(L.rivoli_step_pipe_output_bytes(C.byref(g), C.c_int(B)))
+        self.input_bytes = int(L.rivoli_step_pipe_input_bytes(C.byref(g), B))
+        self.output_bytes = int(L.rivoli_step_pipe_output_bytes(C.byref(g), B))
         off = (C.c_size_t * 5)()
-        ensure_status(L.rivoli_step_pipe_input_offsets(C.byref(g), C.c_int(B), off), "step_pipe_input_offsets")
+        ensure_status(L.rivoli_step_pipe_input_offsets(C.byref(g), B, off), "step_pipe_input_offsets")
         self.offsets = dict(zip(("latent", "index_key", "index_q", "index_w", "q"), (int(o) for o in off)))
 
     def __del__(self):
@@ -278,7 +299,7 @@ class StepPipe:
         return t
 
     def wait(self, ticket: int) -> None:
-        ensure_status(lib().rivoli_step_pipe_wait(self._h, C.c_longlong(ticket)), "step_pipe_wait")
+        ensure_status(lib().rivoli_step_pipe_wait(self._h, ticket), "step_pipe_wait")
 
     def drain(self) -> None:
         ensure_status(lib().rivoli_step_pipe_drain(self._h), "step_pipe_drain")
@@ -289,20 +310,20 @@ class StepPipe:
         return {"upload": float(ms[0]), "kernels_after_upload": float(ms[1]), "download_after_kernels": float(ms[2])}
 
     def stream(self, which: int) -> int:
-        return int(lib().rivoli_step_pipe_stream(self._h, C.c_int(which)) or 0)
+        return int(lib().rivoli_step_pipe_stream(self._h, which) or 0)
 
 
 def index_select_status(g: DsaGeom, B: int, score_stride: int, scratch, stream=None) -> None:
     """Synchronises; raises BackendError(1008) if a bounded device-side wait gave up, (1005) if a block-table
     entry inside a sequence pointed outside the pool."""
-    ensure_status(lib().rivoli_index_select_status(C.byref(g), C.c_int(B), C.c_int(score_stride), _ptr(scratch),
+    ensure_status(lib().rivoli_index_select_status(C.byref(g), B, score_stride, _ptr(scratch),
                                                    _stream(stream)), "index_select_status")
 
 
 def index_select_band_stats(g: DsaGeom, B: int, score_stride: int, scratch, stream=None):
     import numpy as np
     out = np.zeros(B, dtype=np.uint32)
-    ensure_status(lib().rivoli_index_select_band_stats(C.byref(g), C.c_int(B), C.c_int(score_stride),
+    ensure_status(lib().rivoli_index_select_band_stats(C.byref(g), B, score_stride,
                                                        _ptr(scratch), out.ctypes.data_as(C.c_void_p),
                                                        _stream(stream)), "index_select_band_stats")
     return out
@@ -311,12 +332,12 @@ def index_select_band_stats(g: DsaGeom, B: int, score_stride: int, scratch, stre
 def launch_stale_compose_rows(prev_rows, prev_n, cur_rows, cur_n, mode, seq_len, B: int, k: int, out_rows, out_n,
                               stream=None) -> None:
     ensure_status(lib().rivoli_stale_compose_rows(_ptr(prev_rows), _ptr(prev_n), _ptr(cur_rows), _ptr(cur_n), _ptr(mode),
-                                                  _ptr(seq_len), C.c_int(B), C.c_int(k), _ptr(out_rows), _ptr(out_n),
+                                                  _ptr(seq_len), B, k, _ptr(out_rows), _ptr(out_n),
                                                   _stream(stream)), "stale_compose_rows")
 
 
 def attend_paged_scratch_bytes(g: DsaGeom, B: int) -> int:
-    return int(lib().rivoli_mla_attend_paged_scratch_bytes(C.byref(g), C.c_int(B)))
+    return int(lib().rivoli_mla_attend_paged_scratch_bytes(C.byref(g), B))
 
 
 def attend_paged_uses_mma(g: DsaGeom) -> bool:
@@ -341,22 +362,22 @@ def step_set_timing_events(events) -> None:
 
 def attend_mma_test_hook(min_rows: int = -1, withhold: int = 0, max_polls: int = 0) -> None:
     """Test hook of the tensor-core attention (see include/rivoli_kernels.h); not for production callers."""
-    lib().rivoli_attend_mma_test_hook(C.c_int(min_rows), C.c_int(withhold), C.c_int(max_polls))
+    lib().rivoli_attend_mma_test_hook(min_rows, withhold, max_polls)
 
 
 def index_select_test_cluster(cluster: int = 0) -> None:
     """Test hook: force the selection kernel's cluster size (1, 2, 4, 8; 0 = the library's plan)."""
-    lib().rivoli_index_select_test_cluster(C.c_int(cluster))
+    lib().rivoli_index_select_test_cluster(cluster)
 
 
 def attend_simt_scratch_bytes(g: DsaGeom, B: int) -> int:
-    return int(lib().rivoli_attend_simt_scratch_bytes(C.byref(g), C.c_int(B)))
+    return int(lib().rivoli_attend_simt_scratch_bytes(C.byref(g), B))
 
 
 def _attend_paged(fn, name, g, q, latent_pool, latent_scale, block_table, rows, row_stride, n_rows, B, out,
                   out_m, out_lse, scratch, stream):
     ensure_status(fn(C.byref(g), _ptr(q), _ptr(latent_pool), _ptr(latent_scale), _ptr(block_table),
-                     _ptr(rows), C.c_int(row_stride), _ptr(n_rows), C.c_int(B), _ptr(out), _ptr(out_m),
+                     _ptr(rows), row_stride, _ptr(n_rows), B, _ptr(out), _ptr(out_m),
                      _ptr(out_lse), _ptr(scratch), _stream(stream)), name)
 
 
@@ -374,34 +395,28 @@ def launch_attend_simt_paged_bf16(g: DsaGeom, q, latent_pool, latent_scale, bloc
 
 
 def launch_attend_merge_partials(part_out, part_lse, G: int, n_vec: int, kvl: int, out, stream=None) -> None:
-    ensure_status(lib().rivoli_attend_merge_partials(_ptr(part_out), _ptr(part_lse), C.c_int(G),
-                                                     C.c_int(n_vec), C.c_int(kvl), _ptr(out),
+    ensure_status(lib().rivoli_attend_merge_partials(_ptr(part_out), _ptr(part_lse), G,
+                                                     n_vec, kvl, _ptr(out),
                                                      _stream(stream)), "attend_merge_partials")
 
 
 # --- page-range sharded step --------------------------------------------------------------------------------
 def shard_candidate_bytes(g: DsaGeom, B: int) -> int:
-    f = lib().rivoli_shard_candidate_bytes
-    f.restype = C.c_size_t
-    return int(f(C.byref(g), C.c_int(B)))
+    return int(lib().rivoli_shard_candidate_bytes(C.byref(g), B))
 
 
 def shard_partial_bytes(g: DsaGeom, B: int) -> int:
-    f = lib().rivoli_shard_partial_bytes
-    f.restype = C.c_size_t
-    return int(f(C.byref(g), C.c_int(B)))
+    return int(lib().rivoli_shard_partial_bytes(C.byref(g), B))
 
 
 def shard_scratch_bytes(g: DsaGeom, B: int, world: int) -> int:
-    f = lib().rivoli_shard_scratch_bytes
-    f.restype = C.c_size_t
-    return int(f(C.byref(g), C.c_int(B), C.c_int(world)))
+    return int(lib().rivoli_shard_scratch_bytes(C.byref(g), B, world))
 
 
 def launch_shard_candidates(g: DsaGeom, index_q, w, index_pool, index_scale, block_table, local_len, B: int,
                             score_stride: int, rows_l, select_scratch, cand, stream=None) -> None:
     ensure_status(lib().rivoli_shard_candidates(C.byref(g), _ptr(index_q), _ptr(w), _ptr(index_pool), _ptr(index_scale),
-                                                _ptr(block_table), _ptr(local_len), C.c_int(B), C.c_int(score_stride),
+                                                _ptr(block_table), _ptr(local_len), B, score_stride,
                                                 _ptr(rows_l), _ptr(select_scratch), _ptr(cand), _stream(stream)),
                   "shard_candidates")
 
@@ -409,14 +424,14 @@ def launch_shard_candidates(g: DsaGeom, index_q, w, index_pool, index_scale, blo
 def launch_shard_cut_attend(g: DsaGeom, all_cand, rank: int, world: int, rows_l, q, latent_pool, latent_scale,
                             block_table, B: int, rows_att, n_mine, part, shard_scratch, attend_scratch,
                             stream=None) -> None:
-    ensure_status(lib().rivoli_shard_cut_attend(C.byref(g), _ptr(all_cand), C.c_int(rank), C.c_int(world), _ptr(rows_l),
+    ensure_status(lib().rivoli_shard_cut_attend(C.byref(g), _ptr(all_cand), rank, world, _ptr(rows_l),
                                                 _ptr(q), _ptr(latent_pool), _ptr(latent_scale), _ptr(block_table),
-                                                C.c_int(B), _ptr(rows_att), _ptr(n_mine), _ptr(part), _ptr(shard_scratch),
+                                                B, _ptr(rows_att), _ptr(n_mine), _ptr(part), _ptr(shard_scratch),
                                                 _ptr(attend_scratch), _stream(stream)), "shard_cut_attend")
 
 
 def launch_shard_merge(g: DsaGeom, all_part, world: int, B: int, out, stream=None) -> None:
-    ensure_status(lib().rivoli_shard_merge(C.byref(g), _ptr(all_part), C.c_int(world), C.c_int(B), _ptr(out),
+    ensure_status(lib().rivoli_shard_merge(C.byref(g), _ptr(all_part), world, B, _ptr(out),
                                            _stream(stream)), "shard_merge")
 
 
@@ -424,9 +439,9 @@ def launch_shard_step_paged(g: DsaGeom, comm: int, rank: int, world: int, index_
                             index_pool, index_scale, block_table, local_len, B: int, score_stride: int, rows_l,
                             rows_att, n_mine, out, select_scratch, attend_scratch, shard_scratch, stream=None) -> None:
     ensure_status(lib().rivoli_shard_step_paged(
-        C.byref(g), C.c_void_p(comm or 0), C.c_int(rank), C.c_int(world), _ptr(index_q), _ptr(w), _ptr(q),
+        C.byref(g), C.c_void_p(comm or 0), rank, world, _ptr(index_q), _ptr(w), _ptr(q),
         _ptr(latent_pool), _ptr(latent_scale), _ptr(index_pool), _ptr(index_scale), _ptr(block_table), _ptr(local_len),
-        C.c_int(B), C.c_int(score_stride), _ptr(rows_l), _ptr(rows_att), _ptr(n_mine), _ptr(out), _ptr(select_scratch),
+        B, score_stride, _ptr(rows_l), _ptr(rows_att), _ptr(n_mine), _ptr(out), _ptr(select_scratch),
         _ptr(attend_scratch), _ptr(shard_scratch), _stream(stream)), "shard_step_paged")
 
 
@@ -438,7 +453,7 @@ def shard_nccl_unique_id() -> bytes:
 
 def shard_nccl_comm_create(unique_id: bytes, rank: int, world: int) -> int:
     comm = C.c_void_p(0)
-    ensure_status(lib().rivoli_shard_nccl_comm_create(C.c_char_p(unique_id), C.c_int(rank), C.c_int(world),
+    ensure_status(lib().rivoli_shard_nccl_comm_create(C.c_char_p(unique_id), rank, world,
                                                       C.byref(comm)), "shard_nccl_comm_create")
     return int(comm.value or 0)
 
@@ -452,8 +467,8 @@ class PagePool:
     """LIFO page allocator + per-sequence block tables (host memory; C++ ``rivoli::PagePool``)."""
 
     def __init__(self, n_pages: int, n_seqs: int, max_pages_per_seq: int, page_tokens: int):
-        self._h = C.c_void_p(lib().rivoli_pagepool_create(C.c_int(n_pages), C.c_int(n_seqs),
-                                                          C.c_int(max_pages_per_seq), C.c_int(page_tokens)))
+        self._h = C.c_void_p(lib().rivoli_pagepool_create(n_pages, n_seqs,
+                                                          max_pages_per_seq, page_tokens))
         if not self._h:
             raise BackendError("pagepool_create", 1001)
         self.n_pages, self.n_seqs = n_pages, n_seqs
@@ -468,20 +483,20 @@ class PagePool:
             pass
 
     def shuffle(self, seed: int) -> None:
-        lib().rivoli_pagepool_shuffle(self._h, C.c_uint64(seed))
+        lib().rivoli_pagepool_shuffle(self._h, seed)
 
     def reserve(self, seq: int, n_tokens: int) -> None:
-        ensure_status(lib().rivoli_pagepool_reserve(self._h, C.c_int(seq), C.c_int(n_tokens)), "pagepool_reserve")
+        ensure_status(lib().rivoli_pagepool_reserve(self._h, seq, n_tokens), "pagepool_reserve")
 
     def release(self, seq: int) -> None:
-        ensure_status(lib().rivoli_pagepool_release(self._h, C.c_int(seq)), "pagepool_release")
+        ensure_status(lib().rivoli_pagepool_release(self._h, seq), "pagepool_release")
 
     @property
     def n_free(self) -> int:
         return int(lib().rivoli_pagepool_n_free(self._h))
 
     def seq_pages(self, seq: int) -> int:
-        return int(lib().rivoli_pagepool_seq_pages(self._h, C.c_int(seq)))
+        return int(lib().rivoli_pagepool_seq_pages(self._h, seq))
 
     def block_table(self):
         import numpy as np
@@ -499,30 +514,30 @@ class PagePool:
 
 def launch_mla_absorb(q, kvb, kvb_scale, H: int, qh: int, nope: int, vh: int, kvl: int, block: int, nrow: int,
                       qabs) -> None:
-    ensure_status(lib().rivoli_mla_absorb_fp8(_ptr(q), _ptr(kvb), _ptr(kvb_scale), C.c_int(H), C.c_int(qh),
-                                              C.c_int(nope), C.c_int(vh), C.c_int(kvl), C.c_int(block), C.c_int(nrow),
+    ensure_status(lib().rivoli_mla_absorb_fp8(_ptr(q), _ptr(kvb), _ptr(kvb_scale), H, qh,
+                                              nope, vh, kvl, block, nrow,
                                               _ptr(qabs)), "mla_absorb_fp8")
 
 
 def launch_mla_value(clat, kvb, kvb_scale, H: int, nope: int, vh: int, kvl: int, block: int, nrow: int, ctx) -> None:
-    ensure_status(lib().rivoli_mla_value_fp8(_ptr(clat), _ptr(kvb), _ptr(kvb_scale), C.c_int(H), C.c_int(nope),
-                                             C.c_int(vh), C.c_int(kvl), C.c_int(block), C.c_int(nrow), _ptr(ctx)),
+    ensure_status(lib().rivoli_mla_value_fp8(_ptr(clat), _ptr(kvb), _ptr(kvb_scale), H, nope,
+                                             vh, kvl, block, nrow, _ptr(ctx)),
                   "mla_value_fp8")
 
 
 def launch_mla_absorb_batched_bf16(q, kvb, kvb_scale, H: int, qh: int, nope: int, vh: int, kvl: int, rope: int,
                                    block: int, B: int, q_abs, force_simt: bool = False, stream=None) -> None:
-    ensure_status(lib().rivoli_mla_absorb_batched_bf16(_ptr(q), _ptr(kvb), _ptr(kvb_scale), C.c_int(H), C.c_int(qh),
-                                                       C.c_int(nope), C.c_int(vh), C.c_int(kvl), C.c_int(rope),
-                                                       C.c_int(block), C.c_int(B), _ptr(q_abs), C.c_int(int(force_simt)),
+    ensure_status(lib().rivoli_mla_absorb_batched_bf16(_ptr(q), _ptr(kvb), _ptr(kvb_scale), H, qh,
+                                                       nope, vh, kvl, rope,
+                                                       block, B, _ptr(q_abs), int(force_simt),
                                                        _stream(stream)), "mla_absorb_batched_bf16")
 
 
 def launch_mla_value_batched_bf16(clat, kvb, kvb_scale, H: int, nope: int, vh: int, kvl: int, block: int, B: int, ctx,
                                   force_simt: bool = False, stream=None) -> None:
-    ensure_status(lib().rivoli_mla_value_batched_bf16(_ptr(clat), _ptr(kvb), _ptr(kvb_scale), C.c_int(H), C.c_int(nope),
-                                                      C.c_int(vh), C.c_int(kvl), C.c_int(block), C.c_int(B), _ptr(ctx),
-                                                      C.c_int(int(force_simt)), _stream(stream)),
+    ensure_status(lib().rivoli_mla_value_batched_bf16(_ptr(clat), _ptr(kvb), _ptr(kvb_scale), H, nope,
+                                                      vh, kvl, block, B, _ptr(ctx),
+                                                      int(force_simt), _stream(stream)),
                   "mla_value_batched_bf16")
 
 
@@ -537,30 +552,30 @@ class IndexFrontGeom(C.Structure):
 
 
 def launch_gemv_fp8(x, packed, scale, o_dim: int, i_dim: int, block: int, nrow: int, y) -> None:
-    ensure_status(lib().rivoli_gemv_fp8(_ptr(x), _ptr(packed), _ptr(scale), C.c_int(o_dim), C.c_int(i_dim), C.c_int(block),
-                                        C.c_int(nrow), _ptr(y)), "gemv_fp8")
+    ensure_status(lib().rivoli_gemv_fp8(_ptr(x), _ptr(packed), _ptr(scale), o_dim, i_dim, block,
+                                        nrow, _ptr(y)), "gemv_fp8")
 
 
 def launch_layernorm(x, w, b, n: int, eps: float, y) -> None:
-    ensure_status(lib().rivoli_layernorm(_ptr(x), _ptr(w), _ptr(b), C.c_int(n), C.c_float(eps), _ptr(y)), "layernorm")
+    ensure_status(lib().rivoli_layernorm(_ptr(x), _ptr(w), _ptr(b), n, eps, _ptr(y)), "layernorm")
 
 
 def launch_rope_interleave(base, count: int, stride: int, seg: int, pos: int, theta: float) -> None:
-    ensure_status(lib().rivoli_rope_interleave(_ptr(base), C.c_int(count), C.c_int(stride), C.c_int(seg), C.c_int(pos),
-                                               C.c_double(theta)), "rope_interleave")
+    ensure_status(lib().rivoli_rope_interleave(_ptr(base), count, stride, seg, pos,
+                                               theta), "rope_interleave")
 
 
 def index_frontend_scratch_bytes(g: IndexFrontGeom, B: int) -> int:
-    return int(lib().rivoli_index_frontend_scratch_bytes(C.byref(g), C.c_int(B)))
+    return int(lib().rivoli_index_frontend_scratch_bytes(C.byref(g), B))
 
 
 def launch_index_frontend_bf16(g: IndexFrontGeom, x, q_resid, pos, B: int, wk, wk_scale, knorm_w, knorm_b, wq_b, wq_b_scale,
                                wproj, wproj_scale, index_key, index_q, index_w, scratch, force_simt: bool = False,
                                stream=None) -> None:
     ensure_status(lib().rivoli_index_frontend_bf16(
-        C.byref(g), _ptr(x), _ptr(q_resid), _ptr(pos), C.c_int(B), _ptr(wk), _ptr(wk_scale), _ptr(knorm_w), _ptr(knorm_b),
+        C.byref(g), _ptr(x), _ptr(q_resid), _ptr(pos), B, _ptr(wk), _ptr(wk_scale), _ptr(knorm_w), _ptr(knorm_b),
         _ptr(wq_b), _ptr(wq_b_scale), _ptr(wproj), _ptr(wproj_scale), _ptr(index_key), _ptr(index_q), _ptr(index_w),
-        _ptr(scratch), C.c_int(int(force_simt)), _stream(stream)), "index_frontend_bf16")
+        _ptr(scratch), int(force_simt), _stream(stream)), "index_frontend_bf16")
 
 
 def index_frontend_status(stream=None) -> None:
@@ -583,45 +598,45 @@ class V4Geom(C.Structure):
 
 def launch_act_quant_f4_rotated(x, rows: int, d: int, stream=None) -> None:
     """crates/backend/src/hip.rs launcher of ``rivoli_act_quant_f4_rotated`` (in place on f32 rows)."""
-    ensure_status(lib().rivoli_act_quant_f4_rotated(_ptr(x), C.c_int(rows), C.c_int(d), _stream(stream)),
+    ensure_status(lib().rivoli_act_quant_f4_rotated(_ptr(x), rows, d, _stream(stream)),
                   "act_quant_f4_rotated")
 
 
 def launch_index_score_blocks(q, kv, w, score, s: int, n_comp: int, heads: int, hd: int, stream=None) -> None:
-    ensure_status(lib().rivoli_index_score_blocks(_ptr(q), _ptr(kv), _ptr(w), _ptr(score), C.c_int(s), C.c_int(n_comp),
-                                                  C.c_int(heads), C.c_int(hd), _stream(stream)), "index_score_blocks")
+    ensure_status(lib().rivoli_index_score_blocks(_ptr(q), _ptr(kv), _ptr(w), _ptr(score), s, n_comp,
+                                                  heads, hd, _stream(stream)), "index_score_blocks")
 
 
 def launch_gather_attn_shared_kv(q, kv, sink, idxs, m: int, h: int, d: int, topk: int, scale: float, o,
                                  stream=None) -> None:
-    ensure_status(lib().rivoli_gather_attn_shared_kv(_ptr(q), _ptr(kv), _ptr(sink), _ptr(idxs), C.c_int(m), C.c_int(h),
-                                                     C.c_int(d), C.c_int(topk), C.c_float(scale), _ptr(o),
+    ensure_status(lib().rivoli_gather_attn_shared_kv(_ptr(q), _ptr(kv), _ptr(sink), _ptr(idxs), m, h,
+                                                     d, topk, scale, _ptr(o),
                                                      _stream(stream)), "gather_attn_shared_kv")
 
 
 def v4_select_scratch_bytes(g: V4Geom, n_seqs: int) -> int:
-    return int(lib().rivoli_v4_select_scratch_bytes(C.byref(g), C.c_int(n_seqs)))
+    return int(lib().rivoli_v4_select_scratch_bytes(C.byref(g), n_seqs))
 
 
 def launch_v4_select_blocks_bf16(g: V4Geom, n_seqs: int, pos, index_q, index_w, index_kv, sel, scratch,
                                  force_fold: bool = False, packed=None, packed_exp=None, stream=None) -> None:
-    ensure_status(lib().rivoli_v4_select_blocks_bf16(C.byref(g), C.c_int(n_seqs), _ptr(pos), _ptr(index_q), _ptr(index_w),
+    ensure_status(lib().rivoli_v4_select_blocks_bf16(C.byref(g), n_seqs, _ptr(pos), _ptr(index_q), _ptr(index_w),
                                                      _ptr(index_kv), _ptr(packed), _ptr(packed_exp), _ptr(sel),
-                                                     _ptr(scratch), C.c_int(int(force_fold)), _stream(stream)),
+                                                     _ptr(scratch), int(force_fold), _stream(stream)),
                   "v4_select_blocks_bf16")
 
 
 def launch_v4_index_pack_bf16(g: V4Geom, n_seqs: int, row_begin, row_end, max_rows: int, index_kv, packed, packed_exp,
                               stream=None) -> None:
-    ensure_status(lib().rivoli_v4_index_pack_bf16(C.byref(g), C.c_int(n_seqs), _ptr(row_begin), _ptr(row_end),
-                                                  C.c_int(max_rows), _ptr(index_kv), _ptr(packed), _ptr(packed_exp),
+    ensure_status(lib().rivoli_v4_index_pack_bf16(C.byref(g), n_seqs, _ptr(row_begin), _ptr(row_end),
+                                                  max_rows, _ptr(index_kv), _ptr(packed), _ptr(packed_exp),
                                                   _stream(stream)), "v4_index_pack_bf16")
 
 
 def launch_v4_sparse_attend_bf16(g: V4Geom, n_seqs: int, q, kv_cache, sink, sel, cols: int, out,
                                  force_simt: bool = False, stream=None) -> None:
-    ensure_status(lib().rivoli_v4_sparse_attend_bf16(C.byref(g), C.c_int(n_seqs), _ptr(q), _ptr(kv_cache), _ptr(sink),
-                                                     _ptr(sel), C.c_int(cols), _ptr(out), C.c_int(int(force_simt)),
+    ensure_status(lib().rivoli_v4_sparse_attend_bf16(C.byref(g), n_seqs, _ptr(q), _ptr(kv_cache), _ptr(sink),
+                                                     _ptr(sel), cols, _ptr(out), int(force_simt),
                                                      _stream(stream)), "v4_sparse_attend_bf16")
 
 
@@ -640,35 +655,35 @@ class CompFinish(C.Structure):
 
 
 def launch_act_quant_f8_prefix(src, dst, rows: int, row_stride: int, n: int, block: int, stream=None) -> None:
-    ensure_status(lib().rivoli_act_quant_f8_prefix(_ptr(src), _ptr(dst), C.c_int(rows), C.c_int(row_stride), C.c_int(n),
-                                                   C.c_int(block), _stream(stream)), "act_quant_f8_prefix")
+    ensure_status(lib().rivoli_act_quant_f8_prefix(_ptr(src), _ptr(dst), rows, row_stride, n,
+                                                   block, _stream(stream)), "act_quant_f8_prefix")
 
 
 def launch_kv_compress_deposit(kv, score, ape, kv_state, score_state, p: CompGeom, s: int, slot0: int, stream=None) -> None:
     ensure_status(lib().rivoli_kv_compress_deposit(_ptr(kv), _ptr(score), _ptr(ape), _ptr(kv_state), _ptr(score_state),
-                                                   C.byref(p) if p is not None else None, C.c_int(s), C.c_int(slot0),
+                                                   C.byref(p) if p is not None else None, s, slot0,
                                                    _stream(stream)), "kv_compress_deposit")
 
 
 def launch_kv_compress_prefill(kv, score, ape, norm, freqs, out, p: CompGeom, nblk: int, stream=None) -> None:
     f = CompFinish(_ptr(norm), _ptr(freqs), _ptr(out))
-    ensure_status(lib().rivoli_kv_compress_prefill(_ptr(kv), _ptr(score), _ptr(ape), C.byref(f), C.byref(p), C.c_int(nblk),
+    ensure_status(lib().rivoli_kv_compress_prefill(_ptr(kv), _ptr(score), _ptr(ape), C.byref(f), C.byref(p), nblk,
                                                    _stream(stream)), "kv_compress_prefill")
 
 
 def launch_kv_compress_decode(kv_state, score_state, norm, freqs, out, p: CompGeom, start_pos: int, stream=None) -> None:
     f = CompFinish(_ptr(norm), _ptr(freqs), _ptr(out))
     ensure_status(lib().rivoli_kv_compress_decode(_ptr(kv_state), _ptr(score_state), C.byref(f), C.byref(p),
-                                                  C.c_int(start_pos), _stream(stream)), "kv_compress_decode")
+                                                  start_pos, _stream(stream)), "kv_compress_decode")
 
 
 def launch_v4_compress_step_bf16(p: CompGeom, n_seqs: int, pos, kv_proj, score_proj, ape, kv_state, score_state, norm,
                                  freqs, rotate: bool, cache, cache_rows: int, cache_row0: int, prequant=None,
                                  packed=None, packed_exp=None, stream=None) -> None:
     ensure_status(lib().rivoli_v4_compress_step_bf16(
-        C.byref(p), C.c_int(n_seqs), _ptr(pos), _ptr(kv_proj), _ptr(score_proj), _ptr(ape), _ptr(kv_state),
-        _ptr(score_state), _ptr(norm), _ptr(freqs), C.c_int(int(rotate)), _ptr(cache), C.c_int(cache_rows),
-        C.c_int(cache_row0), _ptr(prequant), _ptr(packed), _ptr(packed_exp), _stream(stream)), "v4_compress_step_bf16")
+        C.byref(p), n_seqs, _ptr(pos), _ptr(kv_proj), _ptr(score_proj), _ptr(ape), _ptr(kv_state),
+        _ptr(score_state), _ptr(norm), _ptr(freqs), int(rotate), _ptr(cache), cache_rows,
+        cache_row0, _ptr(prequant), _ptr(packed), _ptr(packed_exp), _stream(stream)), "v4_compress_step_bf16")
 
 
 def kernels_arch() -> str:

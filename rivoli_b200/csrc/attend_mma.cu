@@ -35,9 +35,8 @@
 // head: thread = (head, 16 tokens of the tile), two warps per lane quarter take the two 32-token halves. A head's
 // reference maximum, its running sum and its q scale are registers, and P' leaves as one 16-byte store per term
 // (heads are the rows of the K-major P' operand, tokens its bytes).
-// q arrives as bf16 and is split into its two e4m3 terms by the softmax warps inside the kernel while the
-// first tiles are gathered (a thread converts the row of its own TMEM lane and stores it with tcgen05.st); the output
-// leaves straight from the accumulator registers (64 contiguous bytes per warp store).
+// q arrives as bf16 (one bulk copy) and is split into its two e4m3 terms by the softmax warps inside the kernel while the
+// first tiles are gathered; the output leaves through the idle ring as 8 KiB bulk copies.
 // Online softmax with a LAGGING reference max: as long as no score of a tile exceeds its head's
 // reference by more than 3 (log2) the references stand (one barrier-with-OR per tile, no exchange);
 // otherwise the exact per-head maxima are taken and O is rescaled through TMEM. P' carries 2^5, so
@@ -49,6 +48,7 @@
 
 #include "codec.cuh"
 #include "common.cuh"
+#include "quant.cuh"
 #include "tc_common.cuh"
 
 namespace cg = cooperative_groups;
@@ -95,12 +95,14 @@ constexpr int SM_BARS = SM_FAC + 256;    // mbarriers
 constexpr int SM_MISC = SM_BARS + 256;
 constexpr int SM_XS = SM_MISC + 64;      // f32 [2][64]: this CTA's reference maximum and weight sum per head, read by its cluster
 constexpr int SM_TOTAL = SM_XS + 512;
-constexpr int SM_STAGE = SM_K0;          // f32 [64 heads][512 dims]: this CTA's scaled O, read by its cluster (the ring is idle by then)
-static_assert(AM_H * AM_KVL * 4 <= AM_STAGES * SM_KSTAGE, "the O staging fits the ring");
+constexpr int SM_ZQ = SM_K0 + 3 * SM_KSTAGE;   // q as it arrives, then its codes: ring stages 3 .. 5 before their first tile
+static_assert(SM_ZQ + AM_H * AM_W * 2 <= SM_K0 + AM_STAGES * SM_KSTAGE, "q fits the last stages");
+constexpr int SM_STAGE = SM_K0;          // epilogue (the ring is idle by then): bf16 [64 heads][512 dims], or f32 [splits][heads][512 dims] received from the cluster
+static_assert((AM_H + AM_MAX_SPLITS) * AM_KVL * 4 <= AM_STAGES * SM_KSTAGE, "the O staging fits the ring");
 
 struct AmBars {
     uint64_t k_full[AM_STAGES], k_empty[AM_STAGES], s_full[AM_SBUF], s_empty[AM_SBUF], rope_free[AM_ROPES],
-        p_full, pv_done, q_full;
+        p_full, pv_done, q_full, q_raw;
 };
 static_assert(sizeof(AmBars) <= 256, "barrier block");
 static_assert(SM_TOTAL <= 232448, "shared memory budget");
@@ -133,9 +135,9 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo_bytes
     return d;
 }
 
-// Row of the stacked q operand (= TMEM lane of S) that holds term `t` (0 = hi, 1 = lo) of head h: the two terms of a
-// head lie 16 lanes apart inside one warp's lane quarter.
-__device__ __forceinline__ int q_row(int h, int t) { return 32 * (h >> 4) + 16 * t + (h & 15); }
+// Byte offset of 16-byte piece `c` of head h in the staging of q: pieces 0 .. 35 the hi codes, 36 .. 71 the lo codes; the
+// eight pieces of a 128-byte block are permuted by the head, so that the rows of eight heads lie in different banks.
+__device__ __forceinline__ uint32_t zq_chunk(int h, int c) { return (uint32_t)(((h * 72 + c) ^ (h & 7)) << 4); }
 
 // ---------------------------------------------------------------------------------------------
 // main kernel
@@ -165,6 +167,7 @@ attend_mma_kernel(AttendMmaArgs A) {
         tc::mbar_init(&bars.p_full, AM_SOFTMAX_THREADS);
         tc::mbar_init(&bars.pv_done, 1);
         tc::mbar_init(&bars.q_full, AM_SOFTMAX_THREADS);
+        tc::mbar_init(&bars.q_raw, 1);
         tc::mbar_init_fence();
         *abort_flag = 0;
     }
@@ -181,96 +184,108 @@ attend_mma_kernel(AttendMmaArgs A) {
     //   hi = e4m3(q / s), s = absmax / 448;  lo = e4m3(q / s - hi)   =>  q ~ s * (hi + lo)
     // (the residual of a value of typical size is a normal e4m3 number; below 2^-6 it is kept to 2^-10 absolute,
     // 2^-19 of the head's largest value).
-    // A thread fills the row of its OWN tensor-memory lane: lane l of warp w is the virtual head
-    // (16 (w % 4) + l % 16, term l / 16), and w / 4 picks the half of the 512 latent columns (the rope columns go with
-    // half 0). The two lanes of a head (16 apart) share the work: the hi lane reads the even 8-value chunks of the
-    // half-row and the lo lane the odd ones, each derives BOTH terms of its chunks and hands the other lane the codes
-    // that belong in that lane's row (one shuffle per word). Two passes over the chunks: the absolute maximum, then
-    // the codes - 64 values of the row at a time into 16 registers and from there into 16 tensor-memory columns
-    // (column c = codes 4c .. 4c + 3, lowest byte first, which is the layout the MMA expects of an 8-bit A
-    // operand); the rope codes go to the shared operand tile.
-    // The gather warps do not wait for this: the QK issuer does (q_full) before its first MMA.
+    // The sequence's 72 KiB of q arrive as ONE bulk copy in ring stages 3 to 5, which the gather leaves alone until q_full.
+    // A warp converts eight heads, lanes along a head's row, and writes a head's hi row and lo row over the bf16 row it
+    // read (576 + 576 bytes = 1,152); 16-byte pieces are XOR-swizzled by head. Then a thread moves the row of its OWN
+    // tensor-memory lane (lane l of warp w is the virtual head (16 (w % 4) + l % 16, term l / 16), w / 4 the half of the 512
+    // latent columns): 16 conflict-free 16-byte loads, two tcgen05.st; column c = codes 4c .. 4c + 3, lowest byte first,
+    // which is the layout the MMA expects of an 8-bit A operand; the rope codes go to the shared operand tile.
+    // (A thread per row with 16-byte loads of its own row from global memory took 16,400 cycles at batch 148, 11,000 now, of
+    // which the copy is 3,200.)
+    // The QK issuer waits for q_full before its first MMA.
     // Under a programmatic dependent launch the kernel before this one may still be running. Unless the
     // caller vouches that q was complete before that kernel was even launched (q_early: the fused decode
     // step), q may be that kernel's output and is read only after the dependency wait.
     if (!A.q_early) rv_grid_dep_wait();
     if (warp < AM_SW) {
-        const int sq = warp & 3, half = warp >> 2, term = lane >> 4;
-        const int h = 16 * sq + (lane & 15);
-        const uint16_t* qrow = A.q + ((size_t)b * AM_H + h) * AM_W;
-        const uint4* qn = reinterpret_cast<const uint4*>(qrow + half * 256) + term;   // this lane's chunks: qn[2 m], m = 0..15
-        const uint4* qr = reinterpret_cast<const uint4*>(qrow + AM_KVL) + term;        // rope (half 0): qr[2 m], m = 0..3
-        float amax = 0.0f;
-        auto absmax8 = [&](const uint4 v) {
-            const uint32_t ww[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                amax = fmaxf(amax, fmaxf(fabsf(__uint_as_float(ww[i] << 16)), fabsf(__uint_as_float(ww[i] & 0xffff0000u))));
-        };
-        {
-            uint4 v[16];
-#pragma unroll
-            for (int m = 0; m < 16; ++m) v[m] = qn[2 * m];
-#pragma unroll
-            for (int m = 0; m < 16; ++m) absmax8(v[m]);
+        uint8_t* zq = smem + SM_ZQ;
+        if (tid == 0) {
+            tc::mbar_arrive_expect_tx(&bars.q_raw, AM_H * AM_W * 2);
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                         ::"r"(tc::smem_u32(zq)), "l"(A.q + (size_t)b * AM_H * AM_W), "r"(AM_H * AM_W * 2), "r"(tc::smem_u32(&bars.q_raw)) : "memory");
         }
-        if (half == 0) {
-#pragma unroll
-            for (int m = 0; m < 4; ++m) absmax8(qr[2 * m]);
-        }
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 16));
-        if (lane < 16) s_wmax[half * 64 + h] = amax;
-        tc::named_barrier(3, AM_SOFTMAX_THREADS);
-        amax = fmaxf(s_wmax[h], s_wmax[64 + h]);
-        const float sc = amax > 0.0f ? amax / 448.0f : 1.0f;
-        const float inv = 1.0f / sc;
-        // 8 values -> their 8 hi codes and 8 lo codes (two 32-bit words each)
-        auto codes8 = [&](const uint4 v, uint32_t* hi, uint32_t* lo) {
+        tc::mbar_wait_warp(&bars.q_raw, 0, abort_flag, 55, A.max_polls);
+        // 8 values -> their 8 hi codes and 8 lo codes
+        auto codes8 = [&](const uint4 v, float inv, uint2& hi, uint2& lo) {
             const uint32_t ww[4] = {v.x, v.y, v.z, v.w};
-            hi[0] = hi[1] = lo[0] = lo[1] = 0u;
+            uint16_t ch[4], cl[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const float x0 = __uint_as_float(ww[i] << 16) * inv, x1 = __uint_as_float(ww[i] & 0xffff0000u) * inv;
-                uint16_t ch, cl;
-                asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(ch) : "f"(x1), "f"(x0));
-                const float2 xh = rv_e4m3x2_to_f32x2(ch);
-                asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(cl) : "f"(x1 - xh.y), "f"(x0 - xh.x));
-                hi[i >> 1] |= (uint32_t)ch << (16 * (i & 1));
-                lo[i >> 1] |= (uint32_t)cl << (16 * (i & 1));
+                asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(ch[i]) : "f"(x1), "f"(x0));
+                const float2 xh = rv_e4m3x2_to_f32x2(ch[i]);
+                asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(cl[i]) : "f"(x1 - xh.y), "f"(x0 - xh.x));
             }
+            hi = make_uint2((uint32_t)ch[0] | ((uint32_t)ch[1] << 16), (uint32_t)ch[2] | ((uint32_t)ch[3] << 16));
+            lo = make_uint2((uint32_t)cl[0] | ((uint32_t)cl[1] << 16), (uint32_t)cl[2] | ((uint32_t)cl[3] << 16));
         };
-        const uint32_t lane_addr = ((uint32_t)(sq * 32)) << 16;
-#pragma unroll 1
-        for (int grp = 0; grp < 4; ++grp) {       // 8 chunks of the half-row = 64 values = 16 columns per store
-            uint4 v[4];
+        // the warp's eight absolute maxima together: three shuffles halve the eight values to one head per lane, two more
+        // finish it, and the divisions are done once, lane l for head l / 4
+        constexpr int HPW = AM_H / AM_SW;
+        static_assert(HPW == 8, "eight heads per warp");
+        const uint8_t* wq = zq + warp * HPW * (AM_W * 2);
+        float my_inv;
+        {
+            uint32_t m[HPW];
 #pragma unroll
-            for (int m = 0; m < 4; ++m) v[m] = qn[2 * (grp * 4 + m)];
-            uint32_t r[16];
+            for (int i = 0; i < HPW; ++i) {
+                const uint4* src = reinterpret_cast<const uint4*>(wq + i * (AM_W * 2));
+                m[i] = rv_max_bf16x2(rv_absmax8(src[lane]), rv_absmax8(src[32 + lane]));
+                if (lane < 8) m[i] = rv_max_bf16x2(m[i], rv_absmax8(src[64 + lane]));
+            }
 #pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                uint32_t hi[2], lo[2];
-                codes8(v[m], hi, lo);
-                // this lane's own chunk is 2 m + term of the group; the partner made the codes of chunk 2 m + (1 - term)
+            for (int o = 16, n = HPW / 2; n > 0; o >>= 1, n >>= 1)
 #pragma unroll
-                for (int w = 0; w < 2; ++w) {
-                    const uint32_t own = term ? lo[w] : hi[w];
-                    const uint32_t got = __shfl_xor_sync(0xffffffffu, term ? hi[w] : lo[w], 16);
-                    r[4 * m + w] = term ? got : own;          // even chunk: made by the hi lane
-                    r[4 * m + 2 + w] = term ? own : got;      // odd chunk: made by the lo lane
+                for (int i = 0; i < n; ++i) {
+                    const bool up = lane & o;
+                    const uint32_t keep = up ? m[i + n] : m[i], give = up ? m[i] : m[i + n];
+                    m[i] = rv_max_bf16x2(keep, __shfl_xor_sync(0xffffffffu, give, o));
+                }
+            m[0] = rv_max_bf16x2(m[0], __shfl_xor_sync(0xffffffffu, m[0], 2));
+            m[0] = rv_max_bf16x2(m[0], __shfl_xor_sync(0xffffffffu, m[0], 1));
+            const float amax = __uint_as_float(m[0] << 16);
+            const float sc = amax > 0.0f ? amax / 448.0f : 1.0f;
+            my_inv = 1.0f / sc;
+            if ((lane & 3) == 0) s_ahi[warp * HPW + (lane >> 2)] = sc * A.softmax_scale * 1.4426950408889634f;
+        }
+#pragma unroll 2
+        for (int i = 0; i < HPW; ++i) {
+            const int h = warp * HPW + i;
+            const uint4* src = reinterpret_cast<const uint4*>(wq + i * (AM_W * 2));
+            uint4 v[3];
+            v[0] = src[lane]; v[1] = src[32 + lane];
+            v[2] = lane < 8 ? src[64 + lane] : make_uint4(0u, 0u, 0u, 0u);
+            const float inv = __shfl_sync(0xffffffffu, my_inv, 4 * i);
+            __syncwarp();                              // the whole row is in registers
+#pragma unroll
+            for (int u = 0; u < 3; ++u) {              // (lanes 8 .. 31 of the last pass convert zeros and store nothing)
+                uint2 hi, lo;
+                codes8(v[u], inv, hi, lo);
+                const int vc = lane + 32 * u;
+                if (vc < AM_W / 8) {
+                    *reinterpret_cast<uint2*>(zq + zq_chunk(h, vc >> 1) + (vc & 1) * 8) = hi;
+                    *reinterpret_cast<uint2*>(zq + zq_chunk(h, AM_W / 16 + (vc >> 1)) + (vc & 1) * 8) = lo;
                 }
             }
-            tc::tmem_st16(TM_Q + lane_addr + half * 64 + grp * 16, r);
         }
-        if (half == 0) {
-            const int row_hi = q_row(h, 0), row_lo = q_row(h, 1);
+        tc::named_barrier(3, AM_SOFTMAX_THREADS);
+        {
+            const int sq = warp & 3, half = warp >> 2, term = lane >> 4, h = 16 * sq + (lane & 15);
+            const uint32_t dst = TM_Q + (((uint32_t)(sq * 32)) << 16) + half * 64;
 #pragma unroll
-            for (int m = 0; m < 4; ++m) {          // rope chunk 2 m + term: 8 bytes of the 16-byte chunk m of both rows
-                uint32_t hi[2], lo[2];
-                codes8(qr[2 * m], hi, lo);
-                *reinterpret_cast<uint2*>(smem + SM_QR + sw64_chunk(row_hi, m) + 8 * term) = make_uint2(hi[0], hi[1]);
-                *reinterpret_cast<uint2*>(smem + SM_QR + sw64_chunk(row_lo, m) + 8 * term) = make_uint2(lo[0], lo[1]);
+            for (int g = 0; g < 2; ++g) {
+                uint32_t r[32];
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    *reinterpret_cast<uint4*>(r + 4 * i) = *reinterpret_cast<const uint4*>(zq + zq_chunk(h, term * (AM_W / 16) + half * 16 + g * 8 + i));
+                tc::tmem_st32(dst + g * 32, r);
             }
-            if (term == 0) s_ahi[h] = sc * A.softmax_scale * 1.4426950408889634f;
+            if (half == 0) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    *reinterpret_cast<uint4*>(smem + SM_QR + sw64_chunk(sq * 32 + lane, i)) =
+                        *reinterpret_cast<const uint4*>(zq + zq_chunk(h, term * (AM_W / 16) + AM_KVL / 16 + i));
+            }
         }
         tc::tmem_st_wait();
         tc::fence_proxy_async();
@@ -360,6 +375,7 @@ attend_mma_kernel(AttendMmaArgs A) {
         for (int j = g; j < ntiles && ok; j += AM_GW) {
             const int s = j % AM_STAGES, use = j / AM_STAGES;
             ok = tc::mbar_wait_warp(&bars.k_empty[s], (use & 1) ^ 1, abort_flag, 41, A.max_polls);
+            if (ok && j >= 3 && j < AM_STAGES) ok = tc::mbar_wait_warp(&bars.q_full, 0, abort_flag, 43, A.max_polls);   // these stages held q
             if (!ok) break;
             uint8_t* kbuf = smem + SM_K0 + s * SM_KSTAGE;
 #pragma unroll
@@ -638,44 +654,60 @@ attend_mma_kernel(AttendMmaArgs A) {
             s_fac[h] = l > 0.0f ? 1.0f / l : 0.0f;
         }
         tc::named_barrier(1, AM_SOFTMAX_THREADS);
-        // O^T: this thread's TMEM lane is one latent dim of each 128-dim block; its head columns. For a given head
-        // the 32 lanes of a warp hold 32 consecutive dims, so a warp's store covers 64 contiguous bytes of the bf16
-        // output row (two full sectors) and the output goes to global memory straight from the registers (a split
-        // sequence is merged inside its cluster instead, below).
-        float inv_l[AM_HPT];   // 1 / l of this thread's heads (registers: the stores below must not wait on loads)
-#pragma unroll
-        for (int h = 0; h < AM_HPT; h += 4) {
-            const float4 m4 = *reinterpret_cast<const float4*>(s_fac + h0 + h);
-            inv_l[h] = m4.x; inv_l[h + 1] = m4.y; inv_l[h + 2] = m4.z; inv_l[h + 3] = m4.w;
-        }
+        // O^T: this thread's TMEM lane is one latent dim of each 128-dim block; its head columns. Every MMA of the CTA has
+        // read its operands, so the idle ring takes the bf16 output, eight heads of a token half at a time (all 512 dims:
+        // four accumulator blocks), and each group leaves as one 8 KiB bulk copy while the next is converted. (A split
+        // sequence is merged inside its cluster instead, below.)
+        // 2-byte stores from the registers to global memory took 6,700 cycles for the epilogue, 4,400 this way.
+        if (!skip && !clustered) {
+            uint16_t* stage = reinterpret_cast<uint16_t*>(smem + SM_STAGE);
+            const bool have = ntiles > 0 && ok;
 #pragma unroll 1
-        for (int c = 0; c < 4 && !skip && !clustered; ++c) {
-            const int dim = c * 128 + row;
-            uint32_t r[AM_HPT];
-            if (ntiles > 0 && ok) {
-                tc::tmem_ld32(TM_O + lane_base + c * 64 + h0, r);
+            for (int g = 0; g < AM_HPT / 8; ++g) {
+                const int hg = h0 + g * 8;
+                uint32_t r[4][8];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) tc::tmem_ld8(TM_O + lane_base + c * 64 + hg, r[c]);
                 tc::tmem_ld_wait();
-            } else {
+                const float4 i0 = *reinterpret_cast<const float4*>(s_fac + hg), i1 = *reinterpret_cast<const float4*>(s_fac + hg + 4);
+                const float inv_l[8] = {i0.x, i0.y, i0.z, i0.w, i1.x, i1.y, i1.z, i1.w};
+                uint16_t* sp = stage + hg * AM_KVL + row;
 #pragma unroll
-                for (int h = 0; h < AM_HPT; ++h) r[h] = 0u;
+                for (int c = 0; c < 4; ++c)
+#pragma unroll
+                    for (int i = 0; i < 8; i += 2) {
+                        const float x = have ? __uint_as_float(r[c][i]) * inv_l[i] : 0.0f, y = have ? __uint_as_float(r[c][i + 1]) * inv_l[i + 1] : 0.0f;
+                        uint32_t w2;
+                        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w2) : "f"(y), "f"(x));
+                        sp[i * AM_KVL + c * 128] = (uint16_t)w2;
+                        sp[(i + 1) * AM_KVL + c * 128] = (uint16_t)(w2 >> 16);
+                    }
+                tc::fence_proxy_async();
+                tc::named_barrier(4 + th, AM_SOFTMAX_THREADS / 2);
+                if (sq == 0 && lane == 0) {
+                    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+                                 ::"l"(A.out + ((size_t)b * AM_H + hg) * AM_KVL), "r"(tc::smem_u32(stage + hg * AM_KVL)), "r"(8 * AM_KVL * 2) : "memory");
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                }
             }
-            uint16_t* gp = A.out + ((size_t)b * AM_H + h0) * AM_KVL + dim;
-#pragma unroll
-            for (int hq = 0; hq < AM_HPT; ++hq) gp[hq * AM_KVL] = rv_f32_to_bf16(__uint_as_float(r[hq]) * inv_l[hq]);
+            if (sq == 0 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
         }
     }
 
     if (clustered) {
         // ---- merge of a sequence's splits inside its thread-block cluster ----
-        // Every CTA has published its reference maximum and weight sum per head; each scales its own O^T to the
-        // common reference and the total sum and lays it out as f32 [head][dim] in its (now idle) ring; then CTA r adds up
-        // the heads [64 r / n, 64 (r + 1) / n) over all CTAs through distributed shared memory (plain loads of mapped
-        // addresses) and writes them. All threads of all CTAs take part in the three cluster barriers, whatever a
-        // bounded wait did before: a CTA that gave up publishes weight sums of zero.
+        // Every CTA has published its reference maximum and weight sum per head; each scales its own O^T to the common
+        // reference and the total sum and PUSHES it, head by head, into the idle ring of the CTA that writes that head (CTA
+        // r: the heads [64 r / n, 64 (r + 1) / n)), which then adds the n contributions from its own memory. Remote stores
+        // need no answer; reading the other CTAs' staged O instead took a pass more and 6,800 cycles of waiting for 128 KiB.
+        // All threads of all CTAs take part in both cluster barriers, whatever a bounded wait did before: a CTA that gave up
+        // publishes weight sums of zero.
         cg::cluster_group cluster = cg::this_cluster();
         const int n = A.n_splits;
         float* xs = reinterpret_cast<float*>(smem + SM_XS);
-        float* stage = reinterpret_cast<float*>(smem + SM_STAGE);
+        float* recv = reinterpret_cast<float*>(smem + SM_STAGE);             // [n][hpc][512]
+        uint2* s_dst = reinterpret_cast<uint2*>(smem + SM_P);                 // per head: where its row goes (cluster address), its factor
+        const int hpc = (AM_H + n - 1) / n;
         __syncthreads();
         const bool live = ntiles > 0 && *abort_flag == 0;
         cluster.sync();                                                       // [1] every CTA's (m, l)
@@ -685,16 +717,26 @@ attend_mma_kernel(AttendMmaArgs A) {
             const int h0 = th * AM_HPT;
             if (tid < AM_H) {
                 const int h = tid;
-                float mg = -INFINITY;
-                for (int q = 0; q < n; ++q) mg = fmaxf(mg, cluster.map_shared_rank(xs, q)[h]);
-                float L = 0.0f;
-                for (int q = 0; q < n; ++q) {
-                    const float* px = cluster.map_shared_rank(xs, q);
-                    const float lq = px[64 + h];
-                    if (lq > 0.0f) L += lq * exp2f(px[h] - mg);
+                // every remote load of the merge is in flight before the first is used: one at a time (a loop to a run-time
+                // n) each costs a round trip over the cluster, and there are 16 here and 32 below
+                float mq[AM_MAX_SPLITS], lq[AM_MAX_SPLITS], mg = -INFINITY, L = 0.0f;
+#pragma unroll
+                for (int q = 0; q < AM_MAX_SPLITS; ++q) {
+                    const float* px = cluster.map_shared_rank(xs, q < n ? q : 0);
+                    mq[q] = q < n ? px[h] : -INFINITY;
+                    lq[q] = q < n ? px[64 + h] : 0.0f;
                 }
+#pragma unroll
+                for (int q = 0; q < AM_MAX_SPLITS; ++q) mg = fmaxf(mg, mq[q]);
+#pragma unroll
+                for (int q = 0; q < AM_MAX_SPLITS; ++q)
+                    if (lq[q] > 0.0f) L += lq[q] * exp2f(mq[q] - mg);
                 const float lm = xs[64 + h];
-                s_fac[h] = (L > 0.0f && lm > 0.0f) ? exp2f(xs[h] - mg) / L : 0.0f;
+                const float fac = (live && L > 0.0f && lm > 0.0f) ? exp2f(xs[h] - mg) / L : 0.0f;
+                const int owner = ((h + 1) * n - 1) / AM_H;
+                uint32_t to32;
+                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to32) : "r"(tc::smem_u32(recv + (split * hpc + h - owner * AM_H / n) * AM_KVL)), "r"(owner));
+                s_dst[h] = make_uint2(to32, __float_as_uint(fac));
                 if (split == 0 && !skip) {
                     const float m_nat = (mg - AM_POFF) * 0.6931471805599453f;
                     if (A.out_m) A.out_m[(size_t)b * AM_H + h] = L > 0.0f ? m_nat : -INFINITY;
@@ -705,7 +747,7 @@ attend_mma_kernel(AttendMmaArgs A) {
             tc::tc_fence_after();
 #pragma unroll 1
             for (int c = 0; c < 4; ++c) {
-                const int dim = c * 128 + sq * 32 + lane;
+                const uint32_t off = (uint32_t)(c * 128 + sq * 32 + lane) * 4u;
                 uint32_t r[AM_HPT];
                 if (live) {
                     tc::tmem_ld32(TM_O + lane_base + c * 64 + h0, r);
@@ -715,26 +757,29 @@ attend_mma_kernel(AttendMmaArgs A) {
                     for (int h = 0; h < AM_HPT; ++h) r[h] = 0u;
                 }
 #pragma unroll
-                for (int hq = 0; hq < AM_HPT; ++hq)   // lanes = consecutive dims: conflict-free stores
-                    stage[(h0 + hq) * AM_KVL + dim] = live ? __uint_as_float(r[hq]) * s_fac[h0 + hq] : 0.0f;
+                for (int hq = 0; hq < AM_HPT; ++hq) {   // lanes = consecutive dims: 128 bytes per warp store
+                    const uint2 d = s_dst[h0 + hq];
+                    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(d.x + off), "f"(live ? __uint_as_float(r[hq]) * __uint_as_float(d.y) : 0.0f) : "memory");
+                }
             }
         }
-        cluster.sync();                                                       // [2] every CTA's scaled O
+        cluster.sync();                                                       // [2] every CTA's share of this CTA's heads
         if (warp < AM_SW && !skip) {
             const int hb = split * AM_H / n, he = (split + 1) * AM_H / n;
             for (int e = tid; e < (he - hb) * (AM_KVL / 4); e += AM_SOFTMAX_THREADS) {
-                const int h = hb + e / (AM_KVL / 4), d4 = e % (AM_KVL / 4);
+                const int hl = e / (AM_KVL / 4), d4 = e % (AM_KVL / 4);
                 float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                for (int q = 0; q < n; ++q) {
-                    const float4 v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(stage, q) + h * AM_KVL + d4 * 4);
-                    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-                }
+#pragma unroll
+                for (int q = 0; q < AM_MAX_SPLITS; ++q)
+                    if (q < n) {
+                        const float4 v = *reinterpret_cast<const float4*>(recv + (q * hpc + hl) * AM_KVL + d4 * 4);
+                        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+                    }
                 const uint32_t w0 = (uint32_t)rv_f32_to_bf16(acc.x) | ((uint32_t)rv_f32_to_bf16(acc.y) << 16);
                 const uint32_t w1 = (uint32_t)rv_f32_to_bf16(acc.z) | ((uint32_t)rv_f32_to_bf16(acc.w) << 16);
-                *reinterpret_cast<uint2*>(A.out + ((size_t)b * AM_H + h) * AM_KVL + d4 * 4) = make_uint2(w0, w1);
+                *reinterpret_cast<uint2*>(A.out + ((size_t)b * AM_H + hb + hl) * AM_KVL + d4 * 4) = make_uint2(w0, w1);
             }
         }
-        cluster.sync();                                                       // [3] nobody reads this CTA's memory any more
     }
 
     tc::tc_fence_before();

@@ -242,10 +242,18 @@ index_select_cluster_kernel(SelArgs A) {
             // [1] The first exchange is a PULL: a CTA may touch another CTA's shared memory only once that CTA is known
             // to be running, which its arrival at this barrier proves. Every later exchange pushes.
             cluster.sync();
-            for (int q = 0; q < C; ++q) {
-                const SelXc* src = cluster.map_shared_rank(&xc, q);
-                kmin = min(kmin, src->kmin[q]); kmax = max(kmax, src->kmax[q]);
-                sk_max = fmaxf(sk_max, __uint_as_float(src->skmax[q]));
+            // (all remote loads in flight at once: a loop to a run-time count pays a round trip for each)
+            uint32_t kn[SEL_MAX_CLUSTER], kx[SEL_MAX_CLUSTER], sx[SEL_MAX_CLUSTER];
+#pragma unroll
+            for (int q = 0; q < SEL_MAX_CLUSTER; ++q) {
+                const int qq = q < C ? q : 0;
+                const SelXc* src = cluster.map_shared_rank(&xc, qq);
+                kn[q] = src->kmin[qq]; kx[q] = src->kmax[qq]; sx[q] = src->skmax[qq];
+            }
+#pragma unroll
+            for (int q = 0; q < SEL_MAX_CLUSTER; ++q) {
+                kmin = min(kmin, kn[q]); kmax = max(kmax, kx[q]);
+                sk_max = fmaxf(sk_max, __uint_as_float(sx[q]));
             }
         }
     }
@@ -289,8 +297,11 @@ index_select_cluster_kernel(SelArgs A) {
         {
             uint32_t tot = 0u;
             for (int i = tid; i < SL; i += NT) {
-                uint32_t v = 0u;
-                for (int q = 0; q < C; ++q) v += cluster.map_shared_rank(hist, q)[r * SL + i];
+                uint32_t h[SEL_MAX_CLUSTER], v = 0u;
+#pragma unroll
+                for (int q = 0; q < SEL_MAX_CLUSTER; ++q) h[q] = q < C ? cluster.map_shared_rank(hist, q < C ? q : 0)[r * SL + i] : 0u;
+#pragma unroll
+                for (int q = 0; q < SEL_MAX_CLUSTER; ++q) v += h[q];
                 red_hist[i] = v;
                 tot += v;
             }
