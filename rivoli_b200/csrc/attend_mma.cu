@@ -829,8 +829,8 @@ extern "C" size_t rivoli_attend_mma_scratch_bytes(const DsaGeom* g, int B) {
 extern "C" int rivoli_attend_simt_short_rows(const DsaGeom* g, const uint16_t* q, const uint8_t* latent_pool,
                                              const float* latent_scale, const int32_t* block_table,
                                              const uint32_t* rows, int row_stride, const int32_t* n_rows, int B,
-                                             uint16_t* out, float* out_m, float* out_lse, int rows_hi,
-                                             cudaStream_t st);
+                                             uint16_t* out, float* out_m, float* out_lse, int rows_lo,
+                                             int rows_hi, cudaStream_t st);
 
 // Below this many attended rows a sequence is served by the f32 CUDA-core kernel instead: with one tile
 // or less the two-term fp8 operands of the tensor-core kernel (bf16-class, ~2^-9) no longer average out
@@ -854,12 +854,13 @@ extern "C" __attribute__((visibility("default"))) void rivoli_attend_mma_test_ho
 // q_early != 0: the caller guarantees q was complete before the kernel preceding this call in the stream
 // was launched (the fused decode step), so the query conversion may overlap that kernel's tail.
 // min_rows_hint: a lower bound the caller knows for n_rows over the batch (0 = unknown). With a bound of
-// AM_MIN_ROWS or more no sequence needs the CUDA-core arm and its launch is left out.
+// AM_MIN_ROWS or more no sequence needs the CUDA-core arm and its launch is left out. max_rows: an upper bound; below
+// AM_MIN_ROWS no sequence needs this kernel and the CUDA-core arm serves them all, the empty ones too.
 extern "C" int rivoli_attend_mma_paged_bf16(const DsaGeom* g, const uint16_t* q, const uint8_t* latent_pool,
                                             const float* latent_scale, const int32_t* block_table,
                                             const uint32_t* rows, int row_stride, const int32_t* n_rows, int B,
                                             uint16_t* out, float* out_m, float* out_lse, void* scratch,
-                                            int q_early, int min_rows_hint, void* stream) {
+                                            int q_early, int min_rows_hint, long long max_rows, void* stream) {
     if (!scratch) return 1001;
     if (((uintptr_t)latent_pool | (uintptr_t)scratch | (uintptr_t)q | (uintptr_t)out) & 15) return 1005;
     cudaStream_t st = (cudaStream_t)stream;
@@ -872,10 +873,14 @@ extern "C" int rivoli_attend_mma_paged_bf16(const DsaGeom* g, const uint16_t* q,
 
     // short contexts first (a programmatic dependent of whatever precedes this call; its CTAs leave at once
     // for every other sequence), then the tensor-core kernel as a dependent of that launch
+    long long cap = (long long)g->max_pages_per_seq * g->page_tokens;
+    if (rows && row_stride > cap) cap = row_stride;   // (a row list may name a row twice)
+    const bool only_short = (cap < max_rows ? cap : max_rows) < min_rows;
     if (min_rows > 1)
         if (int e = rivoli_attend_simt_short_rows(g, q, latent_pool, latent_scale, block_table, rows, row_stride, n_rows,
-                                                  B, out, out_m, out_lse, min_rows, st))
+                                                  B, out, out_m, out_lse, only_short ? 0 : 1, min_rows, st))
             return e;
+    if (only_short) return 0;
     rv_drain_error();
     AttendMmaArgs a{q, g->softmax_scale, latent_pool, latent_scale, block_table, rows, row_stride, n_rows,
                     g->page_tokens, g->max_pages_per_seq, g->n_pool_pages, n_splits,

@@ -538,15 +538,15 @@ RIVOLI_API int rivoli_attend_simt_paged_bf16(const DsaGeom* g, const uint16_t* q
                                     (cudaStream_t)stream);
 }
 
-// The sequences of a batch with 0 < n_rows < rows_hi on the CUDA-core kernel: the short-context arm of
+// The sequences of a batch with rows_lo <= n_rows < rows_hi on the CUDA-core kernel: the short-context arm of
 // rivoli_mla_attend_paged_bf16, launched in front of the tensor-core kernel as a programmatic dependent of whatever
-// precedes it in the stream.
+// precedes it in the stream. rows_lo = 0: the caller knows that no sequence reaches rows_hi, and none is left out.
 extern "C" int rivoli_attend_simt_short_rows(const DsaGeom* g, const uint16_t* q, const uint8_t* latent_pool,
                                              const float* latent_scale, const int32_t* block_table,
                                              const uint32_t* rows, int row_stride, const int32_t* n_rows, int B,
-                                             uint16_t* out, float* out_m, float* out_lse, int rows_hi,
-                                             cudaStream_t st) {
+                                             uint16_t* out, float* out_m, float* out_lse, int rows_lo,
+                                             int rows_hi, cudaStream_t st) {
     AttPaged pp{q, latent_pool, latent_scale, block_table, rows, row_stride, n_rows, g->page_tokens,
-                g->max_pages_per_seq, g->n_pool_pages, out, out_m, out_lse, 1, rows_hi};
+                g->max_pages_per_seq, g->n_pool_pages, out, out_m, out_lse, rows_lo, rows_lo ? rows_hi : 0x7fffffff};
     return launch_attend_simt<true>(AttSlab{}, pp, ((uintptr_t)q & 7) == 0, g->n_heads, g->kv_lora, g->rope_dim, g->softmax_scale, 0, B, rows_hi, st);
 }

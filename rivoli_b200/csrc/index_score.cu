@@ -209,6 +209,8 @@ index_score_paged_kernel(DsaGeom g, const uint8_t* __restrict__ qcodes, const fl
     float* sks = smem + IS_DCH * IS_TOK + IS_DCH * NHP - IS_TOK;
     static_assert(IS_TOK * CST <= IS_DCH * IS_TOK + IS_DCH * NHP - IS_TOK, "epilogue tiles overlap");
     const int b = blockIdx.y, t0 = blockIdx.x * IS_TOK, tid = threadIdx.x;
+    rv_grid_dep_trigger();
+    rv_grid_dep_wait();
     const int nt = seq_len[b];
     if (t0 >= nt) return;
     const int nh = g.index_heads, hd = g.index_dim;
@@ -315,9 +317,8 @@ RIVOLI_API int rivoli_index_score_paged(const DsaGeom* g, const uint8_t* qcodes,
     cudaStream_t st = (cudaStream_t)stream;
     rv_drain_error();
 #define RV_LAUNCH_IS(HPW)                                                                         \
-    index_score_paged_kernel<HPW><<<grid, 128, 0, st>>>(*g, qcodes, qscales, w, index_pool,       \
-                                                         index_scale, block_table, seq_len, scores, \
-                                                         score_stride)
+    rv_launch_dependent(index_score_paged_kernel<HPW>, grid, dim3(128), 0, st, *g, qcodes, qscales, w, \
+                        index_pool, index_scale, block_table, seq_len, scores, score_stride)
     if (g->index_heads <= 8) RV_LAUNCH_IS(2);
     else if (g->index_heads <= 16) RV_LAUNCH_IS(4);
     else if (g->index_heads <= 32) RV_LAUNCH_IS(8);

@@ -166,6 +166,12 @@ index_select_cluster_kernel(SelArgs A) {
         for (int j = 0; j < EPT; ++j)
             if (j < nvalid) out[i0 + j] = (uint32_t)(i0 + j);
         if (r == 0 && tid == 0 && A.stats) { A.stats[b * 2] = 0; A.stats[b * 2 + 1] = (unsigned)nt; }
+        if constexpr (!VALUES) {                                              // nobody scored these tokens: look at their pages here
+            for (int lp = r * NT + tid; lp * P < nt; lp += C * NT) {
+                const int pg = lp < g.max_pages_per_seq ? A.block_table[(size_t)b * g.max_pages_per_seq + lp] : 0;
+                if (pg < 0 || pg >= g.n_pool_pages) atomicCAS(A.err, 0, 1005);
+            }
+        }
         return;
     }
 
@@ -618,8 +624,10 @@ bool select_cluster_plan(int B, int score_stride, int* cluster, int* ept, int* t
     // A batch that fills the chip by itself (one CTA per SM) takes ONE CTA of 1024 threads per sequence: no exchange
     // between CTAs at all. Smaller batches spread a sequence over a cluster of 2 to 8 CTAs of 512 threads, about two
     // CTAs per SM at most.
+    // Up to 8,192 tokens a lone CTA is faster than a cluster at any batch: what the tokens cost is less than seven cluster
+    // barriers (one sequence: 2,500 tokens 20.5 -> 14.3 us, 4,099 tokens 22.5 -> 18.4 us; 16,384 tokens the other way round).
     int C = 1, NT = 512;
-    if ((long long)B * 4 < 3 * 148)   // from three quarters of the SMs on, one CTA per sequence (measured at batch 128: 161 against 166 us per step with clusters of 2)
+    if ((long long)B * 4 < 3 * 148 && score_stride > 8192)   // from three quarters of the SMs on, one CTA per sequence (measured at batch 128: 161 against 166 us per step with clusters of 2)
         while (C < SEL_MAX_CLUSTER && (long long)B * C * 2 <= 2 * 148) C *= 2;
     if (g_sel_cluster_override > 0) C = g_sel_cluster_override;
     if (C == 1 && (long long)1024 * 16 >= score_stride) NT = 1024;   // 16 keys per thread fit the 64 registers of a 1024-thread CTA

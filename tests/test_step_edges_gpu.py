@@ -1,0 +1,111 @@
+"""The decode step where its launches differ: score rows at most top_k long (nothing to score), batches in which only some
+sequences need a score, no sequence of 128 rows, and the selection's lone CTA at its edges; rows, pools and counts bit for
+bit against the oracle, and the error word of each path."""
+import numpy as np
+import pytest
+import torch
+
+from oracle.workload import State, attend_close_ref, make_geom
+
+pytestmark = pytest.mark.gpu
+
+
+def dev(a):
+    a = np.ascontiguousarray(a)
+    if a.dtype in (np.uint16, np.uint32):
+        a = a.view(np.int16 if a.dtype == np.uint16 else np.int32)
+    return torch.from_numpy(a).cuda()
+
+
+def _layer(st, fill=None):
+    from rivoli_b200 import backend as be
+    from rivoli_b200.layer import DsaDecodeLayer
+    be.lib()
+    g = make_geom(be.DsaGeom, **st.geom_kw)
+    L = DsaDecodeLayer(g, st.B, max_ctx=int(st.seq_len.max()))
+    for name in ("latent_pool", "latent_scale", "index_pool", "index_scale", "block_table"):
+        getattr(L, name).copy_(dev(getattr(st, name)).view(getattr(L, name).shape))
+    return be, g, L
+
+
+def _step(L, st):
+    return L.step(dev(st.new_latent), dev(st.new_key), dev(st.index_q), dev(st.index_w), dev(st.q), dev(st.row_pos), dev(st.seq_len))
+
+
+CASES = {
+    # all selected: below, at and (last) above top_k, with sequences of one row and of a page edge
+    "all-below": dict(ctx_lens=[100, 255, 1, 64, 65], top_k=256),
+    "all-at": dict(ctx_lens=[256, 130, 127, 128], top_k=256),
+    "one-above": dict(ctx_lens=[257, 256, 1, 255], top_k=256),
+    "below-wide-append": dict(ctx_lens=[40, 200], top_k=256, index_dim=512, kv_lora=512, rope_dim=128),
+    "below-other-geometry": dict(ctx_lens=[40, 200, 33], top_k=256, index_dim=64, index_heads=8, kv_lora=256),
+    "above-other-geometry": dict(ctx_lens=[400, 20, 333], top_k=256, index_dim=64, index_heads=8, kv_lora=256),
+    # only the CUDA-core attention is launched
+    "short": dict(ctx_lens=[127, 1, 64], top_k=2048),
+    "short-top-k": dict(ctx_lens=[900, 127, 128], top_k=127),
+    "not-short": dict(ctx_lens=[128, 1, 64], top_k=2048),
+    # the selection's lone CTA and the first cluster
+    "lone-cta": dict(ctx_lens=[8192, 300], top_k=300),
+    "cluster": dict(ctx_lens=[8193, 301], top_k=300),
+}
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_step_matches_the_oracle(name):
+    kw = dict(CASES[name])
+    lens = kw.pop("ctx_lens")
+    st = State(70, len(lens), lens, **kw)
+    be, g, L = _layer(st)
+    out = _step(L, st)
+    be.device_sync(); L.check_status()
+    want = st.oracle_step()
+    n_sel = L.n_sel.cpu().numpy()
+    np.testing.assert_array_equal(n_sel, want["n_sel"])
+    for b in range(st.B):
+        np.testing.assert_array_equal(L.rows[b, :n_sel[b]].cpu().numpy().view(np.uint32), want["rows"][b, :n_sel[b]])
+    for k in ("latent_pool", "latent_scale", "index_pool", "index_scale"):
+        np.testing.assert_array_equal(getattr(L, k).cpu().numpy().ravel().view(np.uint8), want[k].ravel().view(np.uint8))
+    ok, worst, rms = attend_close_ref(out.view(torch.int16).cpu().numpy().view(np.uint16).reshape(want["out_f32"].shape), want["out_f32"])
+    assert ok and rms <= 1e-2, (worst, rms)
+    # the select operator alone takes the same rows
+    rows = L.rows.clone()
+    L.rows.fill_(-1)
+    L.select(dev(st.index_q), dev(st.index_w), dev(st.seq_len))
+    be.device_sync(); L.check_status()
+    for b in range(st.B):
+        assert torch.equal(L.rows[b, :n_sel[b]], rows[b, :n_sel[b]])
+
+
+def test_short_batch_with_an_empty_sequence():
+    st = State(71, 3, [100, 5, 64])
+    be, g, L = _layer(st)
+    seq_len = st.seq_len.copy()
+    seq_len[1] = 0
+    L.append(*[dev(getattr(st, k)[[0, 2]]) for k in ("new_latent", "new_key", "row_pos")], dev(np.array([0, 2], np.int32)))
+    L.select(dev(st.index_q), dev(st.index_w), dev(seq_len))
+    out = L.attend(dev(st.q))
+    be.device_sync(); L.check_status()
+    assert L.n_sel.tolist() == [100, 0, 64]
+    assert not out[1].any() and bool(torch.isneginf(L.out_lse[1]).all())
+    want = st.oracle_step()["out_f32"]
+    ok, worst, rms = attend_close_ref(out.view(torch.int16).cpu().numpy().view(np.uint16).reshape(want.shape)[[0, 2]], want[[0, 2]])
+    assert ok and rms <= 1e-2, (worst, rms)
+
+
+@pytest.mark.parametrize("lens,top_k", [([200, 100], 256), ([400, 100], 256)])
+def test_a_page_outside_the_pool_is_flagged_where_nothing_is_scored(lens, top_k):
+    """Sequence 1 is selected whole: its bad page raises 1005, one past its length does not."""
+    st = State(72, 2, lens, top_k=top_k)
+    be, g, L = _layer(st)
+    x = (dev(st.index_q), dev(st.index_w), dev(st.seq_len))
+    for page, bad in ((1, True), (2, False)):
+        bt = st.block_table.copy()
+        bt[1, page] = g.n_pool_pages + 3
+        L.block_table.copy_(dev(bt))
+        L.select(*x)
+        if bad:
+            with pytest.raises(be.BackendError) as e:
+                be.index_select_status(g, st.B, L.score_stride, L.select_scratch)
+            assert e.value.code == 1005
+        else:
+            be.index_select_status(g, st.B, L.score_stride, L.select_scratch)
