@@ -480,12 +480,15 @@ int rivoli_v4_index_pack_bf16(const V4Geom* g, int n_seqs, const int32_t* row_be
                               void* stream);
 
 /* out[b][head] bf16 = sparse attention of q[b] bf16 [n_heads][head_dim] over kv_cache[b] rows sel[b][0..cols)
- * with the sink in the denominator. n_heads == 64 and head_dim == 512 run on the tensor cores (one CTA per
- * sequence: the gathered rows are staged once in shared memory and shared by all heads); other shapes on
+ * with the sink in the denominator. n_heads == 64 and head_dim == 512 run on the tensor cores (one CTA, or
+ * one cluster of up to eight, per sequence: a gathered row is staged once in shared memory and serves all heads); other shapes on
  * CUDA cores. 1001 bad sizes, 1002 head_dim > 1024, 1006 cols too large for the CUDA-core staging. */
 int rivoli_v4_sparse_attend_bf16(const V4Geom* g, int n_seqs, const uint16_t* q, const uint16_t* kv_cache,
                                  const float* sink, const int32_t* sel, int cols, uint16_t* out, int force_simt,
                                  void* stream);
+/* Synchronises the stream; 1008 if a bounded wait of the tensor-core form gave up since the last call (the output of such
+ * a sequence is NaN). */
+int rivoli_v4_sparse_attend_status(void* stream);
 
 /* ---- V4 KV compressor, decode arm (crates/backend/kernels/kvcompress.hip; struct layouts of
  * crates/backend/src/abi.rs:24-45) -------------------------------------------------------------------- */

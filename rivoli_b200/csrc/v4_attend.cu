@@ -1,7 +1,14 @@
 // V4 cousin of the decode path, part 2: MQA sparse attention over one shared entry per position, gathered by an
 // explicit index list, with a per-head sink in the softmax denominator.
 // Reference behaviour: crates/backend/kernels/attn.hip:358-465.
+#include <cooperative_groups.h>
+
+#include <atomic>
+
+#include "tc_common.cuh"
 #include "v4_common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -88,289 +95,438 @@ __global__ void __launch_bounds__(GA_THREADS) v4_gather_attn_kernel(const T* __r
 }
 
 // ---------------------------------------------------------------------------------------------------
-// sparse attention, tensor cores: 64 heads x 512 dims, one CTA per sequence.
+// sparse attention, 5th-generation tensor cores: 64 heads x 512 dims, bf16 rows as they lie in the cache.
 //
-// The selected rows are gathered ONCE per sequence into shared memory (64-token tiles, two buffers,
-// cp.async) and serve every head twice: as K of S = q K^T and as V of O += P V. 16 warps:
-//   scores   warp (hg, tq, kh): heads 32hg..+31 x tokens 16tq..+15 over half of the 512 dims (16 k-steps of
-//            m16n8k16); the two halves meet in shared memory through one add each (two addends: the sum does
-//            not depend on their order);
-//   softmax  8 threads per head over the tile's 64 tokens, running max / sum in registers;
-//   values   warp (hg, dg): heads 32hg..+31 x dims 64dg..+63, 4 k-steps over the tile's tokens.
-// Two m-tiles per warp halve the operand reloads from shared memory, which is what bounds this kernel.
-// Rows are 1024 B; the 16-byte chunk c of row r sits at chunk (c ^ (r & 7)) so that the eight rows of an
-// 8x8 ldmatrix tile fall in eight different bank groups.
+// A tile is 64 gathered rows (64 KiB: eight 64-dim chunks of [64 rows][128 B], 128-byte swizzle), two tiles in flight; it
+// serves every head twice, as K and as V:
+//   S^T[64 rows x 64 heads]   = K_tile . Q^T            32 MMAs (M = 64, N = 64, K = 16), tile K-major, Q from shared memory
+//   O^T[512 dims x 64 heads] += K_tile^T . P             4 x 4 MMAs (M = 128, N = 64), the same tile read MN-major
+// Rows of S^T are tokens, so a thread of the softmax holds one token's scores: P leaves as 16-byte pieces of a token's 64
+// heads (MN-major B operand), a head's sum stays in the token's registers until the end, and only the reference maximum
+// needs an exchange: it LAGS (one barrier-with-OR per tile) until a score exceeds it by more than SA_LAG (log2), then the
+// exact maxima are taken and O^T is rescaled in tensor memory. Weights are bf16, the sum is the sum of the rounded weights.
+// TMEM (512 columns): O^T 4 x 64, S^T 2 x 64 (M = 64: row i in lane 32 (i / 16) + i % 16).
+// 12 warps: 0-7 softmax + epilogue (lane quarter = warp % 4, head half = warp / 4), 8 QK issue, 9 PV issue, 10 and 11 gather
+// (32 rows of every tile each, cp.async; masked slots are zero rows).
+// One CTA per sequence; a batch that leaves SMs idle gets a thread-block cluster per sequence (tiles split evenly, at most
+// eight CTAs), merged by pushing scaled O^T rows into the memory of the CTA that writes the head.
+// Bound by the rows an SM can take in (18 bytes a clock): 640 rows x 128 sequences 57 us with mma.sync (operand reloads from
+// shared memory), 33.2 us now; 3 sequences 55 us on three SMs, 14.0 us now.
+// All waits are bounded (tc_common.cuh); one that gives up makes the sequence's output NaN and sets g_sa_err.
 // ---------------------------------------------------------------------------------------------------
-constexpr int SA_H = 64, SA_D = 512, SA_TILE = 64, SA_THREADS = 512;
-constexpr int SA_ROW_BYTES = SA_D * 2;
-constexpr int SA_SQ = 0;                                   // [64 heads][1024 B]
-constexpr int SA_SK = SA_SQ + SA_H * SA_ROW_BYTES;         // 2 x [64 tokens][1024 B]
-constexpr int SA_SS = SA_SK + 2 * SA_TILE * SA_ROW_BYTES;  // f32 [64 heads][68]
-constexpr int SA_SS_LD = 68;
-constexpr int SA_SP = SA_SS + SA_H * SA_SS_LD * 4;         // bf16 [64 heads][64 tokens], chunk-swizzled
-constexpr int SA_FAC = SA_SP + SA_H * SA_TILE * 2;         // f32 [64] rescale of the running output
-constexpr int SA_INV = SA_FAC + SA_H * 4;                  // f32 [64] 1 / denominator
-constexpr int SA_IDX = SA_INV + SA_H * 4;                  // i32 [2][64] the tile's slots
-constexpr int SA_SEL = SA_IDX + 2 * SA_TILE * 4;            // i32 [SA_SEL_MAX] the sequence's selection row
-constexpr int SA_SEL_MAX = 2048;
-constexpr int SA_TOTAL = SA_SEL + SA_SEL_MAX * 4;
+constexpr int SA_H = 64, SA_D = 512, SA_TILE = 64;
+constexpr int SA_SW = 8, SA_QKW = 8, SA_PVW = 9, SA_GW0 = 10, SA_GW = 2;
+constexpr int SA_THREADS = (SA_GW0 + SA_GW) * 32, SA_ST = SA_SW * 32;      // threads, softmax threads
+constexpr int SA_MAX_SPLITS = 8;
+constexpr float SA_LAG = 3.0f;
+constexpr int SA_KSTAGE = SA_TILE * SA_D * 2, SA_CHUNK = SA_TILE * 128;
+constexpr int SA_SQ = 2 * SA_KSTAGE;                       // q: [8 chunks][64 heads][128 B]
+constexpr int SA_SP = SA_SQ + SA_H * SA_D * 2;             // P: 2 x [64 tokens][64 heads] bf16
+constexpr int SA_PBUF = SA_TILE * SA_H * 2;
+constexpr int SA_WMAX = SA_SP + 2 * SA_PBUF;               // f32 [4][64] exchange between the lane quarters
+constexpr int SA_REF = SA_WMAX + 4 * SA_H * 4;             // f32 [64] reference maxima
+constexpr int SA_FAC = SA_REF + SA_H * 4;                  // f32 [64] rescale of O^T; 1 / denominator in the epilogue
+constexpr int SA_XS = SA_FAC + SA_H * 4;                   // f32 [2][64] (reference, sum), read by the cluster
+constexpr int SA_DST = SA_XS + 2 * SA_H * 4;               // uint2 [64] where a head's row goes, its factor
+constexpr int SA_BARS = SA_DST + SA_H * 8;
+constexpr int SA_MISC = SA_BARS + 128;
+constexpr int SA_TOTAL = SA_MISC + 16;
+constexpr int SA_TMO = 0, SA_TMS = 256;                    // tensor memory columns
+static_assert(SA_TOTAL <= 232448, "shared memory budget");
+static_assert((SA_H + SA_MAX_SPLITS) * SA_D * 4 <= SA_SP, "the merge buffers fit the tiles and q");
+__device__ int g_sa_err;
 
+struct SaBars { uint64_t k_full[2], k_empty[2], s_full[2], s_empty[2], p_full[2], q_full; };
+static_assert(sizeof(SaBars) <= 128, "barrier block");
 
-__device__ __forceinline__ uint32_t v4_smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void v4_cp_async16(uint32_t dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void v4_ldsm4(uint32_t addr, uint32_t (&r)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void v4_ldsm4_t(uint32_t addr, uint32_t (&r)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
+struct SaArgs {
+    const uint16_t* q; const uint16_t* kv; size_t kv_rows; const float* sink; const int32_t* sel;
+    int cols, n_splits, q_early;      // q_early: q was complete before the preceding kernel was launched
+    float scale_log2; uint16_t* out;
+};
+
 __device__ __forceinline__ float v4_ex2(float x) {   // 2^x, -inf -> 0; relative error 2^-22
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// Two f32 -> packed bf16x2 (lo = a), round to nearest even, and the two rounded values' sum.
-__device__ __forceinline__ uint32_t v4_pack_bf16x2(float a, float b, float& sum) {
-    uint32_t r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
-    sum += __uint_as_float(r << 16) + __uint_as_float(r & 0xffff0000u);
-    return r;
+// bf16 x bf16 -> f32
+__device__ __forceinline__ uint32_t sa_idesc(int M, int N, uint32_t a_mn, uint32_t b_mn) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (a_mn << 15) | (b_mn << 16) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
-__device__ __forceinline__ void v4_mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+__device__ __forceinline__ void sa_mma(uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
+}
+// Sixteen values per lane -> lane i of each half-warp holds the half-warp's maximum (or sum) of value i.
+template <bool SUM>
+__device__ __forceinline__ float sa_fold16(const float (&v)[16], int lane) {
+    float m[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) m[i] = v[i];
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (i < o) {
+                const bool up = lane & o;
+                const float keep = up ? m[i + o] : m[i], got = __shfl_xor_sync(0xffffffffu, up ? m[i] : m[i + o], o);
+                m[i] = SUM ? keep + got : fmaxf(keep, got);
+            }
+    return m[0];
 }
 
-__global__ void __launch_bounds__(SA_THREADS, 1) v4_sparse_attend_mma_kernel(const uint16_t* __restrict__ q,
-                                                                             const uint16_t* __restrict__ kv_cache,
-                                                                             size_t kv_rows,
-                                                                             const float* __restrict__ sink,
-                                                                             const int32_t* __restrict__ sel, int cols,
-                                                                             float scale_log2,
-                                                                             uint16_t* __restrict__ out) {
+__global__ void __launch_bounds__(SA_THREADS, 1) v4_sparse_attend_kernel(SaArgs A) {
     extern __shared__ __align__(1024) unsigned char sa_smem[];
-    const int b = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t sbase = v4_smem_u32(sa_smem);
-    float* sS = reinterpret_cast<float*>(sa_smem + SA_SS);
-    float* sFac = reinterpret_cast<float*>(sa_smem + SA_FAC);
-    float* sInv = reinterpret_cast<float*>(sa_smem + SA_INV);
-    int32_t* sIdx = reinterpret_cast<int32_t*>(sa_smem + SA_IDX);
-    const uint16_t* kvb = kv_cache + (size_t)b * kv_rows * SA_D;
-    const int32_t* ix = sel + (size_t)b * cols;
-    const int n_tiles = (cols + SA_TILE - 1) / SA_TILE;
-    // chunk (row, c) -> byte offset inside a [rows][1024 B] operand
-    auto swz = [](int row, int c) { return row * SA_ROW_BYTES + ((c ^ (row & 7)) << 4); };
+    SaBars& bars = *reinterpret_cast<SaBars*>(sa_smem + SA_BARS);
+    float* s_wmax = reinterpret_cast<float*>(sa_smem + SA_WMAX);
+    float* s_ref = reinterpret_cast<float*>(sa_smem + SA_REF);
+    float* s_fac = reinterpret_cast<float*>(sa_smem + SA_FAC);
+    float* xs = reinterpret_cast<float*>(sa_smem + SA_XS);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sa_smem + SA_MISC);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(sa_smem + SA_MISC + 4);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int b = blockIdx.x / A.n_splits, split = blockIdx.x - b * A.n_splits;
+    const int32_t* ix = A.sel + (size_t)b * A.cols;
+    const int tiles_all = (A.cols + SA_TILE - 1) / SA_TILE, tps = (tiles_all + A.n_splits - 1) / A.n_splits;
+    const int t0 = split * tps, ntiles = max(0, min(tiles_all, t0 + tps) - t0);
 
-    // chunk `it` (0..7) of this thread's share of tile t: one 16-byte piece of one row
-    auto gather_piece = [&](int t, int buf, int it) {
-        const int ch = tid + it * SA_THREADS, row = ch >> 6, c = ch & 63;
-        const int j = t * SA_TILE + row;
-        const int p = j < cols ? ix[j] : -1;
-        if (c == 0) sIdx[buf * SA_TILE + row] = p;
-        const int off = SA_SK + buf * SA_TILE * SA_ROW_BYTES + swz(row, c);
-        if (p >= 0) v4_cp_async16(sbase + off, kvb + (size_t)p * SA_D + c * 8);
-        else *reinterpret_cast<uint4*>(sa_smem + off) = make_uint4(0, 0, 0, 0);   // masked slot: a row of zeros
-    };
+    if (tid == 0) {
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            tc::mbar_init(&bars.k_full[s], SA_GW * 32); tc::mbar_init(&bars.k_empty[s], 1);
+            tc::mbar_init(&bars.s_full[s], 1); tc::mbar_init(&bars.s_empty[s], SA_SW);
+            tc::mbar_init(&bars.p_full[s], SA_ST);
+        }
+        tc::mbar_init(&bars.q_full, SA_ST);
+        tc::mbar_init_fence();
+        *abort_flag = 0;
+    }
+    if (tid < SA_H) s_ref[tid] = -INFINITY;
+    if (warp == SA_QKW) tc::tmem_alloc<512>(tmem_slot);
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    const uint32_t tmem = *tmem_slot, TM_O = tmem + SA_TMO, TM_S = tmem + SA_TMS;
 
-    // Under a programmatic dependent launch the kernel before this one may still be running, and the caller
-    // may have produced q with it: nothing is read before the dependency wait. Then q of this sequence, the
-    // selection row and the first tile.
+    // Under a programmatic dependent launch the kernel before this one may still be running: nothing it may have written is
+    // read before the dependency wait.
+    if (!A.q_early) rv_grid_dep_wait();
+    if (warp < SA_SW) {   // q of this sequence: 64 rows of 64 16-byte pieces, swizzled; the copies signal the barrier
+#pragma unroll
+        for (int it = 0; it < SA_H * SA_D / 8 / SA_ST; ++it) {
+            const int e = it * SA_ST + tid, row = e >> 6, c = e & 63;
+            tc::cp_async16(tc::smem_u32(sa_smem + SA_SQ + (c >> 3) * SA_CHUNK + tc::sw128_chunk(row, c & 7)),
+                           A.q + ((size_t)b * SA_H + row) * SA_D + c * 8);
+        }
+        tc::cp_async_mbar_arrive_noinc(&bars.q_full);
+    }
     rv_grid_dep_wait();
-#pragma unroll
-    for (int it = 0; it < 8; ++it) {
-        const int ch = tid + it * SA_THREADS, row = ch >> 6, c = ch & 63;
-        v4_cp_async16(sbase + SA_SQ + swz(row, c), q + ((size_t)b * SA_H + row) * SA_D + c * 8);
-    }
-    if (cols <= SA_SEL_MAX) {   // read the row once; the per-tile gathers then take their slots from shared memory
-        int32_t* sSel = reinterpret_cast<int32_t*>(sa_smem + SA_SEL);
-        for (int i = tid; i < cols; i += SA_THREADS) sSel[i] = ix[i];
-        ix = sSel;
-        __syncthreads();
-    }
-#pragma unroll
-    for (int it = 0; it < 8; ++it) gather_piece(0, 0, it);
-    asm volatile("cp.async.commit_group;" ::: "memory");
 
-    // softmax state of head (tid >> 3), replicated in its 8 threads
-    float m_run = -INFINITY, l_run = 0.0f;
-    // output accumulators of warp (hg, dg): 2 m-tiles x 8 n-tiles of 8 dims
-    float acc[2][8][4];
+    if (warp >= SA_GW0) {
+        // ---- gather: warp g fills the rows 32 g .. 32 g + 31 of every tile, half a row (512 bytes) per instruction
+        const int g = warp - SA_GW0;
+        const uint16_t* kvb = A.kv + (size_t)b * A.kv_rows * SA_D;
+        auto slot = [&](int t) -> int {      // of row 32 g + lane
+            const int j = (t0 + t) * SA_TILE + 32 * g + lane;
+            return t < ntiles && j < A.cols ? ix[j] : -1;
+        };
+        int next = slot(0);
+        bool ok = true;
+        for (int t = 0; t < ntiles; ++t) {
+            const int s = t & 1, mine = next;
+            next = slot(t + 1);
+            ok = tc::mbar_wait_warp(&bars.k_empty[s], ((t >> 1) & 1) ^ 1, abort_flag, 91);
+            if (!ok) break;
+            uint8_t* tile = sa_smem + s * SA_KSTAGE;
+#pragma unroll 8
+            for (int r = 0; r < 32; ++r) {
+                const int p = __shfl_sync(0xffffffffu, mine, r), row = 32 * g + r;
+                const uint16_t* src = kvb + (size_t)(p >= 0 ? p : 0) * SA_D + lane * 8;
 #pragma unroll
-    for (int m = 0; m < 2; ++m)
-#pragma unroll
-        for (int n = 0; n < 8; ++n) acc[m][n][0] = acc[m][n][1] = acc[m][n][2] = acc[m][n][3] = 0.0f;
-
-    const int hg = warp & 1;                        // heads 32 hg .. +31
-    const int tq = (warp >> 1) & 3, kh = warp >> 3; // scores: token quarter, half of the dims
-    const int dg = warp >> 1;                       // values: dims 64 dg .. +63
-    const int mi = lane >> 3, l7 = lane & 7;
-
-    for (int t = 0; t < n_tiles; ++t) {
-        const int buf = t & 1;
-        if (t + 1 < n_tiles) {
-#pragma unroll
-            for (int it = 0; it < 8; ++it) gather_piece(t + 1, buf ^ 1, it);
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        __syncthreads();
-        const uint32_t sK = sbase + SA_SK + buf * SA_TILE * SA_ROW_BYTES;
-
-        // ---- scores: S[32 heads][16 tokens] over this warp's half of the dims
-        {
-            float sc[2][2][4];
-#pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int n = 0; n < 2; ++n) sc[m][n][0] = sc[m][n][1] = sc[m][n][2] = sc[m][n][3] = 0.0f;
-            const int arow = 32 * hg + ((mi & 1) << 3) + l7;
-            const int brow = 16 * tq + ((mi >> 1) << 3) + l7;
-            const int ks0 = kh * (SA_D / 32);
-            uint32_t a0[2][4], a1[2][4], bb[2][4];
-            v4_ldsm4(sbase + SA_SQ + swz(arow, 2 * ks0 + (mi >> 1)), a0[0]);
-            v4_ldsm4(sbase + SA_SQ + swz(arow + 16, 2 * ks0 + (mi >> 1)), a1[0]);
-            v4_ldsm4(sK + swz(brow, 2 * ks0 + (mi & 1)), bb[0]);
-#pragma unroll
-            for (int i = 0; i < SA_D / 32; ++i) {
-                const int cur = i & 1, nxt = cur ^ 1, ks = ks0 + i + 1;
-                if (i + 1 < SA_D / 32) {
-                    v4_ldsm4(sbase + SA_SQ + swz(arow, 2 * ks + (mi >> 1)), a0[nxt]);
-                    v4_ldsm4(sbase + SA_SQ + swz(arow + 16, 2 * ks + (mi >> 1)), a1[nxt]);
-                    v4_ldsm4(sK + swz(brow, 2 * ks + (mi & 1)), bb[nxt]);
+                for (int h = 0; h < 2; ++h) {
+                    const int c = h * 32 + lane;
+                    tc::cp_async16_zfill(tc::smem_u32(tile + (c >> 3) * SA_CHUNK + tc::sw128_chunk(row, c & 7)), src + h * 256, p >= 0 ? 16u : 0u);
                 }
-                v4_mma_bf16(sc[0][0], a0[cur], bb[cur][0], bb[cur][1]);
-                v4_mma_bf16(sc[0][1], a0[cur], bb[cur][2], bb[cur][3]);
-                v4_mma_bf16(sc[1][0], a1[cur], bb[cur][0], bb[cur][1]);
-                v4_mma_bf16(sc[1][1], a1[cur], bb[cur][2], bb[cur][3]);
             }
-            // the two halves meet in shared memory: the lower half stores, the upper half adds (a + b: no order to pick)
-            if (kh == 1) __syncthreads();
+            tc::cp_async_mbar_arrive_noinc(&bars.k_full[s]);
+        }
+        tc::cp_async_commit();
+        tc::cp_async_wait<0>();              // (an aborted CTA leaves no copy in flight)
+    } else if (warp == SA_QKW) {
+        if (lane == 0 && ntiles > 0) {
+            const uint32_t id = sa_idesc(SA_TILE, SA_H, 0, 0);
+            const uint64_t dq = tc::smem_desc_sw128(tc::smem_u32(sa_smem + SA_SQ), 16, 1024);
+            bool ok = tc::mbar_wait(&bars.q_full, 0, abort_flag, 92);
+            for (int t = 0; t < ntiles && ok; ++t) {
+                const int s = t & 1;
+                ok = tc::mbar_wait(&bars.k_full[s], (t >> 1) & 1, abort_flag, 93) &&
+                     tc::mbar_wait(&bars.s_empty[s], ((t >> 1) & 1) ^ 1, abort_flag, 94);
+                if (!ok) break;
+                tc::fence_proxy_async();     // the copies wrote through the generic proxy, the MMAs read through the async one
+                tc::tc_fence_after();
+                const uint64_t dk = tc::smem_desc_sw128(tc::smem_u32(sa_smem + s * SA_KSTAGE), 16, 1024);
 #pragma unroll
-            for (int m = 0; m < 2; ++m)
+                for (int k = 0; k < SA_D / 16; ++k) {   // four steps of 32 bytes per chunk; address fields count 16-byte units
+                    const uint64_t off = (uint64_t)(((k >> 2) * SA_CHUNK + (k & 3) * 32) >> 4);
+                    sa_mma(TM_S + s * SA_H, dk + off, dq + off, id, k != 0);
+                }
+                tc::mma_commit(&bars.s_full[s]);
+            }
+        }
+    } else if (warp == SA_PVW) {
+        if (lane == 0 && ntiles > 0) {
+            const uint32_t id = sa_idesc(128, SA_H, 1, 1);
+            bool ok = true;
+            for (int t = 0; t < ntiles && ok; ++t) {
+                const int s = t & 1;
+                ok = tc::mbar_wait(&bars.p_full[s], (t >> 1) & 1, abort_flag, 95);
+                if (!ok) break;
+                tc::fence_proxy_async();
+                tc::tc_fence_after();
+                const uint64_t dv = tc::smem_desc_sw128(tc::smem_u32(sa_smem + s * SA_KSTAGE), SA_CHUNK, 1024);
+                const uint64_t dp = tc::smem_desc_sw128(tc::smem_u32(sa_smem + SA_SP + s * SA_PBUF), 16, 1024);
 #pragma unroll
-                for (int n = 0; n < 2; ++n) {
-                    float2* p0 = reinterpret_cast<float2*>(sS + (32 * hg + 16 * m + (lane >> 2)) * SA_SS_LD + 16 * tq + 8 * n + (lane & 3) * 2);
-                    float2* p1 = p0 + 4 * SA_SS_LD;   // 8 rows down
-                    if (kh == 0) {
-                        *p0 = make_float2(sc[m][n][0], sc[m][n][1]);
-                        *p1 = make_float2(sc[m][n][2], sc[m][n][3]);
-                    } else {
-                        const float2 u = *p0, v = *p1;
-                        *p0 = make_float2(u.x + sc[m][n][0], u.y + sc[m][n][1]);
-                        *p1 = make_float2(v.x + sc[m][n][2], v.y + sc[m][n][3]);
+                for (int c = 0; c < 4; ++c)
+#pragma unroll
+                    for (int k = 0; k < SA_TILE / 16; ++k)   // sixteen tokens = two groups of eight rows
+                        sa_mma(TM_O + c * SA_H, dv + (uint64_t)((2 * c * SA_CHUNK + k * 2048) >> 4), dp + (uint64_t)((k * 2048) >> 4), id, (t | k) != 0);
+                tc::mma_commit(&bars.k_empty[s]);
+            }
+        }
+    } else {
+        // ---- softmax. After the exchange below lane l of warp (sq, th) holds token 16 sq + l % 16 of the tile and the
+        // sixteen heads hb .. hb + 15 (the scores of the upper sixteen columns come from the lane sixteen below).
+        const int sq = warp & 3, th = warp >> 2, tok = 16 * sq + (lane & 15), hb = 32 * th + 16 * (lane >> 4);
+        const uint32_t lane_base = ((uint32_t)(sq * 32)) << 16;
+        const bool up = lane >= 16;
+        float l_acc[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) l_acc[j] = 0.0f;
+        auto live_slot = [&](int t) { const int j = (t0 + t) * SA_TILE + tok; return t < ntiles && j < A.cols && ix[j] >= 0; };
+        bool next_live = live_slot(0), ok = ntiles > 0;
+        for (int t = 0; t < ntiles && ok; ++t) {
+            const int s = t & 1;
+            const bool live = next_live;
+            next_live = live_slot(t + 1);
+            ok = tc::mbar_wait_warp(&bars.s_full[s], (t >> 1) & 1, abort_flag, 96);
+            if (!ok) break;
+            tc::tc_fence_after();
+            float s2[16], dmax = -INFINITY;
+            {
+                uint32_t r[32];
+                tc::tmem_ld32(TM_S + s * SA_H + lane_base + 32 * th, r);
+                tc::tmem_ld_wait();
+                tc::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&bars.s_empty[s]);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const uint32_t other = __shfl_sync(0xffffffffu, r[16 + j], lane & 15);
+                    s2[j] = live ? __uint_as_float(up ? other : r[j]) * A.scale_log2 : -INFINITY;
+                }
+            }
+            float ref[16];
+#pragma unroll
+            for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(ref + j) = *reinterpret_cast<const float4*>(s_ref + hb + j);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) dmax = fmaxf(dmax, s2[j] - ref[j]);   // (a masked slot before any reference: NaN, ignored)
+            uint32_t slow;
+            asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\t"
+                         "bar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                         : "=r"(slow) : "r"(dmax > SA_LAG ? 1u : 0u), "n"(SA_ST) : "memory");
+            if (slow) {
+                s_wmax[sq * SA_H + 32 * th + lane] = sa_fold16<false>(s2, lane);
+                tc::named_barrier(2, SA_ST);
+                if (tid < SA_H) {
+                    const float old = s_ref[tid];
+                    const float m = fmaxf(fmaxf(fmaxf(s_wmax[tid], s_wmax[SA_H + tid]), fmaxf(s_wmax[2 * SA_H + tid], s_wmax[3 * SA_H + tid])), old);
+                    s_ref[tid] = m;
+                    s_fac[tid] = m == -INFINITY ? 1.0f : v4_ex2(old - m);
+                }
+                tc::named_barrier(2, SA_ST);
+                if (t > 0) {   // O^T to the new references, once the values of the tile before have landed
+                    ok = tc::mbar_wait_warp(&bars.k_empty[(t - 1) & 1], ((t - 1) >> 1) & 1, abort_flag, 97);
+                    if (!ok) break;
+                    tc::tc_fence_after();
+#pragma unroll 1
+                    for (int c = 0; c < 4; ++c) {
+                        uint32_t r[32];
+                        tc::tmem_ld32(TM_O + c * SA_H + lane_base + 32 * th, r);
+                        tc::tmem_ld_wait();
+#pragma unroll
+                        for (int h = 0; h < 32; ++h) r[h] = __float_as_uint(__uint_as_float(r[h]) * s_fac[32 * th + h]);
+                        tc::tmem_st32(TM_O + c * SA_H + lane_base + 32 * th, r);
                     }
+                    tc::tmem_st_wait();
+                    tc::tc_fence_before();
                 }
-            if (kh == 0) __syncthreads();
-        }
-        __syncthreads();
-
-        // ---- softmax over the tile: head = tid / 8, tokens 8 * (tid % 8) .. +7
-        {
-            const int head = tid >> 3, part = tid & 7;
-            float sv[8];
-            const float4* srow = reinterpret_cast<const float4*>(sS + head * SA_SS_LD + part * 8);
-            const float4 x0 = srow[0], x1 = srow[1];
-            sv[0] = x0.x; sv[1] = x0.y; sv[2] = x0.z; sv[3] = x0.w; sv[4] = x1.x; sv[5] = x1.y; sv[6] = x1.z; sv[7] = x1.w;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) sv[j] *= scale_log2;
-            float tmax = -INFINITY;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                if (sIdx[buf * SA_TILE + part * 8 + j] < 0) sv[j] = -INFINITY;
-                tmax = fmaxf(tmax, sv[j]);
+                for (int j = 0; j < 16; ++j) { ref[j] = s_ref[hb + j]; l_acc[j] *= s_fac[hb + j]; }
             }
-            tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 1));
-            tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 2));
-            tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 4));
-            const float m_new = fmaxf(m_run, tmax);
-            const float fac = m_new == -INFINITY ? 1.0f : v4_ex2(m_run - m_new);
-            const float m_use = m_new == -INFINITY ? 0.0f : m_new;    // every slot masked so far: all p are 2^-inf = 0
-            uint32_t pk[4];
-            float psum = 0.0f;                                         // the sum of what the value product sees
+            uint32_t pk[8];
 #pragma unroll
-            for (int j = 0; j < 8; j += 2) pk[j >> 1] = v4_pack_bf16x2(v4_ex2(sv[j] - m_use), v4_ex2(sv[j + 1] - m_use), psum);
-            psum += __shfl_xor_sync(0xffffffffu, psum, 1);
-            psum += __shfl_xor_sync(0xffffffffu, psum, 2);
-            psum += __shfl_xor_sync(0xffffffffu, psum, 4);
-            l_run = l_run * fac + psum;
-            m_run = m_new;
-            *reinterpret_cast<uint4*>(sa_smem + SA_SP + head * (SA_TILE * 2) + ((part ^ (head & 7)) << 4)) =
-                make_uint4(pk[0], pk[1], pk[2], pk[3]);
-            if (part == 0) sFac[head] = fac;
-        }
-        __syncthreads();
-
-        // ---- values: O[32 heads][64 dims] += P[32 heads][64 tokens] V[64 tokens][64 dims]
-        {
-#pragma unroll
-            for (int m = 0; m < 2; ++m) {
-                const float f0 = sFac[32 * hg + 16 * m + (lane >> 2)], f1 = sFac[32 * hg + 16 * m + (lane >> 2) + 8];
-                if (f0 != 1.0f || f1 != 1.0f) {
-#pragma unroll
-                    for (int n = 0; n < 8; ++n) { acc[m][n][0] *= f0; acc[m][n][1] *= f0; acc[m][n][2] *= f1; acc[m][n][3] *= f1; }
-                }
+            for (int j = 0; j < 16; j += 2) {
+                // (no reference yet: every score so far is -inf and weighs 0)
+                const float p0 = v4_ex2(s2[j] - (ref[j] == -INFINITY ? 0.0f : ref[j])), p1 = v4_ex2(s2[j + 1] - (ref[j + 1] == -INFINITY ? 0.0f : ref[j + 1]));
+                asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(pk[j >> 1]) : "f"(p1), "f"(p0));
+                l_acc[j] += __uint_as_float(pk[j >> 1] << 16);      // the sum of what the value product sees
+                l_acc[j + 1] += __uint_as_float(pk[j >> 1] & 0xffff0000u);
             }
-            const int prow = 32 * hg + ((mi & 1) << 3) + l7;
+            uint8_t* pb = sa_smem + SA_SP + s * SA_PBUF;            // (the values of tile t - 2 are done: its stage was refilled)
+            *reinterpret_cast<uint4*>(pb + tc::sw128_chunk(tok, hb / 8)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            *reinterpret_cast<uint4*>(pb + tc::sw128_chunk(tok, hb / 8 + 1)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+            tc::fence_proxy_async();
+            tc::mbar_arrive(&bars.p_full[s]);
+        }
+        if (ok) ok = tc::mbar_wait_warp(&bars.k_empty[(ntiles - 1) & 1], ((ntiles - 1) >> 1) & 1, abort_flag, 98);
+        tc::tc_fence_after();
+        tc::named_barrier(1, SA_ST);
+        s_wmax[sq * SA_H + 32 * th + lane] = sa_fold16<true>(l_acc, lane);
+        tc::named_barrier(1, SA_ST);
+        if (tid < SA_H) {
+            const float l = (s_wmax[tid] + s_wmax[SA_H + tid]) + (s_wmax[2 * SA_H + tid] + s_wmax[3 * SA_H + tid]), m = s_ref[tid];
+            xs[tid] = m;
+            xs[SA_H + tid] = l;
+            // the sink joins the denominator only, shifted by the same maximum; a query with every slot masked is loud
+            s_fac[tid] = m == -INFINITY ? NAN : 1.0f / (l + v4_ex2(A.sink[tid] * 1.4426950408889634f - m));
+        }
+        tc::named_barrier(1, SA_ST);
+        // O^T: lane = dim of each 128-dim block. The output is staged in the idle tiles, eight heads at a time, and leaves as
+        // 8 KiB bulk copies. (A split sequence is merged in its cluster below.)
+        if (A.n_splits == 1) {
+            uint16_t* stage = reinterpret_cast<uint16_t*>(sa_smem);
+            const bool have = *abort_flag == 0;
+#pragma unroll 1
+            for (int g = 0; g < 4; ++g) {
+                const int hg = 32 * th + g * 8;
+                uint32_t r[4][8];
 #pragma unroll
-            for (int ks = 0; ks < SA_TILE / 16; ++ks) {
-                uint32_t a0[4], a1[4];
-                v4_ldsm4(sbase + SA_SP + prow * (SA_TILE * 2) + (((2 * ks + (mi >> 1)) ^ (prow & 7)) << 4), a0);
-                v4_ldsm4(sbase + SA_SP + (prow + 16) * (SA_TILE * 2) + (((2 * ks + (mi >> 1)) ^ (prow & 7)) << 4), a1);
-                const int vrow = 16 * ks + ((mi & 1) << 3) + l7;
+                for (int c = 0; c < 4; ++c) tc::tmem_ld8(TM_O + lane_base + c * SA_H + hg, r[c]);
+                tc::tmem_ld_wait();
+                uint16_t* sp = stage + hg * SA_D + sq * 32 + lane;
 #pragma unroll
-                for (int np = 0; np < 4; ++np) {
-                    uint32_t bb[4];
-                    v4_ldsm4_t(sK + swz(vrow, 8 * dg + 2 * np + (mi >> 1)), bb);
-                    v4_mma_bf16(acc[0][2 * np], a0, bb[0], bb[1]);
-                    v4_mma_bf16(acc[0][2 * np + 1], a0, bb[2], bb[3]);
-                    v4_mma_bf16(acc[1][2 * np], a1, bb[0], bb[1]);
-                    v4_mma_bf16(acc[1][2 * np + 1], a1, bb[2], bb[3]);
+                for (int c = 0; c < 4; ++c)
+#pragma unroll
+                    for (int i = 0; i < 8; i += 2) {
+                        const float x = have ? __uint_as_float(r[c][i]) * s_fac[hg + i] : NAN, y = have ? __uint_as_float(r[c][i + 1]) * s_fac[hg + i + 1] : NAN;
+                        uint32_t w2;
+                        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w2) : "f"(y), "f"(x));
+                        sp[i * SA_D + c * 128] = (uint16_t)w2;
+                        sp[(i + 1) * SA_D + c * 128] = (uint16_t)(w2 >> 16);
+                    }
+                tc::fence_proxy_async();
+                tc::named_barrier(4 + th, SA_ST / 2);
+                if (sq == 0 && lane == 0) {
+                    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+                                 ::"l"(A.out + ((size_t)b * SA_H + hg) * SA_D), "r"(tc::smem_u32(stage + hg * SA_D)), "r"(8 * SA_D * 2) : "memory");
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 }
             }
+            if (sq == 0 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
         }
-        __syncthreads();
     }
 
-    // the sink joins the denominator only, shifted by the same running max
-    {
-        const int head = tid >> 3;
-        if ((tid & 7) == 0) {
-            const float l = l_run + v4_ex2(sink[head] * 1.4426950408889634f - m_run);
-            sInv[head] = m_run == -INFINITY ? NAN : 1.0f / l;
+    if (A.n_splits > 1) {
+        // ---- merge: every CTA scales its O^T to the common maximum and the whole denominator and pushes it, head by head,
+        // into the CTA that writes the head. Every thread of every CTA takes part in both cluster barriers.
+        cg::cluster_group cluster = cg::this_cluster();
+        const int n = A.n_splits, hpc = (SA_H + n - 1) / n;
+        float* recv = reinterpret_cast<float*>(sa_smem);                          // [n][hpc][512]
+        uint2* s_dst = reinterpret_cast<uint2*>(sa_smem + SA_DST);
+        __syncthreads();
+        const bool aborted = *abort_flag != 0;
+        cluster.sync();
+        if (warp < SA_SW) {
+            if (tid < SA_H) {
+                float mq[SA_MAX_SPLITS], lq[SA_MAX_SPLITS], mg = -INFINITY;
+#pragma unroll
+                for (int q = 0; q < SA_MAX_SPLITS; ++q) {                         // all in flight
+                    const float* px = cluster.map_shared_rank(xs, q < n ? q : 0);
+                    mq[q] = q < n ? px[tid] : -INFINITY;
+                    lq[q] = q < n ? px[SA_H + tid] : 0.0f;
+                }
+#pragma unroll
+                for (int q = 0; q < SA_MAX_SPLITS; ++q) mg = fmaxf(mg, mq[q]);
+                float L = v4_ex2(A.sink[tid] * 1.4426950408889634f - mg);
+#pragma unroll
+                for (int q = 0; q < SA_MAX_SPLITS; ++q)
+                    if (mq[q] > -INFINITY) L += lq[q] * v4_ex2(mq[q] - mg);
+                const float fac = (mg == -INFINITY || aborted) ? NAN : (xs[tid] == -INFINITY ? 0.0f : v4_ex2(xs[tid] - mg) / L);
+                const int owner = ((tid + 1) * n - 1) / SA_H;
+                uint32_t to;
+                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(tc::smem_u32(recv + (split * hpc + tid - owner * SA_H / n) * SA_D)), "r"(owner));
+                s_dst[tid] = make_uint2(to, __float_as_uint(fac));
+            }
+            tc::named_barrier(1, SA_ST);
+            const int sq = warp & 3, th = warp >> 2;
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+                const uint32_t off = (uint32_t)(c * 128 + sq * 32 + lane) * 4u;
+                uint32_t r[32];
+                if (ntiles > 0) {
+                    tc::tmem_ld32(TM_O + c * SA_H + (((uint32_t)(sq * 32)) << 16) + 32 * th, r);
+                    tc::tmem_ld_wait();
+                } else {
+#pragma unroll
+                    for (int h = 0; h < 32; ++h) r[h] = 0u;
+                }
+#pragma unroll
+                for (int h = 0; h < 32; ++h) {
+                    const uint2 d = s_dst[32 * th + h];
+                    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(d.x + off), "f"(__uint_as_float(r[h]) * __uint_as_float(d.y)) : "memory");
+                }
+            }
+        }
+        cluster.sync();
+        if (warp < SA_SW) {
+            const int h0 = split * SA_H / n, h1 = (split + 1) * SA_H / n;
+            for (int e = tid; e < (h1 - h0) * (SA_D / 4); e += SA_ST) {
+                const int hl = e / (SA_D / 4), d4 = e % (SA_D / 4);
+                float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+                for (int q = 0; q < SA_MAX_SPLITS; ++q)
+                    if (q < n) {
+                        const float4 v = *reinterpret_cast<const float4*>(recv + (q * hpc + hl) * SA_D + d4 * 4);
+                        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+                    }
+                uint2 w;
+                asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w.x) : "f"(acc.y), "f"(acc.x));
+                asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w.y) : "f"(acc.w), "f"(acc.z));
+                *reinterpret_cast<uint2*>(A.out + ((size_t)b * SA_H + h0 + hl) * SA_D + d4 * 4) = w;
+            }
         }
     }
+    tc::tc_fence_before();
     __syncthreads();
-    // bf16 output staged in the q region (q is dead after the last score pass), then whole rows go out in
-    // 16-byte pieces
-#pragma unroll
-    for (int m = 0; m < 2; ++m) {
-        const int r0 = 32 * hg + 16 * m + (lane >> 2);
-        const float i0 = sInv[r0], i1 = sInv[r0 + 8];
-#pragma unroll
-        for (int n = 0; n < 8; ++n) {
-            float unused = 0.0f;
-            const int c = 8 * dg + n;                         // 16-byte chunk of the row: dims 8c .. 8c+7
-            const int off = ((lane & 3) << 2);
-            *reinterpret_cast<uint32_t*>(sa_smem + SA_SQ + swz(r0, c) + off) =
-                v4_pack_bf16x2(acc[m][n][0] * i0, acc[m][n][1] * i0, unused);
-            *reinterpret_cast<uint32_t*>(sa_smem + SA_SQ + swz(r0 + 8, c) + off) =
-                v4_pack_bf16x2(acc[m][n][2] * i1, acc[m][n][3] * i1, unused);
+    if (warp == SA_QKW) tc::tmem_dealloc<512>(tmem);
+    if (tid == 0 && *abort_flag) atomicCAS(&g_sa_err, 0, *abort_flag);
+}
+
+// CTAs per sequence: as many as leave all clusters resident at once (at most eight), and no more than there are tiles to
+// share out evenly.
+int sa_splits(int n_seqs, int tiles) {
+    static std::atomic<int> cache[75];       // largest resident cluster size by batch; 0 = not asked yet
+    if (n_seqs > 74) return 1;
+    int most = cache[n_seqs].load(std::memory_order_relaxed);
+    if (!most) {
+        for (most = 148 / n_seqs < SA_MAX_SPLITS ? 148 / n_seqs : SA_MAX_SPLITS; most > 1; --most) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)(most * n_seqs)); cfg.blockDim = dim3(SA_THREADS); cfg.dynamicSmemBytes = SA_TOTAL;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = (unsigned)most; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+            cfg.attrs = at; cfg.numAttrs = 1;
+            int active = 0;
+            if (cudaOccupancyMaxActiveClusters(&active, v4_sparse_attend_kernel, &cfg) == cudaSuccess && active >= n_seqs) break;
+            (void)cudaGetLastError();
         }
+        if (most < 1) most = 1;
+        cache[n_seqs].store(most, std::memory_order_relaxed);
     }
-    __syncthreads();
-#pragma unroll
-    for (int it = 0; it < 8; ++it) {
-        const int ch = tid + it * SA_THREADS, row = ch >> 6, c = ch & 63;
-        *reinterpret_cast<uint4*>(out + ((size_t)b * SA_H + row) * SA_D + c * 8) =
-            *reinterpret_cast<const uint4*>(sa_smem + SA_SQ + swz(row, c));
-    }
+    const int tps = (tiles + most - 1) / most;
+    return (tiles + tps - 1) / tps;
 }
 
 }  // namespace
@@ -389,19 +545,28 @@ RIVOLI_API int rivoli_gather_attn_shared_kv(const float* q, const float* kv, con
     return rv_launch_status();
 }
 
-RIVOLI_API int rivoli_v4_sparse_attend_bf16(const V4Geom* g, int n_seqs, const uint16_t* q, const uint16_t* kv_cache,
-                                            const float* sink, const int32_t* sel, int cols, uint16_t* out,
-                                            int force_simt, void* stream) {
+// q_early: q was complete before the kernel in front of this call was launched.
+int rivoli_v4_sparse_attend_launch(const V4Geom* g, int n_seqs, const uint16_t* q, const uint16_t* kv_cache, const float* sink,
+                                   const int32_t* sel, int cols, uint16_t* out, int force_simt, int q_early, cudaStream_t st) {
     if (int rc = v4_check_geom(g, n_seqs)) return rc;
     if (cols <= 0) return 1001;
     if (g->head_dim > GA_THREADS * GA_ACC) return 1002;
     const size_t kv_rows = (size_t)g->window + (size_t)g->max_comp;
     rv_drain_error();
-    cudaStream_t st = (cudaStream_t)stream;
     if (!force_simt && g->n_heads == SA_H && g->head_dim == SA_D) {
-        cudaFuncSetAttribute(v4_sparse_attend_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SA_TOTAL);
-        rv_launch_dependent(v4_sparse_attend_mma_kernel, dim3((unsigned)n_seqs), dim3(SA_THREADS), (size_t)SA_TOTAL, st, q,
-                            kv_cache, kv_rows, sink, sel, cols, g->softmax_scale * 1.4426950408889634f, out);
+        rv_allow_smem<v4_sparse_attend_kernel>(SA_TOTAL);
+        const int n = sa_splits(n_seqs, (cols + SA_TILE - 1) / SA_TILE);
+        const SaArgs a{q, kv_cache, kv_rows, sink, sel, cols, n, q_early, g->softmax_scale * 1.4426950408889634f, out};
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)n_seqs * (unsigned)n); cfg.blockDim = dim3(SA_THREADS);
+        cfg.dynamicSmemBytes = (size_t)SA_TOTAL; cfg.stream = st;
+        cudaLaunchAttribute at[2];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        at[1].id = cudaLaunchAttributeClusterDimension;
+        at[1].val.clusterDim.x = (unsigned)n; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+        cfg.attrs = at; cfg.numAttrs = n > 1 ? 2 : 1;
+        (void)cudaLaunchKernelEx(&cfg, v4_sparse_attend_kernel, a);
         return rv_launch_status();
     }
     const size_t smem = ((size_t)g->head_dim + (size_t)cols) * sizeof(float);
@@ -411,4 +576,21 @@ RIVOLI_API int rivoli_v4_sparse_attend_bf16(const V4Geom* g, int n_seqs, const u
     v4_gather_attn_kernel<uint16_t><<<dim3((unsigned)g->n_heads, (unsigned)n_seqs), GA_THREADS, smem, st>>>(
         q, kv_cache, kv_rows * (size_t)g->head_dim, sink, sel, g->n_heads, g->head_dim, cols, g->softmax_scale, out);
     return rv_launch_status();
+}
+
+RIVOLI_API int rivoli_v4_sparse_attend_bf16(const V4Geom* g, int n_seqs, const uint16_t* q, const uint16_t* kv_cache,
+                                            const float* sink, const int32_t* sel, int cols, uint16_t* out,
+                                            int force_simt, void* stream) {
+    return rivoli_v4_sparse_attend_launch(g, n_seqs, q, kv_cache, sink, sel, cols, out, force_simt, 0, (cudaStream_t)stream);
+}
+
+// Synchronises the stream; 1008 if a bounded wait of the sparse attention gave up since the last call.
+RIVOLI_API int rivoli_v4_sparse_attend_status(void* stream) {
+    cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);
+    if (e != cudaSuccess) return -(int)e;
+    int h = 0;
+    e = cudaMemcpyFromSymbol(&h, g_sa_err, sizeof(int));
+    if (e != cudaSuccess) return -(int)e;
+    if (h) { const int z = 0; cudaMemcpyToSymbol(g_sa_err, &z, sizeof(int)); }
+    return h ? 1008 : 0;
 }

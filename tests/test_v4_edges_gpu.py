@@ -49,3 +49,37 @@ def test_spread_rows_per_cta(rows, d):
     t = dev(x.copy())
     be.launch_act_quant_f4_rotated(t, rows, d)
     assert np.array_equal(bits(t.cpu().numpy()), bits(want.reshape(rows, d)))
+
+
+@pytest.mark.parametrize("b,cols", [(1, 1), (1, 63), (1, 64), (2, 65), (3, 640), (1, 1100), (9, 257), (74, 130), (75, 130), (150, 64)])
+def test_sparse_attention_tiles_and_clusters(b, cols):
+    """Column counts around the 64-row tile, batches of every cluster size and of more than one wave; masked slots, a wholly
+    masked tile in front, and scores that keep growing (the reference maxima move in every tile)."""
+    from rivoli_b200 import backend as be
+    be.lib()
+    g = be.V4Geom.make(max_comp=1024)
+    gen = torch.Generator("cuda").manual_seed(1000 * b + cols)
+    R = g.window + g.max_comp
+    q = torch.randn((b, 64, 512), generator=gen, device="cuda").to(torch.bfloat16)
+    kv = torch.randn((b, R, 512), generator=gen, device="cuda").to(torch.bfloat16)
+    sink = torch.randn(64, generator=gen, device="cuda")
+    sel = torch.stack([torch.randperm(R, generator=gen, device="cuda")[:cols] for _ in range(b)]).to(torch.int32)
+    growth = torch.arange(cols, device="cuda", dtype=torch.float32) / max(cols, 1) * 4.0
+    for i in range(0, b, 3):                                     # rows that align with head 0's query ever more
+        rows = kv[i, sel[i].long()].float() + growth[:, None] * q[i, 0].float()[None, :]
+        kv[i, sel[i].long()] = rows.to(torch.bfloat16)
+    sel[torch.rand(sel.shape, generator=gen, device="cuda") < 0.2] = -1
+    if cols > 64:
+        sel[0, :64] = -1
+    sel[:, -1] = 7
+    out = torch.empty((b, 64, 512), dtype=torch.bfloat16, device="cuda")
+    be.launch_v4_sparse_attend_bf16(g, b, q.view(torch.int16), kv.view(torch.int16), sink, sel, cols, out.view(torch.int16))
+    be.v4_sparse_attend_status()
+    for i in range(b):
+        k = kv[i, sel[i].clamp(min=0).long()].double()
+        s = (q[i].double() @ k.T) * g.softmax_scale
+        s[:, sel[i] < 0] = -float("inf")
+        s = torch.cat([s, sink.double()[:, None]], 1).softmax(-1)[:, :-1]
+        want = s @ k
+        err = (out[i].double() - want).abs()
+        assert bool((err <= 1e-2 * want.abs() + 1e-2).all()), (i, err.max().item())
