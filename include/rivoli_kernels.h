@@ -541,6 +541,24 @@ int rivoli_v4_compress_step_bf16(const CompGeom* p, int n_seqs, const int32_t* p
                                  const float* norm, const float* freqs, int rotate, uint16_t* cache, int cache_rows,
                                  int cache_row0, float* prequant, unsigned char* packed, uint32_t* packed_exp,
                                  void* stream);
+/* The per-compressor arguments of that call. */
+typedef struct CompStep {
+    const float* kv_proj; const float* score_proj; const float* ape;
+    float* kv_state; float* score_state;
+    const float* norm; const float* freqs;
+    uint16_t* cache; float* prequant; unsigned char* packed; uint32_t* packed_exp;
+    int32_t rotate, cache_rows, cache_row0;
+} CompStep;
+/* One decode token through a layer in one call, in the order of crates/oracles/src/v4oracle/attention.rs:197-232: the
+ * indexer's compressor, the selection rows, kv_entry bf16 [B][head_dim] into ring slot pos % window of attn_step->cache (the
+ * KV cache: cache_rows = window + max_comp), the attention compressor, the sparse attention. Results of
+ * rivoli_v4_compress_step_bf16 (twice), rivoli_v4_select_blocks_bf16 (index_kv = index_step->cache, max_comp rows per
+ * sequence; its packed arrays) and rivoli_v4_sparse_attend_bf16 in sequence. 1000 null structs, 1003 the compressors' widths
+ * or caches are not the geometry's, else the codes of those calls. */
+int rivoli_v4_token_step_bf16(const V4Geom* g, int n_seqs, const int32_t* pos, const uint16_t* kv_entry, const CompGeom* attn,
+                              const CompStep* attn_step, const CompGeom* index, const CompStep* index_step,
+                              const uint16_t* q, const uint16_t* index_q, const float* index_w, const float* sink,
+                              int32_t* sel, void* scratch, uint16_t* out, void* stream);
 
 /* ---- measurement hook ------------------------------------------------------------------------------------------
  * events[0..5): cudaEvent_t handles that the following rivoli_dsa_decode_step_paged / rivoli_dsa_append_select_paged

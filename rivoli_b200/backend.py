@@ -90,7 +90,8 @@ _SIGNATURES = {
     "index_frontend_scratch_bytes": "pi", "index_frontend_bf16": "ppppi" + "p" * 12 + "ip", "index_frontend_status": "p",
     "act_quant_f4_rotated": "piip", "index_score_blocks": "ppppiiiip", "gather_attn_shared_kv": "ppppiiiifpp",
     "v4_select_scratch_bytes": "pi", "v4_select_blocks_bf16": "pi" + "p" * 8 + "ip", "v4_index_pack_bf16": "pippipppp",
-    "v4_sparse_attend_bf16": "pippppipip", "v4_sparse_attend_status": "p", "act_quant_f8_prefix": "ppiiiip", "kv_compress_deposit": "ppppppiip",
+    "v4_sparse_attend_bf16": "pippppipip", "v4_sparse_attend_status": "p",
+    "v4_token_step_bf16": "pi" + "p" * 14, "act_quant_f8_prefix": "ppiiiip", "kv_compress_deposit": "ppppppiip",
     "kv_compress_prefill": "pppppip", "kv_compress_decode": "ppppip",
     "v4_compress_step_bf16": "pi" + "p" * 8 + "ipiipppp",
     "dsa_step_set_timing_events": "p", "attend_mma_test_hook": "iii", "index_select_test_cluster": "i", "kernels_arch": "",
@@ -680,6 +681,29 @@ def launch_kv_compress_decode(kv_state, score_state, norm, freqs, out, p: CompGe
     f = CompFinish(_ptr(norm), _ptr(freqs), _ptr(out))
     ensure_status(lib().rivoli_kv_compress_decode(_ptr(kv_state), _ptr(score_state), C.byref(f), C.byref(p),
                                                   start_pos, _stream(stream)), "kv_compress_decode")
+
+
+class CompStep(C.Structure):
+    """``CompStep`` of include/rivoli_kernels.h: one compressor's arguments of a decode step."""
+    _fields_ = [(n, C.c_void_p) for n in (
+        "kv_proj", "score_proj", "ape", "kv_state", "score_state", "norm", "freqs", "cache", "prequant", "packed",
+        "packed_exp")] + [(n, C.c_int32) for n in ("rotate", "cache_rows", "cache_row0")]
+
+    @classmethod
+    def make(cls, kv_proj, score_proj, ape, kv_state, score_state, norm, freqs, rotate, cache, cache_rows, cache_row0,
+             packed=None, packed_exp=None) -> "CompStep":
+        return cls(_ptr(kv_proj), _ptr(score_proj), _ptr(ape), _ptr(kv_state), _ptr(score_state), _ptr(norm), _ptr(freqs),
+                   _ptr(cache), None, _ptr(packed), _ptr(packed_exp), int(rotate), cache_rows, cache_row0)
+
+
+def launch_v4_token_step_bf16(g: V4Geom, n_seqs: int, pos, kv_entry, attn: CompGeom, attn_step: CompStep,
+                              index: CompGeom, index_step: CompStep, q, index_q, index_w, sink, sel, scratch, out,
+                              stream=None) -> None:
+    """One decode token through a layer (``rivoli_v4_token_step_bf16``)."""
+    ensure_status(lib().rivoli_v4_token_step_bf16(
+        C.byref(g), n_seqs, _ptr(pos), _ptr(kv_entry), C.byref(attn), C.byref(attn_step), C.byref(index),
+        C.byref(index_step), _ptr(q), _ptr(index_q), _ptr(index_w), _ptr(sink), _ptr(sel), _ptr(scratch), _ptr(out),
+        _stream(stream)), "v4_token_step_bf16")
 
 
 def launch_v4_compress_step_bf16(p: CompGeom, n_seqs: int, pos, kv_proj, score_proj, ape, kv_state, score_state, norm,

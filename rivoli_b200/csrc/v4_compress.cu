@@ -51,8 +51,20 @@ __device__ __forceinline__ void cp_act_quant_block(const float* seg, float* out,
     }
 }
 
-// The same for blocks of 64 with 16-byte accesses: a thread holds four values, sixteen neighbours a block. The scale is a
-// power of two, so the quotient is the exact product with its reciprocal (2^-e is a normal number: e >= -22). Bound by
+// The scale of a block (a power of two) and its reciprocal (2^-e is a normal number: e >= -22), by which a quotient is exact.
+__device__ __forceinline__ float cp_f8_scale(float amax, float& inv) {
+    const uint32_t bits = __float_as_uint(__fmul_rn(amax, __fdiv_rn(1.0f, CP_FP8_MAX)));
+    const int e = (int)((bits >> 23) & 0xffu) - 127 + ((bits & 0x7fffffu) ? 1 : 0);
+    inv = __uint_as_float((uint32_t)(127 - e) << 23);
+    return __uint_as_float((uint32_t)(e + 127) << 23);
+}
+__device__ __forceinline__ float cp_f8_roundtrip(float x, float s, float inv) {
+    float q = __fmul_rn(x, inv);
+    q = q < -CP_FP8_MAX ? -CP_FP8_MAX : (q > CP_FP8_MAX ? CP_FP8_MAX : q);
+    return __fmul_rn(cp_e4m3_roundtrip(q), s);
+}
+
+// The same for blocks of 64 with 16-byte accesses: a thread holds four values, sixteen neighbours a block. Bound by
 // memory (read once, written once); 4,095 rows of 448: 10.3 us with one warp per block and two values per lane, 5.2 us now.
 __global__ void __launch_bounds__(256)
 cp_act_quant_f8_prefix64_kernel(const float* src, float* dst, int rows, int row_stride, int n) {
@@ -66,14 +78,9 @@ cp_act_quant_f8_prefix64_kernel(const float* src, float* dst, int rows, int row_
     float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    const uint32_t bits = __float_as_uint(__fmul_rn(fmaxf(amax, 1e-4f), __fdiv_rn(1.0f, CP_FP8_MAX)));
-    const int e = (int)((bits >> 23) & 0xffu) - 127 + ((bits & 0x7fffffu) ? 1 : 0);
-    const float s = __uint_as_float((uint32_t)(e + 127) << 23), inv = __uint_as_float((uint32_t)(127 - e) << 23);
-    auto one = [&](float x) {
-        float q = __fmul_rn(x, inv);
-        q = q < -CP_FP8_MAX ? -CP_FP8_MAX : (q > CP_FP8_MAX ? CP_FP8_MAX : q);
-        return __fmul_rn(cp_e4m3_roundtrip(q), s);
-    };
+    float inv;
+    const float s = cp_f8_scale(fmaxf(amax, 1e-4f), inv);
+    auto one = [&](float x) { return cp_f8_roundtrip(x, s, inv); };
     if (live) *reinterpret_cast<float4*>(dst + row * row_stride + c) = make_float4(one(v.x), one(v.y), one(v.z), one(v.w));
 }
 
@@ -379,6 +386,197 @@ __global__ void __launch_bounds__(CP_THREADS) cp_step_kernel(CompGeom p, const i
     }
 }
 
+// The same for the overlapping ratio-4 compressor with d = 128, 256 or 512 (what both compressors of a layer are), one or two
+// compressors and the ring write of a decode token in ONE launch: 512 / d sequences per CTA, a thread owns two features of
+// one sequence, so deposit, pooling and the move of the overlap half need no exchange - a closing block's loads (10 rows'
+// worth, the token's own row comes from the projections) are all in flight at once. Values and their order are those of the
+// kernel above, the norm's partial sums included (they meet in shared memory in the order of a 256-thread CTA). Bound by
+// latency: two dependent trips to memory; 128 sequences of d 512 14.4 -> 6.9 us (d 128: 10.3 -> 5.8).
+struct CpStepJob {
+    const float* kv_proj; const float* score_proj; const float* ape; float* kv_state; float* score_state;
+    const float* norm; const float* freqs; uint16_t* cache; float* prequant; uint8_t* packed; uint32_t* packed_exp;
+    float eps; int d, rd, rotate, cache_rows, cache_row0;
+    int cta_end;              // the job's CTAs end here
+};
+struct CpStepArgs {
+    CpStepJob job[2]; const int32_t* pos; int n_jobs, n_seqs;
+    const uint16_t* entry; uint16_t* ring; size_t ring_rows; int window, ring_d;   // ring write: behind the jobs' CTAs
+};
+
+template <int D>
+__device__ __forceinline__ void cp_step4(const CpStepJob& J, const int32_t* __restrict__ pos, int cta, int n_seqs, float* s_row, float* s_red) {
+    constexpr int WPS = D / 64, SEQS = 8 / WPS, CD = 2 * D, NV = D == 512 ? 1 : 2;   // warps per sequence, sequences per CTA
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, grp = warp / WPS, w = warp - grp * WPS;
+    const int b = cta * SEQS + grp, e = (w * 32 + lane) * 2;
+    const bool mine = b < n_seqs;
+    const int sp = mine ? pos[b] : 0, slot = sp & 3;
+    const bool closing = mine && slot == 3;
+    float* kv = J.kv_state + (size_t)(mine ? b : 0) * 8 * CD;
+    float* sc = J.score_state + (size_t)(mine ? b : 0) * 8 * CD;
+    auto ld = [](const float* p) { return *reinterpret_cast<const float2*>(p); };
+    auto st = [](float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; };
+    float2 dk[2], ds[2];      // the token's row, both halves
+    float2 x[8], k[8], x0[3], k0[3];
+    if (mine) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            dk[h] = ld(J.kv_proj + (size_t)b * CD + h * D + e);
+            const float2 s = ld(J.score_proj + (size_t)b * CD + h * D + e), a = ld(J.ape + (size_t)slot * CD + h * D + e);
+            ds[h] = make_float2(s.x + a.x, s.y + a.y);
+        }
+    }
+    if (closing) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { x[j] = ld(sc + j * CD + e); k[j] = ld(kv + j * CD + e); }
+#pragma unroll
+        for (int j = 4; j < 7; ++j) { x[j] = ld(sc + j * CD + D + e); k[j] = ld(kv + j * CD + D + e); x0[j - 4] = ld(sc + j * CD + e); k0[j - 4] = ld(kv + j * CD + e); }
+    }
+    if (mine) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) { st(kv + (4 + slot) * CD + h * D + e, dk[h]); st(sc + (4 + slot) * CD + h * D + e, ds[h]); }
+    }
+    float row[2] = {0.0f, 0.0f};
+    float* my = s_row + grp * D;
+    if (closing) {
+        x[7] = ds[1]; k[7] = dk[1];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {   // the overlap half moves down
+            st(sc + j * CD + e, j < 3 ? x0[j] : ds[0]); st(kv + j * CD + e, j < 3 ? k0[j] : dk[0]);
+            st(sc + j * CD + D + e, x[4 + j]); st(kv + j * CD + D + e, k[4 + j]);
+        }
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            float v[8], mx = -INFINITY, o = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) { v[j] = c ? x[j].y : x[j].x; mx = fmaxf(mx, v[j]); }
+            if (isfinite(mx)) {
+                float sum = 0.0f;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) { v[j] = expf(v[j] - mx); sum += v[j]; }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) o += (c ? k[j].y : k[j].x) * (v[j] / sum);
+            }
+            row[c] = v4_rbf16(o);
+        }
+        st(my + e, make_float2(row[0], row[1]));
+    }
+    __syncthreads();
+    if (closing) {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const int t = (v * WPS + w) * 32 + lane;
+            float part = 0.0f;
+            part += my[t] * my[t];
+            if (D == 512) part += my[t + 256] * my[t + 256];
+            part = rv_warp_sum(part);
+            if (lane == 0) s_red[grp * 8 + v * WPS + w] = part;
+        }
+    }
+    __syncthreads();
+    if (closing) {
+        float t = 0.0f;
+#pragma unroll
+        for (int i = 0; i < NV * WPS; ++i) t += s_red[grp * 8 + i];
+        const float rs = 1.0f / sqrtf(t / (float)D + J.eps);
+        const float2 gain = ld(J.norm + e);
+        row[0] = v4_rbf16(gain.x * (row[0] * rs));
+        row[1] = v4_rbf16(gain.y * (row[1] * rs));
+        const int r0 = e - (D - J.rd);
+        if (r0 >= 0) {
+            const float c = J.freqs[(size_t)(sp - 3) * J.rd + r0], sn = J.freqs[(size_t)(sp - 3) * J.rd + r0 + 1];
+            const float a = row[0], z = row[1];
+            row[0] = v4_rbf16(__fsub_rn(__fmul_rn(a, c), __fmul_rn(z, sn)));
+            row[1] = v4_rbf16(__fadd_rn(__fmul_rn(a, sn), __fmul_rn(z, c)));
+        }
+        if (J.prequant) st(J.prequant + (size_t)b * D + e, make_float2(row[0], row[1]));
+    }
+    const size_t orow = (size_t)(mine ? b : 0) * J.cache_rows + J.cache_row0 + (sp >> 2);
+    if (!J.rotate) {
+        if (closing) {
+            if (w * 64 < D - J.rd) {   // fp8 block-64 on the dims that were not rotated: a block is a warp
+                const float amax = fmaxf(1e-4f, rv_warp_max(fmaxf(fabsf(row[0]), fabsf(row[1]))));
+                float inv;
+                const float s = cp_f8_scale(amax, inv);
+                row[0] = cp_f8_roundtrip(row[0], s, inv);
+                row[1] = cp_f8_roundtrip(row[1], s, inv);
+            }
+            *reinterpret_cast<uint32_t*>(J.cache + orow * D + e) = (uint32_t)rv_f32_to_bf16(row[0]) | ((uint32_t)rv_f32_to_bf16(row[1]) << 16);
+        }
+        return;
+    }
+    if constexpr (D <= V4_ROT_MAX) {
+        if (closing) st(my + e, make_float2(row[0], row[1]));
+        __syncthreads();
+        if (!closing || w != 0) return;
+        constexpr int E = D / 32;
+        float v[E];
+#pragma unroll
+        for (int j = 0; j < E; ++j) v[j] = my[lane * E + j];
+        v4_spread_row<E>(v, lane);
+        uint32_t o[E / 2];
+#pragma unroll
+        for (int j = 0; j < E; j += 2) o[j / 2] = (uint32_t)rv_f32_to_bf16(v[j]) | ((uint32_t)rv_f32_to_bf16(v[j + 1]) << 16);
+#pragma unroll
+        for (int j = 0; j < E / 2; ++j) reinterpret_cast<uint32_t*>(J.cache + orow * D + lane * E)[j] = o[j];
+        if constexpr (D == 128) if (J.packed) {
+            // the scorer's second form of the same row: int8 multiples of the row's unit 2^(pmin - 130), pmin = the smallest
+            // biased exponent any non-empty block's largest magnitude has; the row's word holds pmin, 0 for an all-zero
+            // row, 0xff when the row is not of that form (blocks more than 3 binades apart, magnitudes outside 2^-40 .. 2^40)
+            int pb = 0;
+#pragma unroll
+            for (int j = 0; j < E; ++j) { v[j] = rv_bf16_to_f32(rv_f32_to_bf16(v[j])); pb = max(pb, (int)((__float_as_uint(v[j]) >> 23) & 0xffu)); }
+#pragma unroll
+            for (int q = 1; q < 8; q <<= 1) pb = max(pb, __shfl_xor_sync(0xffffffffu, pb, q));
+            int lo = pb > 0 ? pb : 1000, hi = pb > 0 ? pb : -1000;
+#pragma unroll
+            for (int q = 8; q < 32; q <<= 1) { lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, q)); hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, q)); }
+            const bool form = hi < lo || (lo >= 87 && hi <= 167 && hi - lo <= 3);
+            bool ok = form;
+            uint32_t bytes = 0;
+#pragma unroll
+            for (int j = 0; j < E; ++j) {
+                const float xq = (form && hi >= lo) ? v[j] * __int_as_float((257 - lo) << 23) : 0.0f;
+                const int m = __float2int_rn(xq);
+                ok = ok && (float)m == xq && (hi >= lo || (__float_as_uint(v[j]) & 0x7fffffffu) == 0);
+                bytes |= (uint32_t)(m & 0xff) << (8 * j);
+            }
+            ok = __all_sync(0xffffffffu, ok);
+            reinterpret_cast<uint32_t*>(J.packed + orow * 128)[lane] = bytes;
+            if (lane == 0) J.packed_exp[orow] = ok ? (hi >= lo ? (uint32_t)lo : 0u) : 0xffu;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(CP_THREADS) cp_step4_kernel(CpStepArgs A) {
+    __shared__ __align__(16) float s_row[512];
+    __shared__ float s_red[64];
+    // the wait comes first: whatever is launched behind this kernel then starts after everything in front of it is complete
+    rv_grid_dep_wait();
+    rv_grid_dep_trigger();
+    int cta = (int)blockIdx.x, first = 0;
+    for (int j = 0; j < A.n_jobs; ++j) {
+        const CpStepJob& J = A.job[j];
+        if (cta < J.cta_end) {
+            if (J.d == 512) cp_step4<512>(J, A.pos, cta - first, A.n_seqs, s_row, s_red);
+            else if (J.d == 256) cp_step4<256>(J, A.pos, cta - first, A.n_seqs, s_row, s_red);
+            else cp_step4<128>(J, A.pos, cta - first, A.n_seqs, s_row, s_red);
+            return;
+        }
+        first = J.cta_end;
+    }
+    // the token's window entry into ring slot pos % window: a warp per sequence
+    const int b = (cta - first) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (b >= A.n_seqs) return;
+    const int r = A.pos[b] % A.window, slot = r < 0 ? r + A.window : r;
+    const uint16_t* src = A.entry + (size_t)b * A.ring_d;
+    uint16_t* dst = A.ring + ((size_t)b * A.ring_rows + slot) * A.ring_d;
+    if (A.ring_d % 8 == 0 && (((uintptr_t)A.entry | (uintptr_t)A.ring) & 15) == 0) {
+        for (int i = lane; i < A.ring_d / 8; i += 32) reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
+    } else {
+        for (int i = lane; i < A.ring_d; i += 32) dst[i] = src[i];
+    }
+}
+
 static int cp_guard(const CompGeom& p) {
     if (p.ratio <= 1 || p.d <= 0 || p.rd <= 0 || p.coff < 1 || p.coff > 2) return 1001;
     if (p.rd > p.d || (p.rd & 1)) return 1002;
@@ -456,6 +654,44 @@ RIVOLI_API int rivoli_kv_compress_decode(float* kv_state, float* score_state, co
     return rv_launch_status();
 }
 
+static int cp_step_guard(const CompGeom& p, int rotate, int cache_rows, int cache_row0, const void* packed, const void* packed_exp) {
+    if (int g = cp_guard(p)) return g;
+    if (cache_rows <= 0 || cache_row0 < 0) return 1001;
+    if (rotate && (p.d > V4_ROT_MAX || (p.d & (p.d - 1)) || p.d % 32)) return 1002;
+    if (!rotate && (p.d - p.rd) % 64) return 1004;
+    if ((packed != nullptr) != (packed_exp != nullptr)) return 1001;
+    if (packed && (!rotate || p.d != 128)) return 1002;   // the packed form is the indexer's: spread rows of width 128
+    if ((size_t)p.d * 4 > 48 * 1024) return 1002;
+    return 0;
+}
+
+// The step takes the two-features-per-thread kernel (else: one CTA per sequence, any geometry).
+static bool cp_step4_ok(const CompGeom& p, const CompStep& c, int rotate) {
+    return p.ratio == 4 && (p.d == 128 || p.d == 256 || (p.d == 512 && !rotate)) &&
+           (((uintptr_t)c.kv_proj | (uintptr_t)c.score_proj | (uintptr_t)c.ape | (uintptr_t)c.kv_state | (uintptr_t)c.score_state |
+             (uintptr_t)c.norm | (uintptr_t)c.prequant) & 7) == 0 && (((uintptr_t)c.cache | (uintptr_t)c.packed) & 3) == 0;
+}
+
+static CpStepJob cp_step4_job(const CompGeom& p, const CompStep& c, int n_seqs, int first_cta) {
+    const int seqs = 512 / p.d;
+    return CpStepJob{c.kv_proj, c.score_proj, c.ape, c.kv_state, c.score_state, c.norm, c.freqs, c.cache, c.prequant, c.packed,
+                     c.packed_exp, p.eps, p.d, p.rd, c.rotate, c.cache_rows, c.cache_row0, first_cta + (n_seqs + seqs - 1) / seqs};
+}
+
+static int cp_step_launch(const CompGeom& p, int n_seqs, const int32_t* pos, const CompStep& c, cudaStream_t st) {
+    if (cp_step4_ok(p, c, c.rotate)) {
+        CpStepArgs a{};
+        a.job[0] = cp_step4_job(p, c, n_seqs, 0);
+        a.pos = pos; a.n_jobs = 1; a.n_seqs = n_seqs;
+        rv_launch_dependent(cp_step4_kernel, dim3((unsigned)a.job[0].cta_end), dim3(CP_THREADS), 0, st, a);
+    } else {
+        cp_step_kernel<<<(unsigned)n_seqs, CP_THREADS, (size_t)p.d * 4, st>>>(
+            p, pos, c.kv_proj, c.score_proj, c.ape, c.kv_state, c.score_state, c.norm, c.freqs, c.rotate, c.cache, c.cache_rows,
+            c.cache_row0, c.prequant, c.packed, c.packed_exp);
+    }
+    return rv_launch_status();
+}
+
 RIVOLI_API int rivoli_v4_compress_step_bf16(const CompGeom* pp, int n_seqs, const int32_t* pos, const float* kv_proj,
                                             const float* score_proj, const float* ape, float* kv_state,
                                             float* score_state, const float* norm, const float* freqs, int rotate,
@@ -464,15 +700,50 @@ RIVOLI_API int rivoli_v4_compress_step_bf16(const CompGeom* pp, int n_seqs, cons
     if (!pp) return 1000;
     const CompGeom p = *pp;
     if (int g = cp_guard(p)) return g;
-    if (n_seqs <= 0 || cache_rows <= 0 || cache_row0 < 0) return 1001;
-    if (rotate && (p.d > V4_ROT_MAX || (p.d & (p.d - 1)) || p.d % 32)) return 1002;
-    if (!rotate && (p.d - p.rd) % 64) return 1004;
-    if ((packed != nullptr) != (packed_exp != nullptr)) return 1001;
-    if (packed && (!rotate || p.d != 128)) return 1002;   // the packed form is the indexer's: spread rows of width 128
-    if ((size_t)p.d * 4 > 48 * 1024) return 1002;
+    if (n_seqs <= 0) return 1001;
+    if (int g = cp_step_guard(p, rotate, cache_rows, cache_row0, packed, packed_exp)) return g;
     rv_drain_error();
-    cp_step_kernel<<<(unsigned)n_seqs, CP_THREADS, (size_t)p.d * 4, (cudaStream_t)stream>>>(
-        p, pos, kv_proj, score_proj, ape, kv_state, score_state, norm, freqs, rotate, cache, cache_rows, cache_row0, prequant,
-        packed, packed_exp);
-    return rv_launch_status();
+    return cp_step_launch(p, n_seqs, pos, CompStep{kv_proj, score_proj, ape, kv_state, score_state, norm, freqs, cache, prequant,
+                                                   packed, packed_exp, rotate, cache_rows, cache_row0}, (cudaStream_t)stream);
+}
+
+int rivoli_v4_sparse_attend_launch(const V4Geom* g, int n_seqs, const uint16_t* q, const uint16_t* kv_cache, const float* sink,
+                                   const int32_t* sel, int cols, uint16_t* out, int force_simt, int q_early, cudaStream_t st);
+
+RIVOLI_API int rivoli_v4_token_step_bf16(const V4Geom* g, int n_seqs, const int32_t* pos, const uint16_t* kv_entry,
+                                         const CompGeom* attn, const CompStep* attn_step, const CompGeom* index,
+                                         const CompStep* index_step, const uint16_t* q, const uint16_t* index_q,
+                                         const float* index_w, const float* sink, int32_t* sel, void* scratch, uint16_t* out,
+                                         void* stream) {
+    if (!attn || !index || !attn_step || !index_step) return 1000;
+    if (int rc = v4_check_geom(g, n_seqs)) return rc;
+    if (!pos || !kv_entry) return 1001;
+    for (int j = 0; j < 2; ++j) {
+        const CompStep& c = j ? *attn_step : *index_step;
+        if (int e = cp_step_guard(j ? *attn : *index, c.rotate, c.cache_rows, c.cache_row0, c.packed, c.packed_exp)) return e;
+    }
+    if (index->d != g->index_dim || index_step->cache_rows != g->max_comp || index_step->cache_row0 != 0) return 1003;
+    if (attn->d != g->head_dim || attn_step->cache_rows != g->window + g->max_comp || attn_step->cache_row0 < g->window) return 1003;
+    cudaStream_t st = (cudaStream_t)stream;
+    rv_drain_error();
+    CpStepArgs a{};
+    a.pos = pos; a.n_seqs = n_seqs;
+    a.entry = kv_entry; a.ring = attn_step->cache; a.ring_rows = (size_t)attn_step->cache_rows; a.window = g->window; a.ring_d = g->head_dim;
+    int ctas = 0;
+    for (int j = 0; j < 2; ++j) {   // what the joint launch does not take goes in front of it, on its own
+        const CompGeom& p = j ? *attn : *index;
+        const CompStep& c = j ? *attn_step : *index_step;
+        if (!cp_step4_ok(p, c, c.rotate)) {
+            if (int e = cp_step_launch(p, n_seqs, pos, c, st)) return e;
+        } else {
+            a.job[a.n_jobs] = cp_step4_job(p, c, n_seqs, ctas);
+            ctas = a.job[a.n_jobs++].cta_end;
+        }
+    }
+    rv_launch_dependent(cp_step4_kernel, dim3((unsigned)(ctas + (n_seqs + 7) / 8)), dim3(CP_THREADS), 0, st, a);
+    if (int e = rv_launch_status()) return e;
+    if (int e = rivoli_v4_select_blocks_bf16(g, n_seqs, pos, index_q, index_w, index_step->cache, index_step->packed,
+                                             index_step->packed_exp, sel, scratch, 0, stream))
+        return e;
+    return rivoli_v4_sparse_attend_launch(g, n_seqs, q, attn_step->cache, sink, sel, g->window + g->index_topk, out, 0, 1, st);
 }

@@ -79,6 +79,11 @@ class V4Compressor:
         self.score_state = torch.full((n_seqs, p.ents, p.cd), float("-inf"), dtype=torch.float32, device=dev)
         self.ape, self.norm, self.freqs = ape, norm, freqs
 
+    def step_args(self, kv_proj, score_proj, cache, cache_rows: int, cache_row0: int, packed=None, packed_exp=None) -> be.CompStep:
+        """This compressor's part of ``launch_v4_token_step_bf16``."""
+        return be.CompStep.make(kv_proj, score_proj, self.ape, self.kv_state, self.score_state, self.norm, self.freqs,
+                                self.rotate, cache, cache_rows, cache_row0, packed, packed_exp)
+
     def step(self, pos, kv_proj, score_proj, cache, cache_rows: int, cache_row0: int, packed=None, packed_exp=None,
              prequant=None, stream=None):
         be.launch_v4_compress_step_bf16(self.p, self.B, pos, kv_proj, score_proj, self.ape, self.kv_state,
@@ -98,16 +103,13 @@ class V4TokenStep:
             dev = layer.index_kv.device
             layer.packed = torch.zeros((layer.B, g.max_comp, 128), dtype=torch.uint8, device=dev)
             layer.packed_exp = torch.zeros((layer.B, g.max_comp), dtype=torch.int32, device=dev)
-        self._seq = torch.arange(layer.B, device=layer.kv_cache.device)
 
     def __call__(self, pos, kv_entry, attn_proj, index_proj, q, index_q, index_w, stream=None):
         """pos i32 [B]; kv_entry bf16 bits [B, head_dim] (the token's window entry); attn_proj / index_proj =
         (kv_proj, score_proj) f32 [B, cd] of the two compressors; q, index_q, index_w as for V4DecodeLayer.step."""
         L, g = self.layer, self.layer.g
-        self.index_comp.step(pos, index_proj[0], index_proj[1], L.index_kv, g.max_comp, 0, L.packed, L.packed_exp,
-                             stream=stream)
-        L.select(pos, index_q, index_w, False, stream)
-        # ring write: slot pos % window (plain device copy: torch indexes int16 views of the bf16 bits)
-        L.kv_cache.view(torch.int16)[self._seq, (pos % g.window).long()] = kv_entry.view(torch.int16)
-        self.attn_comp.step(pos, attn_proj[0], attn_proj[1], L.kv_cache, L.kv_rows, g.window, stream=stream)
-        return L.attend(q, False, stream)
+        be.launch_v4_token_step_bf16(
+            g, L.B, pos, kv_entry, self.attn_comp.p, self.attn_comp.step_args(*attn_proj, L.kv_cache, L.kv_rows, g.window),
+            self.index_comp.p, self.index_comp.step_args(*index_proj, L.index_kv, g.max_comp, 0, L.packed, L.packed_exp),
+            q, index_q, index_w, L.sink, L.sel, L.scratch, L.out, stream)
+        return L.out

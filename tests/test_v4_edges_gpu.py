@@ -83,3 +83,50 @@ def test_sparse_attention_tiles_and_clusters(b, cols):
         want = s @ k
         err = (out[i].double() - want).abs()
         assert bool((err <= 1e-2 * want.abs() + 1e-2).all()), (i, err.max().item())
+
+
+@pytest.mark.parametrize("b,d,idim,off", [(1, 512, 128, 0), (3, 512, 128, 0), (5, 256, 64, 0), (9, 128, 128, 0), (2, 192, 128, 0), (4, 512, 128, 1)])
+def test_token_step_equals_its_operators(b, d, idim, off):
+    """The joint call against the operators one by one, bit for bit, over a few tokens: every width of the joint launch, widths
+    and alignments (``off`` floats off a 16-byte line) that go on their own in front of it."""
+    be, rng = _be(), np.random.default_rng(7 * b + d)
+    from rivoli_b200.v4 import V4Compressor, V4DecodeLayer, V4TokenStep
+    runs = []
+    for joint in (True, False):
+        rng = np.random.default_rng(7 * b + d)
+        f32 = lambda *s: dev(rng.standard_normal(s).astype(np.float32))
+        bf = lambda *s: dev(orc.f32_to_bf16(rng.standard_normal(s).astype(np.float32)))
+        g = be.V4Geom.make(n_heads=64 if d == 512 else 4, head_dim=d, window=8, index_heads=4, index_dim=idim, index_topk=3, max_comp=32)
+        L = V4DecodeLayer(g, b)
+        L.kv_cache.copy_(bf(*L.kv_cache.shape).view(torch.uint16))
+        L.sink.copy_(f32(g.n_heads))
+        comps = []
+        for w, rotate in ((d, False), (idim, True)):
+            p = be.CompGeom.make(ratio=4, d=w, rd=64 if w >= 128 else 32)
+            norm, freqs, ape = _comp_fixture(rng, p, 64)
+            c = V4Compressor(p, b, dev(ape), dev(norm), dev(freqs), rotate)
+            c.kv_state.copy_(f32(*c.kv_state.shape)); c.score_state.copy_(f32(*c.score_state.shape))
+            if off:
+                c.ape = torch.cat([torch.zeros(off, device="cuda"), c.ape.flatten()])[off:]
+            comps.append(c)
+        step = V4TokenStep(L, *comps)
+        pos0 = np.arange(b, dtype=np.int32) * 5 + 1
+        outs = []
+        for t in range(6):
+            pos = dev(pos0 + t)
+            x = (bf(b, d), (f32(b, 2 * d), f32(b, 2 * d)), (f32(b, 2 * idim), f32(b, 2 * idim)), bf(b, g.n_heads, d),
+                 bf(b, 4, idim), f32(b, 4))
+            if joint:
+                out = step(pos, *x)
+            else:
+                comps[1].step(pos, *x[2], L.index_kv, g.max_comp, 0, L.packed, L.packed_exp)
+                L.select(pos, x[4], x[5])
+                L.kv_cache.view(torch.int16)[torch.arange(b, device="cuda"), (pos % 8).long()] = x[0].view(torch.int16)
+                comps[0].step(pos, *x[1], L.kv_cache, L.kv_rows, g.window)
+                out = L.attend(x[3])
+            outs.append([a.clone().cpu().contiguous().view(torch.uint8) for a in (out, L.sel, L.kv_cache, L.index_kv) + tuple(
+                s for c in comps for s in (c.kv_state, c.score_state))] + ([] if L.packed is None else [L.packed.cpu(), L.packed_exp.cpu()]))
+        runs.append(outs)
+    for t, (a, w) in enumerate(zip(*runs)):
+        for i, (x, y) in enumerate(zip(a, w)):
+            assert torch.equal(x, y), (t, i)
