@@ -559,6 +559,8 @@ int rivoli_v4_token_step_bf16(const V4Geom* g, int n_seqs, const int32_t* pos, c
                               const CompStep* attn_step, const CompGeom* index, const CompStep* index_step,
                               const uint16_t* q, const uint16_t* index_q, const float* index_w, const float* sink,
                               int32_t* sel, void* scratch, uint16_t* out, void* stream);
+/* Synchronises the stream; 1008 if a bounded wait of the tensor-core block scorer gave up since the last call. */
+int rivoli_v4_select_status(void* stream);
 
 /* ---- measurement hook ------------------------------------------------------------------------------------------
  * events[0..5): cudaEvent_t handles that the following rivoli_dsa_decode_step_paged / rivoli_dsa_append_select_paged

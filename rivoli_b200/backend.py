@@ -90,7 +90,7 @@ _SIGNATURES = {
     "index_frontend_scratch_bytes": "pi", "index_frontend_bf16": "ppppi" + "p" * 12 + "ip", "index_frontend_status": "p",
     "act_quant_f4_rotated": "piip", "index_score_blocks": "ppppiiiip", "gather_attn_shared_kv": "ppppiiiifpp",
     "v4_select_scratch_bytes": "pi", "v4_select_blocks_bf16": "pi" + "p" * 8 + "ip", "v4_index_pack_bf16": "pippipppp",
-    "v4_sparse_attend_bf16": "pippppipip", "v4_sparse_attend_status": "p",
+    "v4_sparse_attend_bf16": "pippppipip", "v4_sparse_attend_status": "p", "v4_select_status": "p",
     "v4_token_step_bf16": "pi" + "p" * 14, "act_quant_f8_prefix": "ppiiiip", "kv_compress_deposit": "ppppppiip",
     "kv_compress_prefill": "pppppip", "kv_compress_decode": "ppppip",
     "v4_compress_step_bf16": "pi" + "p" * 8 + "ipiipppp",
@@ -644,6 +644,11 @@ def launch_v4_sparse_attend_bf16(g: V4Geom, n_seqs: int, q, kv_cache, sink, sel,
 def v4_sparse_attend_status(stream=None) -> None:
     """Raises BackendError(1008) if a bounded wait of the tensor-core sparse attention gave up (synchronises)."""
     ensure_status(lib().rivoli_v4_sparse_attend_status(_stream(stream)), "v4_sparse_attend_status")
+
+
+def v4_select_status(stream=None) -> None:
+    """Raises BackendError(1008) if a bounded wait of the tensor-core block scorer gave up (synchronises)."""
+    ensure_status(lib().rivoli_v4_select_status(_stream(stream)), "v4_select_status")
 
 
 class CompGeom(C.Structure):

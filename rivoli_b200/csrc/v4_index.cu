@@ -7,6 +7,8 @@
 //
 // Storage on this side is bf16 (the reference keeps bf16 VALUES in f32 arrays: every producer on the
 // path ends in a bf16 store), which halves the bytes and feeds the tensor cores directly.
+#include "tc_common.cuh"
+#include "tmap.hpp"
 #include "topk_core.cuh"
 #include "v4_common.cuh"
 
@@ -165,7 +167,7 @@ __global__ void v4_score_blocks_serial_kernel(const float* __restrict__ q, const
 // A CACHED row that is not of that form (a value that is not a multiple of the unit, block scales more
 // than 3 binades apart, a subnormal, magnitudes outside 2^-40 .. 2^40) gets a marker instead of a score
 // and the selection kernel re-scores that column with the ordered CUDA-core fold; a QUERY row outside the
-// form raises the sequence's flag and the whole sequence takes the ordered fold. Exact either way.
+// form marks every column, and the whole sequence takes the ordered fold. Exact either way.
 // ---------------------------------------------------------------------------------------------------
 constexpr int SI_THREADS = 256;
 constexpr int SI_CHUNK = 256;       // blocks (columns) per CTA
@@ -173,6 +175,7 @@ constexpr int SI_SPAN = 3;          // binades between the block scales of one r
 constexpr int SI_NT = 2;            // column tiles of 8 a warp scores per iteration
 constexpr int SI_PMIN = 87, SI_PMAX = 167;     // biased exponents 2^-40 .. 2^40
 constexpr uint32_t SI_REFOLD = 0xffc0deadu;   // score word of a column left to the ordered fold (a NaN no fold produces)
+constexpr uint32_t SI_REFOLD_ALL = 0xffc0deaeu;   // the same of every column: the queries are not of the integer form
 
 __device__ __forceinline__ void v4_mma_s8(int (&d)[4], const uint4& a, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -212,17 +215,12 @@ __device__ __forceinline__ void v4_row_unit(int pmin, int pmax, float& inv, floa
     unit = __int_as_float((pmin - 3) << 23);
 }
 
-// PACKED: the rows come as int8 + row exponent (rivoli_v4_index_pack_bf16), written once when a row enters
-// the cache; otherwise every row is converted from bf16 on every step.
-template <bool PACKED>
+// Every row is converted from bf16 here, on every step (rows that are kept packed take the kernel further down).
 __global__ void __launch_bounds__(SI_THREADS) v4_score_int8_kernel(V4Geom g, const int32_t* __restrict__ pos,
                                                                    const uint16_t* __restrict__ index_q,
                                                                    const float* __restrict__ index_w,
                                                                    const uint16_t* __restrict__ index_kv,
-                                                                   const uint8_t* __restrict__ packed,
-                                                                   const uint32_t* __restrict__ packed_exp,
-                                                                   float* __restrict__ scores,
-                                                                   int32_t* __restrict__ flags) {
+                                                                   float* __restrict__ scores) {
     __shared__ __align__(16) uint32_t qfrag[4 * 4 * 32 * 4];   // [m-tile][block][lane][4 regs]: A fragments, 8 KB
     __shared__ float qunit[64];                                // per head: its row unit (0 = empty row)
     __shared__ float wsh[64];
@@ -268,7 +266,7 @@ __global__ void __launch_bounds__(SI_THREADS) v4_score_int8_kernel(V4Geom g, con
         if (j == 0) qunit[hh] = unit;
         if (tid < 64) wsh[tid] = tid < heads ? index_w[(size_t)b * heads + tid] : 0.0f;
     }
-    __syncthreads();
+    const bool bad_q = __syncthreads_or(!ok);
     const uint16_t* kv = index_kv + (size_t)b * g.max_comp * 128;
     const int grp = lane >> 2, quad = lane & 3;
     const int c_end = min(n_comp, c_begin + SI_CHUNK);
@@ -291,42 +289,27 @@ __global__ void __launch_bounds__(SI_THREADS) v4_score_int8_kernel(V4Geom g, con
             const int c = c0 + 8 * t + grp;
             float ku = 0.0f;
             bool okk = true;                                    // this row (column of the score matrix)
-            if (PACKED) {
-                const uint8_t* prow = packed + ((size_t)b * g.max_comp + c) * 128;
-                const uint32_t e = c < n_comp ? packed_exp[(size_t)b * g.max_comp + c] : 0u;
+            uint2 lo[4], hi[4];
+            int k_lo = 1000, k_hi = -1000;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    b0[t][j] = b1[t][j] = 0u;
-                    if (c < n_comp) {
-                        b0[t][j] = *reinterpret_cast<const uint32_t*>(prow + j * 32 + quad * 4);
-                        b1[t][j] = *reinterpret_cast<const uint32_t*>(prow + j * 32 + 16 + quad * 4);
-                    }
+            for (int j = 0; j < 4; ++j) {
+                lo[j] = hi[j] = make_uint2(0, 0);
+                if (c < n_comp) {
+                    lo[j] = *reinterpret_cast<const uint2*>(kv + (size_t)c * 128 + j * 32 + quad * 4);
+                    hi[j] = *reinterpret_cast<const uint2*>(kv + (size_t)c * 128 + j * 32 + 16 + quad * 4);
                 }
-                if (e == 0xffu) okk = false;                    // the packer could not take this row
-                else if (e != 0u) ku = __int_as_float(((int)e - 3) << 23);
-            } else {
-                uint2 lo[4], hi[4];
-                int k_lo = 1000, k_hi = -1000;
+                // the block's largest exponent over the quad that holds the row, then the row's extremes
+                int pb = max(v4_max_exp4(lo[j].x, lo[j].y), v4_max_exp4(hi[j].x, hi[j].y));
+                pb = max(pb, __shfl_xor_sync(0xffffffffu, pb, 1));
+                pb = max(pb, __shfl_xor_sync(0xffffffffu, pb, 2));
+                if (pb > 0) { k_lo = min(k_lo, pb); k_hi = max(k_hi, pb); }
+            }
+            float inv;
+            v4_row_unit(k_lo, k_hi, inv, ku, okk);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    lo[j] = hi[j] = make_uint2(0, 0);
-                    if (c < n_comp) {
-                        lo[j] = *reinterpret_cast<const uint2*>(kv + (size_t)c * 128 + j * 32 + quad * 4);
-                        hi[j] = *reinterpret_cast<const uint2*>(kv + (size_t)c * 128 + j * 32 + 16 + quad * 4);
-                    }
-                    // the block's largest exponent over the quad that holds the row, then the row's extremes
-                    int pb = max(v4_max_exp4(lo[j].x, lo[j].y), v4_max_exp4(hi[j].x, hi[j].y));
-                    pb = max(pb, __shfl_xor_sync(0xffffffffu, pb, 1));
-                    pb = max(pb, __shfl_xor_sync(0xffffffffu, pb, 2));
-                    if (pb > 0) { k_lo = min(k_lo, pb); k_hi = max(k_hi, pb); }
-                }
-                float inv;
-                v4_row_unit(k_lo, k_hi, inv, ku, okk);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    b0[t][j] = v4_pack4(lo[j].x, lo[j].y, inv, okk);
-                    b1[t][j] = v4_pack4(hi[j].x, hi[j].y, inv, okk);
-                }
+            for (int j = 0; j < 4; ++j) {
+                b0[t][j] = v4_pack4(lo[j].x, lo[j].y, inv, okk);
+                b1[t][j] = v4_pack4(hi[j].x, hi[j].y, inv, okk);
             }
             // a row's verdict sits in the four lanes of its quad
             bad_rows[t] = __ballot_sync(0xffffffffu, !okk);
@@ -365,11 +348,221 @@ __global__ void __launch_bounds__(SI_THREADS) v4_score_int8_kernel(V4Geom g, con
 #pragma unroll 8
             for (int hh = 0; hh < heads; ++hh) acc = __fadd_rn(acc, terms[warp][hh][lane]);
             const bool refold = ((bad_rows[lane >> 3] >> (4 * (lane & 7))) & 0xfu) != 0;
-            scores[(size_t)b * g.max_comp + c0 + lane] = refold ? __uint_as_float(SI_REFOLD) : v4_rbf16_hw(acc);
+            scores[(size_t)b * g.max_comp + c0 + lane] = __uint_as_float(bad_q ? SI_REFOLD_ALL : refold ? SI_REFOLD : __float_as_uint(v4_rbf16_hw(acc)));
         }
         __syncwarp();
     }
-    if (!ok) atomicOr(&flags[b], 1);
+}
+
+// ---------------------------------------------------------------------------------------------------
+// the same scorer on tcgen05 kind::i8, for packed rows: tiles of 128 rows (M; one 16 KiB TMA box of the packed array, already
+// the swizzled K-major operand) against 64 heads (N), K = 128 in four instructions, s32 accumulators in TMEM. A thread of the
+// epilogue owns one row (a TMEM lane) and walks its 64 heads in order, so the ordered head sum needs no exchange at all.
+// Persistent CTAs, two per SM; an item is a run of `tpi` tiles of one sequence. 10 warps: 0-3 epilogue, 4 row producer, 5 MMA
+// issue, 6-9 convert the query of the next item (two operand buffers).
+// Bound by the epilogue's issue slots (7 instructions a head and row) and the rows' bytes, about evenly; 128 sequences of
+// 2,048 rows: 32 us with mma.sync and the terms through shared memory, 11.3 us now.
+// ---------------------------------------------------------------------------------------------------
+constexpr int ST_THREADS = 320, ST_TILE = 128, ST_NS = 4, ST_NACC = 4, ST_TPI = 16;
+constexpr int ST_Q_BYTES = 64 * 128, ST_STAGE = ST_TILE * 128;
+constexpr int ST_SMEM = ST_NS * ST_STAGE + 2 * ST_Q_BYTES + 1024;
+__device__ int g_v4_score_err;
+
+struct StArgs {
+    V4Geom g; const int32_t* pos; const uint16_t* index_q; const float* index_w; const uint32_t* packed_exp; float* scores;
+    int n_seqs, tpi, chunks;
+};
+struct StBars { uint64_t full[ST_NS], empty[ST_NS], tfull[ST_NACC], tempty[ST_NACC], qfull[2], qfree[2]; };
+
+__device__ __forceinline__ uint64_t st_f2(float a, float b) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ uint64_t st_mul2(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t st_add2(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ float2 st_unpack(uint64_t a) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a)); return r; }
+
+__global__ void __launch_bounds__(ST_THREADS) v4_score_tc_kernel(StArgs A, const __grid_constant__ CUtensorMap tm_rows) {
+    extern __shared__ __align__(1024) uint8_t st_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(st_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t* s_q = smem + ST_NS * ST_STAGE;
+    __shared__ StBars bars;
+    __shared__ uint32_t tmem_slot;
+    __shared__ volatile int abort_flag;
+    __shared__ __align__(16) float s_unit[2][64], s_w[2][64];
+    __shared__ int s_bad[2];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const V4Geom& g = A.g;
+    const int heads = g.index_heads;
+    if (tid == 0) {
+        for (int i = 0; i < ST_NS; ++i) { tc::mbar_init(&bars.full[i], 1); tc::mbar_init(&bars.empty[i], 1); }
+        for (int i = 0; i < ST_NACC; ++i) { tc::mbar_init(&bars.tfull[i], 1); tc::mbar_init(&bars.tempty[i], 4); }
+        for (int i = 0; i < 2; ++i) { tc::mbar_init(&bars.qfull[i], 128); tc::mbar_init(&bars.qfree[i], 4); }
+        tc::mbar_init_fence();
+        abort_flag = 0;
+    }
+    if (warp == 5) tc::tmem_alloc<ST_NACC * 64>(&tmem_slot);
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    rv_grid_dep_trigger();
+    rv_grid_dep_wait();
+    const int n_items = A.n_seqs * A.chunks;
+    // sequences that select by position are not scored
+    auto item_rows = [&](int item, int& b, int& t0, int& t1, int& n) {
+        b = item / A.chunks;
+        t0 = (item - b * A.chunks) * A.tpi;
+        n = min((A.pos[b] + 1) / g.ratio, g.max_comp);
+        t1 = n <= g.index_topk ? t0 : min(t0 + A.tpi, (n + ST_TILE - 1) / ST_TILE);
+        return t1 > t0;
+    };
+    int b, t0, t1, n, it = 0, done = 0;
+    bool ok = true;
+    if (warp == 4) {
+        if (lane == 0)
+            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+                if (!item_rows(item, b, t0, t1, n)) continue;
+                for (int t = t0; t < t1 && ok; ++t, ++it) {
+                    const int s = it % ST_NS;
+                    ok = tc::mbar_wait(&bars.empty[s], ((it / ST_NS) & 1) ^ 1, &abort_flag, 11);
+                    if (!ok) break;
+                    tc::mbar_arrive_expect_tx(&bars.full[s], ST_STAGE);   // rows past the array are filled with zeros
+                    tc::tma_load_2d(tc::smem_u32(smem + s * ST_STAGE), &tm_rows, 0, b * g.max_comp + t * ST_TILE, &bars.full[s]);
+                }
+            }
+    } else if (warp == 5) {
+        // instruction descriptor, kind::i8: s8 x s8 -> s32
+        const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((64u >> 3) << 17) | ((uint32_t)(ST_TILE >> 4) << 24);
+        if (lane == 0)
+            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+                if (!item_rows(item, b, t0, t1, n)) continue;
+                const int qb = done & 1;
+                ok = tc::mbar_wait(&bars.qfull[qb], (done >> 1) & 1, &abort_flag, 20);
+                for (int t = t0; t < t1 && ok; ++t, ++it) {
+                    const int s = it % ST_NS, a = it % ST_NACC;
+                    ok = tc::mbar_wait(&bars.full[s], (it / ST_NS) & 1, &abort_flag, 21) &&
+                         tc::mbar_wait(&bars.tempty[a], ((it / ST_NACC) & 1) ^ 1, &abort_flag, 22);
+                    if (!ok) break;
+                    tc::tc_fence_after();
+                    const uint64_t dk = tc::smem_desc_sw128(tc::smem_u32(smem + s * ST_STAGE), 16, 1024);
+                    const uint64_t dq = tc::smem_desc_sw128(tc::smem_u32(s_q + qb * ST_Q_BYTES), 16, 1024);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                                     "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+                                     ::"r"(tmem + a * 64), "l"(dk + 2 * k), "l"(dq + 2 * k), "r"(idesc), "r"(k) : "memory");
+                    tc::mma_commit(&bars.empty[s]);
+                    tc::mma_commit(&bars.tfull[a]);
+                }
+                ++done;
+            }
+    } else if (warp >= 6) {
+        // ---- query of an item: thread = (head, half of the 128 dims), two blocks of 32 each
+        const int t = tid - 192, hh = t >> 1, j0 = (t & 1) * 2;
+        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+            if (!item_rows(item, b, t0, t1, n)) continue;
+            const int qb = done & 1;
+            uint32_t wv[2][16];
+            int lo = 1000, hi = -1000;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                int pb = 0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint4 v = hh < heads ? *reinterpret_cast<const uint4*>(A.index_q + ((size_t)b * heads + hh) * 128 + (j0 + j) * 32 + i * 8)
+                                               : make_uint4(0, 0, 0, 0);
+                    wv[j][4 * i] = v.x; wv[j][4 * i + 1] = v.y; wv[j][4 * i + 2] = v.z; wv[j][4 * i + 3] = v.w;
+                    pb = max(pb, max(v4_max_exp4(v.x, v.y), v4_max_exp4(v.z, v.w)));
+                }
+                if (pb > 0) { lo = min(lo, pb); hi = max(hi, pb); }
+            }
+            lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, 1)); hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, 1));
+            bool fits = true;
+            float inv, unit;
+            v4_row_unit(lo, hi, inv, unit, fits);
+            uint32_t o[2][8];
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int k = 0; k < 8; ++k) o[j][k] = v4_pack4(wv[j][2 * k], wv[j][2 * k + 1], inv, fits);
+            ok = tc::mbar_wait_warp(&bars.qfree[qb], ((done >> 1) & 1) ^ 1, &abort_flag, 12);
+            if (!ok) break;
+            if (t == 0) s_bad[qb] = 0;
+            tc::named_barrier(2, 128);
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                    *reinterpret_cast<uint4*>(s_q + qb * ST_Q_BYTES + tc::sw128_chunk(hh, (j0 + j) * 2 + i)) =
+                        make_uint4(o[j][4 * i], o[j][4 * i + 1], o[j][4 * i + 2], o[j][4 * i + 3]);
+            if ((t & 1) == 0) {
+                s_unit[qb][hh] = unit;
+                s_w[qb][hh] = hh < heads ? A.index_w[(size_t)b * heads + hh] : 0.0f;
+            }
+            if (!fits) s_bad[qb] = 1;
+            tc::fence_proxy_async();
+            tc::mbar_arrive(&bars.qfull[qb]);
+            ++done;
+        }
+    } else {
+        // ---- epilogue
+        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+            if (!item_rows(item, b, t0, t1, n)) continue;
+            const int qb = done & 1;
+            const uint32_t* ep = A.packed_exp + (size_t)b * g.max_comp;
+            uint32_t e_next = t0 * ST_TILE + tid < n ? ep[t0 * ST_TILE + tid] : 0u;
+            ok = tc::mbar_wait_warp(&bars.qfull[qb], (done >> 1) & 1, &abort_flag, 30);
+            const bool bad_q = ok && s_bad[qb] != 0;
+            for (int t = t0; t < t1 && ok; ++t, ++it) {
+                const int a = it % ST_NACC, c = t * ST_TILE + tid;
+                const uint32_t e = e_next;
+                e_next = t + 1 < t1 && c + ST_TILE < n ? ep[c + ST_TILE] : 0u;
+                const float ku = (e == 0u || e == 0xffu) ? 0.0f : __int_as_float(((int)e - 3) << 23);
+                const uint64_t ku2 = st_f2(ku, ku), magic = st_f2(-12582912.0f, -12582912.0f);
+                ok = tc::mbar_wait_warp(&bars.tfull[a], (it / ST_NACC) & 1, &abort_flag, 31);
+                if (!ok) break;
+                tc::tc_fence_after();
+                float acc = 0.0f;
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    uint32_t r[32];
+                    tc::tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + a * 64 + half * 32, r);
+                    tc::tmem_ld_wait();
+                    if (half == 1) {
+                        tc::tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) tc::mbar_arrive(&bars.tempty[a]);
+                    }
+#pragma unroll
+                    for (int h = 0; h < 32; h += 4) {
+                        const float4 u4 = *reinterpret_cast<const float4*>(&s_unit[qb][half * 32 + h]);
+                        const float4 w4 = *reinterpret_cast<const float4*>(&s_w[qb][half * 32 + h]);
+#pragma unroll
+                        for (int i = 0; i < 4; i += 2) {
+                            // |I| < 2^21: 1.5 * 2^23 plus I, read as a float, less 1.5 * 2^23 is float(I)
+                            uint64_t d = st_add2(st_f2(__uint_as_float(0x4b400000u + r[h + i]), __uint_as_float(0x4b400000u + r[h + i + 1])), magic);
+                            d = st_mul2(st_mul2(d, i ? st_f2(u4.z, u4.w) : st_f2(u4.x, u4.y)), ku2);
+                            const float2 dd = st_unpack(d);
+                            uint32_t x;   // bf16 store and relu, times the (signed) head weight, bf16 store
+                            asm("cvt.rn.relu.bf16x2.f32 %0, %1, %2;" : "=r"(x) : "f"(dd.y), "f"(dd.x));
+                            const float2 p = st_unpack(st_mul2(st_f2(__uint_as_float(x << 16), __uint_as_float(x & 0xffff0000u)),
+                                                               i ? st_f2(w4.z, w4.w) : st_f2(w4.x, w4.y)));
+                            asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(x) : "f"(p.y), "f"(p.x));
+                            acc = __fadd_rn(acc, __uint_as_float(x << 16));
+                            acc = __fadd_rn(acc, __uint_as_float(x & 0xffff0000u));   // (heads beyond the model's: weight 0 adds 0)
+                        }
+                    }
+                }
+                if (c < n)
+                    A.scores[(size_t)b * g.max_comp + c] = __uint_as_float(bad_q ? SI_REFOLD_ALL : e == 0xffu ? SI_REFOLD : __float_as_uint(v4_rbf16_hw(acc)));
+            }
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&bars.qfree[qb]);
+            ++done;
+        }
+    }
+    tc::tc_fence_before();
+    __syncthreads();
+    if (warp == 5) tc::tmem_dealloc<ST_NACC * 64>(tmem);
+    if (tid == 0 && abort_flag) atomicCAS(&g_v4_score_err, 0, abort_flag);
 }
 
 // One thread per (row, block of 32): the row's values as int8 multiples of its unit 2^(pmin - 130); the row's word
@@ -468,6 +661,7 @@ __global__ void __launch_bounds__(TK_THREADS) v4_select_kernel(V4Geom g, const i
     int n_comp = (p + 1) / g.ratio;
     n_comp = n_comp < g.max_comp ? n_comp : g.max_comp;
     if (n_comp <= K) {   // every closed block, in order
+        if (tid == 0 && !force_fold) flags[b] = 0;
         for (int c = tid; c < K; c += TK_THREADS) row[W + c] = c < n_comp ? W + c : -1;
         return;
     }
@@ -491,8 +685,10 @@ __global__ void __launch_bounds__(TK_THREADS) v4_select_kernel(V4Geom g, const i
             }
         }
     };
-    if (force_fold || (flags[b] & 1)) {
+    if (force_fold || __float_as_uint(srow[0]) == SI_REFOLD_ALL) {
+        __syncthreads();             // (every thread has looked before the fold overwrites the mark)
         fold_all();
+        if (tid == 0 && !force_fold) flags[b] = 1;
     } else {
         // take the scorer's row; columns it marked are re-scored by the ordered fold, a few per warp
         if (tid == 0) sh.n_bad = 0u;
@@ -527,7 +723,7 @@ __global__ void __launch_bounds__(TK_THREADS) v4_select_kernel(V4Geom g, const i
                 }
             }
         }
-        if (n_bad > 0 && tid == 0) atomicOr(&flags[b], 2);
+        if (tid == 0) flags[b] = n_bad > 0 ? 2 : 0;
     }
     __syncthreads();
     auto key_at = [&](int i) { return v4_total_key(sc[i]); };
@@ -608,18 +804,39 @@ RIVOLI_API int rivoli_v4_select_blocks_bf16(const V4Geom* g, int n_seqs, const i
     float* scores = static_cast<float*>(scratch);
     int32_t* flags = reinterpret_cast<int32_t*>(scores + (size_t)n_seqs * g->max_comp);
     const bool tensor = !force_fold && g->index_dim == 128 && n_seqs <= 65535;
-    if (tensor) {
-        cudaMemsetAsync(flags, 0, (size_t)n_seqs * 4, st);
+    if (tensor && packed && ((uintptr_t)packed & 15) == 0 && ((uintptr_t)index_q & 15) == 0) {
+        const int tiles = (g->max_comp + ST_TILE - 1) / ST_TILE, ctas = 2 * 148;
+        // tiles per item: the run length with the shortest critical path, an item's query counted as one tile
+        int tpi = ST_TPI;
+        long long best = -1;
+        for (int c = ST_TPI; c >= 1; c >>= 1) {
+            const long long items = (long long)n_seqs * ((tiles + c - 1) / c), cost = ((items + ctas - 1) / ctas) * (c + 1);
+            if (best < 0 || cost < best) { best = cost; tpi = c; }
+        }
+        const StArgs a{*g, pos, index_q, index_w, packed_exp, scores, n_seqs, tpi, (tiles + tpi - 1) / tpi};
+        const long long items = (long long)n_seqs * a.chunks;
+        CUtensorMap tm;
+        if (int e = rivoli::make_tmap_rows_sw128(&tm, packed, (uint64_t)n_seqs * g->max_comp, 128, ST_TILE)) return e;
+        rv_allow_smem<v4_score_tc_kernel>(ST_SMEM);
+        rv_launch_dependent(v4_score_tc_kernel, dim3((unsigned)(items < ctas ? items : ctas)), dim3(ST_THREADS), (size_t)ST_SMEM, st, a, tm);
+    } else if (tensor) {
         dim3 grid((unsigned)((g->max_comp + SI_CHUNK - 1) / SI_CHUNK), (unsigned)n_seqs);
-        if (packed)
-            v4_score_int8_kernel<true><<<grid, SI_THREADS, 0, st>>>(*g, pos, index_q, index_w, index_kv, packed, packed_exp,
-                                                                    scores, flags);
-        else
-            v4_score_int8_kernel<false><<<grid, SI_THREADS, 0, st>>>(*g, pos, index_q, index_w, index_kv, packed, packed_exp,
-                                                                     scores, flags);
+        v4_score_int8_kernel<<<grid, SI_THREADS, 0, st>>>(*g, pos, index_q, index_w, index_kv, scores);
     }
+    if (int e = rv_launch_status()) return e;
     cudaFuncSetAttribute(v4_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     rv_launch_dependent(v4_select_kernel, dim3((unsigned)n_seqs), dim3(TK_THREADS), smem, st, *g, pos, index_q, index_w,
                         index_kv, sel, scores, flags, tensor ? 0 : 1);
     return rv_launch_status();
+}
+
+// Synchronises the stream; 1008 if a bounded wait of the tensor-core scorer gave up since the last call.
+RIVOLI_API int rivoli_v4_select_status(void* stream) {
+    cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);
+    if (e != cudaSuccess) return -(int)e;
+    int h = 0;
+    e = cudaMemcpyFromSymbol(&h, g_v4_score_err, sizeof(int));
+    if (e != cudaSuccess) return -(int)e;
+    if (h) { const int z = 0; cudaMemcpyToSymbol(g_v4_score_err, &z, sizeof(int)); }
+    return h ? 1008 : 0;
 }

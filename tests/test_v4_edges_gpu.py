@@ -85,6 +85,50 @@ def test_sparse_attention_tiles_and_clusters(b, cols):
         assert bool((err <= 1e-2 * want.abs() + 1e-2).all()), (i, err.max().item())
 
 
+@pytest.mark.parametrize("b,max_comp,heads", [(1, 127, 64), (1, 129, 3), (2, 2048, 64), (5, 500, 33), (37, 640, 64), (300, 130, 16)])
+def test_packed_scorer_tiles_and_items(b, max_comp, heads):
+    """Packed rows on the tensor cores against the ordered fold: scores, rows and flags for contexts around the 128-row tile,
+    every item length, queries and single rows outside the integer form."""
+    be = _be()
+    g = be.V4Geom.make(max_comp=max_comp, index_heads=heads, index_topk=40)
+    gen = torch.Generator("cuda").manual_seed(b)
+
+    def spread(n):
+        x = torch.randn((n, 128), generator=gen, device="cuda").to(torch.bfloat16).float()
+        be.launch_act_quant_f4_rotated(x, n, 128)
+        return x.to(torch.bfloat16)
+
+    ikv, iq = spread(b * max_comp).view(b, max_comp, 128), spread(b * heads).view(b, heads, 128)
+    iw = torch.randn((b, heads), generator=gen, device="cuda").to(torch.bfloat16).float()
+    want_flags = torch.zeros(b, dtype=torch.int32)
+    n_comp = torch.randint(30, max_comp + 1, (b,), generator=gen, device="cuda")
+    n_comp[0] = max_comp
+    if b > 2:
+        n_comp[1], n_comp[2] = max_comp, 41
+        iq[1, heads - 1, 5] = 0.3711
+        ikv[2, 40, :32] *= 1024.0
+        want_flags[1], want_flags[2] = 1, 2
+    pos = (n_comp * 4).to(torch.int32)
+    packed = torch.zeros((b, max_comp, 128), dtype=torch.uint8, device="cuda")
+    pexp = torch.zeros((b, max_comp), dtype=torch.int32, device="cuda")
+    be.launch_v4_index_pack_bf16(g, b, None, n_comp.to(torch.int32), max_comp, ikv.view(torch.int16), packed, pexp)
+    res = []
+    for fold, p in ((True, None), (False, packed), (False, None)):
+        sel = torch.full((b, g.window + 40), -7, dtype=torch.int32, device="cuda")
+        scratch = torch.full((be.v4_select_scratch_bytes(g, b) // 4,), 5.0, device="cuda")
+        be.launch_v4_select_blocks_bf16(g, b, pos, iq.view(torch.int16), iw, ikv.view(torch.int16), sel, scratch, fold, p,
+                                        None if p is None else pexp)
+        be.v4_select_status()
+        res.append((sel.cpu(), scratch[:b * max_comp].view(b, max_comp).cpu(), scratch[b * max_comp:].view(torch.int32).cpu()))
+    for sel, sc, flags in res[1:]:
+        assert torch.equal(sel, res[0][0])
+        assert torch.equal(flags, want_flags)
+        for i in range(b):
+            n = int(n_comp[i])
+            if n > 40:
+                assert torch.equal(sc[i, :n].view(torch.int32), res[0][1][i, :n].view(torch.int32)), i
+
+
 @pytest.mark.parametrize("b,d,idim,off", [(1, 512, 128, 0), (3, 512, 128, 0), (5, 256, 64, 0), (9, 128, 128, 0), (2, 192, 128, 0), (4, 512, 128, 1)])
 def test_token_step_equals_its_operators(b, d, idim, off):
     """The joint call against the operators one by one, bit for bit, over a few tokens: every width of the joint launch, widths
