@@ -20,8 +20,7 @@
 
 namespace {
 
-constexpr int KP_THREADS = 256;   // 8 warps: loaders by (warp = row, lane = chunk); epilogue by (lane quadrant, column half)
-constexpr int KP_WARPS = KP_THREADS / 32;
+constexpr int KP_THREADS = 256;   // 8 warps; epilogue by (lane quadrant, column half)
 __device__ int g_kp_err;
 
 __device__ __forceinline__ uint64_t kp_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
@@ -69,65 +68,91 @@ struct KpArgs {
     uint16_t* out;
 };
 
+// All of a tile's bytes are requested before anything is waited for: contraction chunks of 64, one cp.async group each
+// (activations, raw codes), then chunk by chunk the codes are converted (two tile buffers) and the chunk's MMAs issued while
+// later chunks are still on their way. The result is staged in the idle activation tiles and leaves as whole rows.
+// 128 sequences, us: absorb 16.4 -> 10.7, value 15.9 -> 11.9 (loads into registers, one conversion pass, two halves of the
+// value contraction one after the other, 16-byte stores to 32 rows at a time); bound by what an SM can take in
+// (192 KiB at 18 bytes a clock in the value kernel), a launch's ramp and the epilogue.
+constexpr int KP_ACHUNK = 16384, KP_WCHUNK = 8192, KP_CONV = 16384;
+
+// Requests activation chunk c (128 sequences from b0 x 64 bf16, swizzled K-major; rows past B are zeros) into `dst`.
+__device__ __forceinline__ void kp_request_acts(const KpArgs& A, int h, int b0, int c, uint8_t* dst) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int e = threadIdx.x + i * KP_THREADS, row = e >> 3, j = e & 7;
+        const bool live = b0 + row < A.B;
+        tc::cp_async16_zfill(tc::smem_u32(dst + tc::sw128_chunk(row, j)),
+                             A.x + ((size_t)(live ? b0 + row : 0) * A.H + h) * A.xs + c * 64 + j * 8, live ? 16u : 0u);
+    }
+}
+// Sixteen e4m3 codes of a raw piece -> two 16-byte bf16 chunks.
+__device__ __forceinline__ void kp_convert16(const uint8_t* raw, uint8_t* d0, uint8_t* d1) {
+    const uint4 v = *reinterpret_cast<const uint4*>(raw);
+    *reinterpret_cast<uint4*>(d0) = kp_codes_to_bf16(make_uint2(v.x, v.y));
+    *reinterpret_cast<uint4*>(d1) = kp_codes_to_bf16(make_uint2(v.z, v.w));
+}
+// Waits until at most `left` of this thread's copy groups are pending (left < 8).
+__device__ __forceinline__ void kp_wait_groups(int left) {
+    switch (left) {
+        case 0: tc::cp_async_wait<0>(); break;
+        case 1: tc::cp_async_wait<1>(); break;
+        case 2: tc::cp_async_wait<2>(); break;
+        case 3: tc::cp_async_wait<3>(); break;
+        case 4: tc::cp_async_wait<4>(); break;
+        case 5: tc::cp_async_wait<5>(); break;
+        case 6: tc::cp_async_wait<6>(); break;
+        default: tc::cp_async_wait<7>(); break;
+    }
+}
+// The 128 x 128 bf16 result staged as [128 rows][256 B], 16-byte chunks XORed with the row: chunk k of row r.
+__device__ __forceinline__ uint32_t kp_stage(int r, int k) { return (uint32_t)(r * 256 + ((k ^ (r & 7)) << 4)); }
+// ... and stored: sixteen lanes a row.
+__device__ __forceinline__ void kp_store_rows(const uint8_t* stage, uint16_t* out, size_t pitch, int rows) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int e = threadIdx.x + i * KP_THREADS, r = e >> 4, k = e & 15;
+        if (r < rows) *reinterpret_cast<uint4*>(out + (size_t)r * pitch + k * 8) = *reinterpret_cast<const uint4*>(stage + kp_stage(r, k));
+    }
+}
+
 // ---------------------------------------------------------------------------------------------
-// absorb: grid (kvl / 128, H), 128 threads. Shared: A [nope/64][128 rows][128 B] | B [2][nope][128 B].
+// absorb: grid (kvl / 128, H). Shared: activation chunks [nope/64][128 rows][128 B] | raw codes [nope/64][64 rows][128 B] |
+// two converted tiles [2 column halves][64 rows][128 B] (MN-major).
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(KP_THREADS)
 kvb_absorb_mma_kernel(KpArgs A) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ uint64_t bar;
+    __shared__ uint64_t bar[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_word;
     volatile int* abort_flag = &abort_word;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int iblk = blockIdx.x, h = blockIdx.y;
-    const int nope = A.nope, kvl = A.kvl, W = A.kvl + A.rope;
-    const int a_bytes = (nope / 64) * 16384;
+    const int nope = A.nope, kvl = A.kvl, W = A.kvl + A.rope, nch = nope / 64;
     uint8_t* sA = smem;
-    uint8_t* sB = smem + a_bytes;
+    uint8_t* sW = sA + nch * KP_ACHUNK;
+    uint8_t* sB = sW + nch * KP_WCHUNK;
     const size_t rbase = (size_t)h * (nope + A.vh);
     const int sc_cols = kvl / 128;
     // runs of d with one scale: [0, cut) and [cut, nope); cut = distance to the next block boundary
     const int cut = min(nope, (int)(128 - (rbase & 127)));
-    const float s0 = A.scale[(rbase >> 7) * sc_cols + iblk];
     const bool two_runs = cut < nope;
-    const float s1 = two_runs ? A.scale[((rbase + cut) >> 7) * sc_cols + iblk] : 0.0f;
-
-    if (tid == 0) { tc::mbar_init(&bar, 1); tc::mbar_init_fence(); abort_word = 0; }
+    if (tid == 0) { tc::mbar_init(&bar[0], 1); tc::mbar_init(&bar[1], 1); tc::mbar_init_fence(); abort_word = 0; }
     if (warp == 0) tc::tmem_alloc<256>(&tmem_slot);
-    // activations of a batch tile: 128 sequences x nope bf16, K-major swizzled; warp = row, lane = 16-byte chunk;
-    // rows past B are zeros. Asynchronous: requested BEFORE the weights are fetched and converted.
-    auto load_acts = [&](int b0) {
-        const int chunks = nope / 8;
-        for (int row = warp; row < 128; row += KP_WARPS) {
-            const bool live = b0 + row < A.B;
-            const uint16_t* src = A.x + ((size_t)(live ? b0 + row : 0) * A.H + h) * A.xs;
-            for (int j = lane; j < chunks; j += 32) {
-                uint8_t* dst = sA + (j >> 3) * 16384 + tc::sw128_chunk(row, j & 7);
-                if (live) tc::cp_async16(tc::smem_u32(dst), src + j * 8);
-                else *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
-            }
+    rv_grid_dep_trigger();
+    rv_grid_dep_wait();
+    for (int c = 0; c < nch; ++c) {
+        kp_request_acts(A, h, 0, c, sA + c * KP_ACHUNK);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int e = tid + i * KP_THREADS, d = e >> 3, j = e & 7;
+            tc::cp_async16(tc::smem_u32(sW + c * KP_WCHUNK + d * 128 + j * 16), A.kvb + (rbase + c * 64 + d) * kvl + iblk * 128 + j * 16);
         }
         tc::cp_async_commit();
-    };
-    load_acts(0);
-    // weights: row d, this CTA's 128 columns = 16 pieces of 8 codes -> bf16 chunks, MN-major tile.
-    // Two rows per warp pass (lane = row half x piece); ALL passes (nope <= 256: at most 16) are in flight
-    // before the first conversion, so the tile costs one memory round trip.
-    {
-        uint2 c[16];
-#pragma unroll
-        for (int u = 0; u < 16; ++u) {
-            const int d = warp * 2 + u * KP_WARPS * 2 + (lane >> 4);
-            c[u] = d < nope ? *reinterpret_cast<const uint2*>(A.kvb + (rbase + d) * kvl + iblk * 128 + (lane & 15) * 8) : make_uint2(0, 0);
-        }
-#pragma unroll
-        for (int u = 0; u < 16; ++u) {
-            const int d = warp * 2 + u * KP_WARPS * 2 + (lane >> 4), pc = lane & 15;
-            if (d < nope)
-                *reinterpret_cast<uint4*>(sB + (pc >> 3) * (nope * 128) + tc::sw128_chunk(d, pc & 7)) = kp_codes_to_bf16(c[u]);
-        }
     }
+    const float s0 = A.scale[(rbase >> 7) * sc_cols + iblk];
+    const float s1 = two_runs ? A.scale[((rbase + cut) >> 7) * sc_cols + iblk] : 0.0f;
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
@@ -136,47 +161,59 @@ kvb_absorb_mma_kernel(KpArgs A) {
     const uint32_t lane_base = ((uint32_t)((warp & 3) * 32)) << 16;   // TMEM lane quadrant of this warp
     const int erow = (warp & 3) * 32 + lane, chalf = warp >> 2;      // epilogue: sequence row, column half
     bool ok = true;
-    int phase = 0;
-    for (int b0 = 0; b0 < A.B && ok; b0 += 128, phase ^= 1) {
-        if (b0 > 0) load_acts(b0);     // the first tile was requested before the weights
-        // the rope segment of q rides along (column block 0 only; thread = sequence row): its loads go out
-        // now and are stored after the MMAs were issued, off every wait's critical path
-        uint4 rope_v[8];
-        const bool rope_mine = iblk == 0 && tid < 128 && b0 + tid < A.B;
-        if (rope_mine) {
-            const uint4* src = reinterpret_cast<const uint4*>(A.x + ((size_t)(b0 + tid) * A.H + h) * A.xs + nope);
+    int done[2] = {0, 0};
+    for (int b0 = 0; b0 < A.B && ok; b0 += 128) {
+        if (b0 > 0)
+            for (int c = 0; c < nch; ++c) { kp_request_acts(A, h, b0, c, sA + c * KP_ACHUNK); tc::cp_async_commit(); }
+        // the rope segment of q rides along (column block 0 only)
+        const int rope16 = A.rope / 8;
+        uint4 rope_v[4];
+        if (iblk == 0) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) rope_v[e] = e < A.rope / 8 ? src[e] : make_uint4(0, 0, 0, 0);
-        }
-        tc::cp_async_wait<0>();
-        tc::fence_proxy_async();
-        __syncthreads();
-        if (tid == 0) {
-            tc::tc_fence_after();
-            const uint32_t a0 = tc::smem_u32(sA), b0a = tc::smem_u32(sB);
-            for (int k = 0; k < nope / 16; ++k) {     // 16 bf16 per MMA; a run boundary is a multiple of 64
-                const int run = (k * 16 >= cut) ? 1 : 0;
-                const bool first = (k * 16 == 0) || (k * 16 == cut);
-#ifdef KP_TEST_KMAJOR   // timing experiment only (wrong numbers): the same tile described as K-major
-                kp_mma(tmem + run * 128, kp_desc(a0 + (k >> 2) * 16384 + (k & 3) * 32, 16, 1024),
-                       kp_desc(b0a + (k >> 2) * 16384 + (k & 3) * 32, 16, 1024), kp_idesc(128, 128, 0), first ? 0u : 1u);
-#else
-                kp_mma(tmem + run * 128, kp_desc(a0 + (k >> 2) * 16384 + (k & 3) * 32, 16, 1024),
-                       kp_desc(b0a + k * 2048, (uint32_t)nope * 128, 1024), idesc, first ? 0u : 1u);
-#endif
+            for (int i = 0; i < 4; ++i) {
+                const int e = tid + i * KP_THREADS, r = rope16 > 0 ? e / rope16 : 128, j = e - r * rope16;
+                if (r < 128 && b0 + r < A.B) rope_v[i] = *reinterpret_cast<const uint4*>(A.x + ((size_t)(b0 + r) * A.H + h) * A.xs + nope + j * 8);
             }
-            tc::mma_commit(&bar);
         }
-        if (rope_mine) {
-            uint4* dst = reinterpret_cast<uint4*>(A.out + ((size_t)(b0 + tid) * A.H + h) * W + kvl);
+        for (int c = 0; c < nch && ok; ++c) {
+            const int wb = c & 1;
+            if (done[wb] > 0) ok = tc::mbar_wait_warp(&bar[wb], (done[wb] - 1) & 1, abort_flag, 71);
+            if (!ok) break;
+            kp_wait_groups(nch - 1 - c);
+            __syncthreads();
+            uint8_t* sb = sB + wb * KP_CONV;
 #pragma unroll
-            for (int e = 0; e < 8; ++e)
-                if (e < A.rope / 8) dst[e] = rope_v[e];
+            for (int i = 0; i < 2; ++i) {
+                const int e = tid + i * KP_THREADS, d = e >> 3, j = e & 7;
+                uint8_t* half = sb + (j >> 2) * 8192;
+                kp_convert16(sW + c * KP_WCHUNK + d * 128 + j * 16, half + tc::sw128_chunk(d, (j & 3) * 2), half + tc::sw128_chunk(d, (j & 3) * 2 + 1));
+            }
+            tc::fence_proxy_async();
+            __syncthreads();
+            if (tid == 0) {
+                tc::tc_fence_after();
+                const uint32_t a0 = tc::smem_u32(sA + c * KP_ACHUNK), w0 = tc::smem_u32(sb);
+                const int run = c * 64 >= cut ? 1 : 0;       // (a run boundary is a multiple of 64)
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    kp_mma(tmem + run * 128, kp_desc(a0 + k * 32, 16, 1024), kp_desc(w0 + k * 2048, 8192, 1024), idesc,
+                           (k == 0 && (c == 0 || c * 64 == cut)) ? 0u : 1u);
+                tc::mma_commit(&bar[wb]);
+            }
+            ++done[wb];
         }
-        ok = tc::mbar_wait_warp(&bar, phase, abort_flag, 71);
+        if (iblk == 0) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int e = tid + i * KP_THREADS, r = rope16 > 0 ? e / rope16 : 128, j = e - r * rope16;
+                if (r < 128 && b0 + r < A.B) *reinterpret_cast<uint4*>(A.out + ((size_t)(b0 + r) * A.H + h) * W + kvl + j * 8) = rope_v[i];
+            }
+        }
+        for (int wb = 0; wb < 2 && ok; ++wb)
+            if (done[wb] > 0) ok = tc::mbar_wait_warp(&bar[wb], (done[wb] - 1) & 1, abort_flag, 72);
         tc::tc_fence_after();
         if (ok) {
-#pragma unroll 1
+#pragma unroll
             for (int c = chalf * 2; c < chalf * 2 + 2; ++c) {
                 uint32_t r0[32], r1[32];
                 tc::tmem_ld32(tmem + lane_base + c * 32, r0);
@@ -186,30 +223,31 @@ kvb_absorb_mma_kernel(KpArgs A) {
 #pragma unroll
                     for (int e = 0; e < 32; ++e) r1[e] = 0u;
                 }
-                if (b0 + erow < A.B) {
-                    uint32_t o[16];
+                uint32_t o[16];
 #pragma unroll
-                    for (int e = 0; e < 32; e += 2) {
-                        const float v0 = fmaf(__uint_as_float(r1[e]), s1, __uint_as_float(r0[e]) * s0);
-                        const float v1 = fmaf(__uint_as_float(r1[e + 1]), s1, __uint_as_float(r0[e + 1]) * s0);
-                        o[e >> 1] = (uint32_t)rv_f32_to_bf16(v0) | ((uint32_t)rv_f32_to_bf16(v1) << 16);
-                    }
-                    uint4* dst = reinterpret_cast<uint4*>(A.out + ((size_t)(b0 + erow) * A.H + h) * W + iblk * 128 + c * 32);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) dst[e] = make_uint4(o[4 * e], o[4 * e + 1], o[4 * e + 2], o[4 * e + 3]);
+                for (int e = 0; e < 32; e += 2) {
+                    const float v0 = fmaf(__uint_as_float(r1[e]), s1, __uint_as_float(r0[e]) * s0);
+                    const float v1 = fmaf(__uint_as_float(r1[e + 1]), s1, __uint_as_float(r0[e + 1]) * s0);
+                    o[e >> 1] = (uint32_t)rv_f32_to_bf16(v0) | ((uint32_t)rv_f32_to_bf16(v1) << 16);
                 }
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    *reinterpret_cast<uint4*>(smem + kp_stage(erow, c * 4 + e)) = make_uint4(o[4 * e], o[4 * e + 1], o[4 * e + 2], o[4 * e + 3]);
             }
         }
         tc::tc_fence_before();
-        __syncthreads();   // TMEM and the A tile are free for the next batch tile
+        __syncthreads();
+        if (ok) kp_store_rows(smem, A.out + ((size_t)b0 * A.H + h) * W + iblk * 128, (size_t)A.H * W, min(128, A.B - b0));
+        __syncthreads();   // TMEM and the A tiles are free for the next batch tile
     }
+    tc::cp_async_wait<0>();
     if (warp == 0) tc::tmem_dealloc<256>(tmem);
     if (tid == 0 && abort_word) atomicCAS(&g_kp_err, 0, abort_word);
 }
 
 // ---------------------------------------------------------------------------------------------
-// value: grid (vh / 128, H), 256 threads; N = 128 value rows = two 64-row scale rows.
-// Shared: A half [kvl/128][128 rows][128 B] (the contraction is fed in two halves) | B [kvl/64][128 rows][128 B].
+// value: grid (vh / 128, H), N = 128 value rows = two 64-row scale rows. Shared: activation chunks [kvl/64][128 rows][128 B] |
+// raw codes [kvl/64][128 rows][64 B] | two converted tiles [128 rows][128 B] (K-major).
 // TMEM: one 128-column accumulator per scale column (kvl / 128 <= 4 runs).
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(KP_THREADS)
@@ -222,54 +260,26 @@ kvb_value_mma_kernel(KpArgs A) {
     volatile int* abort_flag = &abort_word;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int jblk = blockIdx.x, h = blockIdx.y;
-    const int kvl = A.kvl, vh = A.vh;
-    const int kch = kvl / 64;                 // 128-byte K chunks in all
-    const int hch = kch / 2;                  // per half
+    const int kvl = A.kvl, vh = A.vh, nch = kvl / 64;
     uint8_t* sA = smem;
-    uint8_t* sB = smem + hch * 16384;
+    uint8_t* sW = sA + nch * KP_ACHUNK;
+    uint8_t* sB = sW + nch * KP_WCHUNK;
     const size_t row0 = (size_t)h * (A.nope + vh) + A.nope + (size_t)jblk * 128;   // 128 value rows = 2 scale rows
     const int sc_cols = kvl / 128;
-    if (tid < 2 * sc_cols) s_sc[tid / sc_cols][tid % sc_cols] = A.scale[((row0 + (tid / sc_cols) * 64) >> 7) * sc_cols + tid % sc_cols];
     if (tid == 0) { tc::mbar_init(&bar[0], 1); tc::mbar_init(&bar[1], 1); tc::mbar_init_fence(); abort_word = 0; }
     if (warp == 0) tc::tmem_alloc<512>(&tmem_slot);
-    // activations of one half of the contraction for a batch tile: 128 sequences x kvl/2 bf16, K-major
-    // swizzled; warp = row, lane = 16-byte chunk; rows past B are zeros. Asynchronous.
-    auto load_acts = [&](int b0, int half) {
-        const int chunks = kvl / 16;
-        for (int row = warp; row < 128; row += KP_WARPS) {
-            const bool live = b0 + row < A.B;
-            const uint16_t* src = A.x + ((size_t)(live ? b0 + row : 0) * A.H + h) * A.xs + half * (kvl / 2);
-            for (int j = lane; j < chunks; j += 32) {
-                uint8_t* dst = sA + (j >> 3) * 16384 + tc::sw128_chunk(row, j & 7);
-                if (live) tc::cp_async16(tc::smem_u32(dst), src + j * 8);
-                else *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
-            }
+    rv_grid_dep_trigger();
+    rv_grid_dep_wait();
+    for (int c = 0; c < nch; ++c) {
+        kp_request_acts(A, h, 0, c, sA + c * KP_ACHUNK);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int e = tid + i * KP_THREADS, r = e >> 2, j = e & 3;
+            tc::cp_async16(tc::smem_u32(sW + c * KP_WCHUNK + r * 64 + j * 16), A.kvb + (row0 + r) * kvl + c * 64 + j * 16);
         }
         tc::cp_async_commit();
-    };
-    load_acts(0, 0);
-    // weights: 128 rows x kvl codes -> bf16, K-major swizzled tile; warp = row, lane = piece of 8 codes;
-    // all sixteen rows of a warp (32 loads per lane) in flight before the first conversion
-    const int pieces = kvl / 8;
-    {
-        uint2 c[16][2];
-#pragma unroll
-        for (int r = 0; r < 16; ++r) {
-            const uint8_t* wrow = A.kvb + (row0 + warp + r * KP_WARPS) * kvl;
-#pragma unroll
-            for (int u = 0; u < 2; ++u)
-                c[r][u] = lane + 32 * u < pieces ? *reinterpret_cast<const uint2*>(wrow + (lane + 32 * u) * 8) : make_uint2(0, 0);
-        }
-#pragma unroll
-        for (int r = 0; r < 16; ++r) {
-            const int j = warp + r * KP_WARPS;
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const int pc = lane + 32 * u;
-                if (pc < pieces) *reinterpret_cast<uint4*>(sB + (pc >> 3) * 16384 + tc::sw128_chunk(j, pc & 7)) = kp_codes_to_bf16(c[r][u]);
-            }
-        }
     }
+    if (tid < 2 * sc_cols) s_sc[tid / sc_cols][tid % sc_cols] = A.scale[((row0 + (tid / sc_cols) * 64) >> 7) * sc_cols + tid % sc_cols];
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
@@ -278,30 +288,39 @@ kvb_value_mma_kernel(KpArgs A) {
     const uint32_t lane_base = ((uint32_t)((warp & 3) * 32)) << 16;   // TMEM lane quadrant of this warp
     const int erow = (warp & 3) * 32 + lane, chalf = warp >> 2;      // epilogue: sequence row, 64-column half
     bool ok = true;
-    int phase = 0;
-    for (int b0 = 0; b0 < A.B && ok; b0 += 128, phase ^= 1) {
-        for (int half = 0; half < 2 && ok; ++half) {
-            if (b0 > 0 || half > 0) load_acts(b0, half);   // the very first request went out before the weights
-            tc::cp_async_wait<0>();
+    int done[2] = {0, 0};
+    for (int b0 = 0; b0 < A.B && ok; b0 += 128) {
+        if (b0 > 0)
+            for (int c = 0; c < nch; ++c) { kp_request_acts(A, h, b0, c, sA + c * KP_ACHUNK); tc::cp_async_commit(); }
+        for (int c = 0; c < nch && ok; ++c) {
+            const int wb = c & 1;
+            if (done[wb] > 0) ok = tc::mbar_wait_warp(&bar[wb], (done[wb] - 1) & 1, abort_flag, 73);
+            if (!ok) break;
+            kp_wait_groups(nch - 1 - c);
+            __syncthreads();
+            uint8_t* sb = sB + wb * KP_CONV;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int e = tid + i * KP_THREADS, r = e >> 2, j = e & 3;
+                kp_convert16(sW + c * KP_WCHUNK + r * 64 + j * 16, sb + tc::sw128_chunk(r, 2 * j), sb + tc::sw128_chunk(r, 2 * j + 1));
+            }
             tc::fence_proxy_async();
             __syncthreads();
             if (tid == 0) {
                 tc::tc_fence_after();
-                const uint32_t a0 = tc::smem_u32(sA), b0a = tc::smem_u32(sB);
-                const int ks = kvl / 32;                  // MMAs per half; 8 per scale column (128 latent dims)
-                for (int kk = 0; kk < ks; ++kk) {
-                    const int k = half * ks + kk;
-                    kp_mma(tmem + (k >> 3) * 128, kp_desc(a0 + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
-                           kp_desc(b0a + (k >> 2) * 16384 + (k & 3) * 32, 16, 1024), idesc, (k & 7) ? 1u : 0u);
-                }
-                tc::mma_commit(&bar[half]);
+                const uint32_t a0 = tc::smem_u32(sA + c * KP_ACHUNK), w0 = tc::smem_u32(sb);
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    kp_mma(tmem + (c >> 1) * 128, kp_desc(a0 + k * 32, 16, 1024), kp_desc(w0 + k * 32, 16, 1024), idesc, ((c & 1) | k) ? 1u : 0u);
+                tc::mma_commit(&bar[wb]);
             }
-            // the A half may be overwritten (and the accumulators read) only once these MMAs are done
-            ok = tc::mbar_wait_warp(&bar[half], phase, abort_flag, 72 + half);
+            ++done[wb];
         }
+        for (int wb = 0; wb < 2 && ok; ++wb)
+            if (done[wb] > 0) ok = tc::mbar_wait_warp(&bar[wb], (done[wb] - 1) & 1, abort_flag, 74);
         tc::tc_fence_after();
         if (ok) {
-#pragma unroll 1
+#pragma unroll
             for (int c = chalf * 2; c < chalf * 2 + 2; ++c) {
                 float acc[32];
 #pragma unroll
@@ -314,20 +333,21 @@ kvb_value_mma_kernel(KpArgs A) {
 #pragma unroll
                     for (int e = 0; e < 32; ++e) acc[e] = fmaf(__uint_as_float(r[e]), sc, acc[e]);
                 }
-                if (b0 + erow < A.B) {
-                    uint32_t o[16];
+                uint32_t o[16];
 #pragma unroll
-                    for (int e = 0; e < 32; e += 2)
-                        o[e >> 1] = (uint32_t)rv_f32_to_bf16(acc[e]) | ((uint32_t)rv_f32_to_bf16(acc[e + 1]) << 16);
-                    uint4* dst = reinterpret_cast<uint4*>(A.out + ((size_t)(b0 + erow) * A.H + h) * vh + jblk * 128 + c * 32);
+                for (int e = 0; e < 32; e += 2)
+                    o[e >> 1] = (uint32_t)rv_f32_to_bf16(acc[e]) | ((uint32_t)rv_f32_to_bf16(acc[e + 1]) << 16);
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) dst[e] = make_uint4(o[4 * e], o[4 * e + 1], o[4 * e + 2], o[4 * e + 3]);
-                }
+                for (int e = 0; e < 4; ++e)
+                    *reinterpret_cast<uint4*>(smem + kp_stage(erow, c * 4 + e)) = make_uint4(o[4 * e], o[4 * e + 1], o[4 * e + 2], o[4 * e + 3]);
             }
         }
         tc::tc_fence_before();
         __syncthreads();
+        if (ok) kp_store_rows(smem, A.out + ((size_t)b0 * A.H + h) * vh + jblk * 128, (size_t)A.H * vh, min(128, A.B - b0));
+        __syncthreads();
     }
+    tc::cp_async_wait<0>();
     if (warp == 0) tc::tmem_dealloc<512>(tmem);
     if (tid == 0 && abort_word) atomicCAS(&g_kp_err, 0, abort_word);
 }
@@ -350,23 +370,20 @@ extern "C" int rivoli_kvb_mma_supported(int H, int qh, int nope, int vh, int kvl
 extern "C" int rivoli_kvb_absorb_mma(const uint16_t* q, const uint8_t* kvb, const float* scale, int H, int qh, int nope,
                                      int vh, int kvl, int rope, int block, int B, uint16_t* q_abs, cudaStream_t st) {
     const KpArgs a{q, kvb, scale, H, qh, nope, vh, kvl, rope, block, B, q_abs};
-    size_t smem = (size_t)(nope / 64) * 16384 + (size_t)2 * nope * 128;
-#ifdef KP_TEST_ONE_CTA   // timing experiment: one CTA per SM
-    if (smem < 120 * 1024) smem = 120 * 1024;
-#endif
-    cudaFuncSetAttribute(kvb_absorb_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const size_t smem = (size_t)(nope / 64) * (KP_ACHUNK + KP_WCHUNK) + 2 * KP_CONV;
+    rv_allow_smem<kvb_absorb_mma_kernel>(4 * (KP_ACHUNK + KP_WCHUNK) + 2 * KP_CONV);
     rv_drain_error();
-    kvb_absorb_mma_kernel<<<dim3(kvl / 128, H), KP_THREADS, smem, st>>>(a);
+    rv_launch_dependent(kvb_absorb_mma_kernel, dim3(kvl / 128, H), dim3(KP_THREADS), smem, st, a);
     return rv_launch_status();
 }
 
 extern "C" int rivoli_kvb_value_mma(const uint16_t* clat, const uint8_t* kvb, const float* scale, int H, int nope, int vh,
                                     int kvl, int block, int B, uint16_t* ctx, cudaStream_t st) {
     const KpArgs a{clat, kvb, scale, H, kvl, nope, vh, kvl, 0, block, B, ctx};
-    const size_t smem = (size_t)(kvl / 128) * 16384 + (size_t)(kvl / 64) * 16384;
-    cudaFuncSetAttribute(kvb_value_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const size_t smem = (size_t)(kvl / 64) * (KP_ACHUNK + KP_WCHUNK) + 2 * KP_CONV;
+    rv_allow_smem<kvb_value_mma_kernel>(8 * (KP_ACHUNK + KP_WCHUNK) + 2 * KP_CONV);
     rv_drain_error();
-    kvb_value_mma_kernel<<<dim3(vh / 128, H), KP_THREADS, smem, st>>>(a);
+    rv_launch_dependent(kvb_value_mma_kernel, dim3(vh / 128, H), dim3(KP_THREADS), smem, st, a);
     return rv_launch_status();
 }
 
