@@ -70,11 +70,12 @@ struct KpArgs {
 
 // All of a tile's bytes are requested before anything is waited for: contraction chunks of 64, one cp.async group each
 // (activations, raw codes), then chunk by chunk the codes are converted (two tile buffers) and the chunk's MMAs issued while
-// later chunks are still on their way. The result is staged in the idle activation tiles and leaves as whole rows.
-// 128 sequences, us: absorb 16.4 -> 10.7, value 15.9 -> 11.9 (loads into registers, one conversion pass, two halves of the
+// later chunks are still on their way. The result is staged in the idle converted tiles and leaves as whole rows.
+// 128 sequences, us: absorb 16.4 -> 10.4, value 15.9 -> 11.6 (loads into registers, one conversion pass, two halves of the
 // value contraction one after the other, 16-byte stores to 32 rows at a time); bound by what an SM can take in
 // (192 KiB at 18 bytes a clock in the value kernel), a launch's ramp and the epilogue.
 constexpr int KP_ACHUNK = 16384, KP_WCHUNK = 8192, KP_CONV = 16384;
+static_assert(2 * KP_CONV == 128 * 256, "the result fits the converted tiles");
 
 // Requests activation chunk c (128 sequences from b0 x 64 bf16, swizzled K-major; rows past B are zeros) into `dst`.
 __device__ __forceinline__ void kp_request_acts(const KpArgs& A, int h, int b0, int c, uint8_t* dst) {
@@ -179,8 +180,7 @@ kvb_absorb_mma_kernel(KpArgs A) {
             const int wb = c & 1;
             if (done[wb] > 0) ok = tc::mbar_wait_warp(&bar[wb], (done[wb] - 1) & 1, abort_flag, 71);
             if (!ok) break;
-            kp_wait_groups(nch - 1 - c);
-            __syncthreads();
+            kp_wait_groups(nch - 1 - c);   // (a thread converts the codes that it requested itself)
             uint8_t* sb = sB + wb * KP_CONV;
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
@@ -232,12 +232,12 @@ kvb_absorb_mma_kernel(KpArgs A) {
                 }
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                    *reinterpret_cast<uint4*>(smem + kp_stage(erow, c * 4 + e)) = make_uint4(o[4 * e], o[4 * e + 1], o[4 * e + 2], o[4 * e + 3]);
+                    *reinterpret_cast<uint4*>(sB + kp_stage(erow, c * 4 + e)) = make_uint4(o[4 * e], o[4 * e + 1], o[4 * e + 2], o[4 * e + 3]);
             }
         }
         tc::tc_fence_before();
         __syncthreads();
-        if (ok) kp_store_rows(smem, A.out + ((size_t)b0 * A.H + h) * W + iblk * 128, (size_t)A.H * W, min(128, A.B - b0));
+        if (ok) kp_store_rows(sB, A.out + ((size_t)b0 * A.H + h) * W + iblk * 128, (size_t)A.H * W, min(128, A.B - b0));
         __syncthreads();   // TMEM and the A tiles are free for the next batch tile
     }
     tc::cp_async_wait<0>();
@@ -296,8 +296,7 @@ kvb_value_mma_kernel(KpArgs A) {
             const int wb = c & 1;
             if (done[wb] > 0) ok = tc::mbar_wait_warp(&bar[wb], (done[wb] - 1) & 1, abort_flag, 73);
             if (!ok) break;
-            kp_wait_groups(nch - 1 - c);
-            __syncthreads();
+            kp_wait_groups(nch - 1 - c);   // (a thread converts the codes that it requested itself)
             uint8_t* sb = sB + wb * KP_CONV;
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
@@ -339,12 +338,12 @@ kvb_value_mma_kernel(KpArgs A) {
                     o[e >> 1] = (uint32_t)rv_f32_to_bf16(acc[e]) | ((uint32_t)rv_f32_to_bf16(acc[e + 1]) << 16);
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                    *reinterpret_cast<uint4*>(smem + kp_stage(erow, c * 4 + e)) = make_uint4(o[4 * e], o[4 * e + 1], o[4 * e + 2], o[4 * e + 3]);
+                    *reinterpret_cast<uint4*>(sB + kp_stage(erow, c * 4 + e)) = make_uint4(o[4 * e], o[4 * e + 1], o[4 * e + 2], o[4 * e + 3]);
             }
         }
         tc::tc_fence_before();
         __syncthreads();
-        if (ok) kp_store_rows(smem, A.out + ((size_t)b0 * A.H + h) * vh + jblk * 128, (size_t)A.H * vh, min(128, A.B - b0));
+        if (ok) kp_store_rows(sB, A.out + ((size_t)b0 * A.H + h) * vh + jblk * 128, (size_t)A.H * vh, min(128, A.B - b0));
         __syncthreads();
     }
     tc::cp_async_wait<0>();
