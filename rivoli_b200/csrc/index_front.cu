@@ -60,13 +60,15 @@ __global__ void rope_interleave_kernel(float* __restrict__ base, int stride, int
 // ---------------------------------------------------------------------------------------------
 // Batched front end.
 // ---------------------------------------------------------------------------------------------
-struct FrontJob {            // Y[b][o] (+)= sum over a K range of X[b][i] * W[o][i] * scale
+struct FrontMat { const uint8_t* w; const float* scale; int n; };   // weights e4m3 [n][K], block scales
+struct FrontJob {            // Y[b][o] = sum over a K range of X[b][i] * W[o][i] * scale
     const uint16_t* x; int K;                         // activations bf16 [B][K]
-    const uint8_t* w; const float* scale; int N;      // weights e4m3 [N][K], block scales
-    float* partial;                                   // f32 [k_splits][B][N]
-    int n_tiles, k_splits, cta0, tile_n;              // output tiles of tile_n columns, splits of the contraction, first CTA
+    FrontMat m[2]; int N;                             // the outputs are m[0]'s rows, then m[1]'s (n = 0: none); N = both
+    float* partial;                                   // f32 [k_splits][n_tiles][B][tile_n]
+    int n_tiles, k_splits, k_chunks, cta0, tile_n;    // output tiles of tile_n columns, splits of k_chunks x 64 values, first CTA
+    int mask;                                         // 16-byte pieces of a partial row are XORed with (row & mask)
 };
-struct FrontArgs { FrontJob job[3]; int B, block, n_cta; };
+struct FrontArgs { FrontJob job[3]; int n_jobs, B, block, n_cta; };
 
 // CUDA-core split-K GEMM: CTA = (job, 64-output tile, K split), 256 threads = 64 outputs x 4 sequence
 // groups; thread (o, g) folds its K range for sequences g, g + 4, ... (32 accumulators per pass of 128
@@ -77,14 +79,15 @@ __global__ void __launch_bounds__(256)
 front_gemm_simt_kernel(FrontArgs A) {
     __shared__ float ws[FT_KC][FT_N + 1];
     int jid = 0;
-    while (jid < 2 && (int)blockIdx.x >= A.job[jid + 1].cta0) ++jid;
+    while (jid < A.n_jobs - 1 && (int)blockIdx.x >= A.job[jid + 1].cta0) ++jid;
     const FrontJob& J = A.job[jid];
     const int local = blockIdx.x - J.cta0;
     const int tile = local % J.n_tiles, split = local / J.n_tiles;
-    const int kper = ((J.K + J.k_splits - 1) / J.k_splits + FT_KC - 1) / FT_KC * FT_KC;
-    const int k0 = split * kper, k1 = min(J.K, k0 + kper);
-    const int o = tile * FT_N + (threadIdx.x & 63), bq = threadIdx.x >> 6;   // this kernel always plans tile_n == FT_N
+    const int k0 = split * J.k_chunks * 64, k1 = min(J.K, k0 + J.k_chunks * 64);
+    const int bq = threadIdx.x >> 6;   // this kernel always plans tile_n == FT_N and one matrix per job
     const int bsh = rv_log2(A.block), sc_cols = (J.K + A.block - 1) / A.block;
+    rv_grid_dep_wait();
+    rv_grid_dep_trigger();
     // sequences bq, bq + 4, ... ; at most 32 accumulators per thread per pass
     for (int b0 = 0; b0 < A.B; b0 += 128) {
         float acc[32];
@@ -95,7 +98,7 @@ front_gemm_simt_kernel(FrontArgs A) {
             for (int e = threadIdx.x; e < FT_KC * FT_N; e += 256) {
                 const int kk = e % FT_KC, oo = e / FT_KC, i = kc + kk, og = tile * FT_N + oo;
                 float v = 0.0f;
-                if (i < k1 && og < J.N) v = __fmul_rn(rv_e4m3_to_f32(J.w[(size_t)og * J.K + i]), J.scale[(size_t)(og >> bsh) * sc_cols + (i >> bsh)]);
+                if (i < k1 && og < J.N) v = __fmul_rn(rv_e4m3_to_f32(J.m[0].w[(size_t)og * J.K + i]), J.m[0].scale[(size_t)(og >> bsh) * sc_cols + (i >> bsh)]);
                 ws[kk][oo] = v;
             }
             __syncthreads();
@@ -111,28 +114,34 @@ front_gemm_simt_kernel(FrontArgs A) {
                 }
             }
         }
-        if (o < J.N)
 #pragma unroll
-            for (int r = 0; r < 32; ++r) {
-                const int b = b0 + bq + 4 * r;
-                if (b < A.B) J.partial[((size_t)split * A.B + b) * J.N + o] = acc[r];
-            }
+        for (int r = 0; r < 32; ++r) {
+            const int b = b0 + bq + 4 * r;
+            if (b < A.B) J.partial[(((size_t)split * J.n_tiles + tile) * A.B + b) * FT_N + (threadIdx.x & 63)] = acc[r];
+        }
     }
 }
 
 
 // ---------------------------------------------------------------------------------------------
-// The same split-K GEMM on the tensor cores (tcgen05 kind::f16). CTA = (job, output tile, K split);
-// M = 128 sequences, N = the tile (128, or the whole of a narrower matrix), K fed in chunks of 64
-// through three shared-memory stages: activations and raw weight codes arrive by cp.async (two chunks requested
-// ahead), the codes of the current chunk are converted to bf16(code * block scale) (one rounding, 2^-9 relative; a 64-wide chunk of
-// a 128-aligned tile lies inside ONE scale block). The accumulator leaves as the f32 split partial.
+// The same split-K GEMM on the tensor cores (tcgen05 kind::f16). CTA = (job, output tile, K split), one per SM; M = 128
+// sequences, N = the tile (128, the whole of a narrower matrix, or the key and head-weight matrices together: they share
+// their activations, up to 160 columns), K in chunks of 64 through six shared-memory stages, all requested at once.
+// A thread converts the 16 codes that it requested itself to bf16(code * block scale) (one rounding, 2^-9 relative; a
+// 64-wide chunk of a 128-aligned tile lies inside ONE scale block), so a chunk takes one CTA barrier. The accumulator leaves
+// as the f32 split partial: staged in the idle stages, one bulk copy (a CTA's partial rows are contiguous).
+// Bound by what an SM takes in (192 KiB at 18 bytes a clock = 5.4 us at the 64-head model's sizes, activations being read by
+// 32 tiles) and the launch's ramp. 128 sequences: 19 us with three stages, two barriers a chunk and 16-byte stores to 32 rows
+// at a time, then 12.5 us for the epilogue below; 20.5 us together now (31.8).
 // ---------------------------------------------------------------------------------------------
-constexpr int FM_THREADS = 256, FM_WARPS = 8;
-constexpr int FM_NST = 3;                      // stages of (activations 16 KiB | raw weight codes 8 KiB) in flight
-constexpr int FM_STAGE = 16384 + 8192;
-constexpr int FM_BOFF = FM_NST * FM_STAGE;     // two converted weight tiles (bf16, 16 KiB each) follow the stages
-constexpr int FM_SMEM = FM_BOFF + 2 * 16384;   // 104 KiB: two CTAs per SM
+constexpr int FM_THREADS = 256;
+constexpr int FM_NMAX = 160;                                // widest tile
+constexpr int FM_NST = 6;                                   // stages of (activations 16 KiB | raw codes) in flight
+constexpr int FM_STAGE = 16384 + FM_NMAX * 64;
+constexpr int FM_BOFF = FM_NST * FM_STAGE;                  // two converted weight tiles (bf16) follow the stages
+constexpr int FM_SMEM = FM_BOFF + 2 * FM_NMAX * 128;
+static_assert(FM_BOFF % 1024 == 0 && FM_STAGE % 1024 == 0 && (FM_NMAX * 128) % 1024 == 0, "operand tiles are 1024-byte aligned");
+static_assert(128 * FM_NMAX * 4 <= FM_BOFF, "the partial fits the stages");
 
 __device__ __forceinline__ uint64_t fm_desc(uint32_t saddr) {     // K-major, 128-byte swizzle, 8-row groups 1024 B apart
     uint64_t d = 0;
@@ -159,97 +168,102 @@ front_gemm_mma_kernel(FrontArgs A) {
     volatile int* abort_flag = &abort_word;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int jid = 0;
-    while (jid < 2 && (int)blockIdx.x >= A.job[jid + 1].cta0) ++jid;
+    while (jid < A.n_jobs - 1 && (int)blockIdx.x >= A.job[jid + 1].cta0) ++jid;
     const FrontJob& J = A.job[jid];
     const int local = blockIdx.x - J.cta0;
     const int tile = local % J.n_tiles, split = local / J.n_tiles;
-    const int TN = J.tile_n;
-    const int kper = ((J.K + J.k_splits - 1) / J.k_splits + 127) / 128 * 128;
-    const int k0 = split * kper, k1 = min(J.K, k0 + kper);
-    const int nch = k1 > k0 ? (k1 - k0) / 64 : 0;
-    const int sc_cols = J.K / 128;
-    const float* srow = J.scale + (size_t)((tile * TN) >> 7) * sc_cols;
+    const int TN = J.tile_n, K = J.K, n0 = J.n_tiles > 1 ? TN : J.m[0].n;   // (columns of the tile from m[0])
+    const int k0 = split * J.k_chunks * 64, nch = min(J.k_chunks, K / 64 - split * J.k_chunks);
     if (tid == 0) { tc::mbar_init(&bar[0], 1); tc::mbar_init(&bar[1], 1); tc::mbar_init_fence(); abort_word = 0; }
-    if (warp == 0) tc::tmem_alloc<128>(&tmem_slot);
-    tc::tc_fence_before();
-    __syncthreads();
-    tc::tc_fence_after();
-    const uint32_t tmem = tmem_slot;
-    // instruction descriptor: bf16 x bf16 -> f32, both K-major, M = 128, N = TN
-    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-    const uint32_t lane_base = ((uint32_t)((warp & 3) * 32)) << 16;
-    const int erow = (warp & 3) * 32 + lane, chalf = warp >> 2;
+    if (warp == 0) tc::tmem_alloc<256>(&tmem_slot);
+    // the wait comes first: the epilogue kernel, started by the trigger, may then read inputs of this call before its own wait
+    rv_grid_dep_wait();
+    rv_grid_dep_trigger();
+    // this thread's weight pieces: row e / 4, codes 16 (e % 4) .. + 15 of each chunk
+    const uint8_t* pw[3];
+    uint32_t dw[3];
+    bool lw[3], second[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const int e = tid + i * FM_THREADS, row = e >> 2, j = e & 3;
+        lw[i] = row < TN;
+        second[i] = row >= n0;
+        const int r = lw[i] ? row : 0;
+        pw[i] = (r < n0 ? J.m[0].w + (size_t)(tile * TN + r) * K : J.m[1].w + (size_t)(r - n0) * K) + k0 + j * 16;
+        dw[i] = 16384 + row * 64 + j * 16;
+    }
+    const float* sc0 = J.m[0].scale + (size_t)(tile * TN / 128) * (K / 128);
+    const float* sc1 = J.m[1].n ? J.m[1].scale : sc0;
+    const uint32_t smem0 = tc::smem_u32(fm_smem);
     bool ok = true;
     int done[2] = {0, 0};                                   // commits issued per weight buffer so far
+    uint32_t tmem = 0;
+    // instruction descriptor: bf16 x bf16 -> f32, both K-major, M = 128, N = TN
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
     for (int b0 = 0; b0 < A.B && ok; b0 += 128) {
-        // request chunk c: activations (128 sequences x 64 bf16, swizzled K-major; rows past B are zeros) and
-        // the raw codes of TN weight rows x 64; one cp.async group per chunk, requested chunks or not
-        // per-thread copy plan, fixed for the batch tile: 4 activation rows and up to 2 weight rows per thread
-        const uint16_t* pa[4]; uint32_t da[4]; bool la[4];
+        const uint16_t* pa[4]; uint32_t da[4]; uint32_t la[4];   // 4 activation pieces a thread; rows past B are zeros
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int row = warp * 4 + i * FM_WARPS * 4 + (lane >> 3), j = lane & 7;
-            la[i] = b0 + row < A.B;
-            pa[i] = J.x + (size_t)(la[i] ? b0 + row : 0) * J.K + k0 + j * 8;
+            const int e = tid + i * FM_THREADS, row = e >> 3, j = e & 7;
+            la[i] = b0 + row < A.B ? 16u : 0u;
+            pa[i] = J.x + (size_t)(la[i] ? b0 + row : 0) * K + k0 + j * 8;
             da[i] = tc::sw128_chunk(row, j);
         }
-        const uint8_t* pw[2]; uint32_t dw[2]; bool lw[2];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int row = warp * 8 + i * FM_WARPS * 8 + (lane >> 2), j = lane & 3;
-            lw[i] = row < TN;
-            pw[i] = J.w + (size_t)(tile * TN + (lw[i] ? row : 0)) * J.K + k0 + j * 16;
-            dw[i] = 16384 + row * 64 + j * 16;
-        }
-        const uint32_t smem0 = tc::smem_u32(fm_smem);
-        auto request = [&](int c) {
+        auto request = [&](int c) {                          // one cp.async group per call, with or without a chunk
             if (c < nch) {
                 const uint32_t st = smem0 + (c % FM_NST) * FM_STAGE;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    if (la[i]) tc::cp_async16(st + da[i], pa[i] + c * 64);
-                    else *reinterpret_cast<uint4*>(fm_smem + (c % FM_NST) * FM_STAGE + da[i]) = make_uint4(0, 0, 0, 0);
-                }
-#pragma unroll
-                for (int i = 0; i < 2; ++i)
+                for (int i = 0; i < 3; ++i)
                     if (lw[i]) tc::cp_async16(st + dw[i], pw[i] + c * 64);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) tc::cp_async16_zfill(st + da[i], pa[i] + c * 64, la[i]);
             }
             tc::cp_async_commit();
         };
-        request(0);
-        request(1);
+#pragma unroll 1
+        for (int c = 0; c < FM_NST; ++c) request(c);
+        float s0 = sc0[k0 >> 7], s1 = sc1[k0 >> 7];
+        if (b0 == 0) {
+            tc::tc_fence_before();
+            __syncthreads();
+            tc::tc_fence_after();
+            tmem = tmem_slot;
+        }
         for (int c = 0; c < nch && ok; ++c) {
             const int wb = c & 1;
-            // stage (c + 2) % 3 was read by the MMAs of chunk c - 1, weight buffer wb by those of chunk c - 2
-            if (c >= 1) ok = tc::mbar_wait_warp(&bar[(c - 1) & 1], (done[(c - 1) & 1] - 1) & 1, abort_flag, 81);
+            // weight buffer wb and stage (c - 2) % 6 were read by the MMAs of chunk c - 2 (or of the batch tile before)
+            if (done[wb] > 0) ok = tc::mbar_wait_warp(&bar[wb], (done[wb] - 1) & 1, abort_flag, 81);
             if (!ok) break;
-            request(c + 2);
-            tc::cp_async_wait<2>();                          // chunk c has landed (two younger groups may be pending)
-            __syncthreads();
-            const uint8_t* sA = fm_smem + (c % FM_NST) * FM_STAGE;
-            const uint8_t* sW = sA + 16384;
-            uint8_t* sB = fm_smem + FM_BOFF + wb * 16384;
-            const float sc = srow[(k0 + c * 64) >> 7];
-            for (int r0 = warp * 4; r0 < TN; r0 += FM_WARPS * 4) {     // codes -> bf16(code * scale), swizzled K-major
-                const int row = r0 + (lane >> 3), j = lane & 7;
-                const uint2 cw = *reinterpret_cast<const uint2*>(sW + row * 64 + j * 8);
-                uint32_t o[4];
-                const uint32_t w2[2] = {cw.x, cw.y};
+            if (c >= 2) request(c - 2 + FM_NST);
+            if (c == 0) tc::cp_async_wait<5>(); else tc::cp_async_wait<4>();   // this thread's part of chunk c has landed
+            const float n0s = sc0[(k0 + min(c + 1, nch - 1) * 64) >> 7], n1s = sc1[(k0 + min(c + 1, nch - 1) * 64) >> 7];
+            uint8_t* st = fm_smem + (c % FM_NST) * FM_STAGE;
+            uint8_t* sB = fm_smem + FM_BOFF + wb * FM_NMAX * 128;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float2 f = rv_e4m3x2_to_f32x2((uint16_t)(w2[i >> 1] >> (16 * (i & 1))));
-                    const __nv_bfloat162 h = __floats2bfloat162_rn(f.x * sc, f.y * sc);   // finite values: plain RNE
-                    o[i] = *reinterpret_cast<const uint32_t*>(&h);
+            for (int i = 0; i < 3; ++i)
+                if (lw[i]) {
+                    const uint4 cw = *reinterpret_cast<const uint4*>(st + dw[i]);
+                    const float sc = second[i] ? s1 : s0;
+                    const uint32_t w4[4] = {cw.x, cw.y, cw.z, cw.w};
+                    uint32_t o[8];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const float2 f = rv_e4m3x2_to_f32x2((uint16_t)(w4[k >> 1] >> (16 * (k & 1))));
+                        const __nv_bfloat162 h = __floats2bfloat162_rn(f.x * sc, f.y * sc);   // finite values: plain RNE
+                        o[k] = *reinterpret_cast<const uint32_t*>(&h);
+                    }
+                    const int e = tid + i * FM_THREADS, row = e >> 2, j = e & 3;
+                    *reinterpret_cast<uint4*>(sB + tc::sw128_chunk(row, 2 * j)) = make_uint4(o[0], o[1], o[2], o[3]);
+                    *reinterpret_cast<uint4*>(sB + tc::sw128_chunk(row, 2 * j + 1)) = make_uint4(o[4], o[5], o[6], o[7]);
                 }
-                *reinterpret_cast<uint4*>(sB + tc::sw128_chunk(row, j)) = make_uint4(o[0], o[1], o[2], o[3]);
-            }
+            s0 = n0s; s1 = n1s;
             tc::fence_proxy_async();
             __syncthreads();
             if (tid == 0) {
                 tc::tc_fence_after();
-                const uint64_t da0 = fm_desc(tc::smem_u32(sA)), db0 = fm_desc(tc::smem_u32(sB));
+                const uint64_t d_a = fm_desc(tc::smem_u32(st)), d_b = fm_desc(tc::smem_u32(sB));
 #pragma unroll
-                for (int k = 0; k < 4; ++k) fm_mma(tmem, da0 + 2 * k, db0 + 2 * k, idesc, (c | k) ? 1u : 0u);   // +32 bytes = +2 in the address field
+                for (int k = 0; k < 4; ++k) fm_mma(tmem, d_a + 2 * k, d_b + 2 * k, idesc, (c | k) ? 1u : 0u);   // +32 bytes = +2 in the address field
                 tc::mma_commit(&bar[wb]);
             }
             ++done[wb];
@@ -259,142 +273,150 @@ front_gemm_mma_kernel(FrontArgs A) {
         for (int st = 0; st < 2 && ok; ++st)
             if (done[st] > 0) ok = tc::mbar_wait_warp(&bar[st], (done[st] - 1) & 1, abort_flag, 83 + st);
         tc::tc_fence_after();
-        if (ok && nch > 0) {
-            const int ncol_chunks = TN / 32;                 // 32-column chunks; warps 0-3 take the even ones, 4-7 the odd
-            for (int c = chalf; c < ncol_chunks; c += 2) {
-                uint32_t r[32];
-                tc::tmem_ld32(tmem + lane_base + c * 32, r);
+        if (ok) {
+            const int row = (warp & 3) * 32 + lane;
+            for (int c = warp >> 2; c < TN / 16; c += 2) {   // 16-column chunks; warps 0-3 take the even ones, 4-7 the odd
+                uint32_t r[16];
+                tc::tmem_ld16(tmem + (((uint32_t)((warp & 3) * 32)) << 16) + c * 16, r);
                 tc::tmem_ld_wait();
-                if (b0 + erow < A.B) {
-                    float4* dst = reinterpret_cast<float4*>(J.partial + ((size_t)split * A.B + b0 + erow) * J.N + tile * TN + c * 32);
 #pragma unroll
-                    for (int e = 0; e < 8; ++e)
-                        dst[e] = make_float4(__uint_as_float(r[4 * e]), __uint_as_float(r[4 * e + 1]), __uint_as_float(r[4 * e + 2]),
-                                             __uint_as_float(r[4 * e + 3]));
-                }
-            }
-        } else if (ok) {                                     // an empty K range (more splits than 128-blocks): zeros
-            for (int e = tid; e < 128 * TN; e += FM_THREADS) {
-                const int row = e / TN, col = e - row * TN;
-                if (b0 + row < A.B) J.partial[((size_t)split * A.B + b0 + row) * J.N + tile * TN + col] = 0.0f;
+                for (int e = 0; e < 4; ++e)
+                    *reinterpret_cast<uint4*>(fm_smem + row * TN * 4 + (((c * 4 + e) ^ (row & J.mask)) << 4)) =
+                        make_uint4(r[4 * e], r[4 * e + 1], r[4 * e + 2], r[4 * e + 3]);
             }
         }
+        tc::fence_proxy_async();
         tc::tc_fence_before();
         __syncthreads();
+        if (ok && tid == 0) {
+            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+                         ::"l"(J.partial + (((size_t)split * J.n_tiles + tile) * A.B + b0) * TN), "r"(smem0), "r"(min(128, A.B - b0) * TN * 4) : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        }
+        if (b0 + 128 < A.B) __syncthreads();                 // the stages are free for the next batch tile
     }
-    if (warp == 0) tc::tmem_dealloc<128>(tmem);
+    if (warp == 0) tc::tmem_dealloc<256>(tmem_slot);
     if (tid == 0 && abort_word) atomicCAS(&g_front_err, 0, abort_word);
 }
 
+struct EpiPart {             // where the split partials of some outputs lie
+    const float* p; int splits, n_tiles, tile_n, col0, mask;
+    __device__ __forceinline__ const float* at(int s, int B, int b, int n) const {   // split s, output n (a float4 may be read where n % 4 == 0)
+        n += col0;
+        const int tile = n / tile_n, c = n - tile * tile_n;
+        return p + (((size_t)s * n_tiles + tile) * B + b) * tile_n + ((((c >> 2) ^ (b & mask)) << 2) | (c & 3));
+    }
+};
 struct EpiArgs {
-    const float* pk; const float* pq; const float* pw;   // partials [splits][B][N]
-    int sk, sq, sw;                                       // split counts
+    EpiPart k, q, w;
     const float* kn_w; const float* kn_b; const int32_t* pos;
     int B, nh, hd, rope_off, rope_seg; double theta; float eps;
     uint16_t* index_key; uint16_t* index_q; float* index_w;
 };
 
-// One CTA per sequence: reduce the split partials in split order, LayerNorm the key, rotate key and
-// queries at the sequence's position, store bf16 (and the f32 head weights). The rotation angles depend
-// only on (position, pair index): rope_seg / 2 (cos, sin) pairs are computed once in f64 and shared by
-// all index_heads + 1 vectors.
-__global__ void __launch_bounds__(256)
+// One CTA per sequence: reduce the split partials in split order, LayerNorm the key, rotate key and queries at the
+// sequence's position, store bf16 (and the f32 head weights). Eight warps fold the queries, four the key and the weights meanwhile (a CTA of this size fits beside one of the GEMM's, so
+// its f64 work is done before the GEMM ends). The rotation angles depend only on (position, pair index): rope_seg / 2 (cos, sin) pairs are computed once in
+// f64, while the GEMM still runs.
+constexpr int FE_Q = 256, FE_K = 128, FE_THREADS = FE_Q + FE_K;
+__global__ void __launch_bounds__(FE_THREADS)
 front_epilogue_kernel(EpiArgs A) {
-    extern __shared__ float fe_smem[];          // (nh + 1) * hd values: queries then key
-    __shared__ double ss[256], sq[256];
+    extern __shared__ __align__(16) float fe_smem[];          // (nh + 1) * hd values: queries then key
+    __shared__ double s_red[2][FE_K / 32];
     __shared__ float s_cs[512], s_sn[512];
     const int b = blockIdx.x, t = threadIdx.x, nh = A.nh, hd = A.hd;
-    float* qv = fe_smem;
     float* kv = fe_smem + (size_t)nh * hd;
+    rv_grid_dep_trigger();
     const int half = A.rope_seg / 2, pos = A.pos[b];
-    for (int j = t; j < half; j += 256) {
+    for (int j = t; j < half; j += FE_THREADS) {
         const double ang = (double)pos * pow(A.theta, -2.0 * (double)j / (double)A.rope_seg);
         s_cs[j] = (float)cos(ang); s_sn[j] = (float)sin(ang);
     }
-    const int nq4 = nh * hd / 4;                 // index_dim is a multiple of 4 (checked by the launcher)
-    for (int e0 = t; e0 < nq4; e0 += 256 * 4) {      // four elements x up to eight splits of loads in flight per thread
-        float4 a[4];
+    rv_grid_dep_wait();
+    if (t < FE_Q) {
+        const int nq4 = nh * hd / 4;                 // index_dim is a multiple of 4 (checked by the launcher)
+        for (int e0 = t; e0 < nq4; e0 += FE_Q * 2) {     // two elements x four splits of loads in flight per thread
+            float4 a[2];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) a[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int s0 = 0; s0 < A.sq; s0 += 8) {
-            float4 p[4][8];
+            for (int u = 0; u < 2; ++u) a[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int s0 = 0; s0 < A.q.splits; s0 += 4) {
+                float4 p[2][4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
+                for (int u = 0; u < 2; ++u)
 #pragma unroll
-                for (int s = 0; s < 8; ++s) {
-                    const int e = e0 + u * 256;
-                    p[u][s] = (e < nq4 && s0 + s < A.sq)
-                                  ? *reinterpret_cast<const float4*>(A.pq + ((size_t)(s0 + s) * A.B + b) * nh * hd + e * 4)
-                                  : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int s = 0; s < 8; ++s)
-                    if (s0 + s < A.sq) {            // split order; the guard keeps "+ 0" out of the fold
-                        a[u].x = __fadd_rn(a[u].x, p[u][s].x); a[u].y = __fadd_rn(a[u].y, p[u][s].y);
-                        a[u].z = __fadd_rn(a[u].z, p[u][s].z); a[u].w = __fadd_rn(a[u].w, p[u][s].w);
+                    for (int s = 0; s < 4; ++s) {
+                        const int e = e0 + u * FE_Q;
+                        p[u][s] = (e < nq4 && s0 + s < A.q.splits) ? *reinterpret_cast<const float4*>(A.q.at(s0 + s, A.B, b, e * 4))
+                                                                   : make_float4(0.f, 0.f, 0.f, 0.f);
                     }
+#pragma unroll
+                for (int u = 0; u < 2; ++u)
+#pragma unroll
+                    for (int s = 0; s < 4; ++s)
+                        if (s0 + s < A.q.splits) {            // split order; the guard keeps "+ 0" out of the fold
+                            a[u].x = __fadd_rn(a[u].x, p[u][s].x); a[u].y = __fadd_rn(a[u].y, p[u][s].y);
+                            a[u].z = __fadd_rn(a[u].z, p[u][s].z); a[u].w = __fadd_rn(a[u].w, p[u][s].w);
+                        }
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                if (e0 + u * FE_Q < nq4) *reinterpret_cast<float4*>(fe_smem + (e0 + u * FE_Q) * 4) = a[u];
+        }
+    } else {
+        const int kt = t - FE_Q, lane = t & 31, kw = kt >> 5;
+        auto fold = [&](const EpiPart& P, int n) {       // sixteen loads in flight, folded in split order
+            float a = 0.0f;
+            for (int s0 = 0; s0 < P.splits; s0 += 16) {
+                float p[16];
+#pragma unroll
+                for (int s = 0; s < 16; ++s) p[s] = s0 + s < P.splits ? *P.at(s0 + s, A.B, b, n) : 0.0f;
+#pragma unroll
+                for (int s = 0; s < 16; ++s)
+                    if (s0 + s < P.splits) a = __fadd_rn(a, p[s]);
+            }
+            return a;
+        };
+        double s1 = 0.0, s2 = 0.0;
+        for (int e = kt; e < hd; e += FE_K) {
+            const float a = fold(A.k, e);
+            kv[e] = a;
+            s1 += (double)a; s2 += (double)a * (double)a;
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (e0 + u * 256 < nq4) *reinterpret_cast<float4*>(qv + (e0 + u * 256) * 4) = a[u];
+        for (int o = 16; o > 0; o >>= 1) { s1 += __shfl_xor_sync(0xffffffffu, s1, o); s2 += __shfl_xor_sync(0xffffffffu, s2, o); }
+        if (lane == 0) { s_red[0][kw] = s1; s_red[1][kw] = s2; }
+        tc::named_barrier(1, FE_K);
+        s1 = s2 = 0.0;
+#pragma unroll
+        for (int i = 0; i < FE_K / 32; ++i) { s1 += s_red[0][i]; s2 += s_red[1][i]; }
+        const float mean = (float)(s1 / (double)hd);
+        const float var = __fsub_rn((float)(s2 / (double)hd), __fmul_rn(mean, mean));
+        const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(var, A.eps)));
+        for (int e = kt; e < hd; e += FE_K)
+            kv[e] = __fadd_rn(__fmul_rn(__fmul_rn(__fsub_rn(kv[e], mean), inv), A.kn_w[e]), A.kn_b[e]);
+        for (int h = kt; h < nh; h += FE_K) A.index_w[(size_t)b * nh + h] = fold(A.w, h);
     }
-    double s1 = 0.0, s2 = 0.0;
-    for (int e = t; e < hd; e += 256) {
-        float a = 0.0f;
-        for (int s0 = 0; s0 < A.sk; s0 += 8) {       // eight loads in flight, folded in split order
-            float p[8];
-#pragma unroll
-            for (int s = 0; s < 8; ++s) p[s] = s0 + s < A.sk ? A.pk[((size_t)(s0 + s) * A.B + b) * hd + e] : 0.0f;
-#pragma unroll
-            for (int s = 0; s < 8; ++s)
-                if (s0 + s < A.sk) a = __fadd_rn(a, p[s]);
+    __syncthreads();
+    // output i of a vector: rotated pairs inside [rope_off, rope_off + rope_seg), the value itself elsewhere
+    auto value = [&](const float* v, int i) {
+        const int r = i - A.rope_off;
+        if (r < 0 || r >= A.rope_seg) return v[i];
+        const int j = r < half ? r : r - half;
+        const float a = v[A.rope_off + 2 * j], c = v[A.rope_off + 2 * j + 1];
+        return r < half ? __fsub_rn(__fmul_rn(a, s_cs[j]), __fmul_rn(c, s_sn[j])) : __fadd_rn(__fmul_rn(c, s_cs[j]), __fmul_rn(a, s_sn[j]));
+    };
+    for (int p = t; p < (nh + 1) * (hd / 2); p += FE_THREADS) {
+        const int vec = p / (hd / 2), i = 2 * (p - vec * (hd / 2));
+        const float* v = fe_smem + (size_t)vec * hd;
+        const uint16_t x = rv_f32_to_bf16(value(v, i)), y = rv_f32_to_bf16(value(v, i + 1));
+        if (vec < nh) {
+            *reinterpret_cast<uint32_t*>(A.index_q + ((size_t)b * nh + vec) * hd + i) = (uint32_t)x | ((uint32_t)y << 16);
+        } else {
+            A.index_key[(size_t)b * hd + i] = x;
+            A.index_key[(size_t)b * hd + i + 1] = y;
         }
-        kv[e] = a;
-        s1 += (double)a; s2 += (double)a * (double)a;
     }
-    if (t < nh) {
-        float a = 0.0f;
-        for (int s = 0; s < A.sw; ++s) a = __fadd_rn(a, A.pw[((size_t)s * A.B + b) * nh + t]);
-        A.index_w[(size_t)b * nh + t] = a;
-    }
-    ss[t] = s1; sq[t] = s2;
-    __syncthreads();
-    for (int st = 128; st > 0; st >>= 1) {
-        if (t < st) { ss[t] += ss[t + st]; sq[t] += sq[t + st]; }
-        __syncthreads();
-    }
-    const float mean = (float)(ss[0] / (double)hd);
-    const float var = __fsub_rn((float)(sq[0] / (double)hd), __fmul_rn(mean, mean));
-    const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(var, A.eps)));
-    for (int e = t; e < hd; e += 256)
-        kv[e] = __fadd_rn(__fmul_rn(__fmul_rn(__fsub_rn(kv[e], mean), inv), A.kn_w[e]), A.kn_b[e]);
-    __syncthreads();
-    // rotation: (nh + 1) segments of rope_seg at rope_off; every pair is read into registers before any write
-    const int npairs = (nh + 1) * half;
-    float lo[8], hi[8];
-    int cnt = 0;
-    for (int p = t; p < npairs && cnt < 8; p += 256, ++cnt) {
-        const int seg = p / half, j = p - seg * half;
-        const float* v = fe_smem + (size_t)seg * hd + A.rope_off;
-        const float a = v[2 * j], c = v[2 * j + 1], cs = s_cs[j], sn = s_sn[j];
-        lo[cnt] = __fsub_rn(__fmul_rn(a, cs), __fmul_rn(c, sn));
-        hi[cnt] = __fadd_rn(__fmul_rn(c, cs), __fmul_rn(a, sn));
-    }
-    __syncthreads();
-    cnt = 0;
-    for (int p = t; p < npairs && cnt < 8; p += 256, ++cnt) {
-        const int seg = p / half, j = p - seg * half;
-        float* v = fe_smem + (size_t)seg * hd + A.rope_off;
-        v[j] = lo[cnt]; v[half + j] = hi[cnt];
-    }
-    __syncthreads();
-    for (int e = t; e < nh * hd / 2; e += 256) {   // two values per 32-bit store
-        const uint32_t w2 = (uint32_t)rv_f32_to_bf16(qv[2 * e]) | ((uint32_t)rv_f32_to_bf16(qv[2 * e + 1]) << 16);
-        reinterpret_cast<uint32_t*>(A.index_q + (size_t)b * nh * hd)[e] = w2;
-    }
-    for (int e = t; e < hd; e += 256) A.index_key[(size_t)b * hd + e] = rv_f32_to_bf16(kv[e]);
 }
 
 int ceil_div(int a, int b) { return (a + b - 1) / b; }
@@ -446,37 +468,60 @@ static bool front_mma_ok(const IndexFrontGeom* g) {
     return true;
 }
 
+// The jobs of a call and the floats of their partials. Tensor cores: the key and head-weight matrices share their activations
+// and take one tile where that is at most FM_NMAX wide; the split is the chunk count L with the shortest critical path, waves x
+// (L + 4), a launch's ramp and a partial's way out counting as four chunks. CUDA cores: enough CTAs to fill the machine, at
+// least 256 contraction values per split, at most 32 splits.
 static void plan_jobs(const IndexFrontGeom* g, int B, bool mma, FrontArgs* fa, size_t* floats) {
     const int N[3] = {g->index_dim, g->index_heads * g->index_dim, g->index_heads};
     const int K[3] = {g->hidden, g->q_lora, g->hidden};
-    int cta = 0;
-    size_t off = 0;
-    for (int j = 0; j < 3; ++j) {
+    const bool joint = mma && N[0] <= 128 && N[0] + N[2] <= FM_NMAX;
+    fa->n_jobs = joint ? 2 : 3; fa->B = B; fa->block = g->block;
+    for (int j = 0; j < fa->n_jobs; ++j) {
         FrontJob& J = fa->job[j];
-        J.N = N[j]; J.K = K[j];
-        J.tile_n = mma ? (N[j] < 128 ? N[j] : 128) : FT_N;
-        J.n_tiles = ceil_div(N[j], J.tile_n);
-        // enough CTAs to fill the machine, at least 256 contraction values per split, at most 32 splits
+        J.m[0].n = N[j]; J.m[1].n = joint && j == 0 ? N[2] : 0;
+        J.N = J.m[0].n + J.m[1].n; J.K = K[j];
+        J.tile_n = !mma ? FT_N : (J.N <= 128 || J.m[1].n ? J.N : 128);
+        J.n_tiles = ceil_div(J.N, J.tile_n);
+        J.mask = !mma ? 0 : (J.tile_n % 32 == 0 ? 7 : 3);
         int splits = ceil_div(296, J.n_tiles * 3);
         if (splits > K[j] / 256) splits = K[j] / 256;
         if (splits > 32) splits = 32;
         if (splits < 1) splits = 1;
-        J.k_splits = splits;
-        J.cta0 = cta;
-        cta += J.n_tiles * splits;
-        J.partial = reinterpret_cast<float*>(off);   // offset for now, rebased by the caller
-        off += (size_t)splits * B * N[j];
+        J.k_chunks = ceil_div(ceil_div(K[j], splits), 128) * 2;
     }
-    fa->n_cta = cta; fa->B = B; fa->block = g->block;
+    if (mma) {
+        long long best = -1;
+        int pick = 2;
+        for (int L = 2; L <= 64; ++L) {
+            long long ctas = 0;
+            for (int j = 0; j < fa->n_jobs; ++j) ctas += (long long)fa->job[j].n_tiles * ceil_div(fa->job[j].K / 64, L);
+            const long long cost = (ctas + 147) / 148 * (L + 4);
+            if (best < 0 || cost < best) { best = cost; pick = L; }
+        }
+        for (int j = 0; j < fa->n_jobs; ++j) fa->job[j].k_chunks = pick;
+    }
+    int cta = 0;
+    size_t off = 0;
+    for (int j = 0; j < fa->n_jobs; ++j) {
+        FrontJob& J = fa->job[j];
+        J.k_splits = ceil_div(ceil_div(J.K, 64), J.k_chunks);
+        J.cta0 = cta;
+        cta += J.n_tiles * J.k_splits;
+        J.partial = reinterpret_cast<float*>(off);   // offset for now, rebased by the caller
+        off += (size_t)J.k_splits * J.n_tiles * B * J.tile_n;
+    }
+    fa->n_cta = cta;
     *floats = off;
 }
 
 RIVOLI_API size_t rivoli_index_frontend_scratch_bytes(const IndexFrontGeom* g, int B) {
     if (!g || B <= 0) return 0;
     FrontArgs fa;
-    size_t floats = 0;
-    plan_jobs(g, B, front_mma_ok(g), &fa, &floats);   // the split count does not depend on the path
-    return floats * sizeof(float);
+    size_t simt = 0, mma = 0;                        // a call may take either path
+    plan_jobs(g, B, false, &fa, &simt);
+    if (front_mma_ok(g)) plan_jobs(g, B, true, &fa, &mma);
+    return (simt > mma ? simt : mma) * sizeof(float);
 }
 
 RIVOLI_API int rivoli_index_frontend_bf16(const IndexFrontGeom* g, const uint16_t* x, const uint16_t* q_resid,
@@ -501,26 +546,29 @@ RIVOLI_API int rivoli_index_frontend_bf16(const IndexFrontGeom* g, const uint16_
     plan_jobs(g, B, mma, &fa, &floats);
     float* base = static_cast<float*>(scratch);
     const uint16_t* xs[3] = {x, q_resid, x};
-    const unsigned char* ws[3] = {wk, wq_b, wproj};
-    const float* ss[3] = {wk_scale, wq_b_scale, wproj_scale};
-    for (int j = 0; j < 3; ++j) {
-        fa.job[j].x = xs[j]; fa.job[j].w = ws[j]; fa.job[j].scale = ss[j];
+    const FrontMat mats[3] = {{wk, wk_scale, g->index_dim}, {wq_b, wq_b_scale, g->index_heads * g->index_dim}, {wproj, wproj_scale, g->index_heads}};
+    for (int j = 0; j < fa.n_jobs; ++j) {
+        fa.job[j].x = xs[j]; fa.job[j].m[0] = mats[j];
+        if (fa.job[j].m[1].n) fa.job[j].m[1] = mats[2];
         fa.job[j].partial = base + reinterpret_cast<size_t>(fa.job[j].partial);
     }
     rv_drain_error();
     if (mma) {
-        cudaFuncSetAttribute(front_gemm_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FM_SMEM);
-        front_gemm_mma_kernel<<<fa.n_cta, FM_THREADS, FM_SMEM, st>>>(fa);
+        rv_allow_smem<front_gemm_mma_kernel>(FM_SMEM);
+        rv_launch_dependent(front_gemm_mma_kernel, dim3((unsigned)fa.n_cta), dim3(FM_THREADS), (size_t)FM_SMEM, st, fa);
     } else {
-        front_gemm_simt_kernel<<<fa.n_cta, 256, 0, st>>>(fa);
+        rv_launch_dependent(front_gemm_simt_kernel, dim3((unsigned)fa.n_cta), dim3(256), 0, st, fa);
     }
     if (int e = rv_launch_status()) return e;
-    EpiArgs ea{fa.job[0].partial, fa.job[1].partial, fa.job[2].partial, fa.job[0].k_splits, fa.job[1].k_splits,
-               fa.job[2].k_splits, knorm_w, knorm_b, pos, B, g->index_heads, g->index_dim, g->rope_off, g->rope_seg,
-               g->theta, g->eps, index_key, index_q, index_w};
+    auto part = [&](int j, int col0) {
+        const FrontJob& J = fa.job[j];
+        return EpiPart{J.partial, J.k_splits, J.n_tiles, J.tile_n, col0, J.mask};
+    };
+    EpiArgs ea{part(0, 0), part(1, 0), fa.n_jobs == 3 ? part(2, 0) : part(0, g->index_dim), knorm_w, knorm_b, pos, B, g->index_heads,
+               g->index_dim, g->rope_off, g->rope_seg, g->theta, g->eps, index_key, index_q, index_w};
     const size_t smem = (size_t)(g->index_heads + 1) * g->index_dim * sizeof(float);
-    cudaFuncSetAttribute(front_epilogue_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    front_epilogue_kernel<<<B, 256, smem, st>>>(ea);
+    rv_allow_smem<front_epilogue_kernel>(200 * 1024);
+    rv_launch_dependent(front_epilogue_kernel, dim3((unsigned)B), dim3(FE_THREADS), smem, st, ea);
     return rv_launch_status();
 }
 
