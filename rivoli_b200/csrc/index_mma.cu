@@ -253,8 +253,8 @@ index_score_mma_kernel(IndexMmaArgs A, const __grid_constant__ CUtensorMap tm_ke
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = tmem_base_s;
-    rv_grid_dep_trigger();   // the selection kernel may be scheduled; it waits for this grid before reading scores
     rv_grid_dep_wait();      // query codes, head scales and this step's appended keys come from the kernel before
+    rv_grid_dep_trigger();   // the selection kernel may start (after the wait: it reads all but the scores at once)
 
     const int tpi = A.tpi;
     const int max_tiles = (A.score_stride + IM_TILE - 1) / IM_TILE;
@@ -415,7 +415,7 @@ SelectScratch carve(const DsaGeom* g, int B, int score_stride, void* scratch, si
     return s;
 }
 
-constexpr int SEL_MAX_NT = 8 * 512 * 32;   // what one cluster of the selection kernel covers
+constexpr int SEL_MAX_NT = 8 * 16384;   // what one cluster of the selection kernel covers
 
 bool mma_geometry_ok(const DsaGeom* g, int score_stride) {
     return g->index_dim == IM_HD && g->index_heads <= IM_NPAD && g->page_tokens >= 16 && g->page_tokens <= IM_TILE &&

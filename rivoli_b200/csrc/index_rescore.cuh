@@ -2,101 +2,102 @@
 //   cd = left fold over d of qcode[h][d] * kcode[t][d]   (each product of two e4m3 values is exact in f32, so the fused
 //        multiply-add IS the reference's acc + q * k: crates/engine/tests/indexer_kernel.rs:237-249)
 //   dot = (cd * s_q[h]) * s_k[t];  term_h = (w[h] * wscale) * max(dot * dscale, 0);  score = fold over h ascending.
-// A warp takes TOK tokens per pass (their loads are in flight together and they share the decoded q values), lane = head
-// (index_heads <= 32), index_dim = 128 (one 4-code word per lane).
+// A warp takes four consecutive listed tokens per pass (their loads are in flight together and they share the q values), lane =
+// head (index_heads <= 32), index_dim = 128 (one 4-code word per lane). Two tokens ride in one packed f32x2 multiply-add, each
+// half rounded as the scalar one is; with the tokens of a dim side by side and q as (q, q) pairs that is two multiply-adds and
+// two shared-memory loads per dim for four tokens, half of what scalar folds that decoded q on the fly issued.
 #pragma once
-
-#include <type_traits>
 
 #include "codec.cuh"
 #include "common.cuh"
 
 constexpr int RS_HD = 128;
 
-// q codes of one sequence, PACKED as they lie in memory (word w of head h = its dims 4w .. 4w+3), transposed to
-// [word][head] in shared memory (lane = head on both sides: no bank conflicts). qf holds (RS_HD / 4) * 32 words. The fold
-// decodes a word into its four f32 values on the fly (exactly: every e4m3 value is an f32): one shared-memory load per
-// four dims instead of four. All threads of the CTA call it; the caller synchronises afterwards.
-__device__ __forceinline__ void rv_rescore_stage_q(const uint8_t* __restrict__ qcodes_seq, int nh, uint32_t* qf) {
+// q of one sequence as (q, q) pairs, [dim][head] (lane = head: no bank conflicts); RS_HD * 32 of them, zero for absent heads.
+// All threads of the CTA call it; the caller synchronises afterwards.
+__device__ __forceinline__ void rv_rescore_stage_q(const uint8_t* __restrict__ qcodes_seq, int nh, float2* qq) {
     for (int e = threadIdx.x; e < 32 * (RS_HD / 4); e += blockDim.x) {
-        const int h = e & 31, d4 = e >> 5;
-        qf[d4 * 32 + h] = h < nh ? *reinterpret_cast<const uint32_t*>(qcodes_seq + (size_t)h * RS_HD + d4 * 4) : 0u;
+        const int h = e & 31, d = (e >> 5) * 4;
+        const uint32_t c = h < nh ? *reinterpret_cast<const uint32_t*>(qcodes_seq + (size_t)h * RS_HD + d) : 0u;
+        const float2 x = rv_e4m3x2_to_f32x2((uint16_t)(c & 0xffff)), y = rv_e4m3x2_to_f32x2((uint16_t)(c >> 16));
+        qq[d * 32 + h] = make_float2(x.x, x.x);
+        qq[(d + 1) * 32 + h] = make_float2(x.y, x.y);
+        qq[(d + 2) * 32 + h] = make_float2(y.x, y.x);
+        qq[(d + 3) * 32 + h] = make_float2(y.y, y.y);
     }
 }
 
-// Scores the tokens toks[0 .. ln): a pass covers WARPS * TOK of them, warp w taking positions base + w, base + WARPS + w, ...
-// kf = this WARP's staging of TOK key rows as f32 (TOK * RS_HD floats). my_sq / my_wh = this lane's head scale and
-// weight * wscale (0 for lanes >= nh). emit(position, score) is called by one lane per token.
-template <int WARPS, int TOK, class Emit>
-__device__ __forceinline__ void rv_rescore_listed(const uint32_t* toks, uint32_t ln, const uint32_t* qf, float* kf,
+__device__ __forceinline__ uint64_t rs_fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// Scores the tokens toks[0 .. ln): a pass covers WARPS * 4 of them, warp w taking positions base + 4 w .. + 3.
+// kf = this WARP's staging of four key rows as f32, [dim][token] (RS_HD * 4 floats, 16-byte aligned). my_sq / my_wh = this
+// lane's head scale and weight * wscale (0 for lanes >= nh). emit(position, score) is called by one lane per token.
+template <int WARPS, class Emit>
+__device__ __forceinline__ void rv_rescore_listed(const uint32_t* toks, uint32_t ln, const float2* qq, float* kf,
                                                   const int32_t* __restrict__ bt, const DsaGeom& g,
                                                   const uint8_t* __restrict__ index_pool,
                                                   const float* __restrict__ index_scale, float my_sq, float my_wh,
                                                   Emit emit) {
-    static_assert(TOK <= 4, "the fold below is specialised for up to four tokens");
-    constexpr int hd = RS_HD;
+    constexpr int TOK = 4, PAD = 36;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nh = g.index_heads, P = g.page_tokens;
-    for (uint32_t base = 0; base < ln; base += WARPS * TOK) {
-        if (base + warp >= ln) break;
-        const int n_here = min(TOK, (int)((ln - base - warp + WARPS - 1) / WARPS));   // warp-uniform, >= 1
+    const int pshift = 31 - __clz(g.page_tokens);          // page sizes are powers of two
+#pragma unroll 1
+    for (uint32_t p0 = warp * TOK; p0 < ln; p0 += WARPS * TOK) {
+        const int n_here = min(TOK, (int)(ln - p0));
         uint32_t cw[TOK];
         float skv[TOK];
 #pragma unroll
         for (int e = 0; e < TOK; ++e) {
             cw[e] = 0u; skv[e] = 0.0f;
             if (e < n_here) {
-                const int t = (int)toks[base + e * WARPS + warp];
-                int pg = bt[t / P];
+                const int t = (int)toks[p0 + e];
+                int pg = bt[t >> pshift];
                 pg = (pg < 0 || pg >= g.n_pool_pages) ? 0 : pg;
-                const size_t rr = (size_t)pg * P + (t & (P - 1));
-                cw[e] = *reinterpret_cast<const uint32_t*>(index_pool + rr * hd + lane * 4);
+                const size_t rr = ((size_t)pg << pshift) + (t & (g.page_tokens - 1));
+                cw[e] = *reinterpret_cast<const uint32_t*>(index_pool + rr * RS_HD + lane * 4);
                 skv[e] = index_scale[rr];
             }
         }
+        float2 lo[TOK], hi[TOK];
 #pragma unroll
-        for (int e = 0; e < TOK; ++e) {
-            const float2 x = rv_e4m3x2_to_f32x2((uint16_t)(cw[e] & 0xffff)), y = rv_e4m3x2_to_f32x2((uint16_t)(cw[e] >> 16));
-            *reinterpret_cast<float4*>(kf + e * hd + lane * 4) = make_float4(x.x, x.y, y.x, y.y);
-        }
+        for (int e = 0; e < TOK; ++e) { lo[e] = rv_e4m3x2_to_f32x2((uint16_t)(cw[e] & 0xffff)); hi[e] = rv_e4m3x2_to_f32x2((uint16_t)(cw[e] >> 16)); }
+        float4* dst = reinterpret_cast<float4*>(kf) + lane * 4;
+        dst[0] = make_float4(lo[0].x, lo[1].x, lo[2].x, lo[3].x);
+        dst[1] = make_float4(lo[0].y, lo[1].y, lo[2].y, lo[3].y);
+        dst[2] = make_float4(hi[0].x, hi[1].x, hi[2].x, hi[3].x);
+        dst[3] = make_float4(hi[0].y, hi[1].y, hi[2].y, hi[3].y);
         __syncwarp();
-        float cd[TOK];
-#pragma unroll
-        for (int e = 0; e < TOK; ++e) cd[e] = 0.0f;
-        auto fold = [&](auto ntok) {
-            constexpr int NT = decltype(ntok)::value < TOK ? decltype(ntok)::value : TOK;
-#pragma unroll 4
-            for (int d = 0; d < hd; d += 4) {
-                const uint32_t qc = qf[(d >> 2) * 32 + lane];
-                const float2 qlo = rv_e4m3x2_to_f32x2((uint16_t)(qc & 0xffff)), qhi = rv_e4m3x2_to_f32x2((uint16_t)(qc >> 16));
-                const float q0f = qlo.x, q1f = qlo.y, q2f = qhi.x, q3f = qhi.y;
-#pragma unroll
-                for (int e = 0; e < NT; ++e) {
-                    const float4 k4 = *reinterpret_cast<const float4*>(kf + e * hd + d);   // broadcast read
-                    cd[e] = fmaf(q0f, k4.x, cd[e]);
-                    cd[e] = fmaf(q1f, k4.y, cd[e]);
-                    cd[e] = fmaf(q2f, k4.z, cd[e]);
-                    cd[e] = fmaf(q3f, k4.w, cd[e]);
-                }
-            }
-        };
-        if (n_here >= TOK) fold(std::integral_constant<int, TOK>{});
-        else if (n_here == 1) fold(std::integral_constant<int, 1>{});
-        else if (n_here == 2) fold(std::integral_constant<int, 2>{});
-        else fold(std::integral_constant<int, 3>{});
+        uint64_t c01 = 0ull, c23 = 0ull;
+#pragma unroll 16
+        for (int d = 0; d < RS_HD; ++d) {
+            const ulonglong2 k4 = reinterpret_cast<const ulonglong2*>(kf)[d];   // broadcast read
+            const uint64_t q2 = reinterpret_cast<const uint64_t*>(qq)[d * 32 + lane];
+            c01 = rs_fma2(q2, k4.x, c01);
+            c23 = rs_fma2(q2, k4.y, c23);
+        }
+        const float cd[TOK] = {__uint_as_float((uint32_t)c01), __uint_as_float((uint32_t)(c01 >> 32)),
+                               __uint_as_float((uint32_t)c23), __uint_as_float((uint32_t)(c23 >> 32))};
         __syncwarp();
 #pragma unroll
         for (int e = 0; e < TOK; ++e) {
             const float dot = __fmul_rn(__fmul_rn(cd[e], my_sq), skv[e]);
             float rr = __fmul_rn(dot, g.index_dscale);
             rr = rr > 0.0f ? rr : 0.0f;
-            kf[e * hd + lane] = __fmul_rn(my_wh, rr);
+            kf[e * PAD + lane] = __fmul_rn(my_wh, rr);     // (an absent head's term is +0, which changes no sum)
         }
         __syncwarp();
         if (lane < n_here) {
             float acc = 0.0f;
-            for (int h = 0; h < nh; ++h) acc = __fadd_rn(acc, kf[lane * hd + h]);
-            emit(base + lane * WARPS + warp, acc);
+#pragma unroll
+            for (int h = 0; h < 32; h += 4) {
+                const float4 t4 = *reinterpret_cast<const float4*>(kf + lane * PAD + h);
+                acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, t4.x), t4.y), t4.z), t4.w);
+            }
+            emit(p0 + lane, acc);
         }
         __syncwarp();
     }

@@ -9,30 +9,37 @@
 // IDENTICAL to exact scoring + exact top-k (contract and tie rule: crates/backend/kernels/indexer.hip:143-257,
 // crates/core/src/routing.rs:42-61).
 //
-// Layout: CTA `r` of a cluster of C owns the CH = EPT * 512 consecutive tokens [r * CH, (r + 1) * CH), thread t
-// the EPT consecutive tokens from r * CH + t * EPT, keys in registers. What the CTAs of a cluster exchange
-// goes through distributed shared memory (plain loads / stores on mapped addresses), mostly PUSHED into the
-// reader's memory so that a CTA needs nobody else's memory after its last cluster barrier.
+// Layout: CTAs of 1024 threads; CTA `r` of a cluster of C owns the CH consecutive tokens [r * CH, (r + 1) * CH), CH <= 16,384;
+// thread t the four tokens from (it * 1024 + t) * 4 of each of the CTA's up to four steps `it`, keys in shared memory. So every
+// load is a whole line, and the loops over the steps stay loops: a kernel whose code runs once per launch waits for its own
+// instructions (keys in registers, 32 consecutive tokens per thread and everything unrolled: 5.3 warps per issue slot stalled
+// without an instruction, and 16-byte loads 128 bytes apart).
+// What the CTAs of a cluster exchange goes through distributed shared memory, and is PUSHED into the reader's memory before a
+// cluster barrier: no CTA waits for a remote load except in the histogram's reduction.
 //
-//   1. keys; cluster-wide min / max key and max key scale (eps).
+//   1. keys; cluster-wide min / max key and max key scale (eps). What does not depend on the scores (page table, key scales,
+//      query) is loaded before the wait for the scorer.
 //   2. ONE histogram pass over 4096 bins spread linearly in value between the smallest and the largest score:
 //      the distribution decides the bin width, so the bin of the k-th value holds a handful of tokens on
 //      score-like data. Histograms are all-reduced slice by slice, the k-th bin is found by a suffix scan.
-//   3. classification against the band [smallest score of that bin - 2 eps, largest + 2 eps]; band tokens
+//   3. classification against the band [lower edge of that bin - 2 eps, upper edge + 2 eps]; band tokens
 //      are listed per CTA.
 //   4. exact re-score of the CTA's own band tokens (a warp takes 4 at a time, lane = head), the lists are
-//      gathered cluster-wide, every band token is ranked against all of them.
-//   5. ascending write-out: counts are exchanged, each CTA compacts its own contiguous token range.
+//      pushed cluster-wide, band tokens are ranked against all of them.
+//   5. ascending write-out: each CTA compacts its own contiguous token range.
 //
-// A batch that fills the chip by itself runs this kernel as ONE CTA of 1024 threads per sequence (a cluster of one):
-// for that shape the exchanges, the cluster barriers and the list copies are compiled out (SOLO below).
+// A lone CTA (a batch that fills the chip by itself, or few tokens): the exchanges, the cluster barriers and the list copies
+// are compiled out (SOLO below).
 //
 // VALUES: the same selection over given scores (rivoli_index_topk and its batched form): no error band (eps = 0), no key
 // scales and no re-score - the band is the k-th value's bin itself and its tokens are ranked by the scores as they are.
 //
 // If the band does not fit the list (tie-dominated scores: thousands of tokens at the cut) the cluster takes
 // the slow path instead: every band token is re-scored chunk by chunk, the exact keys replace the approximate
-// ones in the registers, and an exact 4 x 8-bit radix selection runs over the whole cluster.
+// ones, and an exact 4 x 8-bit radix selection runs over the whole cluster.
+//
+// A whole step, us, with keys in registers -> now: 4 sequences of 131,072 tokens 85.5 -> 76.1; 32 of up to 32,768 88.3 -> 82.1;
+// 64 of 16,384 104.7 -> 97.2; 128 of 16,384 149.0 -> 145.1; one of 4,099 42.4 -> 39.6.
 #include <cooperative_groups.h>
 
 #include "codec.cuh"
@@ -45,70 +52,41 @@ namespace cg = cooperative_groups;
 
 namespace {
 
-constexpr int SEL_MAX_WARPS = 32;   // CTAs of 512 threads (clusters of 2 to 8) or of 1024 threads (one CTA per sequence)
+constexpr int SEL_NT = 1024, SEL_NW = SEL_NT / 32;
+constexpr int SEL_STEP = SEL_NT * 4;                    // tokens of one step
+constexpr int SEL_STEPS = 4, SEL_CH = SEL_STEP * SEL_STEPS;   // most tokens per CTA
 constexpr int SEL_BINS = 4096;
+static_assert(SEL_BINS == SEL_NT * 4, "a thread scans four bins");
 constexpr int SEL_LIST = 2048;     // band tokens per SEQUENCE the fast path holds (and per chunk on the slow path)
-constexpr int SEL_TOK = 4;         // band tokens a warp re-scores per pass
+constexpr int SEL_RANK_ALL = 512;  // up to this many band tokens every CTA ranks those of the lower ranks too, instead of one more exchange
 constexpr int SEL_HD = RS_HD;      // index dim (one code word per lane)
 
-struct SelXc {                     // per-CTA exchange block; slot q of an array is written by rank q (its own copy in phase 1)
+struct SelXc {                     // per-CTA exchange block; slot q of an array is written by rank q
     uint32_t kmin[SEL_MAX_CLUSTER], kmax[SEL_MAX_CLUSTER], skmax[SEL_MAX_CLUSTER];
-    uint32_t slice_tot[SEL_MAX_CLUSTER];
-    uint32_t bmin[SEL_MAX_CLUSTER], bmax[SEL_MAX_CLUSTER];
     uint32_t n_in[SEL_MAX_CLUSTER], n_band[SEL_MAX_CLUSTER];
     uint32_t n_out[SEL_MAX_CLUSTER];
     uint32_t cnt_gt[SEL_MAX_CLUSTER], cnt_eq[SEL_MAX_CLUSTER];
-    uint32_t red[2][SEL_MAX_WARPS];
-    uint32_t red3[2][3][SEL_MAX_WARPS];
-    uint32_t wcnt[SEL_MAX_WARPS];
-    uint32_t list_n;
-    uint32_t bstar, n_above;
+    uint32_t red[2][SEL_NW];
+    uint32_t red3[3][SEL_NW];
+    uint32_t wcnt[SEL_NW];
+    uint32_t pre[2][SEL_NW];
+    uint32_t list_n, lower;
+    uint32_t bstar;
     uint32_t pivot, need;
 };
 
-// Block-wide reductions over NW warps, one barrier per call (double-buffered partials as in topk_core.cuh).
-template <int NW>
+// Sum over the block, one barrier (double-buffered partials).
 __device__ __forceinline__ uint32_t sel_block_sum(uint32_t v, SelXc& xc, int& buf) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     v = __reduce_add_sync(0xffffffffu, v);
     if (lane == 0) xc.red[buf][warp] = v;
     __syncthreads();
-    const uint32_t t = __reduce_add_sync(0xffffffffu, lane < NW ? xc.red[buf][lane] : 0u);
+    const uint32_t t = __reduce_add_sync(0xffffffffu, xc.red[buf][lane]);
     buf ^= 1;
     return t;
-}
-template <int NW>
-__device__ __forceinline__ uint32_t sel_block_max(uint32_t v, SelXc& xc, int& buf) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    v = __reduce_max_sync(0xffffffffu, v);
-    if (lane == 0) xc.red[buf][warp] = v;
-    __syncthreads();
-    const uint32_t t = __reduce_max_sync(0xffffffffu, lane < NW ? xc.red[buf][lane] : 0u);
-    buf ^= 1;
-    return t;
-}
-template <int NW>
-__device__ __forceinline__ uint32_t sel_block_min(uint32_t v, SelXc& xc, int& buf) {
-    return ~sel_block_max<NW>(~v, xc, buf);
-}
-
-// min, max and a second max over the block in ONE barrier.
-template <int NW>
-__device__ __forceinline__ void sel_block_minmaxmax(uint32_t& mn, uint32_t& mx, uint32_t& mx2, SelXc& xc, int& buf) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    mn = __reduce_min_sync(0xffffffffu, mn);
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    mx2 = __reduce_max_sync(0xffffffffu, mx2);
-    if (lane == 0) { xc.red3[buf][0][warp] = mn; xc.red3[buf][1][warp] = mx; xc.red3[buf][2][warp] = mx2; }
-    __syncthreads();
-    mn = __reduce_min_sync(0xffffffffu, lane < NW ? xc.red3[buf][0][lane] : 0xffffffffu);
-    mx = __reduce_max_sync(0xffffffffu, lane < NW ? xc.red3[buf][1][lane] : 0u);
-    mx2 = __reduce_max_sync(0xffffffffu, lane < NW ? xc.red3[buf][2][lane] : 0u);
-    buf ^= 1;
 }
 
 // Exclusive prefix of `v` over the block in thread order (one barrier).
-template <int NW>
 __device__ __forceinline__ uint32_t sel_block_excl(uint32_t v, SelXc& xc) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t incl = v;
@@ -119,149 +97,208 @@ __device__ __forceinline__ uint32_t sel_block_excl(uint32_t v, SelXc& xc) {
     }
     if (lane == 31) xc.wcnt[warp] = incl;
     __syncthreads();
-    const uint32_t cw = lane < NW ? xc.wcnt[lane] : 0u;
-    const uint32_t pre = __reduce_add_sync(0xffffffffu, lane < warp ? cw : 0u);
-    __syncthreads();                                   // wcnt may be rewritten by the next call
-    return pre + incl - v;
+    return __reduce_add_sync(0xffffffffu, lane < warp ? xc.wcnt[lane] : 0u) + incl - v;
 }
 
-template <int EPT, int NT, bool VALUES>
-__global__ void __launch_bounds__(NT, (NT == 512 && EPT <= 16) ? 2 : 1)
-index_select_cluster_kernel(SelArgs A) {
-    constexpr int NW = NT / 32;
-    // A CTA of 1024 threads is launched only as a cluster of ONE (a batch that fills the chip by itself): every
-    // exchange between CTAs and every cluster barrier falls away at compile time, and with them most of the block
-    // barriers, which is what this latency-bound kernel is made of.
-    constexpr bool SOLO = NT == 1024;
+// For a mask of 4 bits per step: how many bits of tokens before this thread's are set, per step (token order: step, then
+// thread). One barrier; two steps share a word (a step holds at most 4,096 tokens).
+__device__ __forceinline__ void sel_token_excl(uint32_t mask, SelXc& xc, uint32_t (&before)[SEL_STEPS]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t c[2], incl[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        c[u] = (uint32_t)__popc(mask & (0xfu << (8 * u))) | ((uint32_t)__popc(mask & (0xf0u << (8 * u))) << 16);
+        incl[u] = c[u];
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, incl[u], o);
+            if (lane >= o) incl[u] += t;
+        }
+    if (lane == 31) { xc.pre[0][warp] = incl[0]; xc.pre[1][warp] = incl[1]; }
+    __syncthreads();
+    uint32_t run = 0u;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const uint32_t w = xc.pre[u][lane];
+        const uint32_t tot = __reduce_add_sync(0xffffffffu, w);
+        const uint32_t ex = __reduce_add_sync(0xffffffffu, lane < warp ? w : 0u) + incl[u] - c[u];
+        before[2 * u] = run + (ex & 0xffffu);
+        run += tot & 0xffffu;
+        before[2 * u + 1] = run + (ex >> 16);
+        run += tot >> 16;
+    }
+}
+
+template <bool VALUES, bool SOLO>
+__global__ void __launch_bounds__(SEL_NT, 1)
+index_select_kernel(SelArgs A, int CH) {
     cg::cluster_group cluster = cg::this_cluster();
     const int C = SOLO ? 1 : (int)cluster.dim_blocks().x, r = SOLO ? 0 : (int)cluster.block_rank();
+    if constexpr (!SOLO) cluster.barrier_arrive();                        // [0] every CTA runs: its memory may be written
     extern __shared__ __align__(16) uint32_t sel_smem[];
     __shared__ SelXc xc;
-    uint32_t* qf = sel_smem;                                              // [SEL_HD / 4][32] packed q codes, [word][head]
-    float* kfw = reinterpret_cast<float*>(qf + (SEL_HD / 4) * 32);        // [NW][SEL_TOK][SEL_HD] key rows as f32
-    uint32_t* hist = VALUES ? sel_smem : reinterpret_cast<uint32_t*>(kfw + NW * SEL_TOK * SEL_HD);   // [SEL_BINS]; later `dec`
+    uint32_t* keys = sel_smem;                                            // [CH]
+    uint32_t* hist = keys + CH;                                           // [SEL_BINS]; later `dec`
     uint32_t* l_tok = hist + SEL_BINS;                                    // [SEL_LIST] this CTA's band tokens
     uint32_t* l_key = l_tok + SEL_LIST;                                   // [SEL_LIST] their exact keys
-    uint32_t* a_tok = l_key + SEL_LIST;                                   // [SEL_LIST] the cluster's band, gathered
+    uint32_t* red = l_key + SEL_LIST;                                     // [SEL_BINS] reduced histogram, before the re-score
+    float* kfw = reinterpret_cast<float*>(red);                           // [warps][SEL_HD][4] key rows as f32
+    float2* qq = reinterpret_cast<float2*>(kfw + SEL_NW * SEL_HD * 4);    // [SEL_HD][32] (q, q) pairs
+    uint32_t* a_tok = VALUES ? red + SEL_BINS : reinterpret_cast<uint32_t*>(qq + SEL_HD * 32);   // [SEL_LIST] the cluster's band (clusters only)
     uint32_t* a_key = a_tok + SEL_LIST;                                   // [SEL_LIST]
-    uint32_t* red_hist = a_tok;                                           // [SEL_BINS / C] reduced histogram slice (phase 2)
-    uint32_t* slice = l_tok;                                              // [SEL_BINS / C] the slice holding the k-th bin
 
     const DsaGeom& g = A.g;
-    constexpr int hd = SEL_HD;
     const int nh = g.index_heads, P = g.page_tokens;
     const int b = (int)blockIdx.x / C, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     rv_grid_dep_trigger();   // the next kernel may set itself up; it waits for this grid before reading rows
-    rv_grid_dep_wait();      // scores, query codes and the error constant come from the kernels before
+    // The scorer is launched only when all before it is complete and starts this kernel only then, so everything but its
+    // scores may be read before the wait. Given scores come with no such promise.
+    if constexpr (VALUES) rv_grid_dep_wait();
     const int nt = min(VALUES && !A.seq_len ? A.nt_single : A.seq_len[b], A.score_stride);
     const int kk = min(A.k, nt);
     uint32_t* out = A.rows + (size_t)b * A.k;
-    if (r == 0 && tid == 0 && (!VALUES || A.n_sel)) A.n_sel[b] = kk > 0 ? kk : 0;
-    if (kk <= 0) return;                                                  // uniform over the cluster
-    constexpr int CH = EPT * NT;
-    const int i0 = r * CH + tid * EPT;
-    const int nvalid = max(0, min(EPT, nt - i0));
-    if (kk == nt) {                                                       // everything is selected: the identity
-#pragma unroll
-        for (int j = 0; j < EPT; ++j)
-            if (j < nvalid) out[i0 + j] = (uint32_t)(i0 + j);
-        if (r == 0 && tid == 0 && A.stats) { A.stats[b * 2] = 0; A.stats[b * 2 + 1] = (unsigned)nt; }
+    const int c0 = r * CH, nloc = max(0, min(CH, nt - c0));              // this CTA's tokens: [c0, c0 + nloc)
+    const int32_t* bt = A.block_table + (size_t)b * g.max_pages_per_seq;
+    if (kk == nt || kk <= 0) {                                            // everything (or nothing) is selected: the identity
+        if constexpr (!VALUES) rv_grid_dep_wait();
+        if (r == 0 && tid == 0 && (!VALUES || A.n_sel)) A.n_sel[b] = kk > 0 ? kk : 0;
+        for (int i = tid; i < nloc; i += SEL_NT) out[c0 + i] = (uint32_t)(c0 + i);
+        if (r == 0 && tid == 0 && A.stats && kk > 0) { A.stats[b * 2] = 0; A.stats[b * 2 + 1] = (unsigned)nt; }
         if constexpr (!VALUES) {                                              // nobody scored these tokens: look at their pages here
-            for (int lp = r * NT + tid; lp * P < nt; lp += C * NT) {
-                const int pg = lp < g.max_pages_per_seq ? A.block_table[(size_t)b * g.max_pages_per_seq + lp] : 0;
+            for (int lp = r * SEL_NT + tid; lp * P < nt; lp += C * SEL_NT) {
+                const int pg = lp < g.max_pages_per_seq ? bt[lp] : 0;
                 if (pg < 0 || pg >= g.n_pool_pages) atomicCAS(A.err, 0, 1005);
             }
         }
+        if constexpr (!SOLO) cluster.barrier_wait();
         return;
     }
 
     // ---- 1. approximate keys: (unscaled tensor-core score) * key scale of the token --------------------------
     const float* s = A.scores + (size_t)b * (VALUES ? (size_t)A.value_stride : (size_t)A.score_stride);
-    const int32_t* bt = A.block_table + (size_t)b * g.max_pages_per_seq;
-    uint32_t key[EPT];
+    const int steps = (nloc + SEL_STEP - 1) / SEL_STEP;
+    const int pshift = VALUES ? 0 : 31 - __clz(P);
+    auto scale_row = [&](int i) {
+        int pg = bt[i >> pshift];
+        pg = (pg < 0 || pg >= g.n_pool_pages) ? 0 : pg;
+        return ((size_t)pg << pshift) + (i & (P - 1));
+    };
+    uint32_t kmin = 0xffffffffu, kmax = 0u;
     float skm = 0.0f;
-    if constexpr (VALUES) {
-        if (A.vec_ok && nvalid == EPT) {
+    auto take4 = [&](int i4, const float (&v)[4]) {                       // four keys of the token vector at local index i4
+        uint32_t k[4];
 #pragma unroll
-            for (int j = 0; j < EPT; j += 4) {
-                const float4 a = *reinterpret_cast<const float4*>(s + i0 + j);
-                key[j] = topk_key(a.x); key[j + 1] = topk_key(a.y); key[j + 2] = topk_key(a.z); key[j + 3] = topk_key(a.w);
+        for (int e = 0; e < 4; ++e) {
+            k[e] = topk_key(v[e]);
+            if (i4 + e < nloc) { kmin = min(kmin, k[e]); kmax = max(kmax, k[e]); }
+        }
+        *reinterpret_cast<uint4*>(keys + i4) = make_uint4(k[0], k[1], k[2], k[3]);
+    };
+    const float my_sq = !VALUES && lane < nh ? A.qscales[(size_t)b * nh + lane] : 0.0f;      // head constants of the re-score (nh <= 32)
+    const float my_wh = !VALUES && lane < nh ? __fmul_rn(A.w[(size_t)b * nh + lane], g.index_wscale) : 0.0f;
+    for (int i = tid; i < SEL_BINS / 4; i += SEL_NT) reinterpret_cast<uint4*>(hist)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (tid == 0) { xc.list_n = 0; xc.lower = 0; }
+    if (A.vec_ok) {
+        float4 sk[SEL_STEPS], sc[SEL_STEPS];
+        if constexpr (!VALUES) {
+            size_t rr[SEL_STEPS];
+#pragma unroll
+            for (int it = 0; it < SEL_STEPS; ++it) {
+                const int i4 = it * SEL_STEP + tid * 4;
+                rr[it] = i4 < nloc ? scale_row(c0 + i4) : 0;
             }
-        } else {
 #pragma unroll
-            for (int j = 0; j < EPT; ++j) key[j] = j < nvalid ? topk_key(s[i0 + j]) : 0u;
+            for (int it = 0; it < SEL_STEPS; ++it)
+                sk[it] = it * SEL_STEP + tid * 4 < nloc ? *reinterpret_cast<const float4*>(A.index_scale + rr[it]) : make_float4(0.f, 0.f, 0.f, 0.f);
+            rv_rescore_stage_q(A.qcodes + (size_t)b * nh * SEL_HD, nh, qq);
+            rv_grid_dep_wait();
+        }
+#pragma unroll
+        for (int it = 0; it < SEL_STEPS; ++it)
+            sc[it] = it * SEL_STEP + tid * 4 < nloc ? *reinterpret_cast<const float4*>(s + c0 + it * SEL_STEP + tid * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int it = 0; it < SEL_STEPS; ++it) {
+            const int i4 = it * SEL_STEP + tid * 4;
+            if (i4 < nloc) {
+                float v[4] = {sc[it].x, sc[it].y, sc[it].z, sc[it].w};
+                if constexpr (!VALUES) {
+                    const float k4[4] = {sk[it].x, sk[it].y, sk[it].z, sk[it].w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        v[e] *= k4[e];
+                        if (i4 + e < nloc) skm = fmaxf(skm, k4[e]);
+                    }
+                }
+                take4(i4, v);
+            }
         }
     } else {
-        float sc[EPT], sk[EPT];
-        if (A.vec_ok && nvalid == EPT) {
-            size_t rr[EPT / 4];
+        if constexpr (!VALUES) {
+            rv_rescore_stage_q(A.qcodes + (size_t)b * nh * SEL_HD, nh, qq);
+            rv_grid_dep_wait();
+        }
+#pragma unroll 1
+        for (int it = 0; it < steps; ++it) {
+            const int i4 = it * SEL_STEP + tid * 4;
+            if (i4 >= nloc) break;
+            float v[4];
 #pragma unroll
-            for (int j4 = 0; j4 < EPT / 4; ++j4) {
-                const int i = i0 + j4 * 4;
-                int pg = bt[i / P];
-                pg = (pg < 0 || pg >= g.n_pool_pages) ? 0 : pg;
-                rr[j4] = (size_t)pg * P + (i & (P - 1));
-            }
-#pragma unroll
-            for (int j4 = 0; j4 < EPT / 4; ++j4) {
-                const float4 a = *reinterpret_cast<const float4*>(s + i0 + j4 * 4);
-                const float4 c = *reinterpret_cast<const float4*>(A.index_scale + rr[j4]);
-                sc[j4 * 4] = a.x; sc[j4 * 4 + 1] = a.y; sc[j4 * 4 + 2] = a.z; sc[j4 * 4 + 3] = a.w;
-                sk[j4 * 4] = c.x; sk[j4 * 4 + 1] = c.y; sk[j4 * 4 + 2] = c.z; sk[j4 * 4 + 3] = c.w;
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < EPT; ++j) {
-                const int i = i0 + j;
-                sc[j] = 0.0f; sk[j] = 0.0f;
-                if (j < nvalid) {
-                    int pg = bt[i / P];
-                    pg = (pg < 0 || pg >= g.n_pool_pages) ? 0 : pg;
-                    sc[j] = s[i];
-                    sk[j] = A.index_scale[(size_t)pg * P + (i & (P - 1))];
+            for (int e = 0; e < 4; ++e) {
+                v[e] = 0.0f;
+                if (i4 + e < nloc) {
+                    v[e] = s[c0 + i4 + e];
+                    if constexpr (!VALUES) {
+                        const float k1 = A.index_scale[scale_row(c0 + i4 + e)];
+                        v[e] *= k1;
+                        skm = fmaxf(skm, k1);
+                    }
                 }
             }
-        }
-#pragma unroll
-        for (int j = 0; j < EPT; ++j) {
-            key[j] = j < nvalid ? topk_key(sc[j] * sk[j]) : 0u;
-            skm = fmaxf(skm, sk[j]);
+            take4(i4, v);
         }
     }
-    if constexpr (!VALUES) rv_rescore_stage_q(A.qcodes + (size_t)b * nh * hd, nh, qf);
-    for (int i = tid; i < SEL_BINS; i += NT) hist[i] = 0u;
-    if (tid == 0) xc.list_n = 0;
-    int buf = 0;
-    uint32_t kmin = 0xffffffffu, kmax = 0u;
-    float sk_max = 0.0f;
-    {
-        uint32_t mn = 0xffffffffu, mx = 0u;
-#pragma unroll
-        for (int j = 0; j < EPT; ++j)
-            if (j < nvalid) { mn = min(mn, key[j]); mx = max(mx, key[j]); }
-        uint32_t sm = __float_as_uint(skm);                                      // scales are >= 0: bit order = value order
-        sel_block_minmaxmax<NW>(mn, mx, sm, xc, buf);                            // (also orders the zeroing above before the histogram)
-        if constexpr (SOLO) {
-            kmin = mn; kmax = mx; sk_max = __uint_as_float(sm);
-        } else {
-            if (tid == 0) { xc.kmin[r] = mn; xc.kmax[r] = mx; xc.skmax[r] = sm; }
-            // [1] The first exchange is a PULL: a CTA may touch another CTA's shared memory only once that CTA is known
-            // to be running, which its arrival at this barrier proves. Every later exchange pushes.
-            cluster.sync();
-            // (all remote loads in flight at once: a loop to a run-time count pays a round trip for each)
-            uint32_t kn[SEL_MAX_CLUSTER], kx[SEL_MAX_CLUSTER], sx[SEL_MAX_CLUSTER];
-#pragma unroll
-            for (int q = 0; q < SEL_MAX_CLUSTER; ++q) {
-                const int qq = q < C ? q : 0;
-                const SelXc* src = cluster.map_shared_rank(&xc, qq);
-                kn[q] = src->kmin[qq]; kx[q] = src->kmax[qq]; sx[q] = src->skmax[qq];
-            }
-#pragma unroll
-            for (int q = 0; q < SEL_MAX_CLUSTER; ++q) {
-                kmin = min(kmin, kn[q]); kmax = max(kmax, kx[q]);
-                sk_max = fmaxf(sk_max, __uint_as_float(sx[q]));
+    if (r == 0 && tid == 0 && (!VALUES || A.n_sel)) A.n_sel[b] = kk;
+    // keys of this thread's four tokens of step `it` (only this thread reads and writes them until the slow path's end)
+    auto for_keys = [&](auto f) {                                          // f(step, local index, e, key)
+#pragma unroll 1
+        for (int it = 0; it < steps; ++it) {
+            const int i4 = it * SEL_STEP + tid * 4;
+            if (i4 < nloc) {
+                const uint4 k = *reinterpret_cast<const uint4*>(keys + i4);
+                f(it, i4, 0, k.x);
+                if (i4 + 1 < nloc) f(it, i4, 1, k.y);
+                if (i4 + 2 < nloc) f(it, i4, 2, k.z);
+                if (i4 + 3 < nloc) f(it, i4, 3, k.w);
             }
         }
+    };
+    int buf = 0;
+    float sk_max;
+    {
+        uint32_t sm = __reduce_max_sync(0xffffffffu, __float_as_uint(skm));    // scales are >= 0: bit order = value order
+        kmin = __reduce_min_sync(0xffffffffu, kmin);
+        kmax = __reduce_max_sync(0xffffffffu, kmax);
+        if (lane == 0) { xc.red3[0][warp] = kmin; xc.red3[1][warp] = kmax; xc.red3[2][warp] = sm; }
+        __syncthreads();                                                       // (also orders the zeroing above before the histogram)
+        kmin = __reduce_min_sync(0xffffffffu, xc.red3[0][lane]);
+        kmax = __reduce_max_sync(0xffffffffu, xc.red3[1][lane]);
+        sm = __reduce_max_sync(0xffffffffu, xc.red3[2][lane]);
+        if constexpr (!SOLO) {
+            cluster.barrier_wait();                                            // [0]
+            if (tid < C) {
+                SelXc* dst = cluster.map_shared_rank(&xc, tid);
+                dst->kmin[r] = kmin; dst->kmax[r] = kmax; dst->skmax[r] = sm;
+            }
+            cluster.sync();                                                    // [1] everybody's extremes
+            const int q = lane < C ? lane : 0;
+            kmin = __reduce_min_sync(0xffffffffu, xc.kmin[q]);
+            kmax = __reduce_max_sync(0xffffffffu, xc.kmax[q]);
+            sm = __reduce_max_sync(0xffffffffu, xc.skmax[q]);
+        }
+        sk_max = __uint_as_float(sm);
     }
     const float eps = VALUES ? 0.0f : sk_max * A.cb[b];
 
@@ -269,121 +306,65 @@ index_select_cluster_kernel(SelArgs A) {
     // bin(v) = min(4095, int((v - vmin) * inv_w)) is monotone in v, which is all the selection needs: tokens in
     // higher bins than the k-th value's are above it, tokens in lower bins below. (Bins linear in the key BITS
     // would be logarithmic in value: 6 % wide around 1.0.) A degenerate range (all scores equal, or a span
-    // that overflows) gives inv_w = 0 and one bin; the slow path below takes such inputs.
+    // that overflows; given scores may also hold infinities and NaNs) gives inv_w = 0 and one bin, all of it band.
     const float vmin = topk_unkey(kmin), vmax = topk_unkey(kmax);
     float inv_w = (float)SEL_BINS / (vmax - vmin);
     if (!(inv_w > 0.0f) || !(inv_w < 3.0e38f)) inv_w = 0.0f;
-    auto bin_of = [&](uint32_t k) -> uint32_t {
-        if (VALUES && inv_w == 0.0f) return 0u;   // given scores may hold infinities and NaNs: one bin, ordered by key bits alone
-        const float t = (topk_unkey(k) - vmin) * inv_w;
-        return (uint32_t)fminf(t, (float)(SEL_BINS - 1));
-    };
-    {
-        // consecutive tokens often share a bin (runs of ReLU zeros): one shared-memory atomic per run
-        uint32_t cur = 0xffffffffu, run = 0u;
-#pragma unroll
-        for (int j = 0; j < EPT; ++j) {
-            if (j < nvalid) {
-                const uint32_t bin = bin_of(key[j]);
-                if (bin != cur) { if (run) atomicAdd(&hist[cur], run); cur = bin; run = 0u; }
-                ++run;
-            }
-        }
-        if (run) atomicAdd(&hist[cur], run);
-    }
-    __syncthreads();
-    int SL = SEL_BINS;                                                        // bins of the slice that holds the k-th value
-    int s_star = 0;
-    uint32_t above = 0u;                                                      // tokens in slices above the k-th value's
-    uint32_t slice_total = (uint32_t)nt;                                      // tokens in that slice
-    const uint32_t* slice_c = hist;
+    if (inv_w > 0.0f)
+        for_keys([&](int, int, int, uint32_t k) {
+            atomicAdd(&hist[(uint32_t)fminf((topk_unkey(k) - vmin) * inv_w, (float)(SEL_BINS - 1))], 1u);
+        });
+    else if (tid == 0) hist[0] = (uint32_t)nloc;
+    const uint32_t* all = hist;
     if constexpr (!SOLO) {
         cluster.sync();                                                       // [2] every CTA's histogram is complete
-        SL = SEL_BINS / C;                                                    // rank r reduces bins [r * SL, (r + 1) * SL)
-        {
-            uint32_t tot = 0u;
-            for (int i = tid; i < SL; i += NT) {
-                uint32_t h[SEL_MAX_CLUSTER], v = 0u;
+        const int SL4 = SEL_BINS / 4 / C;                                     // rank r reduces its share and pushes it to everybody
+        for (int i = tid; i < SL4; i += SEL_NT) {
+            uint4 h[SEL_MAX_CLUSTER], v = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-                for (int q = 0; q < SEL_MAX_CLUSTER; ++q) h[q] = q < C ? cluster.map_shared_rank(hist, q < C ? q : 0)[r * SL + i] : 0u;
+            for (int q = 0; q < SEL_MAX_CLUSTER; ++q)                         // (all remote loads in flight at once)
+                h[q] = q < C ? reinterpret_cast<const uint4*>(cluster.map_shared_rank(hist, q < C ? q : 0))[r * SL4 + i] : v;
 #pragma unroll
-                for (int q = 0; q < SEL_MAX_CLUSTER; ++q) v += h[q];
-                red_hist[i] = v;
-                tot += v;
-            }
-            tot = sel_block_sum<NW>(tot, xc, buf);
-            if (tid < C) cluster.map_shared_rank(&xc, tid)->slice_tot[r] = tot;
+            for (int q = 0; q < SEL_MAX_CLUSTER; ++q) { v.x += h[q].x; v.y += h[q].y; v.z += h[q].z; v.w += h[q].w; }
+            for (int q = 0; q < C; ++q) reinterpret_cast<uint4*>(cluster.map_shared_rank(red, q))[r * SL4 + i] = v;
         }
+        cluster.sync();                                                       // [3] the whole reduced histogram
+        all = red;
+    } else {
         __syncthreads();
-        cluster.sync();                                                       // [3] reduced slices and their totals
-        for (int q = C - 1; q >= 0; --q) {
-            if (above + xc.slice_tot[q] >= (uint32_t)kk) { s_star = q; break; }
-            above += xc.slice_tot[q];
-        }
-        {
-            const uint32_t* src = cluster.map_shared_rank(red_hist, s_star);
-            for (int i = tid; i < SL; i += NT) slice[i] = src[i];
-        }
-        __syncthreads();
-        slice_total = xc.slice_tot[s_star];
-        slice_c = slice;
     }
     {
-        // suffix scan over the slice: thread t owns bins [t * per, (t + 1) * per), per = ceil(SL / 512)
-        const int per = (SL + NT - 1) / NT;
-        uint32_t mine = 0u;
-        for (int j = 0; j < per; ++j) { const int i = tid * per + j; if (i < SL) mine += slice_c[i]; }
-        const uint32_t before = sel_block_excl<NW>(mine, xc);                     // bins below this thread's
-        const uint32_t total = slice_total;
-        uint32_t acc = above + (total - before - mine);                       // tokens in bins above this thread's
-        for (int j = per - 1; j >= 0; --j) {
-            const int i = tid * per + j;
-            if (i < SL) {
-                const uint32_t h = slice_c[i];
-                if (acc < (uint32_t)kk && (uint32_t)kk <= acc + h) { xc.bstar = (uint32_t)(s_star * SL + i); xc.n_above = acc; }
-                acc += h;
-            }
+        // suffix scan: thread t owns the bins 4 t .. 4 t + 3
+        const uint4 h = reinterpret_cast<const uint4*>(all)[tid];
+        const uint32_t mine = h.x + h.y + h.z + h.w, before = sel_block_excl(mine, xc);
+        uint32_t acc = (uint32_t)nt - before - mine;                          // tokens in bins above this thread's
+        const uint32_t hb[4] = {h.x, h.y, h.z, h.w};
+#pragma unroll
+        for (int j = 3; j >= 0; --j) {
+            if (acc < (uint32_t)kk && (uint32_t)kk <= acc + hb[j]) xc.bstar = (uint32_t)(tid * 4 + j);
+            acc += hb[j];
         }
     }
     __syncthreads();
-    const uint32_t bstar = xc.bstar;
 
     // ---- 3. classification: surely selected / band (re-scored exactly) / surely not -------------------------
-    // The k-th approximate score is one of the tokens of bin `bstar`: it lies between the smallest and the
-    // largest key found there (exact bounds, no reasoning about the rounding of bin_of needed).
-    uint32_t k_lo, k_hi;
-    {
-        uint32_t mn = 0xffffffffu, mx = 0u;
-#pragma unroll
-        for (int j = 0; j < EPT; ++j)
-            if (j < nvalid && bin_of(key[j]) == bstar) { mn = min(mn, key[j]); mx = max(mx, key[j]); }
-        uint32_t unused = 0u;
-        sel_block_minmaxmax<NW>(mn, mx, unused, xc, buf);
-        if constexpr (!SOLO) {
-            if (tid < C) {
-                SelXc* dst = cluster.map_shared_rank(&xc, tid);
-                dst->bmin[r] = mn; dst->bmax[r] = mx;
-            }
-            cluster.sync();                                                   // [3b]
-            mn = 0xffffffffu; mx = 0u;
-            for (int q = 0; q < C; ++q) { mn = min(mn, xc.bmin[q]); mx = max(mx, xc.bmax[q]); }
-        }
-        if constexpr (VALUES) {
-            k_lo = mn; k_hi = mx;
-        } else {
-            const float lo_f = topk_unkey(mn) - 2.0f * eps, hi_f = topk_unkey(mx) + 2.0f * eps;
-            k_lo = lo_f == lo_f ? topk_key(lo_f) : 0u;
-            k_hi = hi_f == hi_f ? topk_key(hi_f) : 0xffffffffu;
-        }
+    // The k-th approximate score is one of the tokens of bin `bstar`: it lies between the bin's edges. Their slack covers
+    // every rounding of bin_of and of the edges (a few 2^-24 of the larger of |vmin|, |vmax|); it only widens the band.
+    uint32_t k_lo = 0u, k_hi = 0xffffffffu;
+    if (inv_w > 0.0f) {
+        const float w = (vmax - vmin) * (1.0f / (float)SEL_BINS), fb = (float)xc.bstar;
+        const float slack = 2.0f * eps + (fabsf(vmin) + fabsf(vmax)) * 1.9073486328125e-6f;   // 2^-19
+        const float lo_f = vmin + fb * w - slack, hi_f = (xc.bstar == SEL_BINS - 1 ? vmax : vmin + (fb + 1.0f) * w) + slack;
+        if (xc.bstar > 0 && lo_f == lo_f) k_lo = topk_key(lo_f);
+        if (hi_f == hi_f) k_hi = topk_key(hi_f);
     }
-    uint32_t m_in = 0u, m_band = 0u;
-#pragma unroll
-    for (int j = 0; j < EPT; ++j) {
-        if (j < nvalid) {
-            if (key[j] > k_hi) m_in |= 1u << j;
-            else if (key[j] >= k_lo) m_band |= 1u << j;
-        }
-    }
+    uint32_t m_in = 0u, m_band = 0u;                                          // bit 4 * step + e
+    for_keys([&](int it, int, int e, uint32_t k) {
+        const uint32_t bit = 1u << (4 * it + e);
+        if (k > k_hi) m_in |= bit;
+        else if (k >= k_lo) m_band |= bit;
+    });
+    auto local_of = [&](int bit) { return ((bit >> 2) * SEL_NT + tid) * 4 + (bit & 3); };
     {   // this CTA's count of surely selected tokens: the warp sums meet at the barrier that closes the list
         const uint32_t v = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(m_in));
         if (lane == 0) xc.red[buf][warp] = v;
@@ -402,95 +383,132 @@ index_select_cluster_kernel(SelArgs A) {
         wbase = __shfl_sync(0xffffffffu, wbase, 31);
         my_pos = wbase + incl - cnt;
         uint32_t pos = my_pos;
-#pragma unroll
-        for (int j = 0; j < EPT; ++j)
-            if (m_band & (1u << j)) {
-                if (pos < SEL_LIST) { l_tok[pos] = (uint32_t)(i0 + j); if (VALUES) l_key[pos] = key[j]; }
-                ++pos;
-            }
+        for (uint32_t m = m_band; m && pos < SEL_LIST; m &= m - 1u, ++pos) {
+            const int i = local_of(__ffs(m) - 1);
+            l_tok[pos] = (uint32_t)(c0 + i);
+            if (VALUES) l_key[pos] = keys[i];
+        }
     }
     __syncthreads();
-    const uint32_t n_in_mine = __reduce_add_sync(0xffffffffu, lane < NW ? xc.red[buf][lane] : 0u);
+    const uint32_t n_in_mine = __reduce_add_sync(0xffffffffu, xc.red[buf][lane]);
     buf ^= 1;
     const uint32_t n_band_mine = xc.list_n;
-    uint32_t n_in = n_in_mine, n_band = n_band_mine;
-    if constexpr (!SOLO) {
-        if (tid < C) {
-            SelXc* dst = cluster.map_shared_rank(&xc, tid);
-            dst->n_in[r] = n_in_mine; dst->n_band[r] = n_band_mine;
-        }
-        cluster.sync();                                                       // [4] (also: nobody reads red_hist any more)
-        n_in = 0u; n_band = 0u;
-        for (int q = 0; q < C; ++q) { n_in += xc.n_in[q]; n_band += xc.n_band[q]; }
-    }
 
-    // this lane's head constants for the exact re-score (nh <= 32)
-    const float my_sq = !VALUES && lane < nh ? A.qscales[(size_t)b * nh + lane] : 0.0f;
-    const float my_wh = !VALUES && lane < nh ? __fmul_rn(A.w[(size_t)b * nh + lane], g.index_wscale) : 0.0f;
     // Exact key of the first `ln` listed tokens -> l_key[position] (0 and ~0 are reserved for "surely out" / "surely in").
     auto rescore = [&](uint32_t ln) {
-        rv_rescore_listed<NW, SEL_TOK>(l_tok, ln, qf, kfw + warp * (SEL_TOK * hd), bt, g, A.index_pool, A.index_scale,
-                                              my_sq, my_wh, [&](uint32_t pos, float score) {
+        rv_rescore_listed<SEL_NW>(l_tok, ln, qq, kfw + warp * (SEL_HD * 4), bt, g, A.index_pool, A.index_scale, my_sq, my_wh,
+                                  [&](uint32_t pos, float score) {
             uint32_t ku = topk_key(score);
             l_key[pos] = ku == 0xffffffffu ? 0xfffffffeu : (ku == 0u ? 1u : ku);
         });
     };
     // ascending write-out of this CTA's tokens whose bit is set in `sel`, from slot `base` on (one barrier)
     auto write_out = [&](uint32_t sel, uint32_t base) {
-        uint32_t pos = base + sel_block_excl<NW>((uint32_t)__popc(sel), xc);
+        uint32_t before[SEL_STEPS];
+        sel_token_excl(sel, xc, before);
 #pragma unroll
-        for (int j = 0; j < EPT; ++j)
-            if (sel & (1u << j)) out[pos++] = (uint32_t)(i0 + j);
+        for (int it = 0; it < SEL_STEPS; ++it) {
+            uint32_t pos = base + before[it];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (sel & (1u << (4 * it + e))) out[pos++] = (uint32_t)(c0 + it * SEL_STEP + tid * 4 + e);
+        }
     };
 
-    if (n_band <= (uint32_t)SEL_LIST) {
-        // ---- 4. common case: the whole band fits the list --------------------------------------------------
-        if constexpr (!VALUES) {
-            rescore(n_band_mine);
-            __syncthreads();
-        }
-        const uint32_t* all_tok = l_tok;                                      // the cluster's band: a lone CTA's own lists
-        const uint32_t* all_key = l_key;
-        if constexpr (!SOLO) {
-            cluster.sync();                                                   // [5] every CTA's exact band keys
-            uint32_t off = 0u;
-            for (int q = 0; q < C; ++q) {
-                const uint32_t nq = xc.n_band[q];
-                const uint32_t* st = cluster.map_shared_rank(l_tok, q);
-                const uint32_t* sk2 = cluster.map_shared_rank(l_key, q);
-                for (uint32_t i = tid; i < nq; i += NT) { a_tok[off + i] = st[i]; a_key[off + i] = sk2[i]; }
-                off += nq;
+    // ---- 4. exact keys of the band -------------------------------------------------------------------------
+    if constexpr (!VALUES) {
+        if (n_band_mine <= (uint32_t)SEL_LIST) rescore(n_band_mine);
+        __syncthreads();
+    }
+    uint32_t n_in = n_in_mine, n_band = n_band_mine;
+    const uint32_t RG = SEL_LIST / C;                                         // entries of one rank in everybody's gathered list
+    bool pushed = true;
+    if constexpr (!SOLO) {
+        {   // a warp serves one destination
+            const int q = warp & (C - 1);
+            uint32_t* dt = cluster.map_shared_rank(a_tok, q) + r * RG;
+            uint32_t* dk = cluster.map_shared_rank(a_key, q) + r * RG;
+            for (uint32_t i = (warp / C) * 32 + lane; i < min(n_band_mine, RG); i += (SEL_NW / C) * 32) { dt[i] = l_tok[i]; dk[i] = l_key[i]; }
+            if (tid < C) {
+                SelXc* dst = cluster.map_shared_rank(&xc, tid);
+                dst->n_in[r] = n_in_mine; dst->n_band[r] = n_band_mine;
             }
-            __syncthreads();
-            all_tok = a_tok; all_key = a_key;
         }
-        // rank each of this CTA's band tokens among ALL band tokens by (exact key descending, index ascending)
+        cluster.sync();                                                       // [4] counts and lists
+        const uint32_t nb = lane < C ? xc.n_band[lane] : 0u;
+        n_in = __reduce_add_sync(0xffffffffu, lane < C ? xc.n_in[lane] : 0u);
+        n_band = __reduce_add_sync(0xffffffffu, nb);
+        pushed = __reduce_max_sync(0xffffffffu, nb) <= RG;
+    }
+
+    if (n_band <= (uint32_t)SEL_LIST) {
+        // ---- common case: the whole band fits the list ------------------------------------------------------
+        const uint32_t* all_tok = SOLO ? l_tok : a_tok;
+        const uint32_t* all_key = SOLO ? l_key : a_key;
+        uint32_t my_base = 0u;                                                // this CTA's tokens in the gathered list
+        auto base_of = [&](int q) {                                           // where rank q's begin
+            if (pushed) return (uint32_t)q * RG;
+            uint32_t o = 0u;
+            for (int j = 0; j < q; ++j) o += xc.n_band[j];
+            return o;
+        };
+        if constexpr (!SOLO) {
+            if (!pushed) {                                                    // one rank's share alone exceeds its slots: pull instead
+                cluster.sync();                                               // nobody writes our gathered list any more
+                for (int q = 0; q < C; ++q) {
+                    const uint32_t nq = xc.n_band[q], off = base_of(q);
+                    const uint32_t* st = cluster.map_shared_rank(l_tok, q);
+                    const uint32_t* sk2 = cluster.map_shared_rank(l_key, q);
+                    for (uint32_t i = tid; i < nq; i += SEL_NT) { a_tok[off + i] = st[i]; a_key[off + i] = sk2[i]; }
+                }
+                cluster.sync();
+            }
+            my_base = base_of(r);
+        }
+        // rank band tokens among ALL of them by (exact key descending, index ascending): this CTA's own, and in a cluster
+        // with a short list those of the lower ranks too, whose number says where this CTA's rows begin
         uint32_t* dec = hist;
         const uint32_t take = (uint32_t)kk - n_in;   // >= 1: fewer than kk tokens lie above the band
-        for (uint32_t q2 = warp; q2 < n_band_mine; q2 += NW) {
-            const uint32_t kq = l_key[q2], tq = l_tok[q2];
-            uint32_t c = 0;
-            for (uint32_t j2 = lane; j2 < n_band; j2 += 32) {
-                const uint32_t kj = all_key[j2];
-                c += (kj > kq || (kj == kq && all_tok[j2] < tq)) ? 1u : 0u;
+        const bool rank_all = !SOLO && n_band <= (uint32_t)SEL_RANK_ALL;
+#pragma unroll 1
+        for (int q = rank_all ? 0 : r; q <= r; ++q) {
+            const uint32_t nq = SOLO ? n_band : xc.n_band[q], off = SOLO ? 0u : base_of(q);
+#pragma unroll 1
+            for (uint32_t i = warp; i < nq; i += SEL_NW) {
+                const uint32_t kq = all_key[off + i], tq = all_tok[off + i];
+                uint32_t c = 0;
+#pragma unroll 1
+                for (int p = 0; p < C; ++p) {
+                    const uint32_t np = SOLO ? n_band : xc.n_band[p], offp = SOLO ? 0u : base_of(p);
+                    for (uint32_t j = lane; j < np; j += 32) {
+                        const uint32_t kj = all_key[offp + j];
+                        c += (kj > kq || (kj == kq && all_tok[offp + j] < tq)) ? 1u : 0u;
+                    }
+                }
+                c = __reduce_add_sync(0xffffffffu, c);
+                if (lane == 0) {
+                    if (q == r) dec[i] = c < take ? 1u : 0u;
+                    else if (c < take) atomicAdd(&xc.lower, 1u);
+                }
             }
-            c = __reduce_add_sync(0xffffffffu, c);
-            if (lane == 0) dec[q2] = c < take ? 1u : 0u;
         }
         __syncthreads();
         uint32_t sel = m_in;
         {
             uint32_t pos = my_pos;
-#pragma unroll
-            for (int j = 0; j < EPT; ++j)
-                if (m_band & (1u << j)) { if (dec[pos]) sel |= 1u << j; ++pos; }
+            for (uint32_t m = m_band; m; m &= m - 1u, ++pos)
+                if (dec[pos]) sel |= m & (0u - m);
         }
         uint32_t base = 0u;
         if constexpr (!SOLO) {
-            const uint32_t n_out_mine = sel_block_sum<NW>((uint32_t)__popc(sel), xc, buf);
-            if (tid < C) cluster.map_shared_rank(&xc, tid)->n_out[r] = n_out_mine;
-            cluster.sync();                                                   // [6] counts; nobody reads our lists any more
-            for (int q = 0; q < r; ++q) base += xc.n_out[q];
+            if (rank_all) {
+                base = __reduce_add_sync(0xffffffffu, lane < r ? xc.n_in[lane] : 0u) + xc.lower;
+            } else {
+                const uint32_t n_out_mine = sel_block_sum((uint32_t)__popc(sel), xc, buf);
+                if (tid < C) cluster.map_shared_rank(&xc, tid)->n_out[r] = n_out_mine;
+                cluster.sync();
+                for (int q = 0; q < r; ++q) base += xc.n_out[q];
+            }
         }
         write_out(sel, base);
         if (r == 0 && tid == 0 && A.stats) { A.stats[b * 2] = n_band; A.stats[b * 2 + 1] = n_in; }
@@ -498,65 +516,71 @@ index_select_cluster_kernel(SelArgs A) {
     }
 
     // ---- slow path (tie-dominated scores): the band does not fit the list --------------------------------------
-    // Exact keys replace the approximate ones in the registers: surely-in -> all ones, surely-out -> 0, band ->
-    // exact key (re-scored in chunks of SEL_LIST consecutive tokens, so a chunk's band always fits the list).
-    for (int c0 = r * CH; !VALUES && c0 < min(nt, (r + 1) * CH); c0 += SEL_LIST) {
-        __syncthreads();
-        if (tid == 0) xc.list_n = 0;
-        __syncthreads();
-        const bool mine = i0 >= c0 && i0 < c0 + SEL_LIST;                 // EPT divides SEL_LIST: a thread's tokens share a chunk
-        uint32_t pos0 = 0u;
-        if (mine && m_band) {
-            pos0 = atomicAdd(&xc.list_n, (uint32_t)__popc(m_band));
-            uint32_t pos = pos0;
-#pragma unroll
-            for (int j = 0; j < EPT; ++j)
-                if (m_band & (1u << j)) l_tok[pos++] = (uint32_t)(i0 + j);
+    // Exact keys replace the approximate ones: surely-in -> all ones, surely-out -> 0, band -> exact key (re-scored in chunks
+    // of SEL_LIST consecutive tokens, so a chunk's band always fits the list).
+    if constexpr (!VALUES) {
+#pragma unroll 1
+        for (int ch = 0; ch < nloc; ch += SEL_LIST) {
+            __syncthreads();
+            if (tid == 0) xc.list_n = 0;
+            __syncthreads();
+            // a thread's four tokens of a step lie in one chunk: which of its bits are in this one
+            const int it = ch / SEL_STEP;
+            const bool mine = (it * SEL_NT + tid) * 4 / SEL_LIST == ch / SEL_LIST;
+            const uint32_t bits = mine ? (m_band >> (4 * it)) & 0xfu : 0u;
+            const int i4 = (it * SEL_NT + tid) * 4;
+            uint32_t pos0 = bits ? atomicAdd(&xc.list_n, (uint32_t)__popc(bits)) : 0u;
+            {
+                uint32_t pos = pos0;
+                for (uint32_t m = bits; m; m &= m - 1u) l_tok[pos++] = (uint32_t)(c0 + i4 + __ffs(m) - 1);
+            }
+            __syncthreads();
+            rescore(xc.list_n);
+            __syncthreads();
+            for (uint32_t m = bits; m; m &= m - 1u) keys[i4 + __ffs(m) - 1] = l_key[pos0++];
         }
-        __syncthreads();
-        rescore(xc.list_n);
-        __syncthreads();
-        if (mine) {
-            uint32_t pos = pos0;
-#pragma unroll
-            for (int j = 0; j < EPT; ++j)
-                if (m_band & (1u << j)) key[j] = l_key[pos++];
+#pragma unroll 1
+        for (int bit = 0; bit < 4 * steps; ++bit) {
+            const int i = local_of(bit);
+            if (i < nloc && !((m_band >> bit) & 1u)) keys[i] = ((m_in >> bit) & 1u) ? 0xffffffffu : 0u;
         }
     }
-#pragma unroll
-    for (int j = 0; j < EPT; ++j)
-        if (!VALUES && j < nvalid && !(m_band & (1u << j))) key[j] = ((m_in >> j) & 1u) ? 0xffffffffu : 0u;
     // exact cluster-wide radix selection, four 8-bit digits, MSB first; per-warp histograms so that ties never
-    // serialise a CTA on one bin; whist aliases `hist`, the CTA's digit histogram goes to a_tok[0..256)
+    // serialise a CTA on one bin; whist takes the place of `hist` and both lists, the CTA's digit histogram goes to red[0 .. 256)
     uint32_t pivot = 0u, mask = 0u, need = (uint32_t)kk;
-    uint32_t* whist = hist;                                                   // [NW][256]
+    uint32_t* whist = hist;                                                   // [warps][256]
+    static_assert(SEL_NW * 256 <= SEL_BINS + 2 * SEL_LIST, "the digit histograms fit");
+    uint32_t* dig = red;
+    uint32_t* sum = red + 256;
+    if constexpr (!SOLO) cluster.sync();                                      // nobody reads our lists any more
+#pragma unroll 1
     for (int sh2 = 24; sh2 >= 0; sh2 -= 8) {
         __syncthreads();
-        for (int i = tid; i < NW * 256; i += NT) whist[i] = 0u;
+        for (int i = tid; i < SEL_NW * 256; i += SEL_NT) whist[i] = 0u;
         __syncthreads();
-#pragma unroll
-        for (int j = 0; j < EPT; ++j)
-            if (j < nvalid && (key[j] & mask) == pivot) atomicAdd(&whist[warp * 256 + ((key[j] >> sh2) & 0xffu)], 1u);
+        for_keys([&](int, int, int, uint32_t k) {
+            if ((k & mask) == pivot) atomicAdd(&whist[warp * 256 + ((k >> sh2) & 0xffu)], 1u);
+        });
         __syncthreads();
         if (tid < 256) {
             uint32_t t = 0;
-#pragma unroll
-            for (int w2 = 0; w2 < NW; ++w2) t += whist[w2 * 256 + tid];
-            a_tok[tid] = t;
+#pragma unroll 8
+            for (int w2 = 0; w2 < SEL_NW; ++w2) t += whist[w2 * 256 + tid];
+            dig[tid] = t;
         }
         __syncthreads();
-        cluster.sync();                                                       // every CTA's digit histogram
+        if constexpr (!SOLO) cluster.sync();                                  // every CTA's digit histogram
         if (tid < 256) {
             uint32_t t = 0;
-            for (int q = 0; q < C; ++q) t += cluster.map_shared_rank(a_tok, q)[tid];
-            a_key[tid] = t;
+            for (int q = 0; q < C; ++q) t += SOLO ? dig[tid] : cluster.map_shared_rank(dig, q)[tid];
+            sum[tid] = t;
         }
         __syncthreads();
         if (warp == 0) {
             // lane owns bins 8 * lane .. 8 * lane + 7; acc = entries in strictly higher bins
             uint32_t h[8], tot = 0;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) { h[j] = a_key[lane * 8 + j]; tot += h[j]; }
+            for (int j = 0; j < 8; ++j) { h[j] = sum[lane * 8 + j]; tot += h[j]; }
             uint32_t incl = tot;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -577,39 +601,41 @@ index_select_cluster_kernel(SelArgs A) {
         pivot = xc.pivot;
         need = xc.need;
         mask |= 0xffu << sh2;
-        cluster.sync();                                                       // a_tok may be rewritten by the next digit
+        if constexpr (!SOLO) cluster.sync();                                  // dig may be rewritten by the next digit
     }
-    // `need` of the tokens tied at the pivot are taken, in ascending global index = ascending rank, then thread
+    // `need` of the tokens tied at the pivot are taken, in ascending global index = ascending rank, then token order
     uint32_t sel_gt = 0u, sel_eq = 0u;
-#pragma unroll
-    for (int j = 0; j < EPT; ++j) {
-        if (j < nvalid) {
-            if (key[j] > pivot) sel_gt |= 1u << j;
-            else if (key[j] == pivot) sel_eq |= 1u << j;
+    for_keys([&](int it, int, int e, uint32_t k) {
+        if (k > pivot) sel_gt |= 1u << (4 * it + e);
+        else if (k == pivot) sel_eq |= 1u << (4 * it + e);
+    });
+    uint32_t base = 0u, eq_lower = 0u;
+    if constexpr (!SOLO) {
+        const uint32_t gt_mine = sel_block_sum((uint32_t)__popc(sel_gt), xc, buf);
+        const uint32_t eq_mine = sel_block_sum((uint32_t)__popc(sel_eq), xc, buf);
+        if (tid < C) {
+            SelXc* dst = cluster.map_shared_rank(&xc, tid);
+            dst->cnt_gt[r] = gt_mine; dst->cnt_eq[r] = eq_mine;
+        }
+        cluster.sync();
+        for (int q = 0; q < r; ++q) {
+            const uint32_t left = need > eq_lower ? need - eq_lower : 0u;
+            base += xc.cnt_gt[q] + min(xc.cnt_eq[q], left);
+            eq_lower += xc.cnt_eq[q];
         }
     }
-    const uint32_t gt_mine = sel_block_sum<NW>((uint32_t)__popc(sel_gt), xc, buf);
-    const uint32_t eq_mine = sel_block_sum<NW>((uint32_t)__popc(sel_eq), xc, buf);
-    if (tid < C) {
-        SelXc* dst = cluster.map_shared_rank(&xc, tid);
-        dst->cnt_gt[r] = gt_mine; dst->cnt_eq[r] = eq_mine;
-    }
-    cluster.sync();
-    uint32_t base = 0u, eq_before = 0u;
-    for (int q = 0; q < r; ++q) {
-        const uint32_t left = need > eq_before ? need - eq_before : 0u;
-        base += xc.cnt_gt[q] + min(xc.cnt_eq[q], left);
-        eq_before += xc.cnt_eq[q];
-    }
-    const uint32_t need_mine = need > eq_before ? need - eq_before : 0u;        // ties this CTA may still take
-    const uint32_t eq_excl = sel_block_excl<NW>((uint32_t)__popc(sel_eq), xc);      // ties in this CTA before this thread's
+    const uint32_t need_mine = need > eq_lower ? need - eq_lower : 0u;          // ties this CTA may still take
+    uint32_t ties[SEL_STEPS];
+    sel_token_excl(sel_eq, xc, ties);
     uint32_t sel = sel_gt;
-    {
-        uint32_t e = eq_excl;
 #pragma unroll
-        for (int j = 0; j < EPT; ++j)
-            if (sel_eq & (1u << j)) { if (e < need_mine) sel |= 1u << j; ++e; }
+    for (int it = 0; it < SEL_STEPS; ++it) {
+        uint32_t e0 = ties[it];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (sel_eq & (1u << (4 * it + e))) { if (e0 < need_mine) sel |= 1u << (4 * it + e); ++e0; }
     }
+    __syncthreads();                                                          // (the prefix partials are written again)
     write_out(sel, base);
     if (r == 0 && tid == 0 && A.stats) { A.stats[b * 2] = n_band; A.stats[b * 2 + 1] = 0; }
 }
@@ -620,24 +646,19 @@ namespace rivoli {
 
 static int g_sel_cluster_override = 0;
 
-bool select_cluster_plan(int B, int score_stride, int* cluster, int* ept, int* threads) {
-    // A batch that fills the chip by itself (one CTA per SM) takes ONE CTA of 1024 threads per sequence: no exchange
-    // between CTAs at all. Smaller batches spread a sequence over a cluster of 2 to 8 CTAs of 512 threads, about two
-    // CTAs per SM at most.
-    // Up to 8,192 tokens a lone CTA is faster than a cluster at any batch: what the tokens cost is less than seven cluster
-    // barriers (one sequence: 2,500 tokens 20.5 -> 14.3 us, 4,099 tokens 22.5 -> 18.4 us; 16,384 tokens the other way round).
-    int C = 1, NT = 512;
-    if ((long long)B * 4 < 3 * 148 && score_stride > 8192)   // from three quarters of the SMs on, one CTA per sequence (measured at batch 128: 161 against 166 us per step with clusters of 2)
-        while (C < SEL_MAX_CLUSTER && (long long)B * C * 2 <= 2 * 148) C *= 2;
+// CTAs per sequence: a lone CTA up to 8,192 tokens at any batch (what the tokens cost is less than the cluster barriers), else
+// two or four while each has an SM of its own, and at least enough for 16,384 tokens each. (Eight only when the tokens need
+// them: their barriers cost more than the shorter steps give - one sequence of 16,384 tokens 43.8 us per step with four, 49.4
+// with eight - and at one CTA per SM sixteen such clusters do not fit the chip at once: 16 sequences 61.3 against 80.5.)
+static bool select_cluster_plan(int B, int score_stride, int* cluster, int* ch) {
+    int C = 1;
+    if (score_stride > 8192)
+        while (C < 4 && (long long)B * C * 2 <= 148) C *= 2;
     if (g_sel_cluster_override > 0) C = g_sel_cluster_override;
-    if (C == 1 && (long long)1024 * 16 >= score_stride) NT = 1024;   // 16 keys per thread fit the 64 registers of a 1024-thread CTA
-    for (;;) {
-        for (int e = 4; e <= 32; e *= 2)
-            if ((long long)C * NT * e >= score_stride) { *cluster = C; *ept = e; *threads = NT; return true; }
-        if (C >= SEL_MAX_CLUSTER) return false;
-        C *= 2;
-        NT = 512;
-    }
+    while (C < SEL_MAX_CLUSTER && (long long)C * SEL_CH < score_stride) C *= 2;
+    *cluster = C;
+    *ch = ((score_stride + C - 1) / C + 3) / 4 * 4;
+    return *ch <= SEL_CH;
 }
 
 }  // namespace rivoli
@@ -650,12 +671,13 @@ extern "C" __attribute__((visibility("default"))) void rivoli_index_select_test_
 
 namespace rivoli {
 
-template <bool VALUES>
-static int launch_select(const SelArgs& a, int B, int C, int ept, int nt, cudaStream_t st) {
-    const size_t lists = SEL_BINS + 4 * SEL_LIST;
-    const size_t smem = (lists + (VALUES ? 0 : (size_t)(SEL_HD / 4) * 32 + (size_t)(nt / 32) * SEL_TOK * SEL_HD)) * 4;
+template <bool VALUES, bool SOLO>
+static int launch_select(const SelArgs& a, int B, int C, int ch, cudaStream_t st) {
+    constexpr size_t fixed = SEL_BINS + 2 * SEL_LIST + (VALUES ? SEL_BINS : SEL_NW * SEL_HD * 4 + SEL_HD * 64) + (SOLO ? 0 : 2 * SEL_LIST);
+    static_assert((fixed + SEL_CH) * 4 + sizeof(SelXc) + 1024 <= 232448, "shared memory budget");
+    const size_t smem = (fixed + (size_t)ch) * 4;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(B * C)); cfg.blockDim = dim3((unsigned)nt); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cfg.gridDim = dim3((unsigned)(B * C)); cfg.blockDim = dim3(SEL_NT); cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -663,48 +685,28 @@ static int launch_select(const SelArgs& a, int B, int C, int ept, int nt, cudaSt
     at[1].val.clusterDim.x = (unsigned)C; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
     cfg.attrs = at; cfg.numAttrs = 2;
     rv_drain_error();
-#define RV_SEL(EPT, NT)                                                                             \
-    do {                                                                                            \
-        rv_allow_smem<index_select_cluster_kernel<EPT, NT, VALUES>>((int)smem);                     \
-        (void)cudaLaunchKernelEx(&cfg, index_select_cluster_kernel<EPT, NT, VALUES>, a);            \
-    } while (0)
-    if (nt == 1024) {
-        if (ept == 4) RV_SEL(4, 1024);
-        else if (ept == 8) RV_SEL(8, 1024);
-        else if (ept == 16) RV_SEL(16, 1024);
-        else return 1002;   // the plans take 1024-thread CTAs only up to 16 keys per thread
-    } else {
-        if (ept == 4) RV_SEL(4, 512);
-        else if (ept == 8) RV_SEL(8, 512);
-        else if (ept == 16) RV_SEL(16, 512);
-        else RV_SEL(32, 512);
-    }
-#undef RV_SEL
+    rv_allow_smem<index_select_kernel<VALUES, SOLO>>((int)((fixed + SEL_CH) * 4));
+    (void)cudaLaunchKernelEx(&cfg, index_select_kernel<VALUES, SOLO>, a, ch);
     return rv_launch_status();
 }
 
 int launch_index_select_cluster(const SelArgs& a, int B, cudaStream_t st) {
-    int C = 1, ept = 4, nt = 512;
-    if (!select_cluster_plan(B, a.score_stride, &C, &ept, &nt)) return 1002;
-    return launch_select<false>(a, B, C, ept, nt, st);
+    int C = 1, ch = 0;
+    if (!select_cluster_plan(B, a.score_stride, &C, &ch)) return 1002;
+    return C == 1 ? launch_select<false, true>(a, B, C, ch, st) : launch_select<false, false>(a, B, C, ch, st);
 }
 
 int launch_topk_values(const float* scores, long long stride, const int32_t* seq_len, int nt_single, int B, int k,
                        uint32_t* rows, int32_t* n_sel, int max_nt, cudaStream_t st) {
-    if (max_nt > SEL_MAX_CLUSTER * 512 * 32 || stride > 0x7fffffff) return 1002;
+    if (max_nt > SEL_MAX_CLUSTER * SEL_CH || stride > 0x7fffffff) return 1002;
     SelArgs a{};
     a.scores = scores; a.score_stride = max_nt; a.value_stride = stride; a.seq_len = seq_len; a.nt_single = nt_single;
     a.rows = rows; a.n_sel = n_sel; a.k = k;
-    a.vec_ok = ((uintptr_t)scores & 15) == 0 && stride % 4 == 0;
-    // no re-score to spread: one CTA of 1024 threads up to 16,384 scores (no exchanges between CTAs; 8,193 scores: 9.7 us,
+    a.vec_ok = ((uintptr_t)scores & 15) == 0 && stride % 4 == 0 && stride >= max_nt;   // (whole vectors are read)
+    // no re-score to spread: a lone CTA up to 16,384 scores (no exchanges between CTAs; 8,193 scores: 9.7 us,
     // four radix passes over shared memory took 14.2), beyond that clusters of eight
-    int C = 1, nt = 1024, ept = 4;
-    while (ept < 16 && nt * ept < max_nt) ept *= 2;
-    if (nt * ept < max_nt) {
-        C = SEL_MAX_CLUSTER; nt = 512; ept = 4;
-        while (ept < 32 && (long long)C * nt * ept < max_nt) ept *= 2;
-    }
-    return launch_select<true>(a, B, C, ept, nt, st);
+    const int C = max_nt <= SEL_CH ? 1 : SEL_MAX_CLUSTER, ch = ((max_nt + C - 1) / C + 3) / 4 * 4;
+    return C == 1 ? launch_select<true, true>(a, B, C, ch, st) : launch_select<true, false>(a, B, C, ch, st);
 }
 
 }  // namespace rivoli

@@ -109,3 +109,49 @@ def test_a_page_outside_the_pool_is_flagged_where_nothing_is_scored(lens, top_k)
             assert e.value.code == 1005
         else:
             be.index_select_status(g, st.B, L.score_stride, L.select_scratch)
+
+
+@pytest.mark.parametrize("cluster", [1, 2, 4, 8])
+@pytest.mark.parametrize("kind", ["spread", "front", "ties", "equal"])
+def test_selection_bands_of_every_cluster(cluster, kind):
+    """Bands that end in each branch: a few tokens per CTA; hundreds in one CTA (more than its slots in the others' lists);
+    thousands of ties; all scores equal. Token counts that leave the last step and the last CTA ragged, against exact scores
+    with the exact top-k."""
+    from rivoli_b200 import backend as be
+    be.lib()
+    n, k = 9001, 700
+    st = State(73, 2, [n, 5000], top_k=k)
+    g = make_geom(be.DsaGeom, **st.geom_kw)
+    P = g.page_tokens
+    rows = (st.block_table[0, np.arange(n) // P].astype(np.int64) * P + np.arange(n) % P)
+    pool, scale = st.index_pool.reshape(-1, 128), st.index_scale
+    if kind == "front":        # the first 600 tokens: the same key, at the cut
+        pool[rows[100:700]] = pool[rows[100]]; scale[rows[100:700]] = scale[rows[100]]
+        pool[rows[700:]] = pool[rows[1]]; scale[rows[700:]] = scale[rows[1]] * np.float32(1e-3)
+        pool[rows[:100]] = pool[rows[100]]; scale[rows[:100]] = scale[rows[100]] * np.float32(1.5)
+        st.index_w[0] = np.abs(st.index_w[0])
+    elif kind == "ties":       # six thousand copies of one key
+        pool[rows[1500:7500]] = pool[rows[1500]]; scale[rows[1500:7500]] = scale[rows[1500]]
+    elif kind == "equal":
+        pool[rows] = pool[rows[0]]; scale[rows] = scale[rows[0]]
+    d = {m: dev(getattr(st, m)) for m in ("index_q", "index_w", "index_pool", "index_scale", "block_table", "seq_len")}
+    got = torch.full((2, k), -1, dtype=torch.int32, device="cuda")
+    n_sel = torch.zeros(2, dtype=torch.int32, device="cuda")
+    scratch = torch.zeros(be.index_select_scratch_bytes(g, 2, n), dtype=torch.uint8, device="cuda")
+    be.index_select_test_cluster(cluster)
+    try:
+        be.launch_index_select_paged(g, d["index_q"], d["index_w"], d["index_pool"], d["index_scale"], d["block_table"],
+                                     d["seq_len"], 2, n, got, n_sel, scratch)
+        be.index_select_status(g, 2, n, scratch)
+    finally:
+        be.index_select_test_cluster(0)
+    codes = torch.zeros(2 * 32 * 128, dtype=torch.uint8, device="cuda")
+    qs = torch.zeros(64, device="cuda")
+    scores = torch.zeros((2, n), device="cuda")
+    want, wn = torch.zeros_like(got), torch.zeros_like(n_sel)
+    be.launch_index_q_quant(d["index_q"], 64, 128, codes, qs)
+    be.launch_index_score_paged(g, codes, qs, d["index_w"], d["index_pool"], d["index_scale"], d["block_table"], d["seq_len"], 2, scores, n)
+    s = scores.cpu().numpy()
+    for b, m in enumerate((n, 5000)):
+        order = np.lexsort((np.arange(m), -s[b, :m].astype(np.float64)))[:k]
+        np.testing.assert_array_equal(got[b].cpu().numpy(), np.sort(order))
