@@ -4,8 +4,7 @@
 //   dot = (cd * s_q[h]) * s_k[t];  term_h = (w[h] * wscale) * max(dot * dscale, 0);  score = fold over h ascending.
 // A warp takes four consecutive listed tokens per pass (their loads are in flight together and they share the q values), lane =
 // head (index_heads <= 32), index_dim = 128 (one 4-code word per lane). Two tokens ride in one packed f32x2 multiply-add, each
-// half rounded as the scalar one is; with the tokens of a dim side by side and q as (q, q) pairs that is two multiply-adds and
-// two shared-memory loads per dim for four tokens, half of what scalar folds that decoded q on the fly issued.
+// half rounded as the scalar one is; the tokens of a dim lie side by side.
 #pragma once
 
 #include "codec.cuh"
@@ -13,18 +12,14 @@
 
 constexpr int RS_HD = 128;
 
-// q of one sequence as (q, q) pairs, [dim][head] (lane = head: no bank conflicts); RS_HD * 32 of them, zero for absent heads.
-// All threads of the CTA call it; the caller synchronises afterwards.
-__device__ __forceinline__ void rv_rescore_stage_q(const uint8_t* __restrict__ qcodes_seq, int nh, float2* qq) {
-    for (int e = threadIdx.x; e < 32 * (RS_HD / 4); e += blockDim.x) {
-        const int h = e & 31, d = (e >> 5) * 4;
-        const uint32_t c = h < nh ? *reinterpret_cast<const uint32_t*>(qcodes_seq + (size_t)h * RS_HD + d) : 0u;
-        const float2 x = rv_e4m3x2_to_f32x2((uint16_t)(c & 0xffff)), y = rv_e4m3x2_to_f32x2((uint16_t)(c >> 16));
-        qq[d * 32 + h] = make_float2(x.x, x.x);
-        qq[(d + 1) * 32 + h] = make_float2(x.y, x.y);
-        qq[(d + 2) * 32 + h] = make_float2(y.x, y.x);
-        qq[(d + 3) * 32 + h] = make_float2(y.y, y.y);
-    }
+// Word e of the q codes of one sequence, PACKED as they lie in memory (word w of head h = its dims 4w .. 4w+3) and transposed
+// to [word][head] (lane = head on both sides: no bank conflicts); RS_QWORDS of them. The fold decodes a word into its four
+// values on the fly (exactly): as (q, q) f32 pairs in shared memory they cost eight times its bandwidth, which then bounds the
+// fold (99 tokens on an SM: 14,000 cycles, 6,300 so).
+constexpr int RS_QWORDS = 32 * (RS_HD / 4);
+__device__ __forceinline__ uint32_t rv_rescore_q_word(const uint8_t* __restrict__ qcodes_seq, int nh, int e) {
+    const int h = e & 31, d4 = e >> 5;
+    return h < nh ? *reinterpret_cast<const uint32_t*>(qcodes_seq + (size_t)h * RS_HD + d4 * 4) : 0u;
 }
 
 __device__ __forceinline__ uint64_t rs_fma2(uint64_t a, uint64_t b, uint64_t c) {
@@ -37,7 +32,7 @@ __device__ __forceinline__ uint64_t rs_fma2(uint64_t a, uint64_t b, uint64_t c) 
 // kf = this WARP's staging of four key rows as f32, [dim][token] (RS_HD * 4 floats, 16-byte aligned). my_sq / my_wh = this
 // lane's head scale and weight * wscale (0 for lanes >= nh). emit(position, score) is called by one lane per token.
 template <int WARPS, class Emit>
-__device__ __forceinline__ void rv_rescore_listed(const uint32_t* toks, uint32_t ln, const float2* qq, float* kf,
+__device__ __forceinline__ void rv_rescore_listed(const uint32_t* toks, uint32_t ln, const uint32_t* qf, float* kf,
                                                   const int32_t* __restrict__ bt, const DsaGeom& g,
                                                   const uint8_t* __restrict__ index_pool,
                                                   const float* __restrict__ index_scale, float my_sq, float my_wh,
@@ -72,12 +67,19 @@ __device__ __forceinline__ void rv_rescore_listed(const uint32_t* toks, uint32_t
         dst[3] = make_float4(hi[0].y, hi[1].y, hi[2].y, hi[3].y);
         __syncwarp();
         uint64_t c01 = 0ull, c23 = 0ull;
-#pragma unroll 16
-        for (int d = 0; d < RS_HD; ++d) {
-            const ulonglong2 k4 = reinterpret_cast<const ulonglong2*>(kf)[d];   // broadcast read
-            const uint64_t q2 = reinterpret_cast<const uint64_t*>(qq)[d * 32 + lane];
-            c01 = rs_fma2(q2, k4.x, c01);
-            c23 = rs_fma2(q2, k4.y, c23);
+#pragma unroll 4
+        for (int d = 0; d < RS_HD; d += 4) {
+            const uint32_t qc = qf[d * 8 + lane];
+            const float2 qa = rv_e4m3x2_to_f32x2((uint16_t)(qc & 0xffff)), qb = rv_e4m3x2_to_f32x2((uint16_t)(qc >> 16));
+            const float q4[4] = {qa.x, qa.y, qb.x, qb.y};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const ulonglong2 k4 = reinterpret_cast<const ulonglong2*>(kf)[d + i];   // broadcast read
+                uint64_t q2;
+                asm("mov.b64 %0, {%1, %1};" : "=l"(q2) : "f"(q4[i]));
+                c01 = rs_fma2(q2, k4.x, c01);
+                c23 = rs_fma2(q2, k4.y, c23);
+            }
         }
         const float cd[TOK] = {__uint_as_float((uint32_t)c01), __uint_as_float((uint32_t)(c01 >> 32)),
                                __uint_as_float((uint32_t)c23), __uint_as_float((uint32_t)(c23 >> 32))};

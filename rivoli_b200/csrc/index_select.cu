@@ -38,8 +38,8 @@
 // the slow path instead: every band token is re-scored chunk by chunk, the exact keys replace the approximate
 // ones, and an exact 4 x 8-bit radix selection runs over the whole cluster.
 //
-// A whole step, us, with keys in registers -> now: 4 sequences of 131,072 tokens 85.5 -> 76.1; 32 of up to 32,768 88.3 -> 82.1;
-// 64 of 16,384 104.7 -> 97.2; 128 of 16,384 149.0 -> 145.1; one of 4,099 42.4 -> 39.6.
+// A whole step, us, with keys in registers -> now: 4 sequences of 131,072 tokens 85.5 -> 64.2; 32 of up to 32,768 88.3 -> 80.5;
+// 64 of 16,384 104.7 -> 92.3; 128 of 16,384 149.0 -> 138.6; 16 of 16,384 65.8 -> 56.9; one of 4,099 42.4 -> 38.0.
 #include <cooperative_groups.h>
 
 #include "codec.cuh"
@@ -58,7 +58,7 @@ constexpr int SEL_STEPS = 4, SEL_CH = SEL_STEP * SEL_STEPS;   // most tokens per
 constexpr int SEL_BINS = 4096;
 static_assert(SEL_BINS == SEL_NT * 4, "a thread scans four bins");
 constexpr int SEL_LIST = 2048;     // band tokens per SEQUENCE the fast path holds (and per chunk on the slow path)
-constexpr int SEL_RANK_ALL = 512;  // up to this many band tokens every CTA ranks those of the lower ranks too, instead of one more exchange
+constexpr int SEL_RANK_ALL = SEL_NT;  // up to this many entries of the gathered list every CTA ranks them all, one per thread, instead of one more exchange
 constexpr int SEL_HD = RS_HD;      // index dim (one code word per lane)
 
 struct SelXc {                     // per-CTA exchange block; slot q of an array is written by rank q
@@ -143,12 +143,11 @@ index_select_kernel(SelArgs A, int CH) {
     uint32_t* keys = sel_smem;                                            // [CH]
     uint32_t* hist = keys + CH;                                           // [SEL_BINS]; later `dec`
     uint32_t* l_tok = hist + SEL_BINS;                                    // [SEL_LIST] this CTA's band tokens
-    uint32_t* l_key = l_tok + SEL_LIST;                                   // [SEL_LIST] their exact keys
-    uint32_t* red = l_key + SEL_LIST;                                     // [SEL_BINS] reduced histogram, before the re-score
+    uint64_t* l_cmp = reinterpret_cast<uint64_t*>(l_tok + SEL_LIST);      // [SEL_LIST] their exact keys, ~token below: larger = ranked higher
+    uint32_t* red = l_tok + 3 * SEL_LIST;                                  // [SEL_BINS] reduced histogram, before the re-score
     float* kfw = reinterpret_cast<float*>(red);                           // [warps][SEL_HD][4] key rows as f32
-    float2* qq = reinterpret_cast<float2*>(kfw + SEL_NW * SEL_HD * 4);    // [SEL_HD][32] (q, q) pairs
-    uint32_t* a_tok = VALUES ? red + SEL_BINS : reinterpret_cast<uint32_t*>(qq + SEL_HD * 32);   // [SEL_LIST] the cluster's band (clusters only)
-    uint32_t* a_key = a_tok + SEL_LIST;                                   // [SEL_LIST]
+    uint32_t* qf = red + SEL_NW * SEL_HD * 4;                             // [RS_QWORDS] packed q codes
+    uint64_t* a_cmp = reinterpret_cast<uint64_t*>(VALUES ? red + SEL_BINS : qf + RS_QWORDS);   // [SEL_LIST] the cluster's band (clusters only)
 
     const DsaGeom& g = A.g;
     const int nh = g.index_heads, P = g.page_tokens;
@@ -157,11 +156,27 @@ index_select_kernel(SelArgs A, int CH) {
     // The scorer is launched only when all before it is complete and starts this kernel only then, so everything but its
     // scores may be read before the wait. Given scores come with no such promise.
     if constexpr (VALUES) rv_grid_dep_wait();
+    // (requested before the sequence's length is known: nothing here waits for another load)
+    const int c0 = r * CH, pshift = VALUES ? 0 : 31 - __clz(P);
+    const int32_t* bt = A.block_table + (size_t)b * g.max_pages_per_seq;
+    uint32_t qw = 0u;
+    int pgs[SEL_STEPS];
+    float my_sq = 0.0f, my_wh = 0.0f, cb = 0.0f;                          // head constants of the re-score (nh <= 32); error constant
+    if constexpr (!VALUES) {
+        static_assert(RS_QWORDS == SEL_NT, "a word per thread");
+        qw = rv_rescore_q_word(A.qcodes + (size_t)b * nh * SEL_HD, nh, tid);
+#pragma unroll
+        for (int it = 0; it < SEL_STEPS; ++it) {                          // (the score rows are no longer than the page table)
+            const int i = c0 + it * SEL_STEP + tid * 4;
+            pgs[it] = it * SEL_STEP + tid * 4 < CH && i < A.score_stride ? bt[i >> pshift] : 0;
+        }
+        if (lane < nh) { my_sq = A.qscales[(size_t)b * nh + lane]; my_wh = __fmul_rn(A.w[(size_t)b * nh + lane], g.index_wscale); }
+        cb = A.cb[b];
+    }
     const int nt = min(VALUES && !A.seq_len ? A.nt_single : A.seq_len[b], A.score_stride);
     const int kk = min(A.k, nt);
     uint32_t* out = A.rows + (size_t)b * A.k;
-    const int c0 = r * CH, nloc = max(0, min(CH, nt - c0));              // this CTA's tokens: [c0, c0 + nloc)
-    const int32_t* bt = A.block_table + (size_t)b * g.max_pages_per_seq;
+    const int nloc = max(0, min(CH, nt - c0));                            // this CTA's tokens: [c0, c0 + nloc)
     if (kk == nt || kk <= 0) {                                            // everything (or nothing) is selected: the identity
         if constexpr (!VALUES) rv_grid_dep_wait();
         if (r == 0 && tid == 0 && (!VALUES || A.n_sel)) A.n_sel[b] = kk > 0 ? kk : 0;
@@ -180,9 +195,7 @@ index_select_kernel(SelArgs A, int CH) {
     // ---- 1. approximate keys: (unscaled tensor-core score) * key scale of the token --------------------------
     const float* s = A.scores + (size_t)b * (VALUES ? (size_t)A.value_stride : (size_t)A.score_stride);
     const int steps = (nloc + SEL_STEP - 1) / SEL_STEP;
-    const int pshift = VALUES ? 0 : 31 - __clz(P);
-    auto scale_row = [&](int i) {
-        int pg = bt[i >> pshift];
+    auto scale_row = [&](int i, int pg) {
         pg = (pg < 0 || pg >= g.n_pool_pages) ? 0 : pg;
         return ((size_t)pg << pshift) + (i & (P - 1));
     };
@@ -197,23 +210,19 @@ index_select_kernel(SelArgs A, int CH) {
         }
         *reinterpret_cast<uint4*>(keys + i4) = make_uint4(k[0], k[1], k[2], k[3]);
     };
-    const float my_sq = !VALUES && lane < nh ? A.qscales[(size_t)b * nh + lane] : 0.0f;      // head constants of the re-score (nh <= 32)
-    const float my_wh = !VALUES && lane < nh ? __fmul_rn(A.w[(size_t)b * nh + lane], g.index_wscale) : 0.0f;
     for (int i = tid; i < SEL_BINS / 4; i += SEL_NT) reinterpret_cast<uint4*>(hist)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if constexpr (!SOLO)                                                  // empty slots of the gathered list rank below every token
+        for (int i = tid; i < SEL_LIST; i += SEL_NT) a_cmp[i] = 0ull;
+    if constexpr (!VALUES) qf[tid] = qw;
     if (tid == 0) { xc.list_n = 0; xc.lower = 0; }
     if (A.vec_ok) {
         float4 sk[SEL_STEPS], sc[SEL_STEPS];
         if constexpr (!VALUES) {
-            size_t rr[SEL_STEPS];
 #pragma unroll
             for (int it = 0; it < SEL_STEPS; ++it) {
                 const int i4 = it * SEL_STEP + tid * 4;
-                rr[it] = i4 < nloc ? scale_row(c0 + i4) : 0;
+                sk[it] = i4 < nloc ? *reinterpret_cast<const float4*>(A.index_scale + scale_row(c0 + i4, pgs[it])) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
-#pragma unroll
-            for (int it = 0; it < SEL_STEPS; ++it)
-                sk[it] = it * SEL_STEP + tid * 4 < nloc ? *reinterpret_cast<const float4*>(A.index_scale + rr[it]) : make_float4(0.f, 0.f, 0.f, 0.f);
-            rv_rescore_stage_q(A.qcodes + (size_t)b * nh * SEL_HD, nh, qq);
             rv_grid_dep_wait();
         }
 #pragma unroll
@@ -236,10 +245,7 @@ index_select_kernel(SelArgs A, int CH) {
             }
         }
     } else {
-        if constexpr (!VALUES) {
-            rv_rescore_stage_q(A.qcodes + (size_t)b * nh * SEL_HD, nh, qq);
-            rv_grid_dep_wait();
-        }
+        if constexpr (!VALUES) rv_grid_dep_wait();
 #pragma unroll 1
         for (int it = 0; it < steps; ++it) {
             const int i4 = it * SEL_STEP + tid * 4;
@@ -251,7 +257,7 @@ index_select_kernel(SelArgs A, int CH) {
                 if (i4 + e < nloc) {
                     v[e] = s[c0 + i4 + e];
                     if constexpr (!VALUES) {
-                        const float k1 = A.index_scale[scale_row(c0 + i4 + e)];
+                        const float k1 = A.index_scale[scale_row(c0 + i4 + e, bt[(c0 + i4 + e) >> pshift])];
                         v[e] *= k1;
                         skm = fmaxf(skm, k1);
                     }
@@ -300,7 +306,7 @@ index_select_kernel(SelArgs A, int CH) {
         }
         sk_max = __uint_as_float(sm);
     }
-    const float eps = VALUES ? 0.0f : sk_max * A.cb[b];
+    const float eps = VALUES ? 0.0f : sk_max * cb;
 
     // ---- 2. one histogram pass: 4096 bins spread linearly IN VALUE between the smallest and the largest score ----
     // bin(v) = min(4095, int((v - vmin) * inv_w)) is monotone in v, which is all the selection needs: tokens in
@@ -386,7 +392,7 @@ index_select_kernel(SelArgs A, int CH) {
         for (uint32_t m = m_band; m && pos < SEL_LIST; m &= m - 1u, ++pos) {
             const int i = local_of(__ffs(m) - 1);
             l_tok[pos] = (uint32_t)(c0 + i);
-            if (VALUES) l_key[pos] = keys[i];
+            if (VALUES) l_cmp[pos] = ((uint64_t)keys[i] << 32) | ~(uint32_t)(c0 + i);
         }
     }
     __syncthreads();
@@ -394,12 +400,13 @@ index_select_kernel(SelArgs A, int CH) {
     buf ^= 1;
     const uint32_t n_band_mine = xc.list_n;
 
-    // Exact key of the first `ln` listed tokens -> l_key[position] (0 and ~0 are reserved for "surely out" / "surely in").
+    // Exact key of the first `ln` listed tokens -> l_cmp[position] (0 and ~0 are reserved for "surely out" / "surely in").
     auto rescore = [&](uint32_t ln) {
-        rv_rescore_listed<SEL_NW>(l_tok, ln, qq, kfw + warp * (SEL_HD * 4), bt, g, A.index_pool, A.index_scale, my_sq, my_wh,
+        rv_rescore_listed<SEL_NW>(l_tok, ln, qf, kfw + warp * (SEL_HD * 4), bt, g, A.index_pool, A.index_scale, my_sq, my_wh,
                                   [&](uint32_t pos, float score) {
             uint32_t ku = topk_key(score);
-            l_key[pos] = ku == 0xffffffffu ? 0xfffffffeu : (ku == 0u ? 1u : ku);
+            ku = ku == 0xffffffffu ? 0xfffffffeu : (ku == 0u ? 1u : ku);
+            l_cmp[pos] = ((uint64_t)ku << 32) | ~l_tok[pos];
         });
     };
     // ascending write-out of this CTA's tokens whose bit is set in `sel`, from slot `base` on (one barrier)
@@ -422,74 +429,70 @@ index_select_kernel(SelArgs A, int CH) {
     }
     uint32_t n_in = n_in_mine, n_band = n_band_mine;
     const uint32_t RG = SEL_LIST / C;                                         // entries of one rank in everybody's gathered list
-    bool pushed = true;
+    uint32_t n_all = n_band_mine;                                             // gathered entries, empty slots included
     if constexpr (!SOLO) {
-        {   // a warp serves one destination
+        {   // a warp serves one destination; entry i of rank r goes to slot i * C + r, so that the lists end close together
             const int q = warp & (C - 1);
-            uint32_t* dt = cluster.map_shared_rank(a_tok, q) + r * RG;
-            uint32_t* dk = cluster.map_shared_rank(a_key, q) + r * RG;
-            for (uint32_t i = (warp / C) * 32 + lane; i < min(n_band_mine, RG); i += (SEL_NW / C) * 32) { dt[i] = l_tok[i]; dk[i] = l_key[i]; }
+            uint64_t* dst = cluster.map_shared_rank(a_cmp, q) + r;
+            for (uint32_t i = (warp / C) * 32 + lane; i < min(n_band_mine, RG); i += (SEL_NW / C) * 32) dst[i * C] = l_cmp[i];
             if (tid < C) {
-                SelXc* dst = cluster.map_shared_rank(&xc, tid);
-                dst->n_in[r] = n_in_mine; dst->n_band[r] = n_band_mine;
+                SelXc* dx = cluster.map_shared_rank(&xc, tid);
+                dx->n_in[r] = n_in_mine; dx->n_band[r] = n_band_mine;
             }
         }
         cluster.sync();                                                       // [4] counts and lists
         const uint32_t nb = lane < C ? xc.n_band[lane] : 0u;
         n_in = __reduce_add_sync(0xffffffffu, lane < C ? xc.n_in[lane] : 0u);
         n_band = __reduce_add_sync(0xffffffffu, nb);
-        pushed = __reduce_max_sync(0xffffffffu, nb) <= RG;
+        n_all = __reduce_max_sync(0xffffffffu, nb) * C;
     }
 
     if (n_band <= (uint32_t)SEL_LIST) {
         // ---- common case: the whole band fits the list ------------------------------------------------------
-        const uint32_t* all_tok = SOLO ? l_tok : a_tok;
-        const uint32_t* all_key = SOLO ? l_key : a_key;
-        uint32_t my_base = 0u;                                                // this CTA's tokens in the gathered list
-        auto base_of = [&](int q) {                                           // where rank q's begin
-            if (pushed) return (uint32_t)q * RG;
-            uint32_t o = 0u;
-            for (int j = 0; j < q; ++j) o += xc.n_band[j];
-            return o;
-        };
-        if constexpr (!SOLO) {
-            if (!pushed) {                                                    // one rank's share alone exceeds its slots: pull instead
-                cluster.sync();                                               // nobody writes our gathered list any more
-                for (int q = 0; q < C; ++q) {
-                    const uint32_t nq = xc.n_band[q], off = base_of(q);
-                    const uint32_t* st = cluster.map_shared_rank(l_tok, q);
-                    const uint32_t* sk2 = cluster.map_shared_rank(l_key, q);
-                    for (uint32_t i = tid; i < nq; i += SEL_NT) { a_tok[off + i] = st[i]; a_key[off + i] = sk2[i]; }
+        const uint64_t* all_cmp = SOLO ? l_cmp : a_cmp;
+        const uint32_t take = (uint32_t)kk - n_in;   // >= 1: fewer than kk tokens lie above the band
+        uint32_t* dec = hist;                                                 // per own list entry: selected
+        uint32_t base = 0u;
+        // Band tokens are ranked among ALL of them by (exact key descending, index ascending).
+        const bool rank_all = n_all <= (uint32_t)SEL_RANK_ALL;
+        if (rank_all) {
+            // an entry per thread; the selected ones of the lower ranks say where this CTA's rows begin
+            if (tid < (int)n_all) {
+                const uint64_t mine = all_cmp[tid];
+                uint32_t c = 0;
+                uint32_t j = 0;
+#pragma unroll 4
+                for (; j + 2 <= n_all; j += 2) {                              // broadcast reads of two entries
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(all_cmp + j);
+                    c += (v.x > mine ? 1u : 0u) + (v.y > mine ? 1u : 0u);
                 }
+                if (j < n_all) c += all_cmp[j] > mine ? 1u : 0u;
+                const bool win = c < take;
+                const int q = SOLO ? 0 : tid & (C - 1);
+                if (q == r) dec[SOLO ? tid : tid / C] = win ? 1u : 0u;        // (an empty slot's entry is never looked at)
+                else if (q < r && win && mine != 0ull) atomicAdd(&xc.lower, 1u);
+            }
+        } else {
+            if (!SOLO && n_all > (uint32_t)SEL_LIST) {                        // one rank's share alone exceeds its slots: pull instead
+                cluster.sync();                                               // nobody writes our gathered list any more
+                uint32_t off = 0u;
+                for (int q = 0; q < C; ++q) {
+                    const uint32_t nq = xc.n_band[q];
+                    const uint64_t* src = cluster.map_shared_rank(l_cmp, q);
+                    for (uint32_t i = tid; i < nq; i += SEL_NT) a_cmp[off + i] = src[i];
+                    off += nq;
+                }
+                n_all = n_band;
                 cluster.sync();
             }
-            my_base = base_of(r);
-        }
-        // rank band tokens among ALL of them by (exact key descending, index ascending): this CTA's own, and in a cluster
-        // with a short list those of the lower ranks too, whose number says where this CTA's rows begin
-        uint32_t* dec = hist;
-        const uint32_t take = (uint32_t)kk - n_in;   // >= 1: fewer than kk tokens lie above the band
-        const bool rank_all = !SOLO && n_band <= (uint32_t)SEL_RANK_ALL;
 #pragma unroll 1
-        for (int q = rank_all ? 0 : r; q <= r; ++q) {
-            const uint32_t nq = SOLO ? n_band : xc.n_band[q], off = SOLO ? 0u : base_of(q);
-#pragma unroll 1
-            for (uint32_t i = warp; i < nq; i += SEL_NW) {
-                const uint32_t kq = all_key[off + i], tq = all_tok[off + i];
+            for (uint32_t i = warp; i < n_band_mine; i += SEL_NW) {           // a warp per own entry
+                const uint64_t mine = l_cmp[i];
                 uint32_t c = 0;
-#pragma unroll 1
-                for (int p = 0; p < C; ++p) {
-                    const uint32_t np = SOLO ? n_band : xc.n_band[p], offp = SOLO ? 0u : base_of(p);
-                    for (uint32_t j = lane; j < np; j += 32) {
-                        const uint32_t kj = all_key[offp + j];
-                        c += (kj > kq || (kj == kq && all_tok[offp + j] < tq)) ? 1u : 0u;
-                    }
-                }
+#pragma unroll 4
+                for (uint32_t j = lane; j < n_all; j += 32) c += all_cmp[j] > mine ? 1u : 0u;
                 c = __reduce_add_sync(0xffffffffu, c);
-                if (lane == 0) {
-                    if (q == r) dec[i] = c < take ? 1u : 0u;
-                    else if (c < take) atomicAdd(&xc.lower, 1u);
-                }
+                if (lane == 0) dec[i] = c < take ? 1u : 0u;
             }
         }
         __syncthreads();
@@ -499,7 +502,6 @@ index_select_kernel(SelArgs A, int CH) {
             for (uint32_t m = m_band; m; m &= m - 1u, ++pos)
                 if (dec[pos]) sel |= m & (0u - m);
         }
-        uint32_t base = 0u;
         if constexpr (!SOLO) {
             if (rank_all) {
                 base = __reduce_add_sync(0xffffffffu, lane < r ? xc.n_in[lane] : 0u) + xc.lower;
@@ -537,7 +539,7 @@ index_select_kernel(SelArgs A, int CH) {
             __syncthreads();
             rescore(xc.list_n);
             __syncthreads();
-            for (uint32_t m = bits; m; m &= m - 1u) keys[i4 + __ffs(m) - 1] = l_key[pos0++];
+            for (uint32_t m = bits; m; m &= m - 1u) keys[i4 + __ffs(m) - 1] = (uint32_t)(l_cmp[pos0++] >> 32);
         }
 #pragma unroll 1
         for (int bit = 0; bit < 4 * steps; ++bit) {
@@ -549,7 +551,7 @@ index_select_kernel(SelArgs A, int CH) {
     // serialise a CTA on one bin; whist takes the place of `hist` and both lists, the CTA's digit histogram goes to red[0 .. 256)
     uint32_t pivot = 0u, mask = 0u, need = (uint32_t)kk;
     uint32_t* whist = hist;                                                   // [warps][256]
-    static_assert(SEL_NW * 256 <= SEL_BINS + 2 * SEL_LIST, "the digit histograms fit");
+    static_assert(SEL_NW * 256 <= SEL_BINS + 3 * SEL_LIST, "the digit histograms fit");
     uint32_t* dig = red;
     uint32_t* sum = red + 256;
     if constexpr (!SOLO) cluster.sync();                                      // nobody reads our lists any more
@@ -648,8 +650,8 @@ static int g_sel_cluster_override = 0;
 
 // CTAs per sequence: a lone CTA up to 8,192 tokens at any batch (what the tokens cost is less than the cluster barriers), else
 // two or four while each has an SM of its own, and at least enough for 16,384 tokens each. (Eight only when the tokens need
-// them: their barriers cost more than the shorter steps give - one sequence of 16,384 tokens 43.8 us per step with four, 49.4
-// with eight - and at one CTA per SM sixteen such clusters do not fit the chip at once: 16 sequences 61.3 against 80.5.)
+// them: their barriers cost what the shorter steps give, and at one CTA per SM sixteen such clusters do not fit the chip at
+// once: 16 sequences of 16,384 tokens 61 us per step with four, 80 with eight.)
 static bool select_cluster_plan(int B, int score_stride, int* cluster, int* ch) {
     int C = 1;
     if (score_stride > 8192)
@@ -673,7 +675,7 @@ namespace rivoli {
 
 template <bool VALUES, bool SOLO>
 static int launch_select(const SelArgs& a, int B, int C, int ch, cudaStream_t st) {
-    constexpr size_t fixed = SEL_BINS + 2 * SEL_LIST + (VALUES ? SEL_BINS : SEL_NW * SEL_HD * 4 + SEL_HD * 64) + (SOLO ? 0 : 2 * SEL_LIST);
+    constexpr size_t fixed = SEL_BINS + 3 * SEL_LIST + (VALUES ? SEL_BINS : SEL_NW * SEL_HD * 4 + RS_QWORDS) + (SOLO ? 0 : 2 * SEL_LIST);
     static_assert((fixed + SEL_CH) * 4 + sizeof(SelXc) + 1024 <= 232448, "shared memory budget");
     const size_t smem = (fixed + (size_t)ch) * 4;
     cudaLaunchConfig_t cfg = {};

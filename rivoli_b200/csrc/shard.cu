@@ -46,8 +46,8 @@ shard_rescore_kernel(DsaGeom g, const uint8_t* __restrict__ qcodes, const float*
                      const float* __restrict__ index_scale, const int32_t* __restrict__ block_table,
                      const uint32_t* __restrict__ rows, const int32_t* __restrict__ n_sel, float* __restrict__ cand) {
     extern __shared__ __align__(16) float sr_smem[];
-    float2* qq = reinterpret_cast<float2*>(sr_smem);       // [RS_HD][32] (q, q) pairs
-    float* kfw = sr_smem + RS_HD * 64;                     // [SH_WARPS][RS_HD][SH_TOK]
+    uint32_t* qf = reinterpret_cast<uint32_t*>(sr_smem);   // [RS_QWORDS] packed q codes
+    float* kfw = sr_smem + RS_QWORDS;                      // [SH_WARPS][RS_HD][SH_TOK]
     const int b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nh = g.index_heads, k = g.top_k;
     const int per_cta = SH_WARPS * SH_TOK * 4;             // candidate slots of one CTA
@@ -57,11 +57,11 @@ shard_rescore_kernel(DsaGeom g, const uint8_t* __restrict__ qcodes, const float*
     for (int j = j0 + tid; j < min(k, j0 + per_cta); j += SH_THREADS)
         if (j >= n) out[j] = -INFINITY;                    // dead slots never beat a live candidate
     if (j0 >= n) return;
-    rv_rescore_stage_q(qcodes + (size_t)b * nh * RS_HD, nh, qq);
+    for (int e = tid; e < RS_QWORDS; e += SH_THREADS) qf[e] = rv_rescore_q_word(qcodes + (size_t)b * nh * RS_HD, nh, e);
     __syncthreads();
     const float my_sq = lane < nh ? qscales[(size_t)b * nh + lane] : 0.0f;
     const float my_wh = lane < nh ? __fmul_rn(w[(size_t)b * nh + lane], g.index_wscale) : 0.0f;
-    rv_rescore_listed<SH_WARPS>(rows + (size_t)b * k + j0, (uint32_t)min(per_cta, n - j0), qq,
+    rv_rescore_listed<SH_WARPS>(rows + (size_t)b * k + j0, (uint32_t)min(per_cta, n - j0), qf,
                                         kfw + warp * (SH_TOK * RS_HD), block_table + (size_t)b * g.max_pages_per_seq, g,
                                         index_pool, index_scale, my_sq, my_wh,
                                         [&](uint32_t pos, float score) { out[j0 + pos] = score; });
@@ -199,7 +199,7 @@ RIVOLI_API int rivoli_shard_candidates(const DsaGeom* g, const uint16_t* index_q
         return e;
     const uint8_t* qcodes; const float* qscales;
     rivoli_index_select_query_codes(g, B, score_stride, select_scratch, &qcodes, &qscales);
-    const size_t smem = ((size_t)RS_HD * 64 + (size_t)SH_WARPS * SH_TOK * RS_HD) * 4;
+    const size_t smem = ((size_t)RS_QWORDS + (size_t)SH_WARPS * SH_TOK * RS_HD) * 4;
     const int per_cta = SH_WARPS * SH_TOK * 4;
     rv_drain_error();
     cudaFuncSetAttribute(shard_rescore_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
