@@ -433,60 +433,66 @@ attend_mma_kernel(AttendMmaArgs A) {
     } else if (warp == AM_QKW) {
         // ------------------------------ QK issuer -------------------------------------------------
         // The two MMA streams, QK(0..n-1) and PV(0..n-1), are each in order and are issued by ONE thread each, from two
-        // warps: a thread blocks on the barriers of its own next instruction group only, so neither stream's control
+        // warps: a warp blocks on the barriers of its own next instruction group only, so neither stream's control
         // latency (barrier observed -> fence -> issue -> commit) sits in the other's way and the tensor pipe takes
         // whichever group arrives first. QK runs ahead of the softmax by up to the four S buffers / ring stages.
-        if (lane == 0 && ntiles > 0) {
+        if (ntiles > 0) {
             const uint32_t id_qk = tc::idesc_e4m3(128, AM_TILE, 0, 0);
             const uint64_t d_qr = smem_desc(tc::smem_u32(smem + SM_QR), 16, 512, 4);
-            bool ok = tc::mbar_wait(&bars.q_full, 0, abort_flag, 51, A.max_polls);
+            bool ok = tc::mbar_wait_warp(&bars.q_full, 0, abort_flag, 51, A.max_polls);
             for (int i = 0; i < ntiles && ok; ++i) {   // S(i) = Qcat . K(i)^T
                 const int s = i % AM_STAGES, use = i / AM_STAGES, rb = i % AM_ROPES, sb = i % AM_SBUF, suse = i / AM_SBUF;
-                ok = tc::mbar_wait(&bars.k_full[s], use & 1, abort_flag, 52, A.max_polls) &&
-                     tc::mbar_wait(&bars.s_empty[sb], (suse & 1) ^ 1, abort_flag, 53, A.max_polls);
+                ok = tc::mbar_wait_warp(&bars.k_full[s], use & 1, abort_flag, 52, A.max_polls) &&
+                     tc::mbar_wait_warp(&bars.s_empty[sb], (suse & 1) ^ 1, abort_flag, 53, A.max_polls);
                 if (!ok) break;
                 tc::fence_proxy_async();   // the copies wrote through the generic proxy, the MMAs read through the async one
                 tc::tc_fence_after();
                 const uint64_t d_k = smem_desc(tc::smem_u32(smem + SM_K0 + s * SM_KSTAGE), 16, 1024, 2);
                 const uint64_t d_rope = smem_desc(tc::smem_u32(smem + SM_ROPE + rb * SM_ROPEBUF), 16, 512, 4);
                 const uint32_t d = TM_S0 + sb * AM_TILE;
-                // rope columns first (A from shared memory): their tile is released as soon as these two are done
+                if (tc::elect_one()) {
+                    // rope columns first (A from shared memory): their tile is released as soon as these two are done
 #pragma unroll
-                for (int k = 0; k < 2; ++k) tc::mma_f8(d, d_qr + (uint64_t)(k * 2), d_rope + (uint64_t)(k * 2), id_qk, k != 0);
-                tc::mma_commit(&bars.rope_free[rb]);
+                    for (int k = 0; k < 2; ++k) tc::mma_f8(d, d_qr + (uint64_t)(k * 2), d_rope + (uint64_t)(k * 2), id_qk, k != 0);
+                    tc::mma_commit(&bars.rope_free[rb]);
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
+                    for (int c = 0; c < 4; ++c)
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)   // A from tensor memory: 32 codes = 8 columns per step; descriptor address fields count 16-byte units
-                        tc::mma_f8_ta(d, TM_Q + (uint32_t)(c * 32 + k * 8), d_k + (uint64_t)((c * SM_KCHUNK + k * 32) >> 4), id_qk, 1);
-                tc::mma_commit(&bars.s_full[sb]);
+                        for (int k = 0; k < 4; ++k)   // A from tensor memory: 32 codes = 8 columns per step; descriptor address fields count 16-byte units
+                            tc::mma_f8_ta(d, TM_Q + (uint32_t)(c * 32 + k * 8), d_k + (uint64_t)((c * SM_KCHUNK + k * 32) >> 4), id_qk, 1);
+                    tc::mma_commit(&bars.s_full[sb]);
+                }
+                __syncwarp();
             }
         }
     } else if (warp == AM_PVW) {
         // ------------------------------ PV issuer -------------------------------------------------
-        if (lane == 0 && ntiles > 0) {
+        if (ntiles > 0) {
             const uint32_t id_pv = tc::idesc_e4m3(128, AM_H, 1, 0);
             const uint64_t d_phi = smem_desc(tc::smem_u32(smem + SM_P), 16, 512, 4);
             const uint64_t d_plo = smem_desc(tc::smem_u32(smem + SM_P + SM_PTERM), 16, 512, 4);
             bool ok = true;
             for (int j = 0; j < ntiles && ok; ++j) {   // O^T += V(j)^T . P'(j)
                 const int s = j % AM_STAGES;
-                ok = tc::mbar_wait(&bars.p_full, j & 1, abort_flag, 54, A.max_polls);
+                ok = tc::mbar_wait_warp(&bars.p_full, j & 1, abort_flag, 54, A.max_polls);
                 if (!ok) break;
                 tc::fence_proxy_async();
                 tc::tc_fence_after();
                 const uint64_t d_v = smem_desc(tc::smem_u32(smem + SM_K0 + s * SM_KSTAGE), SM_KCHUNK, 1024, 2);
+                if (tc::elect_one()) {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
+                    for (int c = 0; c < 4; ++c) {
 #pragma unroll
-                    for (int k = 0; k < 2; ++k)   // p_hi
-                        tc::mma_f8(TM_O + c * 64, d_v + (uint64_t)((c * SM_KCHUNK + k * 4096) >> 4), d_phi + (uint64_t)(k * 2), id_pv, (j | k) != 0);
+                        for (int k = 0; k < 2; ++k)   // p_hi
+                            tc::mma_f8(TM_O + c * 64, d_v + (uint64_t)((c * SM_KCHUNK + k * 4096) >> 4), d_phi + (uint64_t)(k * 2), id_pv, (j | k) != 0);
 #pragma unroll
-                    for (int k = 0; k < 2; ++k)   // p_lo, same accumulator
-                        tc::mma_f8(TM_O + c * 64, d_v + (uint64_t)((c * SM_KCHUNK + k * 4096) >> 4), d_plo + (uint64_t)(k * 2), id_pv, 1);
+                        for (int k = 0; k < 2; ++k)   // p_lo, same accumulator
+                            tc::mma_f8(TM_O + c * 64, d_v + (uint64_t)((c * SM_KCHUNK + k * 4096) >> 4), d_plo + (uint64_t)(k * 2), id_pv, 1);
+                    }
+                    tc::mma_commit(&bars.k_empty[s]);
+                    tc::mma_commit(&bars.pv_done);
                 }
-                tc::mma_commit(&bars.k_empty[s]);
-                tc::mma_commit(&bars.pv_done);
+                __syncwarp();
             }
         }
     } else if (warp < AM_SW) {

@@ -259,7 +259,7 @@ front_gemm_mma_kernel(FrontArgs A) {
             s0 = n0s; s1 = n1s;
             tc::fence_proxy_async();
             __syncthreads();
-            if (tid == 0) {
+            if (warp == 0 && tc::elect_one()) {
                 tc::tc_fence_after();
                 const uint64_t d_a = fm_desc(tc::smem_u32(st)), d_b = fm_desc(tc::smem_u32(sB));
 #pragma unroll

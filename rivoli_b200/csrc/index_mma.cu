@@ -333,7 +333,7 @@ index_score_mma_kernel(IndexMmaArgs A, const __grid_constant__ CUtensorMap tm_ke
                      tc::mbar_wait_warp(&bars.tempty[a], ((it / IM_NACC) & 1) ^ 1, &abort_flag, 22);
                 if (!ok) break;
                 tc::tc_fence_after();
-                if (lane == 0) {
+                if (tc::elect_one()) {
                     const uint32_t ka = tc::smem_u32(s_keys + s * IM_STAGE_BYTES), qa = tc::smem_u32(s_q + qb * IM_Q_BYTES);
 #pragma unroll
                     for (int k = 0; k < IM_HD / 32; ++k)

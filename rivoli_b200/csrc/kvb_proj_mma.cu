@@ -190,7 +190,7 @@ kvb_absorb_mma_kernel(KpArgs A) {
             }
             tc::fence_proxy_async();
             __syncthreads();
-            if (tid == 0) {
+            if (warp == 0 && tc::elect_one()) {
                 tc::tc_fence_after();
                 const uint32_t a0 = tc::smem_u32(sA + c * KP_ACHUNK), w0 = tc::smem_u32(sb);
                 const int run = c * 64 >= cut ? 1 : 0;       // (a run boundary is a multiple of 64)
@@ -305,7 +305,7 @@ kvb_value_mma_kernel(KpArgs A) {
             }
             tc::fence_proxy_async();
             __syncthreads();
-            if (tid == 0) {
+            if (warp == 0 && tc::elect_one()) {
                 tc::tc_fence_after();
                 const uint32_t a0 = tc::smem_u32(sA + c * KP_ACHUNK), w0 = tc::smem_u32(sb);
 #pragma unroll

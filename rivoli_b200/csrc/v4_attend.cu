@@ -255,44 +255,50 @@ __global__ void __launch_bounds__(SA_THREADS, 1) v4_sparse_attend_kernel(SaArgs 
         tc::cp_async_commit();
         tc::cp_async_wait<0>();              // (an aborted CTA leaves no copy in flight)
     } else if (warp == SA_QKW) {
-        if (lane == 0 && ntiles > 0) {
+        if (ntiles > 0) {
             const uint32_t id = sa_idesc(SA_TILE, SA_H, 0, 0);
             const uint64_t dq = tc::smem_desc_sw128(tc::smem_u32(sa_smem + SA_SQ), 16, 1024);
-            bool ok = tc::mbar_wait(&bars.q_full, 0, abort_flag, 92);
+            bool ok = tc::mbar_wait_warp(&bars.q_full, 0, abort_flag, 92);
             for (int t = 0; t < ntiles && ok; ++t) {
                 const int s = t & 1;
-                ok = tc::mbar_wait(&bars.k_full[s], (t >> 1) & 1, abort_flag, 93) &&
-                     tc::mbar_wait(&bars.s_empty[s], ((t >> 1) & 1) ^ 1, abort_flag, 94);
+                ok = tc::mbar_wait_warp(&bars.k_full[s], (t >> 1) & 1, abort_flag, 93) &&
+                     tc::mbar_wait_warp(&bars.s_empty[s], ((t >> 1) & 1) ^ 1, abort_flag, 94);
                 if (!ok) break;
                 tc::fence_proxy_async();     // the copies wrote through the generic proxy, the MMAs read through the async one
                 tc::tc_fence_after();
                 const uint64_t dk = tc::smem_desc_sw128(tc::smem_u32(sa_smem + s * SA_KSTAGE), 16, 1024);
+                if (tc::elect_one()) {
 #pragma unroll
-                for (int k = 0; k < SA_D / 16; ++k) {   // four steps of 32 bytes per chunk; address fields count 16-byte units
-                    const uint64_t off = (uint64_t)(((k >> 2) * SA_CHUNK + (k & 3) * 32) >> 4);
-                    sa_mma(TM_S + s * SA_H, dk + off, dq + off, id, k != 0);
+                    for (int k = 0; k < SA_D / 16; ++k) {   // four steps of 32 bytes per chunk; address fields count 16-byte units
+                        const uint64_t off = (uint64_t)(((k >> 2) * SA_CHUNK + (k & 3) * 32) >> 4);
+                        sa_mma(TM_S + s * SA_H, dk + off, dq + off, id, k != 0);
+                    }
+                    tc::mma_commit(&bars.s_full[s]);
                 }
-                tc::mma_commit(&bars.s_full[s]);
+                __syncwarp();
             }
         }
     } else if (warp == SA_PVW) {
-        if (lane == 0 && ntiles > 0) {
+        if (ntiles > 0) {
             const uint32_t id = sa_idesc(128, SA_H, 1, 1);
             bool ok = true;
             for (int t = 0; t < ntiles && ok; ++t) {
                 const int s = t & 1;
-                ok = tc::mbar_wait(&bars.p_full[s], (t >> 1) & 1, abort_flag, 95);
+                ok = tc::mbar_wait_warp(&bars.p_full[s], (t >> 1) & 1, abort_flag, 95);
                 if (!ok) break;
                 tc::fence_proxy_async();
                 tc::tc_fence_after();
                 const uint64_t dv = tc::smem_desc_sw128(tc::smem_u32(sa_smem + s * SA_KSTAGE), SA_CHUNK, 1024);
                 const uint64_t dp = tc::smem_desc_sw128(tc::smem_u32(sa_smem + SA_SP + s * SA_PBUF), 16, 1024);
+                if (tc::elect_one()) {
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
+                    for (int c = 0; c < 4; ++c)
 #pragma unroll
-                    for (int k = 0; k < SA_TILE / 16; ++k)   // sixteen tokens = two groups of eight rows
-                        sa_mma(TM_O + c * SA_H, dv + (uint64_t)((2 * c * SA_CHUNK + k * 2048) >> 4), dp + (uint64_t)((k * 2048) >> 4), id, (t | k) != 0);
-                tc::mma_commit(&bars.k_empty[s]);
+                        for (int k = 0; k < SA_TILE / 16; ++k)   // sixteen tokens = two groups of eight rows
+                            sa_mma(TM_O + c * SA_H, dv + (uint64_t)((2 * c * SA_CHUNK + k * 2048) >> 4), dp + (uint64_t)((k * 2048) >> 4), id, (t | k) != 0);
+                    tc::mma_commit(&bars.k_empty[s]);
+                }
+                __syncwarp();
             }
         }
     } else {

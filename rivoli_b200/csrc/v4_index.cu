@@ -431,19 +431,19 @@ __global__ void __launch_bounds__(ST_THREADS) v4_score_tc_kernel(StArgs A, const
     } else if (warp == 5) {
         // instruction descriptor, kind::i8: s8 x s8 -> s32
         const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((64u >> 3) << 17) | ((uint32_t)(ST_TILE >> 4) << 24);
-        if (lane == 0)
-            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-                if (!item_rows(item, b, t0, t1, n)) continue;
-                const int qb = done & 1;
-                ok = tc::mbar_wait(&bars.qfull[qb], (done >> 1) & 1, &abort_flag, 20);
-                for (int t = t0; t < t1 && ok; ++t, ++it) {
-                    const int s = it % ST_NS, a = it % ST_NACC;
-                    ok = tc::mbar_wait(&bars.full[s], (it / ST_NS) & 1, &abort_flag, 21) &&
-                         tc::mbar_wait(&bars.tempty[a], ((it / ST_NACC) & 1) ^ 1, &abort_flag, 22);
-                    if (!ok) break;
-                    tc::tc_fence_after();
-                    const uint64_t dk = tc::smem_desc_sw128(tc::smem_u32(smem + s * ST_STAGE), 16, 1024);
-                    const uint64_t dq = tc::smem_desc_sw128(tc::smem_u32(s_q + qb * ST_Q_BYTES), 16, 1024);
+        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+            if (!item_rows(item, b, t0, t1, n)) continue;
+            const int qb = done & 1;
+            ok = tc::mbar_wait_warp(&bars.qfull[qb], (done >> 1) & 1, &abort_flag, 20);
+            for (int t = t0; t < t1 && ok; ++t, ++it) {
+                const int s = it % ST_NS, a = it % ST_NACC;
+                ok = tc::mbar_wait_warp(&bars.full[s], (it / ST_NS) & 1, &abort_flag, 21) &&
+                     tc::mbar_wait_warp(&bars.tempty[a], ((it / ST_NACC) & 1) ^ 1, &abort_flag, 22);
+                if (!ok) break;
+                tc::tc_fence_after();
+                const uint64_t dk = tc::smem_desc_sw128(tc::smem_u32(smem + s * ST_STAGE), 16, 1024);
+                const uint64_t dq = tc::smem_desc_sw128(tc::smem_u32(s_q + qb * ST_Q_BYTES), 16, 1024);
+                if (tc::elect_one()) {
 #pragma unroll
                     for (int k = 0; k < 4; ++k)
                         asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -452,8 +452,10 @@ __global__ void __launch_bounds__(ST_THREADS) v4_score_tc_kernel(StArgs A, const
                     tc::mma_commit(&bars.empty[s]);
                     tc::mma_commit(&bars.tfull[a]);
                 }
-                ++done;
+                __syncwarp();
             }
+            ++done;
+        }
     } else if (warp >= 6) {
         // ---- query of an item: thread = (head, half of the 128 dims), two blocks of 32 each
         const int t = tid - 192, hh = t >> 1, j0 = (t & 1) * 2;
