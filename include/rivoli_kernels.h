@@ -192,6 +192,15 @@ int rivoli_dsa_decode_step_paged(const DsaGeom* g, const uint16_t* latent, const
                                  int score_stride, uint32_t* rows, int32_t* n_sel, void* select_scratch,
                                  const uint16_t* q, uint16_t* out, float* out_m, float* out_lse,
                                  void* attend_scratch, int min_rows_hint, void* stream);
+/* The layer-step of a layer that shares another layer's selection, in one call: rivoli_kv_append_paged (row b belongs to
+ * sequence b) followed by rivoli_mla_attend_paged_bf16 over `rows`, same results; q and min_rows_hint as for
+ * rivoli_dsa_decode_step_paged (the hint here is a lower bound of n_rows over the batch). */
+int rivoli_dsa_append_attend_paged(const DsaGeom* g, const uint16_t* latent, const uint16_t* index_key,
+                                   const int32_t* row_pos, const int32_t* block_table, uint8_t* latent_pool,
+                                   float* latent_scale, uint8_t* index_pool, float* index_scale, int32_t* status, int B,
+                                   const uint32_t* rows, int row_stride, const int32_t* n_rows, const uint16_t* q,
+                                   uint16_t* out, float* out_m, float* out_lse, void* attend_scratch, int min_rows_hint,
+                                   void* stream);
 /* ---- the same step for a caller whose activations live in HOST memory ---------------------------------------
  * No counterpart in the reference, whose engine keeps activations on the device; the stream / event wrappers it
  * would build this from are crates/backend/src/gpustream.rs:16-32. A pipe owns `depth` device-side slots, three

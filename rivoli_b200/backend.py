@@ -69,7 +69,7 @@ _SIGNATURES = {
     "kv_append_paged": "pppppi" + "p" * 7, "index_q_quant": "piippp", "index_score_paged": "p" * 8 + "ipip",
     "index_topk_batched": "pipiippp", "index_select_scratch_bytes": "pii", "index_select_uses_mma": "pi",
     "index_select_paged": "p" * 7 + "iipppp", "dsa_append_select_paged": "p" * 13 + "iipppp",
-    "dsa_decode_step_paged": "p" * 13 + "ii" + "p" * 8 + "ip",
+    "dsa_decode_step_paged": "p" * 13 + "ii" + "p" * 8 + "ip", "dsa_append_attend_paged": "p" * 10 + "ipi" + "p" * 6 + "ip",
     "step_pipe_create": "pii", "step_pipe_destroy": "p", "step_pipe_input_bytes": "pi", "step_pipe_output_bytes": "pi",
     "step_pipe_input_offsets": "pip", "dsa_step_host": "pppppp", "step_pipe_wait": "pq", "step_pipe_drain": "p",
     "step_pipe_leg_ms": "pp", "step_pipe_stream": "pi",
@@ -236,6 +236,17 @@ def launch_index_select_paged(g: DsaGeom, index_q, w, index_pool, index_scale, b
                                                   _ptr(index_scale), _ptr(block_table), _ptr(seq_len),
                                                   B, score_stride, _ptr(rows), _ptr(n_sel),
                                                   _ptr(scratch), _stream(stream)), "index_select_paged")
+
+
+def launch_dsa_append_attend_paged(g: DsaGeom, latent, index_key, row_pos, block_table, latent_pool, latent_scale,
+                                   index_pool, index_scale, status, B: int, rows, row_stride: int, n_rows, q, out, out_m,
+                                   out_lse, attend_scratch, min_rows_hint: int = 0, stream=None) -> None:
+    """Append, then attend over rows another layer selected (``rivoli_dsa_append_attend_paged``)."""
+    ensure_status(lib().rivoli_dsa_append_attend_paged(
+        C.byref(g), _ptr(latent), _ptr(index_key), _ptr(row_pos), _ptr(block_table), _ptr(latent_pool),
+        _ptr(latent_scale), _ptr(index_pool), _ptr(index_scale), _ptr(status), B, _ptr(rows), row_stride, _ptr(n_rows),
+        _ptr(q), _ptr(out), _ptr(out_m), _ptr(out_lse), _ptr(attend_scratch), min_rows_hint, _stream(stream)),
+        "dsa_append_attend_paged")
 
 
 def launch_dsa_append_select_paged(g: DsaGeom, latent, index_key, row_pos, block_table, latent_pool, latent_scale,

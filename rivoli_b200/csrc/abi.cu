@@ -106,6 +106,22 @@ RIVOLI_API int rivoli_dsa_decode_step_paged(const DsaGeom* g, const uint16_t* la
     return e;
 }
 
+// The layer-step of a layer that attends over rows selected elsewhere: append, then attention over `rows`, whose q the append
+// kernel (which lets the attention start only when all before it is complete) covers.
+RIVOLI_API int rivoli_dsa_append_attend_paged(const DsaGeom* g, const uint16_t* latent, const uint16_t* index_key,
+                                              const int32_t* row_pos, const int32_t* block_table, uint8_t* latent_pool,
+                                              float* latent_scale, uint8_t* index_pool, float* index_scale,
+                                              int32_t* status, int B, const uint32_t* rows, int row_stride,
+                                              const int32_t* n_rows, const uint16_t* q, uint16_t* out, float* out_m,
+                                              float* out_lse, void* attend_scratch, int min_rows_hint, void* stream) {
+    if (!q || !out || !rows || !n_rows || !g) return 1001;
+    if (int e = rivoli_kv_append_paged(g, latent, index_key, nullptr, row_pos, B, block_table, latent_pool, latent_scale,
+                                       index_pool, index_scale, status, stream))
+        return e;
+    return attend_paged_dispatch(g, q, latent_pool, latent_scale, block_table, rows, row_stride, n_rows, B, out, out_m,
+                                 out_lse, attend_scratch, 1, min_rows_hint, 0x7fffffff, stream);
+}
+
 // out[v] = sum_g w_g * part_out[g][v] / sum_g w_g,  w_g = exp(lse_g - max_g lse), ascending g.
 // One warp per vector; lanes stride the columns.
 __global__ void __launch_bounds__(256)

@@ -196,6 +196,7 @@ attend_mma_kernel(AttendMmaArgs A) {
     // Under a programmatic dependent launch the kernel before this one may still be running. Unless the
     // caller vouches that q was complete before that kernel was even launched (q_early: the fused decode
     // step), q may be that kernel's output and is read only after the dependency wait.
+    rv_grid_dep_trigger();   // the next kernel may be scheduled as CTAs leave; it waits for this grid first
     if (!A.q_early) rv_grid_dep_wait();
     if (warp < AM_SW) {
         uint8_t* zq = smem + SM_ZQ;

@@ -121,6 +121,7 @@ index_q_prepare_kernel(const uint16_t* __restrict__ q, const float* __restrict__
                        float dscale, uint8_t* __restrict__ codes, float* __restrict__ scales, float* __restrict__ cb,
                        int* __restrict__ err) {
     __shared__ float term[32];
+    rv_grid_dep_wait();
     rv_grid_dep_trigger();   // the scorer may set itself up while this runs; it waits before reading these outputs
     index_q_prepare_block(blockIdx.x, q, w, nh, hd, wscale, dscale, codes, scales, cb, err, term);
 }
@@ -138,6 +139,7 @@ step_prologue_kernel(DsaGeom g, AppendArgs ap, int B, const uint16_t* __restrict
                      uint8_t* __restrict__ codes, float* __restrict__ scales, float* __restrict__ cb,
                      int* __restrict__ err) {
     __shared__ float term[32];
+    rv_grid_dep_wait();
     rv_grid_dep_trigger();   // the scorer may set itself up while this runs; it waits before reading these outputs
     if ((int)blockIdx.x < B) {
         index_q_prepare_block(blockIdx.x, q, w, g.index_heads, g.index_dim, g.index_wscale, g.index_dscale, codes, scales,
@@ -157,6 +159,7 @@ __global__ void __launch_bounds__(256)
 step_quant_kernel(DsaGeom g, AppendArgs ap, int B, const uint16_t* __restrict__ q, uint8_t* __restrict__ codes,
                   float* __restrict__ scales) {
     const int lane = threadIdx.x & 31, id = blockIdx.x * 8 + (threadIdx.x >> 5), n_vec = B * g.index_heads;
+    rv_grid_dep_wait();
     rv_grid_dep_trigger();
     if (id < n_vec) {
         const float s = quant_vec(q + (size_t)id * g.index_dim, g.index_dim, codes + (size_t)id * g.index_dim, lane);
@@ -178,8 +181,8 @@ __global__ void __launch_bounds__(SD_THREADS)
 step_dense_kernel(DsaGeom g, AppendArgs ap, int B, const int32_t* __restrict__ block_table, const int32_t* __restrict__ seq_len,
                   int score_stride, uint32_t* __restrict__ rows, int32_t* __restrict__ n_sel, unsigned int* __restrict__ stats,
                   int* __restrict__ err) {
-    rv_grid_dep_trigger();
     rv_grid_dep_wait();
+    rv_grid_dep_trigger();   // (after the wait: the attention behind this reads its q, which is older, at once)
     const int tid = threadIdx.x, blk = (int)blockIdx.x;
     if (blk < B) {
         const int n = min(min(seq_len[blk], score_stride), g.top_k);
@@ -468,9 +471,8 @@ static int select_impl(const DsaGeom* g, const AppendArgs* ap, const uint16_t* i
             if (int e = rivoli_index_q_quant(index_q, B * nh, hd, s.qcodes, s.qscales, stream)) return e;
         const dim3 grid((unsigned)(B + 1 + (ap ? (B + SD_THREADS / 32 - 1) / (SD_THREADS / 32) : 0)));
         const AppendArgs aa = ap ? *ap : AppendArgs{};
-        if (ap) step_dense_kernel<<<grid, SD_THREADS, 0, st>>>(*g, aa, B, block_table, seq_len, score_stride, rows, n_sel, s.stats, s.err);
-        else rv_launch_dependent(step_dense_kernel, grid, dim3(SD_THREADS), 0, st, *g, aa, B, block_table, seq_len, score_stride, rows, n_sel,
-                                 s.stats, s.err);
+        rv_launch_dependent(step_dense_kernel, grid, dim3(SD_THREADS), 0, st, *g, aa, B, block_table, seq_len, score_stride, rows, n_sel,
+                            s.stats, s.err);
         rv_stage_event(1, st);
         rv_stage_event(2, st);
         return rv_launch_status();
@@ -482,7 +484,7 @@ static int select_impl(const DsaGeom* g, const AppendArgs* ap, const uint16_t* i
         if (ap && narrow) {
             if ((hd % 16) != 0 || hd > 512) return 1004;
             rv_drain_error();
-            step_quant_kernel<<<(B * nh + B + 7) / 8, 256, 0, st>>>(*g, *ap, B, index_q, s.qcodes, s.qscales);
+            rv_launch_dependent(step_quant_kernel, dim3((unsigned)((B * nh + B + 7) / 8)), dim3(256), 0, st, *g, *ap, B, index_q, s.qcodes, s.qscales);
             e = rv_launch_status();
         } else {
             if (ap)
@@ -501,11 +503,11 @@ static int select_impl(const DsaGeom* g, const AppendArgs* ap, const uint16_t* i
     rv_drain_error();
     rv_stage_event(0, st);
     if (ap)
-        step_prologue_kernel<<<B + (B + 31) / 32, 1024, 0, st>>>(*g, *ap, B, index_q, w, s.qcodes, s.qscales, s.cb,
-                                                                 s.err);
+        rv_launch_dependent(step_prologue_kernel, dim3((unsigned)(B + (B + 31) / 32)), dim3(1024), 0, st, *g, *ap, B, index_q, w, s.qcodes,
+                            s.qscales, s.cb, s.err);
     else
-        index_q_prepare_kernel<<<B, 32 * nh, 0, st>>>(index_q, w, nh, hd, g->index_wscale, g->index_dscale, s.qcodes,
-                                                       s.qscales, s.cb, s.err);
+        rv_launch_dependent(index_q_prepare_kernel, dim3((unsigned)B), dim3(32 * nh), 0, st, index_q, w, nh, hd, g->index_wscale,
+                            g->index_dscale, s.qcodes, s.qscales, s.cb, s.err);
     if (int e = rv_launch_status()) return e;
 
     IndexMmaArgs ma{*g, s.qcodes, s.qscales, w, index_pool, index_scale, block_table, seq_len,

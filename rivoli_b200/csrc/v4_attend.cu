@@ -212,6 +212,7 @@ __global__ void __launch_bounds__(SA_THREADS, 1) v4_sparse_attend_kernel(SaArgs 
 
     // Under a programmatic dependent launch the kernel before this one may still be running: nothing it may have written is
     // read before the dependency wait.
+    rv_grid_dep_trigger();   // the next kernel may be scheduled as CTAs leave; it waits for this grid first
     if (!A.q_early) rv_grid_dep_wait();
     if (warp < SA_SW) {   // q of this sequence: 64 rows of 64 16-byte pieces, swizzled; the copies signal the barrier
 #pragma unroll

@@ -108,10 +108,9 @@ class DsaDecodeStack:
         if self.full[i]:
             return self._step_full_stale(i, latent, index_key, index_q, index_w, q, row_pos, seq_len, stream)
         src = self.layers[self.owner[i]]
-        L.append_latent_only(latent, row_pos, stream=stream)
         if self.stale is not None:          # a shared layer serves what its full layer serves at this token
-            return L.attend(q, stream=stream, rows_from=_Served(src))
-        return L.attend(q, stream=stream, rows_from=src)
+            return L.step_shared(latent, q, row_pos, _Served(src), stream=stream)
+        return L.step_shared(latent, q, row_pos, src, stream=stream, min_rows_hint=min_rows_hint)
 
     def _step_full_stale(self, i, latent, index_key, index_q, index_w, q, row_pos, seq_len, stream, seq_len_host=None):
         """Full layer under the stale selection: select into the layer's row buffer as usual, but attend over the

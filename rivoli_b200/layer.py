@@ -100,13 +100,24 @@ class DsaDecodeLayer:
         be.launch_index_topk_batched(self.scores, self.score_stride, seq_len, self.B, g.top_k, self.rows,
                                      self.n_sel, stream)
 
+    def _no_key(self, n: int) -> torch.Tensor:
+        if getattr(self, "_zero_key", None) is None or self._zero_key.shape[0] != n:
+            self._zero_key = torch.zeros((n, self.g.index_dim), dtype=torch.bfloat16, device=self.dev)
+        return self._zero_key
+
     def append_latent_only(self, latent: torch.Tensor, row_pos: torch.Tensor, stream=None) -> None:
         """Cache the step's latent rows of a layer that owns no indexer: the index key that travels with the
         operator is a constant zero row written to this layer's (unused) index pool."""
-        n = latent.shape[0]
-        if getattr(self, "_zero_key", None) is None or self._zero_key.shape[0] != n:
-            self._zero_key = torch.zeros((n, self.g.index_dim), dtype=torch.bfloat16, device=self.dev)
-        self.append(latent, self._zero_key, row_pos, None, stream)
+        self.append(latent, self._no_key(latent.shape[0]), row_pos, None, stream)
+
+    def step_shared(self, latent: torch.Tensor, q: torch.Tensor, row_pos: torch.Tensor, rows_from, stream=None,
+                    min_rows_hint: int = 0) -> torch.Tensor:
+        """``append_latent_only`` and ``attend(q, rows_from=...)`` in one library call, one row per sequence."""
+        be.launch_dsa_append_attend_paged(self.g, latent, self._no_key(self.B), row_pos, self.block_table,
+                                          self.latent_pool, self.latent_scale, self.index_pool, self.index_scale,
+                                          self.status, self.B, rows_from.rows, self.g.top_k, rows_from.n_sel, q, self.out,
+                                          self.out_m, self.out_lse, self.scratch, min_rows_hint, stream)
+        return self.out
 
     def attend(self, q: torch.Tensor, stream=None, dense_len: torch.Tensor | None = None,
                out: torch.Tensor | None = None, rows_from: "DsaDecodeLayer | None" = None) -> torch.Tensor:

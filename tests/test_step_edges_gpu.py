@@ -155,3 +155,26 @@ def test_selection_bands_of_every_cluster(cluster, kind):
     for b, m in enumerate((n, 5000)):
         order = np.lexsort((np.arange(m), -s[b, :m].astype(np.float64)))[:k]
         np.testing.assert_array_equal(got[b].cpu().numpy(), np.sort(order))
+
+
+@pytest.mark.parametrize("lens,hint", [([300, 128, 700], 128), ([300, 5, 127], 0), ([64, 100], 0)])
+def test_shared_layer_step_equals_its_operators(lens, hint):
+    """Append and attention over another layer's rows in one call, bit for bit the two calls: hint taken, short sequences
+    among long ones, only short ones."""
+    st = State(74, len(lens), lens, top_k=256)
+    outs = []
+    for joint in (True, False):
+        be, g, src = _layer(st)
+        src.step(dev(st.new_latent), dev(st.new_key), dev(st.index_q), dev(st.index_w), dev(st.q), dev(st.row_pos), dev(st.seq_len))
+        _, _, L = _layer(st)
+        x = dev(st.new_latent).flip(0).contiguous(), dev(st.q).flip(0).contiguous(), dev(st.row_pos)
+        for _ in range(3):          # back to back: each call starts under the one before it
+            if joint:
+                out = L.step_shared(*x, src, min_rows_hint=hint)
+            else:
+                L.append_latent_only(x[0], x[2])
+                out = L.attend(x[1], rows_from=src)
+        be.device_sync(); L.check_status()
+        outs.append([t.cpu().contiguous().view(torch.uint8) for t in (out, L.out_lse, L.latent_pool, L.latent_scale, L.index_pool)])
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
