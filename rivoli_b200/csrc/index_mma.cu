@@ -43,7 +43,7 @@ constexpr int IM_HD = 128;         // index dim = one 128-byte swizzle row
 constexpr int IM_NPAD = 32;        // heads padded to N = 32
 constexpr int IM_NS = 6;           // key-tile stages in flight
 constexpr int IM_NACC = 4;         // TMEM accumulators (32 columns each)
-constexpr int IM_TPI = 16;         // most tiles per work item (a launch picks fewer when the batch is small: IndexMmaArgs::tpi)
+constexpr int IM_TPI = 16;         // most tiles per work item
 constexpr int IM_THREADS = 192;    // warps 0-3 epilogue, 4 producer, 5 MMA
 constexpr int IM_STAGE_BYTES = IM_TILE * IM_HD;   // 16 KiB
 constexpr int IM_Q_BYTES = IM_NPAD * IM_HD;       // 4 KiB
@@ -56,7 +56,6 @@ struct IndexMmaArgs {
     const uint8_t* index_pool; const float* index_scale; const int32_t* block_table; const int32_t* seq_len;
     float* scores; int score_stride; int B;
     int* err;              // device error word (0 = ok)
-    int tpi;               // tiles per work item, 1 .. IM_TPI: small enough that every persistent CTA gets work
 };
 
 // ---------------------------------------------------------------------------------------------
@@ -218,10 +217,54 @@ struct ImBarriers {
     uint64_t full[IM_NS], empty[IM_NS], tfull[IM_NACC], tempty[IM_NACC], qfree[2];
 };
 
-// Tokens of sequence b that need a score: none if the selection takes them all anyway.
+// Tiles of sequence b that need a score: none if the selection takes all its tokens anyway.
 __device__ __forceinline__ int scored_tokens(const IndexMmaArgs& A, int b) {
     const int nt = min(A.seq_len[b], A.score_stride);
     return nt <= A.g.top_k ? 0 : nt;
+}
+__device__ __forceinline__ int scored_tiles(const IndexMmaArgs& A, int b) { return (scored_tokens(A, b) + IM_TILE - 1) / IM_TILE; }
+
+// A CTA's share: the tiles of all sequences in one row, split evenly over the grid (a ragged batch in equal items of 16 tiles
+// left some CTAs twice the work of others: 32 sequences of 512 to 32,768 tokens 28 us, 19 now). It is walked in items
+// of at most IM_TPI tiles of one sequence; every role of the CTA walks the same items.
+struct ImShare {
+    int b, t, left;        // next tile: tile t of sequence b; tiles left
+    int nt, t1;            // of the current item: the sequence's tokens, its end
+    __device__ __forceinline__ bool next(const IndexMmaArgs& A) {   // advances to the item [t, t1) of sequence b
+        if (left <= 0) return false;
+        for (;; ++b, t = 0) {
+            if (b >= A.B) return false;
+            nt = scored_tokens(A, b);
+            if (t < (nt + IM_TILE - 1) / IM_TILE) break;
+        }
+        t1 = min(min(t + IM_TPI, (nt + IM_TILE - 1) / IM_TILE), t + left);
+        left -= t1 - t;
+        return true;
+    }
+};
+// The share of this CTA, by one warp (two passes over the lengths: all tiles, then where the share begins).
+__device__ __forceinline__ ImShare im_share(const IndexMmaArgs& A) {
+    const int lane = threadIdx.x & 31;
+    int total = 0;
+    for (int b0 = 0; b0 < A.B; b0 += 32) total += __reduce_add_sync(0xffffffffu, b0 + lane < A.B ? scored_tiles(A, b0 + lane) : 0);
+    const int lo = (int)((long long)total * blockIdx.x / gridDim.x), hi = (int)((long long)total * (blockIdx.x + 1) / gridDim.x);
+    ImShare r{0, 0, hi - lo, 0, 0};
+    int before = 0;
+    for (int b0 = 0; b0 < A.B && hi > lo; b0 += 32) {
+        const int n = b0 + lane < A.B ? scored_tiles(A, b0 + lane) : 0;
+        int incl = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += v; }
+        const unsigned hit = __ballot_sync(0xffffffffu, before + incl > lo);
+        if (hit) {
+            const int l = __ffs(hit) - 1;
+            r.b = b0 + l;
+            r.t = lo - (before + __shfl_sync(0xffffffffu, incl - n, l));
+            break;
+        }
+        before += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    return r;
 }
 
 __global__ void __launch_bounds__(IM_THREADS)
@@ -236,6 +279,7 @@ index_score_mma_kernel(IndexMmaArgs A, const __grid_constant__ CUtensorMap tm_ke
     __shared__ volatile int abort_flag;
     __shared__ float s_wh[IM_NPAD];
     __shared__ int s_pg[IM_TPI * (IM_TILE / 16)];
+    __shared__ ImShare s_share;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const DsaGeom& g = A.g;
@@ -251,6 +295,8 @@ index_score_mma_kernel(IndexMmaArgs A, const __grid_constant__ CUtensorMap tm_ke
     // q tiles start zeroed: rows >= nh are never loaded and must contribute exact zeros
     for (int i = tid; i < 2 * IM_Q_BYTES / 16; i += IM_THREADS) reinterpret_cast<uint4*>(s_q)[i] = make_uint4(0, 0, 0, 0);
     if (warp == 5) tc::tmem_alloc<IM_NACC * 32>(&tmem_base_s);
+    // (the lengths are an input of the call whose first kernel is the one before this: complete before that kernel's trigger)
+    if (warp == 4) { const ImShare sh = im_share(A); if (lane == 0) s_share = sh; }
     tc::fence_proxy_async();
     tc::tc_fence_before();
     __syncthreads();
@@ -259,11 +305,7 @@ index_score_mma_kernel(IndexMmaArgs A, const __grid_constant__ CUtensorMap tm_ke
     rv_grid_dep_wait();      // query codes, head scales and this step's appended keys come from the kernel before
     rv_grid_dep_trigger();   // the selection kernel may start (after the wait: it reads all but the scores at once)
 
-    const int tpi = A.tpi;
-    const int max_tiles = (A.score_stride + IM_TILE - 1) / IM_TILE;
-    const int chunks = (max_tiles + tpi - 1) / tpi;
-    const int n_items = A.B * chunks;
-
+    ImShare sh = s_share;
     if (warp == 4) {
         // ------------------------------ producer: TMA page loads ----------------------------------
         // A page is P rows x 128 bytes, contiguous in the pool; one 2-D TMA box per page lands it in
@@ -272,14 +314,11 @@ index_score_mma_kernel(IndexMmaArgs A, const __grid_constant__ CUtensorMap tm_ke
         int it = 0, items_done = 0;
         bool ok = true;
         const int ppt = IM_TILE / P;  // pages per tile (16 <= P <= 128)
-        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-            const int b = item / chunks, c = item - b * chunks;
-            const int nt = scored_tokens(A, b);
-            const int tile_end = min((c + 1) * tpi, (nt + IM_TILE - 1) / IM_TILE);
-            if (c * tpi >= tile_end) continue;
-            const int first_lp = c * tpi * ppt;
+        for (; ok && sh.next(A); sh.t = sh.t1) {
+            const int b = sh.b, nt = sh.nt;
+            const int first_lp = sh.t * ppt;
             __syncwarp();
-            for (int j = lane; j < tpi * ppt; j += 32) {
+            for (int j = lane; j < (sh.t1 - sh.t) * ppt; j += 32) {
                 const int lp = first_lp + j;
                 int pg = -1;
                 const bool live = lp < g.max_pages_per_seq && lp * P < nt;
@@ -292,17 +331,17 @@ index_score_mma_kernel(IndexMmaArgs A, const __grid_constant__ CUtensorMap tm_ke
             }
             __syncwarp();
             const int qb = items_done & 1;
-            for (int tile = c * tpi; tile < tile_end && ok; ++tile) {
+            for (int tile = sh.t; tile < sh.t1 && ok; ++tile) {
                 const int s = it % IM_NS;
                 ok = tc::mbar_wait_warp(&bars.empty[s], ((it / IM_NS) & 1) ^ 1, &abort_flag, 11);
                 if (!ok) break;
-                const bool first = tile == c * tpi;
+                const bool first = tile == sh.t;
                 if (first) {
                     ok = tc::mbar_wait_warp(&bars.qfree[qb], ((items_done >> 1) & 1) ^ 1, &abort_flag, 12);
                     if (!ok) break;
                 }
                 if (lane == 0) {
-                    const int pbase = (tile - c * tpi) * ppt;
+                    const int pbase = (tile - sh.t) * ppt;
                     uint32_t bytes = first ? (uint32_t)nh * IM_HD : 0u;
                     for (int p2 = 0; p2 < ppt; ++p2) bytes += s_pg[pbase + p2] >= 0 ? (uint32_t)P * IM_HD : 0u;
                     tc::mbar_arrive_expect_tx(&bars.full[s], bytes);
@@ -325,12 +364,9 @@ index_score_mma_kernel(IndexMmaArgs A, const __grid_constant__ CUtensorMap tm_ke
         int it = 0, items_done = 0;
         bool ok = true;
         const uint32_t idesc = tc::idesc_e4m3(IM_TILE, IM_NPAD, 0, 0);
-        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-            const int b = item / chunks, c = item - b * chunks;
-            const int nt = scored_tokens(A, b);
-            const int tile_end = min((c + 1) * tpi, (nt + IM_TILE - 1) / IM_TILE);
+        for (; ok && sh.next(A); sh.t = sh.t1) {
             const int qb = items_done & 1;
-            for (int tile = c * tpi; tile < tile_end && ok; ++tile) {
+            for (int tile = sh.t; tile < sh.t1 && ok; ++tile) {
                 const int s = it % IM_NS, a = it % IM_NACC;
                 ok = tc::mbar_wait_warp(&bars.full[s], (it / IM_NS) & 1, &abort_flag, 21) &&
                      tc::mbar_wait_warp(&bars.tempty[a], ((it / IM_NACC) & 1) ^ 1, &abort_flag, 22);
@@ -344,22 +380,19 @@ index_score_mma_kernel(IndexMmaArgs A, const __grid_constant__ CUtensorMap tm_ke
                                    tc::smem_desc_sw128(qa + k * 32, 16, 1024), idesc, k > 0);
                     tc::mma_commit(&bars.empty[s]);
                     tc::mma_commit(&bars.tfull[a]);
-                    if (tile == tile_end - 1) tc::mma_commit(&bars.qfree[qb]);
+                    if (tile == sh.t1 - 1) tc::mma_commit(&bars.qfree[qb]);
                 }
                 __syncwarp();
                 ++it;
             }
-            if (c * tpi < tile_end) ++items_done;      // items without tiles never touched a q buffer
+            ++items_done;
         }
     } else {
         // ------------------------------ epilogue: TMEM -> scores --------------------------------
         int it = 0;
         bool ok = true;
-        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-            const int b = item / chunks, c = item - b * chunks;
-            const int nt = scored_tokens(A, b);
-            const int tile_end = min((c + 1) * tpi, (nt + IM_TILE - 1) / IM_TILE);
-            if (c * tpi >= tile_end) continue;
+        for (; ok && sh.next(A); sh.t = sh.t1) {
+            const int b = sh.b, nt = sh.nt;
             tc::named_barrier(1, 128);  // previous item's constants are no longer read
             if (tid < IM_NPAD) {
                 // a_t / s_k = sum_h (w_h ws s_q[h] ds) * max(cd_h, 0): the exact formula up to a few
@@ -368,7 +401,7 @@ index_score_mma_kernel(IndexMmaArgs A, const __grid_constant__ CUtensorMap tm_ke
                                            g.index_dscale : 0.0f;
             }
             tc::named_barrier(1, 128);
-            for (int tile = c * tpi; tile < tile_end && ok; ++tile) {
+            for (int tile = sh.t; tile < sh.t1 && ok; ++tile) {
                 const int a = it % IM_NACC;
                 const int t = tile * IM_TILE + tid;
                 ok = tc::mbar_wait_warp(&bars.tfull[a], (it / IM_NACC) & 1, &abort_flag, 31);
@@ -511,24 +544,15 @@ static int select_impl(const DsaGeom* g, const AppendArgs* ap, const uint16_t* i
     if (int e = rv_launch_status()) return e;
 
     IndexMmaArgs ma{*g, s.qcodes, s.qscales, w, index_pool, index_scale, block_table, seq_len,
-                    s.scores, score_stride, B, s.err, IM_TPI};
+                    s.scores, score_stride, B, s.err};
     const size_t smem1 = (size_t)IM_NS * IM_STAGE_BYTES + 2 * IM_Q_BYTES + 1024;
     cudaFuncSetAttribute(index_score_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int max_tiles = (score_stride + IM_TILE - 1) / IM_TILE;
-    // work items of 16 tiles; when that leaves SMs without any item (a small batch), smaller items: about four per SM
-    // (measured: 17.9 -> 15.2 us at batch 16 x 16,384 tokens, while batches that already fill the chip lose 10 % to the
-    // per-item set-up with smaller items)
-    if ((long long)B * ((max_tiles + IM_TPI - 1) / IM_TPI) >= 6LL * sms) {
-        ma.tpi = IM_TPI / 2;   // plenty of items: halves of them even out the last round (measured: 160.6 -> 158.6 us per step at batch 128 x 16,384)
-    } else if ((long long)B * ((max_tiles + IM_TPI - 1) / IM_TPI) < sms) {
-        long long tpi = (long long)B * max_tiles / (4LL * sms);
-        ma.tpi = (int)(tpi < 2 ? 2 : (tpi > IM_TPI ? IM_TPI : tpi));
-    }
-    const int n_items = B * ((max_tiles + ma.tpi - 1) / ma.tpi);
-    const int grid = n_items < 2 * sms ? n_items : 2 * sms;
+    // two persistent CTAs per SM; a batch with fewer tiles at most gets as many CTAs
+    const long long most = (long long)B * ((score_stride + IM_TILE - 1) / IM_TILE);
+    const int grid = most < 2 * sms ? (int)most : 2 * sms;
     CUtensorMap tm_keys, tm_q;
     if (int e = rivoli::make_tmap_rows_sw128(&tm_keys, index_pool, (uint64_t)g->n_pool_pages * g->page_tokens, IM_HD,
                                              (uint32_t)g->page_tokens))

@@ -178,3 +178,19 @@ def test_shared_layer_step_equals_its_operators(lens, hint):
         outs.append([t.cpu().contiguous().view(torch.uint8) for t in (out, L.out_lse, L.latent_pool, L.latent_scale, L.index_pool)])
     for a, b in zip(*outs):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("lens", [[257, 3, 300, 256, 128, 9000, 1], [257], [400] * 40, [385, 129] * 20])
+def test_scorer_shares_of_ragged_batches(lens):
+    """Shares of the tiles that begin and end anywhere: sequences without a score between others, more CTAs than tiles, one
+    tile, shares over several sequences; rows against the unfused operators."""
+    st = State(75, len(lens), lens, top_k=256)
+    be, g, L = _layer(st)
+    x = (dev(st.index_q), dev(st.index_w), dev(st.seq_len))
+    L.select(*x)
+    be.device_sync(); L.check_status()
+    got, n = L.rows.clone(), L.n_sel.clone()
+    L.select_unfused(*x)
+    assert torch.equal(n, L.n_sel)
+    for b, k in enumerate(n.tolist()):
+        assert torch.equal(got[b, :k], L.rows[b, :k]), b
