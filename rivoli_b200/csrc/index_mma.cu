@@ -68,50 +68,42 @@ index_q_prepare_block(int b, const uint16_t* __restrict__ q, const float* __rest
     const int h = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (h < nh) {
         const size_t v = (size_t)b * nh + h;
-        // same codec path as rivoli_index_q_quant: 16 values per lane, absmax scale, e4m3 codes
-        float f[16];
-        const bool act = lane * 16 < hd;
-        if (act) {
-            const uint4* p = reinterpret_cast<const uint4*>(q + v * hd + lane * 16);
-            const uint4 p0 = p[0], p1 = p[1];
-            const uint32_t ww[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+        // same codec path as rivoli_index_q_quant (index_dim is 128 here): eight values per lane, sixteen lanes
+        const bool act = lane < IM_HD / 8;
+        const uint4 x = act ? *reinterpret_cast<const uint4*>(q + v * IM_HD + lane * 8) : make_uint4(0u, 0u, 0u, 0u);
+        const float wv = w[v];
+        uint32_t m = rv_absmax8(x);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) { f[2 * i] = __uint_as_float(ww[i] << 16); f[2 * i + 1] = __uint_as_float(ww[i] & 0xffff0000u); }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) f[i] = 0.0f;
-        }
-        float amax = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(f[i]));
-        amax = rv_warp_max(amax);
-        const float scl = rv_scale_from_amax(amax);
+        for (int o = IM_HD / 16; o > 0; o >>= 1) m = rv_max_bf16x2(m, __shfl_xor_sync(0xffffffffu, m, o));
+        const QuantScale qs = rv_quant_scale(__uint_as_float(m << 16));
         float n2 = 0.0f;
         if (act) {
-            uint32_t o[4];
+            uint32_t redo = qs.r == 0.0f ? RV_REDO : 0u;
+            uint2 c = rv_codes8(x, qs, redo);
+            if (redo & RV_REDO) c = rv_codes8_exact(x, qs.s);
+            *reinterpret_cast<uint2*>(codes + v * IM_HD + lane * 8) = c;
+            const uint32_t cc[2] = {c.x, c.y};
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const uint16_t lo = rv_f32x2_to_e4m3x2(__fdiv_rn(f[4 * i], scl), __fdiv_rn(f[4 * i + 1], scl));
-                const uint16_t hi = rv_f32x2_to_e4m3x2(__fdiv_rn(f[4 * i + 2], scl), __fdiv_rn(f[4 * i + 3], scl));
-                o[i] = (uint32_t)lo | ((uint32_t)hi << 16);
-                const float2 a = rv_e4m3x2_to_f32x2(lo), c = rv_e4m3x2_to_f32x2(hi);
-                n2 += a.x * a.x + a.y * a.y + c.x * c.x + c.y * c.y;
+            for (int i = 0; i < 2; ++i) {
+                const float2 lo = rv_e4m3x2_to_f32x2((uint16_t)(cc[i] & 0xffff)), hi = rv_e4m3x2_to_f32x2((uint16_t)(cc[i] >> 16));
+                n2 += lo.x * lo.x + lo.y * lo.y + hi.x * hi.x + hi.y * hi.y;
             }
-            *reinterpret_cast<uint4*>(codes + v * hd + lane * 16) = make_uint4(o[0], o[1], o[2], o[3]);
         }
-        n2 = rv_warp_sum(n2);
+#pragma unroll
+        for (int o = IM_HD / 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
         if (lane == 0) {
-            scales[v] = scl;
-            term[h] = fabsf(w[v] * wscale) * dscale * scl * sqrtf(n2);
+            scales[v] = qs.s;
+            term[h] = fabsf(wv * wscale) * dscale * qs.s * sqrtf(n2);
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        float s = 0.0f;
-        for (int i = 0; i < nh; ++i) s += term[i];
+    if (threadIdx.x < 32) {
+        const float sum = rv_warp_sum(lane < nh ? term[lane] : 0.0f);
         // ||kcode||_2 <= sqrt(hd) * 448; 1.01 covers the roundings of this very sum
-        cb[b] = s * sqrtf((float)hd) * 448.0f * IM_EPS_REL * 1.01f;
-        if (b == 0) *err = 0;   // the scorer's error word starts clean on every call
+        if (lane == 0) {
+            cb[b] = sum * sqrtf((float)hd) * 448.0f * IM_EPS_REL * 1.01f;
+            if (b == 0) *err = 0;   // the scorer's error word starts clean on every call
+        }
     }
 }
 
