@@ -35,7 +35,7 @@
 // head: thread = (head, 16 tokens of the tile), two warps per lane quarter take the two 32-token halves. A head's
 // reference maximum, its running sum and its q scale are registers, and P' leaves as one 16-byte store per term
 // (heads are the rows of the K-major P' operand, tokens its bytes).
-// q arrives as bf16 (one bulk copy) and is split into its two e4m3 terms by the softmax warps inside the kernel while the
+// q arrives as bf16 (bulk copies) and is split into its two e4m3 terms by the softmax warps inside the kernel while the
 // first tiles are gathered; the output leaves through the idle ring as 8 KiB bulk copies.
 // Online softmax with a LAGGING reference max: as long as no score of a tile exceeds its head's
 // reference by more than 3 (log2) the references stand (one barrier-with-OR per tile, no exchange);
@@ -102,7 +102,7 @@ static_assert((AM_H + AM_MAX_SPLITS) * AM_KVL * 4 <= AM_STAGES * SM_KSTAGE, "the
 
 struct AmBars {
     uint64_t k_full[AM_STAGES], k_empty[AM_STAGES], s_full[AM_SBUF], s_empty[AM_SBUF], rope_free[AM_ROPES],
-        p_full, pv_done, q_full, q_raw;
+        p_full, pv_done, q_full, q_raw[AM_SW];
 };
 static_assert(sizeof(AmBars) <= 256, "barrier block");
 static_assert(SM_TOTAL <= 232448, "shared memory budget");
@@ -167,7 +167,8 @@ attend_mma_kernel(AttendMmaArgs A) {
         tc::mbar_init(&bars.p_full, AM_SOFTMAX_THREADS);
         tc::mbar_init(&bars.pv_done, 1);
         tc::mbar_init(&bars.q_full, AM_SOFTMAX_THREADS);
-        tc::mbar_init(&bars.q_raw, 1);
+#pragma unroll
+        for (int s = 0; s < AM_SW; ++s) tc::mbar_init(&bars.q_raw[s], 1);
         tc::mbar_init_fence();
         *abort_flag = 0;
     }
@@ -184,7 +185,7 @@ attend_mma_kernel(AttendMmaArgs A) {
     //   hi = e4m3(q / s), s = absmax / 448;  lo = e4m3(q / s - hi)   =>  q ~ s * (hi + lo)
     // (the residual of a value of typical size is a normal e4m3 number; below 2^-6 it is kept to 2^-10 absolute,
     // 2^-19 of the head's largest value).
-    // The sequence's 72 KiB of q arrive as ONE bulk copy in ring stages 3 to 5, which the gather leaves alone until q_full.
+    // The sequence's 72 KiB of q arrive as one bulk copy per softmax warp in ring stages 3 to 5, which the gather leaves alone until q_full.
     // A warp converts eight heads, lanes along a head's row, and writes a head's hi row and lo row over the bf16 row it
     // read (576 + 576 bytes = 1,152); 16-byte pieces are XOR-swizzled by head. Then a thread moves the row of its OWN
     // tensor-memory lane (lane l of warp w is the virtual head (16 (w % 4) + l % 16, term l / 16), w / 4 the half of the 512
@@ -200,12 +201,14 @@ attend_mma_kernel(AttendMmaArgs A) {
     if (!A.q_early) rv_grid_dep_wait();
     if (warp < AM_SW) {
         uint8_t* zq = smem + SM_ZQ;
-        if (tid == 0) {
-            tc::mbar_arrive_expect_tx(&bars.q_raw, AM_H * AM_W * 2);
+        constexpr uint32_t part = AM_H / AM_SW * AM_W * 2;   // a warp's eight heads: it starts when they are there
+        if (lane == 0) {
+            tc::mbar_arrive_expect_tx(&bars.q_raw[warp], part);
             asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                         ::"r"(tc::smem_u32(zq)), "l"(A.q + (size_t)b * AM_H * AM_W), "r"(AM_H * AM_W * 2), "r"(tc::smem_u32(&bars.q_raw)) : "memory");
+                         ::"r"(tc::smem_u32(zq + warp * part)), "l"(A.q + ((size_t)b * AM_H + warp * (AM_H / AM_SW)) * AM_W), "r"(part), "r"(tc::smem_u32(&bars.q_raw[warp])) : "memory");
         }
-        tc::mbar_wait_warp(&bars.q_raw, 0, abort_flag, 55, A.max_polls);
+        __syncwarp();
+        tc::mbar_wait_warp(&bars.q_raw[warp], 0, abort_flag, 55, A.max_polls);
         // 8 values -> their 8 hi codes and 8 lo codes
         auto codes8 = [&](const uint4 v, float inv, uint2& hi, uint2& lo) {
             const uint32_t ww[4] = {v.x, v.y, v.z, v.w};
