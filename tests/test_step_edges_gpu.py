@@ -194,3 +194,23 @@ def test_scorer_shares_of_ragged_batches(lens):
     assert torch.equal(n, L.n_sel)
     for b, k in enumerate(n.tolist()):
         assert torch.equal(got[b, :k], L.rows[b, :k]), b
+
+
+@pytest.mark.parametrize("lens", [[1, 64, 65, 128, 129, 192, 193], [255, 256, 257, 320, 321], [383, 385, 449, 640] * 19])
+def test_attention_tiles_of_the_gather(lens):
+    """Row counts around the tiles that the gather warps share and those they fill alone, in clusters and (76 sequences) with
+    one CTA per sequence, against the CUDA-core kernel."""
+    st = State(76, len(lens), lens)
+    be, g, L = _layer(st)
+    want = torch.empty_like(L.out)
+    n = dev(st.seq_len)
+    args = (dev(st.q), L.latent_pool, L.latent_scale, L.block_table, None, 0, n, st.B)
+    be.attend_mma_test_hook(min_rows=0)
+    try:
+        be.launch_attend_paged_bf16(g, *args, L.out, L.out_m, L.out_lse, L.scratch)
+        be.attend_paged_status(g, L.scratch)
+    finally:
+        be.attend_mma_test_hook()
+    be.launch_attend_simt_paged_bf16(g, *args, want, None, None, None)
+    a, b = L.out.float(), want.float()
+    assert bool(((a - b).abs() <= 2e-2 * b.abs().amax(dim=(1, 2), keepdim=True) + 1e-3).all()), (a - b).abs().max().item()
