@@ -176,7 +176,13 @@ front_gemm_mma_kernel(FrontArgs A) {
     const int k0 = split * J.k_chunks * 64, nch = min(J.k_chunks, K / 64 - split * J.k_chunks);
     if (tid == 0) { tc::mbar_init(&bar[0], 1); tc::mbar_init(&bar[1], 1); tc::mbar_init_fence(); abort_word = 0; }
     if (warp == 0) tc::tmem_alloc<256>(&tmem_slot);
-    // the wait comes first: the epilogue kernel, started by the trigger, may then read inputs of this call before its own wait
+    // (a prefetch into L2 may precede the wait, whoever writes)
+    for (int e = tid; e < TN * ((nch * 64 + 127) / 128); e += FM_THREADS) {
+        const int row = e % TN, line = e / TN;
+        const uint8_t* w = row < n0 ? J.m[0].w + (size_t)(tile * TN + row) * K : J.m[1].w + (size_t)(row - n0) * K;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(w + k0 + line * 128));
+    }
+    // the wait comes before the trigger: the epilogue kernel may then read inputs of this call before its own wait
     rv_grid_dep_wait();
     rv_grid_dep_trigger();
     // this thread's weight pieces: row e / 4, codes 16 (e % 4) .. + 15 of each chunk

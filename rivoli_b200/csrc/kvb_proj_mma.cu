@@ -87,6 +87,15 @@ __device__ __forceinline__ void kp_request_acts(const KpArgs& A, int h, int b0, 
                              A.x + ((size_t)(live ? b0 + row : 0) * A.H + h) * A.xs + c * 64 + j * 8, live ? 16u : 0u);
     }
 }
+// Asks L2 for `n` runs of `bytes` bytes, `pitch` apart (whole CTA, lines of 128 bytes). Under a programmatic dependent launch a
+// CTA may sit here while the kernel before it finishes; a prefetch into L2 may precede the dependency wait, whoever writes.
+__device__ __forceinline__ void kp_prefetch(const void* base, size_t pitch, int n, int bytes) {
+    const int lines = (bytes + 127) / 128;
+    for (int e = threadIdx.x; e < n * lines; e += KP_THREADS) {
+        const int r = e / lines;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint8_t*>(base) + (size_t)r * pitch + (e - r * lines) * 128));
+    }
+}
 // Sixteen e4m3 codes of a raw piece -> two 16-byte bf16 chunks.
 __device__ __forceinline__ void kp_convert16(const uint8_t* raw, uint8_t* d0, uint8_t* d1) {
     const uint4 v = *reinterpret_cast<const uint4*>(raw);
@@ -140,8 +149,10 @@ kvb_absorb_mma_kernel(KpArgs A) {
     const int cut = min(nope, (int)(128 - (rbase & 127)));
     const bool two_runs = cut < nope;
     if (tid == 0) { tc::mbar_init(&bar[0], 1); tc::mbar_init(&bar[1], 1); tc::mbar_init_fence(); abort_word = 0; }
-    if (warp == 0) tc::tmem_alloc<256>(&tmem_slot);
     rv_grid_dep_trigger();
+    kp_prefetch(A.kvb + rbase * kvl + iblk * 128, (size_t)kvl, nope, 128);
+    kp_prefetch(A.x + (size_t)h * A.xs, (size_t)A.H * A.xs * 2, min(128, A.B), nope * 2);
+    if (warp == 0) tc::tmem_alloc<256>(&tmem_slot);
     rv_grid_dep_wait();
     for (int c = 0; c < nch; ++c) {
         kp_request_acts(A, h, 0, c, sA + c * KP_ACHUNK);
@@ -267,8 +278,10 @@ kvb_value_mma_kernel(KpArgs A) {
     const size_t row0 = (size_t)h * (A.nope + vh) + A.nope + (size_t)jblk * 128;   // 128 value rows = 2 scale rows
     const int sc_cols = kvl / 128;
     if (tid == 0) { tc::mbar_init(&bar[0], 1); tc::mbar_init(&bar[1], 1); tc::mbar_init_fence(); abort_word = 0; }
-    if (warp == 0) tc::tmem_alloc<512>(&tmem_slot);
     rv_grid_dep_trigger();
+    kp_prefetch(A.kvb + row0 * kvl, (size_t)kvl, 128, kvl);
+    kp_prefetch(A.x + (size_t)h * A.xs, (size_t)A.H * A.xs * 2, min(128, A.B), kvl * 2);
+    if (warp == 0) tc::tmem_alloc<512>(&tmem_slot);
     rv_grid_dep_wait();
     for (int c = 0; c < nch; ++c) {
         kp_request_acts(A, h, 0, c, sA + c * KP_ACHUNK);
