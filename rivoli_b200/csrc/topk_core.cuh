@@ -26,16 +26,17 @@ struct TkShared {
     uint32_t pivot, need;
 };
 
-// Four 8-bit passes, MSB first: the key of the kk-th largest entry and how many of the
+// 8-bit passes, MSB first down to bit LAST: the key of the kk-th largest entry and how many of the
 // entries tied at it the selection takes. KeyAt(i) returns the key of element i.
 // Every thread of the CTA must call it. Each warp counts into its own histogram, so tie-heavy
 // arrays (ReLU zeros) never serialise the whole CTA on one bin.
-template <class KeyAt>
+// LAST = 16: two passes, for keys whose upper halves decide (the lower half of the returned pivot is 0).
+template <int LAST = 0, class KeyAt>
 __device__ __forceinline__ void tk_radix_select(KeyAt key_at, int nt, uint32_t kk, TkShared& sh, uint32_t& pivot_out,
                                                 uint32_t& need_out) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     uint32_t pivot = 0u, mask = 0u, need = kk;
-    for (int shift = 24; shift >= 0; shift -= 8) {
+    for (int shift = 24; shift >= LAST; shift -= 8) {
         for (int i = tid; i < TK_WARPS * 256; i += TK_THREADS) (&sh.whist[0][0])[i] = 0u;
         __syncthreads();
         for (int base = 0; base < nt; base += TK_THREADS) {

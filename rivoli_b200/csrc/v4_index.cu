@@ -403,8 +403,8 @@ __global__ void __launch_bounds__(ST_THREADS) v4_score_tc_kernel(StArgs A, const
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = tmem_slot;
-    rv_grid_dep_trigger();
     rv_grid_dep_wait();
+    rv_grid_dep_trigger();   // (after the wait: see the selection kernel)
     const int n_items = A.n_seqs * A.chunks;
     // sequences that select by position are not scored
     auto item_rows = [&](int item, int& b, int& t0, int& t1, int& n) {
@@ -647,10 +647,11 @@ __global__ void __launch_bounds__(TK_THREADS) v4_select_kernel(V4Geom g, const i
 
     const int b = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     rv_grid_dep_trigger();   // the attention kernel may be scheduled; it waits for this grid before it reads anything
-    // Every CTA waits for the scorer first, including those that return early below: the kernel launched after
-    // this one relies on "this grid is complete" implying "everything before it is complete", and `sel` may
-    // still be read by a kernel of the previous step that the scorer's own wait orders.
-    rv_grid_dep_wait();
+    // Every CTA waits for the scorer, including those that return early below: the kernel launched after
+    // this one relies on "this grid is complete" implying "everything before it is complete". Behind the scorer (which
+    // starts this kernel only when all before itself is complete: the readers of `sel` in the step before, the position's
+    // writer) the ring's part of the row is written while it still runs.
+    if (force_fold) rv_grid_dep_wait();
     const int W = g.window, K = g.index_topk, p = pos[b];
     int32_t* row = sel + (size_t)b * (W + K);
     // the ring: oldest first once full, live slots then -1 before that
@@ -662,6 +663,7 @@ __global__ void __launch_bounds__(TK_THREADS) v4_select_kernel(V4Geom g, const i
     }
     int n_comp = (p + 1) / g.ratio;
     n_comp = n_comp < g.max_comp ? n_comp : g.max_comp;
+    if (!force_fold) rv_grid_dep_wait();
     if (n_comp <= K) {   // every closed block, in order
         if (tid == 0 && !force_fold) flags[b] = 0;
         for (int c = tid; c < K; c += TK_THREADS) row[W + c] = c < n_comp ? W + c : -1;
@@ -730,7 +732,9 @@ __global__ void __launch_bounds__(TK_THREADS) v4_select_kernel(V4Geom g, const i
     __syncthreads();
     auto key_at = [&](int i) { return v4_total_key(sc[i]); };
     uint32_t pivot, need;
-    tk_radix_select(key_at, n_comp, (uint32_t)K, sh.tk, pivot, need);
+    // scores are bf16 values: the lower half of a key is 0 under a set sign bit (a value >= +0) and all ones else
+    tk_radix_select<16>(key_at, n_comp, (uint32_t)K, sh.tk, pivot, need);
+    if (!(pivot & 0x80000000u)) pivot |= 0xffffu;
     tk_compact(key_at, n_comp, (uint32_t)K, pivot, need, sh.tk, picked);
     __syncthreads();
     for (int j = tid; j < K; j += TK_THREADS) row[W + j] = W + (int32_t)picked[j];
