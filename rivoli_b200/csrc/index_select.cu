@@ -134,7 +134,7 @@ __device__ __forceinline__ void sel_token_excl(uint32_t mask, SelXc& xc, uint32_
 
 template <bool VALUES, bool SOLO>
 __global__ void __launch_bounds__(SEL_NT, 1)
-index_select_kernel(SelArgs A, int CH) {
+index_select_cluster_kernel(SelArgs A, int CH) {
     cg::cluster_group cluster = cg::this_cluster();
     const int C = SOLO ? 1 : (int)cluster.dim_blocks().x, r = SOLO ? 0 : (int)cluster.block_rank();
     if constexpr (!SOLO) cluster.barrier_arrive();                        // [0] every CTA runs: its memory may be written
@@ -687,8 +687,8 @@ static int launch_select(const SelArgs& a, int B, int C, int ch, cudaStream_t st
     at[1].val.clusterDim.x = (unsigned)C; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
     cfg.attrs = at; cfg.numAttrs = 2;
     rv_drain_error();
-    rv_allow_smem<index_select_kernel<VALUES, SOLO>>((int)((fixed + SEL_CH) * 4));
-    (void)cudaLaunchKernelEx(&cfg, index_select_kernel<VALUES, SOLO>, a, ch);
+    rv_allow_smem<index_select_cluster_kernel<VALUES, SOLO>>((int)((fixed + SEL_CH) * 4));
+    (void)cudaLaunchKernelEx(&cfg, index_select_cluster_kernel<VALUES, SOLO>, a, ch);
     return rv_launch_status();
 }
 
