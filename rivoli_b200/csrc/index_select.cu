@@ -364,6 +364,9 @@ index_select_cluster_kernel(SelArgs A, int CH) {
         if (xc.bstar > 0 && lo_f == lo_f) k_lo = topk_key(lo_f);
         if (hi_f == hi_f) k_hi = topk_key(hi_f);
     }
+    // the histogram is dead (its remote readers passed [3]): counters of the ranking; a lone CTA's list ends in empty slots
+    static_assert(SEL_LIST + SEL_RANK_ALL <= SEL_BINS, "dec and cnt take the histogram's place");
+    hist[SEL_LIST + tid] = 0u;
     uint32_t m_in = 0u, m_band = 0u;                                          // bit 4 * step + e
     for_keys([&](int it, int, int e, uint32_t k) {
         const uint32_t bit = 1u << (4 * it + e);
@@ -399,6 +402,7 @@ index_select_cluster_kernel(SelArgs A, int CH) {
     const uint32_t n_in_mine = __reduce_add_sync(0xffffffffu, xc.red[buf][lane]);
     buf ^= 1;
     const uint32_t n_band_mine = xc.list_n;
+    if (SOLO && tid < 8 && n_band_mine + tid < (uint32_t)SEL_LIST) l_cmp[n_band_mine + tid] = 0ull;
 
     // Exact key of the first `ln` listed tokens -> l_cmp[position] (0 and ~0 are reserved for "surely out" / "surely in").
     auto rescore = [&](uint32_t ln) {
@@ -423,10 +427,9 @@ index_select_cluster_kernel(SelArgs A, int CH) {
     };
 
     // ---- 4. exact keys of the band -------------------------------------------------------------------------
-    if constexpr (!VALUES) {
+    if constexpr (!VALUES)
         if (n_band_mine <= (uint32_t)SEL_LIST) rescore(n_band_mine);
-        __syncthreads();
-    }
+    __syncthreads();
     uint32_t n_in = n_in_mine, n_band = n_band_mine;
     const uint32_t RG = SEL_LIST / C;                                         // entries of one rank in everybody's gathered list
     uint32_t n_all = n_band_mine;                                             // gathered entries, empty slots included
@@ -456,18 +459,29 @@ index_select_cluster_kernel(SelArgs A, int CH) {
         // Band tokens are ranked among ALL of them by (exact key descending, index ascending).
         const bool rank_all = n_all <= (uint32_t)SEL_RANK_ALL;
         if (rank_all) {
-            // an entry per thread; the selected ones of the lower ranks say where this CTA's rows begin
-            if (tid < (int)n_all) {
-                const uint64_t mine = all_cmp[tid];
+            // `parts` threads per entry, each against its share of the list in batches of eight (one pair of entries at a
+            // time costs a shared-memory round trip a pair: 320 entries 8,800 cycles); their counts meet in `cnt`. The
+            // selected entries of the lower ranks say where this CTA's rows begin.
+            uint32_t* cnt = hist + SEL_LIST;                                  // [SEL_RANK_ALL], zeroed with the list
+            const int sh = n_all <= SEL_NT / 8 ? 3 : (n_all <= SEL_NT / 4 ? 2 : (n_all <= SEL_NT / 2 ? 1 : 0));
+            const uint32_t e = (uint32_t)tid & ((SEL_NT >> sh) - 1), per = (((n_all + 7) / 8 + (1u << sh) - 1) >> sh) * 8;
+            const uint64_t mine = e < n_all ? all_cmp[e] : 0ull;
+            if (e < n_all) {
+                const uint32_t j0 = ((uint32_t)tid >> (10 - sh)) * per, j1 = min(j0 + per, (n_all + 7) / 8 * 8);
                 uint32_t c = 0;
-                uint32_t j = 0;
-#pragma unroll 4
-                for (; j + 2 <= n_all; j += 2) {                              // broadcast reads of two entries
-                    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(all_cmp + j);
-                    c += (v.x > mine ? 1u : 0u) + (v.y > mine ? 1u : 0u);
+#pragma unroll 1
+                for (uint32_t j = j0; j < j1; j += 8) {                       // (broadcast reads; the list ends in empty slots)
+                    ulonglong2 v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) v[u] = reinterpret_cast<const ulonglong2*>(all_cmp + j)[u];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) c += (v[u].x > mine ? 1u : 0u) + (v[u].y > mine ? 1u : 0u);
                 }
-                if (j < n_all) c += all_cmp[j] > mine ? 1u : 0u;
-                const bool win = c < take;
+                if (c) atomicAdd(&cnt[e], c);
+            }
+            __syncthreads();
+            if (tid < (int)n_all) {
+                const bool win = cnt[tid] < take;
                 const int q = SOLO ? 0 : tid & (C - 1);
                 if (q == r) dec[SOLO ? tid : tid / C] = win ? 1u : 0u;        // (an empty slot's entry is never looked at)
                 else if (q < r && win && mine != 0ull) atomicAdd(&xc.lower, 1u);
