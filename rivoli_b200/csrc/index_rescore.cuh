@@ -28,18 +28,23 @@ __device__ __forceinline__ uint64_t rs_fma2(uint64_t a, uint64_t b, uint64_t c) 
     return r;
 }
 
-// Scores the tokens toks[0 .. ln): a pass covers WARPS * 4 of them, warp w taking positions base + 4 w .. + 3.
+// Pool row of token t (rows of unmapped pages stand in as page 0).
+__device__ __forceinline__ uint32_t rv_pool_row(const DsaGeom& g, const int32_t* __restrict__ bt, uint32_t t) {
+    const int pshift = 31 - __clz(g.page_tokens), pg = bt[t >> pshift];   // page sizes are powers of two
+    return ((pg < 0 || pg >= g.n_pool_pages ? 0u : (uint32_t)pg) << pshift) + (t & (uint32_t)(g.page_tokens - 1));
+}
+
+// Scores `ln` listed tokens, row_of(position) being a token's pool row: a pass covers WARPS * 4 of them, warp w taking
+// positions base + 4 w .. + 3.
 // kf = this WARP's staging of four key rows as f32, [dim][token] (RS_HD * 4 floats, 16-byte aligned). my_sq / my_wh = this
 // lane's head scale and weight * wscale (0 for lanes >= nh). emit(position, score) is called by one lane per token.
-template <int WARPS, class Emit>
-__device__ __forceinline__ void rv_rescore_listed(const uint32_t* toks, uint32_t ln, const uint32_t* qf, float* kf,
-                                                  const int32_t* __restrict__ bt, const DsaGeom& g,
+template <int WARPS, class RowOf, class Emit>
+__device__ __forceinline__ void rv_rescore_listed(RowOf row_of, uint32_t ln, const uint32_t* qf, float* kf, const DsaGeom& g,
                                                   const uint8_t* __restrict__ index_pool,
                                                   const float* __restrict__ index_scale, float my_sq, float my_wh,
                                                   Emit emit) {
     constexpr int TOK = 4, PAD = 36;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int pshift = 31 - __clz(g.page_tokens);          // page sizes are powers of two
 #pragma unroll 1
     for (uint32_t p0 = warp * TOK; p0 < ln; p0 += WARPS * TOK) {
         const int n_here = min(TOK, (int)(ln - p0));
@@ -49,10 +54,7 @@ __device__ __forceinline__ void rv_rescore_listed(const uint32_t* toks, uint32_t
         for (int e = 0; e < TOK; ++e) {
             cw[e] = 0u; skv[e] = 0.0f;
             if (e < n_here) {
-                const int t = (int)toks[p0 + e];
-                int pg = bt[t >> pshift];
-                pg = (pg < 0 || pg >= g.n_pool_pages) ? 0 : pg;
-                const size_t rr = ((size_t)pg << pshift) + (t & (g.page_tokens - 1));
+                const size_t rr = row_of(p0 + e);
                 cw[e] = *reinterpret_cast<const uint32_t*>(index_pool + rr * RS_HD + lane * 4);
                 skv[e] = index_scale[rr];
             }

@@ -144,7 +144,8 @@ index_select_cluster_kernel(SelArgs A, int CH) {
     uint32_t* hist = keys + CH;                                           // [SEL_BINS]; later `dec`
     uint32_t* l_tok = hist + SEL_BINS;                                    // [SEL_LIST] this CTA's band tokens
     uint64_t* l_cmp = reinterpret_cast<uint64_t*>(l_tok + SEL_LIST);      // [SEL_LIST] their exact keys, ~token below: larger = ranked higher
-    uint32_t* red = l_tok + 3 * SEL_LIST;                                  // [SEL_BINS] reduced histogram, before the re-score
+    uint32_t* l_row = l_tok + 3 * SEL_LIST;                               // [SEL_LIST] their pool rows (the lookup is done where the token is listed)
+    uint32_t* red = l_row + SEL_LIST;                                  // [SEL_BINS] reduced histogram, before the re-score
     float* kfw = reinterpret_cast<float*>(red);                           // [warps][SEL_HD][4] key rows as f32
     uint32_t* qf = red + SEL_NW * SEL_HD * 4;                             // [RS_QWORDS] packed q codes
     uint64_t* a_cmp = reinterpret_cast<uint64_t*>(VALUES ? red + SEL_BINS : qf + RS_QWORDS);   // [SEL_LIST] the cluster's band (clusters only)
@@ -198,6 +199,10 @@ index_select_cluster_kernel(SelArgs A, int CH) {
     auto scale_row = [&](int i, int pg) {
         pg = (pg < 0 || pg >= g.n_pool_pages) ? 0 : pg;
         return ((size_t)pg << pshift) + (i & (P - 1));
+    };
+    auto page_of = [&](int it) { return it < 2 ? (it ? pgs[1] : pgs[0]) : (it == 2 ? pgs[2] : pgs[3]); };   // of this thread's tokens of step `it` (P % 4 == 0)
+    auto row_of_bit = [&](int bit, int i) {                                   // pool row of token c0 + i, bit = 4 * step + e
+        return A.vec_ok ? (uint32_t)scale_row(c0 + i, page_of(bit >> 2)) : rv_pool_row(g, bt, (uint32_t)(c0 + i));
     };
     uint32_t kmin = 0xffffffffu, kmax = 0u;
     float skm = 0.0f;
@@ -268,16 +273,21 @@ index_select_cluster_kernel(SelArgs A, int CH) {
     }
     if (r == 0 && tid == 0 && (!VALUES || A.n_sel)) A.n_sel[b] = kk;
     // keys of this thread's four tokens of step `it` (only this thread reads and writes them until the slow path's end)
-    auto for_keys = [&](auto f) {                                          // f(step, local index, e, key)
+    auto for_keys = [&](auto f) {                                          // f(step, e, key)
 #pragma unroll 1
         for (int it = 0; it < steps; ++it) {
             const int i4 = it * SEL_STEP + tid * 4;
             if (i4 < nloc) {
                 const uint4 k = *reinterpret_cast<const uint4*>(keys + i4);
-                f(it, i4, 0, k.x);
-                if (i4 + 1 < nloc) f(it, i4, 1, k.y);
-                if (i4 + 2 < nloc) f(it, i4, 2, k.z);
-                if (i4 + 3 < nloc) f(it, i4, 3, k.w);
+                f(it, 0, k.x);
+                if (i4 + 4 <= nloc) {
+                    f(it, 1, k.y);
+                    f(it, 2, k.z);
+                    f(it, 3, k.w);
+                } else {
+                    if (i4 + 1 < nloc) f(it, 1, k.y);
+                    if (i4 + 2 < nloc) f(it, 2, k.z);
+                }
             }
         }
     };
@@ -317,7 +327,7 @@ index_select_cluster_kernel(SelArgs A, int CH) {
     float inv_w = (float)SEL_BINS / (vmax - vmin);
     if (!(inv_w > 0.0f) || !(inv_w < 3.0e38f)) inv_w = 0.0f;
     if (inv_w > 0.0f)
-        for_keys([&](int, int, int, uint32_t k) {
+        for_keys([&](int, int, uint32_t k) {
             atomicAdd(&hist[(uint32_t)fminf((topk_unkey(k) - vmin) * inv_w, (float)(SEL_BINS - 1))], 1u);
         });
     else if (tid == 0) hist[0] = (uint32_t)nloc;
@@ -368,11 +378,14 @@ index_select_cluster_kernel(SelArgs A, int CH) {
     static_assert(SEL_LIST + SEL_RANK_ALL <= SEL_BINS, "dec and cnt take the histogram's place");
     hist[SEL_LIST + tid] = 0u;
     uint32_t m_in = 0u, m_band = 0u;                                          // bit 4 * step + e
-    for_keys([&](int it, int, int e, uint32_t k) {
-        const uint32_t bit = 1u << (4 * it + e);
-        if (k > k_hi) m_in |= bit;
-        else if (k >= k_lo) m_band |= bit;
-    });
+    {
+        uint32_t ge = 0u;                                                     // in the band or above it
+        for_keys([&](int it, int e, uint32_t k) {
+            m_in |= (k > k_hi ? 1u << e : 0u) << (4 * it);
+            ge |= (k >= k_lo ? 1u << e : 0u) << (4 * it);
+        });
+        m_band = ge & ~m_in;
+    }
     auto local_of = [&](int bit) { return ((bit >> 2) * SEL_NT + tid) * 4 + (bit & 3); };
     {   // this CTA's count of surely selected tokens: the warp sums meet at the barrier that closes the list
         const uint32_t v = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(m_in));
@@ -393,8 +406,9 @@ index_select_cluster_kernel(SelArgs A, int CH) {
         my_pos = wbase + incl - cnt;
         uint32_t pos = my_pos;
         for (uint32_t m = m_band; m && pos < SEL_LIST; m &= m - 1u, ++pos) {
-            const int i = local_of(__ffs(m) - 1);
+            const int bit = __ffs(m) - 1, i = local_of(bit);
             l_tok[pos] = (uint32_t)(c0 + i);
+            if (!VALUES) l_row[pos] = row_of_bit(bit, i);
             if (VALUES) l_cmp[pos] = ((uint64_t)keys[i] << 32) | ~(uint32_t)(c0 + i);
         }
     }
@@ -406,7 +420,7 @@ index_select_cluster_kernel(SelArgs A, int CH) {
 
     // Exact key of the first `ln` listed tokens -> l_cmp[position] (0 and ~0 are reserved for "surely out" / "surely in").
     auto rescore = [&](uint32_t ln) {
-        rv_rescore_listed<SEL_NW>(l_tok, ln, qf, kfw + warp * (SEL_HD * 4), bt, g, A.index_pool, A.index_scale, my_sq, my_wh,
+        rv_rescore_listed<SEL_NW>([&](uint32_t i) { return l_row[i]; }, ln, qf, kfw + warp * (SEL_HD * 4), g, A.index_pool, A.index_scale, my_sq, my_wh,
                                   [&](uint32_t pos, float score) {
             uint32_t ku = topk_key(score);
             ku = ku == 0xffffffffu ? 0xfffffffeu : (ku == 0u ? 1u : ku);
@@ -548,7 +562,11 @@ index_select_cluster_kernel(SelArgs A, int CH) {
             uint32_t pos0 = bits ? atomicAdd(&xc.list_n, (uint32_t)__popc(bits)) : 0u;
             {
                 uint32_t pos = pos0;
-                for (uint32_t m = bits; m; m &= m - 1u) l_tok[pos++] = (uint32_t)(c0 + i4 + __ffs(m) - 1);
+                for (uint32_t m = bits; m; m &= m - 1u, ++pos) {
+                    const int e = __ffs(m) - 1;
+                    l_tok[pos] = (uint32_t)(c0 + i4 + e);
+                    l_row[pos] = row_of_bit(4 * it + e, i4 + e);
+                }
             }
             __syncthreads();
             rescore(xc.list_n);
@@ -574,7 +592,7 @@ index_select_cluster_kernel(SelArgs A, int CH) {
         __syncthreads();
         for (int i = tid; i < SEL_NW * 256; i += SEL_NT) whist[i] = 0u;
         __syncthreads();
-        for_keys([&](int, int, int, uint32_t k) {
+        for_keys([&](int, int, uint32_t k) {
             if ((k & mask) == pivot) atomicAdd(&whist[warp * 256 + ((k >> sh2) & 0xffu)], 1u);
         });
         __syncthreads();
@@ -621,7 +639,7 @@ index_select_cluster_kernel(SelArgs A, int CH) {
     }
     // `need` of the tokens tied at the pivot are taken, in ascending global index = ascending rank, then token order
     uint32_t sel_gt = 0u, sel_eq = 0u;
-    for_keys([&](int it, int, int e, uint32_t k) {
+    for_keys([&](int it, int e, uint32_t k) {
         if (k > pivot) sel_gt |= 1u << (4 * it + e);
         else if (k == pivot) sel_eq |= 1u << (4 * it + e);
     });
@@ -689,7 +707,7 @@ namespace rivoli {
 
 template <bool VALUES, bool SOLO>
 static int launch_select(const SelArgs& a, int B, int C, int ch, cudaStream_t st) {
-    constexpr size_t fixed = SEL_BINS + 3 * SEL_LIST + (VALUES ? SEL_BINS : SEL_NW * SEL_HD * 4 + RS_QWORDS) + (SOLO ? 0 : 2 * SEL_LIST);
+    constexpr size_t fixed = SEL_BINS + 4 * SEL_LIST + (VALUES ? SEL_BINS : SEL_NW * SEL_HD * 4 + RS_QWORDS) + (SOLO ? 0 : 2 * SEL_LIST);
     static_assert((fixed + SEL_CH) * 4 + sizeof(SelXc) + 1024 <= 232448, "shared memory budget");
     const size_t smem = (fixed + (size_t)ch) * 4;
     cudaLaunchConfig_t cfg = {};

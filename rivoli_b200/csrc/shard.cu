@@ -61,10 +61,11 @@ shard_rescore_kernel(DsaGeom g, const uint8_t* __restrict__ qcodes, const float*
     __syncthreads();
     const float my_sq = lane < nh ? qscales[(size_t)b * nh + lane] : 0.0f;
     const float my_wh = lane < nh ? __fmul_rn(w[(size_t)b * nh + lane], g.index_wscale) : 0.0f;
-    rv_rescore_listed<SH_WARPS>(rows + (size_t)b * k + j0, (uint32_t)min(per_cta, n - j0), qf,
-                                        kfw + warp * (SH_TOK * RS_HD), block_table + (size_t)b * g.max_pages_per_seq, g,
-                                        index_pool, index_scale, my_sq, my_wh,
-                                        [&](uint32_t pos, float score) { out[j0 + pos] = score; });
+    const uint32_t* toks = rows + (size_t)b * k + j0;
+    const int32_t* bt = block_table + (size_t)b * g.max_pages_per_seq;
+    rv_rescore_listed<SH_WARPS>([&](uint32_t i) { return rv_pool_row(g, bt, toks[i]); }, (uint32_t)min(per_cta, n - j0), qf,
+                                kfw + warp * (SH_TOK * RS_HD), g, index_pool, index_scale, my_sq, my_wh,
+                                [&](uint32_t pos, float score) { out[j0 + pos] = score; });
 }
 
 // ---- B: the gathered candidates as one score row per sequence, [rank 0 | rank 1 | ...] --------------------------
