@@ -109,7 +109,7 @@ class V4TokenStep:
         (kv_proj, score_proj) f32 [B, cd] of the two compressors; q, index_q, index_w as for V4DecodeLayer.step."""
         L, g = self.layer, self.layer.g
         be.launch_v4_token_step_bf16(
-            g, L.B, pos, kv_entry, self.attn_comp.p, self.attn_comp.step_args(*attn_proj, L.kv_cache, L.kv_rows, g.window),
+            g, L.B, pos, kv_entry.contiguous(), self.attn_comp.p, self.attn_comp.step_args(*attn_proj, L.kv_cache, L.kv_rows, g.window),
             self.index_comp.p, self.index_comp.step_args(*index_proj, L.index_kv, g.max_comp, 0, L.packed, L.packed_exp),
             q, index_q, index_w, L.sink, L.sel, L.scratch, L.out, stream)
         return L.out
