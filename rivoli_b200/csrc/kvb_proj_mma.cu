@@ -68,13 +68,15 @@ struct KpArgs {
     uint16_t* out;
 };
 
-// All of a tile's bytes are requested before anything is waited for: contraction chunks of 64, one cp.async group each
-// (activations, raw codes), then chunk by chunk the codes are converted (two tile buffers) and the chunk's MMAs issued while
-// later chunks are still on their way. The result is staged in the idle converted tiles and leaves as whole rows.
-// 128 sequences, us: absorb 16.4 -> 10.4, value 15.9 -> 11.6 (loads into registers, one conversion pass, two halves of the
-// value contraction one after the other, 16-byte stores to 32 rows at a time); bound by what an SM can take in
-// (192 KiB at 18 bytes a clock in the value kernel), a launch's ramp and the epilogue.
+// The contraction in chunks of 64, one cp.async group each (activations, raw codes), requested ahead: all of them in the absorb
+// kernel, three in the value kernel. A chunk's codes are converted (two tile buffers) and its MMAs issued while later chunks are
+// on their way. The result is staged in the idle converted tiles and leaves as whole rows.
+// 128 sequences, us: absorb 16.4 -> 10.6, value 15.9 -> 10.9 (loads into registers, one conversion pass, two halves of the
+// value contraction one after the other, 16-byte stores to 32 rows at a time); bound by what an SM takes in
+// (192 KiB at 18 bytes a clock in the value kernel), a launch's ramp and the epilogue. With all eight chunks in flight (224 KiB)
+// a value CTA could not start before both absorb CTAs had left its SM: 48.9 -> 47.3 us for the three projection operators.
 constexpr int KP_ACHUNK = 16384, KP_WCHUNK = 8192, KP_CONV = 16384;
+constexpr int KP_VST = 3;      // chunks in flight in the value kernel
 static_assert(2 * KP_CONV == 128 * 256, "the result fits the converted tiles");
 
 // Requests activation chunk c (128 sequences from b0 x 64 bf16, swizzled K-major; rows past B are zeros) into `dst`.
@@ -257,8 +259,8 @@ kvb_absorb_mma_kernel(KpArgs A) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// value: grid (vh / 128, H), N = 128 value rows = two 64-row scale rows. Shared: activation chunks [kvl/64][128 rows][128 B] |
-// raw codes [kvl/64][128 rows][64 B] | two converted tiles [128 rows][128 B] (K-major).
+// value: grid (vh / 128, H), N = 128 value rows = two 64-row scale rows. Shared: activation chunks [3][128 rows][128 B] |
+// raw codes [3][128 rows][64 B] | two converted tiles [128 rows][128 B] (K-major).
 // TMEM: one 128-column accumulator per scale column (kvl / 128 <= 4 runs).
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(KP_THREADS)
@@ -273,8 +275,8 @@ kvb_value_mma_kernel(KpArgs A) {
     const int jblk = blockIdx.x, h = blockIdx.y;
     const int kvl = A.kvl, vh = A.vh, nch = kvl / 64;
     uint8_t* sA = smem;
-    uint8_t* sW = sA + nch * KP_ACHUNK;
-    uint8_t* sB = sW + nch * KP_WCHUNK;
+    uint8_t* sW = sA + KP_VST * KP_ACHUNK;
+    uint8_t* sB = sW + KP_VST * KP_WCHUNK;
     const size_t row0 = (size_t)h * (A.nope + vh) + A.nope + (size_t)jblk * 128;   // 128 value rows = 2 scale rows
     const int sc_cols = kvl / 128;
     if (tid == 0) { tc::mbar_init(&bar[0], 1); tc::mbar_init(&bar[1], 1); tc::mbar_init_fence(); abort_word = 0; }
@@ -283,15 +285,20 @@ kvb_value_mma_kernel(KpArgs A) {
     kp_prefetch(A.x + (size_t)h * A.xs, (size_t)A.H * A.xs * 2, min(128, A.B), kvl * 2);
     if (warp == 0) tc::tmem_alloc<512>(&tmem_slot);
     rv_grid_dep_wait();
-    for (int c = 0; c < nch; ++c) {
-        kp_request_acts(A, h, 0, c, sA + c * KP_ACHUNK);
+    auto request = [&](int b0, int c) {   // one cp.async group per call, with or without a chunk
+        if (c < nch) {
+            const int st = c % KP_VST;
+            kp_request_acts(A, h, b0, c, sA + st * KP_ACHUNK);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int e = tid + i * KP_THREADS, r = e >> 2, j = e & 3;
-            tc::cp_async16(tc::smem_u32(sW + c * KP_WCHUNK + r * 64 + j * 16), A.kvb + (row0 + r) * kvl + c * 64 + j * 16);
+            for (int i = 0; i < 2; ++i) {
+                const int e = tid + i * KP_THREADS, r = e >> 2, j = e & 3;
+                tc::cp_async16(tc::smem_u32(sW + st * KP_WCHUNK + r * 64 + j * 16), A.kvb + (row0 + r) * kvl + c * 64 + j * 16);
+            }
         }
         tc::cp_async_commit();
-    }
+    };
+#pragma unroll 1
+    for (int c = 0; c < KP_VST; ++c) request(0, c);
     if (tid < 2 * sc_cols) s_sc[tid / sc_cols][tid % sc_cols] = A.scale[((row0 + (tid / sc_cols) * 64) >> 7) * sc_cols + tid % sc_cols];
     tc::tc_fence_before();
     __syncthreads();
@@ -304,23 +311,24 @@ kvb_value_mma_kernel(KpArgs A) {
     int done[2] = {0, 0};
     for (int b0 = 0; b0 < A.B && ok; b0 += 128) {
         if (b0 > 0)
-            for (int c = 0; c < nch; ++c) { kp_request_acts(A, h, b0, c, sA + c * KP_ACHUNK); tc::cp_async_commit(); }
+            for (int c = 0; c < KP_VST; ++c) request(b0, c);
         for (int c = 0; c < nch && ok; ++c) {
             const int wb = c & 1;
             if (done[wb] > 0) ok = tc::mbar_wait_warp(&bar[wb], (done[wb] - 1) & 1, abort_flag, 73);
             if (!ok) break;
-            kp_wait_groups(nch - 1 - c);   // (a thread converts the codes that it requested itself)
+            if (c >= 2) request(b0, c - 2 + KP_VST);   // the stage that the MMAs of chunk c - 2 have read
+            if (c == 0) tc::cp_async_wait<KP_VST - 1>(); else tc::cp_async_wait<KP_VST - 2>();   // (a thread converts the codes that it requested itself)
             uint8_t* sb = sB + wb * KP_CONV;
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const int e = tid + i * KP_THREADS, r = e >> 2, j = e & 3;
-                kp_convert16(sW + c * KP_WCHUNK + r * 64 + j * 16, sb + tc::sw128_chunk(r, 2 * j), sb + tc::sw128_chunk(r, 2 * j + 1));
+                kp_convert16(sW + (c % KP_VST) * KP_WCHUNK + r * 64 + j * 16, sb + tc::sw128_chunk(r, 2 * j), sb + tc::sw128_chunk(r, 2 * j + 1));
             }
             tc::fence_proxy_async();
             __syncthreads();
             if (warp == 0 && tc::elect_one()) {
                 tc::tc_fence_after();
-                const uint32_t a0 = tc::smem_u32(sA + c * KP_ACHUNK), w0 = tc::smem_u32(sb);
+                const uint32_t a0 = tc::smem_u32(sA + (c % KP_VST) * KP_ACHUNK), w0 = tc::smem_u32(sb);
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
                     kp_mma(tmem + (c >> 1) * 128, kp_desc(a0 + k * 32, 16, 1024), kp_desc(w0 + k * 32, 16, 1024), idesc, ((c & 1) | k) ? 1u : 0u);
@@ -392,10 +400,11 @@ extern "C" int rivoli_kvb_absorb_mma(const uint16_t* q, const uint8_t* kvb, cons
 extern "C" int rivoli_kvb_value_mma(const uint16_t* clat, const uint8_t* kvb, const float* scale, int H, int nope, int vh,
                                     int kvl, int block, int B, uint16_t* ctx, cudaStream_t st) {
     const KpArgs a{clat, kvb, scale, H, kvl, nope, vh, kvl, 0, block, B, ctx};
-    const size_t smem = (size_t)(kvl / 64) * (KP_ACHUNK + KP_WCHUNK) + 2 * KP_CONV;
-    rv_allow_smem<kvb_value_mma_kernel>(8 * (KP_ACHUNK + KP_WCHUNK) + 2 * KP_CONV);
+    // beside one CTA of the absorb kernel, but never two on an SM (each takes all of its tensor memory)
+    constexpr int need = KP_VST * (KP_ACHUNK + KP_WCHUNK) + 2 * KP_CONV, smem = need > 116 * 1024 ? need : 116 * 1024;
+    rv_allow_smem<kvb_value_mma_kernel>(smem);
     rv_drain_error();
-    rv_launch_dependent(kvb_value_mma_kernel, dim3(vh / 128, H), dim3(KP_THREADS), smem, st, a);
+    rv_launch_dependent(kvb_value_mma_kernel, dim3(vh / 128, H), dim3(KP_THREADS), (size_t)smem, st, a);
     return rv_launch_status();
 }
 
