@@ -20,7 +20,8 @@
 
 namespace {
 
-constexpr int KP_THREADS = 256;   // 8 warps; epilogue by (lane quadrant, column half)
+constexpr int KP_THREADS = 256;   // warps 0-7 request, convert and store (epilogue by (lane quadrant, column half))
+constexpr int KP_LAUNCH = KP_THREADS + 32;   // warp 8 issues the MMAs: by one of the converting warps that took half of a chunk's time
 __device__ int g_kp_err;
 
 __device__ __forceinline__ uint64_t kp_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
@@ -61,6 +62,12 @@ __device__ __forceinline__ uint4 kp_codes_to_bf16(uint2 c) {
     return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
+__device__ __forceinline__ uint32_t kp_pack(float a, float b) {   // two f32 -> bf16x2, round to nearest even
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+    return r;
+}
+
 struct KpArgs {
     const uint16_t* x;      // activations [B][H][xs] bf16 (xs = row pitch per head)
     const uint8_t* kvb; const float* scale;
@@ -71,7 +78,7 @@ struct KpArgs {
 // The contraction in chunks of 64, one cp.async group each (activations, raw codes), requested ahead: all of them in the absorb
 // kernel, three in the value kernel. A chunk's codes are converted (two tile buffers) and its MMAs issued while later chunks are
 // on their way. The result is staged in the idle converted tiles and leaves as whole rows.
-// 128 sequences, us: absorb 16.4 -> 10.6, value 15.9 -> 10.9 (loads into registers, one conversion pass, two halves of the
+// 128 sequences, us: absorb 16.4 -> 8.6, value 15.9 -> 9.7 (loads into registers, one conversion pass, two halves of the
 // value contraction one after the other, 16-byte stores to 32 rows at a time); bound by what an SM takes in
 // (192 KiB at 18 bytes a clock in the value kernel), a launch's ramp and the epilogue. With all eight chunks in flight (224 KiB)
 // a value CTA could not start before both absorb CTAs had left its SM: 48.9 -> 47.3 us for the three projection operators.
@@ -93,7 +100,7 @@ __device__ __forceinline__ void kp_request_acts(const KpArgs& A, int h, int b0, 
 // CTA may sit here while the kernel before it finishes; a prefetch into L2 may precede the dependency wait, whoever writes.
 __device__ __forceinline__ void kp_prefetch(const void* base, size_t pitch, int n, int bytes) {
     const int lines = (bytes + 127) / 128;
-    for (int e = threadIdx.x; e < n * lines; e += KP_THREADS) {
+    for (int e = threadIdx.x; e < n * lines; e += KP_LAUNCH) {
         const int r = e / lines;
         asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint8_t*>(base) + (size_t)r * pitch + (e - r * lines) * 128));
     }
@@ -132,10 +139,10 @@ __device__ __forceinline__ void kp_store_rows(const uint8_t* stage, uint16_t* ou
 // absorb: grid (kvl / 128, H). Shared: activation chunks [nope/64][128 rows][128 B] | raw codes [nope/64][64 rows][128 B] |
 // two converted tiles [2 column halves][64 rows][128 B] (MN-major).
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(KP_THREADS)
+__global__ void __launch_bounds__(KP_LAUNCH)
 kvb_absorb_mma_kernel(KpArgs A) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ uint64_t bar[2];
+    __shared__ uint64_t bar[2], full[2];   // MMAs of a converted tile done | its conversion done
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_word;
     volatile int* abort_flag = &abort_word;
@@ -150,13 +157,17 @@ kvb_absorb_mma_kernel(KpArgs A) {
     // runs of d with one scale: [0, cut) and [cut, nope); cut = distance to the next block boundary
     const int cut = min(nope, (int)(128 - (rbase & 127)));
     const bool two_runs = cut < nope;
-    if (tid == 0) { tc::mbar_init(&bar[0], 1); tc::mbar_init(&bar[1], 1); tc::mbar_init_fence(); abort_word = 0; }
+    if (tid == 0) {
+        for (int i = 0; i < 2; ++i) { tc::mbar_init(&bar[i], 1); tc::mbar_init(&full[i], KP_THREADS); }
+        tc::mbar_init_fence();
+        abort_word = 0;
+    }
     rv_grid_dep_trigger();
     kp_prefetch(A.kvb + rbase * kvl + iblk * 128, (size_t)kvl, nope, 128);
     kp_prefetch(A.x + (size_t)h * A.xs, (size_t)A.H * A.xs * 2, min(128, A.B), nope * 2);
-    if (warp == 0) tc::tmem_alloc<256>(&tmem_slot);
+    if (warp == 8) tc::tmem_alloc<256>(&tmem_slot);
     rv_grid_dep_wait();
-    for (int c = 0; c < nch; ++c) {
+    if (warp < 8) for (int c = 0; c < nch; ++c) {
         kp_request_acts(A, h, 0, c, sA + c * KP_ACHUNK);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
@@ -177,6 +188,25 @@ kvb_absorb_mma_kernel(KpArgs A) {
     bool ok = true;
     int done[2] = {0, 0};
     for (int b0 = 0; b0 < A.B && ok; b0 += 128) {
+        if (warp == 8) {
+            for (int c = 0; c < nch && ok; ++c) {
+                const int wb = c & 1, run = c * 64 >= cut ? 1 : 0;       // (a run boundary is a multiple of 64)
+                ok = tc::mbar_wait_warp(&full[wb], done[wb]++ & 1, abort_flag, 75);
+                if (!ok) break;
+                tc::tc_fence_after();
+                const uint64_t da = kp_desc(tc::smem_u32(sA + c * KP_ACHUNK), 16, 1024), db = kp_desc(tc::smem_u32(sB + wb * KP_CONV), 8192, 1024);
+                const uint32_t fresh = (c == 0 || c * 64 == cut) ? 0u : 1u;
+                if (tc::elect_one()) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) kp_mma(tmem + run * 128, da + 2 * k, db + 128 * k, idesc, k ? 1u : fresh);   // address fields count 16-byte units
+                    tc::mma_commit(&bar[wb]);
+                }
+                __syncwarp();
+            }
+            __syncthreads();
+            __syncthreads();
+            continue;
+        }
         if (b0 > 0)
             for (int c = 0; c < nch; ++c) { kp_request_acts(A, h, b0, c, sA + c * KP_ACHUNK); tc::cp_async_commit(); }
         // the rope segment of q rides along (column block 0 only)
@@ -202,17 +232,7 @@ kvb_absorb_mma_kernel(KpArgs A) {
                 kp_convert16(sW + c * KP_WCHUNK + d * 128 + j * 16, half + tc::sw128_chunk(d, (j & 3) * 2), half + tc::sw128_chunk(d, (j & 3) * 2 + 1));
             }
             tc::fence_proxy_async();
-            __syncthreads();
-            if (warp == 0 && tc::elect_one()) {
-                tc::tc_fence_after();
-                const uint32_t a0 = tc::smem_u32(sA + c * KP_ACHUNK), w0 = tc::smem_u32(sb);
-                const int run = c * 64 >= cut ? 1 : 0;       // (a run boundary is a multiple of 64)
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    kp_mma(tmem + run * 128, kp_desc(a0 + k * 32, 16, 1024), kp_desc(w0 + k * 2048, 8192, 1024), idesc,
-                           (k == 0 && (c == 0 || c * 64 == cut)) ? 0u : 1u);
-                tc::mma_commit(&bar[wb]);
-            }
+            tc::mbar_arrive(&full[wb]);
             ++done[wb];
         }
         if (iblk == 0) {
@@ -241,7 +261,7 @@ kvb_absorb_mma_kernel(KpArgs A) {
                 for (int e = 0; e < 32; e += 2) {
                     const float v0 = fmaf(__uint_as_float(r1[e]), s1, __uint_as_float(r0[e]) * s0);
                     const float v1 = fmaf(__uint_as_float(r1[e + 1]), s1, __uint_as_float(r0[e + 1]) * s0);
-                    o[e >> 1] = (uint32_t)rv_f32_to_bf16(v0) | ((uint32_t)rv_f32_to_bf16(v1) << 16);
+                    o[e >> 1] = kp_pack(v0, v1);
                 }
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
@@ -254,7 +274,7 @@ kvb_absorb_mma_kernel(KpArgs A) {
         __syncthreads();   // TMEM and the A tiles are free for the next batch tile
     }
     tc::cp_async_wait<0>();
-    if (warp == 0) tc::tmem_dealloc<256>(tmem);
+    if (warp == 8) tc::tmem_dealloc<256>(tmem);
     if (tid == 0 && abort_word) atomicCAS(&g_kp_err, 0, abort_word);
 }
 
@@ -263,10 +283,10 @@ kvb_absorb_mma_kernel(KpArgs A) {
 // raw codes [3][128 rows][64 B] | two converted tiles [128 rows][128 B] (K-major).
 // TMEM: one 128-column accumulator per scale column (kvl / 128 <= 4 runs).
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(KP_THREADS)
+__global__ void __launch_bounds__(KP_LAUNCH)
 kvb_value_mma_kernel(KpArgs A) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ uint64_t bar[2];
+    __shared__ uint64_t bar[2], full[2];   // MMAs of a converted tile done | its conversion done
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_word;
     __shared__ float s_sc[2][4];
@@ -279,11 +299,15 @@ kvb_value_mma_kernel(KpArgs A) {
     uint8_t* sB = sW + KP_VST * KP_WCHUNK;
     const size_t row0 = (size_t)h * (A.nope + vh) + A.nope + (size_t)jblk * 128;   // 128 value rows = 2 scale rows
     const int sc_cols = kvl / 128;
-    if (tid == 0) { tc::mbar_init(&bar[0], 1); tc::mbar_init(&bar[1], 1); tc::mbar_init_fence(); abort_word = 0; }
+    if (tid == 0) {
+        for (int i = 0; i < 2; ++i) { tc::mbar_init(&bar[i], 1); tc::mbar_init(&full[i], KP_THREADS); }
+        tc::mbar_init_fence();
+        abort_word = 0;
+    }
     rv_grid_dep_trigger();
     kp_prefetch(A.kvb + row0 * kvl, (size_t)kvl, 128, kvl);
     kp_prefetch(A.x + (size_t)h * A.xs, (size_t)A.H * A.xs * 2, min(128, A.B), kvl * 2);
-    if (warp == 0) tc::tmem_alloc<512>(&tmem_slot);
+    if (warp == 8) tc::tmem_alloc<512>(&tmem_slot);
     rv_grid_dep_wait();
     auto request = [&](int b0, int c) {   // one cp.async group per call, with or without a chunk
         if (c < nch) {
@@ -297,8 +321,9 @@ kvb_value_mma_kernel(KpArgs A) {
         }
         tc::cp_async_commit();
     };
+    if (warp < 8)
 #pragma unroll 1
-    for (int c = 0; c < KP_VST; ++c) request(0, c);
+        for (int c = 0; c < KP_VST; ++c) request(0, c);
     if (tid < 2 * sc_cols) s_sc[tid / sc_cols][tid % sc_cols] = A.scale[((row0 + (tid / sc_cols) * 64) >> 7) * sc_cols + tid % sc_cols];
     tc::tc_fence_before();
     __syncthreads();
@@ -310,6 +335,24 @@ kvb_value_mma_kernel(KpArgs A) {
     bool ok = true;
     int done[2] = {0, 0};
     for (int b0 = 0; b0 < A.B && ok; b0 += 128) {
+        if (warp == 8) {
+            for (int c = 0; c < nch && ok; ++c) {
+                const int wb = c & 1;
+                ok = tc::mbar_wait_warp(&full[wb], done[wb]++ & 1, abort_flag, 76);
+                if (!ok) break;
+                tc::tc_fence_after();
+                const uint64_t da = kp_desc(tc::smem_u32(sA + (c % KP_VST) * KP_ACHUNK), 16, 1024), db = kp_desc(tc::smem_u32(sB + wb * KP_CONV), 16, 1024);
+                if (tc::elect_one()) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) kp_mma(tmem + (c >> 1) * 128, da + 2 * k, db + 2 * k, idesc, ((c & 1) | k) ? 1u : 0u);
+                    tc::mma_commit(&bar[wb]);
+                }
+                __syncwarp();
+            }
+            __syncthreads();
+            __syncthreads();
+            continue;
+        }
         if (b0 > 0)
             for (int c = 0; c < KP_VST; ++c) request(b0, c);
         for (int c = 0; c < nch && ok; ++c) {
@@ -325,15 +368,7 @@ kvb_value_mma_kernel(KpArgs A) {
                 kp_convert16(sW + (c % KP_VST) * KP_WCHUNK + r * 64 + j * 16, sb + tc::sw128_chunk(r, 2 * j), sb + tc::sw128_chunk(r, 2 * j + 1));
             }
             tc::fence_proxy_async();
-            __syncthreads();
-            if (warp == 0 && tc::elect_one()) {
-                tc::tc_fence_after();
-                const uint32_t a0 = tc::smem_u32(sA + (c % KP_VST) * KP_ACHUNK), w0 = tc::smem_u32(sb);
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    kp_mma(tmem + (c >> 1) * 128, kp_desc(a0 + k * 32, 16, 1024), kp_desc(w0 + k * 32, 16, 1024), idesc, ((c & 1) | k) ? 1u : 0u);
-                tc::mma_commit(&bar[wb]);
-            }
+            tc::mbar_arrive(&full[wb]);
             ++done[wb];
         }
         for (int wb = 0; wb < 2 && ok; ++wb)
@@ -342,24 +377,29 @@ kvb_value_mma_kernel(KpArgs A) {
         if (ok) {
 #pragma unroll
             for (int c = chalf * 2; c < chalf * 2 + 2; ++c) {
-                float acc[32];
 #pragma unroll
-                for (int e = 0; e < 32; ++e) acc[e] = 0.0f;
-                for (int run = 0; run < sc_cols; ++run) {
-                    uint32_t r[32];
-                    tc::tmem_ld32(tmem + lane_base + run * 128 + c * 32, r);
+                for (int q = 0; q < 2; ++q) {                 // sixteen columns: all runs of them in flight together
+                    uint32_t r[4][16];
+#pragma unroll
+                    for (int run = 0; run < 4; ++run)
+                        if (run < sc_cols) tc::tmem_ld16(tmem + lane_base + run * 128 + c * 32 + q * 16, r[run]);
                     tc::tmem_ld_wait();
-                    const float sc = s_sc[chalf][run];
+                    float acc[16];
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) acc[e] = fmaf(__uint_as_float(r[e]), sc, acc[e]);
+                    for (int e = 0; e < 16; ++e) acc[e] = __uint_as_float(r[0][e]) * s_sc[chalf][0];
+#pragma unroll
+                    for (int run = 1; run < 4; ++run)
+                        if (run < sc_cols) {
+                            const float sc = s_sc[chalf][run];
+#pragma unroll
+                            for (int e = 0; e < 16; ++e) acc[e] = fmaf(__uint_as_float(r[run][e]), sc, acc[e]);
+                        }
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+                        *reinterpret_cast<uint4*>(sB + kp_stage(erow, c * 4 + q * 2 + e)) =
+                            make_uint4(kp_pack(acc[8 * e], acc[8 * e + 1]), kp_pack(acc[8 * e + 2], acc[8 * e + 3]),
+                                       kp_pack(acc[8 * e + 4], acc[8 * e + 5]), kp_pack(acc[8 * e + 6], acc[8 * e + 7]));
                 }
-                uint32_t o[16];
-#pragma unroll
-                for (int e = 0; e < 32; e += 2)
-                    o[e >> 1] = (uint32_t)rv_f32_to_bf16(acc[e]) | ((uint32_t)rv_f32_to_bf16(acc[e + 1]) << 16);
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    *reinterpret_cast<uint4*>(sB + kp_stage(erow, c * 4 + e)) = make_uint4(o[4 * e], o[4 * e + 1], o[4 * e + 2], o[4 * e + 3]);
             }
         }
         tc::tc_fence_before();
@@ -368,7 +408,7 @@ kvb_value_mma_kernel(KpArgs A) {
         __syncthreads();
     }
     tc::cp_async_wait<0>();
-    if (warp == 0) tc::tmem_dealloc<512>(tmem);
+    if (warp == 8) tc::tmem_dealloc<512>(tmem);
     if (tid == 0 && abort_word) atomicCAS(&g_kp_err, 0, abort_word);
 }
 
@@ -393,7 +433,7 @@ extern "C" int rivoli_kvb_absorb_mma(const uint16_t* q, const uint8_t* kvb, cons
     const size_t smem = (size_t)(nope / 64) * (KP_ACHUNK + KP_WCHUNK) + 2 * KP_CONV;
     rv_allow_smem<kvb_absorb_mma_kernel>(4 * (KP_ACHUNK + KP_WCHUNK) + 2 * KP_CONV);
     rv_drain_error();
-    rv_launch_dependent(kvb_absorb_mma_kernel, dim3(kvl / 128, H), dim3(KP_THREADS), smem, st, a);
+    rv_launch_dependent(kvb_absorb_mma_kernel, dim3(kvl / 128, H), dim3(KP_LAUNCH), smem, st, a);
     return rv_launch_status();
 }
 
@@ -404,7 +444,7 @@ extern "C" int rivoli_kvb_value_mma(const uint16_t* clat, const uint8_t* kvb, co
     constexpr int need = KP_VST * (KP_ACHUNK + KP_WCHUNK) + 2 * KP_CONV, smem = need > 116 * 1024 ? need : 116 * 1024;
     rv_allow_smem<kvb_value_mma_kernel>(smem);
     rv_drain_error();
-    rv_launch_dependent(kvb_value_mma_kernel, dim3(vh / 128, H), dim3(KP_THREADS), (size_t)smem, st, a);
+    rv_launch_dependent(kvb_value_mma_kernel, dim3(vh / 128, H), dim3(KP_LAUNCH), (size_t)smem, st, a);
     return rv_launch_status();
 }
 
