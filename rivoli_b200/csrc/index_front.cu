@@ -132,9 +132,12 @@ front_gemm_simt_kernel(FrontArgs A) {
 // as the f32 split partial: staged in the idle stages, one bulk copy (a CTA's partial rows are contiguous).
 // Bound by what an SM takes in (192 KiB at 18 bytes a clock = 5.4 us at the 64-head model's sizes, activations being read by
 // 32 tiles) and the launch's ramp. 128 sequences: 19 us with three stages, two barriers a chunk and 16-byte stores to 32 rows
-// at a time, then 12.5 us for the epilogue below; 20.5 us together now (31.8).
+// at a time, then 12.5 us for the epilogue below; 20.6 us together after that (31.8). The MMAs have a warp of their own: one of
+// the converting warps issued them between two chunks, behind a CTA barrier, 18.4 us together for one sequence; 17.3 now, and
+// 19.4 for 128.
 // ---------------------------------------------------------------------------------------------
-constexpr int FM_THREADS = 256;
+constexpr int FM_THREADS = 256;                             // warps 0-7 request, convert and store
+constexpr int FM_LAUNCH = FM_THREADS + 32;                  // warp 8 issues the MMAs
 constexpr int FM_NMAX = 160;                                // widest tile
 constexpr int FM_NST = 6;                                   // stages of (activations 16 KiB | raw codes) in flight
 constexpr int FM_STAGE = 16384 + FM_NMAX * 64;
@@ -159,10 +162,12 @@ __device__ __forceinline__ void fm_mma(uint32_t d_tmem, uint64_t da, uint64_t db
 }
 __device__ int g_front_err;
 
-__global__ void __launch_bounds__(FM_THREADS)
+// (two CTAs' worth of registers, 96 a thread: nine warps leave one of the four register files three of them, beside which
+// three of the epilogue's fit only up to here; 128 and 150 registers cost the epilogue its early start, 19.4 -> 21 us)
+__global__ void __launch_bounds__(FM_LAUNCH, 2)
 front_gemm_mma_kernel(FrontArgs A) {
     extern __shared__ __align__(1024) uint8_t fm_smem[];
-    __shared__ uint64_t bar[2];
+    __shared__ uint64_t bar[2], full[2];   // MMAs of a converted tile done | its conversion done
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_word;
     volatile int* abort_flag = &abort_word;
@@ -174,10 +179,14 @@ front_gemm_mma_kernel(FrontArgs A) {
     const int tile = local % J.n_tiles, split = local / J.n_tiles;
     const int TN = J.tile_n, K = J.K, n0 = J.n_tiles > 1 ? TN : J.m[0].n;   // (columns of the tile from m[0])
     const int k0 = split * J.k_chunks * 64, nch = min(J.k_chunks, K / 64 - split * J.k_chunks);
-    if (tid == 0) { tc::mbar_init(&bar[0], 1); tc::mbar_init(&bar[1], 1); tc::mbar_init_fence(); abort_word = 0; }
-    if (warp == 0) tc::tmem_alloc<256>(&tmem_slot);
+    if (tid == 0) {
+        for (int i = 0; i < 2; ++i) { tc::mbar_init(&bar[i], 1); tc::mbar_init(&full[i], FM_THREADS); }
+        tc::mbar_init_fence();
+        abort_word = 0;
+    }
+    if (warp == 8) tc::tmem_alloc<256>(&tmem_slot);
     // (a prefetch into L2 may precede the wait, whoever writes)
-    for (int e = tid; e < TN * ((nch * 64 + 127) / 128); e += FM_THREADS) {
+    for (int e = tid; e < TN * ((nch * 64 + 127) / 128); e += FM_LAUNCH) {
         const int row = e % TN, line = e / TN;
         const uint8_t* w = row < n0 ? J.m[0].w + (size_t)(tile * TN + row) * K : J.m[1].w + (size_t)(row - n0) * K;
         asm volatile("prefetch.global.L2 [%0];" ::"l"(w + k0 + line * 128));
@@ -192,7 +201,7 @@ front_gemm_mma_kernel(FrontArgs A) {
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const int e = tid + i * FM_THREADS, row = e >> 2, j = e & 3;
-        lw[i] = row < TN;
+        lw[i] = row < TN && warp < 8;
         second[i] = row >= n0;
         const int r = lw[i] ? row : 0;
         pw[i] = (r < n0 ? J.m[0].w + (size_t)(tile * TN + r) * K : J.m[1].w + (size_t)(r - n0) * K) + k0 + j * 16;
@@ -206,12 +215,12 @@ front_gemm_mma_kernel(FrontArgs A) {
     uint32_t tmem = 0;
     // instruction descriptor: bf16 x bf16 -> f32, both K-major, M = 128, N = TN
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-    for (int b0 = 0; b0 < A.B && ok; b0 += 128) {
+    for (int b0 = 0; b0 < A.B; b0 += 128) {                  // (after a wait that gave up too: the barriers stay matched)
         const uint16_t* pa[4]; uint32_t da[4]; uint32_t la[4];   // 4 activation pieces a thread; rows past B are zeros
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int e = tid + i * FM_THREADS, row = e >> 3, j = e & 7;
-            la[i] = b0 + row < A.B ? 16u : 0u;
+            la[i] = b0 + row < A.B && warp < 8 ? 16u : 0u;
             pa[i] = J.x + (size_t)(la[i] ? b0 + row : 0) * K + k0 + j * 8;
             da[i] = tc::sw128_chunk(row, j);
         }
@@ -226,14 +235,33 @@ front_gemm_mma_kernel(FrontArgs A) {
             }
             tc::cp_async_commit();
         };
+        if (warp < 8)
 #pragma unroll 1
-        for (int c = 0; c < FM_NST; ++c) request(c);
+            for (int c = 0; c < FM_NST; ++c) request(c);
         float s0 = sc0[k0 >> 7], s1 = sc1[k0 >> 7];
         if (b0 == 0) {
             tc::tc_fence_before();
             __syncthreads();
             tc::tc_fence_after();
             tmem = tmem_slot;
+        }
+        if (warp == 8) {
+            for (int c = 0; c < nch && ok; ++c) {
+                const int wb = c & 1;
+                ok = tc::mbar_wait_warp(&full[wb], done[wb]++ & 1, abort_flag, 85);
+                if (!ok) break;
+                tc::tc_fence_after();
+                const uint64_t d_a = fm_desc(smem0 + (c % FM_NST) * FM_STAGE), d_b = fm_desc(smem0 + FM_BOFF + wb * FM_NMAX * 128);
+                if (tc::elect_one()) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) fm_mma(tmem, d_a + 2 * k, d_b + 2 * k, idesc, (c | k) ? 1u : 0u);   // +32 bytes = +2 in the address field
+                    tc::mma_commit(&bar[wb]);
+                }
+                __syncwarp();
+            }
+            __syncthreads();
+            if (b0 + 128 < A.B) __syncthreads();
+            continue;
         }
         for (int c = 0; c < nch && ok; ++c) {
             const int wb = c & 1;
@@ -264,14 +292,7 @@ front_gemm_mma_kernel(FrontArgs A) {
                 }
             s0 = n0s; s1 = n1s;
             tc::fence_proxy_async();
-            __syncthreads();
-            if (warp == 0 && tc::elect_one()) {
-                tc::tc_fence_after();
-                const uint64_t d_a = fm_desc(tc::smem_u32(st)), d_b = fm_desc(tc::smem_u32(sB));
-#pragma unroll
-                for (int k = 0; k < 4; ++k) fm_mma(tmem, d_a + 2 * k, d_b + 2 * k, idesc, (c | k) ? 1u : 0u);   // +32 bytes = +2 in the address field
-                tc::mma_commit(&bar[wb]);
-            }
+            tc::mbar_arrive(&full[wb]);
             ++done[wb];
         }
         tc::cp_async_wait<0>();
@@ -302,7 +323,7 @@ front_gemm_mma_kernel(FrontArgs A) {
         }
         if (b0 + 128 < A.B) __syncthreads();                 // the stages are free for the next batch tile
     }
-    if (warp == 0) tc::tmem_dealloc<256>(tmem_slot);
+    if (warp == 8) tc::tmem_dealloc<256>(tmem_slot);
     if (tid == 0 && abort_word) atomicCAS(&g_front_err, 0, abort_word);
 }
 
@@ -561,7 +582,7 @@ RIVOLI_API int rivoli_index_frontend_bf16(const IndexFrontGeom* g, const uint16_
     rv_drain_error();
     if (mma) {
         rv_allow_smem<front_gemm_mma_kernel>(FM_SMEM);
-        rv_launch_dependent(front_gemm_mma_kernel, dim3((unsigned)fa.n_cta), dim3(FM_THREADS), (size_t)FM_SMEM, st, fa);
+        rv_launch_dependent(front_gemm_mma_kernel, dim3((unsigned)fa.n_cta), dim3(FM_LAUNCH), (size_t)FM_SMEM, st, fa);
     } else {
         rv_launch_dependent(front_gemm_simt_kernel, dim3((unsigned)fa.n_cta), dim3(256), 0, st, fa);
     }
