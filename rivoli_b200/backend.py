@@ -58,6 +58,7 @@ class DsaGeom(C.Structure):
 assert C.sizeof(DsaGeom) == 48 and C.alignment(DsaGeom) == 4
 
 _lib = None
+_native = None
 
 # Argument types of the entry points, by their order in include/rivoli_kernels.h: p pointer, i int, f float, d double,
 # z size_t, q 64-bit integer. With them ctypes converts plain integers itself: a call of 25 arguments costs the host
@@ -124,6 +125,17 @@ def lib() -> C.CDLL:
     return _lib
 
 
+def _launch():
+    """The entry points that a decode token or a prompt goes through, as native functions that take tensors, streams and
+    geometries as they are (``csrc/python/launch.cpp``)."""
+    global _native
+    if _native is None:
+        lib()                       # loaded, or the reason why not
+        from . import _launch as native
+        _native = native
+    return _native
+
+
 def _ptr(x):
     """Device address of a tensor, an address as it is, None for NULL."""
     return x if x is None or type(x) is int else x.data_ptr()
@@ -141,36 +153,31 @@ def ensure_status(r: int, name: str) -> None:
 
 # --- Part 1: the reference's launchers ------------------------------------------------------------
 def launch_append_kv(latent, rope, lc8, lscale, rc, pos: int, kvl: int, ropn: int, n_blocks: int) -> None:
-    ensure_status(lib().rivoli_append_kv(_ptr(latent), _ptr(rope), _ptr(lc8), _ptr(lscale), _ptr(rc),
-                                         pos, kvl, ropn, n_blocks),
+    ensure_status((_native or _launch()).append_kv(latent, rope, lc8, lscale, rc, pos, kvl, ropn, n_blocks),
                   "append_kv")
 
 
 def launch_gather_rope(q, qrope, h: int, qh: int, nope: int, ropn: int) -> None:
-    ensure_status(lib().rivoli_gather_rope(_ptr(q), _ptr(qrope), h, qh, nope,
-                                           ropn), "gather_rope")
+    ensure_status((_native or _launch()).gather_rope(q, qrope, h, qh, nope, ropn), "gather_rope")
 
 
 def launch_index_append(k, kcache, pos: int, hd: int) -> None:
-    ensure_status(lib().rivoli_index_append(_ptr(k), _ptr(kcache), pos, hd), "index_append")
+    ensure_status((_native or _launch()).index_append(k, kcache, pos, hd), "index_append")
 
 
 def launch_index_score(q, w, kcache, heads, nt: int, nh: int, nact: int, hd: int, wscale: float,
                        dscale: float, scores) -> None:
-    ensure_status(lib().rivoli_index_score(_ptr(q), _ptr(w), _ptr(kcache), _ptr(heads), nt,
-                                           nh, nact, hd, wscale,
-                                           dscale, _ptr(scores)), "index_score")
+    ensure_status((_native or _launch()).index_score(q, w, kcache, heads, nt, nh, nact, hd, wscale, dscale, scores), "index_score")
 
 
 def launch_index_topk(scores, nt: int, k: int, rows) -> None:
-    ensure_status(lib().rivoli_index_topk(_ptr(scores), nt, k, _ptr(rows)), "index_topk")
+    ensure_status((_native or _launch()).index_topk(scores, nt, k, rows), "index_topk")
 
 
 def launch_attend(qabs, qrope, lc8, lscale, rc, rows, h: int, nr: int, kvl: int, rope: int, n_blocks: int,
                   scale: float, clat, partial) -> None:
-    ensure_status(lib().rivoli_mla_attend(_ptr(qabs), _ptr(qrope), _ptr(lc8), _ptr(lscale), _ptr(rc),
-                                          _ptr(rows), h, nr, kvl, rope,
-                                          n_blocks, scale, _ptr(clat), _ptr(partial)),
+    ensure_status((_native or _launch()).mla_attend(qabs, qrope, lc8, lscale, rc, rows, h, nr, kvl, rope, n_blocks,
+        scale, clat, partial),
                   "mla_attend")
 
 
@@ -194,10 +201,8 @@ def device_sync() -> None:
 # --- Part 2: batched / paged / bf16 -----------------------------------------------------------------
 def launch_kv_append_paged(g: DsaGeom, latent, index_key, row_seq, row_pos, n_rows: int, block_table,
                            latent_pool, latent_scale, index_pool, index_scale, status=None, stream=None) -> None:
-    ensure_status(lib().rivoli_kv_append_paged(C.byref(g), _ptr(latent), _ptr(index_key), _ptr(row_seq),
-                                               _ptr(row_pos), n_rows, _ptr(block_table),
-                                               _ptr(latent_pool), _ptr(latent_scale), _ptr(index_pool),
-                                               _ptr(index_scale), _ptr(status), _stream(stream)),
+    ensure_status((_native or _launch()).kv_append_paged(g, latent, index_key, row_seq, row_pos, n_rows, block_table,
+        latent_pool, latent_scale, index_pool, index_scale, status, stream),
                   "kv_append_paged")
 
 
@@ -232,30 +237,26 @@ def index_select_uses_mma(g: DsaGeom, score_stride: int) -> bool:
 def launch_index_select_paged(g: DsaGeom, index_q, w, index_pool, index_scale, block_table, seq_len, B: int,
                               score_stride: int, rows, n_sel, scratch, stream=None) -> None:
     """Fused indexer (q quant + scores + exact top-k); rows identical to the unfused chain."""
-    ensure_status(lib().rivoli_index_select_paged(C.byref(g), _ptr(index_q), _ptr(w), _ptr(index_pool),
-                                                  _ptr(index_scale), _ptr(block_table), _ptr(seq_len),
-                                                  B, score_stride, _ptr(rows), _ptr(n_sel),
-                                                  _ptr(scratch), _stream(stream)), "index_select_paged")
+    ensure_status((_native or _launch()).index_select_paged(g, index_q, w, index_pool, index_scale, block_table,
+        seq_len, B, score_stride, rows, n_sel, scratch, stream), "index_select_paged")
 
 
 def launch_dsa_append_attend_paged(g: DsaGeom, latent, index_key, row_pos, block_table, latent_pool, latent_scale,
                                    index_pool, index_scale, status, B: int, rows, row_stride: int, n_rows, q, out, out_m,
                                    out_lse, attend_scratch, min_rows_hint: int = 0, stream=None) -> None:
     """Append, then attend over rows another layer selected (``rivoli_dsa_append_attend_paged``)."""
-    ensure_status(lib().rivoli_dsa_append_attend_paged(
-        C.byref(g), _ptr(latent), _ptr(index_key), _ptr(row_pos), _ptr(block_table), _ptr(latent_pool),
-        _ptr(latent_scale), _ptr(index_pool), _ptr(index_scale), _ptr(status), B, _ptr(rows), row_stride, _ptr(n_rows),
-        _ptr(q), _ptr(out), _ptr(out_m), _ptr(out_lse), _ptr(attend_scratch), min_rows_hint, _stream(stream)),
+    ensure_status((_native or _launch()).dsa_append_attend_paged(g, latent, index_key, row_pos, block_table,
+        latent_pool, latent_scale, index_pool, index_scale, status, B, rows, row_stride, n_rows, q, out, out_m,
+        out_lse, attend_scratch, min_rows_hint, stream),
         "dsa_append_attend_paged")
 
 
 def launch_dsa_append_select_paged(g: DsaGeom, latent, index_key, row_pos, block_table, latent_pool, latent_scale,
                                    index_pool, index_scale, status, index_q, w, seq_len, B: int, score_stride: int,
                                    rows, n_sel, scratch, stream=None) -> None:
-    ensure_status(lib().rivoli_dsa_append_select_paged(
-        C.byref(g), _ptr(latent), _ptr(index_key), _ptr(row_pos), _ptr(block_table), _ptr(latent_pool),
-        _ptr(latent_scale), _ptr(index_pool), _ptr(index_scale), _ptr(status), _ptr(index_q), _ptr(w), _ptr(seq_len),
-        B, score_stride, _ptr(rows), _ptr(n_sel), _ptr(scratch), _stream(stream)),
+    ensure_status((_native or _launch()).dsa_append_select_paged(g, latent, index_key, row_pos, block_table,
+        latent_pool, latent_scale, index_pool, index_scale, status, index_q, w, seq_len, B, score_stride, rows, n_sel,
+        scratch, stream),
         "dsa_append_select_paged")
 
 
@@ -264,11 +265,9 @@ def launch_dsa_decode_step_paged(g: DsaGeom, latent, index_key, row_pos, block_t
                                  rows, n_sel, select_scratch, q, out, out_m, out_lse, attend_scratch,
                                  min_rows_hint: int = 0, stream=None) -> None:
     """One decode layer-step in one call: append, select, attend (``rivoli_dsa_decode_step_paged``)."""
-    ensure_status(lib().rivoli_dsa_decode_step_paged(
-        C.byref(g), _ptr(latent), _ptr(index_key), _ptr(row_pos), _ptr(block_table), _ptr(latent_pool),
-        _ptr(latent_scale), _ptr(index_pool), _ptr(index_scale), _ptr(status), _ptr(index_q), _ptr(w), _ptr(seq_len),
-        B, score_stride, _ptr(rows), _ptr(n_sel), _ptr(select_scratch), _ptr(q), _ptr(out),
-        _ptr(out_m), _ptr(out_lse), _ptr(attend_scratch), min_rows_hint, _stream(stream)),
+    ensure_status((_native or _launch()).dsa_decode_step_paged(g, latent, index_key, row_pos, block_table,
+        latent_pool, latent_scale, index_pool, index_scale, status, index_q, w, seq_len, B, score_stride, rows, n_sel,
+        select_scratch, q, out, out_m, out_lse, attend_scratch, min_rows_hint, stream),
         "dsa_decode_step_paged")
 
 
@@ -526,30 +525,24 @@ class PagePool:
 
 def launch_mla_absorb(q, kvb, kvb_scale, H: int, qh: int, nope: int, vh: int, kvl: int, block: int, nrow: int,
                       qabs) -> None:
-    ensure_status(lib().rivoli_mla_absorb_fp8(_ptr(q), _ptr(kvb), _ptr(kvb_scale), H, qh,
-                                              nope, vh, kvl, block, nrow,
-                                              _ptr(qabs)), "mla_absorb_fp8")
+    ensure_status((_native or _launch()).mla_absorb_fp8(q, kvb, kvb_scale, H, qh, nope, vh, kvl, block, nrow, qabs), "mla_absorb_fp8")
 
 
 def launch_mla_value(clat, kvb, kvb_scale, H: int, nope: int, vh: int, kvl: int, block: int, nrow: int, ctx) -> None:
-    ensure_status(lib().rivoli_mla_value_fp8(_ptr(clat), _ptr(kvb), _ptr(kvb_scale), H, nope,
-                                             vh, kvl, block, nrow, _ptr(ctx)),
+    ensure_status((_native or _launch()).mla_value_fp8(clat, kvb, kvb_scale, H, nope, vh, kvl, block, nrow, ctx),
                   "mla_value_fp8")
 
 
 def launch_mla_absorb_batched_bf16(q, kvb, kvb_scale, H: int, qh: int, nope: int, vh: int, kvl: int, rope: int,
                                    block: int, B: int, q_abs, force_simt: bool = False, stream=None) -> None:
-    ensure_status(lib().rivoli_mla_absorb_batched_bf16(_ptr(q), _ptr(kvb), _ptr(kvb_scale), H, qh,
-                                                       nope, vh, kvl, rope,
-                                                       block, B, _ptr(q_abs), int(force_simt),
-                                                       _stream(stream)), "mla_absorb_batched_bf16")
+    ensure_status((_native or _launch()).mla_absorb_batched_bf16(q, kvb, kvb_scale, H, qh, nope, vh, kvl, rope, block,
+        B, q_abs, force_simt, stream), "mla_absorb_batched_bf16")
 
 
 def launch_mla_value_batched_bf16(clat, kvb, kvb_scale, H: int, nope: int, vh: int, kvl: int, block: int, B: int, ctx,
                                   force_simt: bool = False, stream=None) -> None:
-    ensure_status(lib().rivoli_mla_value_batched_bf16(_ptr(clat), _ptr(kvb), _ptr(kvb_scale), H, nope,
-                                                      vh, kvl, block, B, _ptr(ctx),
-                                                      int(force_simt), _stream(stream)),
+    ensure_status((_native or _launch()).mla_value_batched_bf16(clat, kvb, kvb_scale, H, nope, vh, kvl, block, B, ctx,
+        force_simt, stream),
                   "mla_value_batched_bf16")
 
 
@@ -564,17 +557,15 @@ class IndexFrontGeom(C.Structure):
 
 
 def launch_gemv_fp8(x, packed, scale, o_dim: int, i_dim: int, block: int, nrow: int, y) -> None:
-    ensure_status(lib().rivoli_gemv_fp8(_ptr(x), _ptr(packed), _ptr(scale), o_dim, i_dim, block,
-                                        nrow, _ptr(y)), "gemv_fp8")
+    ensure_status((_native or _launch()).gemv_fp8(x, packed, scale, o_dim, i_dim, block, nrow, y), "gemv_fp8")
 
 
 def launch_layernorm(x, w, b, n: int, eps: float, y) -> None:
-    ensure_status(lib().rivoli_layernorm(_ptr(x), _ptr(w), _ptr(b), n, eps, _ptr(y)), "layernorm")
+    ensure_status((_native or _launch()).layernorm(x, w, b, n, eps, y), "layernorm")
 
 
 def launch_rope_interleave(base, count: int, stride: int, seg: int, pos: int, theta: float) -> None:
-    ensure_status(lib().rivoli_rope_interleave(_ptr(base), count, stride, seg, pos,
-                                               theta), "rope_interleave")
+    ensure_status((_native or _launch()).rope_interleave(base, count, stride, seg, pos, theta), "rope_interleave")
 
 
 def index_frontend_scratch_bytes(g: IndexFrontGeom, B: int) -> int:
@@ -584,10 +575,8 @@ def index_frontend_scratch_bytes(g: IndexFrontGeom, B: int) -> int:
 def launch_index_frontend_bf16(g: IndexFrontGeom, x, q_resid, pos, B: int, wk, wk_scale, knorm_w, knorm_b, wq_b, wq_b_scale,
                                wproj, wproj_scale, index_key, index_q, index_w, scratch, force_simt: bool = False,
                                stream=None) -> None:
-    ensure_status(lib().rivoli_index_frontend_bf16(
-        C.byref(g), _ptr(x), _ptr(q_resid), _ptr(pos), B, _ptr(wk), _ptr(wk_scale), _ptr(knorm_w), _ptr(knorm_b),
-        _ptr(wq_b), _ptr(wq_b_scale), _ptr(wproj), _ptr(wproj_scale), _ptr(index_key), _ptr(index_q), _ptr(index_w),
-        _ptr(scratch), int(force_simt), _stream(stream)), "index_frontend_bf16")
+    ensure_status((_native or _launch()).index_frontend_bf16(g, x, q_resid, pos, B, wk, wk_scale, knorm_w, knorm_b,
+        wq_b, wq_b_scale, wproj, wproj_scale, index_key, index_q, index_w, scratch, force_simt, stream), "index_frontend_bf16")
 
 
 def index_frontend_status(stream=None) -> None:
@@ -610,7 +599,7 @@ class V4Geom(C.Structure):
 
 def launch_act_quant_f4_rotated(x, rows: int, d: int, stream=None) -> None:
     """crates/backend/src/hip.rs launcher of ``rivoli_act_quant_f4_rotated`` (in place on f32 rows)."""
-    ensure_status(lib().rivoli_act_quant_f4_rotated(_ptr(x), rows, d, _stream(stream)),
+    ensure_status((_native or _launch()).act_quant_f4_rotated(x, rows, d, stream),
                   "act_quant_f4_rotated")
 
 
@@ -632,9 +621,8 @@ def v4_select_scratch_bytes(g: V4Geom, n_seqs: int) -> int:
 
 def launch_v4_select_blocks_bf16(g: V4Geom, n_seqs: int, pos, index_q, index_w, index_kv, sel, scratch,
                                  force_fold: bool = False, packed=None, packed_exp=None, stream=None) -> None:
-    ensure_status(lib().rivoli_v4_select_blocks_bf16(C.byref(g), n_seqs, _ptr(pos), _ptr(index_q), _ptr(index_w),
-                                                     _ptr(index_kv), _ptr(packed), _ptr(packed_exp), _ptr(sel),
-                                                     _ptr(scratch), int(force_fold), _stream(stream)),
+    ensure_status((_native or _launch()).v4_select_blocks_bf16(g, n_seqs, pos, index_q, index_w, index_kv, packed,
+        packed_exp, sel, scratch, force_fold, stream),
                   "v4_select_blocks_bf16")
 
 
@@ -647,9 +635,8 @@ def launch_v4_index_pack_bf16(g: V4Geom, n_seqs: int, row_begin, row_end, max_ro
 
 def launch_v4_sparse_attend_bf16(g: V4Geom, n_seqs: int, q, kv_cache, sink, sel, cols: int, out,
                                  force_simt: bool = False, stream=None) -> None:
-    ensure_status(lib().rivoli_v4_sparse_attend_bf16(C.byref(g), n_seqs, _ptr(q), _ptr(kv_cache), _ptr(sink),
-                                                     _ptr(sel), cols, _ptr(out), int(force_simt),
-                                                     _stream(stream)), "v4_sparse_attend_bf16")
+    ensure_status((_native or _launch()).v4_sparse_attend_bf16(g, n_seqs, q, kv_cache, sink, sel, cols, out,
+        force_simt, stream), "v4_sparse_attend_bf16")
 
 
 def v4_sparse_attend_status(stream=None) -> None:
@@ -677,20 +664,16 @@ class CompFinish(C.Structure):
 
 
 def launch_act_quant_f8_prefix(src, dst, rows: int, row_stride: int, n: int, block: int, stream=None) -> None:
-    ensure_status(lib().rivoli_act_quant_f8_prefix(_ptr(src), _ptr(dst), rows, row_stride, n,
-                                                   block, _stream(stream)), "act_quant_f8_prefix")
+    ensure_status((_native or _launch()).act_quant_f8_prefix(src, dst, rows, row_stride, n, block, stream), "act_quant_f8_prefix")
 
 
 def launch_kv_compress_deposit(kv, score, ape, kv_state, score_state, p: CompGeom, s: int, slot0: int, stream=None) -> None:
-    ensure_status(lib().rivoli_kv_compress_deposit(_ptr(kv), _ptr(score), _ptr(ape), _ptr(kv_state), _ptr(score_state),
-                                                   C.byref(p) if p is not None else None, s, slot0,
-                                                   _stream(stream)), "kv_compress_deposit")
+    ensure_status((_native or _launch()).kv_compress_deposit(kv, score, ape, kv_state, score_state, p, s, slot0,
+        stream), "kv_compress_deposit")
 
 
 def launch_kv_compress_prefill(kv, score, ape, norm, freqs, out, p: CompGeom, nblk: int, stream=None) -> None:
-    f = CompFinish(_ptr(norm), _ptr(freqs), _ptr(out))
-    ensure_status(lib().rivoli_kv_compress_prefill(_ptr(kv), _ptr(score), _ptr(ape), C.byref(f), C.byref(p), nblk,
-                                                   _stream(stream)), "kv_compress_prefill")
+    ensure_status((_native or _launch()).kv_compress_prefill(kv, score, ape, (norm, freqs, out), p, nblk, stream), "kv_compress_prefill")
 
 
 def launch_kv_compress_decode(kv_state, score_state, norm, freqs, out, p: CompGeom, start_pos: int, stream=None) -> None:
@@ -699,27 +682,13 @@ def launch_kv_compress_decode(kv_state, score_state, norm, freqs, out, p: CompGe
                                                   start_pos, _stream(stream)), "kv_compress_decode")
 
 
-class CompStep(C.Structure):
-    """``CompStep`` of include/rivoli_kernels.h: one compressor's arguments of a decode step."""
-    _fields_ = [(n, C.c_void_p) for n in (
-        "kv_proj", "score_proj", "ape", "kv_state", "score_state", "norm", "freqs", "cache", "prequant", "packed",
-        "packed_exp")] + [(n, C.c_int32) for n in ("rotate", "cache_rows", "cache_row0")]
-
-    @classmethod
-    def make(cls, kv_proj, score_proj, ape, kv_state, score_state, norm, freqs, rotate, cache, cache_rows, cache_row0,
-             packed=None, packed_exp=None) -> "CompStep":
-        return cls(_ptr(kv_proj), _ptr(score_proj), _ptr(ape), _ptr(kv_state), _ptr(score_state), _ptr(norm), _ptr(freqs),
-                   _ptr(cache), None, _ptr(packed), _ptr(packed_exp), int(rotate), cache_rows, cache_row0)
-
-
-def launch_v4_token_step_bf16(g: V4Geom, n_seqs: int, pos, kv_entry, attn: CompGeom, attn_step: CompStep,
-                              index: CompGeom, index_step: CompStep, q, index_q, index_w, sink, sel, scratch, out,
+def launch_v4_token_step_bf16(g: V4Geom, n_seqs: int, pos, kv_entry, attn: CompGeom, attn_step: tuple,
+                              index: CompGeom, index_step: tuple, q, index_q, index_w, sink, sel, scratch, out,
                               stream=None) -> None:
-    """One decode token through a layer (``rivoli_v4_token_step_bf16``)."""
-    ensure_status(lib().rivoli_v4_token_step_bf16(
-        C.byref(g), n_seqs, _ptr(pos), _ptr(kv_entry), C.byref(attn), C.byref(attn_step), C.byref(index),
-        C.byref(index_step), _ptr(q), _ptr(index_q), _ptr(index_w), _ptr(sink), _ptr(sel), _ptr(scratch), _ptr(out),
-        _stream(stream)), "v4_token_step_bf16")
+    """One decode token through a layer (``rivoli_v4_token_step_bf16``); ``attn_step`` and ``index_step`` are the fields of
+    ``CompStep`` (include/rivoli_kernels.h) in order."""
+    ensure_status((_native or _launch()).v4_token_step_bf16(g, n_seqs, pos, kv_entry, attn, attn_step, index,
+        index_step, q, index_q, index_w, sink, sel, scratch, out, stream), "v4_token_step_bf16")
 
 
 def launch_v4_compress_step_bf16(p: CompGeom, n_seqs: int, pos, kv_proj, score_proj, ape, kv_state, score_state, norm,

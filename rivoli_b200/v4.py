@@ -79,10 +79,10 @@ class V4Compressor:
         self.score_state = torch.full((n_seqs, p.ents, p.cd), float("-inf"), dtype=torch.float32, device=dev)
         self.ape, self.norm, self.freqs = ape, norm, freqs
 
-    def step_args(self, kv_proj, score_proj, cache, cache_rows: int, cache_row0: int, packed=None, packed_exp=None) -> be.CompStep:
+    def step_args(self, kv_proj, score_proj, cache, cache_rows: int, cache_row0: int, packed=None, packed_exp=None) -> tuple:
         """This compressor's part of ``launch_v4_token_step_bf16``."""
-        return be.CompStep.make(kv_proj, score_proj, self.ape, self.kv_state, self.score_state, self.norm, self.freqs,
-                                self.rotate, cache, cache_rows, cache_row0, packed, packed_exp)
+        return (kv_proj, score_proj, self.ape, self.kv_state, self.score_state, self.norm, self.freqs, cache, None, packed,
+                packed_exp, self.rotate, cache_rows, cache_row0)
 
     def step(self, pos, kv_proj, score_proj, cache, cache_rows: int, cache_row0: int, packed=None, packed_exp=None,
              prequant=None, stream=None):
