@@ -186,19 +186,24 @@ __global__ void __launch_bounds__(CP_THREADS) cp_prefill_kernel(const float* __r
 // The same for the overlapping ratio-4 compressor with d = 128, 256 or 512 (what both compressors of a layer are): eight
 // entries per block and feature, every projected value used exactly once, so HBM is the bound (8.8 bytes a value). A
 // thread owns two features of one block, d / 2 threads a block: its 8 scores and 8 values are all requested before the
-// first is used (128 bytes per thread; two features and not four, so that five CTAs share an SM: the exponentials of one
-// cover the loads of another), the maximum, the exponentials (one per entry instead of two), the weighted sum and its one
-// division run from registers in the entry order of the kernel above, and the row never leaves them: only the norm's
-// partial sums meet in shared memory, where the positional bias sits too, for the CTA's walk over the grid's blocks.
-// 4,095 blocks of d 512: 124 us with three passes over global memory, 27.7 us now (5.2 TB/s); d 128: 38 -> 7.8.
-constexpr int CP4_THREADS = 256, CP4_CTAS = 5;
+// first is used (128 bytes per thread; two features and not four, so that several CTAs share an SM: the exponentials of one
+// cover the loads of another); the maximum, the exponentials (one per entry instead of two) and the weighted sum run from
+// registers. Values and their order are those of the kernel above and of the decode arms, the quotients and the norm's partial
+// sums included (a row meets in shared memory in the order of a 256-thread CTA): a block has the same bits whether it was
+// pooled from a prompt or token by token. (The sum divided once and the norm summed as the features lie would take 27.7 us
+// instead of 31 at 4,095 blocks of d 512, and land on other codes now and then.) The positional bias sits in shared memory for
+// the CTA's walk over the grid's blocks. Three passes over global memory took 124 us; four CTAs per SM are 2.4 us faster than
+// five, at whose registers the quotients spill, and 11 faster than three.
+constexpr int CP4_THREADS = 256, CP4_CTAS = 4;
 template <int D>
 __global__ void __launch_bounds__(CP4_THREADS, CP4_CTAS) cp_prefill4_kernel(const float* __restrict__ kv,
                                                                             const float* __restrict__ score,
                                                                             const float* __restrict__ ape, CompFinish f,
                                                                             CompGeom p, int nblk) {
     constexpr int WPB = D / 64, GROUPS = CP4_THREADS / 32 / WPB, CD = 2 * D;   // warps per block, blocks per CTA and step
-    __shared__ float red[2][CP4_THREADS / 32];
+    constexpr int NV = D == 512 ? 1 : 2;                // the norm's partial sums a warp takes
+    __shared__ float s_red[8 * GROUPS];
+    __shared__ __align__(16) float s_row[GROUPS * D];
     __shared__ __align__(16) float bias[8][D];          // row j: the positional bias entry j adds to its scores
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, group = warp / WPB;
     const int e = ((warp - group * WPB) * 32 + lane) * 2;
@@ -210,9 +215,9 @@ __global__ void __launch_bounds__(CP4_THREADS, CP4_CTAS) cp_prefill4_kernel(cons
     }
     const float2 gain = *reinterpret_cast<const float2*>(f.norm + e);
     __syncthreads();
-    int it = 0;
-    // whole groups of the CTA step together (the norm's barrier); a group past the end works on the last block and stores nothing
-    for (int b0 = blockIdx.x * GROUPS; b0 < nblk; b0 += gridDim.x * GROUPS, ++it) {
+    float* my = s_row + group * D;
+    // whole groups of the CTA step together (the norm's barriers); a group past the end works on the last block and stores nothing
+    for (int b0 = blockIdx.x * GROUPS; b0 < nblk; b0 += gridDim.x * GROUPS) {
         const bool live = b0 + group < nblk;
         const int b = live ? b0 + group : nblk - 1;
         float2 sc[8], kx[8];
@@ -242,17 +247,25 @@ __global__ void __launch_bounds__(CP4_THREADS, CP4_CTAS) cp_prefill4_kernel(cons
 #pragma unroll
                 for (int j = 0; j < 8; ++j) if (j >= j0) { x[j] = expf(x[j] - mx); sum += x[j]; }
 #pragma unroll
-                for (int j = 0; j < 8; ++j) if (j >= j0) o += (c ? kx[j].y : kx[j].x) * x[j];
-                o /= sum;
+                for (int j = 0; j < 8; ++j) if (j >= j0) o += (c ? kx[j].y : kx[j].x) * (x[j] / sum);
             }
             row[c] = v4_rbf16(o);
         }
-        float part = rv_warp_sum(row[0] * row[0] + row[1] * row[1]);
-        if (lane == 0) red[it & 1][warp] = part;
-        __syncthreads();                               // (two buffers: a warp is at most one step ahead)
-        part = 0.0f;
+        *reinterpret_cast<float2*>(my + e) = make_float2(row[0], row[1]);
+        __syncthreads();
+        const int w = warp - group * WPB;
 #pragma unroll
-        for (int w = 0; w < WPB; ++w) part += red[it & 1][group * WPB + w];
+        for (int v = 0; v < NV; ++v) {
+            const int t = (v * WPB + w) * 32 + lane;
+            float part = my[t] * my[t];
+            if (D == 512) part += my[t + 256] * my[t + 256];
+            part = rv_warp_sum(part);
+            if (lane == 0) s_red[group * 8 + v * WPB + w] = part;
+        }
+        __syncthreads();                               // (the row is written again behind this, the sums behind the next)
+        float part = 0.0f;
+#pragma unroll
+        for (int i = 0; i < NV * WPB; ++i) part += s_red[group * 8 + i];
         const float rs = 1.0f / sqrtf(part / (float)D + p.eps);
         row[0] = v4_rbf16(gain.x * (row[0] * rs));
         row[1] = v4_rbf16(gain.y * (row[1] * rs));

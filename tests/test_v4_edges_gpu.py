@@ -174,3 +174,37 @@ def test_token_step_equals_its_operators(b, d, idim, off):
     for t, (a, w) in enumerate(zip(*runs)):
         for i, (x, y) in enumerate(zip(a, w)):
             assert torch.equal(x, y), (t, i)
+
+
+@pytest.mark.parametrize("d,nblk,rd", [(512, 1, 64), (512, 37, 64), (256, 70, 64), (128, 301, 64), (192, 9, 64)])
+def test_prompt_blocks_are_the_decode_blocks(d, nblk, rd):
+    """A block pooled from a prompt and the same block pooled token by token go through the same operations in the same order:
+    every bit is the same. The values of an entry's two halves cancel, so that an order of its own would show in the result."""
+    be, rng = _be(), np.random.default_rng(d + nblk)
+    p = be.CompGeom.make(ratio=4, d=d, rd=rd)
+    norm, freqs, ape = (dev(a) for a in _comp_fixture(rng, p, nblk * 4))
+    ape *= 0.01
+    kv = dev(rng.standard_normal((nblk * 4, 2, d)).astype(np.float32))
+    kv[:, 0] += 300.0
+    kv[:, 1] -= 300.0
+    kv, sc = kv.reshape(nblk * 4, 2 * d).contiguous(), dev((0.01 * rng.standard_normal((nblk * 4, 2 * d))).astype(np.float32))
+    want = torch.empty((nblk, d), device="cuda")
+    be.launch_kv_compress_prefill(kv, sc, ape, norm, freqs, want, p, nblk)
+    # every block is a sequence of its own: the block before it in the overlap half of its state, then its four tokens
+    kv_state = torch.zeros((nblk, p.ents, p.cd), device="cuda")
+    score_state = torch.full((nblk, p.ents, p.cd), float("-inf"), device="cuda")
+    kb, sb = kv.view(nblk, 4, p.cd), sc.view(nblk, 4, p.cd)
+    kv_state[1:, :4], score_state[1:, :4] = kb[:-1], (sb + ape)[:-1]
+    one_kv, one_score = kv_state[-1].clone(), score_state[-1].clone()
+    cache = torch.zeros((nblk, nblk, d), dtype=torch.uint16, device="cuda")
+    pre = torch.empty((nblk, d), device="cuda")
+    for t in range(4):
+        pos = torch.arange(nblk, device="cuda", dtype=torch.int32) * 4 + t
+        be.launch_v4_compress_step_bf16(p, nblk, pos, kb[:, t].contiguous(), sb[:, t].contiguous(), ape, kv_state, score_state, norm,
+                                        freqs, False, cache, nblk, 0, pre)
+    assert np.array_equal(bits(pre.cpu().numpy()), bits(want.cpu().numpy()))
+    # and the operator of one sequence, which pools a whole state
+    one_kv[4:], one_score[4:] = kb[-1], sb[-1] + ape
+    one = torch.empty(d, device="cuda")
+    be.launch_kv_compress_decode(one_kv, one_score, norm, freqs, one, p, nblk * 4 - 1)
+    assert np.array_equal(bits(one.cpu().numpy()), bits(want[-1].cpu().numpy()))
