@@ -39,7 +39,8 @@ __device__ __forceinline__ float v4_round_scale(float amax) {
 // the operand pairs (j, j + h) stage by stage exactly as the host loop does - in a thread while h < E, between lanes
 // (shuffle) beyond - and which thread evaluates a pair does not change the value. A block of 32 is 32 / E lanes. The scale
 // is a power of two, so the quotient is the exact product with its reciprocal (a normal number: the scale lies between
-// 2^-126 and 2^125). 4,095 rows of 128: 10.3 us with a CTA per row and the row in shared memory, 3.8 us now.
+// 2^-126 and 2^125; an infinite row has an infinite scale and the reciprocal 0, with which an infinite value gives NaN and a
+// finite one 0, both NaN once multiplied by the scale, as with the division). 4,095 rows of 128: 10.3 us with a CTA per row and the row in shared memory, 3.8 us now.
 template <int E>
 __device__ __forceinline__ void v4_spread_row(float (&v)[E], int lane) {
     constexpr int D = E * 32;
@@ -66,7 +67,7 @@ __device__ __forceinline__ void v4_spread_row(float (&v)[E], int lane) {
 #pragma unroll
     for (int o = 1; o < 32 / E; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));   // exact under any association
     const float s = v4_round_scale(fmaxf(amax, __fmul_rn(V4_FP4_MAX, __uint_as_float(1u << 23))));
-    const float inv = __uint_as_float((254u << 23) - __float_as_uint(s));
+    const float inv = isinf(s) ? 0.0f : __uint_as_float((254u << 23) - __float_as_uint(s));
 #pragma unroll
     for (int j = 0; j < E; ++j) {
         float q = __fmul_rn(v[j], inv);

@@ -52,10 +52,12 @@ __device__ __forceinline__ void cp_act_quant_block(const float* seg, float* out,
 }
 
 // The scale of a block (a power of two) and its reciprocal (2^-e is a normal number: e >= -22), by which a quotient is exact.
+// An infinite block has an infinite scale (e = 128) and the reciprocal 0, which gives what the division by infinity does: NaN
+// for an infinite value, 0 for any other, and NaN for both once multiplied by the scale.
 __device__ __forceinline__ float cp_f8_scale(float amax, float& inv) {
     const uint32_t bits = __float_as_uint(__fmul_rn(amax, __fdiv_rn(1.0f, CP_FP8_MAX)));
     const int e = (int)((bits >> 23) & 0xffu) - 127 + ((bits & 0x7fffffu) ? 1 : 0);
-    inv = __uint_as_float((uint32_t)(127 - e) << 23);
+    inv = e == 128 ? 0.0f : __uint_as_float((uint32_t)(127 - e) << 23);
     return __uint_as_float((uint32_t)(e + 127) << 23);
 }
 __device__ __forceinline__ float cp_f8_roundtrip(float x, float s, float inv) {

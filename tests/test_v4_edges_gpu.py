@@ -208,3 +208,22 @@ def test_prompt_blocks_are_the_decode_blocks(d, nblk, rd):
     one = torch.empty(d, device="cuda")
     be.launch_kv_compress_decode(one_kv, one_score, norm, freqs, one, p, nblk * 4 - 1)
     assert np.array_equal(bits(one.cpu().numpy()), bits(want[-1].cpu().numpy()))
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 3.4e38])
+def test_quantisers_of_rows_that_are_not_finite(value):
+    """A block whose largest magnitude is infinite has an infinite scale: nothing of it survives, and no finite number appears."""
+    be, rng = _be(), np.random.default_rng(3)
+    x = rng.standard_normal((5, 512)).astype(np.float32)
+    x[1, 70], x[2, 64:128], x[3, 0], x[3, 447] = value, value, 0.0, value
+    _, want = orc.act_quant_f8_prefix(x.reshape(-1), 5, 512, 448, 64)
+    t = dev(x.reshape(-1).copy())
+    be.launch_act_quant_f8_prefix(t, t, 5, 512, 448, 64)
+    assert np.array_equal(t.cpu().numpy(), np.asarray(want).reshape(-1), equal_nan=True)
+    for d in (32, 64, 128, 256):
+        y = rng.standard_normal((4, d)).astype(np.float32)
+        y[1, 5], y[2, 0], y[2, d - 1] = value, value, value
+        _, want = orc.v4_spread(y, d)
+        t = dev(y.copy())
+        be.launch_act_quant_f4_rotated(t, 4, d)
+        assert np.array_equal(t.cpu().numpy(), want.reshape(4, d), equal_nan=True), d
