@@ -359,7 +359,8 @@ attend_simt_kernel(AttSlab sp, AttPaged pp, int H, int rope, float scale, int nr
             if (pp.out_lse) pp.out_lse[(size_t)b * H + h] = lg > 0.0f ? mg + logf(lg) : -INFINITY;
         }
     };
-    // the CTA's maximum and sum per head, and the weight of each warp's outputs at that maximum
+    // the CTA's maximum and sum per head, and the weight of each warp's outputs at that maximum. A sum of exactly 0 says that
+    // there were no rows (the weight of the maximum is 1); one that is NaN goes on to the denominator and makes the head NaN.
     if (tid < AT_WARPS * HG) {
         const int j = tid % HG, w = tid / HG;
         float mx = -INFINITY, sum = 0.0f;
@@ -367,8 +368,8 @@ attend_simt_kernel(AttSlab sp, AttPaged pp, int H, int rope, float scale, int nr
         for (int v = 0; v < AT_WARPS; ++v) mx = fmaxf(mx, s_m[v][j]);
 #pragma unroll
         for (int v = 0; v < AT_WARPS; ++v)
-            if (s_l[v][j] > 0.0f) sum += s_l[v][j] * expf(s_m[v][j] - mx);
-        s_w[w][j] = s_l[w][j] > 0.0f ? expf(s_m[w][j] - mx) : 0.0f;
+            if (s_l[v][j] != 0.0f) sum += s_l[v][j] * expf(s_m[v][j] - mx);
+        s_w[w][j] = s_l[w][j] != 0.0f ? expf(s_m[w][j] - mx) : 0.0f;
         if (w == 0) { c_m[j] = mx; c_l[j] = sum; }
     }
     __syncthreads();
@@ -376,13 +377,13 @@ attend_simt_kernel(AttSlab sp, AttPaged pp, int H, int rope, float scale, int nr
         float v = 0.0f;
 #pragma unroll
         for (int w = 0; w < AT_WARPS; ++w)
-            if (s_w[w][j] > 0.0f) v = fmaf(at_smem[(size_t)w * WARP_FLOATS + j * KVL + c], s_w[w][j], v);
+            if (s_w[w][j] != 0.0f) v = fmaf(at_smem[(size_t)w * WARP_FLOATS + j * KVL + c], s_w[w][j], v);
         return v;
     };
     if (n_cta == 1) {
         for (int e = tid; e < HG * KVL; e += AT_THREADS) {
             const int j = e / KVL, c = e - j * KVL;
-            if (head0 + j < H) store(head0 + j, c, c_l[j] > 0.0f ? cta_sum(j, c) * (1.0f / c_l[j]) : 0.0f);
+            if (head0 + j < H) store(head0 + j, c, c_l[j] != 0.0f ? cta_sum(j, c) * (1.0f / c_l[j]) : 0.0f);
         }
         if (tid < HG && head0 + tid < H) stats(head0 + tid, c_m[tid], c_l[tid]);
         return;
@@ -404,11 +405,11 @@ attend_simt_kernel(AttSlab sp, AttPaged pp, int H, int rope, float scale, int nr
         float mg = mq;
 #pragma unroll
         for (int o = HG; o < HG * AT_MAX_CLUSTER; o <<= 1) mg = fmaxf(mg, __shfl_xor_sync(0xffffffffu, mg, o));
-        const float wq = lq > 0.0f ? expf(mq - mg) : 0.0f;
+        const float wq = lq != 0.0f ? expf(mq - mg) : 0.0f;
         float lg = lq * wq;
 #pragma unroll
         for (int o = HG; o < HG * AT_MAX_CLUSTER; o <<= 1) lg += __shfl_xor_sync(0xffffffffu, lg, o);
-        if (q < AT_MAX_CLUSTER) s_w[q][j] = wq > 0.0f ? wq / lg : 0.0f;
+        if (q < AT_MAX_CLUSTER) s_w[q][j] = lq != 0.0f ? wq / lg : 0.0f;
         if (q == 0 && rank == 0 && head0 + j < H) stats(head0 + j, mg, lg);
     }
     __syncthreads();
@@ -420,7 +421,7 @@ attend_simt_kernel(AttSlab sp, AttPaged pp, int H, int rope, float scale, int nr
         for (int q = 0; q < AT_MAX_CLUSTER; ++q) o[q] = q < n_cta ? cluster.map_shared_rank(at_smem, q)[e] : 0.0f;   // all in flight
 #pragma unroll
         for (int q = 0; q < AT_MAX_CLUSTER; ++q)
-            if (q < n_cta && s_w[q][j] > 0.0f) v = fmaf(o[q], s_w[q][j], v);   // (a CTA without rows left its array unwritten)
+            if (q < n_cta && s_w[q][j] != 0.0f) v = fmaf(o[q], s_w[q][j], v);   // (a CTA without rows left its array unwritten)
         if (head0 + j < H) store(head0 + j, e - j * KVL, v);
     }
     cluster.sync();                                               // nobody reads this CTA's memory any more

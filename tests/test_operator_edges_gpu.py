@@ -113,3 +113,56 @@ def test_topk_lengths_ties_and_infinities(n, kind):
         got = rows.cpu().numpy().view(np.uint32)
         np.testing.assert_array_equal(got[:k], orc.index_topk(s, k))
         assert (got[k:] == 0xFFFFFFFF).all()
+
+
+@pytest.mark.parametrize("nr", [1, 2, 13, 96, 97, 1537])
+@pytest.mark.parametrize("where", ["q", "row", "score"])
+def test_attend_is_loud_about_values_that_are_not_numbers(nr, where):
+    """A NaN (or a score that overflows) makes the whole output of the heads that see it NaN, and of no other head."""
+    be, r, H, kvl, rope, nb = _be(), orc.Lcg(nr), 6, 512, 64, 4
+    qabs, qrope = r.draws(H * kvl), r.draws(H * rope)
+    lc8 = orc.f32_to_e4m3(r.draws(nr * kvl))
+    lscale = (np.abs(r.draws(nr * nb)) + np.float32(0.01)).astype(np.float32)
+    rc = orc.f32_to_bf16(r.draws(nr * rope))
+    if where == "q":
+        qabs[3 * kvl + 7] = np.nan
+        bad = [3]
+    elif where == "row":
+        lc8[(nr // 2) * kvl + 100] = 0x7F
+        bad = list(range(H))
+    else:
+        qabs[3 * kvl: 4 * kvl] = 0.0
+        qrope[3 * rope: 4 * rope] = 3e38
+        rc[(nr // 2) * rope: (nr // 2 + 1) * rope] = orc.f32_to_bf16(np.full(rope, 3e38, np.float32))
+        qrope[:3 * rope] = 0.0
+        qrope[4 * rope:] = 0.0
+        bad = [3]
+    out = torch.full((H * kvl,), 7.0, device="cuda")
+    be.launch_attend(dev(qabs), dev(qrope), dev(lc8), dev(lscale), dev(rc), None, H, nr, kvl, rope, nb, 0.25, out, None)
+    be.device_sync()
+    nan = np.isnan(out.cpu().numpy().reshape(H, kvl))
+    for h in range(H):
+        assert nan[h].all() if h in bad else not nan[h].any(), h
+
+
+@pytest.mark.parametrize("heads,nr", [(16, 1), (16, 97), (64, 40)])
+def test_paged_attention_is_loud_about_values_that_are_not_numbers(heads, nr):
+    """The same of the paged form, its own geometry and the short sequences of the 64-head one."""
+    be = _be()
+    g = be.DsaGeom.make(n_heads=heads, page_tokens=16, max_pages_per_seq=8, n_pool_pages=16)
+    gen = torch.Generator("cuda").manual_seed(nr)
+    pool = torch.randn(256 * 576, generator=gen, device="cuda").to(torch.float8_e4m3fn).view(torch.uint8)
+    scale = torch.rand(256, generator=gen, device="cuda") + 0.01
+    table = torch.arange(16, dtype=torch.int32, device="cuda").view(2, 8)
+    q = torch.randn((2, heads, 576), generator=gen, device="cuda").to(torch.bfloat16)
+    q[0, 5, 3] = float("nan")
+    pool[(128 + nr - 1) * 576 + 20] = 0x7F                    # the last row of the second sequence
+    out = torch.zeros((2, heads, 512), dtype=torch.bfloat16, device="cuda")
+    n = torch.full((2,), nr, dtype=torch.int32, device="cuda")
+    scratch = torch.zeros(max(16, be.attend_paged_scratch_bytes(g, 2)), dtype=torch.uint8, device="cuda")
+    be.launch_attend_paged_bf16(g, q, pool, scale, table, None, 0, n, 2, out, None, None, scratch)
+    be.device_sync()
+    nan = out.float().isnan().cpu()
+    for h in range(heads):
+        assert bool(nan[0, h].all()) if h == 5 else not bool(nan[0, h].any()), h
+    assert bool(nan[1].all())
