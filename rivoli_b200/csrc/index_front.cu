@@ -191,9 +191,7 @@ front_gemm_mma_kernel(FrontArgs A) {
         const uint8_t* w = row < n0 ? J.m[0].w + (size_t)(tile * TN + row) * K : J.m[1].w + (size_t)(row - n0) * K;
         asm volatile("prefetch.global.L2 [%0];" ::"l"(w + k0 + line * 128));
     }
-    // the wait comes before the trigger: the epilogue kernel may then read inputs of this call before its own wait
     rv_grid_dep_wait();
-    rv_grid_dep_trigger();
     // this thread's weight pieces: row e / 4, codes 16 (e % 4) .. + 15 of each chunk
     const uint8_t* pw[3];
     uint32_t dw[3];
@@ -244,6 +242,9 @@ front_gemm_mma_kernel(FrontArgs A) {
             __syncthreads();
             tc::tc_fence_after();
             tmem = tmem_slot;
+            // Behind the wait: the epilogue kernel may then read inputs of this call before its own. Behind the allocation, which
+            // waits for its columns without a limit: a dependent could take them and then wait for this grid.
+            rv_grid_dep_trigger();
         }
         if (warp == 8) {
             for (int c = 0; c < nch && ok; ++c) {

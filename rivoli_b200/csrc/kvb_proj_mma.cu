@@ -162,10 +162,15 @@ kvb_absorb_mma_kernel(KpArgs A) {
         tc::mbar_init_fence();
         abort_word = 0;
     }
-    rv_grid_dep_trigger();
+    if (warp == 8) tc::tmem_alloc<256>(&tmem_slot);
     kp_prefetch(A.kvb + rbase * kvl + iblk * 128, (size_t)kvl, nope, 128);
     kp_prefetch(A.x + (size_t)h * A.xs, (size_t)A.H * A.xs * 2, min(128, A.B), nope * 2);
-    if (warp == 8) tc::tmem_alloc<256>(&tmem_slot);
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    // Behind the allocation, which waits for its columns without a limit: a dependent that is already on the SM could take them
+    // and then wait for this grid (the value kernel, which takes all of them, does start beside a CTA of this one).
+    rv_grid_dep_trigger();
     rv_grid_dep_wait();
     if (warp < 8) for (int c = 0; c < nch; ++c) {
         kp_request_acts(A, h, 0, c, sA + c * KP_ACHUNK);
@@ -178,9 +183,6 @@ kvb_absorb_mma_kernel(KpArgs A) {
     }
     const float s0 = A.scale[(rbase >> 7) * sc_cols + iblk];
     const float s1 = two_runs ? A.scale[((rbase + cut) >> 7) * sc_cols + iblk] : 0.0f;
-    tc::tc_fence_before();
-    __syncthreads();
-    tc::tc_fence_after();
     const uint32_t tmem = tmem_slot;
     const uint32_t idesc = kp_idesc(128, 128, 1);
     const uint32_t lane_base = ((uint32_t)((warp & 3) * 32)) << 16;   // TMEM lane quadrant of this warp
@@ -304,10 +306,13 @@ kvb_value_mma_kernel(KpArgs A) {
         tc::mbar_init_fence();
         abort_word = 0;
     }
-    rv_grid_dep_trigger();
+    if (warp == 8) tc::tmem_alloc<512>(&tmem_slot);
     kp_prefetch(A.kvb + row0 * kvl, (size_t)kvl, 128, kvl);
     kp_prefetch(A.x + (size_t)h * A.xs, (size_t)A.H * A.xs * 2, min(128, A.B), kvl * 2);
-    if (warp == 8) tc::tmem_alloc<512>(&tmem_slot);
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    rv_grid_dep_trigger();   // (behind the allocation: see the absorb kernel)
     rv_grid_dep_wait();
     auto request = [&](int b0, int c) {   // one cp.async group per call, with or without a chunk
         if (c < nch) {
@@ -325,9 +330,7 @@ kvb_value_mma_kernel(KpArgs A) {
 #pragma unroll 1
         for (int c = 0; c < KP_VST; ++c) request(0, c);
     if (tid < 2 * sc_cols) s_sc[tid / sc_cols][tid % sc_cols] = A.scale[((row0 + (tid / sc_cols) * 64) >> 7) * sc_cols + tid % sc_cols];
-    tc::tc_fence_before();
     __syncthreads();
-    tc::tc_fence_after();
     const uint32_t tmem = tmem_slot;
     const uint32_t idesc = kp_idesc(128, 128, 0);
     const uint32_t lane_base = ((uint32_t)((warp & 3) * 32)) << 16;   // TMEM lane quadrant of this warp
