@@ -550,11 +550,14 @@ attend_mma_kernel(AttendMmaArgs A) {
         float l_acc = 0.0f;                                // sum of this thread's weights of head hd
         float m_ref = -INFINITY;                           // reference max of head hd (the same in its four threads)
         bool ok = ntiles > 0;
-        for (int i = 0; i < ntiles && ok; ++i) {
+        // A warp whose wait gave up brings the others to the slow path of the tile that they are in or come to next, where all
+        // agree to leave.
+        auto give_up = [&]() { (void)tc::barrier_any(1, AM_SOFTMAX_THREADS, true); (void)tc::barrier_any(2, AM_SOFTMAX_THREADS, true); };
+        for (int i = 0; i < ntiles; ++i) {
             const int s = i % AM_STAGES, use = i / AM_STAGES, sb = i % AM_SBUF, suse = i / AM_SBUF;
             ok = tc::mbar_wait_warp(&bars.k_full[s], use & 1, abort_flag, 61, A.max_polls) &&
                  tc::mbar_wait_warp(&bars.s_full[sb], suse & 1, abort_flag, 62, A.max_polls);
-            if (!ok) break;
+            if (!ok) { give_up(); break; }
             tc::tc_fence_after();
             // this thread's 16 tokens: four 16-byte loads per plane (the two half-warps read 64 bytes apart: no bank conflict)
             const float4* ti = reinterpret_cast<const float4*>(s_tok + s * AM_TILE + 32 * th + 16 * tb);
@@ -587,14 +590,8 @@ attend_mma_kernel(AttendMmaArgs A) {
 
             // Fast path: no score of the tile exceeds its head's reference by more than AM_LAG, so the
             // references stand and nothing has to be exchanged. One barrier-with-OR decides for the CTA.
-            uint32_t slow;
-            {
-                const uint32_t mine_slow = dmax > AM_LAG + AM_POFF ? 1u : 0u;   // NaN-free: dmax is -inf or finite or +inf (s2 carries AM_POFF, the reference does not)
-                asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\t"
-                             "bar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
-                             : "=r"(slow) : "r"(mine_slow), "n"(AM_SOFTMAX_THREADS) : "memory");
-            }
-            if (slow) {
+            // NaN-free: dmax is -inf or finite or +inf (s2 carries AM_POFF, the reference does not)
+            if (tc::barrier_any(1, AM_SOFTMAX_THREADS, dmax > AM_LAG + AM_POFF)) {
                 // exact per-head tile max: this thread's 16 tokens, its partner lane's, the other token half's warp
                 {
                     float mx = s2[0];
@@ -603,7 +600,7 @@ attend_mma_kernel(AttendMmaArgs A) {
                     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
                     if (lane < 16) s_wmax[th * 64 + hd] = mx;
                 }
-                tc::named_barrier(2, AM_SOFTMAX_THREADS);
+                if (tc::barrier_any(2, AM_SOFTMAX_THREADS, false)) { ok = false; break; }
                 float fac = 1.0f;
                 {
                     const float tm = fmaxf(s_wmax[hd], s_wmax[64 + hd]) - AM_POFF;
@@ -613,7 +610,8 @@ attend_mma_kernel(AttendMmaArgs A) {
                 }
                 tc::named_barrier(2, AM_SOFTMAX_THREADS);
                 // bring O^T and l to the new references. PV(i-1) must have landed first.
-                if (i >= 1) { ok = tc::mbar_wait_warp(&bars.pv_done, (i - 1) & 1, abort_flag, 63, A.max_polls); if (!ok) break; }
+                if (i >= 1) ok = tc::mbar_wait_warp(&bars.pv_done, (i - 1) & 1, abort_flag, 63, A.max_polls);
+                if (!ok) { if (i + 1 < ntiles) give_up(); break; }
                 tc::tc_fence_after();
                 if (i >= 1) {
                     uint32_t r[AM_HPT];
@@ -661,7 +659,7 @@ attend_mma_kernel(AttendMmaArgs A) {
                 lo_w[j >> 2] = cls[0] | (cls[1] << 16);
             }
             ok = tc::mbar_wait_warp(&bars.pv_done, (i & 1) ^ 1, abort_flag, 64, A.max_polls);   // PV(i - 1) has read the P' tile
-            if (!ok) break;
+            if (!ok) { if (i + 1 < ntiles) give_up(); break; }
             {
                 // row = head, bytes = tokens: this thread's 16 tokens are the 16-byte chunk 2 th + tb of its head's row
                 uint8_t* prow = smem + SM_P + sw64_chunk(hd, 2 * th + tb);

@@ -383,9 +383,9 @@ index_score_mma_kernel(IndexMmaArgs A, const __grid_constant__ CUtensorMap tm_ke
         // ------------------------------ epilogue: TMEM -> scores --------------------------------
         int it = 0;
         bool ok = true;
-        for (; ok && sh.next(A); sh.t = sh.t1) {
+        for (; sh.next(A); sh.t = sh.t1) {
             const int b = sh.b, nt = sh.nt;
-            tc::named_barrier(1, 128);  // previous item's constants are no longer read
+            if (tc::barrier_any(1, 128, !ok)) break;   // previous item's constants are no longer read
             if (tid < IM_NPAD) {
                 // a_t / s_k = sum_h (w_h ws s_q[h] ds) * max(cd_h, 0): the exact formula up to a few
                 // roundings (s_q, s_k, ds > 0 commute with the ReLU); the band covers them

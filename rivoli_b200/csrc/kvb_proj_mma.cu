@@ -189,7 +189,7 @@ kvb_absorb_mma_kernel(KpArgs A) {
     const int erow = (warp & 3) * 32 + lane, chalf = warp >> 2;      // epilogue: sequence row, column half
     bool ok = true;
     int done[2] = {0, 0};
-    for (int b0 = 0; b0 < A.B && ok; b0 += 128) {
+    for (int b0 = 0; b0 < A.B; b0 += 128) {                  // (after a wait that gave up too: the barriers stay matched)
         if (warp == 8) {
             for (int c = 0; c < nch && ok; ++c) {
                 const int wb = c & 1, run = c * 64 >= cut ? 1 : 0;       // (a run boundary is a multiple of 64)
@@ -337,7 +337,7 @@ kvb_value_mma_kernel(KpArgs A) {
     const int erow = (warp & 3) * 32 + lane, chalf = warp >> 2;      // epilogue: sequence row, 64-column half
     bool ok = true;
     int done[2] = {0, 0};
-    for (int b0 = 0; b0 < A.B && ok; b0 += 128) {
+    for (int b0 = 0; b0 < A.B; b0 += 128) {                  // (after a wait that gave up too: the barriers stay matched)
         if (warp == 8) {
             for (int c = 0; c < nch && ok; ++c) {
                 const int wb = c & 1;

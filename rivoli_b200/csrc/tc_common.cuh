@@ -5,7 +5,8 @@
 // Every wait in this file gives up after a fixed number of polls, raises an abort word
 // that all other waits of the CTA observe, and returns false; the kernels then fall
 // through to their common exit (TMEM is released there), so a protocol bug surfaces as an
-// error code on the host and never as a hung GPU.
+// error code on the host and never as a hung GPU. Threads that meet at a barrier inside a loop leave
+// that loop together (barrier_any).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -215,6 +216,15 @@ __device__ __forceinline__ void tmem_stn(uint32_t taddr, const uint32_t* r) {
 // Sub-CTA barrier among `nthreads` threads (ids 1..15; 0 is __syncthreads).
 __device__ __forceinline__ void named_barrier(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
+// The same barrier with an answer: whether `p` holds in any of the threads. Warps can differ on whether a bounded wait gave up
+// (one polls while the phase completes, another looks when the abort word is already up), and a warp that left a loop on its own
+// would leave the others at the loop's barrier for good: a group leaves on this answer, together.
+__device__ __forceinline__ bool barrier_any(int id, int nthreads, bool p) {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, %2, %3, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(r) : "r"((uint32_t)p), "r"(id), "r"(nthreads) : "memory");
+    return r != 0;
 }
 
 }  // namespace tc

@@ -313,12 +313,15 @@ __global__ void __launch_bounds__(SA_THREADS, 1) v4_sparse_attend_kernel(SaArgs 
         for (int j = 0; j < 16; ++j) l_acc[j] = 0.0f;
         auto live_slot = [&](int t) { const int j = (t0 + t) * SA_TILE + tok; return t < ntiles && j < A.cols && ix[j] >= 0; };
         bool next_live = live_slot(0), ok = ntiles > 0;
-        for (int t = 0; t < ntiles && ok; ++t) {
+        // A warp whose wait gave up brings the others to the slow path of the tile that they are in or come to next, where all
+        // agree to leave.
+        auto give_up = [&]() { (void)tc::barrier_any(1, SA_ST, true); (void)tc::barrier_any(2, SA_ST, true); };
+        for (int t = 0; t < ntiles; ++t) {
             const int s = t & 1;
             const bool live = next_live;
             next_live = live_slot(t + 1);
             ok = tc::mbar_wait_warp(&bars.s_full[s], (t >> 1) & 1, abort_flag, 96);
-            if (!ok) break;
+            if (!ok) { give_up(); break; }
             tc::tc_fence_after();
             float s2[16], dmax = -INFINITY;
             {
@@ -339,13 +342,9 @@ __global__ void __launch_bounds__(SA_THREADS, 1) v4_sparse_attend_kernel(SaArgs 
             for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(ref + j) = *reinterpret_cast<const float4*>(s_ref + hb + j);
 #pragma unroll
             for (int j = 0; j < 16; ++j) dmax = fmaxf(dmax, s2[j] - ref[j]);   // (a masked slot before any reference: NaN, ignored)
-            uint32_t slow;
-            asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\t"
-                         "bar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
-                         : "=r"(slow) : "r"(dmax > SA_LAG ? 1u : 0u), "n"(SA_ST) : "memory");
-            if (slow) {
+            if (tc::barrier_any(1, SA_ST, dmax > SA_LAG)) {
                 s_wmax[sq * SA_H + 32 * th + lane] = sa_fold16<false>(s2, lane);
-                tc::named_barrier(2, SA_ST);
+                if (tc::barrier_any(2, SA_ST, false)) { ok = false; break; }
                 if (tid < SA_H) {
                     const float old = s_ref[tid];
                     const float m = fmaxf(fmaxf(fmaxf(s_wmax[tid], s_wmax[SA_H + tid]), fmaxf(s_wmax[2 * SA_H + tid], s_wmax[3 * SA_H + tid])), old);
@@ -355,7 +354,7 @@ __global__ void __launch_bounds__(SA_THREADS, 1) v4_sparse_attend_kernel(SaArgs 
                 tc::named_barrier(2, SA_ST);
                 if (t > 0) {   // O^T to the new references, once the values of the tile before have landed
                     ok = tc::mbar_wait_warp(&bars.k_empty[(t - 1) & 1], ((t - 1) >> 1) & 1, abort_flag, 97);
-                    if (!ok) break;
+                    if (!ok) { if (t + 1 < ntiles) give_up(); break; }
                     tc::tc_fence_after();
 #pragma unroll 1
                     for (int c = 0; c < 4; ++c) {

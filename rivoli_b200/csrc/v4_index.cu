@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(ST_THREADS) v4_score_tc_kernel(StArgs A, const
     } else if (warp >= 6) {
         // ---- query of an item: thread = (head, half of the 128 dims), two blocks of 32 each
         const int t = tid - 192, hh = t >> 1, j0 = (t & 1) * 2;
-        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+        for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
             if (!item_rows(item, b, t0, t1, n)) continue;
             const int qb = done & 1;
             uint32_t wv[2][16];
@@ -486,9 +486,8 @@ __global__ void __launch_bounds__(ST_THREADS) v4_score_tc_kernel(StArgs A, const
 #pragma unroll
                 for (int k = 0; k < 8; ++k) o[j][k] = v4_pack4(wv[j][2 * k], wv[j][2 * k + 1], inv, fits);
             ok = tc::mbar_wait_warp(&bars.qfree[qb], ((done >> 1) & 1) ^ 1, &abort_flag, 12);
-            if (!ok) break;
-            if (t == 0) s_bad[qb] = 0;
-            tc::named_barrier(2, 128);
+            if (ok && t == 0) s_bad[qb] = 0;
+            if (tc::barrier_any(2, 128, !ok)) break;
 #pragma unroll
             for (int j = 0; j < 2; ++j)
 #pragma unroll

@@ -1,5 +1,5 @@
 """Rules of the kernels' control flow that no run can show to hold, read off their sources: what orders an allocation of tensor
-memory against the kernels behind it."""
+memory against the kernels behind it, and what keeps the threads of a group together at their barriers."""
 import glob
 import os
 import re
@@ -26,6 +26,20 @@ def closing(s, i):
     raise AssertionError("unbalanced")
 
 
+def statement(s, i):
+    """End of the statement that begins at or behind ``i``."""
+    while s[i].isspace():
+        i += 1
+    if s[i] == "{":
+        return closing(s, i)
+    m = re.compile(r"(?:for|if|while)\s*\(").match(s, i)
+    if m:
+        return statement(s, closing(s, m.end() - 1))
+    while s[i] != ";":
+        i = closing(s, i) if s[i] in "([{" else i + 1
+    return i + 1
+
+
 def kernels(s):
     return [body(s, m.end()) for m in re.finditer(r"__global__", s)]
 
@@ -44,3 +58,27 @@ def test_dependents_start_behind_the_allocation(path):
         if alloc >= 0 and trigger >= 0:
             between = k.find("__syncthreads()", alloc)
             assert alloc < between < trigger
+
+
+BARRIER = re.compile(r"__syncthreads|named_barrier|barrier_any|give_up|bar\.red|bar\.sync")
+LOOP = re.compile(r"\b(?:for|while)\s*\(")
+
+
+def loops(s):
+    for m in LOOP.finditer(s):
+        head = closing(s, m.end() - 1)
+        yield s[m.end():head - 1], s[head:statement(s, head)]
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=os.path.basename)
+def test_a_wait_that_gave_up_does_not_leave_a_loop_with_barriers(path):
+    """Warps can differ on whether a bounded wait gave up. In a loop whose threads meet at a barrier they go on, or call the
+    others, until the group has agreed to leave (``barrier_any``); a warp that just left would let the others wait for good."""
+    for head, inside in loops(code(path)):
+        if not BARRIER.search(inside):
+            continue
+        assert not re.search(r"\bok\b", head), head
+        own = inside
+        for h, nested in loops(inside):
+            own = own.replace(nested, ";")
+        assert not re.search(r"!\s*ok\s*\)\s*(?:\{\s*)?(?:break|return|continue)", own), own[:400]
