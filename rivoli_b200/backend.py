@@ -145,6 +145,15 @@ def _stream(s):
     return s if s is None or type(s) is int else s.cuda_stream
 
 
+def torch_stream(s, device):
+    """The torch stream that a launch's ``stream`` argument names (None and 0: the default stream), for torch's own operations in
+    its order. What is allocated under it may be dropped as soon as the launch is issued."""
+    import torch
+    if not _stream(s):
+        return torch.cuda.default_stream(device)
+    return torch.cuda.ExternalStream(_stream(s), device=device)
+
+
 def ensure_status(r: int, name: str) -> None:
     """0 = ok, positive = argument guard, negative = -(cudaError_t) (hip.rs:328-336)."""
     if r:

@@ -108,8 +108,11 @@ class V4TokenStep:
         """pos i32 [B]; kv_entry bf16 bits [B, head_dim] (the token's window entry); attn_proj / index_proj =
         (kv_proj, score_proj) f32 [B, cd] of the two compressors; q, index_q, index_w as for V4DecodeLayer.step."""
         L, g = self.layer, self.layer.g
+        if not kv_entry.is_contiguous():        # copied in the order of the launch's stream, which may not be the current one
+            with torch.cuda.stream(be.torch_stream(stream, kv_entry.device)):
+                kv_entry = kv_entry.contiguous()
         be.launch_v4_token_step_bf16(
-            g, L.B, pos, kv_entry.contiguous(), self.attn_comp.p, self.attn_comp.step_args(*attn_proj, L.kv_cache, L.kv_rows, g.window),
+            g, L.B, pos, kv_entry, self.attn_comp.p, self.attn_comp.step_args(*attn_proj, L.kv_cache, L.kv_rows, g.window),
             self.index_comp.p, self.index_comp.step_args(*index_proj, L.index_kv, g.max_comp, 0, L.packed, L.packed_exp),
             q, index_q, index_w, L.sink, L.sel, L.scratch, L.out, stream)
         return L.out

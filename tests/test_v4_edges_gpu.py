@@ -227,3 +227,32 @@ def test_quantisers_of_rows_that_are_not_finite(value):
         t = dev(y.copy())
         be.launch_act_quant_f4_rotated(t, 4, d)
         assert np.array_equal(t.cpu().numpy(), want.reshape(4, d), equal_nan=True), d
+
+
+@pytest.mark.parametrize("as_address", [False, True])
+def test_token_step_takes_a_strided_entry_in_the_order_of_its_stream(as_address):
+    """The entry of a token as a slice of a wider tensor, on a stream that is not the current one, whose work is still pending."""
+    be = _be()
+    from rivoli_b200.v4 import V4Compressor, V4DecodeLayer, V4TokenStep
+    g, b = be.V4Geom.make(max_comp=32, window=8, index_topk=8), 3
+    gen = torch.Generator("cuda").manual_seed(0)
+    f32 = lambda *s: torch.randn(s, generator=gen, device="cuda")
+    bf = lambda *s: f32(*s).to(torch.bfloat16).view(torch.uint16)
+    layer, rng = V4DecodeLayer(g, b), np.random.default_rng(0)
+    comps = []
+    for w, rotate in ((512, False), (128, True)):
+        p = be.CompGeom.make(ratio=4, d=w, rd=64)
+        norm, freqs, ape = _comp_fixture(rng, p, 64)
+        comps.append(V4Compressor(p, b, dev(ape), dev(norm), dev(freqs), rotate))
+    step = V4TokenStep(layer, *comps)
+    wide, pos = bf(b, 3, 512), torch.tensor([4, 9, 17], dtype=torch.int32, device="cuda")
+    x = ((f32(b, 1024), f32(b, 1024)), (f32(b, 256), f32(b, 256)), bf(b, 64, 512), bf(b, 64, 128), f32(b, 64))
+    side = torch.cuda.Stream()
+    step(pos, wide[:, 0].contiguous(), *x)                 # (the kernels are loaded)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(100_000_000)                         # the current stream is busy for some 50 ms
+    step(pos, wide[:, 1], *x, stream=side.cuda_stream if as_address else side)
+    side.synchronize()
+    with torch.cuda.stream(side):
+        got = layer.kv_cache.view(torch.int16)[torch.arange(b, device="cuda"), (pos % 8).long()].cpu()
+    assert torch.equal(got, wide.view(torch.int16)[:, 1].cpu())
