@@ -96,7 +96,8 @@ attend_simt_kernel(AttSlab sp, AttPaged pp, int H, int rope, float scale, int nr
     constexpr bool RING = WIDE && ROPE64;
     constexpr int ROW_BYTES = at_row_bytes(PAGED, KVL), WARP_FLOATS = at_warp_bytes(PAGED, KVL) / 4;
     extern __shared__ __align__(16) float at_smem[];           // per warp: rows in flight, then its outputs [HG][KVL]
-    __shared__ float s_m[AT_WARPS][HG], s_l[AT_WARPS][HG];      // their maxima and sums
+    __shared__ float s_m[AT_WARPS][HG], s_l[AT_WARPS][HG];      // their reference maxima and sums
+    __shared__ float s_top[AT_WARPS][HG], c_top[HG];            // the largest scores, of warps and of the CTA (out_m)
     __shared__ float s_w[AT_MAX_CLUSTER][HG];                    // weights in the merge, of warps and then of CTAs
     __shared__ float c_m[HG], c_l[HG];                          // the CTA's, read by its cluster
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -165,6 +166,7 @@ attend_simt_kernel(AttSlab sp, AttPaged pp, int H, int rope, float scale, int nr
     at_f2 acc[HG][N2];
     const int my_row = lane >> 4, my_head = (lane >> 3) & 1;      // the score this lane's group of eight ends up with
     float m = -INFINITY, l = 0.0f;                                // reference maximum of my_head, sum of its rows of parity my_row
+    float top = -INFINITY;                                        // their largest score, which m follows at a distance
 #pragma unroll
     for (int j = 0; j < HG; ++j)
 #pragma unroll
@@ -307,6 +309,7 @@ attend_simt_kernel(AttSlab sp, AttPaged pp, int H, int rope, float scale, int nr
             s += __shfl_xor_sync(0xffffffffu, s, 2);
             s += __shfl_xor_sync(0xffffffffu, s, 1);
             s = live ? s * scale : -INFINITY;
+            if (PAGED) top = fmaxf(top, s);
             // the reference m follows the maximum at a distance: a weight may reach e^AT_LAG, which f32 holds as well as
             // 1, and the sums are rescaled at a warp's first rows and then hardly ever
             if (__any_sync(0xffffffffu, s > m + AT_LAG)) {
@@ -335,10 +338,11 @@ attend_simt_kernel(AttSlab sp, AttPaged pp, int H, int rope, float scale, int nr
         }
     }
     l += __shfl_xor_sync(0xffffffffu, l, 16);                    // both row parities
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
     if (RING) tc::cp_async_wait<0>();                            // (nothing is in flight; the slots become the output buffer)
 
     // ---- the CTA's warps meet in shared memory (a warp without rows has m = -inf, l = 0) ----
-    if ((lane & 23) == 0) { s_m[warp][my_head] = m; s_l[warp][my_head] = l; }
+    if ((lane & 23) == 0) { s_m[warp][my_head] = m; s_l[warp][my_head] = l; s_top[warp][my_head] = top; }
     if (r_begin < r_end) {
 #pragma unroll
         for (int j = 0; j < HG; ++j)
@@ -353,9 +357,9 @@ attend_simt_kernel(AttSlab sp, AttPaged pp, int H, int rope, float scale, int nr
         if (PAGED) pp.out[((size_t)b * H + h) * KVL + c] = rv_f32_to_bf16(v);
         else sp.clat[(size_t)h * KVL + c] = v;
     };
-    auto stats = [&](int h, float mg, float lg) {
+    auto stats = [&](int h, float most, float mg, float lg) {
         if (PAGED) {
-            if (pp.out_m) pp.out_m[(size_t)b * H + h] = mg;
+            if (pp.out_m) pp.out_m[(size_t)b * H + h] = most;
             if (pp.out_lse) pp.out_lse[(size_t)b * H + h] = lg > 0.0f ? mg + logf(lg) : -INFINITY;
         }
     };
@@ -370,7 +374,13 @@ attend_simt_kernel(AttSlab sp, AttPaged pp, int H, int rope, float scale, int nr
         for (int v = 0; v < AT_WARPS; ++v)
             if (s_l[v][j] != 0.0f) sum += s_l[v][j] * expf(s_m[v][j] - mx);
         s_w[w][j] = s_l[w][j] != 0.0f ? expf(s_m[w][j] - mx) : 0.0f;
-        if (w == 0) { c_m[j] = mx; c_l[j] = sum; }
+        if (w == 0) {
+            c_m[j] = mx; c_l[j] = sum;
+            float most = -INFINITY;
+#pragma unroll
+            for (int v = 0; v < AT_WARPS; ++v) most = fmaxf(most, s_top[v][j]);
+            c_top[j] = most;
+        }
     }
     __syncthreads();
     auto cta_sum = [&](int j, int c) {                            // column c of head j over the CTA's warps
@@ -385,7 +395,7 @@ attend_simt_kernel(AttSlab sp, AttPaged pp, int H, int rope, float scale, int nr
             const int j = e / KVL, c = e - j * KVL;
             if (head0 + j < H) store(head0 + j, c, c_l[j] != 0.0f ? cta_sum(j, c) * (1.0f / c_l[j]) : 0.0f);
         }
-        if (tid < HG && head0 + tid < H) stats(head0 + tid, c_m[tid], c_l[tid]);
+        if (tid < HG && head0 + tid < H) stats(head0 + tid, c_top[tid], c_m[tid], c_l[tid]);
         return;
     }
     // ---- and the cluster's CTAs through distributed shared memory ----
@@ -402,15 +412,18 @@ attend_simt_kernel(AttSlab sp, AttPaged pp, int H, int rope, float scale, int nr
         const int j = lane % HG, q = lane / HG;
         static_assert(HG * AT_MAX_CLUSTER <= 32, "one lane per (CTA, head)");
         const float mq = q < n_cta ? cluster.map_shared_rank(c_m, q)[j] : -INFINITY, lq = q < n_cta ? cluster.map_shared_rank(c_l, q)[j] : 0.0f;
-        float mg = mq;
+        float mg = mq, most = q < n_cta ? cluster.map_shared_rank(c_top, q)[j] : -INFINITY;
 #pragma unroll
-        for (int o = HG; o < HG * AT_MAX_CLUSTER; o <<= 1) mg = fmaxf(mg, __shfl_xor_sync(0xffffffffu, mg, o));
+        for (int o = HG; o < HG * AT_MAX_CLUSTER; o <<= 1) {
+            mg = fmaxf(mg, __shfl_xor_sync(0xffffffffu, mg, o));
+            most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+        }
         const float wq = lq != 0.0f ? expf(mq - mg) : 0.0f;
         float lg = lq * wq;
 #pragma unroll
         for (int o = HG; o < HG * AT_MAX_CLUSTER; o <<= 1) lg += __shfl_xor_sync(0xffffffffu, lg, o);
         if (q < AT_MAX_CLUSTER) s_w[q][j] = lq != 0.0f ? wq / lg : 0.0f;
-        if (q == 0 && rank == 0 && head0 + j < H) stats(head0 + j, mg, lg);
+        if (q == 0 && rank == 0 && head0 + j < H) stats(head0 + j, most, mg, lg);
     }
     __syncthreads();
     const int c_lo = HG * KVL * rank / n_cta, c_hi = HG * KVL * (rank + 1) / n_cta;   // this CTA merges and stores these columns

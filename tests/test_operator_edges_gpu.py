@@ -166,3 +166,28 @@ def test_paged_attention_is_loud_about_values_that_are_not_numbers(heads, nr):
     for h in range(heads):
         assert bool(nan[0, h].all()) if h == 5 else not bool(nan[0, h].any()), h
     assert bool(nan[1].all())
+
+
+@pytest.mark.parametrize("heads,nr", [(16, 0), (16, 2), (3, 97), (16, 700)])
+def test_paged_attention_reports_the_largest_score(heads, nr):
+    """out_m of the CUDA-core form is the largest score itself (the first score is below it by less than what makes the running
+    reference follow), out_lse its log-sum-exp; -inf for an empty sequence."""
+    be = _be()
+    g = be.DsaGeom.make(n_heads=heads, page_tokens=16, max_pages_per_seq=64, n_pool_pages=128)
+    gen = torch.Generator("cuda").manual_seed(nr)
+    pool = torch.randn(2048 * 576, generator=gen, device="cuda").to(torch.float8_e4m3fn)
+    scale = torch.rand(2048, generator=gen, device="cuda") * 0.1 + 0.01
+    table = torch.arange(128, dtype=torch.int32, device="cuda").view(2, 64)
+    q = torch.randn((2, heads, 576), generator=gen, device="cuda").to(torch.bfloat16)
+    out, n = torch.zeros((2, heads, 512), dtype=torch.bfloat16, device="cuda"), torch.full((2,), nr, dtype=torch.int32, device="cuda")
+    out_m, out_lse = torch.zeros((2, heads), device="cuda"), torch.zeros((2, heads), device="cuda")
+    be.launch_attend_simt_paged_bf16(g, q, pool.view(torch.uint8), scale, table, None, 0, n, 2, out, out_m, out_lse, None)
+    be.device_sync()
+    if nr == 0:
+        assert bool((out_m == -float("inf")).all() and (out_lse == -float("inf")).all() and (out == 0).all())
+        return
+    rows = pool.double().view(2048, 576) * scale.double()[:, None]
+    s = torch.stack([q[b].double() @ rows[b * 1024:b * 1024 + nr].T for b in range(2)]) * g.softmax_scale
+    # 576 products of f32 sums: 576 * 2^-24 of the largest partial sum, which is within a few of the scores' own size
+    assert bool(((out_m.double() - s.amax(-1)).abs() <= 1e-4).all())
+    assert bool(((out_lse.double() - s.logsumexp(-1)).abs() <= 1e-4).all())
