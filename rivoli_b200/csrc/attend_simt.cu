@@ -487,16 +487,21 @@ RIVOLI_API size_t rivoli_mla_attend_scratch_floats(int H, int kvl) {
     return (size_t)AT_MAX_SPLITS * (size_t)H * ((size_t)kvl + 2);
 }
 
-RIVOLI_API int rivoli_mla_attend(const float* qabs, const float* qrope, const unsigned char* Lc8,
-                                 const float* Lscale, const unsigned short* Rc, const unsigned int* rows,
-                                 int H, int nr, int kvl, int rope, int n_blocks, float scale, float* clat,
-                                 float* partial) {
+static int mla_attend_guard(int H, int nr, int kvl, int rope, int n_blocks) {
     if (H <= 0 || nr <= 0 || kvl <= 0 || rope <= 0 || n_blocks <= 0) return 1001;
     // The reference's staging bound and width rule, kept so the same shapes are rejected
     // with the same codes (attn.hip:285-293).
     if (((size_t)16 * kvl + (size_t)16 * rope) * sizeof(float) > 65536) return 1002;
     if (kvl > 512 || (kvl % 128) != 0) return 1004;
     if (rope > 128) return 1002;
+    return 0;
+}
+
+RIVOLI_API int rivoli_mla_attend(const float* qabs, const float* qrope, const unsigned char* Lc8,
+                                 const float* Lscale, const unsigned short* Rc, const unsigned int* rows,
+                                 int H, int nr, int kvl, int rope, int n_blocks, float scale, float* clat,
+                                 float* partial) {
+    if (int e = mla_attend_guard(H, nr, kvl, rope, n_blocks)) return e;
     // `partial` is the reference's scratch for a split: this library merges the splits on the chip and leaves it alone,
     // so the result does not depend on whether it was lent.
     (void)partial;
@@ -507,17 +512,14 @@ RIVOLI_API int rivoli_mla_attend(const float* qabs, const float* qrope, const un
 
 // rivoli_mla_attend for callers that have no device memory to lend (everything carved into their own arenas, a decode
 // thread that must not wait for the allocator, a plugin contract that forbids it). The kernel needs no scratch, so this
-// is the same launch, limited to H <= 64 and kvl <= 512 as documented.
-constexpr int NA_MAX_H = 64, NA_MAX_KVL = 512;
+// is the same launch. More than 64 heads stay refused, as the entry point's contract has it: a host may rely on the code.
+constexpr int NA_MAX_H = 64;
 
 RIVOLI_API int rivoli_mla_attend_static(const float* qabs, const float* qrope, const unsigned char* Lc8,
                                         const float* Lscale, const unsigned short* Rc, const unsigned int* rows,
                                         int H, int nr, int kvl, int rope, int n_blocks, float scale, float* clat) {
-    if (H > NA_MAX_H || kvl > NA_MAX_KVL) {
-        if (nr <= 0 || rope <= 0 || n_blocks <= 0) return 1001;
-        if (((size_t)16 * kvl + (size_t)16 * rope) * sizeof(float) > 65536) return 1002;
-        return (kvl > 512 || (kvl % 128) != 0) ? 1004 : 1002;
-    }
+    if (int e = mla_attend_guard(H, nr, kvl, rope, n_blocks)) return e;
+    if (H > NA_MAX_H) return 1002;
     return rivoli_mla_attend(qabs, qrope, Lc8, Lscale, Rc, rows, H, nr, kvl, rope, n_blocks, scale, clat, nullptr);
 }
 

@@ -63,6 +63,20 @@ def test_guards_fire_on_the_host(be):
     assert be.attend_scratch_floats(64, 512) == 16 * 64 * 514
 
 
+def test_attend_static_refuses_in_the_documented_order(be):
+    """Sizes (1001) before the staging bound (1002) before the width (1004) before the head count (1002), whatever else is wrong."""
+    def code(h, nr, kvl, rope, blocks):
+        with pytest.raises(be.BackendError) as e:
+            be.launch_attend_static(0, 0, 0, 0, 0, None, h, nr, kvl, rope, blocks, 1.0, 0)
+        return e.value.code
+    for h, nr, kvl, rope, blocks in [(0, 1, 512, 64, 4), (65, 0, 512, 64, 4), (65, 1, 0, 64, 4), (65, 1, -128, 64, 4), (0, 1, 640, 64, 5),
+                                     (65, 1, 512, 0, 4), (65, 1, 512, 64, 0), (-1, 1, 1024, 64, 8)]:
+        assert code(h, nr, kvl, rope, blocks) == 1001
+    assert code(64, 1, 1024, 64, 8) == 1002 and code(65, 1, 512, 1024, 4) == 1002     # staging
+    assert code(64, 1, 640, 64, 5) == 1004 and code(65, 1, 160, 64, 1) == 1004        # width
+    assert code(64, 1, 512, 129, 4) == 1002 and code(65, 1, 512, 64, 4) == 1002       # rope, heads
+
+
 def test_page_pool_matches_oracle_under_churn(be):
     """Continuous-batching churn: 10 % of sequences finish and are replaced each step;
     page tables and free lists stay bit-identical to the oracle's allocator."""
