@@ -244,9 +244,9 @@ int rivoli_index_select_status(const DsaGeom* g, int B, int score_stride, void* 
 int rivoli_index_select_band_stats(const DsaGeom* g, int B, int score_stride, void* scratch,
                                    uint32_t* host_band, void* stream);
 
-/* Bytes of scratch rivoli_mla_attend_paged_bf16 needs for B sequences (an error word and the
- * split partials). Zero its first 256 bytes once after allocation: the error word is sticky (first
- * failure wins) until rivoli_mla_attend_paged_status reads and clears it. */
+/* Bytes of scratch rivoli_mla_attend_paged_bf16 needs for B sequences: an error word, 256 bytes whatever the batch. Zero
+ * them once after allocation: the error word is sticky (first failure wins) until rivoli_mla_attend_paged_status reads and
+ * clears it. */
 size_t rivoli_mla_attend_paged_scratch_bytes(const DsaGeom* g, int B);
 
 /* Batched, paged form of rivoli_mla_attend (attn.hip:119-232 + combine :241-273).
@@ -332,7 +332,8 @@ int rivoli_shard_nccl_comm_destroy(void* comm);
 
 /* CUDA-core (f32 accumulate) implementation of rivoli_mla_attend_paged_bf16, same contract.
  * No reference counterpart beyond attn.hip:119-232 itself: it is the cross-check of the
- * tensor-core kernel and serves geometries that kernel does not cover. */
+ * tensor-core kernel and serves geometries that kernel does not cover. It needs no scratch (0 bytes; what is lent is left
+ * alone). */
 size_t rivoli_attend_simt_scratch_bytes(const DsaGeom* g, int B);
 int rivoli_attend_simt_paged_bf16(const DsaGeom* g, const uint16_t* q, const uint8_t* latent_pool,
                                   const float* latent_scale, const int32_t* block_table,

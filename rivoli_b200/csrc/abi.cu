@@ -4,7 +4,6 @@
 #include "codec.cuh"
 #include "common.cuh"
 
-extern "C" size_t rivoli_attend_simt_scratch_bytes(const DsaGeom* g, int B);
 extern "C" int rivoli_attend_simt_paged_bf16(const DsaGeom* g, const uint16_t* q, const uint8_t* latent_pool,
                                              const float* latent_scale, const int32_t* block_table,
                                              const uint32_t* rows, int row_stride, const int32_t* n_rows,
@@ -12,7 +11,6 @@ extern "C" int rivoli_attend_simt_paged_bf16(const DsaGeom* g, const uint16_t* q
                                              void* scratch, void* stream);
 
 extern "C" bool rivoli_attend_mma_supported(const DsaGeom* g);
-extern "C" size_t rivoli_attend_mma_scratch_bytes(const DsaGeom* g, int B);
 extern "C" int rivoli_attend_mma_paged_bf16(const DsaGeom* g, const uint16_t* q, const uint8_t* latent_pool,
                                             const float* latent_scale, const int32_t* block_table,
                                             const uint32_t* rows, int row_stride, const int32_t* n_rows, int B,
@@ -20,11 +18,9 @@ extern "C" int rivoli_attend_mma_paged_bf16(const DsaGeom* g, const uint16_t* q,
                                             int q_early, int min_rows_hint, long long max_rows, void* stream);
 extern "C" int rivoli_attend_mma_status(void* scratch, void* stream);
 
+// The error word of the tensor-core kernel, for any geometry and batch: all partial results are merged on the chip.
 RIVOLI_API size_t rivoli_mla_attend_paged_scratch_bytes(const DsaGeom* g, int B) {
-    if (!g || B <= 0) return 0;
-    const size_t a = rivoli_attend_simt_scratch_bytes(g, B);
-    const size_t m = rivoli_attend_mma_supported(g) ? rivoli_attend_mma_scratch_bytes(g, B) : 0;
-    return a > m ? a : m;
+    return g && B > 0 ? 256 : 0;
 }
 
 // 1 when rivoli_mla_attend_paged_bf16 runs on the tensor cores for this geometry (given scratch).
@@ -60,8 +56,7 @@ static int attend_paged_dispatch(const DsaGeom* g, const uint16_t* q, const uint
     if (int e = rv_check_geom(g)) return e;
     if (B <= 0 || !q || !latent_pool || !latent_scale || !block_table || !n_rows || !out) return 1001;
     if (rows && row_stride <= 0) return 1001;
-    // Tensor-core kernel for the model geometry (64 heads, 512 + 64 dims), given scratch (error word and
-    // split partials); inside that call, sequences of fewer than 128 rows go to the CUDA-core kernel.
+    // Tensor-core kernel for the model geometry (64 heads, 512 + 64 dims), given scratch (its error word); inside that call, sequences of fewer than 128 rows go to the CUDA-core kernel.
     // Every other geometry runs on the CUDA-core kernel.
     if (scratch && rivoli_attend_mma_supported(g))
         return rivoli_attend_mma_paged_bf16(g, q, latent_pool, latent_scale, block_table, rows, row_stride, n_rows,

@@ -865,10 +865,6 @@ extern "C" bool rivoli_attend_mma_supported(const DsaGeom* g) {
 
 // scratch layout: [err 256 B]. The error word is sticky: it keeps the first failure
 // until rivoli_attend_mma_status reads and clears it, so it must be zero before the first call.
-extern "C" size_t rivoli_attend_mma_scratch_bytes(const DsaGeom* g, int B) {
-    (void)g; (void)B;
-    return 256;
-}
 
 extern "C" int rivoli_attend_simt_short_rows(const DsaGeom* g, const uint16_t* q, const uint8_t* latent_pool,
                                              const float* latent_scale, const int32_t* block_table,

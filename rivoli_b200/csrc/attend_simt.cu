@@ -40,7 +40,7 @@ constexpr int AT_WARPS = 6;          // two CTAs of six warps per SM: 170 regist
 constexpr int AT_THREADS = AT_WARPS * 32;
 constexpr float AT_LAG = 8.0f;
 constexpr int AT_MAX_CLUSTER = 8;
-constexpr int AT_MAX_SPLITS = 16;    // sizes the caller's scratch (attn.hip:67); this kernel needs none
+constexpr int AT_MAX_SPLITS = 16;    // sizes the scratch of the reference's operator (attn.hip:67); this kernel needs none
 
 constexpr int AT_RING = 8;           // rows in flight per warp (64 rope columns: the model's shape)
 // Shared memory per warp: a row in flight is its latent codes, its rope columns and (slab) one scale per lane; the same
@@ -523,18 +523,8 @@ RIVOLI_API int rivoli_mla_attend_static(const float* qabs, const float* qrope, c
     return rivoli_mla_attend(qabs, qrope, Lc8, Lscale, Rc, rows, H, nr, kvl, rope, n_blocks, scale, clat, nullptr);
 }
 
-// Sizes the scratch that callers of the paged form lend: a pure function of the batch size.
-static int simt_paged_splits(int B) {
-    int n = (2 * 148 + B - 1) / B;
-    if (n > AT_MAX_SPLITS) n = AT_MAX_SPLITS;
-    if (n < 1) n = 1;
-    return n;
-}
-
-RIVOLI_API size_t rivoli_attend_simt_scratch_bytes(const DsaGeom* g, int B) {
-    if (!g || B <= 0) return 0;
-    return (size_t)B * simt_paged_splits(B) * g->n_heads * ((size_t)g->kv_lora + 2) * sizeof(float);
-}
+// None: the splits merge on the chip.
+RIVOLI_API size_t rivoli_attend_simt_scratch_bytes(const DsaGeom*, int) { return 0; }
 
 // Paged bf16 attention on CUDA cores. Same contract as rivoli_mla_attend_paged_bf16.
 RIVOLI_API int rivoli_attend_simt_paged_bf16(const DsaGeom* g, const uint16_t* q, const uint8_t* latent_pool,

@@ -77,6 +77,13 @@ def test_attend_static_refuses_in_the_documented_order(be):
     assert code(64, 1, 512, 129, 4) == 1002 and code(65, 1, 512, 64, 4) == 1002       # rope, heads
 
 
+@pytest.mark.parametrize("heads,batch", [(64, 1), (64, 128), (16, 1), (16, 500)])
+def test_attention_asks_for_no_scratch_that_no_kernel_touches(be, heads, batch):
+    g = be.DsaGeom.make(n_heads=heads, max_pages_per_seq=4, n_pool_pages=8)
+    assert be.attend_paged_scratch_bytes(g, batch) == 256 and be.attend_simt_scratch_bytes(g, batch) == 0
+    assert be.attend_paged_scratch_bytes(g, 0) == 0
+
+
 def test_page_pool_matches_oracle_under_churn(be):
     """Continuous-batching churn: 10 % of sequences finish and are replaced each step;
     page tables and free lists stay bit-identical to the oracle's allocator."""
