@@ -836,11 +836,12 @@ attend_mma_kernel(AttendMmaArgs A) {
 // inside a GPC). A batch is split only as far as all its clusters are resident at once: the largest cluster size
 // (<= 8) for which the device reports room for B clusters; anything more would run as a second wave.
 int mma_splits(int B) {
-    static int cache[149];   // 0 = not asked yet
-    if (B <= 0 || B > 74) return 1;
-    if (cache[B]) return cache[B];
-    cudaFuncSetAttribute(attend_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_TOTAL);
-    int n = 148 / B;
+    constexpr int MOST = 128;
+    static std::atomic<int> cache[MOST + 1];   // by batch; 0 = not asked yet
+    const int sms = rv_sm_count();
+    if (B <= 0 || B > MOST || 2 * B > sms) return 1;
+    if (const int known = cache[B].load(std::memory_order_relaxed)) return known;
+    int n = sms / B;
     if (n > AM_MAX_SPLITS) n = AM_MAX_SPLITS;
     for (; n > 1; --n) {
         cudaLaunchConfig_t cfg = {};
@@ -853,8 +854,9 @@ int mma_splits(int B) {
         if (cudaOccupancyMaxActiveClusters(&active, attend_mma_kernel, &cfg) == cudaSuccess && active >= B) break;
         (void)cudaGetLastError();
     }
-    cache[B] = n < 1 ? 1 : n;
-    return cache[B];
+    if (n < 1) n = 1;
+    cache[B].store(n, std::memory_order_relaxed);
+    return n;
 }
 
 }  // namespace
@@ -878,7 +880,7 @@ extern "C" int rivoli_attend_simt_short_rows(const DsaGeom* g, const uint16_t* q
 constexpr int AM_MIN_ROWS = 128;
 
 // Self-test state (rivoli_attend_mma_test_hook): overrides of the next launches, host side only.
-static int g_am_min_rows_override = -1, g_am_withhold_once = 0, g_am_max_polls = tc::kMaxPolls;
+static std::atomic<int> g_am_min_rows_override{-1}, g_am_withhold_once{0}, g_am_max_polls{tc::kMaxPolls};
 
 // Test hook, not for production callers. min_rows >= 0 replaces AM_MIN_ROWS until reset with -1 (0 sends every
 // sequence to the tensor-core kernel); withhold != 0 makes the NEXT launch leave out one barrier arrival so that
@@ -905,11 +907,12 @@ extern "C" int rivoli_attend_mma_paged_bf16(const DsaGeom* g, const uint16_t* q,
     if (((uintptr_t)latent_pool | (uintptr_t)scratch | (uintptr_t)q | (uintptr_t)out) & 15) return 1005;
     cudaStream_t st = (cudaStream_t)stream;
     int* err = reinterpret_cast<int*>(scratch);
+    rv_allow_smem<attend_mma_kernel>(SM_TOTAL);
     const int n_splits = mma_splits(B);
-    int min_rows = g_am_min_rows_override >= 0 ? g_am_min_rows_override : AM_MIN_ROWS;
+    const int forced = g_am_min_rows_override.load(std::memory_order_relaxed);
+    int min_rows = forced >= 0 ? forced : AM_MIN_ROWS;
     if (min_rows_hint >= min_rows) min_rows = 0;          // the caller vouches that no sequence is that short
-    const int withhold = g_am_withhold_once;
-    g_am_withhold_once = 0;
+    const int withhold = g_am_withhold_once.load(std::memory_order_relaxed) ? g_am_withhold_once.exchange(0) : 0;
 
     // short contexts first (a programmatic dependent of whatever precedes this call; its CTAs leave at once
     // for every other sequence), then the tensor-core kernel as a dependent of that launch
@@ -925,8 +928,7 @@ extern "C" int rivoli_attend_mma_paged_bf16(const DsaGeom* g, const uint16_t* q,
     AttendMmaArgs a{q, g->softmax_scale, latent_pool, latent_scale, block_table, rows, row_stride, n_rows,
                     g->page_tokens, g->max_pages_per_seq, g->n_pool_pages, n_splits,
                     out, out_m, out_lse, err,
-                    min_rows, q_early ? 1 : 0, g_am_max_polls, withhold};
-    cudaFuncSetAttribute(attend_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_TOTAL);
+                    min_rows, q_early ? 1 : 0, g_am_max_polls.load(std::memory_order_relaxed), withhold};
     // one CTA per (sequence, split); the splits of a sequence are one thread-block cluster and merge inside the kernel
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)n_splits, (unsigned)B); cfg.blockDim = dim3(AM_THREADS);

@@ -444,7 +444,7 @@ attend_simt_kernel(AttSlab sp, AttPaged pp, int H, int rope, float scale, int nr
 // and no more than leave every warp about two rows (rows_most: what the host knows of the longest sequence).
 static int simt_cluster(int B, int groups, long long rows_most) {
     int n = 1;
-    while (n < AT_MAX_CLUSTER && (long long)B * groups * n * 2 <= 2 * 148 && (long long)n * AT_WARPS * 2 < rows_most) n *= 2;
+    while (n < AT_MAX_CLUSTER && (long long)B * groups * n * 2 <= 2 * rv_sm_count() && (long long)n * AT_WARPS * 2 < rows_most) n *= 2;
     return n;
 }
 

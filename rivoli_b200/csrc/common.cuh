@@ -39,7 +39,8 @@ static inline void rv_launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3
 
 // Opts a kernel in to `bytes` of dynamic shared memory, once per kernel and device (the attribute lives as long as the
 // context; setting it costs the host about half a microsecond). `bytes` is the most that any launch of this kernel asks
-// for, so threads that race to the first call set the same value.
+// for, so threads that race to the first call set the same value (set to what each launch needs, a thread with a smaller shape
+// could take a larger one's opt-in away between its call and its launch).
 template <auto Kernel>
 static inline void rv_allow_smem(int bytes) {
     static std::atomic<uint64_t> done{0};
@@ -49,6 +50,20 @@ static inline void rv_allow_smem(int bytes) {
     if (dev < 64 && (done.load(std::memory_order_acquire) & bit)) return;
     if (cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess)
         done.fetch_or(dev < 64 ? bit : 0, std::memory_order_release);
+}
+
+// SMs of the current device, asked once per device. (A plan that sizes memory which the caller lends must not depend on the
+// device: it takes RV_SMS, the SMs of a B200.)
+constexpr int RV_SMS = 148;
+static inline int rv_sm_count() {
+    static std::atomic<int> known[64];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return RV_SMS;
+    n = known[dev].load(std::memory_order_relaxed);
+    if (n) return n;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return RV_SMS;
+    known[dev].store(n, std::memory_order_relaxed);
+    return n;
 }
 #endif
 

@@ -156,7 +156,8 @@ fold_gemv_kernel(FoldGemv a) {
 // shared memory at 32 rows: several CTAs per SM, and the first addition starts early).
 static inline int launch_fold_gemv(FoldGemv a, int heads, int R, cudaStream_t st) {
     const int total = heads * a.n_out, most = 32 / R;
-    a.opc = (total + 147) / 148;
+    const int sms = rv_sm_count();
+    a.opc = (total + sms - 1) / sms;
     if (a.opc > most) a.opc = most;
     if (a.opc > a.n_out) a.opc = a.n_out;
     a.blocks = (a.n_out + a.opc - 1) / a.opc;

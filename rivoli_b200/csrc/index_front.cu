@@ -498,7 +498,8 @@ static bool front_mma_ok(const IndexFrontGeom* g) {
 
 // The jobs of a call and the floats of their partials. Tensor cores: the key and head-weight matrices share their activations
 // and take one tile where that is at most FM_NMAX wide; the split is the chunk count L with the shortest critical path, waves x
-// (L + 4), a launch's ramp and a partial's way out counting as four chunks. CUDA cores: enough CTAs to fill the machine, at
+// (L + 4), a launch's ramp and a partial's way out counting as four chunks (a function of geometry and batch alone: it sizes the
+// caller's scratch). CUDA cores: enough CTAs to fill the machine, at
 // least 256 contraction values per split, at most 32 splits.
 static void plan_jobs(const IndexFrontGeom* g, int B, bool mma, FrontArgs* fa, size_t* floats) {
     const int N[3] = {g->index_dim, g->index_heads * g->index_dim, g->index_heads};
@@ -524,7 +525,7 @@ static void plan_jobs(const IndexFrontGeom* g, int B, bool mma, FrontArgs* fa, s
         for (int L = 2; L <= 64; ++L) {
             long long ctas = 0;
             for (int j = 0; j < fa->n_jobs; ++j) ctas += (long long)fa->job[j].n_tiles * ceil_div(fa->job[j].K / 64, L);
-            const long long cost = (ctas + 147) / 148 * (L + 4);
+            const long long cost = (ctas + RV_SMS - 1) / RV_SMS * (L + 4);
             if (best < 0 || cost < best) { best = cost; pick = L; }
         }
         for (int j = 0; j < fa->n_jobs; ++j) fa->job[j].k_chunks = pick;

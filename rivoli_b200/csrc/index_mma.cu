@@ -537,11 +537,9 @@ static int select_impl(const DsaGeom* g, const AppendArgs* ap, const uint16_t* i
 
     IndexMmaArgs ma{*g, s.qcodes, s.qscales, w, index_pool, index_scale, block_table, seq_len,
                     s.scores, score_stride, B, s.err};
-    const size_t smem1 = (size_t)IM_NS * IM_STAGE_BYTES + 2 * IM_Q_BYTES + 1024;
-    cudaFuncSetAttribute(index_score_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    constexpr size_t smem1 = (size_t)IM_NS * IM_STAGE_BYTES + 2 * IM_Q_BYTES + 1024;
+    rv_allow_smem<index_score_mma_kernel>((int)smem1);
+    const int sms = rv_sm_count();
     // two persistent CTAs per SM; a batch with fewer tiles at most gets as many CTAs
     const long long most = (long long)B * ((score_stride + IM_TILE - 1) / IM_TILE);
     const int grid = most < 2 * sms ? (int)most : 2 * sms;

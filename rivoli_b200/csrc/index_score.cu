@@ -180,7 +180,7 @@ RIVOLI_API int rivoli_index_score(const float* q, const float* w, const unsigned
         return rv_launch_status();
     }
     if (smem > 48 * 1024)
-        cudaFuncSetAttribute(index_score_slab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        rv_allow_smem<index_score_slab_kernel>(227 * 1024);
     index_score_slab_kernel<<<(nt + 7) / 8, 256, smem>>>(q, w, kcache, heads, nt, nact, hd, wscale, dscale, scores);
     return rv_launch_status();
 }

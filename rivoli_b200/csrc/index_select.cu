@@ -678,7 +678,7 @@ index_select_cluster_kernel(SelArgs A, int CH) {
 
 namespace rivoli {
 
-static int g_sel_cluster_override = 0;
+static std::atomic<int> g_sel_cluster_override{0};
 
 // CTAs per sequence: a lone CTA up to 8,192 tokens at any batch (what the tokens cost is less than the cluster barriers), else
 // two or four while each has an SM of its own, and at least enough for 16,384 tokens each. (Eight only when the tokens need
@@ -687,8 +687,8 @@ static int g_sel_cluster_override = 0;
 static bool select_cluster_plan(int B, int score_stride, int* cluster, int* ch) {
     int C = 1;
     if (score_stride > 8192)
-        while (C < 4 && (long long)B * C * 2 <= 148) C *= 2;
-    if (g_sel_cluster_override > 0) C = g_sel_cluster_override;
+        while (C < 4 && (long long)B * C * 2 <= rv_sm_count()) C *= 2;
+    if (const int forced = g_sel_cluster_override.load(std::memory_order_relaxed)) C = forced;
     while (C < SEL_MAX_CLUSTER && (long long)C * SEL_CH < score_stride) C *= 2;
     *cluster = C;
     *ch = ((score_stride + C - 1) / C + 3) / 4 * 4;

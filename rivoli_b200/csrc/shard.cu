@@ -203,7 +203,7 @@ RIVOLI_API int rivoli_shard_candidates(const DsaGeom* g, const uint16_t* index_q
     const size_t smem = ((size_t)RS_QWORDS + (size_t)SH_WARPS * SH_TOK * RS_HD) * 4;
     const int per_cta = SH_WARPS * SH_TOK * 4;
     rv_drain_error();
-    cudaFuncSetAttribute(shard_rescore_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    rv_allow_smem<shard_rescore_kernel>((int)smem);
     shard_rescore_kernel<<<dim3((g->top_k + per_cta - 1) / per_cta, B), SH_THREADS, smem, st>>>(
         *g, qcodes, qscales, w, index_pool, index_scale, block_table, rows_l, n_l, cs);
     return rv_launch_status();

@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 namespace rivoli {
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -14,13 +16,16 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 inline EncodeTiledFn encode_tiled_fn() {
-    static EncodeTiledFn fn = nullptr;
+    static std::atomic<EncodeTiledFn> known{nullptr};
+    EncodeTiledFn fn = known.load(std::memory_order_relaxed);
     if (!fn) {
         void* p = nullptr;
         cudaDriverEntryPointQueryResult q;
         if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
+            q == cudaDriverEntryPointSuccess) {
             fn = reinterpret_cast<EncodeTiledFn>(p);
+            known.store(fn, std::memory_order_relaxed);
+        }
     }
     return fn;
 }

@@ -513,11 +513,13 @@ __global__ void __launch_bounds__(SA_THREADS, 1) v4_sparse_attend_kernel(SaArgs 
 // CTAs per sequence: as many as leave all clusters resident at once (at most eight), and no more than there are tiles to
 // share out evenly.
 int sa_splits(int n_seqs, int tiles) {
-    static std::atomic<int> cache[75];       // largest resident cluster size by batch; 0 = not asked yet
-    if (n_seqs > 74) return 1;
+    constexpr int MOST = 128;
+    static std::atomic<int> cache[MOST + 1];   // largest resident cluster size by batch; 0 = not asked yet
+    const int sms = rv_sm_count();
+    if (n_seqs > MOST || 2 * n_seqs > sms) return 1;
     int most = cache[n_seqs].load(std::memory_order_relaxed);
     if (!most) {
-        for (most = 148 / n_seqs < SA_MAX_SPLITS ? 148 / n_seqs : SA_MAX_SPLITS; most > 1; --most) {
+        for (most = sms / n_seqs < SA_MAX_SPLITS ? sms / n_seqs : SA_MAX_SPLITS; most > 1; --most) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3((unsigned)(most * n_seqs)); cfg.blockDim = dim3(SA_THREADS); cfg.dynamicSmemBytes = SA_TOTAL;
             cudaLaunchAttribute at[1];
@@ -545,7 +547,7 @@ RIVOLI_API int rivoli_gather_attn_shared_kv(const float* q, const float* kv, con
     const size_t smem = ((size_t)d + (size_t)topk) * sizeof(float);
     if (smem + sizeof(float) * (GA_THREADS + 2) > 65536) return 1006;
     rv_drain_error();
-    cudaFuncSetAttribute(v4_gather_attn_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    rv_allow_smem<v4_gather_attn_kernel<float>>(65536);
     v4_gather_attn_kernel<float><<<dim3((unsigned)h, (unsigned)m), GA_THREADS, smem, (cudaStream_t)stream>>>(
         q, kv, 0, sink, idxs, h, d, topk, scale, o);
     return rv_launch_status();
@@ -578,7 +580,7 @@ int rivoli_v4_sparse_attend_launch(const V4Geom* g, int n_seqs, const uint16_t* 
     const size_t smem = ((size_t)g->head_dim + (size_t)cols) * sizeof(float);
     if (smem > 200 * 1024) return 1006;
     if (n_seqs > 65535) return 1002;
-    cudaFuncSetAttribute(v4_gather_attn_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    rv_allow_smem<v4_gather_attn_kernel<uint16_t>>(200 * 1024);
     v4_gather_attn_kernel<uint16_t><<<dim3((unsigned)g->n_heads, (unsigned)n_seqs), GA_THREADS, smem, st>>>(
         q, kv_cache, kv_rows * (size_t)g->head_dim, sink, sel, g->n_heads, g->head_dim, cols, g->softmax_scale, out);
     return rv_launch_status();

@@ -645,7 +645,7 @@ RIVOLI_API int rivoli_kv_compress_prefill(const float* kv, const float* score, c
     rv_drain_error();
     const bool wide = (((uintptr_t)kv | (uintptr_t)score | (uintptr_t)ape | (uintptr_t)ff->norm | (uintptr_t)ff->freqs | (uintptr_t)ff->out) & 15) == 0;
     if (p.ratio == 4 && wide && (p.d == 128 || p.d == 256 || p.d == 512)) {
-        const int groups = CP4_THREADS / (p.d / 2), most = CP4_CTAS * 148;
+        const int groups = CP4_THREADS / (p.d / 2), most = CP4_CTAS * rv_sm_count();
         const int ctas = (nblk + groups - 1) / groups;
         const dim3 grid((unsigned)(ctas < most ? ctas : most));
         if (p.d == 512) rv_launch_dependent(cp_prefill4_kernel<512>, grid, dim3(CP4_THREADS), 0, st, kv, score, ape, *ff, p, nblk);

@@ -764,7 +764,7 @@ RIVOLI_API int rivoli_index_score_blocks(const float* q, const float* kv, const 
     cudaStream_t st = (cudaStream_t)stream;
     if (heads <= SC_MAX_HEADS && hd <= SC_MAX_HD && hd % 4 == 0 && s <= 65535) {
         const size_t smem = ((size_t)hd * SC_MAX_HEADS + SC_MAX_HEADS + (size_t)(SCK_THREADS / 32) * SC_CB * hd) * sizeof(float);
-        cudaFuncSetAttribute(v4_score_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        rv_allow_smem<v4_score_blocks_kernel>((SC_MAX_HD * SC_MAX_HEADS + SC_MAX_HEADS + (SCK_THREADS / 32) * SC_CB * SC_MAX_HD) * (int)sizeof(float));
         dim3 grid((unsigned)((n_comp + SCK_BLOCKS_PER_CTA - 1) / SCK_BLOCKS_PER_CTA), (unsigned)s);
         v4_score_blocks_kernel<<<grid, SCK_THREADS, smem, st>>>(q, kv, w, score, n_comp, heads, hd);
     } else {
@@ -810,7 +810,7 @@ RIVOLI_API int rivoli_v4_select_blocks_bf16(const V4Geom* g, int n_seqs, const i
     int32_t* flags = reinterpret_cast<int32_t*>(scores + (size_t)n_seqs * g->max_comp);
     const bool tensor = !force_fold && g->index_dim == 128 && n_seqs <= 65535;
     if (tensor && packed && ((uintptr_t)packed & 15) == 0 && ((uintptr_t)index_q & 15) == 0) {
-        const int tiles = (g->max_comp + ST_TILE - 1) / ST_TILE, ctas = 2 * 148;
+        const int tiles = (g->max_comp + ST_TILE - 1) / ST_TILE, ctas = 2 * rv_sm_count();
         // tiles per item: the run length with the shortest critical path, an item's query counted as one tile
         int tpi = ST_TPI;
         long long best = -1;
@@ -829,7 +829,7 @@ RIVOLI_API int rivoli_v4_select_blocks_bf16(const V4Geom* g, int n_seqs, const i
         v4_score_int8_kernel<<<grid, SI_THREADS, 0, st>>>(*g, pos, index_q, index_w, index_kv, scores);
     }
     if (int e = rv_launch_status()) return e;
-    cudaFuncSetAttribute(v4_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    rv_allow_smem<v4_select_kernel>(227 * 1024);
     rv_launch_dependent(v4_select_kernel, dim3((unsigned)n_seqs), dim3(TK_THREADS), smem, st, *g, pos, index_q, index_w,
                         index_kv, sel, scores, flags, tensor ? 0 : 1);
     return rv_launch_status();
