@@ -111,17 +111,14 @@ __device__ __forceinline__ void kp_convert16(const uint8_t* raw, uint8_t* d0, ui
     *reinterpret_cast<uint4*>(d0) = kp_codes_to_bf16(make_uint2(v.x, v.y));
     *reinterpret_cast<uint4*>(d1) = kp_codes_to_bf16(make_uint2(v.z, v.w));
 }
-// Waits until at most `left` of this thread's copy groups are pending (left < 8).
+// Waits until at most `left` of this thread's copy groups are pending (left < KP_ACHUNKS).
+constexpr int KP_ACHUNKS = 4;      // most chunks of the absorb contraction (rivoli_kvb_mma_supported: nope <= 256)
 __device__ __forceinline__ void kp_wait_groups(int left) {
     switch (left) {
         case 0: tc::cp_async_wait<0>(); break;
         case 1: tc::cp_async_wait<1>(); break;
         case 2: tc::cp_async_wait<2>(); break;
-        case 3: tc::cp_async_wait<3>(); break;
-        case 4: tc::cp_async_wait<4>(); break;
-        case 5: tc::cp_async_wait<5>(); break;
-        case 6: tc::cp_async_wait<6>(); break;
-        default: tc::cp_async_wait<7>(); break;
+        default: tc::cp_async_wait<KP_ACHUNKS - 1>(); break;
     }
 }
 // The 128 x 128 bf16 result staged as [128 rows][256 B], 16-byte chunks XORed with the row: chunk k of row r.
@@ -421,7 +418,7 @@ kvb_value_mma_kernel(KpArgs A) {
 // whose rows straddle at most one block boundary; vh a multiple of 128; the head's row count a multiple
 // of 64; 16-byte aligned activation rows; rope <= 64.
 extern "C" int rivoli_kvb_mma_supported(int H, int qh, int nope, int vh, int kvl, int rope, int block) {
-    if (block != 128 || kvl % 256 || kvl > 512 || nope % 64 || nope > 256 || vh % 128 || (nope + vh) % 64) return 0;
+    if (block != 128 || kvl % 256 || kvl > 512 || nope % 64 || nope > KP_ACHUNKS * 64 || vh % 128 || (nope + vh) % 64) return 0;
     if (qh % 8 || rope % 8 || rope > 64 || H <= 0) return 0;
     for (int h = 0; h < 2 && h < H; ++h) {          // the straddle pattern repeats with period <= 2 heads
         const int off = (h * (nope + vh)) & 127;
@@ -434,7 +431,7 @@ extern "C" int rivoli_kvb_absorb_mma(const uint16_t* q, const uint8_t* kvb, cons
                                      int vh, int kvl, int rope, int block, int B, uint16_t* q_abs, cudaStream_t st) {
     const KpArgs a{q, kvb, scale, H, qh, nope, vh, kvl, rope, block, B, q_abs};
     const size_t smem = (size_t)(nope / 64) * (KP_ACHUNK + KP_WCHUNK) + 2 * KP_CONV;
-    rv_allow_smem<kvb_absorb_mma_kernel>(4 * (KP_ACHUNK + KP_WCHUNK) + 2 * KP_CONV);
+    rv_allow_smem<kvb_absorb_mma_kernel>(KP_ACHUNKS * (KP_ACHUNK + KP_WCHUNK) + 2 * KP_CONV);
     rv_drain_error();
     rv_launch_dependent(kvb_absorb_mma_kernel, dim3(kvl / 128, H), dim3(KP_LAUNCH), smem, st, a);
     return rv_launch_status();
