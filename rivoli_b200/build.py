@@ -56,8 +56,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if r.returncode:
         raise RuntimeError("nvcc failed building librivolikernels.so")
     build_launch()
-    # registers / spills / shared memory per kernel: a build log, kept out of the source tree proper
-    log_dir = os.path.join(HERE, "..", "gpurun_out")
+    # registers / spills / shared memory per kernel: a build log beside the other build products, which are not tracked
+    log_dir = os.path.join(HERE, "..", "build")
     os.makedirs(log_dir, exist_ok=True)
     with open(os.path.join(log_dir, "ptxas_info.txt"), "w") as f:
         f.write(r.stdout + r.stderr)
