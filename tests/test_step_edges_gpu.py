@@ -214,3 +214,33 @@ def test_attention_tiles_of_the_gather(lens):
     be.launch_attend_simt_paged_bf16(g, *args, want, None, None, None)
     a, b = L.out.float(), want.float()
     assert bool(((a - b).abs() <= 2e-2 * b.abs().amax(dim=(1, 2), keepdim=True) + 1e-3).all()), (a - b).abs().max().item()
+
+
+@pytest.mark.parametrize("max_ctx", [16390, 131072, 131136])
+@pytest.mark.parametrize("name", ["all-below", "one-above", "short", "short-top-k", "not-short", "lone-cta", "cluster", "above-other-geometry"])
+def test_step_of_a_layer_built_for_far_longer_sequences(name, max_ctx):
+    """A layer is built for the longest sequence that a server admits, not for the batch at hand: the launch plans follow that
+    length (score rows that no 16-byte load fits, clusters most of whose CTAs have no token, score rows past what the tensor-core
+    scorer takes), the results do not."""
+    from rivoli_b200 import backend as be
+    from rivoli_b200.layer import DsaDecodeLayer
+    be.lib()
+    kw = dict(CASES[name])
+    lens = kw.pop("ctx_lens")
+    st = State(74, len(lens), lens, **kw)
+    g = make_geom(be.DsaGeom, **dict(st.geom_kw, max_pages_per_seq=-(-max_ctx // st.geom_kw["page_tokens"])))
+    L = DsaDecodeLayer(g, st.B, max_ctx=max_ctx)
+    for k in ("latent_pool", "latent_scale", "index_pool", "index_scale"):
+        getattr(L, k).copy_(dev(getattr(st, k)).view(getattr(L, k).shape))
+    L.block_table[:, :st.block_table.shape[1]] = dev(st.block_table)
+    out = _step(L, st)
+    be.device_sync(); L.check_status()
+    want = st.oracle_step()
+    n_sel = L.n_sel.cpu().numpy()
+    np.testing.assert_array_equal(n_sel, want["n_sel"])
+    for b in range(st.B):
+        np.testing.assert_array_equal(L.rows[b, :n_sel[b]].cpu().numpy().view(np.uint32), want["rows"][b, :n_sel[b]])
+    for k in ("latent_pool", "latent_scale", "index_pool", "index_scale"):
+        np.testing.assert_array_equal(getattr(L, k).cpu().numpy().ravel().view(np.uint8), want[k].ravel().view(np.uint8))
+    ok, worst, rms = attend_close_ref(out.view(torch.int16).cpu().numpy().view(np.uint16).reshape(want["out_f32"].shape), want["out_f32"])
+    assert ok and rms <= 1e-2, (worst, rms)
