@@ -75,15 +75,15 @@ struct KpArgs {
     uint16_t* out;
 };
 
-// The contraction in chunks of 64, one cp.async group each (activations, raw codes), requested ahead: all of them in the absorb
-// kernel, three in the value kernel. A chunk's codes are converted (two tile buffers) and its MMAs issued while later chunks are
-// on their way. The result is staged in the idle converted tiles and leaves as whole rows.
+// The contraction in chunks of 64, one cp.async group each (activations, raw codes), all requested ahead. A chunk's codes are
+// converted (two tile buffers) and its MMAs issued while later chunks are on their way; they stay for the next batch tile. The
+// result is staged in the idle converted tiles and leaves as whole rows.
 // 128 sequences, us: absorb 16.4 -> 8.6, value 15.9 -> 9.7 (loads into registers, one conversion pass, two halves of the
 // value contraction one after the other, 16-byte stores to 32 rows at a time); bound by what an SM takes in
-// (192 KiB at 18 bytes a clock in the value kernel), a launch's ramp and the epilogue. With all eight chunks in flight (224 KiB)
-// a value CTA could not start before both absorb CTAs had left its SM: 48.9 -> 47.3 us for the three projection operators.
+// (192 KiB at 18 bytes a clock in the value kernel), a launch's ramp and the epilogue. Three chunks of the value contraction in
+// flight, with which a value CTA can start beside an absorb CTA, are slower in every order of the launches: absorb and value of
+// 128 / 8 sequences back to back 18.2 / 16.2 us, 17.5 / 15.4 so; with a layer's attention between them 88.5 / 38.0 and 87.3 / 36.9.
 constexpr int KP_ACHUNK = 16384, KP_WCHUNK = 8192, KP_CONV = 16384;
-constexpr int KP_VST = 3;      // chunks in flight in the value kernel
 static_assert(2 * KP_CONV == 128 * 256, "the result fits the converted tiles");
 
 // Requests activation chunk c (128 sequences from b0 x 64 bf16, swizzled K-major; rows past B are zeros) into `dst`.
@@ -111,8 +111,8 @@ __device__ __forceinline__ void kp_convert16(const uint8_t* raw, uint8_t* d0, ui
     *reinterpret_cast<uint4*>(d0) = kp_codes_to_bf16(make_uint2(v.x, v.y));
     *reinterpret_cast<uint4*>(d1) = kp_codes_to_bf16(make_uint2(v.z, v.w));
 }
+constexpr int KP_ACHUNKS = 4, KP_VCHUNKS = 8;      // most chunks of a contraction (rivoli_kvb_mma_supported: nope <= 256, kvl <= 512)
 // Waits until at most `left` of this thread's copy groups are pending (left < KP_ACHUNKS).
-constexpr int KP_ACHUNKS = 4;      // most chunks of the absorb contraction (rivoli_kvb_mma_supported: nope <= 256)
 __device__ __forceinline__ void kp_wait_groups(int left) {
     switch (left) {
         case 0: tc::cp_async_wait<0>(); break;
@@ -166,7 +166,7 @@ kvb_absorb_mma_kernel(KpArgs A) {
     __syncthreads();
     tc::tc_fence_after();
     // Behind the allocation, which waits for its columns without a limit: a dependent that is already on the SM could take them
-    // and then wait for this grid (the value kernel, which takes all of them, does start beside a CTA of this one).
+    // and then wait for this grid.
     rv_grid_dep_trigger();
     rv_grid_dep_wait();
     if (warp < 8) for (int c = 0; c < nch; ++c) {
@@ -278,8 +278,8 @@ kvb_absorb_mma_kernel(KpArgs A) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// value: grid (vh / 128, H), N = 128 value rows = two 64-row scale rows. Shared: activation chunks [3][128 rows][128 B] |
-// raw codes [3][128 rows][64 B] | two converted tiles [128 rows][128 B] (K-major).
+// value: grid (vh / 128, H), N = 128 value rows = two 64-row scale rows. Shared: activation chunks [kvl/64][128 rows][128 B] |
+// raw codes [kvl/64][128 rows][64 B] (room for eight of each) | two converted tiles [128 rows][128 B] (K-major).
 // TMEM: one 128-column accumulator per scale column (kvl / 128 <= 4 runs).
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(KP_LAUNCH)
@@ -294,8 +294,8 @@ kvb_value_mma_kernel(KpArgs A) {
     const int jblk = blockIdx.x, h = blockIdx.y;
     const int kvl = A.kvl, vh = A.vh, nch = kvl / 64;
     uint8_t* sA = smem;
-    uint8_t* sW = sA + KP_VST * KP_ACHUNK;
-    uint8_t* sB = sW + KP_VST * KP_WCHUNK;
+    uint8_t* sW = sA + KP_VCHUNKS * KP_ACHUNK;
+    uint8_t* sB = sW + KP_VCHUNKS * KP_WCHUNK;
     const size_t row0 = (size_t)h * (A.nope + vh) + A.nope + (size_t)jblk * 128;   // 128 value rows = 2 scale rows
     const int sc_cols = kvl / 128;
     if (tid == 0) {
@@ -311,21 +311,20 @@ kvb_value_mma_kernel(KpArgs A) {
     tc::tc_fence_after();
     rv_grid_dep_trigger();   // (behind the allocation: see the absorb kernel)
     rv_grid_dep_wait();
-    auto request = [&](int b0, int c) {   // one cp.async group per call, with or without a chunk
-        if (c < nch) {
-            const int st = c % KP_VST;
-            kp_request_acts(A, h, b0, c, sA + st * KP_ACHUNK);
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const int e = tid + i * KP_THREADS, r = e >> 2, j = e & 3;
-                tc::cp_async16(tc::smem_u32(sW + st * KP_WCHUNK + r * 64 + j * 16), A.kvb + (row0 + r) * kvl + c * 64 + j * 16);
-            }
-        }
-        tc::cp_async_commit();
-    };
+    // (a group per chunk that there could be, so that the waits below have constant counts)
     if (warp < 8)
 #pragma unroll 1
-        for (int c = 0; c < KP_VST; ++c) request(0, c);
+        for (int c = 0; c < KP_VCHUNKS; ++c) {
+            if (c < nch) {
+                kp_request_acts(A, h, 0, c, sA + c * KP_ACHUNK);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int e = tid + i * KP_THREADS, r = e >> 2, j = e & 3;
+                    tc::cp_async16(tc::smem_u32(sW + c * KP_WCHUNK + r * 64 + j * 16), A.kvb + (row0 + r) * kvl + c * 64 + j * 16);
+                }
+            }
+            tc::cp_async_commit();
+        }
     if (tid < 2 * sc_cols) s_sc[tid / sc_cols][tid % sc_cols] = A.scale[((row0 + (tid / sc_cols) * 64) >> 7) * sc_cols + tid % sc_cols];
     __syncthreads();
     const uint32_t tmem = tmem_slot;
@@ -341,7 +340,7 @@ kvb_value_mma_kernel(KpArgs A) {
                 ok = tc::mbar_wait_warp(&full[wb], done[wb]++ & 1, abort_flag, 76);
                 if (!ok) break;
                 tc::tc_fence_after();
-                const uint64_t da = kp_desc(tc::smem_u32(sA + (c % KP_VST) * KP_ACHUNK), 16, 1024), db = kp_desc(tc::smem_u32(sB + wb * KP_CONV), 16, 1024);
+                const uint64_t da = kp_desc(tc::smem_u32(sA + c * KP_ACHUNK), 16, 1024), db = kp_desc(tc::smem_u32(sB + wb * KP_CONV), 16, 1024);
                 if (tc::elect_one()) {
 #pragma unroll
                     for (int k = 0; k < 4; ++k) kp_mma(tmem + (c >> 1) * 128, da + 2 * k, db + 2 * k, idesc, ((c & 1) | k) ? 1u : 0u);
@@ -354,18 +353,21 @@ kvb_value_mma_kernel(KpArgs A) {
             continue;
         }
         if (b0 > 0)
-            for (int c = 0; c < KP_VST; ++c) request(b0, c);
+            for (int c = 0; c < KP_VCHUNKS; ++c) {
+                if (c < nch) kp_request_acts(A, h, b0, c, sA + c * KP_ACHUNK);
+                tc::cp_async_commit();
+            }
         for (int c = 0; c < nch && ok; ++c) {
             const int wb = c & 1;
             if (done[wb] > 0) ok = tc::mbar_wait_warp(&bar[wb], (done[wb] - 1) & 1, abort_flag, 73);
             if (!ok) break;
-            if (c >= 2) request(b0, c - 2 + KP_VST);   // the stage that the MMAs of chunk c - 2 have read
-            if (c == 0) tc::cp_async_wait<KP_VST - 1>(); else tc::cp_async_wait<KP_VST - 2>();   // (a thread converts the codes that it requested itself)
+            if (c > 0) tc::cp_async_commit();             // (empty: the group of chunk c stays KP_VCHUNKS - 1 from the newest)
+            tc::cp_async_wait<KP_VCHUNKS - 1>();          // (a thread converts the codes that it requested itself)
             uint8_t* sb = sB + wb * KP_CONV;
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const int e = tid + i * KP_THREADS, r = e >> 2, j = e & 3;
-                kp_convert16(sW + (c % KP_VST) * KP_WCHUNK + r * 64 + j * 16, sb + tc::sw128_chunk(r, 2 * j), sb + tc::sw128_chunk(r, 2 * j + 1));
+                kp_convert16(sW + c * KP_WCHUNK + r * 64 + j * 16, sb + tc::sw128_chunk(r, 2 * j), sb + tc::sw128_chunk(r, 2 * j + 1));
             }
             tc::fence_proxy_async();
             tc::mbar_arrive(&full[wb]);
@@ -418,7 +420,7 @@ kvb_value_mma_kernel(KpArgs A) {
 // whose rows straddle at most one block boundary; vh a multiple of 128; the head's row count a multiple
 // of 64; 16-byte aligned activation rows; rope <= 64.
 extern "C" int rivoli_kvb_mma_supported(int H, int qh, int nope, int vh, int kvl, int rope, int block) {
-    if (block != 128 || kvl % 256 || kvl > 512 || nope % 64 || nope > KP_ACHUNKS * 64 || vh % 128 || (nope + vh) % 64) return 0;
+    if (block != 128 || kvl % 256 || kvl > KP_VCHUNKS * 64 || nope % 64 || nope > KP_ACHUNKS * 64 || vh % 128 || (nope + vh) % 64) return 0;
     if (qh % 8 || rope % 8 || rope > 64 || H <= 0) return 0;
     for (int h = 0; h < 2 && h < H; ++h) {          // the straddle pattern repeats with period <= 2 heads
         const int off = (h * (nope + vh)) & 127;
@@ -440,8 +442,8 @@ extern "C" int rivoli_kvb_absorb_mma(const uint16_t* q, const uint8_t* kvb, cons
 extern "C" int rivoli_kvb_value_mma(const uint16_t* clat, const uint8_t* kvb, const float* scale, int H, int nope, int vh,
                                     int kvl, int block, int B, uint16_t* ctx, cudaStream_t st) {
     const KpArgs a{clat, kvb, scale, H, kvl, nope, vh, kvl, 0, block, B, ctx};
-    // beside one CTA of the absorb kernel, but never two on an SM (each takes all of its tensor memory)
-    constexpr int need = KP_VST * (KP_ACHUNK + KP_WCHUNK) + 2 * KP_CONV, smem = need > 116 * 1024 ? need : 116 * 1024;
+    // (never two on an SM: each takes all of its tensor memory)
+    constexpr int smem = KP_VCHUNKS * (KP_ACHUNK + KP_WCHUNK) + 2 * KP_CONV;
     rv_allow_smem<kvb_value_mma_kernel>(smem);
     rv_drain_error();
     rv_launch_dependent(kvb_value_mma_kernel, dim3(vh / 128, H), dim3(KP_LAUNCH), (size_t)smem, st, a);
