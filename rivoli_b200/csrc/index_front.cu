@@ -134,7 +134,7 @@ front_gemm_simt_kernel(FrontArgs A) {
 // 32 tiles) and the launch's ramp. 128 sequences: 19 us with three stages, two barriers a chunk and 16-byte stores to 32 rows
 // at a time, then 12.5 us for the epilogue below; 20.6 us together after that (31.8). The MMAs have a warp of their own: one of
 // the converting warps issued them between two chunks, behind a CTA barrier, 18.4 us together for one sequence; 17.3 now, and
-// 19.4 for 128.
+// 20 for 128 with cold weights.
 // ---------------------------------------------------------------------------------------------
 constexpr int FM_THREADS = 256;                             // warps 0-7 request, convert and store
 constexpr int FM_LAUNCH = FM_THREADS + 32;                  // warp 8 issues the MMAs

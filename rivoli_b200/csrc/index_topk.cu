@@ -5,7 +5,7 @@
 // reference's crates/backend/kernels/indexer.hip:143-257 and the host rule
 // crates/core/src/routing.rs:42-61 + sort (crates/engine/tests/kernel_vector.rs:126-131).
 //
-// Up to 131,072 scores the selection kernel of index_select.cu does it (keys in registers, one histogram pass linear in
+// Up to 131,072 scores the selection kernel of index_select.cu does it (keys in shared memory, one histogram pass linear in
 // value, only the k-th value's bin ranked). Longer rows take the kernel below: one CTA of 1024 threads per sequence, four
 // radix passes and a compaction sweep over global memory (L2 resident), any length.
 // Compaction uses ballots and a fixed scan order: no atomics decide an output slot.

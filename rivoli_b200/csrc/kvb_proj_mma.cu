@@ -78,9 +78,9 @@ struct KpArgs {
 // The contraction in chunks of 64, one cp.async group each (activations, raw codes), all requested ahead. A chunk's codes are
 // converted (two tile buffers) and its MMAs issued while later chunks are on their way; they stay for the next batch tile. The
 // result is staged in the idle converted tiles and leaves as whole rows.
-// 128 sequences, us: absorb 16.4 -> 8.6, value 15.9 -> 9.7 (loads into registers, one conversion pass, two halves of the
-// value contraction one after the other, 16-byte stores to 32 rows at a time); bound by what an SM takes in
-// (192 KiB at 18 bytes a clock in the value kernel), a launch's ramp and the epilogue. Three chunks of the value contraction in
+// 128 sequences, us, each behind itself with cold weights: absorb 16.4 -> 8.9, value 15.9 -> 9.9 (before: loads into registers,
+// one conversion pass, two halves of the value contraction one after the other, 16-byte stores to 32 rows at a time); bound by
+// what an SM takes in (192 KiB at 18 bytes a clock in the value kernel), a launch's ramp and the epilogue. Three chunks of the value contraction in
 // flight, with which a value CTA can start beside an absorb CTA, are slower in every order of the launches: absorb and value of
 // 128 / 8 sequences back to back 18.2 / 16.2 us, 17.5 / 15.4 so; with a layer's attention between them 88.5 / 38.0 and 87.3 / 36.9.
 constexpr int KP_ACHUNK = 16384, KP_WCHUNK = 8192, KP_CONV = 16384;

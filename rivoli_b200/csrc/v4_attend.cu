@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(GA_THREADS) v4_gather_attn_kernel(const T* __r
 // One CTA per sequence; a batch that leaves SMs idle gets a thread-block cluster per sequence (tiles split evenly, at most
 // eight CTAs), merged by pushing scaled O^T rows into the memory of the CTA that writes the head.
 // Bound by the rows an SM can take in (18 bytes a clock): 640 rows x 128 sequences 57 us with mma.sync (operand reloads from
-// shared memory), 33.2 us now; 3 sequences 55 us on three SMs, 14.0 us now.
+// shared memory), 29.7 us now; 3 sequences 55 us on three SMs, 12.9 us now.
 // All waits are bounded (tc_common.cuh); one that gives up makes the sequence's output NaN and sets g_sa_err.
 // ---------------------------------------------------------------------------------------------------
 constexpr int SA_H = 64, SA_D = 512, SA_TILE = 64;

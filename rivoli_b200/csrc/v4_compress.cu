@@ -186,14 +186,14 @@ __global__ void __launch_bounds__(CP_THREADS) cp_prefill_kernel(const float* __r
 }
 
 // The same for the overlapping ratio-4 compressor with d = 128, 256 or 512 (what both compressors of a layer are): eight
-// entries per block and feature, every projected value used exactly once, so HBM is the bound (8.8 bytes a value). A
-// thread owns two features of one block, d / 2 threads a block: its 8 scores and 8 values are all requested before the
-// first is used (128 bytes per thread; two features and not four, so that several CTAs share an SM: the exponentials of one
-// cover the loads of another); the maximum, the exponentials (one per entry instead of two) and the weighted sum run from
+// entries per block and feature, every projected value used exactly once (8.8 bytes a value): bound by HBM, 4.6 TB/s at
+// d 512, and the issue slots of the exponentials and quotients. A thread owns two features of one block, d / 2 threads a block:
+// its 8 scores and 8 values are all requested before the first is used (128 bytes per thread; two features and not four, so that
+// several CTAs share an SM: the exponentials of one cover the loads of another); the maximum, the exponentials (one per entry instead of two) and the weighted sum run from
 // registers. Values and their order are those of the kernel above and of the decode arms, the quotients and the norm's partial
 // sums included (a row meets in shared memory in the order of a 256-thread CTA): a block has the same bits whether it was
 // pooled from a prompt or token by token. (The sum divided once and the norm summed as the features lie would take 27.7 us
-// instead of 31 at 4,095 blocks of d 512, and land on other codes now and then.) The positional bias sits in shared memory for
+// instead of 30.9 at 4,095 blocks of d 512, and land on other codes now and then.) The positional bias sits in shared memory for
 // the CTA's walk over the grid's blocks. Three passes over global memory took 124 us; four CTAs per SM are 2.4 us faster than
 // five, at whose registers the quotients spill, and 11 faster than three.
 constexpr int CP4_THREADS = 256, CP4_CTAS = 4;

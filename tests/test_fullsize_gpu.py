@@ -147,7 +147,7 @@ def test_cfg2_dense_equivalent_shape():
 
 
 def test_selection_beyond_16384_tokens_uses_the_wide_kernel_and_stays_exact():
-    """Contexts in (16384, 32768] take the 32-keys-per-thread instantiation of the selection kernel: fused
+    """Contexts past the 16,384 tokens of one CTA of the selection kernel take a cluster at any batch: fused
     tensor-core selection == exact CUDA-core chain, bit for bit, on a ragged pair of long contexts."""
     import torch
     from rivoli_b200 import backend as be

@@ -119,7 +119,7 @@ def test_layer_step_matches_oracle(be, case):
             ok, worst = attend_close(u16(out), want["out_f32"])
             assert ok, worst
         assert np.abs(lse.cpu().numpy() - want["lse"]).max() < 2e-2
-        # no-scratch (single split) path
+        # the path without scratch (for the 64-head geometry: no tensor cores)
         out2 = torch.zeros_like(out)
         fn(g, dev(st.q), d["latent_pool"], d["latent_scale"], d["block_table"], rows, g.top_k, n_sel, B, out2,
            None, None, None)

@@ -2,11 +2,10 @@
 
 Some hosts of this library may not call cudaMalloc (all device memory already belongs to
 their own arenas, or their decode thread must never wait on the allocator), so
-``rivoli_mla_attend_static`` keeps the split-KV partials in an array compiled into the
-library instead of taking scratch from the caller. This file checks, through the C ABI, that
-it returns what ``rivoli_mla_attend`` returns with caller scratch - on two calls in a row with
-different inputs, because the built-in array keeps the previous call's partials - and that
-shapes beyond the built-in array are refused. Named so that pytest collects it last.
+``rivoli_mla_attend_static`` takes no scratch from the caller. This file checks, through the
+C ABI, that it returns what ``rivoli_mla_attend`` returns with caller scratch - on calls in a
+row with different inputs and numbers of splits - and that the shapes beyond its contract are
+refused. Named so that pytest collects it last.
 """
 import numpy as np
 import pytest
@@ -41,8 +40,8 @@ def _case(seed, H, nt, kvl, rope):
 def test_static_scratch_attend_matches_caller_scratch_attend():
     from rivoli_b200 import backend as be
     be.lib()
-    # two calls in a row: many splits first, then fewer splits with other data, so stale partials
-    # of the first call sit in the built-in array while the second runs
+    # calls in a row: many splits first, then fewer splits with other data, so that nothing of the
+    # first call may be left where the second merges
     for seed, H, nt in ((0xC1A39ED0, 64, 4608), (0x5F117BAD, 64, 704), (0xB10CC0DE, 20, 130)):
         c = _case(seed, H, nt, 512, 64)
         want = torch.zeros(H * 512, dtype=torch.float32, device="cuda")
@@ -68,7 +67,7 @@ def test_static_scratch_attend_matches_caller_scratch_attend():
 def test_static_scratch_attend_refuses_what_does_not_fit():
     from rivoli_b200 import backend as be
     b = torch.zeros(1 << 16, dtype=torch.float32, device="cuda")
-    for args, code in (((128, 16, 512, 64, 4), 1002),      # more heads than the built-in array holds
+    for args, code in (((128, 16, 512, 64, 4), 1002),      # more heads than the contract has
                        ((8, 16, 640, 64, 5), 1004),        # same width rule as rivoli_mla_attend
                        ((8, 0, 512, 64, 4), 1001)):
         H, nr, kvl, rope, nb = args
