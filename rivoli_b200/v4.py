@@ -104,13 +104,23 @@ class V4TokenStep:
             layer.packed = torch.zeros((layer.B, g.max_comp, 128), dtype=torch.uint8, device=dev)
             layer.packed_exp = torch.zeros((layer.B, g.max_comp), dtype=torch.int32, device=dev)
 
+    def _entry(self, kv_entry, stream):
+        """An entry that does not lie as the kernel reads it: any layout, and what broadcasts to [B, head_dim], copied in the order of
+        the launch's stream, which may not be the current one."""
+        cache = self.layer.kv_cache
+        if kv_entry.device != cache.device:
+            raise RuntimeError(f"kv_entry on {kv_entry.device}, the cache on {cache.device}")
+        with torch.cuda.stream(be.torch_stream(stream, cache.device)):
+            entry = torch.empty((self.layer.B, self.layer.g.head_dim), dtype=torch.int16, device=cache.device)
+            return entry.copy_(kv_entry.view(torch.int16))
+
     def __call__(self, pos, kv_entry, attn_proj, index_proj, q, index_q, index_w, stream=None):
         """pos i32 [B]; kv_entry bf16 bits [B, head_dim] (the token's window entry); attn_proj / index_proj =
         (kv_proj, score_proj) f32 [B, cd] of the two compressors; q, index_q, index_w as for V4DecodeLayer.step."""
         L, g = self.layer, self.layer.g
-        if not kv_entry.is_contiguous():        # copied in the order of the launch's stream, which may not be the current one
-            with torch.cuda.stream(be.torch_stream(stream, kv_entry.device)):
-                kv_entry = kv_entry.contiguous()
+        if not (kv_entry.is_contiguous() and kv_entry.shape == L.out.shape[::2] and kv_entry.element_size() == 2 and
+                kv_entry.get_device() == L.kv_cache.get_device()):
+            kv_entry = self._entry(kv_entry, stream)
         be.launch_v4_token_step_bf16(
             g, L.B, pos, kv_entry, self.attn_comp.p, self.attn_comp.step_args(*attn_proj, L.kv_cache, L.kv_rows, g.window),
             self.index_comp.p, self.index_comp.step_args(*index_proj, L.index_kv, g.max_comp, 0, L.packed, L.packed_exp),

@@ -256,3 +256,32 @@ def test_token_step_takes_a_strided_entry_in_the_order_of_its_stream(as_address)
     with torch.cuda.stream(side):
         got = layer.kv_cache.view(torch.int16)[torch.arange(b, device="cuda"), (pos % 8).long()].cpu()
     assert torch.equal(got, wide.view(torch.int16)[:, 1].cpu())
+
+
+def test_token_step_broadcasts_and_refuses_entries():
+    """An entry that broadcasts to [B, head_dim] is every sequence's; one of another size, width or device is refused, on the host."""
+    be = _be()
+    from rivoli_b200.v4 import V4Compressor, V4DecodeLayer, V4TokenStep
+    g, b = be.V4Geom.make(n_heads=4, max_comp=32, window=8, index_topk=8), 3
+    gen, rng = torch.Generator("cuda").manual_seed(0), np.random.default_rng(0)
+    f32 = lambda *s: torch.randn(s, generator=gen, device="cuda")
+    bf = lambda *s: f32(*s).to(torch.bfloat16)
+    layer, comps = V4DecodeLayer(g, b), []
+    for w, rotate in ((512, False), (128, True)):
+        p = be.CompGeom.make(ratio=4, d=w, rd=64)
+        norm, freqs, ape = _comp_fixture(rng, p, 64)
+        comps.append(V4Compressor(p, b, dev(ape), dev(norm), dev(freqs), rotate))
+    step = V4TokenStep(layer, *comps)
+    pos = torch.tensor([4, 9, 17], dtype=torch.int32, device="cuda")
+    x = ((f32(b, 1024), f32(b, 1024)), (f32(b, 256), f32(b, 256)), bf(b, 4, 512).view(torch.uint16), bf(b, 64, 128).view(torch.uint16), f32(b, 64))
+    ring = lambda: layer.kv_cache.view(torch.int16)[torch.arange(b, device="cuda"), (pos % 8).long()]
+    for entry in (bf(1, 512), bf(512), bf(512, 3).T, bf(3, 512), bf(3, 512).view(torch.uint16)):
+        step(pos, entry, *x)
+        torch.cuda.synchronize()
+        assert torch.equal(ring(), entry.view(torch.int16).expand(b, 512) if entry.stride(-1) == 1 else entry.contiguous().view(torch.int16))
+    before = layer.kv_cache.view(torch.int16).clone()
+    for entry in (bf(2, 512), bf(3, 256), bf(3, 513), f32(3, 512), bf(3, 512).cpu(), bf(1, 3, 512, 1)):
+        with pytest.raises(RuntimeError):
+            step(pos, entry, *x)
+    torch.cuda.synchronize()
+    assert torch.equal(layer.kv_cache.view(torch.int16), before)
