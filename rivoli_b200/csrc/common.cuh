@@ -52,17 +52,17 @@ static inline void rv_allow_smem(int bytes) {
         done.fetch_or(dev < 64 ? bit : 0, std::memory_order_release);
 }
 
-// SMs of the current device, asked once per device. (A plan that sizes memory which the caller lends must not depend on the
-// device: it takes RV_SMS, the SMs of a B200.)
+// SMs of a device, asked once: the devices of a process are taken to be alike (only how well a plan fits hangs on it, and asking
+// which one is current costs a call 0.15 us). A plan that sizes memory which the caller lends must not depend on the device at
+// all: it takes RV_SMS, the SMs of a B200.
 constexpr int RV_SMS = 148;
 static inline int rv_sm_count() {
-    static std::atomic<int> known[64];
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return RV_SMS;
-    n = known[dev].load(std::memory_order_relaxed);
+    static std::atomic<int> known{0};
+    int n = known.load(std::memory_order_relaxed), dev = 0;
     if (n) return n;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return RV_SMS;
-    known[dev].store(n, std::memory_order_relaxed);
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+        return RV_SMS;
+    known.store(n, std::memory_order_relaxed);
     return n;
 }
 #endif

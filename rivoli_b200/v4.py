@@ -99,6 +99,7 @@ class V4TokenStep:
     def __init__(self, layer: V4DecodeLayer, attn_comp: V4Compressor, index_comp: V4Compressor, pack_index: bool = True):
         self.layer, self.attn_comp, self.index_comp = layer, attn_comp, index_comp
         g = layer.g
+        self._entry_shape, self._device = torch.Size((layer.B, g.head_dim)), layer.kv_cache.get_device()
         if pack_index and g.index_dim == 128:
             dev = layer.index_kv.device
             layer.packed = torch.zeros((layer.B, g.max_comp, 128), dtype=torch.uint8, device=dev)
@@ -118,8 +119,8 @@ class V4TokenStep:
         """pos i32 [B]; kv_entry bf16 bits [B, head_dim] (the token's window entry); attn_proj / index_proj =
         (kv_proj, score_proj) f32 [B, cd] of the two compressors; q, index_q, index_w as for V4DecodeLayer.step."""
         L, g = self.layer, self.layer.g
-        if not (kv_entry.is_contiguous() and kv_entry.shape == L.out.shape[::2] and kv_entry.element_size() == 2 and
-                kv_entry.get_device() == L.kv_cache.get_device()):
+        if not (kv_entry.shape == self._entry_shape and kv_entry.is_contiguous() and kv_entry.element_size() == 2 and
+                kv_entry.get_device() == self._device):
             kv_entry = self._entry(kv_entry, stream)
         be.launch_v4_token_step_bf16(
             g, L.B, pos, kv_entry, self.attn_comp.p, self.attn_comp.step_args(*attn_proj, L.kv_cache, L.kv_rows, g.window),
