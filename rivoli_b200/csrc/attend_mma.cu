@@ -828,7 +828,10 @@ attend_mma_kernel(AttendMmaArgs A) {
 
     tc::tc_fence_before();
     __syncthreads();
-    if (warp == AM_QKW) tc::tmem_dealloc<512>(tmem);
+    if (warp == AM_QKW) {
+        tc::settle(*abort_flag);
+        tc::tmem_dealloc<512>(tmem);
+    }
     if (tid == 0 && *abort_flag) atomicCAS(A.err, 0, *abort_flag);
 }
 

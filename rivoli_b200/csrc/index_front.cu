@@ -324,7 +324,10 @@ front_gemm_mma_kernel(FrontArgs A) {
         }
         if (b0 + 128 < A.B) __syncthreads();                 // the stages are free for the next batch tile
     }
-    if (warp == 8) tc::tmem_dealloc<256>(tmem_slot);
+    if (warp == 8) {
+        tc::settle(abort_word);
+        tc::tmem_dealloc<256>(tmem_slot);
+    }
     if (tid == 0 && abort_word) atomicCAS(&g_front_err, 0, abort_word);
 }
 

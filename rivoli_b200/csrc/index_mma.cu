@@ -418,7 +418,10 @@ index_score_mma_kernel(IndexMmaArgs A, const __grid_constant__ CUtensorMap tm_ke
 
     tc::tc_fence_before();
     __syncthreads();
-    if (warp == 5) tc::tmem_dealloc<IM_NACC * 32>(tmem);
+    if (warp == 5) {
+        tc::settle(abort_flag);
+        tc::tmem_dealloc<IM_NACC * 32>(tmem);
+    }
     if (tid == 0 && abort_flag) atomicCAS(A.err, 0, abort_flag);
 }
 

@@ -273,7 +273,10 @@ kvb_absorb_mma_kernel(KpArgs A) {
         __syncthreads();   // TMEM and the A tiles are free for the next batch tile
     }
     tc::cp_async_wait<0>();
-    if (warp == 8) tc::tmem_dealloc<256>(tmem);
+    if (warp == 8) {
+        tc::settle(abort_word);
+        tc::tmem_dealloc<256>(tmem);
+    }
     if (tid == 0 && abort_word) atomicCAS(&g_kp_err, 0, abort_word);
 }
 
@@ -410,7 +413,10 @@ kvb_value_mma_kernel(KpArgs A) {
         __syncthreads();
     }
     tc::cp_async_wait<0>();
-    if (warp == 8) tc::tmem_dealloc<512>(tmem);
+    if (warp == 8) {
+        tc::settle(abort_word);
+        tc::tmem_dealloc<512>(tmem);
+    }
     if (tid == 0 && abort_word) atomicCAS(&g_kp_err, 0, abort_word);
 }
 

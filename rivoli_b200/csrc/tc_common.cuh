@@ -159,6 +159,12 @@ template <int NCOLS>
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr) {  // one full warp
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "n"(NCOLS) : "memory");
 }
+// Before a CTA that gave up on a wait returns: what it has issued (copies into its shared memory, MMAs) lands first. Nothing of it
+// takes more than microseconds; there may be no barrier left that would tell, so a fifth of a millisecond is waited.
+__device__ __forceinline__ void settle(int gave_up) {
+    if (gave_up)
+        for (int i = 0; i < 100; ++i) __nanosleep(2000);
+}
 // 32 lanes x 32 consecutive 32-bit columns: thread i of the warp gets lane (base_lane + i).
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "

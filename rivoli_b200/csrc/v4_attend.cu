@@ -506,7 +506,10 @@ __global__ void __launch_bounds__(SA_THREADS, 1) v4_sparse_attend_kernel(SaArgs 
     }
     tc::tc_fence_before();
     __syncthreads();
-    if (warp == SA_QKW) tc::tmem_dealloc<512>(tmem);
+    if (warp == SA_QKW) {
+        tc::settle(*abort_flag);
+        tc::tmem_dealloc<512>(tmem);
+    }
     if (tid == 0 && *abort_flag) atomicCAS(&g_sa_err, 0, *abort_flag);
 }
 

@@ -562,7 +562,10 @@ __global__ void __launch_bounds__(ST_THREADS) v4_score_tc_kernel(StArgs A, const
     }
     tc::tc_fence_before();
     __syncthreads();
-    if (warp == 5) tc::tmem_dealloc<ST_NACC * 64>(tmem);
+    if (warp == 5) {
+        tc::settle(abort_flag);
+        tc::tmem_dealloc<ST_NACC * 64>(tmem);
+    }
     if (tid == 0 && abort_flag) atomicCAS(&g_v4_score_err, 0, abort_flag);
 }
 

@@ -60,6 +60,14 @@ def test_dependents_start_behind_the_allocation(path):
             assert alloc < between < trigger
 
 
+@pytest.mark.parametrize("path", SOURCES, ids=os.path.basename)
+def test_a_kernel_that_gave_up_lets_its_copies_land(path):
+    """Copies into shared memory and MMAs that are still on their way would land in whatever CTA comes next."""
+    for k in kernels(code(path)):
+        for at in (m.start() for m in re.finditer("tmem_dealloc", k)):
+            assert re.search(r"settle\([^)]*\);\s*tc::$", k[:at])
+
+
 BARRIER = re.compile(r"__syncthreads|named_barrier|barrier_any|give_up|bar\.red|bar\.sync")
 LOOP = re.compile(r"\b(?:for|while)\s*\(")
 
