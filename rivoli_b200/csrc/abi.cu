@@ -15,7 +15,9 @@ extern "C" int rivoli_attend_mma_paged_bf16(const DsaGeom* g, const uint16_t* q,
                                             const float* latent_scale, const int32_t* block_table,
                                             const uint32_t* rows, int row_stride, const int32_t* n_rows, int B,
                                             uint16_t* out, float* out_m, float* out_lse, void* scratch,
-                                            int q_early, int min_rows_hint, long long max_rows, void* stream);
+                                            int q_early, int min_rows_hint, long long max_rows, const int32_t* fresh_pos,
+                                            const int32_t* dense_len, void* stream);
+extern "C" bool rivoli_index_select_takes_all(const DsaGeom* g, int score_stride);
 extern "C" int rivoli_attend_mma_status(void* scratch, void* stream);
 
 // The error word of the tensor-core kernel, for any geometry and batch: all partial results are merged on the chip.
@@ -52,7 +54,8 @@ RIVOLI_API void rivoli_dsa_step_set_timing_events(void* const* events) {
 static int attend_paged_dispatch(const DsaGeom* g, const uint16_t* q, const uint8_t* latent_pool,
                                  const float* latent_scale, const int32_t* block_table, const uint32_t* rows,
                                  int row_stride, const int32_t* n_rows, int B, uint16_t* out, float* out_m,
-                                 float* out_lse, void* scratch, int q_early, int min_rows_hint, long long max_rows, void* stream) {
+                                 float* out_lse, void* scratch, int q_early, int min_rows_hint, long long max_rows,
+                                 const int32_t* fresh_pos, const int32_t* dense_len, void* stream) {
     if (int e = rv_check_geom(g)) return e;
     if (B <= 0 || !q || !latent_pool || !latent_scale || !block_table || !n_rows || !out) return 1001;
     if (rows && row_stride <= 0) return 1001;
@@ -60,7 +63,7 @@ static int attend_paged_dispatch(const DsaGeom* g, const uint16_t* q, const uint
     // Every other geometry runs on the CUDA-core kernel.
     if (scratch && rivoli_attend_mma_supported(g))
         return rivoli_attend_mma_paged_bf16(g, q, latent_pool, latent_scale, block_table, rows, row_stride, n_rows,
-                                            B, out, out_m, out_lse, scratch, q_early, min_rows_hint, max_rows, stream);
+                                            B, out, out_m, out_lse, scratch, q_early, min_rows_hint, max_rows, fresh_pos, dense_len, stream);
     return rivoli_attend_simt_paged_bf16(g, q, latent_pool, latent_scale, block_table, rows, row_stride,
                                          n_rows, B, out, out_m, out_lse, scratch, stream);
 }
@@ -73,7 +76,7 @@ RIVOLI_API int rivoli_mla_attend_paged_bf16(const DsaGeom* g, const uint16_t* q,
     // q may have been written by the kernel launched just before this call: the attention kernel reads it
     // only after its dependency wait.
     return attend_paged_dispatch(g, q, latent_pool, latent_scale, block_table, rows, row_stride, n_rows, B, out, out_m,
-                                 out_lse, scratch, 0, 0, 0x7fffffff, stream);
+                                 out_lse, scratch, 0, 0, 0x7fffffff, nullptr, nullptr, stream);
 }
 
 // One decode layer-step in one call: append the step's token of every sequence, select the attended rows,
@@ -95,8 +98,11 @@ RIVOLI_API int rivoli_dsa_decode_step_paged(const DsaGeom* g, const uint16_t* la
                                                rows, n_sel, select_scratch, stream))
         return e;
     rv_stage_event(3, (cudaStream_t)stream);
+    // where everything is selected, only the appended rows are new to the attention
+    const bool all = rivoli_index_select_takes_all(g, score_stride);
     const int e = attend_paged_dispatch(g, q, latent_pool, latent_scale, block_table, rows, g->top_k, n_sel, B, out, out_m,
-                                        out_lse, attend_scratch, 1, min_rows_hint, score_stride < g->top_k ? score_stride : g->top_k, stream);
+                                        out_lse, attend_scratch, 1, min_rows_hint, score_stride < g->top_k ? score_stride : g->top_k,
+                                        all ? row_pos : nullptr, all ? seq_len : nullptr, stream);
     rv_stage_event(4, (cudaStream_t)stream);
     return e;
 }
@@ -114,7 +120,7 @@ RIVOLI_API int rivoli_dsa_append_attend_paged(const DsaGeom* g, const uint16_t* 
                                        index_pool, index_scale, status, stream))
         return e;
     return attend_paged_dispatch(g, q, latent_pool, latent_scale, block_table, rows, row_stride, n_rows, B, out, out_m,
-                                 out_lse, attend_scratch, 1, min_rows_hint, 0x7fffffff, stream);
+                                 out_lse, attend_scratch, 1, min_rows_hint, 0x7fffffff, row_pos, nullptr, stream);
 }
 
 // out[v] = sum_g w_g * part_out[g][v] / sum_g w_g,  w_g = exp(lse_g - max_g lse), ascending g.

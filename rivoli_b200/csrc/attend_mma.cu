@@ -32,11 +32,14 @@
 // A softmax thread is one TMEM lane = one virtual head, and the q rows are ordered so that the hi and lo terms of a
 // head sit 16 lanes apart in the SAME warp: lanes 0-15 of warp s hold the hi rows of heads 16 s .. 16 s + 15, lanes
 // 16-31 their lo rows. One shuffle per score adds the two terms and leaves each lane with HALF the tokens of its
-// head: thread = (head, 16 tokens of the tile), two warps per lane quarter take the two 32-token halves. A head's
-// reference maximum, its running sum and its q scale are registers, and P' leaves as one 16-byte store per term
-// (heads are the rows of the K-major P' operand, tokens its bytes).
+// head: thread = (head, 32 tokens of the tile). Two groups of four warps take the tiles in turn. A head's
+// running sum and its q scale are registers, its reference maximum is handed from tile to tile through shared memory, and P'
+// leaves as 16-byte stores (heads are the rows of the K-major P' operand, tokens its bytes).
 // q arrives as bf16 (bulk copies) and is split into its two e4m3 terms by the softmax warps inside the kernel while the
 // first tiles are gathered; the output leaves through the idle ring as 8 KiB bulk copies.
+// Where only the step's new tokens can be changing under this kernel (a step that selects everything, a layer that shares a
+// selection), it gathers beside the append in front of it and waits only where it comes to a new token's row: 32 sequences of
+// 2,048 rows 28.3 -> 25.7 us a step, with the other changes noted below.
 // Online softmax with a LAGGING reference max: as long as no score of a tile exceeds its head's
 // reference by more than 3 (log2) the references stand (one barrier-with-OR per tile, no exchange);
 // otherwise the exact per-head maxima are taken and O is rescaled through TMEM. P' carries 2^5, so
@@ -44,14 +47,10 @@
 // A batch too small to fill the chip is split: the CTAs of a sequence form one thread-block cluster (up to 8), each takes
 // a contiguous range of tiles, and they merge their (maximum, sum, O) through distributed shared memory inside the kernel.
 // All waits are bounded (tc_common.cuh).
-#include <cooperative_groups.h>
-
 #include "codec.cuh"
 #include "common.cuh"
 #include "quant.cuh"
 #include "tc_common.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace {
 
@@ -60,6 +59,7 @@ constexpr int AM_STAGES = 6;             // K ring depth
 constexpr int AM_ROPES = 3;              // rope tiles: released right after the two rope MMAs of a tile, so fewer than stages
 constexpr int AM_SBUF = 2;               // S accumulators
 constexpr int AM_GW = 4;                 // gather warps
+constexpr int AM_JOINT = 8;              // a CTA of at most this many tiles has every tile filled by all gather warps
 constexpr int AM_H = 64, AM_KVL = 512, AM_ROPE = 64, AM_W = AM_KVL + AM_ROPE;
 constexpr int AM_SW = 8;                 // softmax + epilogue warps: TMEM lane quarter = warp % 4, token / head half = warp / 4
 constexpr int AM_HPT = 32;               // head columns of O^T a thread owns in the rescale and the epilogue
@@ -92,19 +92,20 @@ constexpr int SM_AHI = SM_TOK + 3 * SM_TOKPLANE;   // f32 [64] per-head q scale 
 constexpr int SM_WMAX = SM_AHI + 256;    // f32 [2][64] exchange between the two token halves
 constexpr int SM_FAC = SM_WMAX + 512;    // f32 [64] rescale factor of the current tile; 1 / l in the epilogue
 constexpr int SM_BARS = SM_FAC + 256;    // mbarriers
-constexpr int SM_MISC = SM_BARS + 256;
-constexpr int SM_XS = SM_MISC + 64;      // f32 [2][64]: this CTA's reference maximum and weight sum per head, read by its cluster
-constexpr int SM_TOTAL = SM_XS + 512;
-constexpr int SM_ZQ = SM_K0 + 3 * SM_KSTAGE;   // q as it arrives, then its codes: ring stages 3 .. 5 before their first tile
-static_assert(SM_ZQ + AM_H * AM_W * 2 <= SM_K0 + AM_STAGES * SM_KSTAGE, "q fits the last stages");
+constexpr int SM_MISC = SM_BARS + 320;
+constexpr int SM_MREF = SM_MISC + 64;   // f32 [64] reference maximum per head, as the last tile decided it
+constexpr int SM_TOTAL = SM_MREF + 256;
+constexpr int SM_ZQ = SM_K0 + 3 * SM_KSTAGE;   // q as it arrives: ring stages 3 .. 5 before their first tile
+constexpr int SM_ZROW = AM_W * 2 + 16;
+static_assert(SM_ZQ + AM_H * SM_ZROW <= SM_K0 + AM_STAGES * SM_KSTAGE, "q fits the last stages");
 constexpr int SM_STAGE = SM_K0;          // epilogue (the ring is idle by then): bf16 [64 heads][512 dims], or f32 [splits][heads][512 dims] received from the cluster
 static_assert((AM_H + AM_MAX_SPLITS) * AM_KVL * 4 <= AM_STAGES * SM_KSTAGE, "the O staging fits the ring");
 
 struct AmBars {
     uint64_t k_full[AM_STAGES], k_empty[AM_STAGES], s_full[AM_SBUF], s_empty[AM_SBUF], rope_free[AM_ROPES],
-        p_full, pv_done, q_full, q_raw[AM_SW];
+        p_full, pv_done[2], dec[2], q_full, q_raw[4];
 };
-static_assert(sizeof(AmBars) <= 256, "barrier block");
+static_assert(sizeof(AmBars) <= 320, "barrier block");
 static_assert(SM_TOTAL <= 232448, "shared memory budget");
 static_assert(SM_QR % 1024 == 0 && SM_P % 1024 == 0 && SM_ROPE % 1024 == 0, "operand tiles are 1024-byte aligned");
 
@@ -120,6 +121,10 @@ struct AttendMmaArgs {
     int min_rows;      // sequences with 0 < n_rows < min_rows are served by the CUDA-core kernel of the same call
     int q_early;       // 1: q was complete before the preceding kernel was launched, so it may be read before the grid-dependency wait
     int max_polls;     // poll limit of every bounded wait
+    // The token of sequence b' at fresh_pos[b'], b' < n_fresh, is appended by the kernel before this one; all else that this one reads
+    // was complete before that kernel started, so that its rows may be fetched beside it. NULL: no such promise.
+    const int32_t* fresh_pos; int n_fresh;
+    int row_cap;       // most rows of a sequence without a row list (beside its page table)
     int withhold;      // self-test: one gather warp never signals its part of the first tile (the waits on it must run out cleanly)
 };
 
@@ -135,10 +140,6 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo_bytes
     return d;
 }
 
-// Byte offset of 16-byte piece `c` of head h in the staging of q: pieces 0 .. 35 the hi codes, 36 .. 71 the lo codes; the
-// eight pieces of a 128-byte block are permuted by the head, so that the rows of eight heads lie in different banks.
-__device__ __forceinline__ uint32_t zq_chunk(int h, int c) { return (uint32_t)(((h * 72 + c) ^ (h & 7)) << 4); }
-
 // ---------------------------------------------------------------------------------------------
 // main kernel
 // ---------------------------------------------------------------------------------------------
@@ -150,6 +151,7 @@ attend_mma_kernel(AttendMmaArgs A) {
     float* s_ahi = reinterpret_cast<float*>(smem + SM_AHI);
     float* s_wmax = reinterpret_cast<float*>(smem + SM_WMAX);
     float* s_fac = reinterpret_cast<float*>(smem + SM_FAC);
+    float* s_mref = reinterpret_cast<float*>(smem + SM_MREF);
     uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(smem + SM_MISC);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SM_MISC + 4);
 
@@ -161,17 +163,19 @@ attend_mma_kernel(AttendMmaArgs A) {
 #pragma unroll
         for (int s = 0; s < AM_STAGES; ++s) { tc::mbar_init(&bars.k_full[s], AM_GW * (32 + 1)); tc::mbar_init(&bars.k_empty[s], 1); }
 #pragma unroll
-        for (int s = 0; s < AM_SBUF; ++s) { tc::mbar_init(&bars.s_full[s], 1); tc::mbar_init(&bars.s_empty[s], AM_SW); }
+        for (int s = 0; s < AM_SBUF; ++s) { tc::mbar_init(&bars.s_full[s], 2); tc::mbar_init(&bars.s_empty[s], AM_SW / 2); }
 #pragma unroll
         for (int s = 0; s < AM_ROPES; ++s) tc::mbar_init(&bars.rope_free[s], 1);
-        tc::mbar_init(&bars.p_full, AM_SOFTMAX_THREADS);
-        tc::mbar_init(&bars.pv_done, 1);
+        tc::mbar_init(&bars.p_full, AM_SOFTMAX_THREADS / 2);
+#pragma unroll
+        for (int s = 0; s < 2; ++s) { tc::mbar_init(&bars.pv_done[s], 1); tc::mbar_init(&bars.dec[s], AM_SW / 2); }
         tc::mbar_init(&bars.q_full, AM_SOFTMAX_THREADS);
 #pragma unroll
-        for (int s = 0; s < AM_SW; ++s) tc::mbar_init(&bars.q_raw[s], 1);
+        for (int s = 0; s < 4; ++s) tc::mbar_init(&bars.q_raw[s], 1);
         tc::mbar_init_fence();
         *abort_flag = 0;
     }
+    if (tid < AM_H) s_mref[tid] = -INFINITY;
     if (warp == AM_QKW) tc::tmem_alloc<512>(tmem_base_s);
 
     tc::fence_proxy_async();
@@ -185,14 +189,13 @@ attend_mma_kernel(AttendMmaArgs A) {
     //   hi = e4m3(q / s), s = absmax / 448;  lo = e4m3(q / s - hi)   =>  q ~ s * (hi + lo)
     // (the residual of a value of typical size is a normal e4m3 number; below 2^-6 it is kept to 2^-10 absolute,
     // 2^-19 of the head's largest value).
-    // The sequence's 72 KiB of q arrive as one bulk copy per softmax warp in ring stages 3 to 5, which the gather leaves alone until q_full.
-    // A warp converts eight heads, lanes along a head's row, and writes a head's hi row and lo row over the bf16 row it
-    // read (576 + 576 bytes = 1,152); 16-byte pieces are XOR-swizzled by head. Then a thread moves the row of its OWN
-    // tensor-memory lane (lane l of warp w is the virtual head (16 (w % 4) + l % 16, term l / 16), w / 4 the half of the 512
-    // latent columns): 16 conflict-free 16-byte loads, two tcgen05.st; column c = codes 4c .. 4c + 3, lowest byte first,
-    // which is the layout the MMA expects of an 8-bit A operand; the rope codes go to the shared operand tile.
-    // (A thread per row with 16-byte loads of its own row from global memory took 16,400 cycles at batch 148, 11,000 now, of
-    // which the copy is 3,200.)
+    // The sequence's 72 KiB of q arrive as one bulk copy per head in ring stages 3 to 5, which the gather leaves alone until q_full;
+    // a head's row is 16 bytes longer there than its 1,152, so that the rows of eight heads lie in different banks.
+    // Lane l of warp w converts the values of head 16 (w % 4) + l % 16 that the half w / 4 of the row has on its side l / 16: 128
+    // latent and 16 rope values, both terms; one shuffle a word then gives each lane one term of both sides, which is a run of
+    // the row of its OWN tensor-memory lane (virtual head): column c = codes 4c .. 4c + 3, lowest byte first, which is the
+    // layout the MMA expects of an 8-bit A operand. The rope codes go to the shared operand tile.
+    // (Converted a row per warp, staged in shared memory and read back by the rows' lanes it took 6,800 cycles behind the copy.)
     // The QK issuer waits for q_full before its first MMA.
     // Under a programmatic dependent launch the kernel before this one may still be running. Unless the
     // caller vouches that q was complete before that kernel was even launched (q_early: the fused decode
@@ -201,16 +204,33 @@ attend_mma_kernel(AttendMmaArgs A) {
     if (!A.q_early) rv_grid_dep_wait();
     if (warp < AM_SW) {
         uint8_t* zq = smem + SM_ZQ;
-        constexpr uint32_t part = AM_H / AM_SW * AM_W * 2;   // a warp's eight heads: it starts when they are there
-        if (lane == 0) {
-            tc::mbar_arrive_expect_tx(&bars.q_raw[warp], part);
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                         ::"r"(tc::smem_u32(zq + warp * part)), "l"(A.q + ((size_t)b * AM_H + warp * (AM_H / AM_SW)) * AM_W), "r"(part), "r"(tc::smem_u32(&bars.q_raw[warp])) : "memory");
+        const int sq = warp & 3, half = warp >> 2, term = lane >> 4, h = 16 * sq + (lane & 15);
+        if (half == 0) {
+            if (lane == 0) tc::mbar_arrive_expect_tx(&bars.q_raw[sq], 16 * AM_W * 2);
+            __syncwarp();
+            if (lane < 16)
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                             ::"r"(tc::smem_u32(zq + h * SM_ZROW)), "l"(A.q + ((size_t)b * AM_H + h) * AM_W), "r"(AM_W * 2), "r"(tc::smem_u32(&bars.q_raw[sq])) : "memory");
+            __syncwarp();
         }
-        __syncwarp();
-        tc::mbar_wait_warp(&bars.q_raw[warp], 0, abort_flag, 55, A.max_polls);
+        tc::mbar_wait_warp(&bars.q_raw[sq], 0, abort_flag, 55, A.max_polls);
+        const uint4* src = reinterpret_cast<const uint4*>(zq + h * SM_ZROW + half * AM_KVL + term * (AM_KVL / 2));
+        const uint4* rsrc = reinterpret_cast<const uint4*>(zq + h * SM_ZROW + AM_KVL * 2 + half * AM_ROPE + term * (AM_ROPE / 2));
+        float inv;
+        {
+            uint32_t m = rv_max_bf16x2(rv_absmax8(rsrc[0]), rv_absmax8(rsrc[1]));
+#pragma unroll 4
+            for (int c = 0; c < 16; ++c) m = rv_max_bf16x2(m, rv_absmax8(src[c]));
+            m = rv_max_bf16x2(m, __shfl_xor_sync(0xffffffffu, m, 16));
+            if (term == 0) s_wmax[half * 64 + h] = __uint_as_float(m << 16);
+            tc::named_barrier(3, AM_SOFTMAX_THREADS);
+            const float amax = fmaxf(s_wmax[h], s_wmax[64 + h]);
+            const float sc = amax > 0.0f ? amax / 448.0f : 1.0f;
+            inv = 1.0f / sc;
+            if (half == 0 && term == 0) s_ahi[h] = sc * A.softmax_scale * 1.4426950408889634f;
+        }
         // 8 values -> their 8 hi codes and 8 lo codes
-        auto codes8 = [&](const uint4 v, float inv, uint2& hi, uint2& lo) {
+        auto codes8 = [&](const uint4 v, uint2& hi, uint2& lo) {
             const uint32_t ww[4] = {v.x, v.y, v.z, v.w};
             uint16_t ch[4], cl[4];
 #pragma unroll
@@ -223,73 +243,36 @@ attend_mma_kernel(AttendMmaArgs A) {
             hi = make_uint2((uint32_t)ch[0] | ((uint32_t)ch[1] << 16), (uint32_t)ch[2] | ((uint32_t)ch[3] << 16));
             lo = make_uint2((uint32_t)cl[0] | ((uint32_t)cl[1] << 16), (uint32_t)cl[2] | ((uint32_t)cl[3] << 16));
         };
-        // the warp's eight absolute maxima together: three shuffles halve the eight values to one head per lane, two more
-        // finish it, and the divisions are done once, lane l for head l / 4
-        constexpr int HPW = AM_H / AM_SW;
-        static_assert(HPW == 8, "eight heads per warp");
-        const uint8_t* wq = zq + warp * HPW * (AM_W * 2);
-        float my_inv;
-        {
-            uint32_t m[HPW];
+        // a converted chunk -> this lane's term of the first and of the second side
+        auto exchange = [&](const uint2 hi, const uint2 lo, uint32_t* first, uint32_t* second) {
+            const uint2 keep = term ? lo : hi, give = term ? hi : lo;
+            const uint2 got = make_uint2(__shfl_xor_sync(0xffffffffu, give.x, 16), __shfl_xor_sync(0xffffffffu, give.y, 16));
+            first[0] = term ? got.x : keep.x; first[1] = term ? got.y : keep.y;
+            second[0] = term ? keep.x : got.x; second[1] = term ? keep.y : got.y;
+        };
+        const uint32_t dst = TM_Q + (((uint32_t)(sq * 32)) << 16) + half * 64;
+#pragma unroll 1
+        for (int g = 0; g < 4; ++g) {                  // (a loop: code that runs once is waited for)
+            uint32_t r0[8], r1[8];
 #pragma unroll
-            for (int i = 0; i < HPW; ++i) {
-                const uint4* src = reinterpret_cast<const uint4*>(wq + i * (AM_W * 2));
-                m[i] = rv_max_bf16x2(rv_absmax8(src[lane]), rv_absmax8(src[32 + lane]));
-                if (lane < 8) m[i] = rv_max_bf16x2(m[i], rv_absmax8(src[64 + lane]));
-            }
-#pragma unroll
-            for (int o = 16, n = HPW / 2; n > 0; o >>= 1, n >>= 1)
-#pragma unroll
-                for (int i = 0; i < n; ++i) {
-                    const bool up = lane & o;
-                    const uint32_t keep = up ? m[i + n] : m[i], give = up ? m[i] : m[i + n];
-                    m[i] = rv_max_bf16x2(keep, __shfl_xor_sync(0xffffffffu, give, o));
-                }
-            m[0] = rv_max_bf16x2(m[0], __shfl_xor_sync(0xffffffffu, m[0], 2));
-            m[0] = rv_max_bf16x2(m[0], __shfl_xor_sync(0xffffffffu, m[0], 1));
-            const float amax = __uint_as_float(m[0] << 16);
-            const float sc = amax > 0.0f ? amax / 448.0f : 1.0f;
-            my_inv = 1.0f / sc;
-            if ((lane & 3) == 0) s_ahi[warp * HPW + (lane >> 2)] = sc * A.softmax_scale * 1.4426950408889634f;
-        }
-#pragma unroll 2
-        for (int i = 0; i < HPW; ++i) {
-            const int h = warp * HPW + i;
-            const uint4* src = reinterpret_cast<const uint4*>(wq + i * (AM_W * 2));
-            uint4 v[3];
-            v[0] = src[lane]; v[1] = src[32 + lane];
-            v[2] = lane < 8 ? src[64 + lane] : make_uint4(0u, 0u, 0u, 0u);
-            const float inv = __shfl_sync(0xffffffffu, my_inv, 4 * i);
-            __syncwarp();                              // the whole row is in registers
-#pragma unroll
-            for (int u = 0; u < 3; ++u) {              // (lanes 8 .. 31 of the last pass convert zeros and store nothing)
+            for (int c = 0; c < 4; ++c) {
                 uint2 hi, lo;
-                codes8(v[u], inv, hi, lo);
-                const int vc = lane + 32 * u;
-                if (vc < AM_W / 8) {
-                    *reinterpret_cast<uint2*>(zq + zq_chunk(h, vc >> 1) + (vc & 1) * 8) = hi;
-                    *reinterpret_cast<uint2*>(zq + zq_chunk(h, AM_W / 16 + (vc >> 1)) + (vc & 1) * 8) = lo;
-                }
+                codes8(src[g * 4 + c], hi, lo);
+                exchange(hi, lo, r0 + 2 * c, r1 + 2 * c);
             }
+            tc::tmem_st8(dst + g * 8, r0);
+            tc::tmem_st8(dst + 32 + g * 8, r1);
         }
-        tc::named_barrier(3, AM_SOFTMAX_THREADS);
         {
-            const int sq = warp & 3, half = warp >> 2, term = lane >> 4, h = 16 * sq + (lane & 15);
-            const uint32_t dst = TM_Q + (((uint32_t)(sq * 32)) << 16) + half * 64;
+            uint32_t r0[4], r1[4];
 #pragma unroll
-            for (int g = 0; g < 2; ++g) {
-                uint32_t r[32];
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    *reinterpret_cast<uint4*>(r + 4 * i) = *reinterpret_cast<const uint4*>(zq + zq_chunk(h, term * (AM_W / 16) + half * 16 + g * 8 + i));
-                tc::tmem_st32(dst + g * 32, r);
+            for (int c = 0; c < 2; ++c) {
+                uint2 hi, lo;
+                codes8(rsrc[c], hi, lo);
+                exchange(hi, lo, r0 + 2 * c, r1 + 2 * c);
             }
-            if (half == 0) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    *reinterpret_cast<uint4*>(smem + SM_QR + sw64_chunk(sq * 32 + lane, i)) =
-                        *reinterpret_cast<const uint4*>(zq + zq_chunk(h, term * (AM_W / 16) + AM_KVL / 16 + i));
-            }
+            *reinterpret_cast<uint4*>(smem + SM_QR + sw64_chunk(sq * 32 + lane, 2 * half)) = make_uint4(r0[0], r0[1], r0[2], r0[3]);
+            *reinterpret_cast<uint4*>(smem + SM_QR + sw64_chunk(sq * 32 + lane, 2 * half + 1)) = make_uint4(r1[0], r1[1], r1[2], r1[3]);
         }
         tc::tmem_st_wait();
         tc::fence_proxy_async();
@@ -299,13 +282,15 @@ attend_mma_kernel(AttendMmaArgs A) {
     }
 
     // With q_early everything above read only inputs that predate the preceding kernel, so it overlapped
-    // that kernel's tail; the selected rows and their counts are read below.
-    rv_grid_dep_wait();
+    // that kernel's tail; the selected rows and their counts are read below (of a call that appends and selects nothing
+    // they predate it as well: the gather below waits where it comes to a row that may be new).
+    const bool fresh = A.fresh_pos != nullptr;
+    if (!fresh) rv_grid_dep_wait();
     int nr = A.n_rows[b];
     // a row list whose first entry is the dense marker stands for "row j = token j" over the first n_rows tokens
     const bool listed = A.rows && A.rows[(size_t)b * A.row_stride] != 0xffffffffu;
     {
-        const long long cap = listed ? A.row_stride : (long long)A.max_pages * P;
+        const long long cap = listed ? A.row_stride : min((long long)A.row_cap, (long long)A.max_pages * P);
         nr = (int)max(0LL, min((long long)nr, cap));
     }
     // Short contexts belong to the CUDA-core kernel launched by the same call: this CTA touches no output.
@@ -317,14 +302,19 @@ attend_mma_kernel(AttendMmaArgs A) {
     const int r_begin = split * tps * AM_TILE;
     const int r_end = min(nr, r_begin + tps * AM_TILE);
     const int ntiles = r_end > r_begin ? (r_end - r_begin + AM_TILE - 1) / AM_TILE : 0;
-
+    float2 my_ml = make_float2(-INFINITY, 0.0f);   // a split's reference maximum and weight sum of a head (one thread per head)
+    const bool publishes = warp < AM_SW / 2 && lane < 16;                 // that thread
+    const int ph = 16 * (warp & 3) + (lane & 15);                         // and its head
+    auto cluster_arrive = []() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); };
+    auto cluster_wait = []() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); };
 
     if (warp >= AM_GW0 && ntiles > 0) {
         // ------------------------------ gather producers ------------------------------------------
-        // The first four tiles are filled together, sixteen rows of each by every warp: the first is there after a quarter of
-        // the time that a tile per warp would take. Then warp g fills the tiles g + 4, g + 8, ... (ring stage = tile % 6), a
-        // tile per warp: sixteen rows of every tile throughout held the latent copies of all warps back at the next tile's
-        // rope buffer (batch 128: 59.4 -> 63.5 us). All in plain program order, and never waiting for
+        // The first four tiles, or all of a CTA that has at most eight, are filled together, sixteen rows of each by every warp:
+        // the first is there after a quarter of the time that a tile per warp would take. Then warp g fills the tiles g + 4,
+        // g + 8, ... (ring stage = tile % 6), a tile per warp: sixteen rows of every tile throughout held the latent copies of all
+        // warps back at the next tile's rope buffer (batch 128: 59.4 -> 63.5 us), and four tiles that land together leave the
+        // MMAs waiting for 3,500 cycles where eight are all there is. All in plain program order, and never waiting for
         // a copy to land: a thread's copies signal the stage's barrier themselves when they are complete
         // (cp.async.mbarrier.arrive), so the warp goes straight on to its next tile as soon as that tile's stage is
         // free. A lane resolves the addresses of two rows of its warp's tile.
@@ -344,8 +334,10 @@ attend_mma_kernel(AttendMmaArgs A) {
         const int32_t* btp = A.block_table + (size_t)b * A.max_pages;
         const int pshift = 31 - __clz(P);                  // page sizes are powers of two (checked by the host entry)
         static_assert(AM_GW * 16 == AM_TILE, "sixteen rows per warp of the first four tiles");
-        auto load_tok = [&](int j, int u) -> uint32_t {     // j = tile of the split; j = g stands for the warp's rows of tiles 0 .. 3
-            const int ri = r_begin + (j < AM_GW ? (2 * u + (lane >> 4)) * AM_TILE + 16 * g + (lane & 15) : j * AM_TILE + u * 32 + lane);
+        const int n_joint = ntiles <= AM_JOINT ? AM_JOINT / AM_GW : 1;      // the warp's steps that are shared tiles
+        auto load_tok = [&](int n, int u) -> uint32_t {     // this lane's u-th row of the warp's step n
+            const int ri = r_begin + n * AM_GW * AM_TILE +
+                           (n < n_joint ? (2 * u + (lane >> 4)) * AM_TILE + 16 * g + (lane & 15) : g * AM_TILE + u * 32 + lane);
             if (ri >= r_end) return NONE;
             return rowp ? rowp[ri] : (uint32_t)ri;
         };
@@ -361,20 +353,68 @@ attend_mma_kernel(AttendMmaArgs A) {
         uint32_t tk[2][AM_LOOK], tok[2][AM_LOOK], row[2][AM_LOOK];
         int32_t pg[2][AM_LOOK];
         float scl[2][AM_LOOK];
+        // prologue: all token loads at once, then the page entries, then the scales of the first tiles
+        // Rows that the kernel before may still be writing are marked in a bitmap by a hash of the pool row (in the P' tile, which
+        // is not in use before the first QK): a tile of the first four that holds a marked row waits for that kernel, and so
+        // does everything behind them. A hash that two rows share only makes a tile wait.
+        uint32_t* marks = reinterpret_cast<uint32_t*>(smem + SM_P);
+        constexpr int MARK_BITS = 2 * SM_PTERM * 8, AM_GT = AM_GW * 32;
+        auto mark_of = [](uint32_t r) { return (r * 2654435761u) >> 16; };
+        static_assert(MARK_BITS == 1 << 16, "sixteen hash bits");
+        const int gt = g * 32 + lane;
+        int fp[2] = {-1, -1};
+        if (fresh) {
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {   // prologue: all token loads at once, then the page entries, then the scales of the first tiles
-            uint32_t t0[AM_LOOK];
-            int32_t p0[AM_LOOK];
+            for (int v = 0; v < 2; ++v)
+                if (gt + v * AM_GT < A.n_fresh) fp[v] = A.fresh_pos[gt + v * AM_GT];
+#pragma unroll
+            for (int v = 0; v < MARK_BITS / 128 / AM_GT; ++v) reinterpret_cast<uint4*>(marks)[gt + v * AM_GT] = make_uint4(0u, 0u, 0u, 0u);
+        }
+        uint32_t t0[2][AM_LOOK];
+        int32_t p0[2][AM_LOOK];
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
 #pragma unroll
             for (int k = 0; k < AM_LOOK; ++k) {
-                t0[k] = load_tok(g + AM_GW * k, u); tok[u][k] = load_tok(g + AM_GW * (AM_LOOK + k), u);
-                tk[u][k] = load_tok(g + AM_GW * (2 * AM_LOOK + k), u);
+                t0[u][k] = load_tok(k, u); tok[u][k] = load_tok(AM_LOOK + k, u);
+                tk[u][k] = load_tok(2 * AM_LOOK + k, u);
             }
+        uint32_t hits[2] = {0u, 0u};   // lanes whose row of the first four tiles is marked
+        uint32_t fr[2] = {NONE, NONE};
+        if (fresh) {
 #pragma unroll
-            for (int k = 0; k < AM_LOOK; ++k) { p0[k] = load_pg(t0[k]); pg[u][k] = load_pg(tok[u][k]); }
-#pragma unroll
-            for (int k = 0; k < AM_LOOK; ++k) { row[u][k] = pool_row(t0[k], p0[k]); scl[u][k] = load_scl(row[u][k]); }
+            for (int v = 0; v < 2; ++v) {
+                const uint32_t lp = (uint32_t)fp[v] >> pshift;
+                const int32_t fpg = fp[v] >= 0 && lp < (uint32_t)A.max_pages ? A.block_table[(size_t)(gt + v * AM_GT) * A.max_pages + lp] : -1;
+                fr[v] = pool_row((uint32_t)fp[v], fpg);
+            }
         }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int k = 0; k < AM_LOOK; ++k) { p0[u][k] = load_pg(t0[u][k]); pg[u][k] = load_pg(tok[u][k]); }
+        if (fresh) {
+            tc::named_barrier(2, AM_GT);
+#pragma unroll
+            for (int v = 0; v < 2; ++v)
+                if (fr[v] != NONE) atomicOr(marks + (mark_of(fr[v]) >> 5), 1u << (mark_of(fr[v]) & 31));
+            tc::named_barrier(2, AM_GT);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+#pragma unroll
+            for (int k = 0; k < AM_LOOK; ++k) { row[u][k] = pool_row(t0[u][k], p0[u][k]); scl[u][k] = load_scl(row[u][k]); }
+            if (fresh) hits[u] = __ballot_sync(0xffffffffu, row[u][0] != NONE && ((marks[mark_of(row[u][0]) >> 5] >> (mark_of(row[u][0]) & 31)) & 1u));
+        }
+        bool waited = !fresh;
+        auto wait_fresh = [&]() {
+            rv_grid_dep_wait();
+            waited = true;
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+#pragma unroll
+                for (int k = 0; k < AM_LOOK; ++k) scl[u][k] = load_scl(row[u][k]);
+        };
         // Each lane owns the addresses of two rows, but the COPIES are issued row by row with the 32 lanes of
         // the warp on 32 consecutive 16-byte chunks (the pool row travels by shuffle): one warp
         // instruction then reads 512 contiguous bytes instead of 32 scattered 16-byte pieces. A row past the end
@@ -395,8 +435,8 @@ attend_mma_kernel(AttendMmaArgs A) {
             tc::cp_async16_zfill(tc::smem_u32(rope + sw64_chunk(slot, lane & 3)),
                                  A.pool + (r != NONE ? (size_t)r * AM_W + 512 + (lane & 3) * 16 : 0), r != NONE ? 16u : 0u);
         };
-        // advance the chain past the warp's step at tile j: every value consumed here was requested AM_LOOK iterations ago
-        auto advance = [&](int j) {
+        // advance the chain past the warp's step n: every value consumed here was requested AM_LOOK iterations ago
+        auto advance = [&](int n) {
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 const uint32_t row_new = pool_row(tok[u][0], pg[u][0]);
@@ -407,68 +447,66 @@ attend_mma_kernel(AttendMmaArgs A) {
                 }
                 row[u][AM_LOOK - 1] = row_new; scl[u][AM_LOOK - 1] = load_scl(row_new);
                 tok[u][AM_LOOK - 1] = tok_new; pg[u][AM_LOOK - 1] = load_pg(tok_new);
-                tk[u][AM_LOOK - 1] = load_tok(j + AM_GW * 3 * AM_LOOK, u);
+                tk[u][AM_LOOK - 1] = load_tok(n + 3 * AM_LOOK, u);
             }
         };
         // A stage is full when every copy has landed (the lanes' arrivals by the copies themselves: 32 from each of the four
         // warps, or four times 32 from the one that fills it) and the token words are written (plain arrivals, four in all,
         // which also publish those stores).
-        // tiles 0 .. 3: fresh stages; the last of them and the last rope buffer wait like any other
+        const int n_steps = ntiles <= n_joint * AM_GW ? n_joint : (ntiles - 1 - g + AM_GW) / AM_GW;
 #pragma unroll 1
-        for (int j = 0; j < AM_GW && j < ntiles && ok; ++j) {
-            if (j >= AM_ROPES)
-                ok = tc::mbar_wait_warp(&bars.q_full, 0, abort_flag, 43, A.max_polls);   // stages 3 to 5 held q
-            if (!ok) break;
-            uint8_t* kbuf = smem + SM_K0 + j * SM_KSTAGE;
-            const uint32_t src = j < 2 ? row[0][0] : row[1][0];
-            const float sc = j < 2 ? scl[0][0] : scl[1][0];
-            const int l0 = (j & 1) * 16;                   // the lanes that hold this tile's rows
-#pragma unroll
-            for (int it = 0; it < 16; ++it) copy_latent(kbuf, __shfl_sync(0xffffffffu, src, l0 + it), 16 * g + it);
-            const int rb = j % AM_ROPES;
-            ok = tc::mbar_wait_warp(&bars.rope_free[rb], ((j / AM_ROPES) & 1) ^ 1, abort_flag, 42, A.max_polls);
-            if (!ok) break;
-#pragma unroll
-            for (int it = 0; it < 2; ++it) {
-                const int rl = it * 8 + (lane >> 2);
-                copy_rope(smem + SM_ROPE + rb * SM_ROPEBUF, __shfl_sync(0xffffffffu, src, l0 + rl), 16 * g + rl);
-            }
-            tc::cp_async_mbar_arrive_noinc(&bars.k_full[j]);
-            if ((lane >> 4) == (j & 1)) token_words(j, 16 * g + (lane & 15), src, sc);
-            __syncwarp();
-            if (lane == 0 && !(A.withhold && j == 0 && g == 0)) tc::mbar_arrive(&bars.k_full[j]);
-        }
-        advance(g);
-        for (int j = g + AM_GW; j < ntiles && ok; j += AM_GW) {
-            const int s = j % AM_STAGES, use = j / AM_STAGES;
-            ok = tc::mbar_wait_warp(&bars.k_empty[s], (use & 1) ^ 1, abort_flag, 41, A.max_polls);
-            if (ok && j < AM_STAGES) ok = tc::mbar_wait_warp(&bars.q_full, 0, abort_flag, 43, A.max_polls);   // these stages held q
-            if (!ok) break;
-            uint8_t* kbuf = smem + SM_K0 + s * SM_KSTAGE;
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
+        for (int n = 0; n < n_steps && ok; ++n) {
+            const bool joint = n < n_joint;
+#pragma unroll 1
+            for (int t = joint ? 0 : g; ; ++t) {
+                const int j = n * AM_GW + t, s = j % AM_STAGES, rb = j % AM_ROPES;
+                const bool last = t >= (joint ? AM_GW : g + 1) || j >= ntiles;
+                const int l0 = (t & 1) * 16;                   // (joint) the lanes that hold this tile's rows
+                if (!waited && (last || (((t < 2 ? hits[0] : hits[1]) >> l0) & 0xffffu))) wait_fresh();
+                if (last) break;
+                if (j >= AM_STAGES) ok = tc::mbar_wait_warp(&bars.k_empty[s], ((j / AM_STAGES) & 1) ^ 1, abort_flag, 41, A.max_polls);
+                else if (j >= AM_ROPES) ok = tc::mbar_wait_warp(&bars.q_full, 0, abort_flag, 43, A.max_polls);   // stages 3 to 5 held q
+                if (!ok) break;
+                uint8_t* kbuf = smem + SM_K0 + s * SM_KSTAGE;
+                if (joint) {
+                    const uint32_t src = t < 2 ? row[0][0] : row[1][0];
 #pragma unroll 8
-                for (int it = 0; it < 32; ++it) copy_latent(kbuf, __shfl_sync(0xffffffffu, row[u][0], it), u * 32 + it);
-            }
-            // a rope tile is free as soon as the two rope MMAs of the tile that used it last are done
-            const int rb = j % AM_ROPES;
-            ok = tc::mbar_wait_warp(&bars.rope_free[rb], ((j / AM_ROPES) & 1) ^ 1, abort_flag, 42, A.max_polls);
-            if (!ok) break;
+                    for (int it = 0; it < 16; ++it) copy_latent(kbuf, __shfl_sync(0xffffffffu, src, l0 + it), 16 * g + it);
+                } else {
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-#pragma unroll
-                for (int it = 0; it < 4; ++it) {
-                    const int rl = it * 8 + (lane >> 2);
-                    copy_rope(smem + SM_ROPE + rb * SM_ROPEBUF, __shfl_sync(0xffffffffu, row[u][0], rl), u * 32 + rl);
+                    for (int u = 0; u < 2; ++u) {
+#pragma unroll 8
+                        for (int it = 0; it < 32; ++it) copy_latent(kbuf, __shfl_sync(0xffffffffu, row[u][0], it), u * 32 + it);
+                    }
                 }
+                // a rope tile is free as soon as the two rope MMAs of the tile that used it last are done
+                ok = tc::mbar_wait_warp(&bars.rope_free[rb], ((j / AM_ROPES) & 1) ^ 1, abort_flag, 42, A.max_polls);
+                if (!ok) break;
+                uint8_t* rope = smem + SM_ROPE + rb * SM_ROPEBUF;
+                const int own = joint ? 1 : AM_GW;             // arrivals: this warp's share of the stage's
+                if (joint) {
+#pragma unroll
+                    for (int it = 0; it < 2; ++it) {
+                        const int rl = it * 8 + (lane >> 2);
+                        copy_rope(rope, __shfl_sync(0xffffffffu, t < 2 ? row[0][0] : row[1][0], l0 + rl), 16 * g + rl);
+                    }
+                    tc::cp_async_mbar_arrive_noinc(&bars.k_full[s]);
+                    if ((lane >> 4) == (t & 1)) token_words(s, 16 * g + (lane & 15), t < 2 ? row[0][0] : row[1][0], t < 2 ? scl[0][0] : scl[1][0]);
+                } else {
+#pragma unroll
+                    for (int it = 0; it < 8; ++it) {
+                        const int rl = it * 8 + (lane >> 2);
+                        copy_rope(rope, __shfl_sync(0xffffffffu, row[it >> 2][0], rl & 31), rl);
+                    }
+#pragma unroll
+                    for (int it = 0; it < AM_GW; ++it) tc::cp_async_mbar_arrive_noinc(&bars.k_full[s]);
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) token_words(s, u * 32 + lane, row[u][0], scl[u][0]);
+                }
+                __syncwarp();
+                if (lane < own && !(A.withhold && j == 0 && g == 0)) tc::mbar_arrive(&bars.k_full[s]);
             }
-#pragma unroll
-            for (int i = 0; i < AM_GW; ++i) tc::cp_async_mbar_arrive_noinc(&bars.k_full[s]);
-#pragma unroll
-            for (int u = 0; u < 2; ++u) token_words(s, u * 32 + lane, row[u][0], scl[u][0]);
-            __syncwarp();
-            if (lane < AM_GW) tc::mbar_arrive(&bars.k_full[s]);
-            advance(j);
+            advance(n);
         }
     } else if (warp == AM_QKW) {
         // ------------------------------ QK issuer -------------------------------------------------
@@ -501,6 +539,7 @@ attend_mma_kernel(AttendMmaArgs A) {
                         for (int k = 0; k < 4; ++k)   // A from tensor memory: 32 codes = 8 columns per step; descriptor address fields count 16-byte units
                             tc::mma_f8_ta(d, TM_Q + (uint32_t)(c * 32 + k * 8), d_k + (uint64_t)((c * SM_KCHUNK + k * 32) >> 4), id_qk, 1);
                     tc::mma_commit(&bars.s_full[sb]);
+                    tc::mbar_arrive(&bars.s_full[sb]);   // hands the token words on: this thread has seen k_full
                 }
                 __syncwarp();
             }
@@ -530,49 +569,56 @@ attend_mma_kernel(AttendMmaArgs A) {
                             tc::mma_f8(TM_O + c * 64, d_v + (uint64_t)((c * SM_KCHUNK + k * 4096) >> 4), d_plo + (uint64_t)(k * 2), id_pv, 1);
                     }
                     tc::mma_commit(&bars.k_empty[s]);
-                    tc::mma_commit(&bars.pv_done);
+                    tc::mma_commit(&bars.pv_done[j & 1]);
                 }
                 __syncwarp();
             }
         }
     } else if (warp < AM_SW) {
         // ------------------------------ softmax + epilogue ---------------------------------------
-        // S: TMEM lane = virtual head. Warp (sq, th): lane quarter sq = warp % 4 (heads 16 sq .. 16 sq + 15, hi terms in
-        // lanes 0-15 and lo terms in lanes 16-31), token half th = warp / 4 (columns 32 th .. 32 th + 31 of the tile).
-        // After the hi + lo exchange lane l keeps the 16 tokens 32 th + 16 (l / 16) .. + 15 of head 16 sq + l % 16.
-        // O^T: TMEM lane = latent dim 32 sq + lane of each 128-dim block, head columns 32 th .. 32 th + 31.
+        // S: TMEM lane = virtual head; lane quarter sq = warp % 4 (heads 16 sq .. 16 sq + 15, hi terms in lanes 0-15 and lo terms in
+        // lanes 16-31). The warps are two groups of four that take the tiles in turn, so that the round trips of one tile (to
+        // tensor memory, to its barriers, through the shuffles) run beside those of the other: eight warps on one tile spent
+        // 2,000 - 2,300 cycles in a row on it, whatever the order, and that was the loop's period (batch 128 x 2,048 rows:
+        // 1.32 us a tile, 1.27 so; there the rows that an SM takes in are the bound now).
+        // After the hi + lo exchange lane l keeps the tokens 32 hf + 16 (l / 16) .. + 15 of each half hf of the tile, of head
+        // 16 sq + l % 16.
+        // O^T: TMEM lane = latent dim 32 sq + lane of each 128-dim block; in the epilogue th = warp / 4 is the half of the heads.
         const int sq = warp & 3, th = warp >> 2, tb = lane >> 4;
         const int hd = 16 * sq + (lane & 15);
         const int row = sq * 32 + lane;
         const uint32_t lane_base = ((uint32_t)(sq * 32)) << 16;
         const int h0 = th * AM_HPT;
+        constexpr int AM_GROUP_THREADS = AM_SOFTMAX_THREADS / 2;
         const float a_h = s_ahi[hd];
-        float l_acc = 0.0f;                                // sum of this thread's weights of head hd
-        float m_ref = -INFINITY;                           // reference max of head hd (the same in its four threads)
+        float l_acc = 0.0f;                                // sum of this thread's weights of head hd, at the reference m_ref
+        float m_ref = -INFINITY;                           // reference max of head hd
         bool ok = ntiles > 0;
-        // A warp whose wait gave up brings the others to the slow path of the tile that they are in or come to next, where all
-        // agree to leave.
-        auto give_up = [&]() { (void)tc::barrier_any(1, AM_SOFTMAX_THREADS, true); (void)tc::barrier_any(2, AM_SOFTMAX_THREADS, true); };
-        for (int i = 0; i < ntiles; ++i) {
-            const int s = i % AM_STAGES, use = i / AM_STAGES, sb = i % AM_SBUF, suse = i / AM_SBUF;
-            ok = tc::mbar_wait_warp(&bars.k_full[s], use & 1, abort_flag, 61, A.max_polls) &&
-                 tc::mbar_wait_warp(&bars.s_full[sb], suse & 1, abort_flag, 62, A.max_polls);
+        // A warp whose wait gave up brings the others of its group to the slow path of the tile that they are in or come to next,
+        // where all agree to leave.
+        auto give_up = [&]() { (void)tc::barrier_any(6 + th, AM_GROUP_THREADS, true); (void)tc::barrier_any(8 + th, AM_GROUP_THREADS, true); };
+        for (int i = th; i < ntiles; i += 2) {
+            const int s = i % AM_STAGES;
+            ok = tc::mbar_wait_warp(&bars.s_full[th], (i >> 1) & 1, abort_flag, 62, A.max_polls);
             if (!ok) { give_up(); break; }
             tc::tc_fence_after();
-            // this thread's 16 tokens: four 16-byte loads per plane (the two half-warps read 64 bytes apart: no bank conflict)
-            const float4* ti = reinterpret_cast<const float4*>(s_tok + s * AM_TILE + 32 * th + 16 * tb);
-            float s2[16];
-            float dmax = -INFINITY;               // max over this thread's tokens of s2' - reference
-            {
+            // this thread's 32 tokens: 16-byte loads per plane (the two half-warps read 64 bytes apart: no bank conflict)
+            const float4* ti = reinterpret_cast<const float4*>(s_tok + s * AM_TILE + 16 * tb);
+            float s2[32];
+            float mx = -INFINITY;                 // max over this thread's tokens of s2
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
                 uint32_t r[32];
-                tc::tmem_ld32(TM_S0 + sb * AM_TILE + lane_base + 32 * th, r);
+                tc::tmem_ld32(TM_S0 + th * AM_TILE + lane_base + 32 * hf, r);
                 tc::tmem_ld_wait();
-                tc::tc_fence_before();
-                __syncwarp();
-                if (lane == 0) tc::mbar_arrive(&bars.s_empty[sb]);
+                if (hf == 1) {
+                    tc::tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive(&bars.s_empty[th]);
+                }
 #pragma unroll
                 for (int j4 = 0; j4 < 4; ++j4) {
-                    const float4 ts = ti[j4], tc2 = ti[SM_TOKPLANE / 16 + j4];
+                    const float4 ts = ti[8 * hf + j4], tc2 = ti[SM_TOKPLANE / 16 + 8 * hf + j4];
                     const float sc4[4] = {ts.x, ts.y, ts.z, ts.w}, c24[4] = {tc2.x, tc2.y, tc2.z, tc2.w};
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
@@ -582,60 +628,65 @@ attend_mma_kernel(AttendMmaArgs A) {
                         const float raw = mine + __shfl_xor_sync(0xffffffffu, give, 16);
                         // rows past the end are exact zeros in shared memory, so their raw scores are 0 and an
                         // additive -inf makes every weight of theirs exactly 0 without a select per element
-                        s2[j] = fmaf(raw, a_h * sc4[e], c24[e]);
-                        dmax = fmaxf(dmax, s2[j] - m_ref);   // reference is -inf before the first tile
+                        s2[16 * hf + j] = fmaf(raw, a_h * sc4[e], c24[e]);
+                        mx = fmaxf(mx, s2[16 * hf + j]);
                     }
                 }
             }
+            // The references as tile i - 1 left them (the other group's tile)
+            if (i > 0) {
+                ok = tc::mbar_wait_warp(&bars.dec[th ^ 1], ((i - 1) >> 1) & 1, abort_flag, 65, A.max_polls);
+                if (!ok) { give_up(); break; }
+                const float m_now = s_mref[hd];
+                if (m_now != m_ref) { l_acc *= exp2f(m_ref - m_now); m_ref = m_now; }
+            }
+            // asked ahead (a look at a barrier takes 200 cycles beside the MMAs, one whose phase is complete as well)
+            const bool pv_ready = i == 0 || tc::mbar_test(&bars.pv_done[th ^ 1], ((i - 1) >> 1) & 1);   // PV(i - 1) has read the P' tile
 
             // Fast path: no score of the tile exceeds its head's reference by more than AM_LAG, so the
-            // references stand and nothing has to be exchanged. One barrier-with-OR decides for the CTA.
-            // NaN-free: dmax is -inf or finite or +inf (s2 carries AM_POFF, the reference does not)
-            if (tc::barrier_any(1, AM_SOFTMAX_THREADS, dmax > AM_LAG + AM_POFF)) {
-                // exact per-head tile max: this thread's 16 tokens, its partner lane's, the other token half's warp
-                {
-                    float mx = s2[0];
-#pragma unroll
-                    for (int j = 1; j < 16; ++j) mx = fmaxf(mx, s2[j]);
-                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-                    if (lane < 16) s_wmax[th * 64 + hd] = mx;
-                }
-                if (tc::barrier_any(2, AM_SOFTMAX_THREADS, false)) { ok = false; break; }
+            // references stand and nothing has to be exchanged. One barrier-with-OR decides for the group, and the other group
+            // for its tile then.
+            // (before the first live tile the reference is -inf; s2 carries AM_POFF, the reference does not)
+            if (tc::barrier_any(6 + th, AM_GROUP_THREADS, mx - m_ref > AM_LAG + AM_POFF)) {
+                // exact per-head tile max: this thread's tokens and its partner lane's
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
                 float fac = 1.0f;
                 {
-                    const float tm = fmaxf(s_wmax[hd], s_wmax[64 + hd]) - AM_POFF;
+                    const float tm = mx - AM_POFF;
                     if (m_ref == -INFINITY) { if (tm > -INFINITY) m_ref = tm; }          // first live tile of this head
                     else if (tm > m_ref) { fac = exp2f(m_ref - tm); m_ref = tm; }          // any growth is taken now
-                    if (th == 0 && lane < 16) s_fac[hd] = fac;
+                    if (lane < 16) { s_fac[hd] = fac; s_mref[hd] = m_ref; }
                 }
-                tc::named_barrier(2, AM_SOFTMAX_THREADS);
+                if (tc::barrier_any(8 + th, AM_GROUP_THREADS, false)) { ok = false; break; }
                 // bring O^T and l to the new references. PV(i-1) must have landed first.
-                if (i >= 1) ok = tc::mbar_wait_warp(&bars.pv_done, (i - 1) & 1, abort_flag, 63, A.max_polls);
-                if (!ok) { if (i + 1 < ntiles) give_up(); break; }
+                if (i >= 1) ok = tc::mbar_wait_warp(&bars.pv_done[th ^ 1], ((i - 1) >> 1) & 1, abort_flag, 63, A.max_polls);
+                if (!ok) { if (i + 2 < ntiles) give_up(); break; }
                 tc::tc_fence_after();
                 if (i >= 1) {
-                    uint32_t r[AM_HPT];
+                    uint32_t r[32];
 #pragma unroll 1
-                    for (int c = 0; c < 4; ++c) {   // this thread's dim lane, its head columns of each block
-                        tc::tmem_ld32(TM_O + lane_base + c * 64 + h0, r);
+                    for (int c = 0; c < 8; ++c) {   // this thread's dim lane, half the head columns of a block at a time
+                        tc::tmem_ld32(TM_O + lane_base + c * 32, r);
                         tc::tmem_ld_wait();
 #pragma unroll
-                        for (int h = 0; h < AM_HPT; ++h) r[h] = __float_as_uint(__uint_as_float(r[h]) * s_fac[h0 + h]);
-                        tc::tmem_st32(TM_O + lane_base + c * 64 + h0, r);
+                        for (int h = 0; h < 32; ++h) r[h] = __float_as_uint(__uint_as_float(r[h]) * s_fac[(c & 1) * 32 + h]);
+                        tc::tmem_st32(TM_O + lane_base + c * 32, r);
                     }
                     tc::tmem_st_wait();
                 }
                 l_acc *= fac;
                 tc::tc_fence_before();
             }
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&bars.dec[th]);     // the other group may decide on its tile
             // P'' = 2^(s2' - m) = weight * s_tok * 2^AM_POFF as two e4m3 terms (via f16: p <= 256 and the
             // residual p - hi are exact enough in half precision); l accumulates the plain weight.
             // A head that has seen no live token yet has no reference: its scores are all -inf and weigh 0.
             const float m_use = m_ref == -INFINITY ? 0.0f : m_ref;
-            uint32_t hi_w[4], lo_w[4];
+            uint32_t hi_w[8], lo_w[8];
 #pragma unroll
-            for (int j = 0; j < 16; j += 4) {
-                const float4 ti4 = ti[2 * (SM_TOKPLANE / 16) + (j >> 2)];
+            for (int j = 0; j < 32; j += 4) {
+                const float4 ti4 = ti[2 * (SM_TOKPLANE / 16) + 8 * (j >> 4) + ((j & 15) >> 2)];
                 const float inv4[4] = {ti4.x, ti4.y, ti4.z, ti4.w};
                 uint32_t chs[2], cls[2];
 #pragma unroll
@@ -658,25 +709,27 @@ attend_mma_kernel(AttendMmaArgs A) {
                 hi_w[j >> 2] = chs[0] | (chs[1] << 16);
                 lo_w[j >> 2] = cls[0] | (cls[1] << 16);
             }
-            ok = tc::mbar_wait_warp(&bars.pv_done, (i & 1) ^ 1, abort_flag, 64, A.max_polls);   // PV(i - 1) has read the P' tile
-            if (!ok) { if (i + 1 < ntiles) give_up(); break; }
-            {
-                // row = head, bytes = tokens: this thread's 16 tokens are the 16-byte chunk 2 th + tb of its head's row
-                uint8_t* prow = smem + SM_P + sw64_chunk(hd, 2 * th + tb);
-                *reinterpret_cast<uint4*>(prow) = make_uint4(hi_w[0], hi_w[1], hi_w[2], hi_w[3]);
-                *reinterpret_cast<uint4*>(prow + SM_PTERM) = make_uint4(lo_w[0], lo_w[1], lo_w[2], lo_w[3]);
+            if (!__all_sync(0xffffffffu, pv_ready)) ok = tc::mbar_wait_warp(&bars.pv_done[th ^ 1], ((i - 1) >> 1) & 1, abort_flag, 64, A.max_polls);
+            if (!ok) { if (i + 2 < ntiles) give_up(); break; }
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+                // row = head, bytes = tokens: this thread's 16 tokens of a half are the 16-byte chunk 2 hf + tb of its head's row
+                uint8_t* prow = smem + SM_P + sw64_chunk(hd, 2 * hf + tb);
+                *reinterpret_cast<uint4*>(prow) = make_uint4(hi_w[4 * hf], hi_w[4 * hf + 1], hi_w[4 * hf + 2], hi_w[4 * hf + 3]);
+                *reinterpret_cast<uint4*>(prow + SM_PTERM) = make_uint4(lo_w[4 * hf], lo_w[4 * hf + 1], lo_w[4 * hf + 2], lo_w[4 * hf + 3]);
             }
             tc::fence_proxy_async();
             tc::mbar_arrive(&bars.p_full);
         }
 
         // ---- epilogue ----
-        if (ok && ntiles > 0) ok = tc::mbar_wait_warp(&bars.pv_done, (ntiles - 1) & 1, abort_flag, 65, A.max_polls);
-        tc::tc_fence_after();
-        // l per head: its four threads (two lanes 16 apart in each of the two token-half warps) meet by one shuffle
+        rv_grid_dep_wait();   // (the grid is not to be complete before the kernel in front of it)
+        // l per head: its four threads (two lanes 16 apart in a warp of each group) meet at the last reference by one shuffle
         // and one exchange through shared memory.
         tc::named_barrier(1, AM_SOFTMAX_THREADS);
         {
+            const float m_now = s_mref[hd];
+            if (m_now != m_ref) { l_acc *= exp2f(m_ref - m_now); m_ref = m_now; }
             const float mine = l_acc + __shfl_xor_sync(0xffffffffu, l_acc, 16);
             if (lane < 16) s_wmax[th * 64 + hd] = mine;
         }
@@ -686,9 +739,7 @@ attend_mma_kernel(AttendMmaArgs A) {
             const float l = s_wmax[h] + s_wmax[64 + h];
             const float m_nat = (m_ref - AM_POFF) * 0.6931471805599453f;   // natural-log units (l and O carry 2^AM_POFF)
             if (clustered) {
-                float* xs = reinterpret_cast<float*>(smem + SM_XS);
-                xs[h] = (l > 0.0f && ok) ? m_ref : -INFINITY;
-                xs[64 + h] = (l > 0.0f && ok) ? l : 0.0f;
+                my_ml = (l > 0.0f && ok) ? make_float2(m_ref, l) : make_float2(-INFINITY, 0.0f);
             } else if (skip) {
                 // nothing: the sequence's output and statistics are written by the CUDA-core kernel
             } else {
@@ -697,6 +748,8 @@ attend_mma_kernel(AttendMmaArgs A) {
             }
             s_fac[h] = l > 0.0f ? 1.0f / l : 0.0f;
         }
+        if (ok && ntiles > 0) ok = tc::mbar_wait_warp(&bars.pv_done[(ntiles - 1) & 1], ((ntiles - 1) >> 1) & 1, abort_flag, 66, A.max_polls);
+        tc::tc_fence_after();
         tc::named_barrier(1, AM_SOFTMAX_THREADS);
         // O^T: this thread's TMEM lane is one latent dim of each 128-dim block; its head columns. Every MMA of the CTA has
         // read its operands, so the idle ring takes the bf16 output, eight heads of a token half at a time (all 512 dims:
@@ -740,55 +793,39 @@ attend_mma_kernel(AttendMmaArgs A) {
 
     if (clustered) {
         // ---- merge of a sequence's splits inside its thread-block cluster ----
-        // Every CTA has published its reference maximum and weight sum per head; each scales its own O^T to the common
-        // reference and the total sum and PUSHES it, head by head, into the idle ring of the CTA that writes that head (CTA
-        // r: the heads [64 r / n, 64 (r + 1) / n)), which then adds the n contributions from its own memory. Remote stores
-        // need no answer; reading the other CTAs' staged O instead took a pass more and 6,800 cycles of waiting for 128 KiB.
+        // Each CTA PUSHES its O^T, as it is, head by head into the idle ring of the CTA that writes that head (CTA r: the heads
+        // [64 r / n, 64 (r + 1) / n)), and its reference maximum and weight sum of the head beside it; that CTA brings the n
+        // contributions to the common reference and the total sum while it adds them from its own memory. So nothing has to be
+        // exchanged before the push (maxima and sums first, and O^T scaled by its sender, cost two more barriers and 2 us), and
+        // remote stores need no answer. Distributed shared memory takes 21 bytes a clock, whatever the width of the stores; a CTA's
+        // own share does not go through it.
         // All threads of all CTAs take part in both cluster barriers, whatever a bounded wait did before: a CTA that gave up
-        // publishes weight sums of zero.
-        cg::cluster_group cluster = cg::this_cluster();
+        // sends weight sums of zero.
         const int n = A.n_splits;
-        float* xs = reinterpret_cast<float*>(smem + SM_XS);
-        float* recv = reinterpret_cast<float*>(smem + SM_STAGE);             // [n][hpc][512]
-        uint2* s_dst = reinterpret_cast<uint2*>(smem + SM_P);                 // per head: where its row goes (cluster address), its factor
+        float* recv = reinterpret_cast<float*>(smem + SM_STAGE);              // [n][hpc][512]
+        float2* ml = reinterpret_cast<float2*>(smem + SM_QR);                 // [n][hpc]: (maximum, sum) of rank q
+        float* wts = reinterpret_cast<float*>(smem + SM_P);                   // [hpc][8]: what rank q's row counts
         const int hpc = (AM_H + n - 1) / n;
-        __syncthreads();
         const bool live = ntiles > 0 && *abort_flag == 0;
-        cluster.sync();                                                       // [1] every CTA's (m, l)
+        cluster_arrive();
+        cluster_wait();                                                       // [1] every CTA's MMAs have read their ring and q
         if (warp < AM_SW) {
             const int sq = warp & 3, th = warp >> 2;
             const uint32_t lane_base = ((uint32_t)(sq * 32)) << 16;
             const int h0 = th * AM_HPT;
-            if (tid < AM_H) {
-                const int h = tid;
-                // every remote load of the merge is in flight before the first is used: one at a time (a loop to a run-time
-                // n) each costs a round trip over the cluster, and there are 16 here and 32 below
-                float mq[AM_MAX_SPLITS], lq[AM_MAX_SPLITS], mg = -INFINITY, L = 0.0f;
-#pragma unroll
-                for (int q = 0; q < AM_MAX_SPLITS; ++q) {
-                    const float* px = cluster.map_shared_rank(xs, q < n ? q : 0);
-                    mq[q] = q < n ? px[h] : -INFINITY;
-                    lq[q] = q < n ? px[64 + h] : 0.0f;
-                }
-#pragma unroll
-                for (int q = 0; q < AM_MAX_SPLITS; ++q) mg = fmaxf(mg, mq[q]);
-#pragma unroll
-                for (int q = 0; q < AM_MAX_SPLITS; ++q)
-                    if (lq[q] > 0.0f) L += lq[q] * exp2f(mq[q] - mg);
-                const float lm = xs[64 + h];
-                const float fac = (live && L > 0.0f && lm > 0.0f) ? exp2f(xs[h] - mg) / L : 0.0f;
-                const int owner = ((h + 1) * n - 1) / AM_H;
-                uint32_t to32;
-                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to32) : "r"(tc::smem_u32(recv + (split * hpc + h - owner * AM_H / n) * AM_KVL)), "r"(owner));
-                s_dst[h] = make_uint2(to32, __float_as_uint(fac));
-                if (split == 0 && !skip) {
-                    const float m_nat = (mg - AM_POFF) * 0.6931471805599453f;
-                    if (A.out_m) A.out_m[(size_t)b * AM_H + h] = L > 0.0f ? m_nat : -INFINITY;
-                    if (A.out_lse) A.out_lse[(size_t)b * AM_H + h] = L > 0.0f ? m_nat + logf(L) : -INFINITY;
-                }
+            auto owner_of = [&](int h) { return ((h + 1) * n - 1) / AM_H; };
+            // lane l: where this CTA's row of head h0 + l goes
+            const int ho = owner_of(h0 + lane);
+            const uint32_t own32 = tc::smem_u32(recv + (split * hpc + h0 + lane - ho * AM_H / n) * AM_KVL);
+            uint32_t to32;
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to32) : "r"(own32), "r"(ho));
+            if (ho == split) to32 = own32;                                    // (an address of this CTA's own window)
+            if (publishes) {
+                const int o = owner_of(ph);
+                uint32_t m32;
+                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(m32) : "r"(tc::smem_u32(ml + split * hpc + ph - o * AM_H / n)), "r"(o));
+                asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(m32), "f"(live ? my_ml.x : -INFINITY), "f"(live ? my_ml.y : 0.0f) : "memory");
             }
-            tc::named_barrier(1, AM_SOFTMAX_THREADS);
-            tc::tc_fence_after();
 #pragma unroll 1
             for (int c = 0; c < 4; ++c) {
                 const uint32_t off = (uint32_t)(c * 128 + sq * 32 + lane) * 4u;
@@ -802,26 +839,60 @@ attend_mma_kernel(AttendMmaArgs A) {
                 }
 #pragma unroll
                 for (int hq = 0; hq < AM_HPT; ++hq) {   // lanes = consecutive dims: 128 bytes per warp store
-                    const uint2 d = s_dst[h0 + hq];
-                    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(d.x + off), "f"(live ? __uint_as_float(r[hq]) * __uint_as_float(d.y) : 0.0f) : "memory");
+                    const uint32_t d = __shfl_sync(0xffffffffu, to32, hq);
+                    asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(d + off), "r"(r[hq]) : "memory");
                 }
             }
         }
-        cluster.sync();                                                       // [2] every CTA's share of this CTA's heads
-        if (warp < AM_SW && !skip) {
-            const int hb = split * AM_H / n, he = (split + 1) * AM_H / n;
-            for (int e = tid; e < (he - hb) * (AM_KVL / 4); e += AM_SOFTMAX_THREADS) {
+        cluster_arrive();
+        cluster_wait();                                                       // [2] every CTA's share of this CTA's heads
+        // (short loops from here on: code that runs once per launch comes in from L2, at a tenth of the rate that it issues at)
+        const int hb = split * AM_H / n, heads = (split + 1) * AM_H / n - hb;
+        // eight lanes a head (a lane per rank) work out what each rank's row counts
+        const int wh = tid >> 3, wq = tid & 7;
+        const bool told = wh < heads && wq < n;
+        const float2 part = told ? ml[wq * hpc + wh] : make_float2(-INFINITY, 0.0f);
+        float mg = part.x, L;
+        static_assert(AM_MAX_SPLITS == 8 && AM_H / 2 * 8 <= AM_THREADS, "eight lanes a head, at most half of the heads");
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) mg = fmaxf(mg, __shfl_xor_sync(0xffffffffu, mg, o));
+        {
+            const float w = part.y > 0.0f ? exp2f(part.x - mg) : 0.0f;
+            L = part.y * w;
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+            if (told) wts[wh * AM_MAX_SPLITS + wq] = L > 0.0f ? w / L : 0.0f;
+        }
+        __syncthreads();
+        if (!skip) {
+#pragma unroll 1
+            for (int e = tid; e < heads * (AM_KVL / 4); e += AM_THREADS) {
                 const int hl = e / (AM_KVL / 4), d4 = e % (AM_KVL / 4);
                 float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 1
+                for (int q0 = 0; q0 < n; q0 += 4) {
+                    const float4 w4 = *reinterpret_cast<const float4*>(wts + hl * AM_MAX_SPLITS + q0);
+                    const float w[4] = {w4.x, w4.y, w4.z, w4.w};
+                    float4 v[4];
 #pragma unroll
-                for (int q = 0; q < AM_MAX_SPLITS; ++q)
-                    if (q < n) {
-                        const float4 v = *reinterpret_cast<const float4*>(recv + (q * hpc + hl) * AM_KVL + d4 * 4);
-                        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-                    }
-                const uint32_t w0 = (uint32_t)rv_f32_to_bf16(acc.x) | ((uint32_t)rv_f32_to_bf16(acc.y) << 16);
-                const uint32_t w1 = (uint32_t)rv_f32_to_bf16(acc.z) | ((uint32_t)rv_f32_to_bf16(acc.w) << 16);
+                    for (int q = 0; q < 4; ++q)
+                        if (q0 + q < n) v[q] = *reinterpret_cast<const float4*>(recv + ((q0 + q) * hpc + hl) * AM_KVL + d4 * 4);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (q0 + q < n) {
+                            acc.x = fmaf(v[q].x, w[q], acc.x); acc.y = fmaf(v[q].y, w[q], acc.y);
+                            acc.z = fmaf(v[q].z, w[q], acc.z); acc.w = fmaf(v[q].w, w[q], acc.w);
+                        }
+                }
+                uint32_t w0, w1;
+                asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w0) : "f"(acc.y), "f"(acc.x));
+                asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w1) : "f"(acc.w), "f"(acc.z));
                 *reinterpret_cast<uint2*>(A.out + ((size_t)b * AM_H + hb + hl) * AM_KVL + d4 * 4) = make_uint2(w0, w1);
+            }
+            if (wq == 0 && told) {
+                const float m_nat = (mg - AM_POFF) * 0.6931471805599453f;
+                if (A.out_m) A.out_m[(size_t)b * AM_H + hb + wh] = L > 0.0f ? m_nat : -INFINITY;
+                if (A.out_lse) A.out_lse[(size_t)b * AM_H + hb + wh] = L > 0.0f ? m_nat + logf(L) : -INFINITY;
             }
         }
     }
@@ -901,11 +972,15 @@ extern "C" __attribute__((visibility("default"))) void rivoli_attend_mma_test_ho
 // min_rows_hint: a lower bound the caller knows for n_rows over the batch (0 = unknown). With a bound of
 // AM_MIN_ROWS or more no sequence needs the CUDA-core arm and its launch is left out. max_rows: an upper bound; below
 // AM_MIN_ROWS no sequence needs this kernel and the CUDA-core arm serves them all, the empty ones too.
+// fresh_pos (with q_early): the launch before this call's first appends ONE token per sequence, at these positions, and writes nothing
+// else that the attention reads, but rows and n_rows if dense_len is given: they are then the first min(dense_len[b], max_rows)
+// tokens of each sequence.
 extern "C" int rivoli_attend_mma_paged_bf16(const DsaGeom* g, const uint16_t* q, const uint8_t* latent_pool,
                                             const float* latent_scale, const int32_t* block_table,
                                             const uint32_t* rows, int row_stride, const int32_t* n_rows, int B,
                                             uint16_t* out, float* out_m, float* out_lse, void* scratch,
-                                            int q_early, int min_rows_hint, long long max_rows, void* stream) {
+                                            int q_early, int min_rows_hint, long long max_rows, const int32_t* fresh_pos,
+                                            const int32_t* dense_len, void* stream) {
     if (!scratch) return 1001;
     if (((uintptr_t)latent_pool | (uintptr_t)scratch | (uintptr_t)q | (uintptr_t)out) & 15) return 1005;
     cudaStream_t st = (cudaStream_t)stream;
@@ -928,10 +1003,12 @@ extern "C" int rivoli_attend_mma_paged_bf16(const DsaGeom* g, const uint16_t* q,
             return e;
     if (only_short) return 0;
     rv_drain_error();
-    AttendMmaArgs a{q, g->softmax_scale, latent_pool, latent_scale, block_table, rows, row_stride, n_rows,
+    if (B > 2 * AM_GW * 32) fresh_pos = dense_len = nullptr;   // (two marked rows per gather thread)
+    AttendMmaArgs a{q, g->softmax_scale, latent_pool, latent_scale, block_table, dense_len ? nullptr : rows, row_stride, dense_len ? dense_len : n_rows,
                     g->page_tokens, g->max_pages_per_seq, g->n_pool_pages, n_splits,
                     out, out_m, out_lse, err,
-                    min_rows, q_early ? 1 : 0, g_am_max_polls.load(std::memory_order_relaxed), withhold};
+                    min_rows, q_early ? 1 : 0, g_am_max_polls.load(std::memory_order_relaxed),
+                    fresh_pos, B, dense_len ? (int)max_rows : 0x7fffffff, withhold};
     // one CTA per (sequence, split); the splits of a sequence are one thread-block cluster and merge inside the kernel
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)n_splits, (unsigned)B); cfg.blockDim = dim3(AM_THREADS);

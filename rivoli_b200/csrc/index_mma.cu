@@ -472,6 +472,11 @@ RIVOLI_API int rivoli_kv_append_paged(const DsaGeom* g, const uint16_t* latent, 
                                       const int32_t* block_table, uint8_t* latent_pool, float* latent_scale,
                                       uint8_t* index_pool, float* index_scale, int32_t* status, void* stream);
 
+// Whether the score rows are no longer than top_k and one launch takes the place of prologue, scorer and selection.
+extern "C" bool rivoli_index_select_takes_all(const DsaGeom* g, int score_stride) {
+    return score_stride <= g->top_k && rv_append_chunks(*g) <= 3 * 32;
+}
+
 // `ap` != NULL: the step's append (one new token per sequence) rides in the same launch as the
 // query preparation.
 static int select_impl(const DsaGeom* g, const AppendArgs* ap, const uint16_t* index_q, const float* w,
@@ -491,7 +496,7 @@ static int select_impl(const DsaGeom* g, const AppendArgs* ap, const uint16_t* i
     const int nh = g->index_heads, hd = g->index_dim;
     const bool narrow = rv_append_chunks(*g) <= 3 * 32;   // what the append inside a prologue launch covers
 
-    if (score_stride <= g->top_k && narrow) {
+    if (rivoli_index_select_takes_all(g, score_stride)) {
         rv_drain_error();
         rv_stage_event(0, st);
         // (the query codes stay part of the operator's scratch: the sharded step reads them after it)
