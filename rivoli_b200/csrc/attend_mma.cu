@@ -794,60 +794,70 @@ attend_mma_kernel(AttendMmaArgs A) {
     if (clustered) {
         // ---- merge of a sequence's splits inside its thread-block cluster ----
         // Each CTA PUSHES its O^T, as it is, head by head into the idle ring of the CTA that writes that head (CTA r: the heads
-        // [64 r / n, 64 (r + 1) / n)), and its reference maximum and weight sum of the head beside it; that CTA brings the n
+        // [HZ r / n, HZ (r + 1) / n) of the cluster's HZ), and its reference maximum and weight sum of the head beside it; that CTA brings the n
         // contributions to the common reference and the total sum while it adds them from its own memory. So nothing has to be
         // exchanged before the push (maxima and sums first, and O^T scaled by its sender, cost two more barriers and 2 us), and
         // remote stores need no answer. Distributed shared memory takes 21 bytes a clock, whatever the width of the stores; a CTA's
         // own share does not go through it.
+        // A batch of a few sequences leaves SMs idle even so: then gridDim.z clusters attend over the same rows, and each pushes
+        // and writes 64 / gridDim.z of the heads (the push and the sums are what a small batch waits for: 5,500 + 2,000 cycles
+        // of its 16,000 behind the last score).
         // All threads of all CTAs take part in both cluster barriers, whatever a bounded wait did before: a CTA that gave up
         // sends weight sums of zero.
         const int n = A.n_splits;
         float* recv = reinterpret_cast<float*>(smem + SM_STAGE);              // [n][hpc][512]
         float2* ml = reinterpret_cast<float2*>(smem + SM_QR);                 // [n][hpc]: (maximum, sum) of rank q
         float* wts = reinterpret_cast<float*>(smem + SM_P);                   // [hpc][8]: what rank q's row counts
-        const int hpc = (AM_H + n - 1) / n;
+        const int lgz = 6 - (31 - __clz((int)gridDim.z)), HZ = 1 << lgz, hz0 = (int)blockIdx.z << lgz;   // the heads that this cluster writes
+        static_assert(AM_H == 1 << 6, "shifts");
+        const int hpc = (HZ + n - 1) / n;
         const bool live = ntiles > 0 && *abort_flag == 0;
         cluster_arrive();
         cluster_wait();                                                       // [1] every CTA's MMAs have read their ring and q
         if (warp < AM_SW) {
             const int sq = warp & 3, th = warp >> 2;
             const uint32_t lane_base = ((uint32_t)(sq * 32)) << 16;
-            const int h0 = th * AM_HPT;
-            auto owner_of = [&](int h) { return ((h + 1) * n - 1) / AM_H; };
-            // lane l: where this CTA's row of head h0 + l goes
-            const int ho = owner_of(h0 + lane);
-            const uint32_t own32 = tc::smem_u32(recv + (split * hpc + h0 + lane - ho * AM_H / n) * AM_KVL);
+            auto owner_of = [&](int i) { return ((i + 1) * n - 1) >> lgz; };
+            // a warp takes 32 heads: its th's half of them and all dims, or the half that holds the cluster's heads and th's half of the
+            // dims; lane l: where this CTA's row of head win + l goes
+            const int win = HZ == AM_H ? 32 * th : hz0 & 32;
+            const int hl = min(max(win + lane - hz0, 0), HZ - 1), ho = owner_of(hl);
+            const uint32_t own32 = tc::smem_u32(recv + (split * hpc + hl - ho * HZ / n) * AM_KVL);
             uint32_t to32;
             asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to32) : "r"(own32), "r"(ho));
             if (ho == split) to32 = own32;                                    // (an address of this CTA's own window)
-            if (publishes) {
-                const int o = owner_of(ph);
+            if (publishes && ph >= hz0 && ph < hz0 + HZ) {
+                const int i = ph - hz0, o = owner_of(i);
                 uint32_t m32;
-                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(m32) : "r"(tc::smem_u32(ml + split * hpc + ph - o * AM_H / n)), "r"(o));
+                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(m32) : "r"(tc::smem_u32(ml + split * hpc + i - o * HZ / n)), "r"(o));
                 asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(m32), "f"(live ? my_ml.x : -INFINITY), "f"(live ? my_ml.y : 0.0f) : "memory");
             }
+            const int c0 = HZ == AM_H ? 0 : 2 * th, c1 = HZ == AM_H ? 4 : c0 + 2;
 #pragma unroll 1
-            for (int c = 0; c < 4; ++c) {
+            for (int c = c0; c < c1; ++c) {
                 const uint32_t off = (uint32_t)(c * 128 + sq * 32 + lane) * 4u;
-                uint32_t r[AM_HPT];
+                uint32_t r[32];
                 if (live) {
-                    tc::tmem_ld32(TM_O + lane_base + c * 64 + h0, r);
+                    tc::tmem_ld32(TM_O + lane_base + c * 64 + win, r);
                     tc::tmem_ld_wait();
                 } else {
 #pragma unroll
-                    for (int h = 0; h < AM_HPT; ++h) r[h] = 0u;
+                    for (int h = 0; h < 32; ++h) r[h] = 0u;
                 }
 #pragma unroll
-                for (int hq = 0; hq < AM_HPT; ++hq) {   // lanes = consecutive dims: 128 bytes per warp store
-                    const uint32_t d = __shfl_sync(0xffffffffu, to32, hq);
-                    asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(d + off), "r"(r[hq]) : "memory");
-                }
+                for (int h8 = 0; h8 < 32; h8 += 8)
+                    if (win + h8 >= hz0 && win + h8 < hz0 + HZ)
+#pragma unroll
+                        for (int h = h8; h < h8 + 8; ++h) {   // lanes = consecutive dims: 128 bytes per warp store
+                            const uint32_t d = __shfl_sync(0xffffffffu, to32, h);
+                            asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(d + off), "r"(r[h]) : "memory");
+                        }
             }
         }
         cluster_arrive();
         cluster_wait();                                                       // [2] every CTA's share of this CTA's heads
         // (short loops from here on: code that runs once per launch comes in from L2, at a tenth of the rate that it issues at)
-        const int hb = split * AM_H / n, heads = (split + 1) * AM_H / n - hb;
+        const int h_lo = split * HZ / n, heads = (split + 1) * HZ / n - h_lo, hb = hz0 + h_lo;
         // eight lanes a head (a lane per rank) work out what each rank's row counts
         const int wh = tid >> 3, wq = tid & 7;
         const bool told = wh < heads && wq < n;
@@ -908,14 +918,16 @@ attend_mma_kernel(AttendMmaArgs A) {
 
 // A CTA takes a whole SM (shared memory), and the CTAs of a sequence form one thread-block cluster (co-scheduled
 // inside a GPC). A batch is split only as far as all its clusters are resident at once: the largest cluster size
-// (<= 8) for which the device reports room for B clusters; anything more would run as a second wave.
-int mma_splits(int B) {
+// (<= 8) for which the device reports room for B clusters; anything more would run as a second wave. What room is left then
+// goes to clusters that share a sequence's heads (a power of two of them, eight heads or more and a head per CTA each).
+struct MmaPlan { int splits, shares; };
+MmaPlan mma_plan(int B) {
     constexpr int MOST = 128;
-    static std::atomic<int> cache[MOST + 1];   // by batch; 0 = not asked yet
+    static std::atomic<int> cache[MOST + 1];   // by batch: splits + 256 * shares; 0 = not asked yet
     const int sms = rv_sm_count();
-    if (B <= 0 || B > MOST || 2 * B > sms) return 1;
-    if (const int known = cache[B].load(std::memory_order_relaxed)) return known;
-    int n = sms / B;
+    if (B <= 0 || B > MOST || 2 * B > sms) return {1, 1};
+    if (const int known = cache[B].load(std::memory_order_relaxed)) return {known & 255, known >> 8};
+    int n = sms / B, active = 0;
     if (n > AM_MAX_SPLITS) n = AM_MAX_SPLITS;
     for (; n > 1; --n) {
         cudaLaunchConfig_t cfg = {};
@@ -924,13 +936,15 @@ int mma_splits(int B) {
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = (unsigned)n; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
         cfg.attrs = at; cfg.numAttrs = 1;
-        int active = 0;
+        active = 0;
         if (cudaOccupancyMaxActiveClusters(&active, attend_mma_kernel, &cfg) == cudaSuccess && active >= B) break;
         (void)cudaGetLastError();
     }
     if (n < 1) n = 1;
-    cache[B].store(n, std::memory_order_relaxed);
-    return n;
+    int z = 1;
+    while (n > 1 && z < 8 && AM_H / (2 * z) >= n && 2 * z * B <= active) z *= 2;
+    cache[B].store(n + 256 * z, std::memory_order_relaxed);
+    return {n, z};
 }
 
 }  // namespace
@@ -986,7 +1000,7 @@ extern "C" int rivoli_attend_mma_paged_bf16(const DsaGeom* g, const uint16_t* q,
     cudaStream_t st = (cudaStream_t)stream;
     int* err = reinterpret_cast<int*>(scratch);
     rv_allow_smem<attend_mma_kernel>(SM_TOTAL);
-    const int n_splits = mma_splits(B);
+    const MmaPlan plan = mma_plan(B);
     const int forced = g_am_min_rows_override.load(std::memory_order_relaxed);
     int min_rows = forced >= 0 ? forced : AM_MIN_ROWS;
     if (min_rows_hint >= min_rows) min_rows = 0;          // the caller vouches that no sequence is that short
@@ -1005,20 +1019,20 @@ extern "C" int rivoli_attend_mma_paged_bf16(const DsaGeom* g, const uint16_t* q,
     rv_drain_error();
     if (B > 2 * AM_GW * 32) fresh_pos = dense_len = nullptr;   // (two marked rows per gather thread)
     AttendMmaArgs a{q, g->softmax_scale, latent_pool, latent_scale, block_table, dense_len ? nullptr : rows, row_stride, dense_len ? dense_len : n_rows,
-                    g->page_tokens, g->max_pages_per_seq, g->n_pool_pages, n_splits,
+                    g->page_tokens, g->max_pages_per_seq, g->n_pool_pages, plan.splits,
                     out, out_m, out_lse, err,
                     min_rows, q_early ? 1 : 0, g_am_max_polls.load(std::memory_order_relaxed),
                     fresh_pos, B, dense_len ? (int)max_rows : 0x7fffffff, withhold};
     // one CTA per (sequence, split); the splits of a sequence are one thread-block cluster and merge inside the kernel
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)n_splits, (unsigned)B); cfg.blockDim = dim3(AM_THREADS);
+    cfg.gridDim = dim3((unsigned)plan.splits, (unsigned)B, (unsigned)plan.shares); cfg.blockDim = dim3(AM_THREADS);
     cfg.dynamicSmemBytes = (size_t)SM_TOTAL; cfg.stream = st;
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = (unsigned)n_splits; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
-    cfg.attrs = at; cfg.numAttrs = n_splits > 1 ? 2 : 1;
+    at[1].val.clusterDim.x = (unsigned)plan.splits; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = plan.splits > 1 ? 2 : 1;
     (void)cudaLaunchKernelEx(&cfg, attend_mma_kernel, a);
     return rv_launch_status();
 }
