@@ -26,8 +26,8 @@
 // the k-th largest values satisfy |A_k - E_k| <= eps, so a_t > A_k + 2 eps implies
 // o_t > E_k (selected) and a_t < A_k - 2 eps implies o_t < E_k (not selected); everything
 // else is decided on exact scores. eps per sequence = max key scale * sum_h |w_h ws| ds
-// s_q[h] ||qcode_h||_2 * sqrt(hd) * 448 * 2^-16: a Cauchy-Schwarz bound on sum |q_d k_d|
-// times 2^-16 relative error. The sequential fold's own worst case is hd * 2^-24 = 2^-17
+// s_q[h] ||qcode_h||_1 * 448 * 2^-16: a bound on sum |q_d k_d| (no key code exceeds 448; with the
+// 2-norms of both it was a quarter wider, and the band with it) times 2^-16 relative error. The sequential fold's own worst case is hd * 2^-24 = 2^-17
 // of sum |q_d k_d|; the tensor core measured 2^-21.9 on full-range random codes.
 #include "codec.cuh"
 #include "common.cuh"
@@ -76,7 +76,7 @@ index_q_prepare_block(int b, const uint16_t* __restrict__ q, const float* __rest
 #pragma unroll
         for (int o = IM_HD / 16; o > 0; o >>= 1) m = rv_max_bf16x2(m, __shfl_xor_sync(0xffffffffu, m, o));
         const QuantScale qs = rv_quant_scale(__uint_as_float(m << 16));
-        float n2 = 0.0f;
+        float n1 = 0.0f;
         if (act) {
             uint32_t redo = qs.r == 0.0f ? RV_REDO : 0u;
             uint2 c = rv_codes8(x, qs, redo);
@@ -86,22 +86,22 @@ index_q_prepare_block(int b, const uint16_t* __restrict__ q, const float* __rest
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const float2 lo = rv_e4m3x2_to_f32x2((uint16_t)(cc[i] & 0xffff)), hi = rv_e4m3x2_to_f32x2((uint16_t)(cc[i] >> 16));
-                n2 += lo.x * lo.x + lo.y * lo.y + hi.x * hi.x + hi.y * hi.y;
+                n1 += fabsf(lo.x) + fabsf(lo.y) + fabsf(hi.x) + fabsf(hi.y);
             }
         }
 #pragma unroll
-        for (int o = IM_HD / 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+        for (int o = IM_HD / 16; o > 0; o >>= 1) n1 += __shfl_xor_sync(0xffffffffu, n1, o);
         if (lane == 0) {
             scales[v] = qs.s;
-            term[h] = fabsf(wv * wscale) * dscale * qs.s * sqrtf(n2);
+            term[h] = fabsf(wv * wscale) * dscale * qs.s * n1;
         }
     }
     __syncthreads();
     if (threadIdx.x < 32) {
         const float sum = rv_warp_sum(lane < nh ? term[lane] : 0.0f);
-        // ||kcode||_2 <= sqrt(hd) * 448; 1.01 covers the roundings of this very sum
+        // no key code is larger than 448; 1.01 covers the roundings of this very sum
         if (lane == 0) {
-            cb[b] = sum * sqrtf((float)hd) * 448.0f * IM_EPS_REL * 1.01f;
+            cb[b] = sum * 448.0f * IM_EPS_REL * 1.01f;
             if (b == 0) *err = 0;   // the scorer's error word starts clean on every call
         }
     }
@@ -563,7 +563,7 @@ static int select_impl(const DsaGeom* g, const AppendArgs* ap, const uint16_t* i
 
     const SelArgs ra{*g, s.scores, score_stride, seq_len, s.qcodes, s.qscales, w, s.cb,
                      index_pool, index_scale, block_table, rows, n_sel, g->top_k, s.stats,
-                     (score_stride % 4 == 0 && ((uintptr_t)index_scale & 15) == 0 && g->page_tokens % 4 == 0) ? 1 : 0, s.err};
+                     (((uintptr_t)index_scale & 15) == 0 && g->page_tokens % 4 == 0) ? 1 : 0, score_stride % 4 == 0 ? 1 : 0, s.err};
     return rivoli::launch_index_select_cluster(ra, B, st);
 }
 

@@ -231,9 +231,21 @@ index_select_cluster_kernel(SelArgs A, int CH) {
             }
             rv_grid_dep_wait();
         }
+        if (A.vec_scores) {
 #pragma unroll
-        for (int it = 0; it < SEL_STEPS; ++it)
-            sc[it] = it * SEL_STEP + tid * 4 < nloc ? *reinterpret_cast<const float4*>(s + c0 + it * SEL_STEP + tid * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int it = 0; it < SEL_STEPS; ++it)
+                sc[it] = it * SEL_STEP + tid * 4 < nloc ? *reinterpret_cast<const float4*>(s + c0 + it * SEL_STEP + tid * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        } else {                                                          // rows of any length: the same tokens, a score at a time
+#pragma unroll
+            for (int it = 0; it < SEL_STEPS; ++it) {
+                const int i4 = it * SEL_STEP + tid * 4;
+                const float* p = s + c0 + i4;
+                sc[it].x = i4 < nloc ? p[0] : 0.f;
+                sc[it].y = i4 + 1 < nloc ? p[1] : 0.f;
+                sc[it].z = i4 + 2 < nloc ? p[2] : 0.f;
+                sc[it].w = i4 + 3 < nloc ? p[3] : 0.f;
+            }
+        }
 #pragma unroll
         for (int it = 0; it < SEL_STEPS; ++it) {
             const int i4 = it * SEL_STEP + tid * 4;
@@ -737,7 +749,8 @@ int launch_topk_values(const float* scores, long long stride, const int32_t* seq
     SelArgs a{};
     a.scores = scores; a.score_stride = max_nt; a.value_stride = stride; a.seq_len = seq_len; a.nt_single = nt_single;
     a.rows = rows; a.n_sel = n_sel; a.k = k;
-    a.vec_ok = ((uintptr_t)scores & 15) == 0 && stride % 4 == 0 && stride >= max_nt;   // (whole vectors are read)
+    a.vec_ok = 1;
+    a.vec_scores = ((uintptr_t)scores & 15) == 0 && stride % 4 == 0 && stride >= max_nt;   // (whole vectors are read)
     // no re-score to spread: a lone CTA up to 16,384 scores (no exchanges between CTAs; 8,193 scores: 9.7 us,
     // four radix passes over shared memory took 14.2), beyond that clusters of eight
     const int C = max_nt <= SEL_CH ? 1 : SEL_MAX_CLUSTER, ch = ((max_nt + C - 1) / C + 3) / 4 * 4;
