@@ -49,6 +49,7 @@
 // All waits are bounded (tc_common.cuh).
 #include "codec.cuh"
 #include "common.cuh"
+#include "o_merge.cuh"
 #include "quant.cuh"
 #include "tc_common.cuh"
 
@@ -66,7 +67,7 @@ constexpr int AM_HPT = 32;               // head columns of O^T a thread owns in
 constexpr int AM_SOFTMAX_THREADS = AM_SW * 32;
 constexpr int AM_QKW = AM_SW, AM_PVW = AM_SW + 1, AM_GW0 = AM_SW + 2;   // warp roles: QK issue, PV issue, first gather warp
 constexpr int AM_THREADS = (AM_GW0 + AM_GW) * 32;
-constexpr int AM_MAX_SPLITS = 8;     // CTAs per sequence = thread-block cluster size
+constexpr int AM_MAX_SPLITS = om::MAX_N;     // CTAs per sequence = thread-block cluster size
 // P'' = 2^(s2' - m_ref + AM_POFF) with m_ref lagging the true maximum by at most AM_LAG, so
 // P'' <= 2^(AM_POFF + AM_LAG) = 256 < 448 while typical weights (a few binades below the maximum)
 // land where BOTH e4m3 terms are normal numbers. In the code s2 carries the offset (s2 = s2' + AM_POFF)
@@ -99,7 +100,7 @@ constexpr int SM_ZQ = SM_K0 + 3 * SM_KSTAGE;   // q as it arrives: ring stages 3
 constexpr int SM_ZROW = AM_W * 2 + 16;
 static_assert(SM_ZQ + AM_H * SM_ZROW <= SM_K0 + AM_STAGES * SM_KSTAGE, "q fits the last stages");
 constexpr int SM_STAGE = SM_K0;          // epilogue (the ring is idle by then): bf16 [64 heads][512 dims], or f32 [splits][heads][512 dims] received from the cluster
-static_assert((AM_H + AM_MAX_SPLITS) * AM_KVL * 4 <= AM_STAGES * SM_KSTAGE, "the O staging fits the ring");
+static_assert(om::H == AM_H && om::D == AM_KVL && om::recv_floats(AM_MAX_SPLITS) * 4 <= AM_STAGES * SM_KSTAGE, "the O staging fits the ring");
 
 struct AmBars {
     uint64_t k_full[AM_STAGES], k_empty[AM_STAGES], s_full[AM_SBUF], s_empty[AM_SBUF], rope_free[AM_ROPES],
@@ -305,8 +306,6 @@ attend_mma_kernel(AttendMmaArgs A) {
     float2 my_ml = make_float2(-INFINITY, 0.0f);   // a split's reference maximum and weight sum of a head (one thread per head)
     const bool publishes = warp < AM_SW / 2 && lane < 16;                 // that thread
     const int ph = 16 * (warp & 3) + (lane & 15);                         // and its head
-    auto cluster_arrive = []() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); };
-    auto cluster_wait = []() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); };
 
     if (warp >= AM_GW0 && ntiles > 0) {
         // ------------------------------ gather producers ------------------------------------------
@@ -792,117 +791,37 @@ attend_mma_kernel(AttendMmaArgs A) {
     }
 
     if (clustered) {
-        // ---- merge of a sequence's splits inside its thread-block cluster ----
-        // Each CTA PUSHES its O^T, as it is, head by head into the idle ring of the CTA that writes that head (CTA r: the heads
-        // [HZ r / n, HZ (r + 1) / n) of the cluster's HZ), and its reference maximum and weight sum of the head beside it; that CTA brings the n
-        // contributions to the common reference and the total sum while it adds them from its own memory. So nothing has to be
-        // exchanged before the push (maxima and sums first, and O^T scaled by its sender, cost two more barriers and 2 us), and
-        // remote stores need no answer. Distributed shared memory takes 21 bytes a clock, whatever the width of the stores; a CTA's
-        // own share does not go through it.
-        // A batch of a few sequences leaves SMs idle even so: then gridDim.z clusters attend over the same rows, and each pushes
-        // and writes 64 / gridDim.z of the heads (the push and the sums are what a small batch waits for: 5,500 + 2,000 cycles
-        // of its 16,000 behind the last score).
+        // ---- merge of a sequence's splits inside its thread-block cluster (o_merge.cuh) ----
         // All threads of all CTAs take part in both cluster barriers, whatever a bounded wait did before: a CTA that gave up
         // sends weight sums of zero.
-        const int n = A.n_splits;
+        const om::Share S(A.n_splits, split, (int)gridDim.z, (int)blockIdx.z);
         float* recv = reinterpret_cast<float*>(smem + SM_STAGE);              // [n][hpc][512]
         float2* ml = reinterpret_cast<float2*>(smem + SM_QR);                 // [n][hpc]: (maximum, sum) of rank q
         float* wts = reinterpret_cast<float*>(smem + SM_P);                   // [hpc][8]: what rank q's row counts
-        const int lgz = 6 - (31 - __clz((int)gridDim.z)), HZ = 1 << lgz, hz0 = (int)blockIdx.z << lgz;   // the heads that this cluster writes
-        static_assert(AM_H == 1 << 6, "shifts");
-        const int hpc = (HZ + n - 1) / n;
         const bool live = ntiles > 0 && *abort_flag == 0;
-        cluster_arrive();
-        cluster_wait();                                                       // [1] every CTA's MMAs have read their ring and q
+        om::cluster_arrive();
+        om::cluster_wait();                                                   // [1] every CTA's MMAs have read their ring and q
         if (warp < AM_SW) {
-            const int sq = warp & 3, th = warp >> 2;
-            const uint32_t lane_base = ((uint32_t)(sq * 32)) << 16;
-            auto owner_of = [&](int i) { return ((i + 1) * n - 1) >> lgz; };
-            // a warp takes 32 heads: its th's half of them and all dims, or the half that holds the cluster's heads and th's half of the
-            // dims; lane l: where this CTA's row of head win + l goes
-            const int win = HZ == AM_H ? 32 * th : hz0 & 32;
-            const int hl = min(max(win + lane - hz0, 0), HZ - 1), ho = owner_of(hl);
-            const uint32_t own32 = tc::smem_u32(recv + (split * hpc + hl - ho * HZ / n) * AM_KVL);
-            uint32_t to32;
-            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to32) : "r"(own32), "r"(ho));
-            if (ho == split) to32 = own32;                                    // (an address of this CTA's own window)
-            if (publishes && ph >= hz0 && ph < hz0 + HZ) {
-                const int i = ph - hz0, o = owner_of(i);
-                uint32_t m32;
-                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(m32) : "r"(tc::smem_u32(ml + split * hpc + i - o * HZ / n)), "r"(o));
-                asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(m32), "f"(live ? my_ml.x : -INFINITY), "f"(live ? my_ml.y : 0.0f) : "memory");
-            }
-            const int c0 = HZ == AM_H ? 0 : 2 * th, c1 = HZ == AM_H ? 4 : c0 + 2;
-#pragma unroll 1
-            for (int c = c0; c < c1; ++c) {
-                const uint32_t off = (uint32_t)(c * 128 + sq * 32 + lane) * 4u;
-                uint32_t r[32];
-                if (live) {
-                    tc::tmem_ld32(TM_O + lane_base + c * 64 + win, r);
-                    tc::tmem_ld_wait();
-                } else {
-#pragma unroll
-                    for (int h = 0; h < 32; ++h) r[h] = 0u;
-                }
-#pragma unroll
-                for (int h8 = 0; h8 < 32; h8 += 8)
-                    if (win + h8 >= hz0 && win + h8 < hz0 + HZ)
-#pragma unroll
-                        for (int h = h8; h < h8 + 8; ++h) {   // lanes = consecutive dims: 128 bytes per warp store
-                            const uint32_t d = __shfl_sync(0xffffffffu, to32, h);
-                            asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(d + off), "r"(r[h]) : "memory");
-                        }
-            }
+            if (publishes) om::push_stats(S, ml, ph, live ? my_ml : make_float2(-INFINITY, 0.0f));
+            om::push_rows(S, TM_O, recv, live, warp, lane);
         }
-        cluster_arrive();
-        cluster_wait();                                                       // [2] every CTA's share of this CTA's heads
-        // (short loops from here on: code that runs once per launch comes in from L2, at a tenth of the rate that it issues at)
-        const int h_lo = split * HZ / n, heads = (split + 1) * HZ / n - h_lo, hb = hz0 + h_lo;
+        om::cluster_arrive();
+        om::cluster_wait();                                                   // [2] every CTA's share of this CTA's heads
         // eight lanes a head (a lane per rank) work out what each rank's row counts
+        static_assert(om::MAX_N == 8 && AM_H / 2 * 8 <= AM_THREADS, "eight lanes a head, at most half of the heads");
         const int wh = tid >> 3, wq = tid & 7;
-        const bool told = wh < heads && wq < n;
-        const float2 part = told ? ml[wq * hpc + wh] : make_float2(-INFINITY, 0.0f);
-        float mg = part.x, L;
-        static_assert(AM_MAX_SPLITS == 8 && AM_H / 2 * 8 <= AM_THREADS, "eight lanes a head, at most half of the heads");
-#pragma unroll
-        for (int o = 1; o < 8; o <<= 1) mg = fmaxf(mg, __shfl_xor_sync(0xffffffffu, mg, o));
-        {
-            const float w = part.y > 0.0f ? exp2f(part.x - mg) : 0.0f;
-            L = part.y * w;
-#pragma unroll
-            for (int o = 1; o < 8; o <<= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
-            if (told) wts[wh * AM_MAX_SPLITS + wq] = L > 0.0f ? w / L : 0.0f;
-        }
+        const bool told = wh < S.heads && wq < S.n;
+        const float2 part = told ? ml[wq * S.hpc + wh] : make_float2(-INFINITY, 0.0f);
+        const float mg = om::fold8<false>(part.x), w = part.y > 0.0f ? exp2f(part.x - mg) : 0.0f, L = om::fold8<true>(part.y * w);
+        if (told) wts[wh * om::MAX_N + wq] = L > 0.0f ? w / L : 0.0f;
         __syncthreads();
         if (!skip) {
-#pragma unroll 1
-            for (int e = tid; e < heads * (AM_KVL / 4); e += AM_THREADS) {
-                const int hl = e / (AM_KVL / 4), d4 = e % (AM_KVL / 4);
-                float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll 1
-                for (int q0 = 0; q0 < n; q0 += 4) {
-                    const float4 w4 = *reinterpret_cast<const float4*>(wts + hl * AM_MAX_SPLITS + q0);
-                    const float w[4] = {w4.x, w4.y, w4.z, w4.w};
-                    float4 v[4];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        if (q0 + q < n) v[q] = *reinterpret_cast<const float4*>(recv + ((q0 + q) * hpc + hl) * AM_KVL + d4 * 4);
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        if (q0 + q < n) {
-                            acc.x = fmaf(v[q].x, w[q], acc.x); acc.y = fmaf(v[q].y, w[q], acc.y);
-                            acc.z = fmaf(v[q].z, w[q], acc.z); acc.w = fmaf(v[q].w, w[q], acc.w);
-                        }
-                }
-                uint32_t w0, w1;
-                asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w0) : "f"(acc.y), "f"(acc.x));
-                asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w1) : "f"(acc.w), "f"(acc.z));
-                *reinterpret_cast<uint2*>(A.out + ((size_t)b * AM_H + hb + hl) * AM_KVL + d4 * 4) = make_uint2(w0, w1);
-            }
+            om::write_rows(S, recv, wts, A.out + (size_t)b * AM_H * AM_KVL, tid, AM_THREADS);
             if (wq == 0 && told) {
+                const size_t at = (size_t)b * AM_H + S.hz0 + S.lo + wh;
                 const float m_nat = (mg - AM_POFF) * 0.6931471805599453f;
-                if (A.out_m) A.out_m[(size_t)b * AM_H + hb + wh] = L > 0.0f ? m_nat : -INFINITY;
-                if (A.out_lse) A.out_lse[(size_t)b * AM_H + hb + wh] = L > 0.0f ? m_nat + logf(L) : -INFINITY;
+                if (A.out_m) A.out_m[at] = L > 0.0f ? m_nat : -INFINITY;
+                if (A.out_lse) A.out_lse[at] = L > 0.0f ? m_nat + logf(L) : -INFINITY;
             }
         }
     }
@@ -919,7 +838,7 @@ attend_mma_kernel(AttendMmaArgs A) {
 // A CTA takes a whole SM (shared memory), and the CTAs of a sequence form one thread-block cluster (co-scheduled
 // inside a GPC). A batch is split only as far as all its clusters are resident at once: the largest cluster size
 // (<= 8) for which the device reports room for B clusters; anything more would run as a second wave. What room is left then
-// goes to clusters that share a sequence's heads (a power of two of them, eight heads or more and a head per CTA each).
+// goes to clusters that share a sequence's heads.
 struct MmaPlan { int splits, shares; };
 MmaPlan mma_plan(int B) {
     constexpr int MOST = 128;
@@ -941,8 +860,7 @@ MmaPlan mma_plan(int B) {
         (void)cudaGetLastError();
     }
     if (n < 1) n = 1;
-    int z = 1;
-    while (n > 1 && z < 8 && AM_H / (2 * z) >= n && 2 * z * B <= active) z *= 2;
+    const int z = om::shares(n, B, active);
     cache[B].store(n + 256 * z, std::memory_order_relaxed);
     return {n, z};
 }

@@ -1,14 +1,11 @@
 // V4 cousin of the decode path, part 2: MQA sparse attention over one shared entry per position, gathered by an
 // explicit index list, with a per-head sink in the softmax denominator.
 // Reference behaviour: crates/backend/kernels/attn.hip:358-465.
-#include <cooperative_groups.h>
-
 #include <atomic>
 
+#include "o_merge.cuh"
 #include "tc_common.cuh"
 #include "v4_common.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace {
 
@@ -117,7 +114,7 @@ __global__ void __launch_bounds__(GA_THREADS) v4_gather_attn_kernel(const T* __r
 constexpr int SA_H = 64, SA_D = 512, SA_TILE = 64;
 constexpr int SA_SW = 8, SA_QKW = 8, SA_PVW = 9, SA_GW0 = 10, SA_GW = 2;
 constexpr int SA_THREADS = (SA_GW0 + SA_GW) * 32, SA_ST = SA_SW * 32;      // threads, softmax threads
-constexpr int SA_MAX_SPLITS = 8;
+constexpr int SA_MAX_SPLITS = om::MAX_N;
 constexpr float SA_LAG = 3.0f;
 constexpr int SA_KSTAGE = SA_TILE * SA_D * 2, SA_CHUNK = SA_TILE * 128;
 constexpr int SA_SQ = 2 * SA_KSTAGE;                       // q: [8 chunks][64 heads][128 B]
@@ -126,14 +123,13 @@ constexpr int SA_PBUF = SA_TILE * SA_H * 2;
 constexpr int SA_WMAX = SA_SP + 2 * SA_PBUF;               // f32 [4][64] exchange between the lane quarters
 constexpr int SA_REF = SA_WMAX + 4 * SA_H * 4;             // f32 [64] reference maxima
 constexpr int SA_FAC = SA_REF + SA_H * 4;                  // f32 [64] rescale of O^T; 1 / denominator in the epilogue
-constexpr int SA_XS = SA_FAC + SA_H * 4;                   // f32 [2][64] (reference, sum), read by the cluster
-constexpr int SA_DST = SA_XS + 2 * SA_H * 4;               // uint2 [64] where a head's row goes, its factor
-constexpr int SA_BARS = SA_DST + SA_H * 8;
+constexpr int SA_ML = SA_FAC + SA_H * 4;                   // float2 [n][hpc] (reference, sum) of this CTA's heads, from the cluster
+constexpr int SA_BARS = SA_ML + (SA_H + SA_MAX_SPLITS) * 8;
 constexpr int SA_MISC = SA_BARS + 128;
 constexpr int SA_TOTAL = SA_MISC + 16;
 constexpr int SA_TMO = 0, SA_TMS = 256;                    // tensor memory columns
 static_assert(SA_TOTAL <= 232448, "shared memory budget");
-static_assert((SA_H + SA_MAX_SPLITS) * SA_D * 4 <= SA_SP, "the merge buffers fit the tiles and q");
+static_assert(om::H == SA_H && om::D == SA_D && om::recv_floats(SA_MAX_SPLITS) * 4 <= SA_SP, "the merge buffers fit the tiles and q");
 __device__ int g_sa_err;
 
 struct SaBars { uint64_t k_full[2], k_empty[2], s_full[2], s_empty[2], p_full[2], q_full; };
@@ -183,7 +179,6 @@ __global__ void __launch_bounds__(SA_THREADS, 1) v4_sparse_attend_kernel(SaArgs 
     float* s_wmax = reinterpret_cast<float*>(sa_smem + SA_WMAX);
     float* s_ref = reinterpret_cast<float*>(sa_smem + SA_REF);
     float* s_fac = reinterpret_cast<float*>(sa_smem + SA_FAC);
-    float* xs = reinterpret_cast<float*>(sa_smem + SA_XS);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sa_smem + SA_MISC);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sa_smem + SA_MISC + 4);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -191,6 +186,7 @@ __global__ void __launch_bounds__(SA_THREADS, 1) v4_sparse_attend_kernel(SaArgs 
     const int32_t* ix = A.sel + (size_t)b * A.cols;
     const int tiles_all = (A.cols + SA_TILE - 1) / SA_TILE, tps = (tiles_all + A.n_splits - 1) / A.n_splits;
     const int t0 = split * tps, ntiles = max(0, min(tiles_all, t0 + tps) - t0);
+    float2 my_ml = make_float2(-INFINITY, 0.0f);         // a split's reference maximum and weight sum of head tid
 
     if (tid == 0) {
 #pragma unroll
@@ -386,18 +382,17 @@ __global__ void __launch_bounds__(SA_THREADS, 1) v4_sparse_attend_kernel(SaArgs 
             tc::fence_proxy_async();
             tc::mbar_arrive(&bars.p_full[s]);
         }
-        if (ok) ok = tc::mbar_wait_warp(&bars.k_empty[(ntiles - 1) & 1], ((ntiles - 1) >> 1) & 1, abort_flag, 98);
-        tc::tc_fence_after();
         tc::named_barrier(1, SA_ST);
         s_wmax[sq * SA_H + 32 * th + lane] = sa_fold16<true>(l_acc, lane);
         tc::named_barrier(1, SA_ST);
         if (tid < SA_H) {
             const float l = (s_wmax[tid] + s_wmax[SA_H + tid]) + (s_wmax[2 * SA_H + tid] + s_wmax[3 * SA_H + tid]), m = s_ref[tid];
-            xs[tid] = m;
-            xs[SA_H + tid] = l;
+            my_ml = make_float2(m, l);
             // the sink joins the denominator only, shifted by the same maximum; a query with every slot masked is loud
             s_fac[tid] = m == -INFINITY ? NAN : 1.0f / (l + v4_ex2(A.sink[tid] * 1.4426950408889634f - m));
         }
+        if (ok) ok = tc::mbar_wait_warp(&bars.k_empty[(ntiles - 1) & 1], ((ntiles - 1) >> 1) & 1, abort_flag, 98);
+        tc::tc_fence_after();
         tc::named_barrier(1, SA_ST);
         // O^T: lane = dim of each 128-dim block. The output is staged in the idle tiles, eight heads at a time, and leaves as
         // 8 KiB bulk copies. (A split sequence is merged in its cluster below.)
@@ -435,74 +430,31 @@ __global__ void __launch_bounds__(SA_THREADS, 1) v4_sparse_attend_kernel(SaArgs 
     }
 
     if (A.n_splits > 1) {
-        // ---- merge: every CTA scales its O^T to the common maximum and the whole denominator and pushes it, head by head,
-        // into the CTA that writes the head. Every thread of every CTA takes part in both cluster barriers.
-        cg::cluster_group cluster = cg::this_cluster();
-        const int n = A.n_splits, hpc = (SA_H + n - 1) / n;
-        float* recv = reinterpret_cast<float*>(sa_smem);                          // [n][hpc][512]
-        uint2* s_dst = reinterpret_cast<uint2*>(sa_smem + SA_DST);
+        // ---- merge inside the cluster (o_merge.cuh). Every thread of every CTA takes part in both cluster barriers; a CTA that
+        // gave up sends sums that make the output NaN.
+        const om::Share S(A.n_splits, split, (int)gridDim.y, (int)blockIdx.y);
+        float* recv = reinterpret_cast<float*>(sa_smem);                      // [n][hpc][512]
+        float2* ml = reinterpret_cast<float2*>(sa_smem + SA_ML);              // [n][hpc]: (maximum, sum) of rank q
+        float* wts = reinterpret_cast<float*>(sa_smem + SA_SP);               // [hpc][8]: what rank q's row counts
+        om::cluster_arrive();
+        om::cluster_wait();                                                   // [1] every CTA's MMAs have read their tiles and q
+        if (warp < SA_SW) {
+            if (tid < SA_H) om::push_stats(S, ml, tid, *abort_flag ? make_float2(0.0f, NAN) : my_ml);
+            om::push_rows(S, TM_O, recv, ntiles > 0, warp, lane);
+        }
+        om::cluster_arrive();
+        om::cluster_wait();                                                   // [2] every CTA's share of this CTA's heads
+        static_assert(om::MAX_N == 8 && SA_H / 2 * 8 <= SA_THREADS, "eight lanes a head, at most half of the heads");
+        const int wh = tid >> 3, wq = tid & 7;
+        const bool told = wh < S.heads && wq < S.n;
+        const float2 part = told ? ml[wq * S.hpc + wh] : make_float2(-INFINITY, 0.0f);
+        const float mg = om::fold8<false>(part.x), w = part.x > -INFINITY ? v4_ex2(part.x - mg) : 0.0f, L = om::fold8<true>(part.y * w);
+        if (told) {
+            const float sink = A.sink[S.hz0 + S.lo + wh] * 1.4426950408889634f;
+            wts[wh * om::MAX_N + wq] = mg == -INFINITY ? NAN : w / (L + v4_ex2(sink - mg));
+        }
         __syncthreads();
-        const bool aborted = *abort_flag != 0;
-        cluster.sync();
-        if (warp < SA_SW) {
-            if (tid < SA_H) {
-                float mq[SA_MAX_SPLITS], lq[SA_MAX_SPLITS], mg = -INFINITY;
-#pragma unroll
-                for (int q = 0; q < SA_MAX_SPLITS; ++q) {                         // all in flight
-                    const float* px = cluster.map_shared_rank(xs, q < n ? q : 0);
-                    mq[q] = q < n ? px[tid] : -INFINITY;
-                    lq[q] = q < n ? px[SA_H + tid] : 0.0f;
-                }
-#pragma unroll
-                for (int q = 0; q < SA_MAX_SPLITS; ++q) mg = fmaxf(mg, mq[q]);
-                float L = v4_ex2(A.sink[tid] * 1.4426950408889634f - mg);
-#pragma unroll
-                for (int q = 0; q < SA_MAX_SPLITS; ++q)
-                    if (mq[q] > -INFINITY) L += lq[q] * v4_ex2(mq[q] - mg);
-                const float fac = (mg == -INFINITY || aborted) ? NAN : (xs[tid] == -INFINITY ? 0.0f : v4_ex2(xs[tid] - mg) / L);
-                const int owner = ((tid + 1) * n - 1) / SA_H;
-                uint32_t to;
-                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(tc::smem_u32(recv + (split * hpc + tid - owner * SA_H / n) * SA_D)), "r"(owner));
-                s_dst[tid] = make_uint2(to, __float_as_uint(fac));
-            }
-            tc::named_barrier(1, SA_ST);
-            const int sq = warp & 3, th = warp >> 2;
-#pragma unroll 1
-            for (int c = 0; c < 4; ++c) {
-                const uint32_t off = (uint32_t)(c * 128 + sq * 32 + lane) * 4u;
-                uint32_t r[32];
-                if (ntiles > 0) {
-                    tc::tmem_ld32(TM_O + c * SA_H + (((uint32_t)(sq * 32)) << 16) + 32 * th, r);
-                    tc::tmem_ld_wait();
-                } else {
-#pragma unroll
-                    for (int h = 0; h < 32; ++h) r[h] = 0u;
-                }
-#pragma unroll
-                for (int h = 0; h < 32; ++h) {
-                    const uint2 d = s_dst[32 * th + h];
-                    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(d.x + off), "f"(__uint_as_float(r[h]) * __uint_as_float(d.y)) : "memory");
-                }
-            }
-        }
-        cluster.sync();
-        if (warp < SA_SW) {
-            const int h0 = split * SA_H / n, h1 = (split + 1) * SA_H / n;
-            for (int e = tid; e < (h1 - h0) * (SA_D / 4); e += SA_ST) {
-                const int hl = e / (SA_D / 4), d4 = e % (SA_D / 4);
-                float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll
-                for (int q = 0; q < SA_MAX_SPLITS; ++q)
-                    if (q < n) {
-                        const float4 v = *reinterpret_cast<const float4*>(recv + (q * hpc + hl) * SA_D + d4 * 4);
-                        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-                    }
-                uint2 w;
-                asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w.x) : "f"(acc.y), "f"(acc.x));
-                asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w.y) : "f"(acc.w), "f"(acc.z));
-                *reinterpret_cast<uint2*>(A.out + ((size_t)b * SA_H + h0 + hl) * SA_D + d4 * 4) = w;
-            }
-        }
+        om::write_rows(S, recv, wts, A.out + (size_t)b * SA_H * SA_D, tid, SA_THREADS);
     }
     tc::tc_fence_before();
     __syncthreads();
@@ -514,30 +466,41 @@ __global__ void __launch_bounds__(SA_THREADS, 1) v4_sparse_attend_kernel(SaArgs 
 }
 
 // CTAs per sequence: as many as leave all clusters resident at once (at most eight), and no more than there are tiles to
-// share out evenly.
-int sa_splits(int n_seqs, int tiles) {
+// share out evenly; then the clusters that share its heads.
+struct SaPlan { int splits, shares; };
+int sa_resident(int n_seqs, int n) {           // clusters of n CTAs that are resident at once
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(n * n_seqs)); cfg.blockDim = dim3(SA_THREADS); cfg.dynamicSmemBytes = SA_TOTAL;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)n; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    int active = 0;
+    if (cudaOccupancyMaxActiveClusters(&active, v4_sparse_attend_kernel, &cfg) == cudaSuccess) return active;
+    (void)cudaGetLastError();
+    return 0;
+}
+SaPlan sa_plan(int n_seqs, int tiles) {
     constexpr int MOST = 128;
     static std::atomic<int> cache[MOST + 1];   // largest resident cluster size by batch; 0 = not asked yet
+    static std::atomic<int> room[SA_MAX_SPLITS + 1];   // resident clusters by size, plus 1
     const int sms = rv_sm_count();
-    if (n_seqs > MOST || 2 * n_seqs > sms) return 1;
+    if (n_seqs > MOST || 2 * n_seqs > sms) return {1, 1};
     int most = cache[n_seqs].load(std::memory_order_relaxed);
     if (!most) {
-        for (most = sms / n_seqs < SA_MAX_SPLITS ? sms / n_seqs : SA_MAX_SPLITS; most > 1; --most) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((unsigned)(most * n_seqs)); cfg.blockDim = dim3(SA_THREADS); cfg.dynamicSmemBytes = SA_TOTAL;
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = (unsigned)most; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-            cfg.attrs = at; cfg.numAttrs = 1;
-            int active = 0;
-            if (cudaOccupancyMaxActiveClusters(&active, v4_sparse_attend_kernel, &cfg) == cudaSuccess && active >= n_seqs) break;
-            (void)cudaGetLastError();
-        }
+        for (most = sms / n_seqs < SA_MAX_SPLITS ? sms / n_seqs : SA_MAX_SPLITS; most > 1; --most)
+            if (sa_resident(n_seqs, most) >= n_seqs) break;
         if (most < 1) most = 1;
         cache[n_seqs].store(most, std::memory_order_relaxed);
     }
-    const int tps = (tiles + most - 1) / most;
-    return (tiles + tps - 1) / tps;
+    const int tps = (tiles + most - 1) / most, n = (tiles + tps - 1) / tps;
+    if (n < 2) return {1, 1};
+    int active = room[n].load(std::memory_order_relaxed) - 1;
+    if (active < 0) {
+        active = sa_resident(n_seqs, n);
+        room[n].store(active + 1, std::memory_order_relaxed);
+    }
+    return {n, om::shares(n, n_seqs, active)};
 }
 
 }  // namespace
@@ -566,10 +529,11 @@ int rivoli_v4_sparse_attend_launch(const V4Geom* g, int n_seqs, const uint16_t* 
     rv_drain_error();
     if (!force_simt && g->n_heads == SA_H && g->head_dim == SA_D) {
         rv_allow_smem<v4_sparse_attend_kernel>(SA_TOTAL);
-        const int n = sa_splits(n_seqs, (cols + SA_TILE - 1) / SA_TILE);
+        const SaPlan plan = sa_plan(n_seqs, (cols + SA_TILE - 1) / SA_TILE);
+        const int n = plan.splits;
         const SaArgs a{q, kv_cache, kv_rows, sink, sel, cols, n, q_early, g->softmax_scale * 1.4426950408889634f, out};
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)n_seqs * (unsigned)n); cfg.blockDim = dim3(SA_THREADS);
+        cfg.gridDim = dim3((unsigned)n_seqs * (unsigned)n, (unsigned)plan.shares); cfg.blockDim = dim3(SA_THREADS);
         cfg.dynamicSmemBytes = (size_t)SA_TOTAL; cfg.stream = st;
         cudaLaunchAttribute at[2];
         at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
