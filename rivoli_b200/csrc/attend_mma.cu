@@ -348,7 +348,8 @@ attend_mma_kernel(AttendMmaArgs A) {
         auto pool_row = [&](uint32_t t, int32_t pg) -> uint32_t {
             return (t != NONE && pg >= 0 && pg < A.n_pool_pages) ? (uint32_t)pg * (uint32_t)P + (t & (uint32_t)(P - 1)) : NONE;
         };
-        auto load_scl = [&](uint32_t r) -> float { return r != NONE ? A.pscale[r] : 0.0f; };
+        // (not through L1: a line that holds an older scale of a new token may have been read beside the append)
+        auto load_scl = [&](uint32_t r) -> float { return r != NONE ? __ldcg(A.pscale + r) : 0.0f; };
         uint32_t tk[2][AM_LOOK], tok[2][AM_LOOK], row[2][AM_LOOK];
         int32_t pg[2][AM_LOOK];
         float scl[2][AM_LOOK];
@@ -839,30 +840,42 @@ attend_mma_kernel(AttendMmaArgs A) {
 // inside a GPC). A batch is split only as far as all its clusters are resident at once: the largest cluster size
 // (<= 8) for which the device reports room for B clusters; anything more would run as a second wave. What room is left then
 // goes to clusters that share a sequence's heads.
+// A CTA of one tile would leave one of its two softmax groups idle, and two tiles take hardly longer: a list of few rows (a small
+// top_k) is split to two tiles per CTA (15 sequences of 512 rows: 30.0 us a step with eight CTAs each, 28.9 with four; 10 of 256 rows 29.4 with four, 26.8 with two).
 struct MmaPlan { int splits, shares; };
-MmaPlan mma_plan(int B) {
+int mma_resident(int B, int n) {           // clusters of n CTAs that are resident at once
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)n, (unsigned)B); cfg.blockDim = dim3(AM_THREADS); cfg.dynamicSmemBytes = SM_TOTAL;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)n; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    int active = 0;
+    if (cudaOccupancyMaxActiveClusters(&active, attend_mma_kernel, &cfg) == cudaSuccess) return active;
+    (void)cudaGetLastError();
+    return 0;
+}
+MmaPlan mma_plan(int B, long long tiles) {
     constexpr int MOST = 128;
-    static std::atomic<int> cache[MOST + 1];   // by batch: splits + 256 * shares; 0 = not asked yet
+    static std::atomic<int> cache[MOST + 1];            // largest resident cluster size by batch; 0 = not asked yet
+    static std::atomic<int> room[AM_MAX_SPLITS + 1];    // resident clusters by size, plus 1
     const int sms = rv_sm_count();
     if (B <= 0 || B > MOST || 2 * B > sms) return {1, 1};
-    if (const int known = cache[B].load(std::memory_order_relaxed)) return {known & 255, known >> 8};
-    int n = sms / B, active = 0;
-    if (n > AM_MAX_SPLITS) n = AM_MAX_SPLITS;
-    for (; n > 1; --n) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)n, (unsigned)B); cfg.blockDim = dim3(AM_THREADS); cfg.dynamicSmemBytes = SM_TOTAL;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = (unsigned)n; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-        cfg.attrs = at; cfg.numAttrs = 1;
-        active = 0;
-        if (cudaOccupancyMaxActiveClusters(&active, attend_mma_kernel, &cfg) == cudaSuccess && active >= B) break;
-        (void)cudaGetLastError();
+    int n = cache[B].load(std::memory_order_relaxed);
+    if (!n) {
+        for (n = sms / B < AM_MAX_SPLITS ? sms / B : AM_MAX_SPLITS; n > 1; --n)
+            if (mma_resident(B, n) >= B) break;
+        if (n < 1) n = 1;
+        cache[B].store(n, std::memory_order_relaxed);
     }
-    if (n < 1) n = 1;
-    const int z = om::shares(n, B, active);
-    cache[B].store(n + 256 * z, std::memory_order_relaxed);
-    return {n, z};
+    if (2LL * n > tiles + 1) n = (int)((tiles + 1) / 2);
+    if (n < 2) return {1, 1};
+    int active = room[n].load(std::memory_order_relaxed) - 1;
+    if (active < 0) {
+        active = mma_resident(B, n);
+        room[n].store(active + 1, std::memory_order_relaxed);
+    }
+    return {n, om::shares(n, B, active)};
 }
 
 }  // namespace
@@ -918,7 +931,6 @@ extern "C" int rivoli_attend_mma_paged_bf16(const DsaGeom* g, const uint16_t* q,
     cudaStream_t st = (cudaStream_t)stream;
     int* err = reinterpret_cast<int*>(scratch);
     rv_allow_smem<attend_mma_kernel>(SM_TOTAL);
-    const MmaPlan plan = mma_plan(B);
     const int forced = g_am_min_rows_override.load(std::memory_order_relaxed);
     int min_rows = forced >= 0 ? forced : AM_MIN_ROWS;
     if (min_rows_hint >= min_rows) min_rows = 0;          // the caller vouches that no sequence is that short
@@ -929,6 +941,8 @@ extern "C" int rivoli_attend_mma_paged_bf16(const DsaGeom* g, const uint16_t* q,
     long long cap = (long long)g->max_pages_per_seq * g->page_tokens;
     if (rows && row_stride > cap) cap = row_stride;   // (a row list may name a row twice)
     const bool only_short = (cap < max_rows ? cap : max_rows) < min_rows;
+    // (by the length of the list and not by what a step knows of its batch: the same split, and bits, as the operator alone)
+    const MmaPlan plan = mma_plan(B, ((rows ? (long long)row_stride : cap) + AM_TILE - 1) / AM_TILE);
     if (min_rows > 1)
         if (int e = rivoli_attend_simt_short_rows(g, q, latent_pool, latent_scale, block_table, rows, row_stride, n_rows,
                                                   B, out, out_m, out_lse, only_short ? 0 : 1, min_rows, st))

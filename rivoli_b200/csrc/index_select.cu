@@ -40,7 +40,7 @@
 //
 // A whole step, us, with keys in registers and with them here, when that was changed: 4 sequences of 131,072 tokens 85.5 -> 64.2; 32
 // of up to 32,768 88.3 -> 80.5; 64 of 16,384 104.7 -> 92.3; 128 of 16,384 149.0 -> 138.6; 16 of 16,384 65.8 -> 56.9; one of 4,099
-// 42.4 -> 38.0. Other kernels of the step have changed since: 56.9, 65.0, 88.4, 126.2, 49.5 and 34.0 now.
+// 42.4 -> 38.0. Other kernels of the step have changed since, and this one: 52.3 for 4 of 131,072, 125.0 for 128 of 16,384, 29.6 for one of 4,099 now.
 #include <cooperative_groups.h>
 
 #include "codec.cuh"
