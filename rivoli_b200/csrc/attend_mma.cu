@@ -840,8 +840,9 @@ attend_mma_kernel(AttendMmaArgs A) {
 // inside a GPC). A batch is split only as far as all its clusters are resident at once: the largest cluster size
 // (<= 8) for which the device reports room for B clusters; anything more would run as a second wave. What room is left then
 // goes to clusters that share a sequence's heads.
-// A CTA of one tile would leave one of its two softmax groups idle, and two tiles take hardly longer: a list of few rows (a small
-// top_k) is split to two tiles per CTA (15 sequences of 512 rows: 30.0 us a step with eight CTAs each, 28.9 with four; 10 of 256 rows 29.4 with four, 26.8 with two).
+// The split follows the batch alone: cut to two tiles per CTA where the list is short, the same rows gave other bits in a list of
+// another length, 1.2 % further from their 64-bit value (each CTA has reference maxima of its own, and fewer of them serve the
+// same rows); steps of one to four sequences of 256 - 1,024 tokens took 2 - 12 % longer so, of eight to twenty 4 - 12 % less.
 struct MmaPlan { int splits, shares; };
 int mma_resident(int B, int n) {           // clusters of n CTAs that are resident at once
     cudaLaunchConfig_t cfg = {};
@@ -855,7 +856,7 @@ int mma_resident(int B, int n) {           // clusters of n CTAs that are reside
     (void)cudaGetLastError();
     return 0;
 }
-MmaPlan mma_plan(int B, long long tiles) {
+MmaPlan mma_plan(int B) {
     constexpr int MOST = 128;
     static std::atomic<int> cache[MOST + 1];            // largest resident cluster size by batch; 0 = not asked yet
     static std::atomic<int> room[AM_MAX_SPLITS + 1];    // resident clusters by size, plus 1
@@ -868,7 +869,6 @@ MmaPlan mma_plan(int B, long long tiles) {
         if (n < 1) n = 1;
         cache[B].store(n, std::memory_order_relaxed);
     }
-    if (2LL * n > tiles + 1) n = (int)((tiles + 1) / 2);
     if (n < 2) return {1, 1};
     int active = room[n].load(std::memory_order_relaxed) - 1;
     if (active < 0) {
@@ -941,8 +941,7 @@ extern "C" int rivoli_attend_mma_paged_bf16(const DsaGeom* g, const uint16_t* q,
     long long cap = (long long)g->max_pages_per_seq * g->page_tokens;
     if (rows && row_stride > cap) cap = row_stride;   // (a row list may name a row twice)
     const bool only_short = (cap < max_rows ? cap : max_rows) < min_rows;
-    // (by the length of the list and not by what a step knows of its batch: the same split, and bits, as the operator alone)
-    const MmaPlan plan = mma_plan(B, ((rows ? (long long)row_stride : cap) + AM_TILE - 1) / AM_TILE);
+    const MmaPlan plan = mma_plan(B);
     if (min_rows > 1)
         if (int e = rivoli_attend_simt_short_rows(g, q, latent_pool, latent_scale, block_table, rows, row_stride, n_rows,
                                                   B, out, out_m, out_lse, only_short ? 0 : 1, min_rows, st))
