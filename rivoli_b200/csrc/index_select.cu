@@ -133,7 +133,9 @@ __device__ __forceinline__ void sel_token_excl(uint32_t mask, SelXc& xc, uint32_
     }
 }
 
-template <bool VALUES, bool SOLO>
+// VEC: the score rows allow 16-byte loads (a kernel of its own: both forms in one cost the clusters' kernel a spill of 8 bytes, and
+// given scores, which take the loop further below instead, four predicated steps for the one or two that hold scores).
+template <bool VALUES, bool SOLO, bool VEC>
 __global__ void __launch_bounds__(SEL_NT, 1)
 index_select_cluster_kernel(SelArgs A, int CH) {
     cg::cluster_group cluster = cg::this_cluster();
@@ -221,7 +223,7 @@ index_select_cluster_kernel(SelArgs A, int CH) {
         for (int i = tid; i < SEL_LIST; i += SEL_NT) a_cmp[i] = 0ull;
     if constexpr (!VALUES) qf[tid] = qw;
     if (tid == 0) { xc.list_n = 0; xc.lower = 0; }
-    if (A.vec_ok) {
+    if (VALUES ? VEC : A.vec_ok != 0) {
         float4 sk[SEL_STEPS], sc[SEL_STEPS];
         if constexpr (!VALUES) {
 #pragma unroll
@@ -231,35 +233,32 @@ index_select_cluster_kernel(SelArgs A, int CH) {
             }
             rv_grid_dep_wait();
         }
-        if (A.vec_scores) {
+        // (rows of any length: the same tokens, a score at a time, two steps in flight; all four cost a spill of 16 bytes)
+        constexpr int AHEAD = VEC ? SEL_STEPS : 2;
 #pragma unroll
-            for (int it = 0; it < SEL_STEPS; ++it)
-                sc[it] = it * SEL_STEP + tid * 4 < nloc ? *reinterpret_cast<const float4*>(s + c0 + it * SEL_STEP + tid * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-        } else {                                                          // rows of any length: the same tokens, a score at a time
+        for (int it0 = 0; it0 < SEL_STEPS; it0 += AHEAD) {
 #pragma unroll
-            for (int it = 0; it < SEL_STEPS; ++it) {
-                const int i4 = it * SEL_STEP + tid * 4;
+            for (int u = 0; u < AHEAD; ++u) {
+                const int i4 = (it0 + u) * SEL_STEP + tid * 4;
                 const float* p = s + c0 + i4;
-                sc[it].x = i4 < nloc ? p[0] : 0.f;
-                sc[it].y = i4 + 1 < nloc ? p[1] : 0.f;
-                sc[it].z = i4 + 2 < nloc ? p[2] : 0.f;
-                sc[it].w = i4 + 3 < nloc ? p[3] : 0.f;
+                if constexpr (VEC) sc[u] = i4 < nloc ? *reinterpret_cast<const float4*>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+                else sc[u] = make_float4(i4 < nloc ? p[0] : 0.f, i4 + 1 < nloc ? p[1] : 0.f, i4 + 2 < nloc ? p[2] : 0.f, i4 + 3 < nloc ? p[3] : 0.f);
             }
-        }
 #pragma unroll
-        for (int it = 0; it < SEL_STEPS; ++it) {
-            const int i4 = it * SEL_STEP + tid * 4;
-            if (i4 < nloc) {
-                float v[4] = {sc[it].x, sc[it].y, sc[it].z, sc[it].w};
-                if constexpr (!VALUES) {
-                    const float k4[4] = {sk[it].x, sk[it].y, sk[it].z, sk[it].w};
+            for (int u = 0; u < AHEAD; ++u) {
+                const int it = it0 + u, i4 = it * SEL_STEP + tid * 4;
+                if (i4 < nloc) {
+                    float v[4] = {sc[u].x, sc[u].y, sc[u].z, sc[u].w};
+                    if constexpr (!VALUES) {
+                        const float k4[4] = {sk[it].x, sk[it].y, sk[it].z, sk[it].w};
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        v[e] *= k4[e];
-                        if (i4 + e < nloc) skm = fmaxf(skm, k4[e]);
+                        for (int e = 0; e < 4; ++e) {
+                            v[e] *= k4[e];
+                            if (i4 + e < nloc) skm = fmaxf(skm, k4[e]);
+                        }
                     }
+                    take4(i4, v);
                 }
-                take4(i4, v);
             }
         }
     } else {
@@ -761,7 +760,7 @@ extern "C" __attribute__((visibility("default"))) void rivoli_index_select_test_
 
 namespace rivoli {
 
-template <bool VALUES, bool SOLO>
+template <bool VALUES, bool SOLO, bool VEC>
 static int launch_select(const SelArgs& a, int B, int C, int ch, cudaStream_t st) {
     constexpr size_t fixed = SEL_BINS + 4 * SEL_LIST + (VALUES ? SEL_BINS : SEL_NW * SEL_HD * 4 + RS_QWORDS) + (SOLO ? 0 : 2 * SEL_LIST);
     static_assert((fixed + SEL_CH) * 4 + sizeof(SelXc) + 1024 <= 232448, "shared memory budget");
@@ -775,15 +774,16 @@ static int launch_select(const SelArgs& a, int B, int C, int ch, cudaStream_t st
     at[1].val.clusterDim.x = (unsigned)C; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
     cfg.attrs = at; cfg.numAttrs = 2;
     rv_drain_error();
-    rv_allow_smem<index_select_cluster_kernel<VALUES, SOLO>>((int)((fixed + SEL_CH) * 4));
-    (void)cudaLaunchKernelEx(&cfg, index_select_cluster_kernel<VALUES, SOLO>, a, ch);
+    rv_allow_smem<index_select_cluster_kernel<VALUES, SOLO, VEC>>((int)((fixed + SEL_CH) * 4));
+    (void)cudaLaunchKernelEx(&cfg, index_select_cluster_kernel<VALUES, SOLO, VEC>, a, ch);
     return rv_launch_status();
 }
 
 int launch_index_select_cluster(const SelArgs& a, int B, cudaStream_t st) {
     int C = 1, ch = 0;
     if (!select_cluster_plan(B, a.score_stride, &C, &ch)) return 1002;
-    return C == 1 ? launch_select<false, true>(a, B, C, ch, st) : launch_select<false, false>(a, B, C, ch, st);
+    if (a.vec_scores) return C == 1 ? launch_select<false, true, true>(a, B, C, ch, st) : launch_select<false, false, true>(a, B, C, ch, st);
+    return C == 1 ? launch_select<false, true, false>(a, B, C, ch, st) : launch_select<false, false, false>(a, B, C, ch, st);
 }
 
 int launch_topk_values(const float* scores, long long stride, const int32_t* seq_len, int nt_single, int B, int k,
@@ -798,12 +798,12 @@ int launch_topk_values(const float* scores, long long stride, const int32_t* seq
     SelArgs a{};
     a.scores = scores; a.score_stride = max_nt; a.value_stride = stride; a.seq_len = seq_len; a.nt_single = nt_single;
     a.rows = rows; a.n_sel = n_sel; a.k = k;
-    a.vec_ok = 1;
     a.vec_scores = ((uintptr_t)scores & 15) == 0 && stride % 4 == 0 && stride >= max_nt;   // (whole vectors are read)
     // no re-score to spread: a lone CTA up to 16,384 scores (no exchanges between CTAs; 8,193 scores: 9.7 us,
     // four radix passes over shared memory took 14.2), beyond that clusters of eight
     const int C = max_nt <= SEL_CH ? 1 : SEL_MAX_CLUSTER, ch = ((max_nt + C - 1) / C + 3) / 4 * 4;
-    return C == 1 ? launch_select<true, true>(a, B, C, ch, st) : launch_select<true, false>(a, B, C, ch, st);
+    if (a.vec_scores) return C == 1 ? launch_select<true, true, true>(a, B, C, ch, st) : launch_select<true, false, true>(a, B, C, ch, st);
+    return C == 1 ? launch_select<true, true, false>(a, B, C, ch, st) : launch_select<true, false, false>(a, B, C, ch, st);
 }
 
 }  // namespace rivoli

@@ -16,7 +16,7 @@ struct SelArgs {
     const uint8_t* index_pool; const float* index_scale; const int32_t* block_table;
     uint32_t* rows; int32_t* n_sel; int k;
     unsigned int* stats;   // [B][2]: band size, sure-in count (may be NULL)
-    int vec_ok;            // key scales allow 16-byte loads
+    int vec_ok;            // key scales allow 16-byte loads (paged scores)
     int vec_scores;        // score rows do
     int* err;              // error word of the scorer
     int nt_single; long long value_stride;   // selection over given scores: tokens when seq_len is NULL, pitch of the score rows
