@@ -88,7 +88,7 @@ kv_append_paged_kernel(DsaGeom g, const uint16_t* __restrict__ latent, const uin
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
     rv_grid_dep_wait();
-    rv_grid_dep_trigger();   // (after the wait: an attention launched behind this reads its q, which is older, at once)
+    rv_grid_dep_trigger();   // (after the wait: an attention launched behind this reads its q, rows, counts and all pool rows but these new ones at once)
     if (row >= n_rows) return;
     AppendRow<PASSES> a;
     append_row_load<PASSES>(a, g, latent, index_key, row, row_seq ? row_seq[row] : row, row_pos[row], block_table, lane);

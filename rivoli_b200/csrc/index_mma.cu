@@ -174,7 +174,7 @@ step_dense_kernel(DsaGeom g, AppendArgs ap, int B, const int32_t* __restrict__ b
                   int score_stride, uint32_t* __restrict__ rows, int32_t* __restrict__ n_sel, unsigned int* __restrict__ stats,
                   int* __restrict__ err) {
     rv_grid_dep_wait();
-    rv_grid_dep_trigger();   // (after the wait: the attention behind this reads its q, which is older, at once)
+    rv_grid_dep_trigger();   // (after the wait: the attention behind this reads its q, the lengths and all pool rows but the new ones at once)
     const int tid = threadIdx.x, blk = (int)blockIdx.x;
     if (blk < B) {
         const int n = min(min(seq_len[blk], score_stride), g.top_k);

@@ -90,3 +90,15 @@ def test_a_wait_that_gave_up_does_not_leave_a_loop_with_barriers(path):
         for h, nested in loops(inside):
             own = own.replace(nested, ";")
         assert not re.search(r"!\s*ok\s*\)\s*(?:\{\s*)?(?:break|return|continue)", own), own[:400]
+
+
+@pytest.mark.parametrize("name", ["kv_append_paged_kernel", "step_dense_kernel", "step_prologue_kernel", "index_q_prepare_kernel", "index_score_mma_kernel"])
+def test_a_kernel_whose_dependents_read_ahead_waits_first(name):
+    """The kernels behind these read what is older than them before their own wait: the attention its q, its row list and counts and
+    all pool rows but the step's new ones, the selection everything but the scores. It is complete only if the kernel between them lets
+    its dependents in behind its own wait."""
+    found = [body(s, m.start()) for s in map(code, SOURCES) for m in re.finditer(r"__global__[^;{]*?\b" + name + r"\s*\(", s)]
+    assert len(found) == 1
+    k = found[0]
+    assert k.count("rv_grid_dep_wait()") == 1 and k.count("rv_grid_dep_trigger()") == 1
+    assert k.index("rv_grid_dep_wait()") < k.index("rv_grid_dep_trigger()")
