@@ -277,6 +277,13 @@ ATTEND_CASES = {
     "cluster-of-6": dict(seed=47, B=24, ctx=[513, 129] + [200 + 29 * i for i in range(22)], top_k=512),
     "cluster-of-5": dict(seed=48, B=29, ctx=[640] + [150 + 17 * i for i in range(28)], top_k=512),
     "cluster-of-3": dict(seed=49, B=40, ctx=[384, 128, 1] + [140 + 11 * i for i in range(37)], top_k=256),
+    # the same with lists that give every CTA of a cluster several tiles, and some sequences fewer tiles than CTAs
+    "full-cluster-of-8": dict(seed=50, B=12, ctx=[2048, 2200, 130, 1025] + [1900 + 60 * i for i in range(8)], top_k=2048),
+    "full-cluster-of-7": dict(seed=51, B=20, ctx=[2048, 2200, 130, 1025] + [1500 + 50 * i for i in range(16)], top_k=2048),
+    "full-cluster-of-6": dict(seed=52, B=24, ctx=[2048, 2200, 130, 900] + [1400 + 50 * i for i in range(20)], top_k=2048),
+    "full-cluster-of-5": dict(seed=53, B=29, ctx=[2048, 2200, 130, 700] + [1300 + 40 * i for i in range(25)], top_k=2048),
+    "full-cluster-of-3": dict(seed=54, B=40, ctx=[2048, 2200, 130, 500] + [1000 + 40 * i for i in range(36)], top_k=2048),
+    "full-cluster-of-2": dict(seed=55, B=60, ctx=[2048, 2200, 130, 300] + [600 + 30 * i for i in range(56)], top_k=2048),
 }
 
 

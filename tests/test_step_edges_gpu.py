@@ -28,8 +28,8 @@ def _layer(st, fill=None):
     return be, g, L
 
 
-def _step(L, st):
-    return L.step(dev(st.new_latent), dev(st.new_key), dev(st.index_q), dev(st.index_w), dev(st.q), dev(st.row_pos), dev(st.seq_len))
+def _step(L, st, **kw):
+    return L.step(dev(st.new_latent), dev(st.new_key), dev(st.index_q), dev(st.index_w), dev(st.q), dev(st.row_pos), dev(st.seq_len), **kw)
 
 
 CASES = {
