@@ -513,7 +513,7 @@ attend_mma_kernel(AttendMmaArgs A) {
         // The two MMA streams, QK(0..n-1) and PV(0..n-1), are each in order and are issued by ONE thread each, from two
         // warps: a warp blocks on the barriers of its own next instruction group only, so neither stream's control
         // latency (barrier observed -> fence -> issue -> commit) sits in the other's way and the tensor pipe takes
-        // whichever group arrives first. QK runs ahead of the softmax by up to the four S buffers / ring stages.
+        // whichever group arrives first. QK runs ahead of the softmax by the two S buffers.
         if (ntiles > 0) {
             const uint32_t id_qk = tc::idesc_e4m3(128, AM_TILE, 0, 0);
             const uint64_t d_qr = smem_desc(tc::smem_u32(smem + SM_QR), 16, 512, 4);

@@ -106,7 +106,8 @@ __global__ void __launch_bounds__(GA_THREADS) v4_gather_attn_kernel(const T* __r
 // 12 warps: 0-7 softmax + epilogue (lane quarter = warp % 4, head half = warp / 4), 8 QK issue, 9 PV issue, 10 and 11 gather
 // (32 rows of every tile each, cp.async; masked slots are zero rows).
 // One CTA per sequence; a batch that leaves SMs idle gets a thread-block cluster per sequence (tiles split evenly, at most
-// eight CTAs), merged by pushing scaled O^T rows into the memory of the CTA that writes the head.
+// eight CTAs), or several that share its heads, merged as o_merge.cuh says: O^T rows are pushed as they are to the CTA that
+// writes the head, which weighs them.
 // Bound by the rows an SM can take in (18 bytes a clock): 640 rows x 128 sequences 57 us with mma.sync (operand reloads from
 // shared memory), 29.7 us now; 3 sequences 55 us on three SMs, 12.9 us now.
 // All waits are bounded (tc_common.cuh); one that gives up makes the sequence's output NaN and sets g_sa_err.
