@@ -580,7 +580,8 @@ attend_mma_kernel(AttendMmaArgs A) {
         // lanes 16-31). The warps are two groups of four that take the tiles in turn, so that the round trips of one tile (to
         // tensor memory, to its barriers, through the shuffles) run beside those of the other: eight warps on one tile spent
         // 2,000 - 2,300 cycles in a row on it, whatever the order, and that was the loop's period (batch 128 x 2,048 rows:
-        // 1.32 us a tile, 1.27 so; there the rows that an SM takes in are the bound now).
+        // 1.32 us a tile, 1.27 so in a step; alone and from cold caches 1.34).
+        // (A lone tile shared by both groups, a half of its tokens each, was 0.3 - 4 % slower: 1 x 256 rows 10.8 -> 11.1 us a step.)
         // After the hi + lo exchange lane l keeps the tokens 32 hf + 16 (l / 16) .. + 15 of each half hf of the tile, of head
         // 16 sq + l % 16.
         // O^T: TMEM lane = latent dim 32 sq + lane of each 128-dim block; in the epilogue th = warp / 4 is the half of the heads.

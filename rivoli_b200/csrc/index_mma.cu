@@ -125,7 +125,9 @@ struct AppendArgs {
     uint8_t* latent_pool; float* latent_scale; uint8_t* index_pool; float* index_scale; int32_t* status;
 };
 
-constexpr int PROLOGUE_ROWS = 4;   // appended by a block: four of them instead of 32, stack of 32 sequences 175.0 -> 173.6 us
+// Rows appended by a block, 32 -> 4, us a step: 32 sequences of 4,096 45.7 -> 44.7, of up to 32,768 61.8 -> 61.0, 64 of 8,192 68.8 -> 68.2;
+// 1, 2, 8 and 128 sequences the same within 0.2 %.
+constexpr int PROLOGUE_ROWS = 4;
 __global__ void __launch_bounds__(1024)
 step_prologue_kernel(DsaGeom g, AppendArgs ap, int B, const uint16_t* __restrict__ q, const float* __restrict__ w,
                      uint8_t* __restrict__ codes, float* __restrict__ scales, float* __restrict__ cb,

@@ -40,7 +40,7 @@
 //
 // A whole step, us, with keys in registers and with them here, when that was changed: 4 sequences of 131,072 tokens 85.5 -> 64.2; 32
 // of up to 32,768 88.3 -> 80.5; 64 of 16,384 104.7 -> 92.3; 128 of 16,384 149.0 -> 138.6; 16 of 16,384 65.8 -> 56.9; one of 4,099
-// 42.4 -> 38.0. Other kernels of the step have changed since, and this one: 52.3 for 4 of 131,072, 125.0 for 128 of 16,384, 29.6 for one of 4,099 now.
+// 42.4 -> 38.0. Other kernels of the step have changed since, and this one: 52.5 for 4 of 131,072, 129 for 128 of 16,384, 29.3 for one of 4,099 now.
 #include <cooperative_groups.h>
 
 #include "codec.cuh"
@@ -134,7 +134,8 @@ __device__ __forceinline__ void sel_token_excl(uint32_t mask, SelXc& xc, uint32_
 }
 
 // VEC: the score rows allow 16-byte loads (a kernel of its own: both forms in one cost the clusters' kernel a spill of 8 bytes, and
-// given scores, which take the loop further below instead, four predicated steps for the one or two that hold scores).
+// given scores, which take the loop further below instead, four predicated steps for the one or two that hold scores). us a step or
+// pass with both in one -> apart: 1 x 4,099 30.2 -> 29.3, 2 x 15,001 34.0 -> 33.6, 1 x 1,024 23.8 -> 22.5, operators at 8,193 123.0 -> 122.7.
 template <bool VALUES, bool SOLO, bool VEC>
 __global__ void __launch_bounds__(SEL_NT, 1)
 index_select_cluster_kernel(SelArgs A, int CH) {
