@@ -688,12 +688,13 @@ index_select_cluster_kernel(SelArgs A, int CH) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// The same selection over at most 1024 given scores: a thread per score, one CTA per sequence. The k-th largest key is found bit
+// The same selection over at most 768 given scores: a thread per score, one CTA per sequence. The k-th largest key is found bit
 // by bit from the top, a barrier that counts per bit; ties at it go to the lower indices. Bound by its 32 barriers (1 us with nine
-// warps). 257 scores in a step of one short sequence: 16.8 us a step with the kernel above, 15.3 with this one, which reads the scores
-// once and keeps nothing but a key per thread.
+// warps; they take longer the more warps meet at them). It reads the scores once and keeps nothing but a key per thread. us a step of
+// the 16-head layer, the kernel above -> this one: one sequence of 100 tokens 16.7 -> 14.8, 257 16.6 -> 15.3, 512 16.7 -> 15.8, 768 16.8
+// both, 1,024 16.8 -> 17.6; four of 640 18.2 -> 17.7, 1,024 18.2 -> 21.2; eight of 768 19.4 -> 19.1, 896 19.3 -> 19.4. So up to 768.
 // ---------------------------------------------------------------------------------------------
-constexpr int SEL_SMALL = 1024;
+constexpr int SEL_SMALL = 768;
 
 __global__ void __launch_bounds__(SEL_SMALL)
 index_select_small_kernel(const float* __restrict__ scores, long long stride, const int32_t* __restrict__ seq_len, int nt_single,

@@ -1,4 +1,4 @@
-"""The selection over at most 1,024 given scores (a key per thread) at the edges of its warps and of its range, against the
+"""The selection over few given scores (a key per thread up to 768, the large kernel beyond) at the edges of its warps and of its range, against the
 oracle: ties, zeros of both signs, infinities, counts of none, one, all but one and all."""
 import numpy as np
 import pytest
@@ -23,7 +23,7 @@ def _scores(kind, b, n, rng):
     return s
 
 
-@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 257, 1023, 1024, 1025])
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 257, 767, 768, 769, 1023, 1024, 1025])
 @pytest.mark.parametrize("kind", ["spread", "ties", "equal", "special"])
 def test_rows_of_few_scores(n, kind):
     from rivoli_b200 import backend as be
