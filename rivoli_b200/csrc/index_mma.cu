@@ -125,11 +125,11 @@ struct AppendArgs {
     uint8_t* latent_pool; float* latent_scale; uint8_t* index_pool; float* index_scale; int32_t* status;
 };
 
-// Rows appended by a block, 32 -> 4, us a step: 32 sequences of 4,096 45.7 -> 44.7, of up to 32,768 61.8 -> 61.0, 64 of 8,192 68.8 -> 68.2;
-// 1, 2, 8 and 128 sequences the same within 0.2 %.
-constexpr int PROLOGUE_ROWS = 4;
+// Rows appended by a block: 4 while every block has an SM of its own so, else 32. 32 -> 4 rows, us a step: 32 sequences of 4,096 45.7 ->
+// 44.7, of up to 32,768 61.8 -> 61.0, 64 of 8,192 68.8 -> 68.2, 90 of 2,000 - 4,000 38.1 -> 37.2; but 128 of 4,000 - 8,000 58.7 -> 59.6.
+constexpr int PROLOGUE_ROWS_FEW = 4, PROLOGUE_ROWS_MOST = 32;
 __global__ void __launch_bounds__(1024)
-step_prologue_kernel(DsaGeom g, AppendArgs ap, int B, const uint16_t* __restrict__ q, const float* __restrict__ w,
+step_prologue_kernel(DsaGeom g, AppendArgs ap, int B, int per_block, const uint16_t* __restrict__ q, const float* __restrict__ w,
                      uint8_t* __restrict__ codes, float* __restrict__ scales, float* __restrict__ cb,
                      int* __restrict__ err) {
     __shared__ float term[32];
@@ -140,8 +140,8 @@ step_prologue_kernel(DsaGeom g, AppendArgs ap, int B, const uint16_t* __restrict
                               cb, err, term);
         return;
     }
-    const int row = ((int)blockIdx.x - B) * PROLOGUE_ROWS + (threadIdx.x >> 5);
-    if (row >= B || (threadIdx.x >> 5) >= PROLOGUE_ROWS) return;
+    const int row = ((int)blockIdx.x - B) * per_block + (threadIdx.x >> 5);
+    if (row >= B || (int)(threadIdx.x >> 5) >= per_block) return;
     AppendRow<3> a;
     append_row_load<3>(a, g, ap.latent, ap.index_key, row, row, ap.row_pos[row], ap.block_table, threadIdx.x & 31);
     append_row_store<3>(a, g, ap.latent_pool, ap.latent_scale, ap.index_pool, ap.index_scale, ap.status, threadIdx.x & 31);
@@ -538,10 +538,11 @@ static int select_impl(const DsaGeom* g, const AppendArgs* ap, const uint16_t* i
 
     rv_drain_error();
     rv_stage_event(0, st);
-    if (ap)
-        rv_launch_dependent(step_prologue_kernel, dim3((unsigned)(B + (B + PROLOGUE_ROWS - 1) / PROLOGUE_ROWS)), dim3(1024), 0, st, *g, *ap, B, index_q, w, s.qcodes,
+    if (ap) {
+        const int per_block = B + (B + PROLOGUE_ROWS_FEW - 1) / PROLOGUE_ROWS_FEW <= rv_sm_count() ? PROLOGUE_ROWS_FEW : PROLOGUE_ROWS_MOST;
+        rv_launch_dependent(step_prologue_kernel, dim3((unsigned)(B + (B + per_block - 1) / per_block)), dim3(1024), 0, st, *g, *ap, B, per_block, index_q, w, s.qcodes,
                             s.qscales, s.cb, s.err);
-    else
+    } else
         rv_launch_dependent(index_q_prepare_kernel, dim3((unsigned)B), dim3(32 * nh), 0, st, index_q, w, nh, hd, g->index_wscale,
                             g->index_dscale, s.qcodes, s.qscales, s.cb, s.err);
     if (int e = rv_launch_status()) return e;

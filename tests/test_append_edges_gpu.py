@@ -75,3 +75,18 @@ def test_magnitudes_zeros_infinities_and_nans():
 def test_geometries(kvl, rope, hd):
     rng = np.random.RandomState(kvl + hd)
     _append_both(bf16_normal(rng, (19, kvl + rope)), bf16_normal(rng, (19, hd)), kv_lora=kvl, rope_dim=rope, index_dim=hd, index_heads=8)
+
+
+@pytest.mark.parametrize("batch", [1, 4, 5, 117, 118, 119, 128, 129])    # few and many rows a block, the line between them at 148 SMs
+def test_the_append_inside_a_step(batch):
+    """The rows that a step with a selection appends beside its query preparation are those of the append alone."""
+    from oracle.workload import State
+    from tests.test_step_edges_gpu import _layer, _step, dev
+    st = State(97, batch, [200 + b % 3 for b in range(batch)], top_k=64)
+    be, g, a = _layer(st)
+    _, _, b = _layer(st)
+    _step(a, st)
+    b.append(dev(st.new_latent), dev(st.new_key), dev(st.row_pos))
+    be.device_sync(); a.check_status(); b.check_status()
+    for name in ("latent_pool", "latent_scale", "index_pool", "index_scale"):
+        assert torch.equal(getattr(a, name), getattr(b, name))
