@@ -125,8 +125,9 @@ struct AppendArgs {
     uint8_t* latent_pool; float* latent_scale; uint8_t* index_pool; float* index_scale; int32_t* status;
 };
 
-// Rows appended by a block: 4 while every block has an SM of its own so, else 32. 32 -> 4 rows, us a step: 32 sequences of 4,096 45.7 ->
-// 44.7, of up to 32,768 61.8 -> 61.0, 64 of 8,192 68.8 -> 68.2, 90 of 2,000 - 4,000 38.1 -> 37.2; but 128 of 4,000 - 8,000 58.7 -> 59.6.
+// Rows appended by a block: 4, or 8 or 16 where only so every block has an SM of its own, else 32. 32 -> 4 rows, us a step: 32 sequences
+// of 4,096 45.7 -> 44.7, of up to 32,768 61.8 -> 61.0, 64 of 8,192 68.8 -> 68.2, 90 of 2,000 - 4,000 38.1 -> 37.2. At 128 sequences of 900 /
+// 4,000 - 8,000 tokens: 4 rows 36.5 / 59.8, 32 rows 35.9 / 59.2, 8 rows (144 blocks) 35.4 / 58.6; 119 of 900: 35.6, 35.9, 34.6.
 constexpr int PROLOGUE_ROWS_FEW = 4, PROLOGUE_ROWS_MOST = 32;
 __global__ void __launch_bounds__(1024)
 step_prologue_kernel(DsaGeom g, AppendArgs ap, int B, int per_block, const uint16_t* __restrict__ q, const float* __restrict__ w,
@@ -539,7 +540,8 @@ static int select_impl(const DsaGeom* g, const AppendArgs* ap, const uint16_t* i
     rv_drain_error();
     rv_stage_event(0, st);
     if (ap) {
-        const int per_block = B + (B + PROLOGUE_ROWS_FEW - 1) / PROLOGUE_ROWS_FEW <= rv_sm_count() ? PROLOGUE_ROWS_FEW : PROLOGUE_ROWS_MOST;
+        int per_block = PROLOGUE_ROWS_FEW;
+        while (per_block < PROLOGUE_ROWS_MOST && B + (B + per_block - 1) / per_block > rv_sm_count()) per_block *= 2;
         rv_launch_dependent(step_prologue_kernel, dim3((unsigned)(B + (B + per_block - 1) / per_block)), dim3(1024), 0, st, *g, *ap, B, per_block, index_q, w, s.qcodes,
                             s.qscales, s.cb, s.err);
     } else
